@@ -83,6 +83,22 @@ def test_gemm_f32(cuda_device, m, n, k):
     assert torch.equal(alone[0], together[0])
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 68, 32), (3, 8200, 260), (8, 64, 1024), (9, 130, 1028), (33, 2052, 2044), (65, 8200, 516), (130, 20000, 512)])
+def test_gemm_f32_rows_of_pieces(cuda_device, m, n, k):
+    """Rows of whole 16-byte pieces: parts of K, edges of tiles, few rows; row strides beyond the rows."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(12)
+    a, w = torch.randn(m, k + 4, generator=g).cuda()[:, :k], torch.randn(n, k + 8, generator=g).cuda()[:, :k]
+    out = ops.gemm_f32(a, w)
+    # a chain of k FMAs is off by at most k roundings of its partial sums, each within the sum of the products' sizes
+    bound = 2.0 ** -24 * k * (a.abs().double() @ w.abs().double().t())
+    assert bool(((out.double() - a.double() @ w.double().t()).abs() <= bound).all())
+    for rows in (1, 3, 9, 33):
+        if rows < m:
+            assert torch.equal(ops.gemm_f32(a[:rows], w), out[:rows])  # whichever kernel and tile a row meets
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_swiglu_and_bias(cuda_device, dtype):
     from models_b200.kernels import ops
