@@ -13,6 +13,7 @@ LIBRARIES = [
     ("mb_talking_attention", ["talking_attention.cu"], {}),
     ("mb_gated_recurrence", ["gated_recurrence.cu"], {}),
     ("mb_gated_delta", ["gated_delta.cu"], {}),
+    ("mb_gated_delta_chunks", ["gated_delta_chunks.cu"], {}),
     ("mb_gated_attention", ["gated_attention.cu"], {}),
     ("mb_retention", ["retention.cu"], {}),
     ("mb_result_norm", ["result_norm.cu"], {}),

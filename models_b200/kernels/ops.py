@@ -1273,6 +1273,23 @@ def gated_delta_library():
     return load_library("mb_gated_delta", ["gated_delta.cu"])
 
 
+def gated_delta_chunks_library():
+    """The form for long steps."""
+    return load_library("mb_gated_delta_chunks", ["gated_delta_chunks.cu"])
+
+
+DELTA_CHUNK_MIN_ROWS = 64  # steps that bring fewer tokens to every sequence are walked token by token
+
+
+def gated_delta_chunks_takes(conv: torch.Tensor, gate_in: torch.Tensor, gain: torch.Tensor, out: torch.Tensor, dim: int, vdim: int, parts_at,
+                             max_q_len: int) -> bool:
+    """Steps of many tokens, key heads of 64 numbers and value heads of 64 or 128, rows of whole fours that start on one's boundary;
+    `parts_at`: the first columns of the convolved rows' parts."""
+    return (max_q_len >= DELTA_CHUNK_MIN_ROWS and dim == 64 and vdim in (64, 128) and conv.stride(0) % 4 == 0 and conv.data_ptr() % 16 == 0
+            and all(at % 4 == 0 for at in parts_at) and gain.data_ptr() % 16 == 0
+            and all(t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0 for t in (gate_in, out)))
+
+
 CONV_ACTIVATIONS = {None: 0, "silu": 1}
 
 
@@ -1321,14 +1338,15 @@ def short_conv(x: torch.Tensor, weights: torch.Tensor, state: torch.Tensor, stat
 def gated_delta_scan(conv: torch.Tensor, q_at: int, k_at: int, v_at: int, a_in: torch.Tensor, b_in: torch.Tensor, gate_in: torch.Tensor,
                      decay: torch.Tensor, dt_bias: torch.Tensor, gain: torch.Tensor, unit_eps: float, eps: float, state: torch.Tensor,
                      state_offset: int, slots: torch.Tensor, cu_q: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int,
-                     out: torch.Tensor, out_scale: float = 1.0) -> None:
+                     out: torch.Tensor, out_scale: float = 1.0, max_q_len: int = 0) -> None:
     """The gated delta rule over the new tokens of every sequence.  `conv` float32 [tokens, n] holds the convolved q (kv_heads
     heads of `dim` from column q_at), k (from k_at) and v (heads heads of `vdim` from v_at); q and k become unit vectors
-    x / sqrt(sum x^2 + unit_eps), q times dim^-1/2 (in place: `conv` is changed); beta = sigmoid(b_in), g = exp(decay * softplus(a_in + dt_bias)) per head
+    x / sqrt(sum x^2 + unit_eps), q times dim^-1/2 (`conv` may be changed); beta = sigmoid(b_in), g = exp(decay * softplus(a_in + dt_bias)) per head
     (decay = -exp(A_log)); per head, from the sequence's float32 state S [heads, dim, vdim] at `state_offset` floats into its
     row of `state` (updated in place): S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q; out = out_scale * o / rms(o)
     * gain * silu(gate_in), rms over the head (eps `eps`).  a_in, b_in [tokens, heads], gate_in and out [tokens, heads * vdim]
-    are column slices; a_in, b_in and gate_in share one row stride."""
+    are column slices; a_in, b_in and gate_in share one row stride.  `max_q_len`: the most new tokens of a sequence (0: not known);
+    steps of many tokens are computed in chunks of 64 where the sizes allow it."""
     _cuda(conv, a_in, b_in, gate_in, decay, dt_bias, gain, state, slots, cu_q, out)
     _int32(slots, "slots")
     _int32(cu_q, "cu_q")
@@ -1345,6 +1363,16 @@ def gated_delta_scan(conv: torch.Tensor, q_at: int, k_at: int, v_at: int, a_in: 
         if t.dtype != torch.float32 or t.numel() != n or not t.is_contiguous():
             raise KernelError(f"gated_delta_scan: {name} must be contiguous float32 of {n} elements")
     rows, stride = _state_rows(state, state_offset, heads * dim * vdim, "gated_delta_scan")
+    if gated_delta_chunks_takes(conv, gate_in, gain, out, dim, vdim, (q_at, k_at, v_at), max_q_len):
+        lib = gated_delta_chunks_library()
+        places = tokens // lib.mb_gated_delta_chunk_tokens() + cu_q.numel() - 1
+        scratch = torch.empty((places * heads * (2 * 64 * vdim + 2 * 64 * 64 + 128),), dtype=torch.float32, device=conv.device)
+        _run(lib, lib.mb_gated_delta_chunks(_p(conv), conv.stride(0), _p(a_in), _p(b_in), _p(gate_in), a_in.stride(0), _code(out.dtype), _p(decay),
+                                            _p(dt_bias), _p(gain), ctypes.c_float(unit_eps), ctypes.c_float(eps), rows, stride, _p(slots),
+                                            _p(cu_q), cu_q.numel() - 1, tokens, int(max_q_len), _p(scratch), _p(out), out.stride(0),
+                                            ctypes.c_float(out_scale), heads, kv_heads, dim, vdim, q_at, k_at, v_at, _stream()))
+        _launches[0] += 2  # three kernels: the chunks' systems, the carried states, the results
+        return
     raw = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=conv.device)  # the read-outs, between the walk and the norm
     lib = gated_delta_library()
     _run(lib, lib.mb_gated_delta_scan(_p(conv), conv.stride(0), _p(a_in), _p(b_in), _p(gate_in), a_in.stride(0), _code(out.dtype), _p(decay),

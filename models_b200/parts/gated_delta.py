@@ -83,7 +83,7 @@ class GatedDeltaMixer(SplitPart, Mixer):
                               store_tail=True)
         ops.gated_delta_scan(conv, 0, self.qk_width, 2 * self.qk_width, a_in, b_in, gate, self.decay, self.dt_bias, self.gain,
                              s.unit_eps, s.eps, run.state, 0, batch.slots, batch.cu_q, H, s.num_kv_heads, s.head_dim, s.value_dim,
-                             mid, scale)
+                             mid, scale, max_q_len=batch.max_q_len)
 
 
 register_part("mixer", "gated_delta", GatedDeltaMixer)

@@ -899,3 +899,34 @@ def test_wide_qkv_product_with_rotation_and_cache_write(cuda_device, batch, head
     stored = (kflat.abs().sum(dim=(1, 2)) > 0).sum()
     assert int(stored) == batch - 1  # exactly the rows with a cache position wrote
     assert ops.gemm_tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("lengths", [[64], [1, 127, 64], [65, 0, 200, 63]])
+def test_gated_delta_chunks(cuda_device, dtype, vdim, lengths):
+    """Chunks of 64 against the walk token by token, from states that are not zero: the same float arithmetic in another order."""
+    from models_b200.kernels import ops
+
+    heads, kv_heads, dim = 4, 2, 64
+    g = torch.Generator().manual_seed(21)
+    tokens, width = sum(lengths), 2 * kv_heads * dim + heads * vdim
+    conv = torch.randn(tokens, width, generator=g).cuda()
+    wide = torch.randn(tokens, 2 * heads + heads * vdim, generator=g).to(dtype).cuda()
+    a_in, b_in, gate = wide[:, :heads], wide[:, heads:2 * heads], wide[:, 2 * heads:]
+    decay = -torch.tensor([0.01, 0.5, 4.0, 16.0]).cuda()
+    dt_bias, gain = torch.randn(heads, generator=g).cuda(), (1 + 0.1 * torch.randn(vdim, generator=g)).cuda()
+    state0 = torch.randn(len(lengths) + 1, heads * dim * vdim + 5, generator=g).cuda()
+    slots = torch.arange(len(lengths), dtype=torch.int32).flip(0).contiguous().cuda()
+    cu_q = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    found = []
+    for most in (0, max(lengths)):
+        state, out = state0.clone(), torch.zeros(tokens, heads * vdim, dtype=dtype).cuda()
+        ops.gated_delta_scan(conv.clone(), 0, kv_heads * dim, 2 * kv_heads * dim, a_in, b_in, gate, decay, dt_bias, gain, 1e-6, 1e-6, state, 3,
+                             slots, cu_q, heads, kv_heads, dim, vdim, out, 0.5, max_q_len=most)
+        found.append((out.float(), state))
+    (out, state), (chunk_out, chunk_state) = found
+    # sums of at most 64 + 64 products a token either way; the states' numbers are of size one to ten
+    assert torch.allclose(chunk_state, state, rtol=1e-4, atol=1e-4)
+    assert torch.equal(chunk_state[:, :3], state0[:, :3]) and torch.equal(chunk_state[-1], state0[-1])
+    close(chunk_out, out, dtype, scale=4.0)
