@@ -145,10 +145,53 @@ argmax_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
     cluster_leave_together();  // (the first block has read the others' results)
 }
 
-// The candidates (probability, id) in shared memory, unused entries (-1, max int): sorted by probability
-// descending and id ascending (bitonic over the smallest power of two that holds k), cut at the shortest prefix whose mass
-// reaches `nucleus` (crossing token included), then the inverse-CDF draw r = u * kept mass.
-// `grown`: where the picked id is stored a second time (the end of the row's history), or null.
+// From candidates in order (probability descending, id ascending), entries behind them -1: cut at the shortest prefix whose mass
+// reaches `nucleus` (crossing token included), then the inverse-CDF draw r = u * kept mass.  The first warp; `sorted_p` is
+// overwritten with the running masses.  `grown`: where the picked id is stored a second time (the end of the row's history), or null.
+__device__ __forceinline__ void pick_sorted(float* sorted_p, const int* sorted_id, int k, float nucleus, float u, int* out, int* grown) {
+    const int lane = threadIdx.x;
+    if (lane >= 32) return;
+    int cutoff = k;
+    float cumulative = 0.0f;
+    if (lane == 0) {
+        // one chain of additions in order; four at a time, so that it waits for shared memory a quarter as often
+        for (int i = 0; i < k && cutoff == k; i += 4) {
+            const float4 p = *reinterpret_cast<const float4*>(sorted_p + i);
+            const float next[4] = {p.x, p.y, p.z, p.w};
+            float running[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (i + j >= k) break;
+                cumulative += next[j];
+                running[j] = cumulative;
+                if (cumulative >= nucleus) {
+                    cutoff = i + j + 1;
+                    break;
+                }
+            }
+            *reinterpret_cast<float4*>(sorted_p + i) = make_float4(running[0], running[1], running[2], running[3]);
+            if (cumulative >= nucleus) break;
+        }
+    }
+    __syncwarp();
+    cutoff = __shfl_sync(0xffffffffu, cutoff, 0);
+    const float target = u * __shfl_sync(0xffffffffu, cumulative, 0);
+    int at = cutoff - 1;  // (rounding may leave the target unreached)
+    for (int base = 0; base < cutoff; base += 32) {
+        const unsigned reached = __ballot_sync(0xffffffffu, base + lane < cutoff && sorted_p[base + lane] >= target);
+        if (reached) {
+            at = base + __ffs(reached) - 1;
+            break;
+        }
+    }
+    if (lane == 0) {
+        *out = sorted_id[at];
+        if (grown) *grown = sorted_id[at];
+    }
+}
+
+// The candidates (probability, id) in shared memory, unused entries (-1, max int): sorted (bitonic over the smallest power of two
+// that holds k) and drawn from.
 __device__ void sort_and_pick(float* sorted_p, int* sorted_id, int k, float nucleus, float u, int* out, int* grown) {
     const int tid = threadIdx.x;
     int span = 32;  // the candidates lie in the first k entries: a power of two that holds them is all that is sorted
@@ -169,29 +212,7 @@ __device__ void sort_and_pick(float* sorted_p, int* sorted_id, int k, float nucl
             __syncthreads();
         }
     }
-    if (tid == 0) {
-        float cumulative = 0.0f;
-        int cutoff = k;
-        for (int i = 0; i < k; ++i) {
-            cumulative += sorted_p[i];
-            if (cumulative >= nucleus) {
-                cutoff = i + 1;
-                break;
-            }
-        }
-        const float target = u * cumulative;  // the kept mass: the same additions in the same order
-        float acc = 0.0f;
-        int pick = sorted_id[cutoff - 1];
-        for (int i = 0; i < cutoff; ++i) {
-            acc += sorted_p[i];
-            if (acc >= target) {
-                pick = sorted_id[i];
-                break;
-            }
-        }
-        *out = pick;
-        if (grown) *grown = pick;
-    }
+    pick_sorted(sorted_p, sorted_id, k, nucleus, u, out, grown);
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -206,7 +227,7 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
     __shared__ float float_scratch[32];
     __shared__ int int_scratch[32];
     __shared__ int histogram[256];
-    __shared__ float sorted_p[kMaxSorted];
+    __shared__ __align__(16) float sorted_p[kMaxSorted];
     __shared__ int sorted_id[kMaxSorted];
     __shared__ int shared_int[4];
 
@@ -410,9 +431,16 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
 // runs on all blocks at once; maxima, sums and the radix histograms meet through distributed shared memory
 // (always added in block order, so the result does not depend on timing); the candidates are gathered into
 // the first block's shared memory, which sorts them and draws.  grid (kSampleBlocks, rows).
+//
+// Few candidates (k <= kFewCandidates) need no histograms: the maxima of the row's 256 warps are 256 of its values, so the k-th
+// largest of them is at most the row's k-th largest, and hardly more than k values reach it (40 of 128,256 random values: 44).
+// They are gathered while the exponentials are summed; should more reach it than can be sorted, the histograms decide.
+// (64 rows of 128,256, k 20 to 64: 119 us with histograms and one block a multiprocessor, 53 with this and two.)
 constexpr int kSampleBlocks = 8;
+constexpr int kFewCandidates = 128;
+constexpr float kThresholdSlack = 1e-5f;  // of a scaled logit: more than the exponential's rounding can turn around
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
 sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int vocab, float* __restrict__ work,
                            int* __restrict__ counts, const float* __restrict__ temperature, const int* __restrict__ top_k,
                            const float* __restrict__ top_p, const float* __restrict__ penalty,
@@ -425,13 +453,15 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     __shared__ int int_scratch[32];
     __shared__ int histogram[256];      // of this block's ids
     __shared__ int histogram_all[256];  // of the whole row
-    __shared__ float sorted_p[kMaxSorted];  // the candidates: filled and used in the cluster's first block only
+    __shared__ __align__(16) float sorted_p[kMaxSorted];  // the candidates: filled and used in the cluster's first block only
     __shared__ int sorted_id[kMaxSorted];
     __shared__ Best slot_best;
     __shared__ float slot_sum;
     __shared__ int slot_ties;
     __shared__ int gathered;            // first block: candidates gathered so far
     __shared__ int shared_int[4];
+    __shared__ float warp_tops[kSampleBlocks * 32];
+    __shared__ float few_threshold;
 
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -517,12 +547,44 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         return;
     }
 
+    const float u = uniforms ? uniforms[r] : philox_uniform(seeds[r], counters[r]);
+    int k = top_k[r];
+    if (k <= 0 || k > vocab) k = vocab;
+    const float nucleus = top_p[r];
+    float* first_p = cluster.map_shared_rank(sorted_p, 0);
+    int* first_id = cluster.map_shared_rank(sorted_id, 0);
+    int* first_gathered = cluster.map_shared_rank(&gathered, 0);
+    int* const grown = (append && h_row) ? h_row + history_len[r] : nullptr;
+
+    const bool few = k <= kFewCandidates && k < vocab;
+    float threshold = CUDART_INF_F;
+    if (few) {
+        if (tid < kSampleBlocks * 32) warp_tops[tid] = cluster.map_shared_rank(best_scratch, tid >> 5)[tid & 31].value;
+        __syncthreads();
+        if (tid < kSampleBlocks * 32) {
+            const float mine_top = warp_tops[tid];
+            int above = 0;
+#pragma unroll 8
+            for (int j = 0; j < kSampleBlocks * 32; ++j) above += warp_tops[j] > mine_top || (warp_tops[j] == mine_top && j < tid);
+            if (above == k - 1) few_threshold = mine_top;
+        }
+        __syncthreads();
+        threshold = few_threshold - kThresholdSlack;
+    }
+
     // softmax over the whole vocabulary
     float local = 0.0f;
     for (int i = begin + tid; i < end; i += kThreads) {
-        const float e = expf(w[i] - top.value);
+        const float v = w[i], e = expf(v - top.value);
         w[i] = e;
         local += e;
+        if (few && v >= threshold) {
+            const int at = atomicAdd(first_gathered, 1);
+            if (at < kMaxSorted) {
+                first_p[at] = e;
+                first_id[at] = i;
+            }
+        }
     }
     {
         const float block = block_sum(local, float_scratch);
@@ -531,13 +593,47 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     cluster.sync();
     float sum = 0.0f;
     for (int b = 0; b < kSampleBlocks; ++b) sum += *cluster.map_shared_rank(&slot_sum, b);
+    if (few) {
+        const int count = *first_gathered;
+        if (count >= k && count <= kMaxSorted) {
+            cluster.sync();  // everybody has read the sums and the count
+            if (part != 0) return;
+            // probabilities, and every candidate's place among them: as many as come before it
+            float p = 0.0f;
+            int id = 0, place = 0;
+            if (tid < count) {
+                p = sorted_p[tid] / sum;
+                id = sorted_id[tid];
+                sorted_p[tid] = p;
+            }
+            __syncthreads();
+            if (tid < count)
+#pragma unroll 4
+                for (int j = 0; j < count; ++j) {
+                    const float other = sorted_p[j];
+                    place += other > p || (other == p && sorted_id[j] < id);
+                }
+            __syncthreads();
+            if (tid < count) {
+                sorted_p[place] = p;
+                sorted_id[place] = id;
+            }
+            __syncthreads();
+            pick_sorted(sorted_p, sorted_id, k, nucleus, u, out + r, grown);
+            return;
+        }
+        cluster.sync();  // everybody has read the count: the first block's arrays start anew
+        if (part == 0) {
+            if (tid == 0) gathered = 0;
+            for (int i = tid; i < kMaxSorted; i += kThreads) {
+                sorted_p[i] = -1.0f;
+                sorted_id[i] = 0x7fffffff;
+            }
+        }
+        // (the histograms' barriers lie between this and the next candidate)
+    }
     for (int i = begin + tid; i < end; i += kThreads) w[i] = w[i] / sum;
     __syncthreads();
-
-    const float u = uniforms ? uniforms[r] : philox_uniform(seeds[r], counters[r]);
-    int k = top_k[r];
-    if (k <= 0 || k > vocab) k = vocab;
-    const float nucleus = top_p[r];
 
     if (k == vocab && nucleus >= 1.0f && vocab > kMaxSorted) {
         // Nothing is cut: the draw walks the whole vocabulary in id order (the same distribution as walking it by
@@ -678,9 +774,6 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     }
 
     // gather the candidates into the first block
-    float* first_p = cluster.map_shared_rank(sorted_p, 0);
-    int* first_id = cluster.map_shared_rank(sorted_id, 0);
-    int* first_gathered = cluster.map_shared_rank(&gathered, 0);
     const bool all_ties = (k == vocab) || tie_count == need_ties;
     int my_ties = 0;
     for (int i = begin + tid; i < end; i += kThreads) {
@@ -722,7 +815,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     }
     cluster.sync();  // the first block's arrays are complete; the others are done
     if (part != 0) return;
-    sort_and_pick(sorted_p, sorted_id, k, nucleus, u, out + r, (append && h_row) ? h_row + history_len[r] : nullptr);
+    sort_and_pick(sorted_p, sorted_id, k, nucleus, u, out + r, grown);
 }
 
 }  // namespace mb

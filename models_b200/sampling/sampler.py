@@ -10,6 +10,7 @@ from __future__ import annotations
 import secrets
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..kernels import ops
@@ -66,14 +67,11 @@ class BatchSampler:
             for r in requests:
                 if r.history is not None:
                     self._history_on_device(r)
-        temperature, top_k, top_p, penalty, seeds, counters, history_rows, history_len = self._parameters(requests)
+        temperature, top_k, top_p, penalty, seeds, counters, history_rows, history_len, most = self._parameters(requests)
         counts = torch.empty((rows, self.vocab), dtype=torch.int32, device=self.device) if penalised else None
         if not penalised:
             history_rows = history_len = None
         work = torch.empty((rows, self.vocab), dtype=torch.float32, device=self.device)
-        # the largest candidate set among the rows that cut anything (1 if none does): it picks the kernel
-        most = max([min(r.options.top_k, self.vocab) for r in requests
-                    if r.options.top_k < self.vocab or r.options.top_p < 1.0] or [1])
         out = ops.sample_rows(logits, work, counts, temperature, top_k, top_p, penalty, None, history_len, seeds, counters,
                               max_candidates=most, history_rows=history_rows, append=history_rows is not None)
         for r in requests:
@@ -95,36 +93,47 @@ class BatchSampler:
             r.history_sent = len(r.history)
 
     def _parameters(self, requests: Sequence[RequestSampling]):
-        """The per-row options on the device, sent as one asynchronous copy from pinned memory (a
-        copy from ordinary memory would wait for every step that is still queued)."""
-        rows = len(requests)
-        if self._staging is None or self._staging[0][0].numel() < 48 * rows:
-            size = 48 * max(64, rows)
-            self._staging = [(torch.empty((size,), dtype=torch.uint8).pin_memory(), torch.cuda.Event()) for _ in range(4)]
-        host, event = self._staging[self._staging_next]
+        """The per-row options on the device, sent as one asynchronous copy from pinned memory (a copy from ordinary memory
+        would wait for every step that is still queued), and the largest candidate set among the rows that cut anything (1 if
+        none does): it picks the kernel.  The buffer holds 8-byte words: three per row (seed, draws, address of the history),
+        then five 4-byte numbers per row (temperature, top_p, penalty, top_k, length of the history).  The rows are walked once
+        and filled in through numpy: building tensors of lists took longer than the kernel."""
+        rows, vocab = len(requests), self.vocab
+        words = 3 * rows + (5 * rows + 1) // 2
+        if self._staging is None or self._staging[0][0].numel() < words:
+            size = max(6 * 64, words)
+            self._staging = []
+            for _ in range(4):
+                host = torch.empty((size,), dtype=torch.int64).pin_memory()
+                self._staging.append((host, host.numpy(), torch.cuda.Event()))
+        host, longs, event = self._staging[self._staging_next]
         self._staging_next = (self._staging_next + 1) % len(self._staging)
         event.synchronize()  # the copy that last read this buffer, four calls ago
-        device = torch.empty((48 * rows,), dtype=torch.uint8, device=self.device)
-
-        def views(buffer):
-            floats = buffer[: 12 * rows].view(torch.float32).view(3, rows)
-            ints = buffer[12 * rows: 16 * rows].view(torch.int32)
-            longs = buffer[16 * rows: 40 * rows].view(torch.int64).view(3, rows)
-            lens = buffer[40 * rows: 44 * rows].view(torch.int32)
-            return floats, ints, longs, lens
-
-        floats, ints, longs, lens = views(host)
-        floats.copy_(torch.tensor([[r.options.temperature for r in requests], [r.options.top_p for r in requests],
-                                   [r.options.repetition_penalty for r in requests]], dtype=torch.float32))
-        ints.copy_(torch.tensor([min(r.options.top_k, self.vocab) for r in requests], dtype=torch.int32))
-        longs.copy_(torch.tensor([[r.seed for r in requests], [r.draws for r in requests],
-                                  [r.history_device.data_ptr() if r.history_device is not None else 0 for r in requests]],
-                                 dtype=torch.int64))
-        lens.copy_(torch.tensor([r.history_sent if r.history_device is not None else 0 for r in requests], dtype=torch.int32))
-        device.copy_(host[: 48 * rows], non_blocking=True)
+        seeds, draws, addresses, temperatures, top_ps, penalties, top_ks, lengths, most = [], [], [], [], [], [], [], [], 1
+        for r in requests:
+            o, history = r.options, r.history_device
+            top_k = min(o.top_k, vocab)
+            if top_k > most and (o.top_k < vocab or o.top_p < 1.0):
+                most = top_k
+            seeds.append(r.seed)
+            draws.append(r.draws)
+            addresses.append(history.data_ptr() if history is not None else 0)
+            temperatures.append(o.temperature)
+            top_ps.append(o.top_p)
+            penalties.append(o.repetition_penalty)
+            top_ks.append(top_k)
+            lengths.append(r.history_sent if history is not None else 0)
+        longs[:3 * rows] = seeds + draws + addresses
+        small = longs[3 * rows:words]
+        small.view(np.float32)[:3 * rows] = temperatures + top_ps + penalties
+        small.view(np.int32)[3 * rows:5 * rows] = top_ks + lengths
+        device = torch.empty((words,), dtype=torch.int64, device=self.device)
+        device.copy_(host[:words], non_blocking=True)
         event.record()
-        floats, ints, longs, lens = views(device)
-        return floats[0], ints, floats[1], floats[2], longs[0], longs[1], longs[2], lens
+        seeds, draws, addresses, rest = device.split((rows, rows, rows, words - 3 * rows))
+        temperature, top_p, penalty, _ = rest.view(torch.float32).split((rows, rows, rows, 2 * (words - 3 * rows) - 3 * rows))
+        top_k, length = rest.view(torch.int32)[3 * rows:5 * rows].split(rows)
+        return temperature, top_k, top_p, penalty, seeds, draws, addresses, length, most
 
     @staticmethod
     def record(requests: Sequence[RequestSampling], tokens: Sequence[int]) -> None:

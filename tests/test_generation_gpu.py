@@ -385,6 +385,26 @@ def test_sampling_over_a_cluster_follows_the_reference_pipeline(cuda_device, voc
     assert float(seen.sum()) == 1.0 and float((seen - expected).abs().max()) < 0.07, seen
 
 
+@pytest.mark.parametrize("vocab", [1031, 5003])
+def test_sampling_with_few_candidates_at_the_edges_of_its_rule(cuda_device, vocab):
+    """k at both sides of the rule's line, more values at the threshold than can be sorted, values that are almost equal, and -inf."""
+    from models_b200.sampling import BatchSampler, RequestSampling, SamplingOptions, philox_uniform
+
+    g = torch.Generator().manual_seed(vocab)
+    options = [SamplingOptions(temperature=1.0, top_k=k, top_p=p, seed=k) for k in (1, 2, 31, 127, 128, 129) for p in (0.6, 1.0)]
+    logits = torch.randn(len(options), vocab, generator=g) * 4
+    logits[2, :] = 1.5                                                  # everything ties
+    logits[5, 100:900] = 20.0                                           # 800 ties
+    logits[7, :] = 3.0 + 1e-6 * torch.arange(vocab).float()             # neighbours a few roundings apart
+    logits[8, 200:] = -float("inf")
+    logits[9, 5:] = -float("inf")                                       # fewer finite values than k
+    requests = [RequestSampling(o, [0]) for o in options]
+    got = BatchSampler(vocab, "cuda:0").sample(logits.cuda(), requests).tolist()
+    for row, o in enumerate(options):
+        want, _ = expected_draw(logits[row].numpy(), [], o, philox_uniform(o.seed, 0))
+        assert got[row] == want, (row, o, got[row], want)
+
+
 def test_sampling_is_reproducible_and_follows_the_distribution(cuda_device):
     import models_b200
     from models_b200.sampling import BatchSampler, RequestSampling, SamplingOptions
