@@ -1,0 +1,382 @@
+// Retention for long steps in bfloat16: chunks of 64 tokens on the tensor cores.  What is computed is what retention.cu's walk
+// computes token by token (see there), for key heads of 64 numbers and value heads of 64 or 128:
+//   S_t = a S_(t-1) + k_t v_t^T,   o_t = S_t^T q_t   (a: the head's decay; q, k, v activated, rotated and scaled as the walk does)
+// and within a chunk that starts from the state S_0, for its token i = 0, 1, ...:
+//   o_i = a^(i + 1) S_0^T q_i + sum_(j <= i) a^(i - j) (q_i . k_j) v_j,     S_end = a^n S_0 + sum_j a^(n - 1 - j) k_j v_j^T
+// Three kernels: what every chunk adds to the state, a product per (chunk, head); the states that the chunks start from, element by
+// element in the chunks' order; every chunk's results, with the head's norm and gate where the caller wants them here.
+// The numbers between the first products and the last one are floats: every operand goes into its products as two bfloat16 numbers,
+// its rounding and the rounding of what that left (16 bits of mantissa), three of the four products of parts, added up in float.
+// Three sequences of 2,048 tokens in all, 16 heads of 64 x 128 with activated projections: 208 us as the walk in runs (98, 70 and 40),
+// which float multiply-adds from shared memory bound; here 23, 9 and 60 us, bound by the instructions that activate and split
+// what every chunk reads.
+#include "common.cuh"
+
+MB_DEFINE_LAST_ERROR()
+
+namespace mb {
+
+using bf16 = __nv_bfloat16;
+
+constexpr int kChunk = 64;    // tokens of a chunk
+constexpr int kDim = 64;      // a key head's numbers
+constexpr int kThreads = 128;
+constexpr int kKeyRow = kDim + 8;                // bfloat16 numbers of a padded row: ldmatrix without bank conflicts
+constexpr int kKeyPlane = kChunk * kKeyRow;      // the roundings of 64 rows; the rests lie behind them
+
+template <int V>
+struct Values {
+    static constexpr int row = V + 8, plane = 64 * row;
+};
+
+struct RetentionArgs {
+    const bf16 *q, *k, *v, *g;  // column slices with one row stride
+    int in_stride;
+    const int* positions;
+    const float *cos_table, *sin_table;
+    int rotary_dim;
+    const float* decay;
+    float key_scale, eps, out_scale;
+    float* state;  // [slots][heads][kDim][V]
+    const int *slots, *cu_q;
+    int heads, input_act;
+    bf16* out;
+    int out_stride;
+    float* raw_out;
+    int raw_stride;
+    float* added;  // scratch by (place of the chunk, head): [kDim][V]
+    bf16* starts;  // scratch by (place, head): [2][kDim][V], roundings and rests
+};
+
+// Every sequence's chunks lie one after another, a sequence's first place being floor(first / 64) + seq (a sequence of n tokens has
+// ceil(n / 64) chunks, and floor(f / 64) + ceil(n / 64) <= floor((f + n) / 64) + 1).
+__device__ __forceinline__ size_t place_of(int first, int seq, int chunk) { return (size_t)(first / kChunk) + seq + chunk; }
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t at) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_turned(uint32_t (&r)[4], uint32_t at) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two floats as a pair of bfloat16 roundings and the pair of what the roundings left over.
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    const float2 back = __bfloat1622float2(h);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a - back.x, b - back.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
+// d[tile] += a (roundings, rests) . b for two neighbouring tiles of eight columns; the four products of parts but the last.
+__device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], const uint32_t (&a_hi)[4], const uint32_t (&a_lo)[4],
+                                               const uint32_t (&b_hi)[4], const uint32_t (&b_lo)[4]) {
+    mma_bf16(d0, a_lo, b_hi[0], b_hi[1]);
+    mma_bf16(d1, a_lo, b_hi[2], b_hi[3]);
+    mma_bf16(d0, a_hi, b_lo[0], b_lo[1]);
+    mma_bf16(d1, a_hi, b_lo[2], b_lo[3]);
+    mma_bf16(d0, a_hi, b_hi[0], b_hi[1]);
+    mma_bf16(d1, a_hi, b_hi[2], b_hi[3]);
+}
+
+// The rows of `count` tokens (64 with zeros behind them) of a head, `kCols` columns from `src`, activated, rotated (rotary > 0),
+// times weight[row] (or 1), in two planes of rows of `row` numbers.
+template <int kCols>
+__device__ __forceinline__ void stage_rows(bf16* planes, int row_numbers, int plane_numbers, const bf16* src, const RetentionArgs& args, int count,
+                                           int rotary, int position0, const float* weight) {
+    const int half = rotary / 2;
+#pragma unroll 2
+    for (int i = threadIdx.x; i < kChunk * kCols / 8; i += kThreads) {
+        const int row = i / (kCols / 8), c = i % (kCols / 8) * 8;
+        float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (row < count) {
+            const bf16* from = src + (size_t)row * args.in_stride;
+            load8(from + c, x);
+            if (args.input_act >= 0)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = gate_activation(args.input_act, x[j]);
+            if (c < rotary)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int d = c + j;
+                    if (d >= rotary) break;
+                    const bool first = d < half;
+                    float partner = __bfloat162float(from[first ? d + half : d - half]);
+                    if (args.input_act >= 0) partner = gate_activation(args.input_act, partner);
+                    const size_t at = (size_t)(position0 + row) * half + (first ? d : d - half);
+                    x[j] = x[j] * args.cos_table[at] + (first ? -1.0f : 1.0f) * partner * args.sin_table[at];
+                }
+            const float factor = weight != nullptr ? weight[row] : 1.0f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] *= factor;
+        }
+        uint4 hi, lo;
+        split_pair(x[0], x[1], hi.x, lo.x);
+        split_pair(x[2], x[3], hi.y, lo.y);
+        split_pair(x[4], x[5], hi.z, lo.z);
+        split_pair(x[6], x[7], hi.w, lo.w);
+        *reinterpret_cast<uint4*>(planes + row * row_numbers + c) = hi;
+        *reinterpret_cast<uint4*>(planes + plane_numbers + row * row_numbers + c) = lo;
+    }
+}
+
+// grid (heads, most chunks of a sequence, sequences); block kThreads.  A warp has 16 coordinates of what the chunk adds.
+template <int V>
+__global__ void __launch_bounds__(kThreads)
+retention_chunk_adds_kernel(const RetentionArgs args) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    extern __shared__ __align__(16) unsigned char shared[];
+    bf16* keys = reinterpret_cast<bf16*>(shared);
+    bf16* values = keys + 2 * kKeyPlane;
+    __shared__ float weight[kChunk];
+    const int head = blockIdx.x, chunk = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
+    const int first = args.cu_q[seq], count = min(kChunk, args.cu_q[seq + 1] - first - chunk * kChunk);
+    if (count <= 0) return;
+    const size_t token0 = (size_t)first + chunk * kChunk;
+    if (tid < kChunk) weight[tid] = tid < count ? args.key_scale * powf(args.decay[head], (float)(count - 1 - tid)) : 0.0f;
+    stage_rows<V>(values, Values<V>::row, Values<V>::plane, args.v + token0 * args.in_stride + (size_t)head * V, args, count, 0, 0, nullptr);
+    __syncthreads();
+    const int position0 = args.rotary_dim > 0 ? args.positions[first] + chunk * kChunk : 0;
+    stage_rows<kDim>(keys, kKeyRow, kKeyPlane, args.k + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, weight);
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31;
+    float acc[V / 8][4] = {};
+    const uint32_t key_at = smem_u32(keys) + (((lane >> 4) * 8 + (lane & 7)) * kKeyRow + 16 * warp + ((lane >> 3) & 1) * 8) * 2;
+    const uint32_t value_at = smem_u32(values) + ((lane & 15) * Values<V>::row + (lane >> 4) * 8) * 2;
+#pragma unroll
+    for (int j = 0; j < kChunk; j += 16) {
+        uint32_t a_hi[4], a_lo[4];
+        ldmatrix4_turned(a_hi, key_at + j * kKeyRow * 2);
+        ldmatrix4_turned(a_lo, key_at + (kKeyPlane + j * kKeyRow) * 2);
+#pragma unroll
+        for (int n = 0; n < V / 8; n += 2) {
+            uint32_t b_hi[4], b_lo[4];
+            ldmatrix4_turned(b_hi, value_at + (j * Values<V>::row + 8 * n) * 2);
+            ldmatrix4_turned(b_lo, value_at + (Values<V>::plane + j * Values<V>::row + 8 * n) * 2);
+            split_products(acc[n], acc[n + 1], a_hi, a_lo, b_hi, b_lo);
+        }
+    }
+    float* to = args.added + (place_of(first, seq, chunk) * args.heads + head) * kDim * V + (size_t)(16 * warp + (lane >> 2)) * V + 2 * (lane & 3);
+#pragma unroll
+    for (int n = 0; n < V / 8; ++n) {
+        *reinterpret_cast<float2*>(to + 8 * n) = make_float2(acc[n][0], acc[n][1]);
+        *reinterpret_cast<float2*>(to + 8 * V + 8 * n) = make_float2(acc[n][2], acc[n][3]);
+    }
+}
+
+// grid (kDim * V / 4 / 128, heads, sequences); block 128: four neighbouring elements a thread.  S before every chunk to `starts`, the
+// state after the last one to the state area; eight chunks' additions are asked for at a time.
+template <int V>
+__global__ void __launch_bounds__(128)
+retention_chunk_starts_kernel(const RetentionArgs args) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int head = blockIdx.y, seq = blockIdx.z, e = (blockIdx.x * 128 + threadIdx.x) * 4;
+    const int first = args.cu_q[seq], tokens = args.cu_q[seq + 1] - first;
+    if (tokens <= 0) return;
+    const int chunks = (tokens + kChunk - 1) / kChunk;
+    const size_t item = place_of(first, seq, 0) * args.heads + head, stride = (size_t)args.heads * kDim * V;
+    const float* added = args.added + item * kDim * V + e;
+    bf16* start = args.starts + 2 * item * kDim * V + e;
+    float* stored = args.state + ((size_t)args.slots[seq] * args.heads + head) * kDim * V + e;
+    const float a = args.decay[head], whole = powf(a, (float)kChunk), last = powf(a, (float)(tokens - (chunks - 1) * kChunk));
+    float4 s = *reinterpret_cast<const float4*>(stored);
+    constexpr int kAtOnce = 8;
+    for (int c0 = 0; c0 < chunks; c0 += kAtOnce) {
+        float4 b[kAtOnce];
+#pragma unroll
+        for (int i = 0; i < kAtOnce; ++i)
+            if (c0 + i < chunks) b[i] = __ldcg(reinterpret_cast<const float4*>(added + (c0 + i) * stride));
+#pragma unroll
+        for (int i = 0; i < kAtOnce; ++i) {
+            if (c0 + i >= chunks) break;
+            uint2 hi, lo;
+            split_pair(s.x, s.y, hi.x, lo.x);
+            split_pair(s.z, s.w, hi.y, lo.y);
+            *reinterpret_cast<uint2*>(start + 2 * (c0 + i) * stride) = hi;
+            *reinterpret_cast<uint2*>(start + 2 * (c0 + i) * stride + kDim * V) = lo;
+            const float keep = c0 + i + 1 < chunks ? whole : last;
+            s = make_float4(fmaf(keep, s.x, b[i].x), fmaf(keep, s.y, b[i].y), fmaf(keep, s.z, b[i].z), fmaf(keep, s.w, b[i].w));
+        }
+    }
+    *reinterpret_cast<float4*>(stored) = s;
+}
+
+// grid (heads, most chunks of a sequence, sequences); block kThreads: a warp has 16 tokens and all V columns of their results.
+template <int V>
+__global__ void __launch_bounds__(kThreads)
+retention_chunk_results_kernel(const RetentionArgs args) {
+    constexpr int kRow = Values<V>::row, kPlane = Values<V>::plane;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    extern __shared__ __align__(16) unsigned char shared[];
+    bf16* queries = reinterpret_cast<bf16*>(shared);
+    bf16* keys = queries + 2 * kKeyPlane;
+    bf16* values = keys + 2 * kKeyPlane;
+    bf16* start = values + 2 * kPlane;
+    __shared__ float power[kChunk + 1];
+    const int head = blockIdx.x, chunk = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
+    const int first = args.cu_q[seq], count = min(kChunk, args.cu_q[seq + 1] - first - chunk * kChunk);
+    if (count <= 0) return;
+    const size_t token0 = (size_t)first + chunk * kChunk;
+    {
+        const bf16* from = args.starts + 2 * (place_of(first, seq, chunk) * args.heads + head) * kDim * V;
+#pragma unroll 4
+        for (int i = tid; i < 2 * kDim * V / 8; i += kThreads) copy16_async(smem_u32(start + i / (V / 8) * kRow + i % (V / 8) * 8), from + 8 * i);  // (the planes' rows run on)
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    if (tid <= kChunk) power[tid] = powf(args.decay[head], (float)tid);
+    const int position0 = args.rotary_dim > 0 ? args.positions[first] + chunk * kChunk : 0;
+    stage_rows<kDim>(queries, kKeyRow, kKeyPlane, args.q + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, nullptr);
+    stage_rows<kDim>(keys, kKeyRow, kKeyPlane, args.k + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, nullptr);
+    stage_rows<V>(values, kRow, kPlane, args.v + token0 * args.in_stride + (size_t)head * V, args, count, 0, 0, nullptr);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31, group = lane >> 2, pair = 2 * (lane & 3);
+    const uint32_t query_at = smem_u32(queries) + ((16 * warp + (lane & 15)) * kKeyRow + (lane >> 4) * 8) * 2;
+    const uint32_t across = ((lane & 15) * kRow + (lane >> 4) * 8) * 2;  // [k][column] tiles of V columns
+    const uint32_t start_at = smem_u32(start) + across, value_at = smem_u32(values) + across;
+    const uint32_t key_at = smem_u32(keys) + (((lane >> 4) * 8 + (lane & 7)) * kKeyRow + ((lane >> 3) & 1) * 8) * 2;
+    float acc[V / 8][4] = {}, weights[kChunk / 8][4] = {};
+#pragma unroll
+    for (int d = 0; d < kDim; d += 16) {
+        uint32_t a_hi[4], a_lo[4];
+        ldmatrix4(a_hi, query_at + d * 2);
+        ldmatrix4(a_lo, query_at + (kKeyPlane + d) * 2);
+#pragma unroll
+        for (int n = 0; n < V / 8; n += 2) {  // S_0^T q
+            uint32_t b_hi[4], b_lo[4];
+            ldmatrix4_turned(b_hi, start_at + (d * kRow + 8 * n) * 2);
+            ldmatrix4_turned(b_lo, start_at + (kPlane + d * kRow + 8 * n) * 2);
+            split_products(acc[n], acc[n + 1], a_hi, a_lo, b_hi, b_lo);
+        }
+#pragma unroll
+        for (int n = 0; n < kChunk / 8; n += 2) {  // q . k over the tokens up to the warp's last
+            if (n > 2 * warp) break;
+            uint32_t b_hi[4], b_lo[4];
+            ldmatrix4(b_hi, key_at + (8 * n * kKeyRow + d) * 2);
+            ldmatrix4(b_lo, key_at + (kKeyPlane + 8 * n * kKeyRow + d) * 2);
+            split_products(weights[n], weights[n + 1], a_hi, a_lo, b_hi, b_lo);
+        }
+    }
+    const int row = 16 * warp + group;
+#pragma unroll
+    for (int n = 0; n < V / 8; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[n][i] *= power[row + 8 * (i / 2) + 1];
+#pragma unroll
+    for (int n = 0; n < kChunk / 8; n += 2) {
+        if (n > 2 * warp) break;
+#pragma unroll
+        for (int m = n; m < n + 2; ++m)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int age = row + 8 * (i / 2) - (8 * m + pair + i % 2);
+                weights[m][i] = age >= 0 ? weights[m][i] * (args.key_scale * power[max(age, 0)]) : 0.0f;
+            }
+        uint32_t a_hi[4], a_lo[4];
+        split_pair(weights[n][0], weights[n][1], a_hi[0], a_lo[0]);
+        split_pair(weights[n][2], weights[n][3], a_hi[1], a_lo[1]);
+        split_pair(weights[n + 1][0], weights[n + 1][1], a_hi[2], a_lo[2]);
+        split_pair(weights[n + 1][2], weights[n + 1][3], a_hi[3], a_lo[3]);
+#pragma unroll
+        for (int c = 0; c < V / 8; c += 2) {
+            uint32_t b_hi[4], b_lo[4];
+            ldmatrix4_turned(b_hi, value_at + (8 * n * kRow + 8 * c) * 2);
+            ldmatrix4_turned(b_lo, value_at + (kPlane + 8 * n * kRow + 8 * c) * 2);
+            split_products(acc[c], acc[c + 1], a_hi, a_lo, b_hi, b_lo);
+        }
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int to = row + 8 * half;
+        float factor = args.out_scale;
+        if (args.raw_out == nullptr) {  // a row's V results lie with four neighbouring lanes
+            float squares = 0.0f;
+#pragma unroll
+            for (int n = 0; n < V / 8; ++n) squares = fmaf(acc[n][2 * half], acc[n][2 * half], fmaf(acc[n][2 * half + 1], acc[n][2 * half + 1], squares));
+            squares += __shfl_xor_sync(0xffffffffu, squares, 1);
+            squares += __shfl_xor_sync(0xffffffffu, squares, 2);
+            factor /= sqrtf(squares / (float)V + args.eps);
+        }
+        if (to >= count) continue;
+        const size_t column = (size_t)head * V + pair;
+        if (args.raw_out != nullptr) {
+            float* dst = args.raw_out + (token0 + to) * args.raw_stride + column;
+#pragma unroll
+            for (int n = 0; n < V / 8; ++n) *reinterpret_cast<float2*>(dst + 8 * n) = make_float2(acc[n][2 * half] * factor, acc[n][2 * half + 1] * factor);
+        } else {
+            const bf16* gate = args.g + (token0 + to) * args.in_stride + column;
+            bf16* dst = args.out + (token0 + to) * args.out_stride + column;
+#pragma unroll
+            for (int n = 0; n < V / 8; ++n) {
+                const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gate + 8 * n));
+                *reinterpret_cast<__nv_bfloat162*>(dst + 8 * n) = __floats2bfloat162_rn(acc[n][2 * half] * factor * (z.x / (1.0f + expf(-z.x))),
+                                                                                       acc[n][2 * half + 1] * factor * (z.y / (1.0f + expf(-z.y))));
+            }
+        }
+    }
+}
+
+template <typename Kernel>
+static int reserve(Kernel kernel, int bytes) {
+    cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (status != cudaSuccess) return fail("retention_chunks: cannot reserve %d bytes of shared memory: %s", bytes, cudaGetErrorString(status));
+    return 0;
+}
+
+template <int V>
+static int launch_chunks(const RetentionArgs& args, int sequences, int chunks, cudaStream_t stream) {
+    constexpr int adds = (2 * kKeyPlane + 2 * Values<V>::plane) * 2, results = (4 * kKeyPlane + 4 * Values<V>::plane) * 2;
+    if (int status = reserve(retention_chunk_adds_kernel<V>, adds)) return status;
+    if (int status = reserve(retention_chunk_results_kernel<V>, results)) return status;
+    const dim3 grid(args.heads, chunks, sequences);
+    MB_LAUNCH("retention_chunks", (retention_chunk_adds_kernel<V>), grid, dim3(kThreads), adds, stream, true, args);
+    MB_LAUNCH("retention_chunks", (retention_chunk_starts_kernel<V>), dim3(kDim * V / 512, args.heads, sequences), dim3(128), 0, stream, true, args);
+    MB_LAUNCH("retention_chunks", (retention_chunk_results_kernel<V>), grid, dim3(kThreads), results, stream, true, args);
+    return check_launch("retention_chunks");
+}
+
+}  // namespace mb
+
+using namespace mb;
+
+MB_EXPORT int mb_retention_chunk_tokens() { return kChunk; }
+
+// Arguments as mb_retention_scan's, bfloat16 storage, head_dim 64, value_dim 64 or 128, whole aligned rows (see the checks).  added:
+// (places * heads * 64 * value_dim) floats, starts: twice as many bfloat16 numbers, with places = tokens / 64 + sequences.
+MB_EXPORT int mb_retention_chunks(const void* q, const void* k, const void* v, const void* g, int in_stride, const int* positions,
+                                  const float* cos_table, const float* sin_table, int rotary_dim, const float* decay, float key_scale, float eps,
+                                  float* state, const int* slots, const int* cu_q, int sequences, int heads, int head_dim, int value_dim, void* out,
+                                  int out_stride, float out_scale, int max_q_len, float* added, void* starts, int input_act, float* raw_out,
+                                  int raw_stride, cudaStream_t stream) {
+    if (sequences <= 0 || heads <= 0 || max_q_len <= 0) return 0;
+    if (input_act >= MB_ACT_COUNT) return fail("retention_chunks: unknown activation code %d", input_act);
+    if (head_dim != kDim || (value_dim != 64 && value_dim != 128)) return fail("retention_chunks: heads of %d and %d numbers are not built (64 and 64 or 128 are)", head_dim, value_dim);
+    if (rotary_dim < 0 || rotary_dim % 2 || rotary_dim > head_dim || (rotary_dim > 0 && (!cos_table || !sin_table)))
+        return fail("retention_chunks: rotary_dim %d must be even, at most %d, and come with its tables", rotary_dim, head_dim);
+    if (!raw_out && (!out || !g)) return fail("retention_chunks: results go to raw_out, or gated to out");
+    const int chunks = (max_q_len + kChunk - 1) / kChunk;
+    if (sequences > 65535 || chunks > 65535 || heads > 65535) return fail("retention_chunks: %d sequences of up to %d chunks and %d heads exceed the grid", sequences, chunks, heads);
+    if (in_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)k & 15) || ((uintptr_t)v & 15) || ((uintptr_t)state & 15) || ((uintptr_t)added & 15) ||
+        ((uintptr_t)starts & 15) || (raw_out && (raw_stride % 2 || ((uintptr_t)raw_out & 7))) ||
+        (!raw_out && (out_stride % 2 || ((uintptr_t)out & 3) || ((uintptr_t)g & 3))))
+        return fail("retention_chunks: rows of whole, aligned pieces are needed");
+    RetentionArgs args{};
+    args.q = (const bf16*)q, args.k = (const bf16*)k, args.v = (const bf16*)v, args.g = (const bf16*)g, args.in_stride = in_stride;
+    args.positions = positions, args.cos_table = cos_table, args.sin_table = sin_table, args.rotary_dim = rotary_dim;
+    args.decay = decay, args.key_scale = key_scale, args.eps = eps, args.out_scale = out_scale;
+    args.state = state, args.slots = slots, args.cu_q = cu_q, args.heads = heads, args.input_act = input_act;
+    args.out = (bf16*)out, args.out_stride = out_stride, args.raw_out = raw_out, args.raw_stride = raw_stride;
+    args.added = added, args.starts = (bf16*)starts;
+    return value_dim == 64 ? launch_chunks<64>(args, sequences, chunks, stream) : launch_chunks<128>(args, sequences, chunks, stream);
+}

@@ -16,6 +16,7 @@ LIBRARIES = [
     ("mb_gated_delta_chunks", ["gated_delta_chunks.cu"], {}),
     ("mb_gated_attention", ["gated_attention.cu"], {}),
     ("mb_retention", ["retention.cu"], {}),
+    ("mb_retention_chunks", ["retention_chunks.cu"], {}),
     ("mb_result_norm", ["result_norm.cu"], {}),
     ("mb_state_space", ["state_space.cu"], {}),
     ("mb_hyper_streams", ["hyper_streams.cu"], {}),

@@ -1153,6 +1153,26 @@ def retention_library():
     return load_library("mb_retention", ["retention.cu"])
 
 
+def retention_chunks_library():
+    """The form for long bfloat16 steps."""
+    return load_library("mb_retention_chunks", ["retention_chunks.cu"])
+
+
+RETENTION_CHUNK_MIN_ROWS = 64  # steps that bring fewer tokens to every sequence are walked
+
+
+def retention_chunks_takes(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[torch.Tensor], out: Optional[torch.Tensor],
+                           raw_out: Optional[torch.Tensor], state: torch.Tensor, head_dim: int, value_dim: int, max_q_len: int) -> bool:
+    """bfloat16 steps of many tokens, key heads of 64 numbers and value heads of 64 or 128, rows that start on 16 bytes (results on a
+    pair's boundary)."""
+    if raw_out is not None:
+        pairs = raw_out.stride(0) % 2 == 0 and raw_out.data_ptr() % 8 == 0
+    else:
+        pairs = out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0 and g.data_ptr() % 4 == 0
+    return (pairs and q.dtype == torch.bfloat16 and max_q_len >= RETENTION_CHUNK_MIN_ROWS and head_dim == 64 and value_dim in (64, 128)
+            and q.stride(0) % 8 == 0 and state.data_ptr() % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)))
+
+
 def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, positions: torch.Tensor,
                    cos: Optional[torch.Tensor], sin: Optional[torch.Tensor], rotary_dim: int, decay: torch.Tensor,
                    key_scale: float, eps: float, state: torch.Tensor, slots: torch.Tensor, cu_q: torch.Tensor, heads: int,
@@ -1168,7 +1188,8 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.T
     [tokens, heads * value_dim], may be a column slice): out_scale * o is written there and nothing else (no norm, no gate;
     `g` and `out` may then be None) -- what follows is the caller's, for instance `group_norm_gate`.
     `max_q_len`: the most new tokens of any sequence.  Beyond `run_length` tokens (None: RETENTION_RUN once a step brings
-    more than twice as many) the sequences are walked in runs of that many tokens at once, through scratch memory."""
+    more than twice as many) the sequences are walked in runs of that many tokens at once, through scratch memory; with
+    run_length None, long bfloat16 steps are computed in chunks of 64 on the tensor cores where the sizes allow it."""
     _cuda(q, k, v, g, positions, cos, sin, decay, state, slots, cu_q, out, raw_out)
     _int32(positions, "positions")
     _int32(slots, "slots")
@@ -1199,6 +1220,18 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.T
             raise KernelError("retention_scan: rotation needs float32 cos/sin tables")
         if cos.shape[-1] != rotary_dim // 2 or cos.shape != sin.shape or not cos.is_contiguous() or not sin.is_contiguous():
             raise KernelError(f"retention_scan: cos/sin tables must be contiguous [positions, {rotary_dim // 2}]")
+    if run_length is None and retention_chunks_takes(q, k, v, g, out, raw_out, state, head_dim, value_dim, max_q_len):
+        lib = retention_chunks_library()
+        items = (tokens // lib.mb_retention_chunk_tokens() + cu_q.numel() - 1) * heads * head_dim * value_dim
+        added = torch.empty((items,), dtype=torch.float32, device=q.device)
+        starts = torch.empty((2 * items,), dtype=torch.bfloat16, device=q.device)
+        _run(lib, lib.mb_retention_chunks(_p(q), _p(k), _p(v), _p(g), q.stride(0), _p(positions), _p(cos), _p(sin), rotary_dim, _p(decay),
+                                          ctypes.c_float(key_scale), ctypes.c_float(eps), _p(state), _p(slots), _p(cu_q), cu_q.numel() - 1, heads,
+                                          head_dim, value_dim, _p(out), out.stride(0) if out is not None else 0, ctypes.c_float(out_scale),
+                                          max_q_len, _p(added), _p(starts), activation_code(input_activation) if input_activation is not None else -1,
+                                          _p(raw_out), raw_out.stride(0) if raw_out is not None else 0, _stream()))
+        _launches[0] += 2  # three kernels
+        return
     lib = retention_library()
     if run_length is None:
         run_length = RETENTION_RUN if max_q_len > 2 * RETENTION_RUN else 0

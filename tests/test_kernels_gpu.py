@@ -930,3 +930,44 @@ def test_gated_delta_chunks(cuda_device, dtype, vdim, lengths):
     assert torch.allclose(chunk_state, state, rtol=1e-4, atol=1e-4)
     assert torch.equal(chunk_state[:, :3], state0[:, :3]) and torch.equal(chunk_state[-1], state0[-1])
     close(chunk_out, out, dtype, scale=4.0)
+
+
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("lengths", [[64], [1, 127, 64], [65, 0, 200, 63]])
+@pytest.mark.parametrize("whole", [True, False])
+def test_retention_chunks(cuda_device, vdim, lengths, whole):
+    """Chunks of 64 on the tensor cores against the walk, from states that are not zero: raw results of activated projections, and
+    rotated ones with the head's norm and gate."""
+    from models_b200.kernels import ops
+
+    heads, dim = 3, 64
+    g = torch.Generator().manual_seed(22)
+    tokens = sum(lengths)
+    proj = torch.randn(tokens, heads * (2 * dim + 2 * vdim), generator=g).bfloat16().cuda()
+    q, k, v, gate = proj.split([heads * dim, heads * dim, heads * vdim, heads * vdim], dim=1)
+    decay = torch.tensor([0.97, 0.5, 0.0]).cuda()
+    state0 = torch.randn(len(lengths) + 1, heads, dim, vdim, generator=g).cuda()
+    slots = torch.arange(len(lengths), dtype=torch.int32).flip(0).contiguous().cuda()
+    cu_q = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    starts = [5, 0, 11, 2][:len(lengths)]
+    positions = torch.cat([torch.arange(s, s + n) for s, n in zip(starts, lengths)]).to(torch.int32).cuda()
+    angle = torch.rand(300, 24, generator=g) * 6
+    cos, sin = angle.cos().cuda(), angle.sin().cuda()
+    found = []
+    for run_length in (0, None):  # the walk, and what the dispatch picks
+        state = state0.clone()
+        raw = torch.zeros(tokens, heads * vdim).cuda() if whole else None
+        out = None if whole else torch.zeros(tokens, heads * vdim).bfloat16().cuda()
+        ops.retention_scan(q, k, v, None if whole else gate, positions, None if whole else cos, None if whole else sin, 0 if whole else 48, decay,
+                           0.3, 1e-6, state, slots, cu_q, heads, dim, vdim, out, 0.5, max(lengths), run_length=run_length,
+                           input_activation="silu" if whole else None, raw_out=raw)
+        found.append(((raw if whole else out).float(), state))
+    (out, state), (chunk_out, chunk_state) = found
+    # an operand's two parts leave less than 2^-17 of it, a product of two such less than 2^-16 + 2^-18; sums over them stay within that
+    # of the root of their squares, the results' size here, but for cancellation (a factor of a few)
+    assert torch.equal(chunk_state[-1], state0[-1])
+    assert float((chunk_state - state).norm() / state.norm()) < 2.0 ** -15
+    if whole:
+        assert float((chunk_out - out).norm() / out.norm()) < 2.0 ** -15
+    else:
+        close(chunk_out, out, torch.bfloat16)
