@@ -3,10 +3,18 @@
 // head size: -DMB_HEAD_DIM=64 or 128; or for sizes of its own, with FLOAT WEIGHTS (below): -DMB_KEY_DIM (64 .. 256) and
 // -DMB_VALUE_DIM (64, 128), both multiples of 64, -DMB_CONTIGUOUS=0 or 1, and -DMB_TURNED_DIM (0 or a multiple of 64).
 //
+// -DMB_SHAPED=1 (paged, float weights): scores and results with the variations of gated_attention.cu -- a factor per head, a bound
+// cap * tanh(score / cap), one more term of score 0 in the denominator, a result whose pairs (2m, 2m + 1) are turned back by the
+// query's position.  The bound costs a thread two more special-function results per score (tanh(x) = 1 - 2 / (1 + e^(2x))), and
+// that unit is what bounds it: 2,048 tokens, 16 heads of 64 and 128, 64 us under a profiler (166 in
+// gated_attention_tc.cu).
+//
 // MB_CONTIGUOUS: a prompt that starts its sequence brings every key it sees itself, so keys and values are read from the step's own
 // rows ([tokens][heads * size]) instead of the cache's pages.  Key and value heads may then be padded to these sizes with zero
 // columns (a query may hold anything finite there), and a key may have MB_TURNED_DIM coordinates more that all heads share
 // ([tokens][MB_TURNED_DIM]), the query's own ones beside them ([tokens][heads * MB_TURNED_DIM]), zeros behind their real ones.
+// A step on top of cached positions reads such rows as well, made of the cache's before: every sequence's keys then lie `key_rows`
+// rows apart, from its position 0 on.
 //
 // A block takes 128 consecutive query tokens of one head and walks the visible cache pages (64 keys
 // each).  Its six warps have three roles:
@@ -52,6 +60,9 @@
 #else
 #define MB_FLOAT_WEIGHTS 1
 #endif
+#ifndef MB_SHAPED
+#define MB_SHAPED 0
+#endif
 #if !defined(MB_KEY_DIM) || !defined(MB_VALUE_DIM) || !defined(MB_TURNED_DIM) || !defined(MB_CONTIGUOUS)
 #error "compile with -DMB_HEAD_DIM, or with -DMB_KEY_DIM, -DMB_TURNED_DIM, -DMB_VALUE_DIM and -DMB_CONTIGUOUS"
 #endif
@@ -61,7 +72,8 @@ MB_DEFINE_LAST_ERROR()
 namespace mb {
 
 constexpr int KD = MB_KEY_DIM, RD = MB_TURNED_DIM, VD = MB_VALUE_DIM;
-constexpr bool kFloatWeights = MB_FLOAT_WEIGHTS != 0, kContiguous = MB_CONTIGUOUS != 0;
+constexpr bool kFloatWeights = MB_FLOAT_WEIGHTS != 0, kContiguous = MB_CONTIGUOUS != 0, kShaped = MB_SHAPED != 0;
+static_assert(!kShaped || (kFloatWeights && !kContiguous), "shaped scores are built with float weights over pages");
 static_assert(KD % 64 == 0 && KD >= 64 && RD % 64 == 0 && KD + RD <= 256, "keys of 64 .. 256 numbers in steps of 64");
 static_assert(VD == 64 || VD == 128, "values of 64 or 128 numbers");
 static_assert(RD == 0 || kContiguous, "shared key coordinates come with rows of their own");
@@ -217,6 +229,14 @@ struct AttentionArgs {
     int value_columns;    // numbers of a head's result that are stored (the rest is padding)
     const bf16* gate;     // [tokens][heads] (row stride gate_stride) or null: head h's result is multiplied by sigmoid(gate[t][h])
     int gate_stride;
+    int gate_element;     // != 0: the gate is [tokens][heads * value_columns], element by element
+    int key_rows;         // kContiguous: 0, or how many rows of keys and values a sequence has (from its position 0 on)
+    // kShaped
+    const float* head_scale;  // [heads] factors on the scores, or null
+    float softcap;            // 0: scores are not bounded
+    int sink;                 // != 0: one more term of score 0 in the denominator
+    const float* turn_cos;    // [positions][VD / 2] with turn_sin, or null
+    const float* turn_sin;
 };
 
 // roles in the status record: 1 TMA (stage free), 2 MMA (queries), 3 MMA (keys), 4 MMA (probabilities),
@@ -300,7 +320,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             for (int t = 0; t < pages; ++t) {
                 const int stage = t % kStages;
                 const uint32_t free_parity = ((t / kStages) & 1) ^ 1;
-                const int row = kContiguous ? q_begin + (t_begin + t) * kKeys : (table[t_begin + t] * args.kv_heads + kv_head) * kKeys;
+                const int row = kContiguous ? (args.key_rows > 0 ? seq * args.key_rows : q_begin) + (t_begin + t) * kKeys : (table[t_begin + t] * args.kv_heads + kv_head) * kKeys;
                 const int key_column = kContiguous ? kv_head * KD : 0, value_column = kContiguous ? kv_head * VD : 0;
                 if (!mbar_wait(k_empty + 8 * stage, free_parity, 1)) break;
                 mbar_expect_tx(k_full + 8 * stage, kKeyTileBytes);
@@ -368,7 +388,10 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         const uint32_t my_output = tmem_output + lane_base;
         const int row_pos = row < valid ? pos0 + row : -1;  // a row beyond the sequence sees nothing
         const int row_first = (window > 0 && row_pos - window + 1 > 0) ? row_pos - window + 1 : 0;
-        const float scale_log2 = args.scale * 1.4426950408889634f;
+        // (shaped scores are finished, scale and all, before their maximum is taken)
+        const float shaped_scale = kShaped ? args.scale * (args.head_scale != nullptr ? args.head_scale[head] : 1.0f) : 1.0f;
+        const float cap = kShaped ? args.softcap : 0.0f, cap_exponent = cap > 0.0f ? shaped_scale * (2.0f * 1.4426950408889634f / cap) : 0.0f;
+        const float scale_log2 = (kShaped ? 1.0f : args.scale) * 1.4426950408889634f;
         const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
         // `base` is the score the exponents are taken against.  It follows the running maximum lazily:
         // it moves (and the output so far is rescaled) only when the maximum has grown by more than
@@ -387,6 +410,16 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 #pragma unroll
             for (int c = 0; c < kCols; c += 32) tmem_load_32_raw(my_scores + c, &s[c]);
             tmem_wait_loads();
+            if (kShaped) {
+                if (cap > 0.0f) {
+#pragma unroll
+                    for (int i = 0; i < kCols; ++i)  // cap * tanh(z / cap)
+                        s[i] = __float_as_uint(cap - __fdividef(2.0f * cap, 1.0f + fast_exp2(__uint_as_float(s[i]) * cap_exponent)));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kCols; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) * shaped_scale);
+                }
+            }
             const int key_base = (t_begin + t) * kKeys;
             if (!(key_base + kCols - 1 <= row_pos && key_base >= row_first)) {  // not the whole page is visible to this row
 #pragma unroll
@@ -485,8 +518,9 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         }
         if (ok) {
             tcgen05_fence_after();
+            if (kShaped && args.sink) run_sum += exp2f(-base * scale_log2);
             float inv = exp2f(kTruncationLift) / run_sum;  // the sum holds the lifted probabilities, the products their truncations
-            if (kFloatWeights && args.gate != nullptr && row < valid)
+            if (kFloatWeights && args.gate != nullptr && !args.gate_element && row < valid)
                 inv *= 1.0f / (1.0f + expf(-__bfloat162float(args.gate[(size_t)(q_begin + t0 + row) * args.gate_stride + head])));
             const int value_columns = kFloatWeights ? args.value_columns : VD;
             bf16* dst = args.out + (size_t)(q_begin + t0 + row) * args.out_row_stride + (size_t)head * value_columns;
@@ -502,6 +536,23 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                         float piece[8];
 #pragma unroll
                         for (int j = 0; j < 8; ++j) piece[j] = __uint_as_float(r[i + j]) * inv;
+                        if (kContiguous && args.gate_element) {
+                            float z[8];
+                            load8(args.gate + (size_t)(q_begin + t0 + row) * args.gate_stride + (size_t)head * value_columns + c + i, z);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) piece[j] *= 1.0f / (1.0f + expf(-z[j]));
+                        }
+                        if (kShaped && args.turn_cos != nullptr) {  // back by the query's position
+                            const size_t at = (size_t)row_pos * (VD / 2) + (c + i) / 2;
+                            const float4 cs = *reinterpret_cast<const float4*>(args.turn_cos + at), sn = *reinterpret_cast<const float4*>(args.turn_sin + at);
+                            const float cosines[4] = {cs.x, cs.y, cs.z, cs.w}, sines[4] = {sn.x, sn.y, sn.z, sn.w};
+#pragma unroll
+                            for (int m = 0; m < 4; ++m) {
+                                const float x = piece[2 * m], y = piece[2 * m + 1];
+                                piece[2 * m] = x * cosines[m] + y * sines[m];
+                                piece[2 * m + 1] = y * cosines[m] - x * sines[m];
+                            }
+                        }
                         store8(dst + c + i, piece);
                     }
                 }
@@ -548,11 +599,21 @@ static int check_prefill(const void* q, int q_row_stride, const void* out, int o
 // q: bfloat16 rows (row stride q_row_stride) of total_rows tokens, head h at columns [h * KD, +KD); out likewise with VD.
 // k_pool [pages][kv_heads][64][KD], v_pool [pages][kv_heads][64][VD]: bfloat16.  block_table: int32 [sequences][max_blocks];
 // cu_q: int32 [sequences + 1]; kv_lens: int32 [sequences] (the new tokens included).
+// MB_SHAPED: also head_scale (or null), softcap, sink and the tables that turn the result back (16-byte aligned, or null).
 MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int total_rows, void* out, int out_row_stride,
                                            const void* k_pool, const void* v_pool, int pool_pages, const int* block_table,
                                            int max_blocks, const int* cu_q, const int* kv_lens, int sequences, int max_q_len,
                                            int heads, int kv_heads, int page_size, int window, float scale,
+#if MB_SHAPED
+                                           const float* head_scale, float softcap, int sink, const float* turn_cos, const float* turn_sin,
+#endif
                                            cudaStream_t stream) {
+#if !MB_SHAPED
+    const float *head_scale = nullptr, *turn_cos = nullptr, *turn_sin = nullptr;
+    const float softcap = 0.0f;
+    const int sink = 0;
+#endif
+    if (((uintptr_t)turn_cos | (uintptr_t)turn_sin) & 15) return fail("prefill_attention_tcgen05: the tables that turn the result back must start on 16-byte boundaries");
     if (sequences <= 0 || max_q_len <= 0) return 0;
     if (int status = check_prefill(q, q_row_stride, out, out_row_stride, sequences, max_q_len, heads, kv_heads)) return status;
     if (page_size != kKeys) return fail("prefill_attention_tcgen05: the cache page must hold %d positions, got %d", kKeys, page_size);
@@ -562,7 +623,8 @@ MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int 
     if (int status = make_map(&map_q, q, total_rows, heads * KD, q_row_stride, kQRows)) return status;
     if (int status = make_map(&map_k, k_pool, pool_pages * kv_heads * kKeys, KD, KD, kKeys)) return status;
     if (int status = make_map(&map_v, v_pool, pool_pages * kv_heads * kKeys, VD, VD, kKeys)) return status;
-    const AttentionArgs args{(bf16*)out, out_row_stride, block_table, max_blocks, cu_q, kv_lens, heads, kv_heads, window, scale, KD, VD, nullptr, 0};
+    const AttentionArgs args{(bf16*)out, out_row_stride, block_table, max_blocks, cu_q, kv_lens, heads, kv_heads, window, scale, KD, VD, nullptr, 0, 0, 0,
+                             head_scale, softcap, sink, turn_cos, turn_sin};
     return launch_prefill(map_q, map_k, map_v, map_q, map_k, args, sequences, max_q_len, stream);
 }
 #else
@@ -570,11 +632,13 @@ MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int 
 // own coordinates at columns [h * q_head_columns, +KD) (what lies there behind the real ones meets zero columns of the keys and must
 // be finite; q_columns: columns of a row in all); q_turned [total_rows][heads * RD], k_turned [total_rows][RD] (RD > 0).  k, v: rows of
 // total_rows tokens with kv_heads heads of KD and of VD (row stride kv_row_stride).  out: [total_rows][heads * value_columns].
-// gate (or null): bfloat16 [total_rows][heads], the heads' results are multiplied by its sigmoid.
+// gate (or null): bfloat16 [total_rows][heads], the heads' results are multiplied by its sigmoid; gate_element: [total_rows][heads *
+// value_columns], 16-byte aligned rows.  key_rows n > 0 (a multiple of 64): k, v and k_turned have key_total rows, n for every sequence,
+// of which kv_lens say how many are there; the step's tokens are the last of them.
 MB_EXPORT int mb_prompt_attention_tcgen05(const void* q, int q_row_stride, int q_head_columns, int q_columns, const void* q_turned,
                                           const void* k, const void* v, int kv_row_stride, const void* k_turned, int total_rows, void* out,
-                                          int out_row_stride, int value_columns, const void* gate, int gate_stride, const int* cu_q,
-                                          const int* kv_lens, int sequences, int max_q_len, int heads, int kv_heads, int window,
+                                          int out_row_stride, int value_columns, const void* gate, int gate_stride, int gate_element,
+                                          int key_rows, int key_total, const int* cu_q, const int* kv_lens, int sequences, int max_q_len, int heads, int kv_heads, int window,
                                           float scale, cudaStream_t stream) {
     if (sequences <= 0 || max_q_len <= 0) return 0;
     if (int status = check_prefill(q, q_row_stride, out, out_row_stride, sequences, max_q_len, heads, kv_heads)) return status;
@@ -582,18 +646,22 @@ MB_EXPORT int mb_prompt_attention_tcgen05(const void* q, int q_row_stride, int q
         return fail("prompt_attention_tcgen05: heads of %d query columns and %d value columns", q_head_columns, value_columns);
     if (((uintptr_t)k & 15) || ((uintptr_t)v & 15) || ((uintptr_t)q_turned & 15) || ((uintptr_t)k_turned & 15) || (RD > 0 && (!q_turned || !k_turned)))
         return fail("prompt_attention_tcgen05: keys, values and shared coordinates must be there and start on 16-byte boundaries");
+    if (key_rows < 0 || key_rows % kKeys || (key_rows > 0 && (long long)key_rows * sequences > key_total))
+        return fail("prompt_attention_tcgen05: %d rows of keys do not hold %d for each of %d sequences", key_total, key_rows, sequences);
+    if (gate_element && (!gate || gate_stride % 8 || ((uintptr_t)gate & 15))) return fail("prompt_attention_tcgen05: a gate of elements needs 16-byte aligned rows");
+    if (key_rows == 0) key_total = total_rows;
     CUtensorMap map_q, map_k, map_v, map_q_turned, map_k_turned;
     if (int status = make_map(&map_q, q, total_rows, q_columns, q_row_stride, kQRows)) return status;
-    if (int status = make_map(&map_k, k, total_rows, kv_heads * KD, kv_row_stride, kKeys)) return status;
-    if (int status = make_map(&map_v, v, total_rows, kv_heads * VD, kv_row_stride, kKeys)) return status;
+    if (int status = make_map(&map_k, k, key_total, kv_heads * KD, kv_row_stride, kKeys)) return status;
+    if (int status = make_map(&map_v, v, key_total, kv_heads * VD, kv_row_stride, kKeys)) return status;
     map_q_turned = map_q;
     map_k_turned = map_k;
     if (RD > 0) {
         if (int status = make_map(&map_q_turned, q_turned, total_rows, heads * RD, heads * RD, kQRows)) return status;
-        if (int status = make_map(&map_k_turned, k_turned, total_rows, RD, RD, kKeys)) return status;
+        if (int status = make_map(&map_k_turned, k_turned, key_total, RD, RD, kKeys)) return status;
     }
     const AttentionArgs args{(bf16*)out, out_row_stride, nullptr, 0, cu_q, kv_lens, heads, kv_heads, window, scale, q_head_columns, value_columns,
-                             (const bf16*)gate, gate_stride};
+                             (const bf16*)gate, gate_stride, gate_element, key_rows, nullptr, 0.0f, 0, nullptr, nullptr};
     return launch_prefill(map_q, map_k, map_v, map_q_turned, map_k_turned, args, sequences, max_q_len, stream);
 }
 #endif

@@ -15,6 +15,7 @@ LIBRARIES = [
     ("mb_gated_delta", ["gated_delta.cu"], {}),
     ("mb_gated_delta_chunks", ["gated_delta_chunks.cu"], {}),
     ("mb_gated_attention", ["gated_attention.cu"], {}),
+    ("mb_latent_gather", ["latent_gather.cu"], {}),
     ("mb_retention", ["retention.cu"], {}),
     ("mb_retention_chunks", ["retention_chunks.cu"], {}),
     ("mb_result_norm", ["result_norm.cu"], {}),
@@ -49,6 +50,7 @@ LIBRARIES = [
     ("mb_prefill_attention_tcgen05", ["prefill_attention_tcgen05.cu"], {"MB_HEAD_DIM": 128}),
     ("mb_prefill_attention_tcgen05", ["prefill_attention_tcgen05.cu"], {"MB_KEY_DIM": 128, "MB_VALUE_DIM": 128, "MB_TURNED_DIM": 0, "MB_CONTIGUOUS": 0}),
     ("mb_prefill_attention_tcgen05", ["prefill_attention_tcgen05.cu"], {"MB_KEY_DIM": 64, "MB_VALUE_DIM": 128, "MB_TURNED_DIM": 64, "MB_CONTIGUOUS": 1}),
+    ("mb_prefill_attention_tcgen05", ["prefill_attention_tcgen05.cu"], {"MB_KEY_DIM": 64, "MB_VALUE_DIM": 128, "MB_TURNED_DIM": 0, "MB_CONTIGUOUS": 0, "MB_SHAPED": 1}),
     # the tensor-core attention with weights mixed across heads is compiled per (heads, key size, value size);
     # these are the sizes of the benchmark's models of that design
     ("mb_talking_attention_tc", ["talking_attention_tc.cu"], {"MB_HEADS": 8, "MB_KEY_DIM": 64, "MB_VALUE_DIM": 128}),

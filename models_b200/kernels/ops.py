@@ -826,11 +826,12 @@ def gated_attention_tc_takes(q: torch.Tensor, out: torch.Tensor, k_pool: torch.T
     return gate is None or gate_kind != "element" or (gate.stride(0) % 2 == 0 and gate.data_ptr() % 4 == 0)
 
 
-def float_weight_attention_library(key_dim: int, value_dim: int, turned: int = 0, contiguous: bool = False):
+def float_weight_attention_library(key_dim: int, value_dim: int, turned: int = 0, contiguous: bool = False, shaped: bool = False):
     """The tcgen05 prompt attention with float weights, compiled for these sizes (multiples of 64) at first use."""
-    return load_library("mb_prefill_attention_tcgen05", ["prefill_attention_tcgen05.cu"],
-                        {"MB_KEY_DIM": int(key_dim), "MB_VALUE_DIM": int(value_dim), "MB_TURNED_DIM": int(turned),
-                         "MB_CONTIGUOUS": 1 if contiguous else 0})
+    sizes = {"MB_KEY_DIM": int(key_dim), "MB_VALUE_DIM": int(value_dim), "MB_TURNED_DIM": int(turned), "MB_CONTIGUOUS": 1 if contiguous else 0}
+    if shaped:
+        sizes["MB_SHAPED"] = 1
+    return load_library("mb_prefill_attention_tcgen05", ["prefill_attention_tcgen05.cu"], sizes)
 
 
 def float_weight_attention_takes(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_pool: Optional[torch.Tensor], head_dim: int,
@@ -844,20 +845,24 @@ def float_weight_attention_takes(q: torch.Tensor, out: torch.Tensor, k_pool: tor
 
 def prompt_attention(q: torch.Tensor, q_tail: Optional[torch.Tensor], k: torch.Tensor, v: torch.Tensor, k_tail: Optional[torch.Tensor],
                      out: torch.Tensor, cu_q: torch.Tensor, kv_lens: torch.Tensor, max_q_len: int, heads: int, head_columns: int,
-                     value_columns: int, scale: float, gate: Optional[torch.Tensor] = None, window: int = 0) -> None:
+                     value_columns: int, scale: float, gate: Optional[torch.Tensor] = None, window: int = 0,
+                     gate_kind: str = "head", key_rows: int = 0) -> None:
     """Causal softmax attention of prompts that start their sequences, on the tcgen05 tensor cores with float weights: every key comes
     from the step's own rows.  bfloat16: k [T, heads * KD] and v [T, heads * VD] (column slices with one row stride; KD, VD multiples
     of 64, heads padded with zero columns), k_tail [T, RD] shared by all heads and q_tail [T, heads * RD] (or None, None); q [T, ...] holds
     head h's own coordinates from column h * head_columns on; out [T, heads * value_columns]; gate [T, heads]: head h's result is
-    multiplied by its sigmoid.  `window` n > 0: query i sees key j only if i - j < n."""
+    multiplied by its sigmoid, or, gate_kind "element", a gate [T, heads * value_columns] element by element.  `window` n > 0: query i
+    sees key j only if i - j < n.  `key_rows` n > 0 (a multiple of 64): a step on top of cached positions; k, v and k_tail have n rows for
+    every sequence, its positions from 0 on, the step's own ones last."""
     _cuda(q, q_tail, k, v, k_tail, out, cu_q, kv_lens, gate)
     _int32(cu_q, "cu_q")
     _int32(kv_lens, "kv_lens")
     rows = q.shape[0]
-    for name, t in (("q", q), ("k", k), ("v", v), ("out", out)):
+    keys = key_rows * kv_lens.numel() if key_rows else rows
+    for name, t, n in (("q", q, rows), ("k", k, keys), ("v", v, keys), ("out", out, rows)):
         _columns(t, name)
-        if t.dtype != torch.bfloat16 or t.shape[0] != rows:
-            raise KernelError(f"prompt_attention: {name} must be bfloat16 with {rows} rows, got {tuple(t.shape)} {t.dtype}")
+        if t.dtype != torch.bfloat16 or t.shape[0] != n:
+            raise KernelError(f"prompt_attention: {name} must be bfloat16 with {n} rows, got {tuple(t.shape)} {t.dtype}")
     key_dim, value_dim = k.shape[1] // heads, v.shape[1] // heads
     if k.shape[1] != heads * key_dim or v.shape[1] != heads * value_dim or k.stride(0) != v.stride(0) or key_dim % 64 or value_dim % 64:
         raise KernelError(f"prompt_attention: keys {tuple(k.shape)} and values {tuple(v.shape)} are no {heads} heads of whole 64 columns")
@@ -866,17 +871,18 @@ def prompt_attention(q: torch.Tensor, q_tail: Optional[torch.Tensor], k: torch.T
     turned = 0
     if k_tail is not None:
         turned = k_tail.shape[1]
-        if q_tail is None or tuple(k_tail.shape) != (rows, turned) or tuple(q_tail.shape) != (rows, heads * turned) \
+        if q_tail is None or tuple(k_tail.shape) != (keys, turned) or tuple(q_tail.shape) != (rows, heads * turned) \
                 or not k_tail.is_contiguous() or not q_tail.is_contiguous() or k_tail.dtype != q.dtype or q_tail.dtype != q.dtype:
             raise KernelError("prompt_attention: shared key coordinates need contiguous [T, n] and [T, heads * n] rows")
     if gate is not None:
         _columns(gate, "gate")
-        if gate.dtype != q.dtype or tuple(gate.shape) != (rows, heads):
-            raise KernelError(f"prompt_attention: a gate per head cannot be {tuple(gate.shape)} {gate.dtype}")
+        if gate.dtype != q.dtype or gate_kind not in ("head", "element") or tuple(gate.shape) != (rows, heads if gate_kind == "head" else out.shape[1]):
+            raise KernelError(f"prompt_attention: a gate of kind {gate_kind!r} cannot be {tuple(gate.shape)} {gate.dtype}")
     lib = float_weight_attention_library(key_dim, value_dim, turned, True)
     _run(lib, lib.mb_prompt_attention_tcgen05(
         _p(q), q.stride(0), int(head_columns), q.shape[1], _p(q_tail), _p(k), _p(v), k.stride(0), _p(k_tail), rows, _p(out), out.stride(0),
-        int(value_columns), _p(gate), gate.stride(0) if gate is not None else 0, _p(cu_q), _p(kv_lens), kv_lens.numel(), int(max_q_len), heads,
+        int(value_columns), _p(gate), gate.stride(0) if gate is not None else 0,
+        1 if gate is not None and gate_kind == "element" else 0, int(key_rows), keys, _p(cu_q), _p(kv_lens), kv_lens.numel(), int(max_q_len), heads,
         heads, int(window), ctypes.c_float(scale), _stream()))
 
 
@@ -913,7 +919,7 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
     sequence's position 0; `window` n > 0: only if i - j < n.
     `kernel`: None picks the decode form for steps of one token per sequence (the keys cut into runs with a block each;
     the grid follows the page table's width, not the lengths, so that a captured step stays valid), the tensor-core form
-    where it applies (bfloat16 steps of many tokens; plain softmax attention of suitable sizes on the tcgen05 ones, "tcgen05"), else the form with a warp per (token, head); decode steps of 8 heads and
+    where it applies (bfloat16 steps of many tokens; softmax attention of suitable sizes without distance, bias or gate on the tcgen05 ones; plain scores: "tcgen05"), else the form with a warp per (token, head); decode steps of 8 heads and
     more over rows they share run on the tensor cores, "tc_decode", where the sizes allow; "decode", "tc", "tcgen05",
     "tc_decode" or "rows" asks for one of them."""
     if weights not in ("softmax", "sigmoid"):
@@ -1015,6 +1021,15 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
             _p(q), q.stride(0), q.shape[0], _p(out), out.stride(0), _p(k_pool), _p(v_pool), k_pool.shape[0], _p(block_table),
             block_table.shape[1], _p(cu_q), _p(kv_lens), sequences, max_q_len, heads, kv_heads, page_size, int(window), ctypes.c_float(scale),
             _stream()))
+        return
+    shaped = (weights == "softmax" and slope_exponent == 0.0 and head_bias is None and gate is None and block == 0
+              and (turn_cos is None or (turn_cos.data_ptr() % 16 == 0 and turn_sin.data_ptr() % 16 == 0)))
+    if kernel is None and shaped and float_weight_attention_takes(q, out, k_pool, v_pool, head_dim, value_dim, max_q_len):
+        lib = float_weight_attention_library(head_dim, value_dim, shaped=True)
+        _run(lib, lib.mb_prefill_attention_tcgen05(
+            _p(q), q.stride(0), q.shape[0], _p(out), out.stride(0), _p(k_pool), _p(v_pool), k_pool.shape[0], _p(block_table),
+            block_table.shape[1], _p(cu_q), _p(kv_lens), sequences, max_q_len, heads, kv_heads, page_size, int(window), ctypes.c_float(scale),
+            _p(head_scale), ctypes.c_float(softcap), 1 if sink else 0, _p(turn_cos), _p(turn_sin), _stream()))
         return
     if kernel == "tc" or (kernel is None and gated_attention_tc_takes(q, out, k_pool, head_dim, value_dim, max_q_len, gate, gate_kind, v_pool)):
         if not gated_attention_tc_takes(q, out, k_pool, head_dim, value_dim, max(max_q_len, GATED_TC_MIN_ROWS), gate, gate_kind, v_pool):
@@ -1144,6 +1159,24 @@ def latent_rows(k: torch.Tensor, gain: torch.Tensor, turned: int, cos: Optional[
                                  q.stride(0) if q is not None else 0, head_columns - turned, heads, _p(q_tail), int(padded), _code(k.dtype), rows,
                                  _stream()))
     return own, tail, q_tail
+
+
+def latent_gather(k_pool: torch.Tensor, latent: int, padded: int, block_table: torch.Tensor, kv_lens: torch.Tensor, rows_per: int):
+    """The rows that a latent attention's sequences hold in their cache pool [pages, 1, page_size, latent + turned] (bfloat16), `rows_per`
+    (a multiple of 64) for every sequence, from its position 0 on: latents [sequences * rows_per, latent] and, where there is a tail,
+    tails [sequences * rows_per, padded] with zeros behind the turned numbers.  Rows behind a sequence's last 64 are not written."""
+    _cuda(k_pool, block_table, kv_lens)
+    _int32(block_table, "block_table")
+    _int32(kv_lens, "kv_lens")
+    turned, sequences = k_pool.shape[3] - latent, kv_lens.numel()
+    if k_pool.dtype != torch.bfloat16 or k_pool.dim() != 4 or k_pool.shape[1] != 1 or not k_pool.is_contiguous() or turned < 0:
+        raise KernelError(f"latent_gather: the pool must be contiguous bfloat16 [pages, 1, page_size, latent + turned], got {tuple(k_pool.shape)} {k_pool.dtype}")
+    latents = torch.empty((sequences * rows_per, latent), dtype=k_pool.dtype, device=k_pool.device)
+    tails = torch.empty((sequences * rows_per, padded), dtype=k_pool.dtype, device=k_pool.device) if turned else None
+    lib = load_library("mb_latent_gather", ["latent_gather.cu"])
+    _run(lib, lib.mb_latent_gather(_p(k_pool), latent, turned, int(padded), _p(block_table), block_table.shape[1], k_pool.shape[2], _p(kv_lens),
+                                   sequences, int(rows_per), _p(latents), _p(tails), _stream()))
+    return latents, tails
 
 
 RETENTION_RUN = 64  # tokens of a run when a long step's recurrence is walked in runs

@@ -15,9 +15,10 @@ row's first latent_dim numbers.  (Rotated pairs (2i, 2i + 1) are brought side by
 parts meet in dot products only, so the order of their coordinates is nobody's business but theirs, and the kernels know one
 pairing.)  A window.  A gate per element.  Rows that another run cached (`own_rows` False).
 
-A prompt that starts its sequences sees no row but its own, and there the other order is cheaper: one product expands every row of
-the step into the heads' keys and values, and the attention runs over those (with the shared rotated part beside them), a third of the
-multiplications per query and key.  Steps that continue a sequence, and sizes the kernel does not take, stay in the latent space.
+For a prompt the other order is cheaper: one product expands every row that it sees into the heads' keys and values, and the attention
+runs over those (with the shared rotated part beside them), a third of the multiplications per query and key.  A prompt that starts its
+sequences expands its own rows; one on top of cached positions the sequences' rows, gathered from the cache.  Shorter steps (see
+EXPANDED_TOKENS), and sizes the kernel does not take, stay in the latent space.
 """
 
 from __future__ import annotations
@@ -31,6 +32,15 @@ from .base import Mixer, RunContext
 from .linear import linear, stack_columns, stack_rows
 from .registry import build_part, register_part
 from .split import SplitPart
+
+
+# Expanding costs a prompt three launches more than staying in the latent space and saves it multiplications (16 heads of 64 + 64 and
+# 128, rows of 256 + 64, queries with a latent and a window of 1,024; microseconds expanded / in the latent space): 128 tokens on 256
+# cached ones 159 / 134, 4 x 128 on 300 152 / 158, 4 x 128 on 1,500 (13 rows gathered for a token) 153 / 226, 2 x 765 on 700 154 / 350,
+# 2,048 on 1,500 155 / 446.  Prompts that start their sequences and whose queries have no latent save a launch as well: they expand from
+# the kernel's least step on.
+EXPANDED_TOKENS = 512
+EXPANDED_ROWS = 16  # most rows gathered for a token
 
 
 def _whole(size: int) -> int:
@@ -107,7 +117,7 @@ class LatentAttentionMixer(SplitPart, Mixer):
 
         self.expand = None
         K, D, V = s.latent_dim, s.head_dim, s.value_dim
-        if (rt.mode == "bfloat16" and s.own_rows and not s.query_latent and (not s.gated or s.gate_kind == "head") and K % 8 == 0
+        if (rt.mode == "bfloat16" and s.own_rows and K % 8 == 0
                 and (D + self.turned) % 8 == 0 and V % 8 == 0 and V <= 128 and _whole(D) + _whole(self.turned) <= 256):
             # every head's key and value matrices padded with zero rows to whole 64s: [heads * keys; heads * values] x latent
             pad = lambda m, size: torch.nn.functional.pad(m, (0, 0, 0, _whole(size) - size)).reshape(-1, K)  # noqa: E731
@@ -129,6 +139,34 @@ class LatentAttentionMixer(SplitPart, Mixer):
         # one row per position, read as key and as value
         return KvRequest(1, self.row_width, self.spec.window, 0)
 
+    def _expanded_rows(self, batch, group, run: RunContext, mid: torch.Tensor, gate):
+        """How many rows of every sequence the step expands into keys and values: 0 for its own rows alone, None for none."""
+        if (self.expand is None or batch.max_q_len < ops.TCGEN05_ATTENTION_MIN_ROWS or mid.stride(0) % 8 or mid.data_ptr() % 16
+                or (gate is not None and self.spec.gate_kind == "element" and (gate.stride(0) % 8 or gate.data_ptr() % 16))):
+            return None
+        fresh = getattr(batch, "fresh", False)
+        if mid.shape[0] < EXPANDED_TOKENS and (not fresh or self.spec.query_latent or self.spec.gate_kind == "element"):
+            return None
+        if fresh:
+            return 0
+        # (the page tables' width and not the lengths: a captured step replays for every length its class holds)
+        per = -(-group.block_table.shape[1] * run.k_pool.shape[2] // 64) * 64
+        fits = run.k_pool.shape[2] % 64 == 0 and self.turned % 8 == 0 and per * batch.kv_lens.numel() <= EXPANDED_ROWS * mid.shape[0]
+        return per if fits else None
+
+    def _expanded(self, q, down, gate, mid, batch, group, run: RunContext, cos, sin, key_rows: int) -> None:
+        s = self.spec
+        if q.stride(0) % 8 or q.data_ptr() % 16:
+            q = q.contiguous()
+        own, tail, q_tail = ops.latent_rows(down, self.latent_gain, self.turned, cos, sin, batch.positions, s.eps, run.k_pool, group.slot_mapping,
+                                            q=q, heads=s.num_heads, head_columns=s.head_dim + self.turned, padded=_whole(self.turned))
+        if key_rows:
+            own, tail = ops.latent_gather(run.k_pool, s.latent_dim, _whole(self.turned), group.block_table, batch.kv_lens, key_rows)
+        expanded = linear(own, self.expand, own.dtype)
+        at = s.num_heads * _whole(s.head_dim)
+        ops.prompt_attention(q, q_tail, expanded[:, :at], expanded[:, at:], tail, mid, batch.cu_q, batch.kv_lens, batch.max_q_len, s.num_heads,
+                             s.head_dim + self.turned, s.value_dim, s.scale, gate, s.window or 0, s.gate_kind if gate is not None else "head", key_rows)
+
     def inner(self, proj: torch.Tensor, mid: torch.Tensor, batch, run: RunContext, scale: float = 1.0) -> None:
         s = self.spec
         if run.k_pool is None:
@@ -141,24 +179,19 @@ class LatentAttentionMixer(SplitPart, Mixer):
         part = lambda role: proj[:, self.columns[role]] if role in self.columns else None  # noqa: E731
         cos, sin = (self.rope.cos, self.rope.sin) if self.rope is not None else (None, None)
         down_q, down, gate = part("down_q"), part("down"), part("gate")
-        q_rows = None
-        if down_q is None and down is not None:
+        expanded_rows = self._expanded_rows(batch, group, run, mid, gate)
+        if down_q is not None:
+            # (a prompt that expands its rows makes them beside its queries' tails, below)
+            own = down if expanded_rows is None else None
+            q = linear(ops.latent_prepare(down_q, self.query_gain, self.up_q.shape[1], own, self.latent_gain if own is not None else None, self.turned,
+                                          cos, sin, batch.positions, s.eps, run.k_pool, group.slot_mapping), self.up_q, proj.dtype)
+        else:
             q = part("q")
-            fresh = (self.expand is not None and getattr(batch, "fresh", False) and batch.max_q_len >= ops.TCGEN05_ATTENTION_MIN_ROWS
-                     and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and mid.stride(0) % 8 == 0 and mid.data_ptr() % 16 == 0)
-            more = {"q": q, "heads": s.num_heads, "head_columns": s.head_dim + self.turned, "padded": _whole(self.turned)} if fresh else {}
-            own, tail, q_tail = ops.latent_rows(down, self.latent_gain, self.turned, cos, sin, batch.positions, s.eps, run.k_pool,
-                                                group.slot_mapping, **more)
-            if fresh:
-                at = s.num_heads * _whole(s.head_dim)
-                expanded = linear(own, self.expand, own.dtype)
-                ops.prompt_attention(q, q_tail, expanded[:, :at], expanded[:, at:], tail, mid, batch.cu_q, batch.kv_lens, batch.max_q_len,
-                                     s.num_heads, s.head_dim + self.turned, s.value_dim, s.scale, gate, s.window or 0)
-                return
-        elif down_q is not None:
-            q_rows = ops.latent_prepare(down_q, self.query_gain if down_q is not None else None, self.up_q.shape[1] if down_q is not None else 0,
-                                        down, self.latent_gain, self.turned, cos, sin, batch.positions, s.eps, run.k_pool, group.slot_mapping)
-        q = part("q") if down_q is None else linear(q_rows, self.up_q, proj.dtype)
+        if expanded_rows is not None:
+            self._expanded(q, down, gate, mid, batch, group, run, cos, sin, expanded_rows)
+            return
+        if down_q is None and down is not None:
+            ops.latent_rows(down, self.latent_gain, self.turned, cos, sin, batch.positions, s.eps, run.k_pool, group.slot_mapping)
         rows = proj.shape[0]
         q_latent = torch.empty((rows, s.num_heads * self.row_width), dtype=proj.dtype, device=proj.device)
         ops.head_linear(q, self.into_latent, q_latent, s.num_heads, turned=self.turned, cos=cos, sin=sin, positions=batch.positions)

@@ -971,3 +971,89 @@ def test_retention_chunks(cuda_device, vdim, lengths, whole):
         assert float((chunk_out - out).norm() / out.norm()) < 2.0 ** -15
     else:
         close(chunk_out, out, torch.bfloat16)
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 64)])
+@pytest.mark.parametrize("cap,sink,turned", [(5.0, True, True), (0.0, True, False), (30.0, False, True)])
+def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
+    """Prompts at the edges of query tiles and pages, some on top of cached positions, with factors of either sign on the scores, against
+    the kernel with a warp per row."""
+    from models_b200.kernels import ops
+
+    heads, kv_heads, page = 4, 2, 64
+    g = torch.Generator().manual_seed(31)
+    q_lens, past = [33, 64, 129, 1, 70], [0, 100, 64, 5, 0]
+    lens = [a + b for a, b in zip(q_lens, past)]
+    pages = [-(-n // page) for n in lens]
+    table = torch.zeros(len(lens), max(pages), dtype=torch.int32)
+    order = (torch.randperm(sum(pages), generator=g) + 1).to(torch.int32)
+    at = 0
+    for i, n in enumerate(pages):
+        table[i, :n] = order[at:at + n]
+        at += n
+    k_pool, v_pool = (torch.randn(sum(pages) + 1, kv_heads, page, d, generator=g).bfloat16() for d in (dim, vdim))
+    for i, n in enumerate(lens):  # what lies behind a sequence's end belongs to nobody
+        if n % page:
+            k_pool[table[i, n // page], :, n % page:] = v_pool[table[i, n // page], :, n % page:] = float("nan")
+    T = sum(q_lens)
+    q = torch.randn(T, heads * dim, generator=g).bfloat16().cuda()
+    head_scale = torch.tensor([1.0, -0.7, 2.0, 0.0]).cuda()
+    angle = torch.rand(max(lens), vdim // 2, generator=g) * 6
+    turn = (angle.cos().cuda(), angle.sin().cuda()) if turned else (None, None)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()  # noqa: E731
+    outs = []
+    for kernel in (None, "rows"):
+        out = torch.full((T, heads * vdim), float("nan")).bfloat16().cuda()
+        with ops.recording() as names:
+            ops.gated_attention(q, out, k_pool.cuda(), v_pool.cuda(), table.cuda(), i32(np.concatenate([[0], np.cumsum(q_lens)]).tolist()), i32(lens),
+                                max(q_lens), heads, kv_heads, dim, vdim, "softmax", dim ** -0.5, head_scale=head_scale, softcap=cap, sink=sink,
+                                turn_cos=turn[0], turn_sin=turn[1], kernel=kernel)
+        assert names == ["gated_attention"]
+        outs.append(out.float())
+    # float weights either way: what differs is a rounding to bfloat16 of the result here and there
+    assert float((outs[0] - outs[1]).abs().max()) <= 2.0 ** -7 * float(outs[1].abs().max())
+    assert float((outs[0] - outs[1]).norm()) <= 2.0 ** -9 * float(outs[1].norm())
+
+
+@pytest.mark.parametrize("query_latent,gate_kind,window,turned", [(128, "element", 0, 64), (0, "head", 90, 32), (128, None, 64, 0)])
+@pytest.mark.parametrize("q_lens,past", [([70, 200], [0, 0]), ([150, 64, 129], [100, 0, 37]), ([33], [31])])
+def test_latent_prompts_expand_the_rows_they_see(cuda_device, monkeypatch, query_latent, gate_kind, window, turned, q_lens, past):
+    """A prompt whose rows are expanded into keys and values, from a sequence's start and on top of cached positions, gives what the
+    attention in the latent space gives."""
+    from models_b200.cache import KvCache
+    from models_b200.config.specs import LatentAttentionSpec, RopeSpec
+    from models_b200.engine.batch import build_step_batch
+    from models_b200.parts import RunContext, Runtime, build_part, latent_attention
+
+    monkeypatch.setattr(latent_attention, "EXPANDED_TOKENS", 0)
+    width, heads, dim, vdim, rank = 256, 4, 64, 128, 128
+    g = torch.Generator().manual_seed(41)
+    roles = ["down_q", "down_q_norm", "up_q", "q", "down", "down_norm", "up_k", "up_v", "gate", "o"]
+    spec = LatentAttentionSpec(hidden_size=width, num_heads=heads, head_dim=dim, value_dim=vdim, latent_dim=rank, scale=(dim + turned) ** -0.5, eps=1e-6,
+                               gated=gate_kind is not None, weights={r: r for r in roles}, query_latent=query_latent,
+                               position=RopeSpec(turned, 1e4, "half") if turned else None, window=window or None, gate_kind=gate_kind or "head")
+    outs = []
+    for expanded in (True, False):
+        mixer = build_part("mixer", spec, Runtime(torch.device("cuda:0"), "bfloat16", max_positions=512))
+        draw = torch.Generator().manual_seed(5)
+        mixer.load({p.name: (torch.randn(p.shape, generator=draw) * p.shape[-1] ** -0.5).bfloat16() if len(p.shape) > 1
+                    else 1 + 0.1 * torch.randn(p.shape, generator=draw) for p in mixer.parameters()})
+        assert mixer.expand is not None
+        if not expanded:
+            mixer.expand = None
+        cache = KvCache([mixer.kv_request()], [None], 64 * 20, len(q_lens))
+        cache.allocate_storage(lambda shape: torch.full(shape, float("nan"), dtype=torch.bfloat16, device="cuda:0"))
+        run = RunContext(run=0)
+        run.group, run.k_pool, run.v_pool = cache.pools(0)
+        slots = [cache.open_slot() for _ in q_lens]
+        rows = torch.Generator().manual_seed(6)
+        for counts in (past, q_lens):
+            entries = [(s, n) for s, n in zip(slots, counts) if n]
+            if entries:
+                cache.append(entries)
+                batch = build_step_batch(cache, [(s, [0] * n, []) for s, n in entries], torch.device("cuda:0"))
+                cache.commit(entries)
+                out = mixer.forward(torch.randn(sum(n for _, n in entries), width, generator=rows).bfloat16().cuda(), batch, run)
+        outs.append(out.float())
+    # keys, values and queries pass through bfloat16 at other places: four roundings' worth
+    assert float((outs[0] - outs[1]).norm()) <= 4 * 2.0 ** -8 * float(outs[1].norm())
