@@ -16,7 +16,7 @@
 //             queries go to the query buffer, keys and values straight into the paged cache
 //             (backend-java/.../llama/LlamaForwardPass.java:1070-1086).
 //
-// Layout of the work.  A block of four warps owns 16 weight rows at a time and walks a sequence of
+// Layout of the work.  A block of four warps (eight where it has one row tile of a long K) owns 16 weight rows at a time and walks a sequence of
 // such row tiles; its warps split the
 // block's part of K.  Each warp streams its rows with cp.async through a private four-stage ring in
 // shared memory, 128 columns per stage, and the stages run on across row tiles, so loads stay in flight
@@ -50,8 +50,11 @@ using bf16 = __nv_bfloat16;
 enum { PRO_NONE = 0, PRO_NORM = 1, PRO_PRE = 2 };
 enum { EPI_BF16 = 0, EPI_F32 = 1, EPI_RESIDUAL = 2, EPI_SWIGLU = 3, EPI_ROPE = 4, EPI_TANH = 5, EPI_SIDE = 6, EPI_PAIRS = 7 };
 
-constexpr int kWarps = 4;
-constexpr int kThreads = kWarps * 32;
+// Forms of a block: four warps that walk row tiles and keep the activations of their part of K, or eight with one row tile whose
+// activations pass through rings beside the weights'.  (Eight that walk tiles lost what the fuller last round gained: 8,192 pairs of
+// rows, 13.3 us in a chain of them with four warps, 14.2 with eight.)
+enum { FORM_FOUR = 0, FORM_EIGHT_STREAMED = 1 };
+__host__ __device__ constexpr int warps_of(int form) { return form == FORM_FOUR ? 4 : 8; }
 constexpr int kMaxResident = 4;  // most blocks per multiprocessor the planner counts on
 constexpr int kDepth = 4;        // stages of the weight ring
 constexpr int kStep = 128;       // columns per stage: 32 per piece, a lane takes 8 of each piece
@@ -138,9 +141,10 @@ struct SkinnyArgs {
     int pair_offset;      // EPI_SWIGLU: the up tile starts pair_offset rows after the gate tile
     int activation;       // EPI_SWIGLU: the gate's activation (MB_ACT_*)
     int k_split;          // blocks of a cluster that share K
-    int k_unit;           // columns per block, a multiple of 4 * kStep
+    int k_unit;           // columns per block, a multiple of kStep for every warp
     int k_warp;           // columns per warp, a multiple of kStep
     int clusters;         // clusters (of k_split blocks) in the grid; each walks row tiles cluster, cluster + clusters, ...
+    int form;             // FORM_*
     int dependent;        // launch as a programmatic dependent of the kernel before it
     // EPI_ROPE
     int heads, kv_heads, head_dim, page_size;
@@ -153,26 +157,32 @@ struct SkinnyArgs {
 };
 
 // Shared memory of a block, in bytes from the start:
-//   activations  [NT*8 rows][k_unit*2 + 64]          (row stride = 64 mod 128 keeps 8-lane phases conflict-free)
-//   ring         [4 warps][kDepth][2 halves][kPieces][32 lanes][16]
-//   partial      [2 buffers][4 warps][16][NT*8] floats, then sums of squares [NT*8], [4][NT*8]
-template <int NT, int EPI>
+//   activations  [NT*8 rows][k_unit*2 + 64]          (row stride = 64 mod 128 keeps 8-lane phases conflict-free),
+//                or, streamed, rings [warps][kDepth][NT][kPieces][32 lanes][16]
+//   ring         [warps][kDepth][2 halves][kPieces][32 lanes][16]
+//   partial      [2 buffers][warps][16][NT*8] floats, then sums of squares [NT*8], [warps][NT*8]
+template <int NT, int EPI, int kForm>
 struct SmemPlan {
+    static constexpr int kWarps = warps_of(kForm);
     static constexpr int COLS = NT * 8;
     static constexpr int kStageBytes = 2 * kPieces * 32 * 16;
     static constexpr int kPartialFloats = kWarps * 16 * COLS;
     static __host__ __device__ int x_stride(int k_unit) { return k_unit * 2 + 64; }
-    static __host__ __device__ int ring_offset(int k_unit) { return COLS * x_stride(k_unit); }
+    static constexpr int kXStageBytes = NT * kPieces * 32 * 16;
+    static __host__ __device__ int ring_offset(int k_unit) { return kForm == FORM_EIGHT_STREAMED ? kWarps * kDepth * kXStageBytes : COLS * x_stride(k_unit); }
     static __host__ __device__ int partial_offset(int k_unit) { return ring_offset(k_unit) + kWarps * kDepth * kStageBytes; }
     static __host__ __device__ int total(int k_unit) {
         return partial_offset(k_unit) + (2 * kPartialFloats + COLS + kWarps * COLS) * (int)sizeof(float);
     }
 };
 
-template <int NT, int PRO, int EPI>
-__global__ void __launch_bounds__(kThreads)
+template <int NT, int PRO, int EPI, int kForm>
+__global__ void __launch_bounds__(warps_of(kForm) * 32)
 skinny_gemm_kernel(const SkinnyArgs args) {
-    using Plan = SmemPlan<NT, EPI>;
+    using Plan = SmemPlan<NT, EPI, kForm>;
+    constexpr int kWarps = warps_of(kForm), kThreads = kWarps * 32;
+    constexpr bool kStreamed = kForm == FORM_EIGHT_STREAMED;  // activations in rings (one row tile: each is read once)
+    static_assert(!kStreamed || PRO != PRO_NORM, "rows that the kernel normalises are staged whole");
     constexpr int COLS = Plan::COLS;
     constexpr bool kPaired = EPI == EPI_SWIGLU || EPI == EPI_ROPE;  // MMA rows 8..15 are the partners of rows 0..7
     constexpr int kTileRows = kPaired ? 8 : 16;  // output rows (or pairs) per tile
@@ -197,7 +207,12 @@ skinny_gemm_kernel(const SkinnyArgs args) {
 
     // where this lane reads its activations: row group_id (and 8, 16, ... further), its warp's columns of K, the lane's 8 of every 32
     const int x_stride = Plan::x_stride(args.k_unit);
-    const uint32_t x_lane = smem_base + group_id * x_stride + ((k_begin - part_begin) + 8 * tid4) * 2;
+    const uint32_t x_lane = kStreamed ? smem_base + warp * kDepth * Plan::kXStageBytes + lane * 16
+                                      : smem_base + group_id * x_stride + ((k_begin - part_begin) + 8 * tid4) * 2;
+    auto x_at = [&](int nt, int step, int c) {
+        return kStreamed ? x_lane + (step % kDepth) * Plan::kXStageBytes + (nt * kPieces + c) * 512
+                         : x_lane + nt * 8 * x_stride + (step * kStep + 32 * c) * 2;
+    };
     // Activations that arrive as bfloat16 are not staged ahead of the products: every lane fetches exactly the pieces that
     // it will read itself (no barrier, not even within the warp), those of a step of K together with the step's weights.
     auto issue_activations = [&](int step) {
@@ -206,7 +221,7 @@ skinny_gemm_kernel(const SkinnyArgs args) {
 #pragma unroll
             for (int c = 0; c < kPieces; ++c) {
                 const int row = nt * 8 + group_id, col = k_begin + step * kStep + 32 * c + 8 * tid4;
-                const uint32_t dst = x_lane + nt * 8 * x_stride + (step * kStep + 32 * c) * 2;
+                const uint32_t dst = x_at(nt, step, c);
                 if (row < args.batch && col < k_end) cp_async16(dst, args.x + (size_t)row * args.ldx + col);
                 else sts128_zero(dst);
             }
@@ -362,6 +377,7 @@ skinny_gemm_kernel(const SkinnyArgs args) {
     bool sq_gathered = args.k_split == 1;
 
 
+    float held_scale = 0.0f;  // 1 / rms of the column of this thread's first finishing item (the same in every tile), from the first tile on
     // ---- row tile after row tile; the ring keeps running across them
     int stage_index = 0;
     for (int local = 0; local < tiles_mine; ++local) {
@@ -381,7 +397,7 @@ skinny_gemm_kernel(const SkinnyArgs args) {
             for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
                 for (int c = 0; c < kPieces; ++c) {
-                    const uint4 xv = lds128(x_lane + nt * 8 * x_stride + (step * kStep + 32 * c) * 2);
+                    const uint4 xv = lds128(x_at(nt, step, c));
                     mma_bf16(acc[nt], wv[0][c].x, wv[1][c].x, wv[0][c].y, wv[1][c].y, xv.x, xv.y);
                     mma_bf16(acc[nt], wv[0][c].z, wv[1][c].z, wv[0][c].w, wv[1][c].w, xv.z, xv.w);
                 }
@@ -469,15 +485,17 @@ skinny_gemm_kernel(const SkinnyArgs args) {
                     if (kPaired || pairs) second += from[(w * 16 + row_in_tile + 8) * COLS + col];
                 }
             }
-            if (PRO == PRO_NORM) {
-                const float inv_rms = 1.0f / sqrtf(sq_total[col] / (float)args.k + args.eps);
-                value *= inv_rms;
-                second *= inv_rms;
-            }
-            if (PRO == PRO_PRE) {
-                float sum = 0.0f;
-                for (int w = 0; w < kWarps; ++w) sum += sq_warp[w * COLS + col];
-                const float inv_rms = 1.0f / sqrtf(sum / (float)args.k + args.eps);
+            if (PRO != PRO_NONE) {
+                const bool first_item = i == (int)threadIdx.x;
+                float inv_rms = held_scale;
+                if (local == 0 || !first_item) {
+                    float sum = 0.0f;
+                    if (PRO == PRO_NORM) sum = sq_total[col];
+                    else
+                        for (int w = 0; w < kWarps; ++w) sum += sq_warp[w * COLS + col];
+                    inv_rms = 1.0f / sqrtf(sum / (float)args.k + args.eps);
+                    if (first_item) held_scale = inv_rms;
+                }
                 value *= inv_rms;
                 second *= inv_rms;
             }
@@ -565,11 +583,11 @@ skinny_gemm_kernel(const SkinnyArgs args) {
     if (args.k_split > 1) cluster_leave_together();
 }
 
-template <int NT, int PRO, int EPI>
+template <int NT, int PRO, int EPI, int kForm = FORM_FOUR>
 static int launch(const SkinnyArgs& args, cudaStream_t stream) {
-    using Plan = SmemPlan<NT, EPI>;
+    using Plan = SmemPlan<NT, EPI, kForm>;
     const int smem = Plan::total(args.k_unit);
-    auto kernel = skinny_gemm_kernel<NT, PRO, EPI>;
+    auto kernel = skinny_gemm_kernel<NT, PRO, EPI, kForm>;
     static int reserved = 0;
     if (smem > reserved) {
         cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -578,7 +596,7 @@ static int launch(const SkinnyArgs& args, cudaStream_t stream) {
     }
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(args.clusters * args.k_split);
-    config.blockDim = dim3(kThreads);
+    config.blockDim = dim3(warps_of(kForm) * 32);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     cudaLaunchAttribute attribute[2];
@@ -595,8 +613,14 @@ static int launch(const SkinnyArgs& args, cudaStream_t stream) {
     return check_launch("skinny_gemm");
 }
 
+// The products that may have one row tile a block and a long K.
+template <int EPI>
+constexpr bool kStreamable = EPI == EPI_BF16 || EPI == EPI_F32 || EPI == EPI_RESIDUAL || EPI == EPI_TANH;
+
 template <int PRO, int EPI>
 static int launch_nt(const SkinnyArgs& args, cudaStream_t stream) {
+    if constexpr (PRO == PRO_NONE && kStreamable<EPI>)
+        if (args.form == FORM_EIGHT_STREAMED) return launch<1, PRO, EPI, FORM_EIGHT_STREAMED>(args, stream);
     if (args.batch <= 8) return launch<1, PRO, EPI>(args, stream);
     if (args.batch <= 16) return launch<2, PRO, EPI>(args, stream);
     if (PRO != PRO_NONE) return fail("skinny_gemm: the norm prologues take at most 16 rows, got %d", args.batch);
@@ -647,9 +671,9 @@ static int skinny_gemm(const void* w, int ldw, int n, int k, int batch, const vo
                       : (epilogue == EPI_SWIGLU || epilogue == EPI_ROPE) ? (rows_total + 7) / 8 : (rows_total + 15) / 16;
     const int cols = batch <= 8 ? 8 : (batch <= 16 ? 16 : 32);
     auto smem_for = [&](int split) {
-        const int k_unit = ((k + split - 1) / split + kWarps * kStep - 1) / (kWarps * kStep) * (kWarps * kStep);
-        return (size_t)cols * (k_unit * 2 + 64) + (size_t)kWarps * kDepth * (2 * kPieces * 512) +
-               (size_t)(2 * kWarps * 16 * cols + (1 + kWarps) * cols) * sizeof(float);
+        const int k_unit = ((k + split - 1) / split + 4 * kStep - 1) / (4 * kStep) * (4 * kStep);
+        return (size_t)cols * (k_unit * 2 + 64) + (size_t)4 * kDepth * (2 * kPieces * 512) +
+               (size_t)(2 * 4 * 16 * cols + (1 + 4) * cols) * sizeof(float);
     };
     auto resident_for = [&](int split) {
         const size_t per_sm = 220 * 1024 / smem_for(split);
@@ -660,12 +684,19 @@ static int skinny_gemm(const void* w, int ldw, int n, int k, int batch, const vo
     if (smem_for(split) > 200 * 1024)
         return fail("skinny_gemm: %d activation rows of %d columns do not fit shared memory", batch, k);
     args.k_split = split;
-    args.k_unit = ((k + split - 1) / split + kWarps * kStep - 1) / (kWarps * kStep) * (kWarps * kStep);
-    args.k_warp = args.k_unit / kWarps;
-    const int resident_clusters = resident_for(split) / split;
+    const int prologue = norm ? PRO_NORM : (args.ssq_parts ? PRO_PRE : PRO_NONE);
+    const bool streamable = epilogue == EPI_BF16 || epilogue == EPI_F32 || epilogue == EPI_RESIDUAL || epilogue == EPI_TANH;
+    args.form = FORM_FOUR;
+    // One row tile a block and a K so long that its activations leave room for one block on a multiprocessor: eight warps and rings
+    // for the activations keep twice the weights in flight and halve a warp's steps (2,048 rows, K 8,192: 9.1 us in a chain of them,
+    // and 8.0; at K 2,048 there was nothing to gain).
+    if (streamable && prologue == PRO_NONE && split == 1 && batch <= 8 && tiles <= multiprocessors && k > 4096) args.form = FORM_EIGHT_STREAMED;
+    const int warps = warps_of(args.form);
+    args.k_unit = ((k + split - 1) / split + warps * kStep - 1) / (warps * kStep) * (warps * kStep);
+    args.k_warp = args.k_unit / warps;
+    const int resident_clusters = args.form == FORM_FOUR ? resident_for(split) / split : multiprocessors;
     args.clusters = tiles < resident_clusters ? tiles : resident_clusters;
     if (args.clusters < 1) args.clusters = 1;
-    const int prologue = norm ? PRO_NORM : (args.ssq_parts ? PRO_PRE : PRO_NONE);
     if (prologue == PRO_PRE && (batch > 16 || args.ssq_count <= 0 || ((uintptr_t)args.ssq_parts & 15)))
         return fail("skinny_gemm: parts of sums of squares come with at most 16 rows, a count, and 16-byte alignment");
     if (args.emit_gain && (epilogue != EPI_RESIDUAL || !args.emit_rows || !args.emit_ssq))
