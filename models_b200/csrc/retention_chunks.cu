@@ -5,11 +5,14 @@
 //   o_i = a^(i + 1) S_0^T q_i + sum_(j <= i) a^(i - j) (q_i . k_j) v_j,     S_end = a^n S_0 + sum_j a^(n - 1 - j) k_j v_j^T
 // Three kernels: what every chunk adds to the state, a product per (chunk, head); the states that the chunks start from, element by
 // element in the chunks' order; every chunk's results, with the head's norm and gate where the caller wants them here.
-// The numbers between the first products and the last one are floats: every operand goes into its products as two bfloat16 numbers,
-// its rounding and the rounding of what that left (16 bits of mantissa), three of the four products of parts, added up in float.
+// The numbers between the first products and the last one are floats, and none of their 24 bits is lost on the way into a product:
+// every operand is three bfloat16 numbers, its rounding, the rounding of what that left and of what this left, and six of the nine
+// products of parts are added up in float (the other three are below 2^-26 of the product).
+// Against 64 bits, over steps of 64 to 2,048 tokens: the state is off by 6e-8 to 9e-8 of itself (the walk in runs: 0.9e-7 to 1.4e-7), the
+// raw results by 0.7e-7 to 1.1e-7 (0.8e-7 to 1.8e-7); with two parts the operands would be cut to 16 bits.
 // Three sequences of 2,048 tokens in all, 16 heads of 64 x 128 with activated projections: 208 us as the walk in runs (98, 70 and 40),
-// which float multiply-adds from shared memory bound; here 23, 9 and 60 us, bound by the instructions that activate and split
-// what every chunk reads.
+// which float multiply-adds from shared memory bound; here 32, 14 and 58 us, bound by the six products for one and by the
+// instructions that activate and split what every chunk reads.
 #include "common.cuh"
 
 MB_DEFINE_LAST_ERROR()
@@ -20,9 +23,10 @@ using bf16 = __nv_bfloat16;
 
 constexpr int kChunk = 64;    // tokens of a chunk
 constexpr int kDim = 64;      // a key head's numbers
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;  // eight warps: four of 16 rows each for either half of the V columns
 constexpr int kKeyRow = kDim + 8;                // bfloat16 numbers of a padded row: ldmatrix without bank conflicts
-constexpr int kKeyPlane = kChunk * kKeyRow;      // the roundings of 64 rows; the rests lie behind them
+constexpr int kKeyPlane = kChunk * kKeyRow;      // one part of 64 rows; an operand's three planes lie one after another
+constexpr int kParts = 3;
 
 template <int V>
 struct Values {
@@ -44,8 +48,7 @@ struct RetentionArgs {
     int out_stride;
     float* raw_out;
     int raw_stride;
-    float* added;  // scratch by (place of the chunk, head): [kDim][V]
-    bf16* starts;  // scratch by (place, head): [2][kDim][V], roundings and rests
+    float* starts;  // scratch by (place of the chunk, head): [kDim][V], what the chunk adds, then the state that it starts from
 };
 
 // Every sequence's chunks lie one after another, a sequence's first place being floor(first / 64) + seq (a sequence of n tokens has
@@ -64,31 +67,59 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Two floats as a pair of bfloat16 roundings and the pair of what the roundings left over.
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+// Two floats as pairs of bfloat16 numbers: their roundings, the roundings of what those left, and of what these left.
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    const float2 back = __bfloat1622float2(h);
+    float2 back = __bfloat1622float2(h);
+    a -= back.x, b -= back.y;
+    const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
+    back = __bfloat1622float2(m);
     const __nv_bfloat162 l = __floats2bfloat162_rn(a - back.x, b - back.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
+    mid = *reinterpret_cast<const uint32_t*>(&m);
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
-__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+// Eight floats into an operand's three planes.
+__device__ __forceinline__ void store_parts(bf16* to, int plane, const float (&x)[8]) {
+    uint4 hi, mid, lo;
+    split_pair(x[0], x[1], hi.x, mid.x, lo.x);
+    split_pair(x[2], x[3], hi.y, mid.y, lo.y);
+    split_pair(x[4], x[5], hi.z, mid.z, lo.z);
+    split_pair(x[6], x[7], hi.w, mid.w, lo.w);
+    *reinterpret_cast<uint4*>(to) = hi;
+    *reinterpret_cast<uint4*>(to + plane) = mid;
+    *reinterpret_cast<uint4*>(to + 2 * plane) = lo;
 }
 
-// d[tile] += a (roundings, rests) . b for two neighbouring tiles of eight columns; the four products of parts but the last.
-__device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], const uint32_t (&a_hi)[4], const uint32_t (&a_lo)[4],
-                                               const uint32_t (&b_hi)[4], const uint32_t (&b_lo)[4]) {
-    mma_bf16(d0, a_lo, b_hi[0], b_hi[1]);
-    mma_bf16(d1, a_lo, b_hi[2], b_hi[3]);
-    mma_bf16(d0, a_hi, b_lo[0], b_lo[1]);
-    mma_bf16(d1, a_hi, b_lo[2], b_lo[3]);
-    mma_bf16(d0, a_hi, b_hi[0], b_hi[1]);
-    mma_bf16(d1, a_hi, b_hi[2], b_hi[3]);
+using Parts = uint32_t[kParts][4];
+__device__ __forceinline__ void load_parts(Parts& r, uint32_t at, int plane) {
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) ldmatrix4(r[i], at + 2 * i * plane);
+}
+__device__ __forceinline__ void load_parts_turned(Parts& r, uint32_t at, int plane) {
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) ldmatrix4_turned(r[i], at + 2 * i * plane);
+}
+// d[tile] += a . b for two neighbouring tiles of eight columns.  The tensor cores cut their sums off where a float addition rounds, so
+// the sixteen products of roundings, whose sum has few bits to lose, and the smaller ones, the smallest first, start from zero and are
+// added as floats (all in one chain: results of 2,048 tokens off by 8.9e-7 where the walk is off by 1e-7).
+__device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], const Parts& a, const Parts& b) {
+    float p0[4] = {}, p1[4] = {}, r0[4] = {}, r1[4] = {};
+#pragma unroll
+    for (int order = kParts - 1; order > 0; --order)
+#pragma unroll
+        for (int i = 0; i <= order; ++i) {
+            mma_bf16(r0, a[i], b[order - i][0], b[order - i][1]);
+            mma_bf16(r1, a[i], b[order - i][2], b[order - i][3]);
+        }
+    mma_bf16(p0, a[0], b[0][0], b[0][1]);
+    mma_bf16(p1, a[0], b[0][2], b[0][3]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d0[i] += p0[i] + r0[i], d1[i] += p1[i] + r1[i];
 }
 
 // The rows of `count` tokens (64 with zeros behind them) of a head, `kCols` columns from `src`, activated, rotated (rotary > 0),
-// times weight[row] (or 1), in two planes of rows of `row` numbers.
+// times weight[row] (or 1), in planes of rows of `row_numbers`.
 template <int kCols>
 __device__ __forceinline__ void stage_rows(bf16* planes, int row_numbers, int plane_numbers, const bf16* src, const RetentionArgs& args, int count,
                                            int rotary, int position0, const float* weight) {
@@ -118,17 +149,12 @@ __device__ __forceinline__ void stage_rows(bf16* planes, int row_numbers, int pl
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] *= factor;
         }
-        uint4 hi, lo;
-        split_pair(x[0], x[1], hi.x, lo.x);
-        split_pair(x[2], x[3], hi.y, lo.y);
-        split_pair(x[4], x[5], hi.z, lo.z);
-        split_pair(x[6], x[7], hi.w, lo.w);
-        *reinterpret_cast<uint4*>(planes + row * row_numbers + c) = hi;
-        *reinterpret_cast<uint4*>(planes + plane_numbers + row * row_numbers + c) = lo;
+        store_parts(planes + row * row_numbers + c, plane_numbers, x);
     }
 }
 
-// grid (heads, most chunks of a sequence, sequences); block kThreads.  A warp has 16 coordinates of what the chunk adds.
+// grid (heads, most chunks of a sequence, sequences); block kThreads.  A warp has 16 coordinates and half of the columns of what the
+// chunk adds.
 template <int V>
 __global__ void __launch_bounds__(kThreads)
 retention_chunk_adds_kernel(const RetentionArgs args) {
@@ -136,7 +162,7 @@ retention_chunk_adds_kernel(const RetentionArgs args) {
     grid_dependency_wait();
     extern __shared__ __align__(16) unsigned char shared[];
     bf16* keys = reinterpret_cast<bf16*>(shared);
-    bf16* values = keys + 2 * kKeyPlane;
+    bf16* values = keys + kParts * kKeyPlane;
     __shared__ float weight[kChunk];
     const int head = blockIdx.x, chunk = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
     const int first = args.cu_q[seq], count = min(kChunk, args.cu_q[seq + 1] - first - chunk * kChunk);
@@ -148,33 +174,30 @@ retention_chunk_adds_kernel(const RetentionArgs args) {
     const int position0 = args.rotary_dim > 0 ? args.positions[first] + chunk * kChunk : 0;
     stage_rows<kDim>(keys, kKeyRow, kKeyPlane, args.k + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, weight);
     __syncthreads();
-    const int warp = tid >> 5, lane = tid & 31;
-    float acc[V / 8][4] = {};
-    const uint32_t key_at = smem_u32(keys) + (((lane >> 4) * 8 + (lane & 7)) * kKeyRow + 16 * warp + ((lane >> 3) & 1) * 8) * 2;
-    const uint32_t value_at = smem_u32(values) + ((lane & 15) * Values<V>::row + (lane >> 4) * 8) * 2;
+    const int tile = (tid >> 5) & 3, column0 = (tid >> 7) * (V / 2), lane = tid & 31;
+    float acc[V / 16][4] = {};
+    const uint32_t key_at = smem_u32(keys) + (((lane >> 4) * 8 + (lane & 7)) * kKeyRow + 16 * tile + ((lane >> 3) & 1) * 8) * 2;
+    const uint32_t value_at = smem_u32(values) + ((lane & 15) * Values<V>::row + column0 + (lane >> 4) * 8) * 2;
 #pragma unroll
     for (int j = 0; j < kChunk; j += 16) {
-        uint32_t a_hi[4], a_lo[4];
-        ldmatrix4_turned(a_hi, key_at + j * kKeyRow * 2);
-        ldmatrix4_turned(a_lo, key_at + (kKeyPlane + j * kKeyRow) * 2);
+        Parts a, b;
+        load_parts_turned(a, key_at + j * kKeyRow * 2, kKeyPlane);
 #pragma unroll
-        for (int n = 0; n < V / 8; n += 2) {
-            uint32_t b_hi[4], b_lo[4];
-            ldmatrix4_turned(b_hi, value_at + (j * Values<V>::row + 8 * n) * 2);
-            ldmatrix4_turned(b_lo, value_at + (Values<V>::plane + j * Values<V>::row + 8 * n) * 2);
-            split_products(acc[n], acc[n + 1], a_hi, a_lo, b_hi, b_lo);
+        for (int n = 0; n < V / 16; n += 2) {
+            load_parts_turned(b, value_at + (j * Values<V>::row + 8 * n) * 2, Values<V>::plane);
+            split_products(acc[n], acc[n + 1], a, b);
         }
     }
-    float* to = args.added + (place_of(first, seq, chunk) * args.heads + head) * kDim * V + (size_t)(16 * warp + (lane >> 2)) * V + 2 * (lane & 3);
+    float* to = args.starts + (place_of(first, seq, chunk) * args.heads + head) * kDim * V + (size_t)(16 * tile + (lane >> 2)) * V + column0 + 2 * (lane & 3);
 #pragma unroll
-    for (int n = 0; n < V / 8; ++n) {
+    for (int n = 0; n < V / 16; ++n) {
         *reinterpret_cast<float2*>(to + 8 * n) = make_float2(acc[n][0], acc[n][1]);
         *reinterpret_cast<float2*>(to + 8 * V + 8 * n) = make_float2(acc[n][2], acc[n][3]);
     }
 }
 
-// grid (kDim * V / 4 / 128, heads, sequences); block 128: four neighbouring elements a thread.  S before every chunk to `starts`, the
-// state after the last one to the state area; eight chunks' additions are asked for at a time.
+// grid (kDim * V / 4 / 128, heads, sequences); block 128: four neighbouring elements a thread.  S before every chunk in the place of
+// what the chunk adds, the state after the last one to the state area; eight chunks' additions are asked for at a time.
 template <int V>
 __global__ void __launch_bounds__(128)
 retention_chunk_starts_kernel(const RetentionArgs args) {
@@ -185,8 +208,7 @@ retention_chunk_starts_kernel(const RetentionArgs args) {
     if (tokens <= 0) return;
     const int chunks = (tokens + kChunk - 1) / kChunk;
     const size_t item = place_of(first, seq, 0) * args.heads + head, stride = (size_t)args.heads * kDim * V;
-    const float* added = args.added + item * kDim * V + e;
-    bf16* start = args.starts + 2 * item * kDim * V + e;
+    float* start = args.starts + item * kDim * V + e;
     float* stored = args.state + ((size_t)args.slots[seq] * args.heads + head) * kDim * V + e;
     const float a = args.decay[head], whole = powf(a, (float)kChunk), last = powf(a, (float)(tokens - (chunks - 1) * kChunk));
     float4 s = *reinterpret_cast<const float4*>(stored);
@@ -195,15 +217,11 @@ retention_chunk_starts_kernel(const RetentionArgs args) {
         float4 b[kAtOnce];
 #pragma unroll
         for (int i = 0; i < kAtOnce; ++i)
-            if (c0 + i < chunks) b[i] = __ldcg(reinterpret_cast<const float4*>(added + (c0 + i) * stride));
+            if (c0 + i < chunks) b[i] = __ldcg(reinterpret_cast<const float4*>(start + (c0 + i) * stride));
 #pragma unroll
         for (int i = 0; i < kAtOnce; ++i) {
             if (c0 + i >= chunks) break;
-            uint2 hi, lo;
-            split_pair(s.x, s.y, hi.x, lo.x);
-            split_pair(s.z, s.w, hi.y, lo.y);
-            *reinterpret_cast<uint2*>(start + 2 * (c0 + i) * stride) = hi;
-            *reinterpret_cast<uint2*>(start + 2 * (c0 + i) * stride + kDim * V) = lo;
+            *reinterpret_cast<float4*>(start + (c0 + i) * stride) = s;
             const float keep = c0 + i + 1 < chunks ? whole : last;
             s = make_float4(fmaf(keep, s.x, b[i].x), fmaf(keep, s.y, b[i].y), fmaf(keep, s.z, b[i].z), fmaf(keep, s.w, b[i].w));
         }
@@ -211,66 +229,86 @@ retention_chunk_starts_kernel(const RetentionArgs args) {
     *reinterpret_cast<float4*>(stored) = s;
 }
 
-// grid (heads, most chunks of a sequence, sequences); block kThreads: a warp has 16 tokens and all V columns of their results.
+// grid (heads, most chunks of a sequence, sequences); block kThreads: a warp has 16 tokens and half of the V columns of their
+// results (both halves' warps make the weights that they share).  The values take the start's place in shared memory, so that two blocks
+// fit on a multiprocessor; they wait in registers until then.
 template <int V>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
 retention_chunk_results_kernel(const RetentionArgs args) {
     constexpr int kRow = Values<V>::row, kPlane = Values<V>::plane;
     grid_launch_dependents();
     grid_dependency_wait();
     extern __shared__ __align__(16) unsigned char shared[];
     bf16* queries = reinterpret_cast<bf16*>(shared);
-    bf16* keys = queries + 2 * kKeyPlane;
-    bf16* values = keys + 2 * kKeyPlane;
-    bf16* start = values + 2 * kPlane;
-    __shared__ float power[kChunk + 1];
+    bf16* keys = queries + kParts * kKeyPlane;
+    bf16* wide = keys + kParts * kKeyPlane;
+    __shared__ float power[kChunk + 1], square_sums[2][kChunk];
     const int head = blockIdx.x, chunk = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
     const int first = args.cu_q[seq], count = min(kChunk, args.cu_q[seq + 1] - first - chunk * kChunk);
     if (count <= 0) return;
     const size_t token0 = (size_t)first + chunk * kChunk;
+    constexpr int kPieces = 64 * V / 8 / kThreads;  // eights of the start, and of the values, that a thread brings
     {
-        const bf16* from = args.starts + 2 * (place_of(first, seq, chunk) * args.heads + head) * kDim * V;
-#pragma unroll 4
-        for (int i = tid; i < 2 * kDim * V / 8; i += kThreads) copy16_async(smem_u32(start + i / (V / 8) * kRow + i % (V / 8) * 8), from + 8 * i);  // (the planes' rows run on)
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const float* from = args.starts + (place_of(first, seq, chunk) * args.heads + head) * kDim * V;
+        float x[kPieces][8];
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) load8(from + 8 * (tid + i * kThreads), x[i]);
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int piece = tid + i * kThreads;
+            store_parts(wide + piece / (V / 8) * kRow + piece % (V / 8) * 8, kPlane, x[i]);
+        }
     }
     if (tid <= kChunk) power[tid] = powf(args.decay[head], (float)tid);
     const int position0 = args.rotary_dim > 0 ? args.positions[first] + chunk * kChunk : 0;
     stage_rows<kDim>(queries, kKeyRow, kKeyPlane, args.q + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, nullptr);
     stage_rows<kDim>(keys, kKeyRow, kKeyPlane, args.k + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, nullptr);
-    stage_rows<V>(values, kRow, kPlane, args.v + token0 * args.in_stride + (size_t)head * V, args, count, 0, 0, nullptr);
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    uint4 raw_values[kPieces];
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+        const int piece = tid + i * kThreads, row = piece / (V / 8);
+        raw_values[i] = make_uint4(0, 0, 0, 0);
+        if (row < count) raw_values[i] = *reinterpret_cast<const uint4*>(args.v + (token0 + row) * args.in_stride + (size_t)head * V + piece % (V / 8) * 8);
+    }
     __syncthreads();
-    const int warp = tid >> 5, lane = tid & 31, group = lane >> 2, pair = 2 * (lane & 3);
+    const int warp = (tid >> 5) & 3, half_columns = tid >> 7, column0 = half_columns * (V / 2), lane = tid & 31, group = lane >> 2, pair = 2 * (lane & 3);
     const uint32_t query_at = smem_u32(queries) + ((16 * warp + (lane & 15)) * kKeyRow + (lane >> 4) * 8) * 2;
-    const uint32_t across = ((lane & 15) * kRow + (lane >> 4) * 8) * 2;  // [k][column] tiles of V columns
-    const uint32_t start_at = smem_u32(start) + across, value_at = smem_u32(values) + across;
+    const uint32_t wide_at = smem_u32(wide) + ((lane & 15) * kRow + column0 + (lane >> 4) * 8) * 2;  // [k][column] tiles of V columns
     const uint32_t key_at = smem_u32(keys) + (((lane >> 4) * 8 + (lane & 7)) * kKeyRow + ((lane >> 3) & 1) * 8) * 2;
-    float acc[V / 8][4] = {}, weights[kChunk / 8][4] = {};
+    float acc[V / 16][4] = {}, weights[kChunk / 8][4] = {};
 #pragma unroll
     for (int d = 0; d < kDim; d += 16) {
-        uint32_t a_hi[4], a_lo[4];
-        ldmatrix4(a_hi, query_at + d * 2);
-        ldmatrix4(a_lo, query_at + (kKeyPlane + d) * 2);
+        Parts a, b;
+        load_parts(a, query_at + d * 2, kKeyPlane);
 #pragma unroll
-        for (int n = 0; n < V / 8; n += 2) {  // S_0^T q
-            uint32_t b_hi[4], b_lo[4];
-            ldmatrix4_turned(b_hi, start_at + (d * kRow + 8 * n) * 2);
-            ldmatrix4_turned(b_lo, start_at + (kPlane + d * kRow + 8 * n) * 2);
-            split_products(acc[n], acc[n + 1], a_hi, a_lo, b_hi, b_lo);
+        for (int n = 0; n < V / 16; n += 2) {  // S_0^T q
+            load_parts_turned(b, wide_at + (d * kRow + 8 * n) * 2, kPlane);
+            split_products(acc[n], acc[n + 1], a, b);
         }
 #pragma unroll
         for (int n = 0; n < kChunk / 8; n += 2) {  // q . k over the tokens up to the warp's last
             if (n > 2 * warp) break;
-            uint32_t b_hi[4], b_lo[4];
-            ldmatrix4(b_hi, key_at + (8 * n * kKeyRow + d) * 2);
-            ldmatrix4(b_lo, key_at + (kKeyPlane + 8 * n * kKeyRow + d) * 2);
-            split_products(weights[n], weights[n + 1], a_hi, a_lo, b_hi, b_lo);
+            load_parts(b, key_at + (8 * n * kKeyRow + d) * 2, kKeyPlane);
+            split_products(weights[n], weights[n + 1], a, b);
         }
     }
+    __syncthreads();  // nobody reads the start any more
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+        const int piece = tid + i * kThreads;
+        const uint32_t w[4] = {raw_values[i].x, raw_values[i].y, raw_values[i].z, raw_values[i].w};
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[2 * j] = __uint_as_float(w[j] << 16), x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+        if (args.input_act >= 0 && piece / (V / 8) < count)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = gate_activation(args.input_act, x[j]);
+        store_parts(wide + piece / (V / 8) * kRow + piece % (V / 8) * 8, kPlane, x);
+    }
+    __syncthreads();
     const int row = 16 * warp + group;
 #pragma unroll
-    for (int n = 0; n < V / 8; ++n)
+    for (int n = 0; n < V / 16; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[n][i] *= power[row + 8 * (i / 2) + 1];
 #pragma unroll
@@ -283,42 +321,45 @@ retention_chunk_results_kernel(const RetentionArgs args) {
                 const int age = row + 8 * (i / 2) - (8 * m + pair + i % 2);
                 weights[m][i] = age >= 0 ? weights[m][i] * (args.key_scale * power[max(age, 0)]) : 0.0f;
             }
-        uint32_t a_hi[4], a_lo[4];
-        split_pair(weights[n][0], weights[n][1], a_hi[0], a_lo[0]);
-        split_pair(weights[n][2], weights[n][3], a_hi[1], a_lo[1]);
-        split_pair(weights[n + 1][0], weights[n + 1][1], a_hi[2], a_lo[2]);
-        split_pair(weights[n + 1][2], weights[n + 1][3], a_hi[3], a_lo[3]);
+        Parts a, b;
+        split_pair(weights[n][0], weights[n][1], a[0][0], a[1][0], a[2][0]);
+        split_pair(weights[n][2], weights[n][3], a[0][1], a[1][1], a[2][1]);
+        split_pair(weights[n + 1][0], weights[n + 1][1], a[0][2], a[1][2], a[2][2]);
+        split_pair(weights[n + 1][2], weights[n + 1][3], a[0][3], a[1][3], a[2][3]);
 #pragma unroll
-        for (int c = 0; c < V / 8; c += 2) {
-            uint32_t b_hi[4], b_lo[4];
-            ldmatrix4_turned(b_hi, value_at + (8 * n * kRow + 8 * c) * 2);
-            ldmatrix4_turned(b_lo, value_at + (kPlane + 8 * n * kRow + 8 * c) * 2);
-            split_products(acc[c], acc[c + 1], a_hi, a_lo, b_hi, b_lo);
+        for (int c = 0; c < V / 16; c += 2) {
+            load_parts_turned(b, wide_at + (8 * n * kRow + 8 * c) * 2, kPlane);
+            split_products(acc[c], acc[c + 1], a, b);
         }
+    }
+    if (args.raw_out == nullptr) {  // a row's V results lie with four neighbouring lanes of two warps
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float squares = 0.0f;
+#pragma unroll
+            for (int n = 0; n < V / 16; ++n) squares = fmaf(acc[n][2 * half], acc[n][2 * half], fmaf(acc[n][2 * half + 1], acc[n][2 * half + 1], squares));
+            squares += __shfl_xor_sync(0xffffffffu, squares, 1);
+            squares += __shfl_xor_sync(0xffffffffu, squares, 2);
+            if (pair == 0) square_sums[half_columns][row + 8 * half] = squares;
+        }
+        __syncthreads();
     }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int to = row + 8 * half;
         float factor = args.out_scale;
-        if (args.raw_out == nullptr) {  // a row's V results lie with four neighbouring lanes
-            float squares = 0.0f;
-#pragma unroll
-            for (int n = 0; n < V / 8; ++n) squares = fmaf(acc[n][2 * half], acc[n][2 * half], fmaf(acc[n][2 * half + 1], acc[n][2 * half + 1], squares));
-            squares += __shfl_xor_sync(0xffffffffu, squares, 1);
-            squares += __shfl_xor_sync(0xffffffffu, squares, 2);
-            factor /= sqrtf(squares / (float)V + args.eps);
-        }
+        if (args.raw_out == nullptr) factor /= sqrtf((square_sums[0][to] + square_sums[1][to]) / (float)V + args.eps);
         if (to >= count) continue;
-        const size_t column = (size_t)head * V + pair;
+        const size_t column = (size_t)head * V + column0 + pair;
         if (args.raw_out != nullptr) {
             float* dst = args.raw_out + (token0 + to) * args.raw_stride + column;
 #pragma unroll
-            for (int n = 0; n < V / 8; ++n) *reinterpret_cast<float2*>(dst + 8 * n) = make_float2(acc[n][2 * half] * factor, acc[n][2 * half + 1] * factor);
+            for (int n = 0; n < V / 16; ++n) *reinterpret_cast<float2*>(dst + 8 * n) = make_float2(acc[n][2 * half] * factor, acc[n][2 * half + 1] * factor);
         } else {
             const bf16* gate = args.g + (token0 + to) * args.in_stride + column;
             bf16* dst = args.out + (token0 + to) * args.out_stride + column;
 #pragma unroll
-            for (int n = 0; n < V / 8; ++n) {
+            for (int n = 0; n < V / 16; ++n) {
                 const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gate + 8 * n));
                 *reinterpret_cast<__nv_bfloat162*>(dst + 8 * n) = __floats2bfloat162_rn(acc[n][2 * half] * factor * (z.x / (1.0f + expf(-z.x))),
                                                                                        acc[n][2 * half + 1] * factor * (z.y / (1.0f + expf(-z.y))));
@@ -336,7 +377,7 @@ static int reserve(Kernel kernel, int bytes) {
 
 template <int V>
 static int launch_chunks(const RetentionArgs& args, int sequences, int chunks, cudaStream_t stream) {
-    constexpr int adds = (2 * kKeyPlane + 2 * Values<V>::plane) * 2, results = (4 * kKeyPlane + 4 * Values<V>::plane) * 2;
+    constexpr int adds = kParts * (kKeyPlane + Values<V>::plane) * 2, results = kParts * (2 * kKeyPlane + Values<V>::plane) * 2;
     if (int status = reserve(retention_chunk_adds_kernel<V>, adds)) return status;
     if (int status = reserve(retention_chunk_results_kernel<V>, results)) return status;
     const dim3 grid(args.heads, chunks, sequences);
@@ -352,12 +393,12 @@ using namespace mb;
 
 MB_EXPORT int mb_retention_chunk_tokens() { return kChunk; }
 
-// Arguments as mb_retention_scan's, bfloat16 storage, head_dim 64, value_dim 64 or 128, whole aligned rows (see the checks).  added:
-// (places * heads * 64 * value_dim) floats, starts: twice as many bfloat16 numbers, with places = tokens / 64 + sequences.
+// Arguments as mb_retention_scan's, bfloat16 storage, head_dim 64, value_dim 64 or 128, whole aligned rows (see the checks).  starts:
+// (places * heads * 64 * value_dim) floats, with places = tokens / 64 + sequences.
 MB_EXPORT int mb_retention_chunks(const void* q, const void* k, const void* v, const void* g, int in_stride, const int* positions,
                                   const float* cos_table, const float* sin_table, int rotary_dim, const float* decay, float key_scale, float eps,
                                   float* state, const int* slots, const int* cu_q, int sequences, int heads, int head_dim, int value_dim, void* out,
-                                  int out_stride, float out_scale, int max_q_len, float* added, void* starts, int input_act, float* raw_out,
+                                  int out_stride, float out_scale, int max_q_len, float* starts, int input_act, float* raw_out,
                                   int raw_stride, cudaStream_t stream) {
     if (sequences <= 0 || heads <= 0 || max_q_len <= 0) return 0;
     if (input_act >= MB_ACT_COUNT) return fail("retention_chunks: unknown activation code %d", input_act);
@@ -367,7 +408,7 @@ MB_EXPORT int mb_retention_chunks(const void* q, const void* k, const void* v, c
     if (!raw_out && (!out || !g)) return fail("retention_chunks: results go to raw_out, or gated to out");
     const int chunks = (max_q_len + kChunk - 1) / kChunk;
     if (sequences > 65535 || chunks > 65535 || heads > 65535) return fail("retention_chunks: %d sequences of up to %d chunks and %d heads exceed the grid", sequences, chunks, heads);
-    if (in_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)k & 15) || ((uintptr_t)v & 15) || ((uintptr_t)state & 15) || ((uintptr_t)added & 15) ||
+    if (in_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)k & 15) || ((uintptr_t)v & 15) || ((uintptr_t)state & 15) ||
         ((uintptr_t)starts & 15) || (raw_out && (raw_stride % 2 || ((uintptr_t)raw_out & 7))) ||
         (!raw_out && (out_stride % 2 || ((uintptr_t)out & 3) || ((uintptr_t)g & 3))))
         return fail("retention_chunks: rows of whole, aligned pieces are needed");
@@ -377,6 +418,6 @@ MB_EXPORT int mb_retention_chunks(const void* q, const void* k, const void* v, c
     args.decay = decay, args.key_scale = key_scale, args.eps = eps, args.out_scale = out_scale;
     args.state = state, args.slots = slots, args.cu_q = cu_q, args.heads = heads, args.input_act = input_act;
     args.out = (bf16*)out, args.out_stride = out_stride, args.raw_out = raw_out, args.raw_stride = raw_stride;
-    args.added = added, args.starts = (bf16*)starts;
+    args.starts = starts;
     return value_dim == 64 ? launch_chunks<64>(args, sequences, chunks, stream) : launch_chunks<128>(args, sequences, chunks, stream);
 }

@@ -1256,12 +1256,11 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.T
     if run_length is None and retention_chunks_takes(q, k, v, g, out, raw_out, state, head_dim, value_dim, max_q_len):
         lib = retention_chunks_library()
         items = (tokens // lib.mb_retention_chunk_tokens() + cu_q.numel() - 1) * heads * head_dim * value_dim
-        added = torch.empty((items,), dtype=torch.float32, device=q.device)
-        starts = torch.empty((2 * items,), dtype=torch.bfloat16, device=q.device)
+        starts = torch.empty((items,), dtype=torch.float32, device=q.device)
         _run(lib, lib.mb_retention_chunks(_p(q), _p(k), _p(v), _p(g), q.stride(0), _p(positions), _p(cos), _p(sin), rotary_dim, _p(decay),
                                           ctypes.c_float(key_scale), ctypes.c_float(eps), _p(state), _p(slots), _p(cu_q), cu_q.numel() - 1, heads,
                                           head_dim, value_dim, _p(out), out.stride(0) if out is not None else 0, ctypes.c_float(out_scale),
-                                          max_q_len, _p(added), _p(starts), activation_code(input_activation) if input_activation is not None else -1,
+                                          max_q_len, _p(starts), activation_code(input_activation) if input_activation is not None else -1,
                                           _p(raw_out), raw_out.stride(0) if raw_out is not None else 0, _stream()))
         _launches[0] += 2  # three kernels
         return
