@@ -346,6 +346,60 @@ group_norm_gate_kernel(const float* __restrict__ raw, int raw_stride, const floa
     }
 }
 
+// The same in eights, a row's numbers held from the sum to the store: rows of up to 256 * 8 * kMost numbers that start on eights.
+// (2,048 rows of 2,048, float
+// and bfloat16, 34 MB: 23.6 us number by number, bound by its loads in flight; 10.8 in eights.)
+template <typename T, int kMost>
+__global__ void __launch_bounds__(256)
+group_norm_gate_vec8_kernel(const float* __restrict__ raw, int raw_stride, const float* __restrict__ gain, const T* __restrict__ gate,
+                            int gate_stride, T* __restrict__ out, int out_stride, int width, float eps, int gate_sigmoid) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    __shared__ float scratch[32];
+    const size_t row = blockIdx.x;
+    float x[kMost][8], g[kMost][8];
+    float ssq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) {
+        const int c = (threadIdx.x + 256 * i) * 8;
+        if (c >= width) break;
+        load8(raw + row * raw_stride + c, x[i]);
+        load8(gate + row * gate_stride + c, g[i]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ssq = fmaf(x[i][j], x[i][j], ssq);
+    }
+    const float inverse = 1.0f / sqrtf(block_sum(ssq, scratch) / (float)width + eps);
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) {
+        const int c = (threadIdx.x + 256 * i) * 8;
+        if (c >= width) break;
+        float scale[8];
+        load8(gain + c, scale);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float s = 1.0f / (1.0f + expf(-g[i][j]));
+            x[i][j] = x[i][j] * inverse * scale[j] * (gate_sigmoid ? s : g[i][j] * s);
+        }
+        store8(out + row * out_stride + c, x[i]);
+    }
+}
+
+template <typename T>
+int launch_group_norm_gate(const float* raw, int raw_stride, const float* gain, const void* gate, int gate_stride, void* out, int out_stride,
+                           int rows, int width, float eps, int gate_sigmoid, cudaStream_t stream) {
+    const uintptr_t piece = 8 * sizeof(T) < 16 ? 8 * sizeof(T) : 16;  // (a float's eights are two loads of 16 bytes)
+    const bool eights = width % 8 == 0 && raw_stride % 4 == 0 && ((size_t)gate_stride * sizeof(T)) % piece == 0 && ((size_t)out_stride * sizeof(T)) % piece == 0 &&
+                        !(((uintptr_t)raw | (uintptr_t)gain) & 15) && !(((uintptr_t)gate | (uintptr_t)out) % piece);
+#define MB_NORM(KERNEL)                                                                                                                     \
+    MB_LAUNCH("group_norm_gate", KERNEL, dim3(rows), dim3(256), 0, stream, true, raw, raw_stride, gain, (const T*)gate, gate_stride, (T*)out, \
+              out_stride, width, eps, gate_sigmoid)
+    if (eights && width <= 256 * 8) MB_NORM((group_norm_gate_vec8_kernel<T, 1>));
+    else if (eights && width <= 256 * 8 * 4) MB_NORM((group_norm_gate_vec8_kernel<T, 4>));
+    else MB_NORM((group_norm_gate_kernel<T>));
+#undef MB_NORM
+    return 0;
+}
+
 }  // namespace mb
 
 using namespace mb;
@@ -353,15 +407,9 @@ using namespace mb;
 MB_EXPORT int mb_group_norm_gate(const float* raw, int raw_stride, const float* gain, const void* gate, int gate_stride, void* out,
                                  int out_stride, int dtype, int rows, int width, float eps, int gate_sigmoid, cudaStream_t stream) {
     if (rows <= 0 || width <= 0) return 0;
-    if (dtype == MB_F32)
-        MB_LAUNCH("group_norm_gate", group_norm_gate_kernel<float>, dim3(rows), dim3(256), 0, stream, true, raw, raw_stride, gain,
-                  (const float*)gate, gate_stride, (float*)out, out_stride, width, eps, gate_sigmoid);
-    else if (dtype == MB_BF16)
-        MB_LAUNCH("group_norm_gate", group_norm_gate_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, true, raw, raw_stride, gain,
-                  (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)out, out_stride, width, eps, gate_sigmoid);
-    else
-        return fail("group_norm_gate: unknown dtype code %d", dtype);
-    return 0;
+    if (dtype == MB_F32) return launch_group_norm_gate<float>(raw, raw_stride, gain, gate, gate_stride, out, out_stride, rows, width, eps, gate_sigmoid, stream);
+    if (dtype == MB_BF16) return launch_group_norm_gate<__nv_bfloat16>(raw, raw_stride, gain, gate, gate_stride, out, out_stride, rows, width, eps, gate_sigmoid, stream);
+    return fail("group_norm_gate: unknown dtype code %d", dtype);
 }
 
 // q, k: [tokens, >= heads * head_dim]; v, g: [tokens, >= heads * value_dim]; all four column slices of one tensor

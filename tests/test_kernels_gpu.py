@@ -973,6 +973,28 @@ def test_retention_chunks(cuda_device, vdim, lengths, whole):
         close(chunk_out, out, torch.bfloat16)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [8, 2040, 2048, 2056, 8192, 8200])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_group_norm_gate_in_eights(cuda_device, dtype, width, shift):
+    """Rows at the edges of the form in eights and off its alignment, against 64 bits."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(width)
+    raw, gain = torch.randn(3, width + 8, generator=g)[:, shift:shift + width], 1 + 0.1 * torch.randn(width, generator=g)
+    gate = torch.randn(3, width + 8, generator=g).to(dtype)[:, shift:shift + width]
+    for name in ("sigmoid", "silu"):
+        rows = torch.full((3, width + 8), 7.0, dtype=dtype, device=cuda_device)
+        moved = [torch.empty(3, width + 8, dtype=t.dtype, device=cuda_device)[:, shift:shift + width] for t in (raw, gate)]
+        for to, t in zip(moved, (raw, gate)):
+            to.copy_(t)
+        ops.group_norm_gate(moved[0], gain.cuda(), moved[1], rows[:, shift:shift + width], 1e-5, name)
+        x, z = raw.double(), gate.double()
+        want = x / (x.pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * gain.double() * torch.sigmoid(z) * (z if name == "silu" else 1)
+        close(rows[:, shift:shift + width].float(), want.float(), dtype)
+        assert bool((rows[:, :shift] == 7).all()) and bool((rows[:, shift + width:] == 7).all())
+
+
 @pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 64)])
 @pytest.mark.parametrize("cap,sink,turned", [(5.0, True, True), (0.0, True, False), (30.0, False, True)])
 def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
