@@ -227,6 +227,63 @@ __global__ void rotate_norm_store_pairs_kernel(T* __restrict__ q, int q_stride, 
     }
 }
 
+// The same in eights for many tokens: a thread a piece of eight numbers, a head's pieces in neighbouring lanes (head_dim / 8 is a power
+// of two up to 32), the values' pieces behind the heads'.  Every row, head and table row starts on its pieces' boundary, and the
+// rotations end on one.  grid (tokens); block: the pieces rounded up to whole warps, at most 1,024 (which then take several each).
+// (2,048 tokens, 16 and 4 heads of 64, values of 128: 27 us as pairs, a warp a head, bound by the chains of its loads; 10.7 in eights.)
+__global__ void __launch_bounds__(1024)
+rotate_norm_store_vec8_kernel(__nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k, int k_stride,
+                              const __nv_bfloat16* __restrict__ v, int v_stride, const int* __restrict__ positions, float eps, Rotation rotation,
+                              __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool, const int* __restrict__ slot_mapping, int heads,
+                              int kv_heads, int head_dim, int value_dim, int page_size) {
+    grid_launch_dependents();
+    const int token = blockIdx.x;
+    const int pos = positions[token], slot = slot_mapping[token];  // (written before the step began)
+    grid_dependency_wait();
+    const size_t page = slot >= 0 ? slot / page_size : 0, offset = slot >= 0 ? slot % page_size : 0;
+    const int per_head = head_dim / 8, head_pieces = (heads + kv_heads) * per_head, pieces = head_pieces + kv_heads * (value_dim / 8);
+    auto turn = [&](float (&x)[8], const float* cos, const float* sin, int dim, int first) {
+        const size_t at = (size_t)pos * (dim / 2) + first / 2;
+        const float4 c4 = *reinterpret_cast<const float4*>(cos + at), s4 = *reinterpret_cast<const float4*>(sin + at);
+        const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float a = x[2 * i], b = x[2 * i + 1];
+            x[2 * i] = a * c[i] - b * s[i];
+            x[2 * i + 1] = b * c[i] + a * s[i];
+        }
+    };
+    for (int base = 0; base < pieces; base += blockDim.x) {  // (whole warps stay: the heads' sums are shuffles)
+        const int piece = base + threadIdx.x;
+        const bool of_head = piece < head_pieces;
+        const int head = of_head ? piece / per_head : 0, first = of_head ? piece % per_head * 8 : 0;
+        float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (of_head) {
+            load8(head < heads ? q + (size_t)token * q_stride + (size_t)head * head_dim + first : k + (size_t)token * k_stride + (size_t)(head - heads) * head_dim + first, x);
+            if (first < rotation.dim) turn(x, rotation.cos, rotation.sin, rotation.dim, first);
+        }
+        float factor = 1.0f;
+        if (rotation.unit) {
+            float ssq = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ssq = fmaf(x[i], x[i], ssq);
+            for (int o = 1; o < per_head; o <<= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+            factor = 1.0f / sqrtf(ssq / (float)head_dim + eps);
+        }
+        if (of_head) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] *= factor;
+            if (head < heads) store8(q + (size_t)token * q_stride + (size_t)head * head_dim + first, x);
+            else if (slot >= 0) store8(k_pool + ((page * kv_heads + head - heads) * page_size + offset) * head_dim + first, x);
+        } else if (piece < pieces && slot >= 0) {
+            const int value = (piece - head_pieces) * 8, value_head = value / value_dim, value_first = value % value_dim;
+            load8(v + (size_t)token * v_stride + value, x);
+            if (value_first < rotation.value_dim_rotated) turn(x, rotation.value_cos, rotation.value_sin, rotation.value_dim_rotated, value_first);
+            store8(v_pool + ((page * kv_heads + value_head) * page_size + offset) * value_dim + value_first, x);
+        }
+    }
+}
+
 template <typename T>
 __global__ void norm_store_kernel(T* __restrict__ q, int q_stride, const T* __restrict__ k, int k_stride,
                                   const T* __restrict__ v, int v_stride, const int* __restrict__ positions,
@@ -1294,6 +1351,18 @@ int launch_rotate_norm_store(void* q, int q_stride, const void* k, int k_stride,
                              int kv_heads, int head_dim, int value_dim, int page_size, cudaStream_t stream) {
     const int warps = heads + kv_heads < 4 ? 4 : (heads + kv_heads > 16 ? 16 : heads + kv_heads);
     const bool turns = rotation.dim > 0 || rotation.value_dim_rotated > 0;
+    const int per_head = head_dim / 8;
+    if (sizeof(T) == 2 && (rotation.interleaved || !turns) && head_dim % 8 == 0 && per_head <= 32 && (per_head & (per_head - 1)) == 0 && value_dim % 8 == 0 &&
+        q_stride % 8 == 0 && k_stride % 8 == 0 && v_stride % 8 == 0 && rotation.dim % 8 == 0 && rotation.value_dim_rotated % 8 == 0 &&
+        !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)rotation.cos | (uintptr_t)rotation.sin |
+           (uintptr_t)rotation.value_cos | (uintptr_t)rotation.value_sin) & 15)) {
+        const int pieces = (heads + kv_heads) * per_head + kv_heads * (value_dim / 8), threads = (pieces + 31) / 32 * 32;
+        using bf16 = __nv_bfloat16;
+        MB_LAUNCH("rotate_norm_store", rotate_norm_store_vec8_kernel, dim3(tokens), dim3(threads < 1024 ? threads : 1024), 0, stream, true, (bf16*)q,
+                  q_stride, (const bf16*)k, k_stride, (const bf16*)v, v_stride, positions, eps, rotation, (bf16*)k_pool, (bf16*)v_pool, slot_mapping,
+                  heads, kv_heads, head_dim, value_dim, page_size);
+        return 0;
+    }
     const uintptr_t two = 2 * sizeof(T);
     if ((rotation.interleaved || !turns) && head_dim % 2 == 0 && value_dim % 2 == 0 && q_stride % 2 == 0 && k_stride % 2 == 0 &&
         v_stride % 2 == 0 && !((uintptr_t)q % two) && !((uintptr_t)k % two) && !((uintptr_t)v % two) && !((uintptr_t)k_pool % two) &&

@@ -995,6 +995,38 @@ def test_group_norm_gate_in_eights(cuda_device, dtype, width, shift):
         assert bool((rows[:, :shift] == 7).all()) and bool((rows[:, shift + width:] == 7).all())
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,rotary,value_rotary", [(16, 4, 64, 128, 64, 128), (3, 1, 8, 8, 8, 0), (5, 5, 256, 24, 0, 8),
+                                                                         (32, 8, 128, 128, 40, 16)])
+@pytest.mark.parametrize("unit", [True, False])
+def test_rotate_norm_store_in_eights(cuda_device, heads, kv_heads, dim, vdim, rotary, value_rotary, unit):
+    """The form in eights against the general one, which rows that start off its alignment take: rotations that end within a head, a
+    token without a slot, more pieces than a block has threads."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(dim + vdim)
+    tokens, page, widths = 5, 64, (heads * dim, kv_heads * dim, kv_heads * vdim)
+    rows = [torch.randn(tokens, w, generator=g).bfloat16().cuda() for w in widths]
+    positions = torch.tensor([0, 1, 77, 150, 2], dtype=torch.int32).cuda()
+    slots = torch.tensor([64, 130, -1, 191, 65], dtype=torch.int32).cuda()
+    angle, value_angle = torch.rand(200, max(rotary, 2) // 2, generator=g) * 6, torch.rand(200, max(value_rotary, 2) // 2, generator=g) * 6
+    tables = [t.cuda() for a in (angle, value_angle) for t in (a.cos(), a.sin())]
+    found = []
+    for shift in (0, 2):  # (pairs stay aligned, eights do not)
+        wide = [torch.zeros(tokens, w + 8, dtype=torch.bfloat16, device=cuda_device) for w in widths]
+        q, k, v = (t[:, shift:shift + w] for t, w in zip(wide, widths))
+        for to, t in zip((q, k, v), rows):
+            to.copy_(t)
+        pools = [torch.zeros(3, kv_heads, page, d, dtype=torch.bfloat16, device=cuda_device) for d in (dim, vdim)]
+        ops.rotate_norm_store(q, k, v, positions, tables[0], tables[1], rotary, True, unit, 1e-5, tables[2], tables[3], value_rotary, *pools, slots,
+                              heads, kv_heads, dim, vdim)
+        found.append([q.float()] + [pool.float() for pool in pools])
+        assert all(bool((t[:, :shift] == 0).all()) and bool((t[:, shift + w:] == 0).all()) for t, w in zip(wide, widths))
+    # the same floats but for the order of a head's squares: a rounding to bfloat16 may fall to the other side
+    for here, there in zip(*found):
+        assert torch.allclose(here, there, rtol=2.0 ** -7, atol=0)
+        assert float((here != there).float().mean()) < 0.01
+
+
 @pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 64)])
 @pytest.mark.parametrize("cap,sink,turned", [(5.0, True, True), (0.0, True, False), (30.0, False, True)])
 def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
