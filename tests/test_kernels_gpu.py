@@ -1027,6 +1027,25 @@ def test_rotate_norm_store_in_eights(cuda_device, heads, kv_heads, dim, vdim, ro
         assert float((here != there).float().mean()) < 0.01
 
 
+@pytest.mark.parametrize("batch", [1, 3, 8])
+@pytest.mark.parametrize("n,k", [(2048, 4104), (37, 5000), (16, 8192), (2360, 8192)])
+def test_skinny_gemm_streams_activations(cuda_device, batch, n, k):
+    """One row tile a block and a long K: the shortest one, one that ends within a step, rows that end within a tile, and 148 tiles."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(n + k)
+    w, x = (torch.randn(n, k, generator=g) * 0.05).bfloat16(), torch.randn(batch, k, generator=g).bfloat16()
+    exact = x.double() @ w.double().t()
+    scale, wd = float(exact.abs().max()), w.cuda()
+    xd = torch.full((batch, k + 8), 9.0, dtype=torch.bfloat16, device=cuda_device)[:, :k]
+    xd.copy_(x)
+    # k float additions of products that are exact, the eight warps' sums among them
+    assert float((ops.skinny_gemm(wd, ops.EPI_F32, x=xd).double().cpu() - exact).abs().max()) < 2.0 ** -23 * scale * math.sqrt(k) * 4
+    out = torch.randn(batch, n, generator=g)
+    got = ops.skinny_gemm(wd, ops.EPI_RESIDUAL, x=xd, out=out.cuda())
+    assert float((got.double().cpu() - out.double() - exact).abs().max()) < 2.0 ** -23 * (scale + 4) * math.sqrt(k) * 4
+
+
 @pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 64)])
 @pytest.mark.parametrize("cap,sink,turned", [(5.0, True, True), (0.0, True, False), (30.0, False, True)])
 def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
