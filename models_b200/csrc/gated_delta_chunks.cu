@@ -1,4 +1,4 @@
-// The gated delta rule for long steps: chunks of 64 tokens, float arithmetic throughout.  What is computed is what
+// The gated delta rule for long steps: chunks of 64 tokens on the tensor cores.  What is computed is what
 // gated_delta.cu's walk computes token by token (see there):
 //   S <- g_t S;   u_t = beta_t (v_t - S^T k_t);   S <- S + k_t u_t^T;   o_t = S^T q_t
 // Within a chunk that starts from the state S_0, with G_i the product of the chunk's g up to token i:
@@ -8,17 +8,22 @@
 // The first line is a triangular system in the chunk's u (the UT form of products of Householder-like factors: Bischof and
 // Van Loan 1987; for delta rules Yang et al. 2024), linear in S_0: u = x - y S_0, where x and y solve it for the right sides
 // beta v and beta G k.  Three kernels:
-//   1. delta_chunks_solve: per (chunk, head) the system's matrix, x [64][V], y [64][64] and the keys weighted by G_end / G_j,
-//      by forward substitution, a thread for every two columns of the right sides;
-//   2. delta_chunks_carry: per (head, 16 columns of S) from chunk to chunk: u = x - y S_0 (over x), S_0 left for kernel 3,
-//      S_end; the only serial part, two 64 x 64 x 16 products a chunk;
+//   1. delta_chunks_solve: per (chunk, head) the system's matrix, x [64][V], y [64][64] and the keys weighted by G_end / G_j; the
+//      system is solved 16 rows at a time, with the inverses of its 16 x 16 diagonal blocks, a warp for 32 of the right sides'
+//      columns;
+//   2. delta_chunks_carry: per (head, 16 columns of S) from chunk to chunk: u = x - y S_0 (over x), S_0 left for kernel 3, S_end; the
+//      only serial part, two 64 x 64 x 16 products a chunk;
 //   3. delta_chunks_results: per (chunk, head) o, its norm, gain and gate.
 // The ratios G_i / G_j come from differences of sums of log g that are kept in 64 bits, so that a late token's ratios lose
-// nothing to the size of the sums.
+// nothing to the size of the sums.  What lies between products is float, and products take it whole (split_products.cuh).
+// Against 64 bits, over steps of 64 to 2,048 tokens: the state is off by 1.2e-7 to 1.3e-7 of itself (the walk: 1.9e-7 to 3.3e-7), the
+// results by 1.4e-7 (2e-7).
 // One sequence of 2,048 tokens, 16 heads of 64 x 128: the walk's chain of 2,048 tokens is bound by its latency (618 us, and 30 for
-// the kernels around it); here 56, 102 and 68 us, bound by what the operands take from shared memory (the carrying kernel: by the
-// latency of two warps).
+// the kernels around it); the three kernels took 58, 105 and 71 us as float multiply-adds, bound by what the operands take from
+// shared memory and by the latency of few warps; 54, 67 and 60 here (a layer: 310 us, and 247), where the carrying kernel is bound by
+// its chunk's two products one after the other, the others by six products for one and the splitting of what they read.
 #include "common.cuh"
+#include "split_products.cuh"
 
 MB_DEFINE_LAST_ERROR()
 
@@ -27,7 +32,11 @@ namespace mb {
 constexpr int kChunk = 64;    // tokens of a chunk
 constexpr int kDim = 64;      // a key head's coordinates
 constexpr int kColumns = 16;  // columns of S that a block of the carrying kernel owns
-constexpr int kPad = 4;       // floats behind the rows of a transposed tile
+constexpr int kCarryThreads = 128, kResultThreads = 256;
+constexpr int kRow = kDim + 8;            // bfloat16 numbers of a padded row of 64: ldmatrix without bank conflicts
+constexpr int kPlane = kChunk * kRow;
+constexpr int kNarrowRow = kColumns + 8;  // and of rows of 16
+constexpr int kNarrowPlane = kChunk * kNarrowRow;
 
 struct DeltaChunkArgs {
     const float* conv;  // convolved rows: q at column q_at (kv_heads heads of kDim), k at k_at, v at v_at (heads heads of V)
@@ -42,104 +51,115 @@ struct DeltaChunkArgs {
     void* out;
     int out_stride;
     int heads, kv_heads;
-    // scratch, by (place of the chunk, head): u [64][V], y transposed [64 d][64 i], weighted keys [64 i][64 d], S_0 [64 d][V], sums of log g
-    float *u, *y, *keys, *starts;
+    // scratch by (place of the chunk, head): x, then u [64][V]; S_0 [64][V]; in three parts y [64 i][64 d] and weighted keys [64 i][64 d];
+    // sums of log g [64]
+    float *u, *starts;
+    bf16 *y, *keys;
     double* logs;
 };
 
 __device__ __forceinline__ float sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float softplus(float v) { return fmaxf(v, 0.0f) + log1pf(expf(-fabsf(v))); }
 
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
-    uint64_t d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
+__device__ __forceinline__ void copy16_async(bf16* dst, const bf16* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ uint64_t twice(float v) { return pair_of(v, v); }
-__device__ __forceinline__ float2 floats_of(uint64_t v) { return make_float2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32))); }
-__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {  // two float FMAs
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ void copy16_async(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copies_sent() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void copies_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
+__device__ __forceinline__ float2 load_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 load_pair(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
+__device__ __forceinline__ void store_pair(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void store_pair(bf16* p, float a, float b) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b); }
 
 // Where a chunk's scratch lies: every sequence's chunks one after another, a sequence's first place being floor(first / 64) + seq
 // (a sequence of n tokens has ceil(n / 64) chunks, and floor(f / 64) + ceil(n / 64) <= floor((f + n) / 64) + 1).
 __device__ __forceinline__ size_t place_of(int first, int seq, int chunk) { return (size_t)(first / kChunk) + seq + chunk; }
 
-// The unit rows of a chunk's 64 tokens, times `factor`, transposed into tile [kDim][kChunk + kPad]; 128 threads, thread (row, half)
-// takes 32 coordinates of a row and leaves them in `own` too.  Rows beyond `count` are zeros.  parts: shared [2][kChunk].
-__device__ __forceinline__ void unit_rows(const float* rows, int stride, int count, float unit_eps, float factor, float* tile, float* parts,
-                                          float (&own)[32]) {
-    const int row = threadIdx.x % kChunk, half = threadIdx.x / kChunk;
-    float squares = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-        const float4 x = row < count ? *reinterpret_cast<const float4*>(rows + (size_t)row * stride + half * 32 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        own[i] = x.x, own[i + 1] = x.y, own[i + 2] = x.z, own[i + 3] = x.w;
-        squares = fmaf(x.x, x.x, squares), squares = fmaf(x.y, x.y, squares), squares = fmaf(x.z, x.z, squares), squares = fmaf(x.w, x.w, squares);
-    }
-    parts[half * kChunk + row] = squares;
-    __syncthreads();
-    const float scale = factor / sqrtf(parts[row] + parts[kChunk + row] + unit_eps);
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        own[i] *= scale;
-        tile[(half * 32 + i) * (kChunk + kPad) + row] = own[i];
-    }
+// Two floats, and four, as their parts.
+__device__ __forceinline__ void split_two(float a, float b, bf16* at, int plane) {
+    uint32_t hi, mid, lo;
+    split_pair(a, b, hi, mid, lo);
+    *reinterpret_cast<uint32_t*>(at) = hi;
+    *reinterpret_cast<uint32_t*>(at + plane) = mid;
+    *reinterpret_cast<uint32_t*>(at + 2 * plane) = lo;
+}
+__device__ __forceinline__ void split_four(float4 v, bf16* at, int plane) {
+    uint2 hi, mid, lo;
+    split_pair(v.x, v.y, hi.x, mid.x, lo.x);
+    split_pair(v.z, v.w, hi.y, mid.y, lo.y);
+    *reinterpret_cast<uint2*>(at) = hi;
+    *reinterpret_cast<uint2*>(at + plane) = mid;
+    *reinterpret_cast<uint2*>(at + 2 * plane) = lo;
 }
 
-// acc[8 rows][4 columns] += a^T b over 64 steps: a [64][kChunk + kPad] at rows row0 .. +3 and row0 + 32 .. +35, b likewise at col0 .. +3.
-__device__ __forceinline__ void tile_8x4(const float* a, const float* b, int row0, int col0, uint64_t (&acc)[8][2]) {
-#pragma unroll 8
-    for (int d = 0; d < 64; ++d) {
-        const float4 lo = *reinterpret_cast<const float4*>(a + d * (kChunk + kPad) + row0), hi = *reinterpret_cast<const float4*>(a + d * (kChunk + kPad) + row0 + 32);
-        const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(b + d * (kChunk + kPad) + col0);
-        const float rows[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+// The unit rows of a chunk's 64 tokens, times `factor`, into planes of padded rows; sixteen lanes a row, a thread's four coordinates of
+// every row that it takes are left in `x`.  Rows beyond `count` are zeros.  unit (or null): the rows' factors.
+template <int kThreads>
+struct UnitRows {
+    static constexpr int at_once = kThreads / 16, passes = (kChunk + at_once - 1) / at_once;
+    float4 x[passes];
+    __device__ __forceinline__ UnitRows(const float* rows, int stride, int count, float unit_eps, float factor, bf16* planes, float* unit) {
+        const int d = (threadIdx.x % 16) * 4;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const uint64_t x = twice(rows[r]);
-            acc[r][0] = fma_pair(x, c.x, acc[r][0]);
-            acc[r][1] = fma_pair(x, c.y, acc[r][1]);
+        for (int i = 0; i < passes; ++i) {
+            const int row = threadIdx.x / 16 + at_once * i;
+            x[i] = row < count ? *reinterpret_cast<const float4*>(rows + (size_t)row * stride + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int i = 0; i < passes; ++i) {
+            const int row = threadIdx.x / 16 + at_once * i;
+            float squares = fmaf(x[i].x, x[i].x, fmaf(x[i].y, x[i].y, fmaf(x[i].z, x[i].z, x[i].w * x[i].w)));
+#pragma unroll
+            for (int offset = 1; offset < 16; offset <<= 1) squares += __shfl_xor_sync(0xffffffffu, squares, offset);
+            const float scale = factor / sqrtf(squares + unit_eps);
+            x[i] = make_float4(scale * x[i].x, scale * x[i].y, scale * x[i].z, scale * x[i].w);
+            if (row >= kChunk) continue;
+            split_four(x[i], planes + row * kRow + d, kPlane);
+            if (unit != nullptr && d == 0) unit[row] = scale;
         }
     }
+};
+
+// Where a lane's ldmatrix addresses start within a tile of rows of `row` numbers, in bytes: of a left operand [row][k] or a right one
+// [k][column], and of a right one [column][k] or a left one [k][row].
+__device__ __forceinline__ uint32_t lanes_by_row(int row) { return (((threadIdx.x & 31) & 15) * row + ((threadIdx.x & 31) >> 4) * 8) * 2; }
+__device__ __forceinline__ uint32_t lanes_by_column(int row) {
+    const int lane = threadIdx.x & 31;
+    return (((lane >> 4) * 8 + (lane & 7)) * row + ((lane >> 3) & 1) * 8) * 2;
 }
 
-// grid (heads, most chunks of a sequence, sequences); block 128.
-// shared: keys transposed [64][68], matrix transposed [j][i] [64][64], right sides [64][V + 64], sums of log g, beta, parts.
+// grid (heads, most chunks of a sequence, sequences); block threads: a warp for 32 columns of the right sides.
 template <int V>
 struct SolvePlan {
-    static constexpr int kRight = V + kDim;
-    static constexpr int keys = 0, matrix = keys + kDim * (kChunk + kPad), right = matrix + kChunk * kChunk, logs = right + kChunk * kRight,
-                         beta = logs + 2 * kChunk, parts = beta + kChunk, total = parts + 2 * kChunk;
+    static constexpr int right = V + kDim, threads = right, right_row = right + 8, solved_rows = 48, right_plane = solved_rows * right_row;
+    static constexpr int inverse_row = 24, inverse_plane = kChunk * inverse_row, diagonal_row = 17;
+    // bfloat16 numbers: the matrix, the inverses of its diagonal blocks; the keys, whose place the solved rows take; then floats: the
+    // diagonal blocks, beta, the keys' factors, (64 bits) logs
+    static constexpr int matrix = 0, inverse = matrix + kParts * kPlane, keys = inverse + kParts * inverse_plane,
+                         floats = keys + kParts * (right_plane > kPlane ? right_plane : kPlane);
+    static constexpr int bytes = floats * 2 + (kChunk * diagonal_row + 2 * kChunk) * 4 + kChunk * 8;
+    static_assert(floats * 2 % 16 == 0 && (kChunk * diagonal_row + 2 * kChunk) % 2 == 0, "the logs lie on eight bytes");
 };
 
 template <typename T, int V>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(SolvePlan<V>::threads, 2)
 delta_chunks_solve_kernel(const DeltaChunkArgs args) {
     using Plan = SolvePlan<V>;
     grid_launch_dependents();
     grid_dependency_wait();
-    extern __shared__ __align__(16) float shared[];
-    float* keys = shared + Plan::keys;
-    float* matrix = shared + Plan::matrix;
-    float* right = shared + Plan::right;
-    double* logs = reinterpret_cast<double*>(shared + Plan::logs);
-    float* beta = shared + Plan::beta;
+    extern __shared__ __align__(16) unsigned char shared[];
+    bf16* planes = reinterpret_cast<bf16*>(shared);
+    bf16 *keys = planes + Plan::keys, *matrix = planes + Plan::matrix, *inverse = planes + Plan::inverse, *solved = keys;
+    float* diagonal = reinterpret_cast<float*>(planes + Plan::floats);
+    float* beta = diagonal + kChunk * Plan::diagonal_row;
+    float* unit = beta + kChunk;
+    double* logs = reinterpret_cast<double*>(unit + kChunk);
     const int head = blockIdx.x, chunk = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
     const int first = args.cu_q[seq], count = min(kChunk, args.cu_q[seq + 1] - first - chunk * kChunk);
     if (count <= 0) return;
     const size_t token0 = (size_t)first + chunk * kChunk;
     const size_t at = place_of(first, seq, chunk) * args.heads + head;
     const float* rows = args.conv + token0 * args.conv_stride;
+    const float* key_rows = rows + args.k_at + head / (args.heads / args.kv_heads) * kDim;
+    const float* value_rows = rows + args.v_at + (size_t)head * V;
     // gates: a token beyond the chunk's last neither forgets nor writes
     double log_g = 0.0;
     if (tid < kChunk) {
@@ -159,344 +179,357 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
         }
         logs[tid] = log_g;
     }
-    float own[32];
-    unit_rows(rows + args.k_at + head / (args.heads / args.kv_heads) * kDim, args.conv_stride, count, args.unit_eps, 1.0f, keys, shared + Plan::parts, own);
-    if (tid >= 32 && tid < kChunk) logs[tid] = log_g + logs[31];  // (the barrier inside unit_rows lies between)
-    // the values' right sides: beta v
-    for (int i = tid; i < kChunk * (V / 4); i += 128) {
-        const int row = i / (V / 4), c = i % (V / 4) * 4;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (row < count) v = *reinterpret_cast<const float4*>(rows + (size_t)row * args.conv_stride + args.v_at + (size_t)head * V + c);
-        const float b = beta[row];
-        *reinterpret_cast<float4*>(right + row * Plan::kRight + c) = make_float4(b * v.x, b * v.y, b * v.z, b * v.w);
-    }
+    const UnitRows<Plan::threads> k(key_rows, args.conv_stride, count, args.unit_eps, 1.0f, keys, unit);
+    __syncthreads();
+    if (tid >= 32 && tid < kChunk) logs[tid] = log_g + logs[31];
     __syncthreads();
     {
-        // the keys' right sides beta G k, and the keys weighted for the chunk's end
-        const int row = tid % kChunk, half = tid / kChunk;
-        const float to_row = beta[row] * expf((float)logs[row]), to_end = expf((float)(logs[kChunk - 1] - logs[row]));
-        float* weighted = args.keys + at * kChunk * kDim + row * kDim + half * 32;
+        bf16* weighted = args.keys + kParts * at * kChunk * kDim + (tid % 16) * 4;
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-            *reinterpret_cast<float4*>(right + row * Plan::kRight + V + half * 32 + i) =
-                make_float4(to_row * own[i], to_row * own[i + 1], to_row * own[i + 2], to_row * own[i + 3]);
-            *reinterpret_cast<float4*>(weighted + i) = make_float4(to_end * own[i], to_end * own[i + 1], to_end * own[i + 2], to_end * own[i + 3]);
+        for (int i = 0; i < k.passes; ++i) {
+            const int row = tid / 16 + k.at_once * i;
+            if (row >= kChunk) break;
+            const float to_end = expf((float)(logs[kChunk - 1] - logs[row]));
+            split_four(make_float4(to_end * k.x[i].x, to_end * k.x[i].y, to_end * k.x[i].z, to_end * k.x[i].w), weighted + row * kDim, kChunk * kDim);
         }
         if (tid < kChunk) args.logs[at * kChunk + tid] = logs[tid];
     }
-    {
-        // matrix[j][i] = beta_i G_i / G_j (k_i . k_j) for j < i
-        const int row0 = (tid % 8) * 4, col0 = (tid / 8) * 4;  // rows j, columns i
-        uint64_t acc[8][2];
+    const int warp = tid >> 5, group = (tid & 31) >> 2, pair = 2 * (tid & 3);
+    if (warp < kChunk / 16) {
+        // matrix[i][j] = beta_i G_i / G_j (k_i . k_j) for j < i: rows 16 * warp .. + 15, the columns up to them
+        float acc[kChunk / 8][4] = {};
+        const uint32_t left = smem_u32(keys) + 16 * warp * kRow * 2 + lanes_by_row(kRow), right = smem_u32(keys) + lanes_by_column(kRow);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0;
-        tile_8x4(keys, keys, row0, col0, acc);
+        for (int d = 0; d < kDim; d += 16) {
+            Parts a, b;
+            load_parts(a, left + d * 2, kPlane);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int j = row0 + (r / 4) * 32 + r % 4;
-            const float2 lo = floats_of(acc[r][0]), hi = floats_of(acc[r][1]);
-            float v[4] = {lo.x, lo.y, hi.x, hi.y};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int i = col0 + c;
-                v[c] = j < i ? v[c] * beta[i] * expf((float)(logs[i] - logs[j])) : 0.0f;
+            for (int n = 0; n < kChunk / 8; n += 2) {
+                if (n > 2 * warp) break;
+                load_parts(b, right + (8 * n * kRow + d) * 2, kPlane);
+                split_products(acc[n], acc[n + 1], a, b);
             }
-            *reinterpret_cast<float4*>(matrix + j * kChunk + col0) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+#pragma unroll
+        for (int n = 0; n < kChunk / 8; ++n) {
+            if (n > 2 * warp + 1) break;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int i = 16 * warp + group + 8 * half, j = 8 * n + pair;
+                const float b = beta[i];
+                const float lo = j < i ? acc[n][2 * half] * b * expf((float)(logs[i] - logs[j])) : 0.0f;
+                const float hi = j + 1 < i ? acc[n][2 * half + 1] * b * expf((float)(logs[i] - logs[j + 1])) : 0.0f;
+                split_two(lo, hi, matrix + i * kRow + j, kPlane);
+                if (n >= 2 * warp) diagonal[i * Plan::diagonal_row + j % 16] = lo, diagonal[i * Plan::diagonal_row + j % 16 + 1] = hi;
+            }
+        }
+    }
+    // a warp's columns of the right sides, beta v and beta G k, as products leave their results; all four blocks of 16 rows
+    constexpr int kTiles = 4;  // tiles of eight columns
+    const int column0 = warp * kTiles * 8;
+    const bool of_values = column0 < V;
+    const float* source = of_values ? value_rows + column0 + pair : key_rows + column0 - V + pair;
+    float right[kChunk / 16][kTiles][4];
+#pragma unroll
+    for (int r = 0; r < kChunk / 8; ++r) {
+        const int row = 8 * r + group;
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n) {
+            float2 x = make_float2(0.0f, 0.0f);
+            if (row < count) x = load_pair(source + (size_t)row * args.conv_stride + 8 * n);
+            const float scale = of_values ? beta[row] : beta[row] * expf((float)logs[row]) * unit[row];
+            right[r / 2][n][2 * (r % 2)] = scale * x.x, right[r / 2][n][2 * (r % 2) + 1] = scale * x.y;
         }
     }
     __syncthreads();
-    // forward substitution, 16 rows at a time; a thread's two columns are its own from here on
-    for (int column = 2 * tid; column < Plan::kRight; column += 256) {
-#pragma unroll 1
-        for (int row0 = 0; row0 < kChunk; row0 += 16) {
-            uint64_t acc[16];
+    if (tid < kChunk) {
+        // a column of the inverse of a diagonal block I + M: z_r = (r == c) - sum_(s < r) M[r][s] z_s
+        const int block = tid / 16, c = tid % 16;
+        float z[16];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) acc[r] = *reinterpret_cast<const uint64_t*>(right + (row0 + r) * Plan::kRight + column);
-#pragma unroll 4
-            for (int j = 0; j < row0; ++j) {
-                const float2 x = *reinterpret_cast<const float2*>(right + j * Plan::kRight + column);
-                const uint64_t minus = pair_of(-x.x, -x.y);
+        for (int r = 0; r < 16; ++r) {
+            float sum = r == c ? 1.0f : 0.0f;
 #pragma unroll
-                for (int r = 0; r < 16; r += 4) {
-                    const float4 m = *reinterpret_cast<const float4*>(matrix + j * kChunk + row0 + r);
-                    acc[r] = fma_pair(twice(m.x), minus, acc[r]);
-                    acc[r + 1] = fma_pair(twice(m.y), minus, acc[r + 1]);
-                    acc[r + 2] = fma_pair(twice(m.z), minus, acc[r + 2]);
-                    acc[r + 3] = fma_pair(twice(m.w), minus, acc[r + 3]);
-                }
+            for (int s = 0; s < r; ++s) sum = fmaf(-diagonal[(16 * block + r) * Plan::diagonal_row + s], z[s], sum);
+            z[r] = sum;
+            uint32_t hi, mid, lo;
+            split_pair(sum, 0.0f, hi, mid, lo);
+            unsigned short* to = reinterpret_cast<unsigned short*>(inverse + (16 * block + r) * Plan::inverse_row + c);
+            to[0] = (unsigned short)hi, to[Plan::inverse_plane] = (unsigned short)mid, to[2 * Plan::inverse_plane] = (unsigned short)lo;
+        }
+    }
+    __syncthreads();  // (nobody reads the keys any more either)
+    // a warp's columns are its own from here on; a block of 16 rows: z = right - sum over the blocks before of M x, x = inverse . z.  The
+    // last block's z takes the first one's place, which nothing reads after it.
+    const uint32_t matrix_at = smem_u32(matrix) + lanes_by_row(kRow), inverse_at = smem_u32(inverse) + lanes_by_row(Plan::inverse_row),
+                   solved_at = smem_u32(solved) + column0 * 2 + lanes_by_row(Plan::right_row);
+#pragma unroll
+    for (int block = 0; block < kChunk / 16; ++block) {
+        const int row0 = 16 * block < Plan::solved_rows ? 16 * block : 0;
+        float acc[kTiles][4] = {};
+        auto accumulate = [&](uint32_t left, int left_plane, int k0) {  // acc += left (16 x 16) . rows k0 .. k0 + 15 of the solved columns
+            Parts a, b;
+            load_parts(a, left, left_plane);
+#pragma unroll
+            for (int n = 0; n < kTiles; n += 2) {
+                load_parts_turned(b, solved_at + (k0 * Plan::right_row + 8 * n) * 2, Plan::right_plane);
+                split_products(acc[n], acc[n + 1], a, b);
             }
+        };
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const float2 x = floats_of(acc[j]);
-                const uint64_t minus = pair_of(-x.x, -x.y);
-                *reinterpret_cast<uint64_t*>(right + (row0 + j) * Plan::kRight + column) = acc[j];
+        for (int c = 0; c < block; ++c) accumulate(matrix_at + (16 * block * kRow + 16 * c) * 2, kPlane, 16 * c);
+        __syncwarp();
+        bf16* mine = solved + (row0 + group) * Plan::right_row + column0 + pair;
 #pragma unroll
-                for (int r = j + 1; r < 16; ++r) acc[r] = fma_pair(twice(matrix[(row0 + j) * kChunk + row0 + r]), minus, acc[r]);
+        for (int n = 0; n < kTiles; ++n) {
+            split_two(right[block][n][0] - acc[n][0], right[block][n][1] - acc[n][1], mine + 8 * n, Plan::right_plane);
+            split_two(right[block][n][2] - acc[n][2], right[block][n][3] - acc[n][3], mine + 8 * Plan::right_row + 8 * n, Plan::right_plane);
+            acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+        }
+        __syncwarp();
+        accumulate(inverse_at + 16 * block * Plan::inverse_row * 2, Plan::inverse_plane, row0);
+        __syncwarp();
+        const int row = 16 * block + group;
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n) {
+            if (block + 1 < kChunk / 16) {
+                split_two(acc[n][0], acc[n][1], mine + 8 * n, Plan::right_plane);
+                split_two(acc[n][2], acc[n][3], mine + 8 * Plan::right_row + 8 * n, Plan::right_plane);
             }
-            if (column < V) {
-#pragma unroll
-                for (int r = 0; r < 16; ++r) *reinterpret_cast<uint64_t*>(args.u + (at * kChunk + row0 + r) * V + column) = acc[r];
+            if (of_values) {
+                float* x = args.u + (at * kChunk + row) * V + column0 + 8 * n + pair;
+                store_pair(x, acc[n][0], acc[n][1]);
+                store_pair(x + 8 * V, acc[n][2], acc[n][3]);
             } else {
-                float* y = args.y + at * kDim * kChunk + (size_t)(column - V) * kChunk + row0;  // transposed
-#pragma unroll
-                for (int r = 0; r < 16; r += 4) {
-                    const float2 a = floats_of(acc[r]), b = floats_of(acc[r + 1]), c = floats_of(acc[r + 2]), d = floats_of(acc[r + 3]);
-                    *reinterpret_cast<float4*>(y + r) = make_float4(a.x, b.x, c.x, d.x);
-                    *reinterpret_cast<float4*>(y + kChunk + r) = make_float4(a.y, b.y, c.y, d.y);
-                }
+                bf16* y = args.y + kParts * at * kChunk * kDim + (size_t)row * kDim + column0 - V + 8 * n + pair;
+                split_two(acc[n][0], acc[n][1], y, kChunk * kDim);
+                split_two(acc[n][2], acc[n][3], y + 8 * kDim, kChunk * kDim);
             }
         }
+        __syncwarp();
     }
 }
 
-// grid (V / kColumns, heads, sequences); block 64: thread (four, group) holds S at coordinates 4 * four .. +3 and columns
-// 4 * group .. +3, and the same places of u.  The next chunk's y, keys and x arrive by cp.async while this one's are used.
+// grid (V / kColumns, heads, sequences); block kCarryThreads: a warp has 16 coordinates of S (and 16 tokens of u) at the block's columns,
+// as its products leave them.  The next chunk's y and keys arrive by cp.async, its x in registers, while this one's are used.
+constexpr int kCarryStage = 2 * kParts * kPlane;                                          // y, keys
+constexpr int kCarryBytes = (2 * kCarryStage + 2 * kParts * kNarrowPlane) * 2;            // and S, u
+
 template <int V>
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(kCarryThreads)
 delta_chunks_carry_kernel(const DeltaChunkArgs args) {
     grid_launch_dependents();
     grid_dependency_wait();
-    constexpr int kStage = 2 * kDim * kChunk + kChunk * kColumns;  // y, keys, x
-    extern __shared__ __align__(16) float shared[];
-    float* s_tile = shared + 2 * kStage;           // [64 d][16]
-    float* u_tile = s_tile + kDim * kColumns;      // [64 i][16]
+    extern __shared__ __align__(16) unsigned char shared[];
+    bf16* stages = reinterpret_cast<bf16*>(shared);
+    bf16 *s_planes = stages + 2 * kCarryStage, *u_planes = s_planes + kParts * kNarrowPlane;
     const int column0 = blockIdx.x * kColumns, head = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
     const int first = args.cu_q[seq], tokens = args.cu_q[seq + 1] - first;
     if (tokens <= 0) return;
     const int chunks = (tokens + kChunk - 1) / kChunk;
-    const int four = (tid % 16) * 4, group = (tid / 16) * 4;
+    const int warp = tid >> 5, group = (tid & 31) >> 2, pair = 2 * (tid & 3);
+    const int row = 16 * warp + group;  // and row + 8
     const size_t place0 = place_of(first, seq, 0);
-    float* stored = args.state + (size_t)args.slots[seq] * args.state_stride + (size_t)head * kDim * V + column0 + group;
+    auto item = [&](int chunk) { return (place0 + chunk) * args.heads + head; };
     auto fetch = [&](int chunk) {
-        float* stage = shared + (chunk & 1) * kStage;
-        const size_t at = (place0 + chunk) * args.heads + head;
-        const float *y = args.y + at * kDim * kChunk, *keys = args.keys + at * kChunk * kDim, *x = args.u + at * kChunk * V + column0;
-#pragma unroll 8
-        for (int i = tid; i < kDim * kChunk / 4; i += 64) {
-            copy16_async(stage + 4 * i, y + 4 * i);
-            copy16_async(stage + kDim * kChunk + 4 * i, keys + 4 * i);
-        }
+        bf16* stage = stages + (chunk & 1) * kCarryStage;
+        const bf16 *y = args.y + kParts * item(chunk) * kChunk * kDim, *keys = args.keys + kParts * item(chunk) * kChunk * kDim;
 #pragma unroll
-        for (int i = tid; i < kChunk * kColumns / 4; i += 64)
-            copy16_async(stage + 2 * kDim * kChunk + 4 * i, x + (size_t)(i / (kColumns / 4)) * V + i % (kColumns / 4) * 4);
-        copies_sent();
+        for (int i = tid; i < kParts * kChunk * kDim / 8; i += kCarryThreads) {  // (the planes' rows run on)
+            copy16_async(stage + i / 8 * kRow + i % 8 * 8, y + 8 * i);
+            copy16_async(stage + kParts * kPlane + i / 8 * kRow + i % 8 * 8, keys + 8 * i);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    float2 x[2][2];
+    float log_keep;
+    auto fetch_x = [&](int chunk) {
+        const float* from = args.u + item(chunk) * kChunk * V + column0 + pair;
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            x[n][0] = load_pair(from + (size_t)row * V + 8 * n);
+            x[n][1] = load_pair(from + (size_t)(row + 8) * V + 8 * n);
+        }
+        log_keep = (float)args.logs[item(chunk) * kChunk + kChunk - 1];
     };
     fetch(0);
-    uint64_t s[4][2];
+    fetch_x(0);
+    float* stored = args.state + (size_t)args.slots[seq] * args.state_stride + (size_t)head * kDim * V + column0 + pair;
+    float s[2][4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const float* from = stored + (size_t)(four + r) * V;
-        s[r][0] = pair_of(from[0], from[1]), s[r][1] = pair_of(from[2], from[3]);
-    }
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[n][i] = stored[(size_t)(row + 8 * (i / 2)) * V + 8 * n + i % 2];
+    const uint32_t s_at = smem_u32(s_planes) + lanes_by_row(kNarrowRow), u_at = smem_u32(u_planes) + lanes_by_row(kNarrowRow);
+    const uint32_t y_at = smem_u32(stages) + 16 * warp * kRow * 2 + lanes_by_row(kRow);
+    const uint32_t key_at = smem_u32(stages) + (kParts * kPlane + 16 * warp) * 2 + lanes_by_column(kRow);
     for (int chunk = 0; chunk < chunks; ++chunk) {
-        const size_t at = (place0 + chunk) * args.heads + head;
-        float* start = args.starts + at * kDim * V + column0 + group;
+        float* start = args.starts + item(chunk) * kDim * V + column0 + pair;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const ulonglong2 row = make_ulonglong2(s[r][0], s[r][1]);
-            *reinterpret_cast<ulonglong2*>(s_tile + (four + r) * kColumns + group) = row;
-            *reinterpret_cast<ulonglong2*>(start + (size_t)(four + r) * V) = row;
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                split_two(s[n][2 * half], s[n][2 * half + 1], s_planes + (row + 8 * half) * kNarrowRow + 8 * n + pair, kNarrowPlane);
+                store_pair(start + (size_t)(row + 8 * half) * V + 8 * n, s[n][2 * half], s[n][2 * half + 1]);
+            }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();  // S, y and the keys are there; nobody reads the other stage any more
+        if (chunk + 1 < chunks) fetch(chunk + 1);
+        const uint32_t stage = (chunk & 1) * kCarryStage * 2;
+        const float keep = expf(log_keep);
+        float product[2][4] = {};
+#pragma unroll
+        for (int d = 0; d < kDim; d += 16) {
+            Parts a, b;
+            load_parts(a, y_at + stage + d * 2, kPlane);
+            load_parts_turned(b, s_at + d * kNarrowRow * 2, kNarrowPlane);
+            split_products(product[0], product[1], a, b);
         }
-        const float keep = expf((float)args.logs[at * kChunk + kChunk - 1]);
-        if (chunk + 1 < chunks) {
-            fetch(chunk + 1);  // (its buffer was last read before the barrier that closed the chunk before)
-            copies_wait<1>();
-        } else {
-            copies_wait<0>();
-        }
+        float* to = args.u + item(chunk) * kChunk * V + column0 + pair;
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const float lo = x[n][half].x - product[n][2 * half], hi = x[n][half].y - product[n][2 * half + 1];
+                split_two(lo, hi, u_planes + (row + 8 * half) * kNarrowRow + 8 * n + pair, kNarrowPlane);
+                store_pair(to + (size_t)(row + 8 * half) * V + 8 * n, lo, hi);
+            }
+        if (chunk + 1 < chunks) fetch_x(chunk + 1);
         __syncthreads();
-        const float* stage = shared + (chunk & 1) * kStage;
-        {
-            uint64_t u[4][2];  // u = x - y S_0
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(stage + 2 * kDim * kChunk + (four + r) * kColumns + group);
-                u[r][0] = x.x, u[r][1] = x.y;
-            }
-#pragma unroll 16
-            for (int d = 0; d < kDim; ++d) {
-                const float4 y = *reinterpret_cast<const float4*>(stage + d * kChunk + four);
-                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(s_tile + d * kColumns + group);
-                const float rows[4] = {y.x, y.y, y.z, y.w};
+        for (int n = 0; n < 2; ++n)
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const uint64_t minus = twice(-rows[r]);
-                    u[r][0] = fma_pair(minus, b.x, u[r][0]);
-                    u[r][1] = fma_pair(minus, b.y, u[r][1]);
-                }
-            }
-            float* to = args.u + at * kChunk * V + column0 + group;
+            for (int i = 0; i < 4; ++i) s[n][i] *= keep;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const ulonglong2 row = make_ulonglong2(u[r][0], u[r][1]);
-                *reinterpret_cast<ulonglong2*>(u_tile + (four + r) * kColumns + group) = row;
-                *reinterpret_cast<ulonglong2*>(to + (size_t)(four + r) * V) = row;
-            }
+        for (int i = 0; i < kChunk; i += 16) {
+            Parts a, b;
+            load_parts_turned(a, key_at + stage + i * kRow * 2, kPlane);
+            load_parts_turned(b, u_at + i * kNarrowRow * 2, kNarrowPlane);
+            split_products(s[0], s[1], a, b);
         }
-        __syncthreads();
-        const uint64_t kept = twice(keep);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) s[r][0] = fma_pair(kept, s[r][0], 0), s[r][1] = fma_pair(kept, s[r][1], 0);
-#pragma unroll 16
-        for (int i = 0; i < kChunk; ++i) {
-            const float4 k = *reinterpret_cast<const float4*>(stage + kDim * kChunk + i * kDim + four);
-            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(u_tile + i * kColumns + group);
-            const float rows[4] = {k.x, k.y, k.z, k.w};
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const uint64_t x = twice(rows[r]);
-                s[r][0] = fma_pair(x, b.x, s[r][0]);
-                s[r][1] = fma_pair(x, b.y, s[r][1]);
-            }
-        }
-        __syncthreads();  // the chunk's buffers and tiles may be written again
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        float* to = stored + (size_t)(four + r) * V;
-        const float2 lo = floats_of(s[r][0]), hi = floats_of(s[r][1]);
-        to[0] = lo.x, to[1] = lo.y, to[2] = hi.x, to[3] = hi.y;
-    }
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) stored[(size_t)(row + 8 * (i / 2)) * V + 8 * n + i % 2] = s[n][i];
 }
 
-template <typename T>
-__device__ __forceinline__ float4 load4(const T* p);
-template <>
-__device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
-template <>
-__device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p);
-    return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
-}
-__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-}
-
-// grid (heads, most chunks of a sequence, sequences); block 128: thread (rows 4 * (tid / 16) .. +3 and 32 on, columns
-// 4 * (tid % 16) .. +3 of every 64).  shared: queries and keys transposed [64][68] (the second becomes the products' weights
-// [j][i]), one [64][V] tile for S_0 and then u, sums of log g, parts.
+// grid (heads, most chunks of a sequence, sequences); block kResultThreads: a warp has 16 tokens and half of the V columns of their
+// results (both halves' warps make the weights that they share).  u takes the start's place in shared memory, so that two blocks fit on
+// a multiprocessor.
 template <int V>
 struct ResultPlan {
-    static constexpr int queries = 0, keys = queries + kDim * (kChunk + kPad), tile = keys + kDim * (kChunk + kPad), logs = tile + kDim * V,
-                         parts = logs + 2 * kChunk, total = parts + 2 * kChunk;
+    static constexpr int wide_row = V + 8, wide_plane = 64 * wide_row;
+    static constexpr int queries = 0, keys = queries + kParts * kPlane, wide = keys + kParts * kPlane, bytes = (wide + kParts * wide_plane) * 2;
 };
 
 template <typename T, int V>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kResultThreads, 2)
 delta_chunks_results_kernel(const DeltaChunkArgs args) {
     using Plan = ResultPlan<V>;
-    constexpr int kFours = V / 64;
     grid_launch_dependents();
     grid_dependency_wait();
-    extern __shared__ __align__(16) float shared[];
-    float* queries = shared + Plan::queries;
-    float* keys = shared + Plan::keys;
-    float* tile = shared + Plan::tile;
-    double* logs = reinterpret_cast<double*>(shared + Plan::logs);
+    extern __shared__ __align__(16) unsigned char shared[];
+    bf16* planes = reinterpret_cast<bf16*>(shared);
+    __shared__ double logs[kChunk];
+    __shared__ float square_sums[2][kChunk];
     const int head = blockIdx.x, chunk = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
     const int first = args.cu_q[seq], count = min(kChunk, args.cu_q[seq + 1] - first - chunk * kChunk);
     if (count <= 0) return;
     const size_t token0 = (size_t)first + chunk * kChunk;
     const size_t at = place_of(first, seq, chunk) * args.heads + head;
     auto bring = [&](const float* from) {
-#pragma unroll 8
-        for (int i = tid; i < 64 * V / 4; i += 128) copy16_async(tile + 4 * i, from + 4 * i);
-        copies_sent();
+        constexpr int kPieces = 64 * V / 8 / kResultThreads;
+        float x[kPieces][8];
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) load8(from + 8 * (tid + i * kResultThreads), x[i]);
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int piece = tid + i * kResultThreads;
+            store_parts(planes + Plan::wide + piece / (V / 8) * Plan::wide_row + piece % (V / 8) * 8, Plan::wide_plane, x[i]);
+        }
     };
     bring(args.starts + at * kDim * V);
     if (tid < kChunk) logs[tid] = args.logs[at * kChunk + tid];
     const float* rows = args.conv + token0 * args.conv_stride;
     const int qk_head = head / (args.heads / args.kv_heads);
-    {
-        float own[32];
-        unit_rows(rows + args.k_at + qk_head * kDim, args.conv_stride, count, args.unit_eps, 1.0f, keys, shared + Plan::parts, own);
-        __syncthreads();
-        unit_rows(rows + args.q_at + qk_head * kDim, args.conv_stride, count, args.unit_eps, 0.125f, queries, shared + Plan::parts, own);  // 64^(-1/2)
-    }
-    copies_wait<0>();
+    UnitRows<kResultThreads>(rows + args.k_at + qk_head * kDim, args.conv_stride, count, args.unit_eps, 1.0f, planes + Plan::keys, nullptr);
+    UnitRows<kResultThreads>(rows + args.q_at + qk_head * kDim, args.conv_stride, count, args.unit_eps, 0.125f, planes + Plan::queries, nullptr);  // 64^(-1/2)
     __syncthreads();
-    const int row0 = (tid / 16) * 4, col0 = (tid % 16) * 4;
-    uint64_t acc[8][2 * kFours];
+    const int warp = (tid >> 5) & 3, half_columns = tid >> 7, column0 = half_columns * (V / 2), group = (tid & 31) >> 2, pair = 2 * (tid & 3);
+    const uint32_t base = smem_u32(planes);
+    const uint32_t query_at = base + (Plan::queries + 16 * warp * kRow) * 2 + lanes_by_row(kRow), key_at = base + Plan::keys * 2 + lanes_by_column(kRow);
+    const uint32_t wide_at = base + (Plan::wide + column0) * 2 + lanes_by_row(Plan::wide_row);
+    float acc[V / 16][4] = {}, weights[kChunk / 8][4] = {};
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+    for (int d = 0; d < kDim; d += 16) {
+        Parts a, b;
+        load_parts(a, query_at + d * 2, kPlane);
 #pragma unroll
-        for (int c = 0; c < 2 * kFours; ++c) acc[r][c] = 0;
-    auto product = [&](const float* a) {  // acc += a^T tile
-#pragma unroll 4
-        for (int d = 0; d < 64; ++d) {
-            const float4 lo = *reinterpret_cast<const float4*>(a + d * (kChunk + kPad) + row0), hi = *reinterpret_cast<const float4*>(a + d * (kChunk + kPad) + row0 + 32);
-            const float left[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-            ulonglong2 b[kFours];
-#pragma unroll
-            for (int f = 0; f < kFours; ++f) b[f] = *reinterpret_cast<const ulonglong2*>(tile + d * V + 64 * f + col0);
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const uint64_t x = twice(left[r]);
-#pragma unroll
-                for (int f = 0; f < kFours; ++f) {
-                    acc[r][2 * f] = fma_pair(x, b[f].x, acc[r][2 * f]);
-                    acc[r][2 * f + 1] = fma_pair(x, b[f].y, acc[r][2 * f + 1]);
-                }
-            }
+        for (int n = 0; n < V / 16; n += 2) {  // S_0^T q
+            load_parts_turned(b, wide_at + (d * Plan::wide_row + 8 * n) * 2, Plan::wide_plane);
+            split_products(acc[n], acc[n + 1], a, b);
         }
-    };
-    product(queries);  // S_0^T q
-    __syncthreads();   // the tile may be written again
+#pragma unroll
+        for (int n = 0; n < kChunk / 8; n += 2) {  // q . k over the tokens up to the warp's last
+            if (n > 2 * warp) break;
+            load_parts(b, key_at + (8 * n * kRow + d) * 2, kPlane);
+            split_products(weights[n], weights[n + 1], a, b);
+        }
+    }
+    __syncthreads();  // nobody reads the start any more
     bring(args.u + at * kChunk * V);
+    const int row = 16 * warp + group;
+    const float from_start[2] = {expf((float)logs[row]), expf((float)logs[row + 8])};
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const uint64_t g = twice(expf((float)logs[row0 + (r / 4) * 32 + r % 4]));
+    for (int n = 0; n < V / 16; ++n)
 #pragma unroll
-        for (int c = 0; c < 2 * kFours; ++c) acc[r][c] = fma_pair(g, acc[r][c], 0);
-    }
-    {
-        // weights[j][i] = G_i / G_j (q_i . k_j) for j <= i, over the keys
-        const int j0 = (tid % 8) * 4, i0 = (tid / 8) * 4;
-        uint64_t w[8][2];
+        for (int i = 0; i < 4; ++i) acc[n][i] *= from_start[i / 2];
+    __syncthreads();
 #pragma unroll
-        for (int r = 0; r < 8; ++r) w[r][0] = w[r][1] = 0;
-        tile_8x4(keys, queries, j0, i0, w);
-        __syncthreads();  // everybody has read the keys
+    for (int n = 0; n < kChunk / 8; n += 2) {
+        if (n > 2 * warp) break;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int j = j0 + (r / 4) * 32 + r % 4;
-            const float2 lo = floats_of(w[r][0]), hi = floats_of(w[r][1]);
-            float v[4] = {lo.x, lo.y, hi.x, hi.y};
+        for (int m = n; m < n + 2; ++m)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) v[c] = j <= i0 + c ? v[c] * expf((float)(logs[i0 + c] - logs[j])) : 0.0f;
-            *reinterpret_cast<float4*>(keys + j * (kChunk + kPad) + i0) = make_float4(v[0], v[1], v[2], v[3]);
+            for (int i = 0; i < 4; ++i) {
+                const int to = row + 8 * (i / 2), from = 8 * m + pair + i % 2;
+                weights[m][i] = from <= to ? weights[m][i] * expf((float)(logs[to] - logs[from])) : 0.0f;
+            }
+        Parts a, b;
+        split_pair(weights[n][0], weights[n][1], a[0][0], a[1][0], a[2][0]);
+        split_pair(weights[n][2], weights[n][3], a[0][1], a[1][1], a[2][1]);
+        split_pair(weights[n + 1][0], weights[n + 1][1], a[0][2], a[1][2], a[2][2]);
+        split_pair(weights[n + 1][2], weights[n + 1][3], a[0][3], a[1][3], a[2][3]);
+#pragma unroll
+        for (int c = 0; c < V / 16; c += 2) {
+            load_parts_turned(b, wide_at + (8 * n * Plan::wide_row + 8 * c) * 2, Plan::wide_plane);
+            split_products(acc[c], acc[c + 1], a, b);
         }
     }
-    copies_wait<0>();
-    __syncthreads();
-    product(keys);
-    // a row's V results lie with sixteen neighbouring lanes
-    const T* gate = (const T*)args.gate_in + token0 * args.in_stride + (size_t)head * V;
-    T* out = (T*)args.out + token0 * args.out_stride + (size_t)head * V;
+    // norm, gain and gate: a row's V results lie with four neighbouring lanes of two warps
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int row = row0 + (r / 4) * 32 + r % 4;
+    for (int half = 0; half < 2; ++half) {
         float squares = 0.0f;
 #pragma unroll
-        for (int c = 0; c < 2 * kFours; ++c) {
-            const float2 o = floats_of(acc[r][c]);
-            squares = fmaf(o.x, o.x, squares), squares = fmaf(o.y, o.y, squares);
-        }
+        for (int n = 0; n < V / 16; ++n) squares = fmaf(acc[n][2 * half], acc[n][2 * half], fmaf(acc[n][2 * half + 1], acc[n][2 * half + 1], squares));
+        squares += __shfl_xor_sync(0xffffffffu, squares, 1);
+        squares += __shfl_xor_sync(0xffffffffu, squares, 2);
+        if (pair == 0) square_sums[half_columns][row + 8 * half] = squares;
+    }
+    __syncthreads();
 #pragma unroll
-        for (int offset = 1; offset < 16; offset <<= 1) squares += __shfl_xor_sync(0xffffffffu, squares, offset);
-        if (row < count) {
-            const float inv = args.out_scale / sqrtf(squares / (float)V + args.eps);
+    for (int half = 0; half < 2; ++half) {
+        const int to = row + 8 * half;
+        if (to >= count) continue;
+        const float inv = args.out_scale / sqrtf((square_sums[0][to] + square_sums[1][to]) / (float)V + args.eps);
+        const size_t column = (size_t)head * V + column0 + pair;
+        const T* gate = (const T*)args.gate_in + (token0 + to) * args.in_stride + column;
+        T* dst = (T*)args.out + (token0 + to) * args.out_stride + column;
 #pragma unroll
-            for (int f = 0; f < kFours; ++f) {
-                const int c = 64 * f + col0;
-                const float4 z = load4<T>(gate + (size_t)row * args.in_stride + c), gain = *reinterpret_cast<const float4*>(args.gain + c);
-                const float2 lo = floats_of(acc[r][2 * f]), hi = floats_of(acc[r][2 * f + 1]);
-                store4(out + (size_t)row * args.out_stride + c,
-                       make_float4(lo.x * inv * gain.x * (z.x * sigmoid(z.x)), lo.y * inv * gain.y * (z.y * sigmoid(z.y)),
-                                   hi.x * inv * gain.z * (z.z * sigmoid(z.z)), hi.y * inv * gain.w * (z.w * sigmoid(z.w))));
-            }
+        for (int n = 0; n < V / 16; ++n) {
+            const float2 z = load_pair(gate + 8 * n), gain = load_pair(args.gain + column0 + 8 * n + pair);
+            store_pair(dst + 8 * n, acc[n][2 * half] * inv * gain.x * (z.x * sigmoid(z.x)), acc[n][2 * half + 1] * inv * gain.y * (z.y * sigmoid(z.y)));
         }
     }
 }
@@ -510,15 +543,15 @@ static int reserve(Kernel kernel, int bytes) {
 
 template <typename T, int V>
 static int launch_chunks(const DeltaChunkArgs& args, int sequences, int chunks, cudaStream_t stream) {
-    constexpr int solve = SolvePlan<V>::total * 4, carry = (2 * (2 * kDim * kChunk + kChunk * kColumns) + (kDim + kChunk) * kColumns) * 4,
-                  results = ResultPlan<V>::total * 4;
+    constexpr int solve = SolvePlan<V>::bytes, results = ResultPlan<V>::bytes;
     if (int status = reserve(delta_chunks_solve_kernel<T, V>, solve)) return status;
-    if (int status = reserve(delta_chunks_carry_kernel<V>, carry)) return status;
+    if (int status = reserve(delta_chunks_carry_kernel<V>, kCarryBytes)) return status;
     if (int status = reserve(delta_chunks_results_kernel<T, V>, results)) return status;
     const dim3 grid(args.heads, chunks, sequences);
-    MB_LAUNCH("gated_delta_chunks", (delta_chunks_solve_kernel<T, V>), grid, dim3(128), solve, stream, true, args);
-    MB_LAUNCH("gated_delta_chunks", (delta_chunks_carry_kernel<V>), dim3(V / kColumns, args.heads, sequences), dim3(64), carry, stream, true, args);
-    MB_LAUNCH("gated_delta_chunks", (delta_chunks_results_kernel<T, V>), grid, dim3(128), results, stream, true, args);
+    MB_LAUNCH("gated_delta_chunks", (delta_chunks_solve_kernel<T, V>), grid, dim3(SolvePlan<V>::threads), solve, stream, true, args);
+    MB_LAUNCH("gated_delta_chunks", (delta_chunks_carry_kernel<V>), dim3(V / kColumns, args.heads, sequences), dim3(kCarryThreads), kCarryBytes, stream, true,
+              args);
+    MB_LAUNCH("gated_delta_chunks", (delta_chunks_results_kernel<T, V>), grid, dim3(kResultThreads), results, stream, true, args);
     return check_launch("gated_delta_chunks");
 }
 
@@ -529,7 +562,7 @@ using namespace mb;
 MB_EXPORT int mb_gated_delta_chunk_tokens() { return kChunk; }
 
 // Arguments as mb_gated_delta_scan's, with key heads of 64 numbers and value heads of 64 or 128; conv is only read.  scratch: floats,
-// (places * heads) * (2 * 64 * vdim + 2 * 64 * 64 + 128), 16-byte aligned, with places = tokens / 64 + sequences.
+// (places * heads) * (2 * 64 * vdim + 3 * 64 * 64 + 128), 16-byte aligned, with places = tokens / 64 + sequences.
 MB_EXPORT int mb_gated_delta_chunks(const float* conv, int conv_stride, const void* a_in, const void* b_in, const void* gate_in, int in_stride,
                                     int dtype, const float* decay, const float* dt_bias, const float* gain, float unit_eps, float eps, float* state,
                                     size_t state_stride, const int* slots, const int* cu_q, int sequences, int tokens, int max_q_len, float* scratch,
@@ -553,9 +586,9 @@ MB_EXPORT int mb_gated_delta_chunks(const float* conv, int conv_stride, const vo
     const size_t items = ((size_t)tokens / kChunk + sequences) * heads;
     args.u = scratch;
     args.starts = args.u + items * kChunk * vdim;
-    args.y = args.starts + items * kDim * vdim;
-    args.keys = args.y + items * kDim * kChunk;
-    args.logs = reinterpret_cast<double*>(args.keys + items * kChunk * kDim);
+    args.y = reinterpret_cast<bf16*>(args.starts + items * kDim * vdim);
+    args.keys = args.y + kParts * items * kChunk * kDim;
+    args.logs = reinterpret_cast<double*>(args.keys + kParts * items * kChunk * kDim);
     if (dtype == MB_F32) return vdim == 64 ? launch_chunks<float, 64>(args, sequences, chunks, stream) : launch_chunks<float, 128>(args, sequences, chunks, stream);
     if (dtype == MB_BF16)
         return vdim == 64 ? launch_chunks<__nv_bfloat16, 64>(args, sequences, chunks, stream) : launch_chunks<__nv_bfloat16, 128>(args, sequences, chunks, stream);

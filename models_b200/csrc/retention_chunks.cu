@@ -5,28 +5,24 @@
 //   o_i = a^(i + 1) S_0^T q_i + sum_(j <= i) a^(i - j) (q_i . k_j) v_j,     S_end = a^n S_0 + sum_j a^(n - 1 - j) k_j v_j^T
 // Three kernels: what every chunk adds to the state, a product per (chunk, head); the states that the chunks start from, element by
 // element in the chunks' order; every chunk's results, with the head's norm and gate where the caller wants them here.
-// The numbers between the first products and the last one are floats, and none of their 24 bits is lost on the way into a product:
-// every operand is three bfloat16 numbers, its rounding, the rounding of what that left and of what this left, and six of the nine
-// products of parts are added up in float (the other three are below 2^-26 of the product).
+// The numbers between the first products and the last one are floats, and products take them whole (split_products.cuh).
 // Against 64 bits, over steps of 64 to 2,048 tokens: the state is off by 6e-8 to 9e-8 of itself (the walk in runs: 0.9e-7 to 1.4e-7), the
 // raw results by 0.7e-7 to 1.1e-7 (0.8e-7 to 1.8e-7); with two parts the operands would be cut to 16 bits.
 // Three sequences of 2,048 tokens in all, 16 heads of 64 x 128 with activated projections: 208 us as the walk in runs (98, 70 and 40),
 // which float multiply-adds from shared memory bound; here 32, 14 and 58 us, bound by the six products for one and by the
 // instructions that activate and split what every chunk reads.
 #include "common.cuh"
+#include "split_products.cuh"
 
 MB_DEFINE_LAST_ERROR()
 
 namespace mb {
-
-using bf16 = __nv_bfloat16;
 
 constexpr int kChunk = 64;    // tokens of a chunk
 constexpr int kDim = 64;      // a key head's numbers
 constexpr int kThreads = 256;  // eight warps: four of 16 rows each for either half of the V columns
 constexpr int kKeyRow = kDim + 8;                // bfloat16 numbers of a padded row: ldmatrix without bank conflicts
 constexpr int kKeyPlane = kChunk * kKeyRow;      // one part of 64 rows; an operand's three planes lie one after another
-constexpr int kParts = 3;
 
 template <int V>
 struct Values {
@@ -54,69 +50,6 @@ struct RetentionArgs {
 // Every sequence's chunks lie one after another, a sequence's first place being floor(first / 64) + seq (a sequence of n tokens has
 // ceil(n / 64) chunks, and floor(f / 64) + ceil(n / 64) <= floor((f + n) / 64) + 1).
 __device__ __forceinline__ size_t place_of(int first, int seq, int chunk) { return (size_t)(first / kChunk) + seq + chunk; }
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t at) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
-}
-__device__ __forceinline__ void ldmatrix4_turned(uint32_t (&r)[4], uint32_t at) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
-}
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// Two floats as pairs of bfloat16 numbers: their roundings, the roundings of what those left, and of what these left.
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    float2 back = __bfloat1622float2(h);
-    a -= back.x, b -= back.y;
-    const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
-    back = __bfloat1622float2(m);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(a - back.x, b - back.y);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    mid = *reinterpret_cast<const uint32_t*>(&m);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-// Eight floats into an operand's three planes.
-__device__ __forceinline__ void store_parts(bf16* to, int plane, const float (&x)[8]) {
-    uint4 hi, mid, lo;
-    split_pair(x[0], x[1], hi.x, mid.x, lo.x);
-    split_pair(x[2], x[3], hi.y, mid.y, lo.y);
-    split_pair(x[4], x[5], hi.z, mid.z, lo.z);
-    split_pair(x[6], x[7], hi.w, mid.w, lo.w);
-    *reinterpret_cast<uint4*>(to) = hi;
-    *reinterpret_cast<uint4*>(to + plane) = mid;
-    *reinterpret_cast<uint4*>(to + 2 * plane) = lo;
-}
-
-using Parts = uint32_t[kParts][4];
-__device__ __forceinline__ void load_parts(Parts& r, uint32_t at, int plane) {
-#pragma unroll
-    for (int i = 0; i < kParts; ++i) ldmatrix4(r[i], at + 2 * i * plane);
-}
-__device__ __forceinline__ void load_parts_turned(Parts& r, uint32_t at, int plane) {
-#pragma unroll
-    for (int i = 0; i < kParts; ++i) ldmatrix4_turned(r[i], at + 2 * i * plane);
-}
-// d[tile] += a . b for two neighbouring tiles of eight columns.  The tensor cores cut their sums off where a float addition rounds, so
-// the sixteen products of roundings, whose sum has few bits to lose, and the smaller ones, the smallest first, start from zero and are
-// added as floats (all in one chain: results of 2,048 tokens off by 8.9e-7 where the walk is off by 1e-7).
-__device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], const Parts& a, const Parts& b) {
-    float p0[4] = {}, p1[4] = {}, r0[4] = {}, r1[4] = {};
-#pragma unroll
-    for (int order = kParts - 1; order > 0; --order)
-#pragma unroll
-        for (int i = 0; i <= order; ++i) {
-            mma_bf16(r0, a[i], b[order - i][0], b[order - i][1]);
-            mma_bf16(r1, a[i], b[order - i][2], b[order - i][3]);
-        }
-    mma_bf16(p0, a[0], b[0][0], b[0][1]);
-    mma_bf16(p1, a[0], b[0][2], b[0][3]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) d0[i] += p0[i] + r0[i], d1[i] += p1[i] + r1[i];
-}
 
 // The rows of `count` tokens (64 with zeros behind them) of a head, `kCols` columns from `src`, activated, rotated (rotary > 0),
 // times weight[row] (or 1), in planes of rows of `row_numbers`.

@@ -1,0 +1,77 @@
+// Products of floats on the tensor cores (mma.sync m16n8k16) that keep a float's 24 bits: every operand is three bfloat16 numbers, its
+// rounding, the rounding of what that left and of what this left, and six of the nine products of parts are added up in float (the
+// other three are below 2^-26 of the product).  Operands lie in shared memory as three planes, one after another.
+#pragma once
+
+#include <cuda_bf16.h>
+#include <stdint.h>
+
+namespace mb {
+
+using bf16 = __nv_bfloat16;
+constexpr int kParts = 3;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t at) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_turned(uint32_t (&r)[4], uint32_t at) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two floats as pairs of bfloat16 numbers: their roundings, the roundings of what those left, and of what these left.
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    float2 back = __bfloat1622float2(h);
+    a -= back.x, b -= back.y;
+    const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
+    back = __bfloat1622float2(m);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a - back.x, b - back.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    mid = *reinterpret_cast<const uint32_t*>(&m);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// Eight floats into an operand's three planes.
+__device__ __forceinline__ void store_parts(bf16* to, int plane, const float (&x)[8]) {
+    uint4 hi, mid, lo;
+    split_pair(x[0], x[1], hi.x, mid.x, lo.x);
+    split_pair(x[2], x[3], hi.y, mid.y, lo.y);
+    split_pair(x[4], x[5], hi.z, mid.z, lo.z);
+    split_pair(x[6], x[7], hi.w, mid.w, lo.w);
+    *reinterpret_cast<uint4*>(to) = hi;
+    *reinterpret_cast<uint4*>(to + plane) = mid;
+    *reinterpret_cast<uint4*>(to + 2 * plane) = lo;
+}
+
+using Parts = uint32_t[kParts][4];
+__device__ __forceinline__ void load_parts(Parts& r, uint32_t at, int plane) {
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) ldmatrix4(r[i], at + 2 * i * plane);
+}
+__device__ __forceinline__ void load_parts_turned(Parts& r, uint32_t at, int plane) {
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) ldmatrix4_turned(r[i], at + 2 * i * plane);
+}
+// d[tile] += a . b for two neighbouring tiles of eight columns.  The tensor cores cut their sums off where a float addition rounds, so
+// the sixteen products of roundings, whose sum has few bits to lose, and the smaller ones, the smallest first, start from zero and are
+// added as floats (all in one chain: results of 2,048 tokens off by 8.9e-7 where the walk is off by 1e-7).
+__device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], const Parts& a, const Parts& b) {
+    float p0[4] = {}, p1[4] = {}, r0[4] = {}, r1[4] = {};
+#pragma unroll
+    for (int order = kParts - 1; order > 0; --order)
+#pragma unroll
+        for (int i = 0; i <= order; ++i) {
+            mma_bf16(r0, a[i], b[order - i][0], b[order - i][1]);
+            mma_bf16(r1, a[i], b[order - i][2], b[order - i][3]);
+        }
+    mma_bf16(p0, a[0], b[0][0], b[0][1]);
+    mma_bf16(p1, a[0], b[0][2], b[0][3]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d0[i] += p0[i] + r0[i], d1[i] += p1[i] + r1[i];
+}
+
+}  // namespace mb

@@ -1431,7 +1431,7 @@ def gated_delta_scan(conv: torch.Tensor, q_at: int, k_at: int, v_at: int, a_in: 
     if gated_delta_chunks_takes(conv, gate_in, gain, out, dim, vdim, (q_at, k_at, v_at), max_q_len):
         lib = gated_delta_chunks_library()
         places = tokens // lib.mb_gated_delta_chunk_tokens() + cu_q.numel() - 1
-        scratch = torch.empty((places * heads * (2 * 64 * vdim + 2 * 64 * 64 + 128),), dtype=torch.float32, device=conv.device)
+        scratch = torch.empty((places * heads * (2 * 64 * vdim + 3 * 64 * 64 + 128),), dtype=torch.float32, device=conv.device)
         _run(lib, lib.mb_gated_delta_chunks(_p(conv), conv.stride(0), _p(a_in), _p(b_in), _p(gate_in), a_in.stride(0), _code(out.dtype), _p(decay),
                                             _p(dt_bias), _p(gain), ctypes.c_float(unit_eps), ctypes.c_float(eps), rows, stride, _p(slots),
                                             _p(cu_q), cu_q.numel() - 1, tokens, int(max_q_len), _p(scratch), _p(out), out.stride(0),
