@@ -1027,6 +1027,26 @@ def test_rotate_norm_store_in_eights(cuda_device, heads, kv_heads, dim, vdim, ro
         assert float((here != there).float().mean()) < 0.01
 
 
+@pytest.mark.parametrize("activation", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("rows", [129, 300, 512])
+def test_gated_prompt_product_with_rows_of_zeros(cuda_device, activation, rows):
+    """Rows of nothing but zeros, which pad a step, within a piece of other rows, as whole pieces and at the end: their results are
+    zero, and the other rows' what they are without them."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(rows)
+    a, w = torch.randn(rows, 256, generator=g).bfloat16().cuda(), (torch.randn(1024, 256, generator=g) * 0.05).bfloat16().cuda()
+    epilogue = ops.EPI_SWIGLU | ops.activation_code(activation) << 8  # (the epilogue carries its activation above its code)
+    want = ops.gemm_tcgen05(a, w, epilogue)
+    empty = torch.zeros(rows, dtype=torch.bool)
+    empty[[5, 40, rows - 1]] = True
+    empty[64:100] = True
+    zeroed = a.clone()
+    zeroed[empty.cuda()] = 0
+    got = ops.gemm_tcgen05(zeroed, w, epilogue)
+    assert bool((got[empty.cuda()] == 0).all()) and torch.equal(got[~empty.cuda()], want[~empty.cuda()])
+
+
 @pytest.mark.parametrize("batch", [1, 3, 8])
 @pytest.mark.parametrize("n,k", [(2048, 4104), (37, 5000), (16, 8192), (2360, 8192)])
 def test_skinny_gemm_streams_activations(cuda_device, batch, n, k):
