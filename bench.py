@@ -908,7 +908,7 @@ def rolevik_kernels(z, peak, prompt=2048, batch=8, context=1536):
         def delta():
             conv = ops.short_conv(proj[:, :C], conv_w, state, floats, slots, cu, q_len, activation="silu", store_tail=True)
             ops.gated_delta_scan(conv, 0, DG * D, 2 * DG * D, proj[:, C:C + DH], proj[:, C + 8:C + 8 + DH], proj[:, C + 16:], decay, dt_bias, gain,
-                                 1e-6, 1e-6, state, 0, slots, cu, DH, DG, D, DV, y)
+                                 1e-6, 1e-6, state, 0, slots, cu, DH, DG, D, DV, y, max_q_len=q_len)
 
         us = time_kernel(delta)
         moved = rows * (C * 2 + C * 8 + 2 * DH * DV * 2) + sequences * floats * 8
