@@ -466,7 +466,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 tmem_load_32_issue(taddr + c + 32 * part, v);
                                 tmem_load_32_issue(taddr + 128 + c + 32 * part, u);
                                 tmem_load_wait();
-                                // Rows beyond the last, and those that pad a step, are zeros, and a division of zero takes its long way:
+                                // Rows beyond the last are zeros, and a division of zero takes its long way:
                                 // 50 us for 437 rows of 2,048 with 16,384 weight rows where 512 took 34.  A gated zero is zero under
                                 // every activation, so pieces of nothing but zeros stay as they are: 33 us.
                                 uint32_t bits = 0;

@@ -1030,7 +1030,7 @@ def test_rotate_norm_store_in_eights(cuda_device, heads, kv_heads, dim, vdim, ro
 @pytest.mark.parametrize("activation", ["silu", "gelu_tanh"])
 @pytest.mark.parametrize("rows", [129, 300, 512])
 def test_gated_prompt_product_with_rows_of_zeros(cuda_device, activation, rows):
-    """Rows of nothing but zeros, which pad a step, within a piece of other rows, as whole pieces and at the end: their results are
+    """Rows of nothing but zeros within a piece of other rows, as whole pieces and at the end: their results are
     zero, and the other rows' what they are without them."""
     from models_b200.kernels import ops
 
