@@ -376,8 +376,14 @@ skinny_gemm_kernel(const SkinnyArgs args) {
     }
     bool sq_gathered = args.k_split == 1;
 
-
     float held_scale = 0.0f;  // 1 / rms of the column of this thread's first finishing item (the same in every tile), from the first tile on
+    auto inverse_rms = [&](int col) {
+        float sum = 0.0f;
+        if (PRO == PRO_NORM) sum = sq_total[col];
+        else
+            for (int w = 0; w < kWarps; ++w) sum += sq_warp[w * COLS + col];
+        return 1.0f / sqrtf(sum / (float)args.k + args.eps);
+    };
     // ---- row tile after row tile; the ring keeps running across them
     int stage_index = 0;
     for (int local = 0; local < tiles_mine; ++local) {
@@ -466,6 +472,8 @@ skinny_gemm_kernel(const SkinnyArgs args) {
         } else {
             __syncthreads();
         }
+        // (whether or not the item lies outside this tile: in another one it may not)
+        if (PRO != PRO_NONE && local == 0 && (int)threadIdx.x / kTileRows < args.batch) held_scale = inverse_rms(threadIdx.x / kTileRows);
         for (int i = threadIdx.x; i < kTileRows * COLS; i += kThreads) {
             const int row_in_tile = i % kTileRows, col = i / kTileRows;  // neighbouring threads store neighbouring output columns
             const int row = tile * kTileRows + row_in_tile;
@@ -486,16 +494,7 @@ skinny_gemm_kernel(const SkinnyArgs args) {
                 }
             }
             if (PRO != PRO_NONE) {
-                const bool first_item = i == (int)threadIdx.x;
-                float inv_rms = held_scale;
-                if (local == 0 || !first_item) {
-                    float sum = 0.0f;
-                    if (PRO == PRO_NORM) sum = sq_total[col];
-                    else
-                        for (int w = 0; w < kWarps; ++w) sum += sq_warp[w * COLS + col];
-                    inv_rms = 1.0f / sqrtf(sum / (float)args.k + args.eps);
-                    if (first_item) held_scale = inv_rms;
-                }
+                const float inv_rms = i == (int)threadIdx.x ? held_scale : inverse_rms(col);
                 value *= inv_rms;
                 second *= inv_rms;
             }

@@ -129,6 +129,30 @@ def test_product_with_two_kinds_of_rows(cuda_device, plain, pairs, k, rows):
     check(ops.skinny_gemm_pairs(dev(w), plain, wide[:, 8:8 + pairs], clamp, x=dev(xf * gain), norm_parts=(parts, 3, k, 1e-4)), wide, normed)
 
 
+@pytest.mark.parametrize("rows", [1, 8])
+@pytest.mark.parametrize("plain", [1601, 1607, 1612])
+def test_pairs_behind_the_last_tile_of_plain_rows(cuda_device, plain, rows):
+    """More tiles than blocks: the block whose first tile is the last one of the plain rows, which end within it, scales its later tiles of
+    pairs by the rows' norms like every other."""
+    from models_b200.kernels import ops
+
+    pairs, k, clamp = 4800, 64, (0.7, 1.702, 1.0)
+    g = torch.Generator().manual_seed(plain)
+    dev = lambda t, d=torch.bfloat16: t.to(d).to(cuda_device).contiguous()  # noqa: E731
+    w = _rounded(torch.randn(plain + 2 * pairs, k, generator=g) * k ** -0.5, torch.bfloat16)
+    xf, gain = torch.randn(rows, k, generator=g) * 3, 1 + 0.3 * torch.randn(k, generator=g)
+    want = (pr.over_rms(xf.double(), 1e-4) * gain.double()) @ w.double().T
+    want_pairs = _clamped(want[:, plain:plain + pairs], want[:, plain + pairs:], *clamp)
+    parts, squares = torch.zeros((3, ops.SSQ_COLUMNS), dtype=torch.float32, device=cuda_device), (xf.double() ** 2).sum(1)
+    parts[0, :rows], parts[2, :rows] = dev(squares * 0.25, torch.float32), dev(squares * 0.75, torch.float32)
+    for rows_as in ({"xf": dev(xf, torch.float32), "gain": dev(gain, torch.float32), "eps": 1e-4}, {"x": dev(xf * gain), "norm_parts": (parts, 3, k, 1e-4)}):
+        mid = torch.empty((rows, pairs), dtype=torch.bfloat16, device=cuda_device)
+        out = ops.skinny_gemm_pairs(dev(w), plain, mid, clamp, **rows_as)
+        # (the bounds of the test above; rows that miss their factor are off by all of their size)
+        assert scaled_error(out.double().cpu(), want[:, :plain]) < 1.5e-2
+        assert scaled_error(mid.double().cpu(), want_pairs) < 2e-2
+
+
 @pytest.mark.parametrize("rows", [9, 40, 128, 129, 300])
 @pytest.mark.parametrize("pairs,k", [(40, 64), (264, 520), (1024, 256)])
 def test_clamped_pairs_in_the_tensor_core_products(cuda_device, rows, pairs, k):
