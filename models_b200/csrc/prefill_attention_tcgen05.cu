@@ -615,6 +615,8 @@ MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int 
 #endif
     if (((uintptr_t)turn_cos | (uintptr_t)turn_sin) & 15) return fail("prefill_attention_tcgen05: the tables that turn the result back must start on 16-byte boundaries");
     if (sequences <= 0 || max_q_len <= 0) return 0;
+    if (softcap < 0.0f) return fail("prefill_attention_tcgen05: softcap %g", softcap);
+    if ((turn_cos == nullptr) != (turn_sin == nullptr)) return fail("prefill_attention_tcgen05: turning the result back needs both tables");
     if (int status = check_prefill(q, q_row_stride, out, out_row_stride, sequences, max_q_len, heads, kv_heads)) return status;
     if (page_size != kKeys) return fail("prefill_attention_tcgen05: the cache page must hold %d positions, got %d", kKeys, page_size);
     if (((uintptr_t)k_pool & 15) || ((uintptr_t)v_pool & 15)) return fail("prefill_attention_tcgen05: the cache pools must start on 16-byte boundaries");

@@ -1108,6 +1108,19 @@ def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
     assert float((outs[0] - outs[1]).norm()) <= 2.0 ** -9 * float(outs[1].norm())
 
 
+@pytest.mark.parametrize("max_q_len,kernel", [(1, None), (64, None), (64, "tc"), (64, "rows")])
+def test_a_negative_bound_on_scores_is_refused(cuda_device, max_q_len, kernel):
+    """Whichever kernel a call meets."""
+    from models_b200.kernels import ops
+
+    q, out = (torch.zeros(max_q_len, 2 * 64, dtype=torch.bfloat16, device=cuda_device) for _ in range(2))
+    pools = [torch.zeros(2, 1, 64, 64, dtype=torch.bfloat16, device=cuda_device) for _ in range(2)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda_device)  # noqa: E731
+    with pytest.raises(ops.KernelError, match="softcap -1"):
+        ops.gated_attention(q, out, *pools, i32([[1]]), i32([0, max_q_len]), i32([max_q_len]), max_q_len, 2, 1, 64, 64, "softmax", 0.125, softcap=-1.0,
+                            kernel=kernel)
+
+
 @pytest.mark.parametrize("query_latent,gate_kind,window,turned", [(128, "element", 0, 64), (0, "head", 90, 32), (128, None, 64, 0)])
 @pytest.mark.parametrize("q_lens,past", [([70, 200], [0, 0]), ([150, 64, 129], [100, 0, 37]), ([33], [31])])
 def test_latent_prompts_expand_the_rows_they_see(cuda_device, monkeypatch, query_latent, gate_kind, window, turned, q_lens, past):
