@@ -283,6 +283,14 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
         local += e;
     }
     const float sum = block_sum(local, float_scratch);
+    if (!(sum == sum)) {  // a NaN or an infinity among the logits: no order to draw from, the row takes its first maximum
+        if (tid == 0) {
+            const int token = top.index == 0x7fffffff ? 0 : top.index;
+            out[r] = token;
+            if (append && h_row) h_row[history_len[r]] = token;
+        }
+        return;
+    }
     for (int i = tid; i < vocab; i += kThreads) w[i] = w[i] / sum;
     __syncthreads();
 
@@ -593,6 +601,15 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     cluster.sync();
     float sum = 0.0f;
     for (int b = 0; b < kSampleBlocks; ++b) sum += *cluster.map_shared_rank(&slot_sum, b);
+    if (!(sum == sum)) {  // a NaN or an infinity among the logits: no order to draw from, the row takes its first maximum
+        if (part == 0 && tid == 0) {
+            const int token = top.index == 0x7fffffff ? 0 : top.index;
+            out[r] = token;
+            if (grown) *grown = token;
+        }
+        cluster.sync();  // everybody has read the sums
+        return;
+    }
     if (few) {
         const int count = *first_gathered;
         if (count >= k && count <= kMaxSorted) {

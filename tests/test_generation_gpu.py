@@ -405,6 +405,25 @@ def test_sampling_with_few_candidates_at_the_edges_of_its_rule(cuda_device, voca
         assert got[row] == want, (row, o, got[row], want)
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("top_p", [0.9, 1.0])
+def test_a_row_without_an_order_takes_its_first_maximum(cuda_device, value, top_p):
+    """Every probability of a row with a NaN or an infinity is NaN; what it draws depends on neither timing nor the kernel."""
+    from models_b200.sampling import BatchSampler, RequestSampling, SamplingOptions
+
+    vocab = 5003
+    logits = torch.randn(1, vocab, generator=torch.Generator().manual_seed(3))
+    logits[0, 700] = value
+    want = 700 if value == float("inf") else int(logits[0].nan_to_num(-float("inf")).argmax())
+    # few candidates, histograms, more candidates than are sorted (a block a row), everything
+    for ks in ((1, 5, 40, 128), (129, 1000), (40, 2000) if top_p == 1.0 else (), (40, vocab) if top_p == 1.0 else ()):
+        requests = [RequestSampling(SamplingOptions(top_k=k, top_p=top_p, seed=1), [0]) for k in ks]
+        if ks:
+            rows = logits.repeat(len(ks), 1).cuda()
+            for _ in range(5):
+                assert BatchSampler(vocab, "cuda:0").sample(rows, requests).tolist() == [want] * len(ks), ks
+
+
 def test_sampling_is_reproducible_and_follows_the_distribution(cuda_device):
     import models_b200
     from models_b200.sampling import BatchSampler, RequestSampling, SamplingOptions
