@@ -564,7 +564,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     int* first_gathered = cluster.map_shared_rank(&gathered, 0);
     int* const grown = (append && h_row) ? h_row + history_len[r] : nullptr;
 
-    const bool few = k <= kFewCandidates && k < vocab;
+    bool few = k <= kFewCandidates && k < vocab;
     float threshold = CUDART_INF_F;
     if (few) {
         if (tid < kSampleBlocks * 32) warp_tops[tid] = cluster.map_shared_rank(best_scratch, tid >> 5)[tid & 31].value;
@@ -578,19 +578,23 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         }
         __syncthreads();
         threshold = few_threshold - kThresholdSlack;
+        few = threshold > -CUDART_INF_F;  // (fewer warps than k with a finite value: every value would reach it)
     }
 
     // softmax over the whole vocabulary
     float local = 0.0f;
+    bool gathers = few;  // a thread that finds no place left stops: the histograms will decide
     for (int i = begin + tid; i < end; i += kThreads) {
         const float v = w[i], e = expf(v - top.value);
         w[i] = e;
         local += e;
-        if (few && v >= threshold) {
+        if (gathers && v >= threshold) {
             const int at = atomicAdd(first_gathered, 1);
             if (at < kMaxSorted) {
                 first_p[at] = e;
                 first_id[at] = i;
+            } else {
+                gathers = false;
             }
         }
     }
