@@ -5,8 +5,9 @@
 // out[r] = sum_c W[r, c] * x[c] (integrallis/models, backend-java/.../ops/TensorOps.java:61-63).
 // Every output element is the sum, in order, of up to eight chains of FMAs over consecutive parts of
 // c = 0..K-1, each in ascending order; the parts follow from N and K alone, so a row's result does not
-// depend on how many other rows the call carries, on where the row sits in a tile or on which of the
-// kernels below computes it.
+// depend on how many other rows the call carries, on where the row sits in a tile, on its alignment or on
+// which of the kernels below computes it.  (A decode product that need not be row-invariant takes gemv_f32_kernel,
+// whose sums run over lanes.)
 //
 // Bound by shared memory and the FMA pipe together: a lane's 8 x 8 results take 16 operands per column
 // of K, 64 bytes through a 128-byte port for the 64 FMAs, both 16 cycles of a multiprocessor per warp.
@@ -27,13 +28,21 @@ constexpr int kTileM = 64, kTileN = 64, kTileK = 16;
 // Any sizes, strides and alignments.
 __global__ void __launch_bounds__(256)
 gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, float* __restrict__ c,
-                int ldc, int m, int n, int k) {
+                int ldc, int m, int n, int k, int part_length) {
     __shared__ float a_tile[kTileK][kTileM + 4];
     __shared__ float w_tile[kTileK][kTileN + 4];
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
     const int row0 = blockIdx.y * kTileM, col0 = blockIdx.x * kTileN;
-    float acc[4][4] = {};
+    float acc[4][4] = {}, sum[4][4] = {};
     for (int k0 = 0; k0 < k; k0 += kTileK) {
+        if (k0 > 0 && k0 % part_length == 0)  // the next part's chains begin (part_length is a multiple of kTileK)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    sum[i][j] = k0 == part_length ? acc[i][j] : sum[i][j] + acc[i][j];
+                    acc[i][j] = 0.0f;
+                }
         // 64 rows x 16 columns of each operand; 256 threads, 4 elements each
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -65,7 +74,7 @@ gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int gc = col0 + tx * 4 + j;
-            if (gc < n) c[(size_t)gr * ldc + gc] = acc[i][j];
+            if (gc < n) c[(size_t)gr * ldc + gc] = k > part_length ? sum[i][j] + acc[i][j] : acc[i][j];
         }
     }
 }
@@ -195,7 +204,7 @@ gemm_f32_tiled_kernel(const float* __restrict__ a, int lda, const float* __restr
                 make_float4(low_of(acc[i][2 * j]), high_of(acc[i][2 * j]), low_of(acc[i][2 * j + 1]), high_of(acc[i][2 * j + 1]));
     }
     cg::this_cluster().sync();
-    const int rows_here = kRows / parts;  // (parts is 2 or 4, kRows a multiple of 32)
+    const int rows_here = kRows / parts;  // (parts is 2, 4 or 8, kRows a multiple of 32)
     for (int i = threadIdx.x; i < rows_here * kCols; i += kThreads) {
         const int r = part * rows_here + i / kCols, col = i % kCols;
         float sum = tiled_part(tiled_shared, 0)[r * kCols + col];
@@ -288,7 +297,7 @@ gemm_f32_few_kernel(const float* __restrict__ a, int lda, const float* __restric
 
 // Few rows (decode): one warp per output column, lanes stride over K, rows kept in registers.
 // The per-lane partial sums are combined in a fixed butterfly, so results are reproducible; the
-// order differs from the tiled kernel's single chain, which is rounding only.
+// order differs from the other kernels' sums of chains, which is rounding only.
 template <int kRows>
 __global__ void __launch_bounds__(256)
 gemv_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, float* __restrict__ c,
@@ -370,14 +379,14 @@ MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, floa
         gemv_f32_kernel<8><<<blocks, 256, 0, stream>>>(a, lda, w, ldw, c, ldc, m, n, k);
         return check_launch("gemv_f32");
     }
+    // Parts of K, by n and k alone, so that every m and every kernel gives a row the same bits: one chain of 2,048 to 8,192
+    // products per result leaves a matrix of few columns with too few of them at work (384 rows, 2,048 columns, K 8,192: 689 us
+    // whole, 322 in eight; 2,048 columns, K 2,048: 174 and 94), and shorter chains round less (1.6e-6 and 0.6e-6 from the sums
+    // in 64 bits).  Wide matrices gain less (16,384 columns: 596 us whole, 576 in four, 625 in eight).
+    int parts = n <= 8192 ? 8 : 4;
+    while (parts > 1 && k < 128 * parts) parts /= 2;
+    const int part_length = ((k + parts - 1) / parts + kFewStep - 1) / kFewStep * kFewStep;
     if (k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)a & 15) && !((uintptr_t)w & 15)) {
-        // Parts of K, by n and k alone, so that every m gives a row the same bits: one chain of 2,048 to 8,192 products per
-        // result leaves a matrix of few columns with too few of them at work (384 rows, 2,048 columns, K 8,192: 689 us whole,
-        // 322 in eight; 2,048 columns, K 2,048: 174 and 94), and shorter chains round less (1.6e-6 and 0.6e-6 from the sums in
-        // 64 bits).  Wide matrices gain less (16,384 columns: 596 us whole, 576 in four, 625 in eight).
-        int parts = n <= 8192 ? 8 : 4;
-        while (parts > 1 && k < 128 * parts) parts /= 2;
-        const int part_length = ((k + parts - 1) / parts + kFewStep - 1) / kFewStep * kFewStep;
         if (m <= kFewRows) {
             if (m <= 2) return launch_few<2>(a, lda, w, ldw, c, ldc, m, n, k, parts, part_length, stream);
             if (m <= 4) return launch_few<4>(a, lda, w, ldw, c, ldc, m, n, k, parts, part_length, stream);
@@ -391,6 +400,6 @@ MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, floa
     }
     const dim3 grid((n + kTileN - 1) / kTileN, (m + kTileM - 1) / kTileM);
     if (grid.y > 65535) return fail("gemm_f32: %d rows exceed the grid limit", m);
-    gemm_f32_kernel<<<grid, 256, 0, stream>>>(a, lda, w, ldw, c, ldc, m, n, k);
+    gemm_f32_kernel<<<grid, 256, 0, stream>>>(a, lda, w, ldw, c, ldc, m, n, k, part_length);
     return check_launch("gemm_f32");
 }

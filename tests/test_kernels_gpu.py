@@ -99,6 +99,21 @@ def test_gemm_f32_rows_of_pieces(cuda_device, m, n, k):
             assert torch.equal(ops.gemm_f32(a[:rows], w), out[:rows])  # whichever kernel and tile a row meets
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 72, 2048), (5, 200, 260), (40, 130, 1028), (70, 8200, 516), (130, 64, 2048)])
+def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
+    """Operands whose rows do not start on 16 bytes meet another kernel: the same chains over the same parts of K."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(13)
+    a, w = torch.randn(m, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    aligned = ops.gemm_f32(a, w)
+    for shifts in ((1, 0), (0, 3), (2, 1)):
+        moved = [torch.empty(t.shape[0], k + 4, device=cuda_device)[:, by:by + k] for t, by in zip((a, w), shifts)]
+        for to, t in zip(moved, (a, w)):
+            to.copy_(t)
+        assert torch.equal(ops.gemm_f32(*moved), aligned)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_swiglu_and_bias(cuda_device, dtype):
     from models_b200.kernels import ops
