@@ -109,7 +109,7 @@ struct UnitRows {
             float squares = fmaf(x[i].x, x[i].x, fmaf(x[i].y, x[i].y, fmaf(x[i].z, x[i].z, x[i].w * x[i].w)));
 #pragma unroll
             for (int offset = 1; offset < 16; offset <<= 1) squares += __shfl_xor_sync(0xffffffffu, squares, offset);
-            const float scale = factor / sqrtf(squares + unit_eps);
+            const float scale = row < count ? factor / sqrtf(squares + unit_eps) : 0.0f;  // (unit_eps may be zero)
             x[i] = make_float4(scale * x[i].x, scale * x[i].y, scale * x[i].z, scale * x[i].w);
             if (row >= kChunk) continue;
             split_four(x[i], planes + row * kRow + d, kPlane);

@@ -947,6 +947,42 @@ def test_gated_delta_chunks(cuda_device, dtype, vdim, lengths):
     close(chunk_out, out, dtype, scale=4.0)
 
 
+def _delta_call(lengths, heads, kv_heads, vdim, dtype, seed, unit_eps=1e-6, spoil=None):
+    """The gated delta rule over sequences of these lengths, from states that are not zero, as a function of max_q_len: (results, states)
+    by the walk (0) or in chunks.  `spoil` changes the convolved rows."""
+    from models_b200.kernels import ops
+
+    dim, g = 64, torch.Generator().manual_seed(seed)
+    tokens = sum(lengths)
+    conv = torch.randn(tokens, 2 * kv_heads * dim + heads * vdim, generator=g)
+    if spoil is not None:
+        spoil(conv)
+    conv, wide = conv.cuda(), torch.randn(tokens, 2 * heads + heads * vdim, generator=g).to(dtype).cuda()
+    decay = -torch.tensor([(0.01, 0.5, 4.0, 16.0)[h % 4] for h in range(heads)]).cuda()
+    dt_bias, gain = torch.randn(heads, generator=g).cuda(), (1 + 0.1 * torch.randn(vdim, generator=g)).cuda()
+    state0 = torch.randn(len(lengths), heads * dim * vdim, generator=g).cuda()
+    slots = torch.arange(len(lengths), dtype=torch.int32).cuda()
+    cu_q = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+
+    def call(max_q_len):
+        state, out = state0.clone(), torch.zeros(tokens, heads * vdim, dtype=dtype).cuda()
+        ops.gated_delta_scan(conv.clone(), 0, kv_heads * dim, 2 * kv_heads * dim, wide[:, :heads], wide[:, heads:2 * heads], wide[:, 2 * heads:], decay,
+                             dt_bias, gain, unit_eps, 1e-6, state, 0, slots, cu_q, heads, kv_heads, dim, vdim, out, 0.5, max_q_len=max_q_len)
+        return out.float(), state
+
+    return call
+
+
+@pytest.mark.parametrize("lengths", [[65], [100, 64, 3]])
+def test_gated_delta_chunks_without_an_epsilon(cuda_device, lengths):
+    """Keys that are divided by their own length alone: the empty rows of a chunk that is not full have none."""
+    call = _delta_call(lengths, 4, 2, 64, torch.float32, 5, unit_eps=0.0)
+    (out, state), (chunk_out, chunk_state) = call(0), call(max(lengths))
+    # the bounds of the test above
+    assert bool(out.isfinite().all()) and torch.allclose(chunk_state, state, rtol=1e-4, atol=1e-4)
+    close(chunk_out, out, torch.float32, scale=4.0)
+
+
 @pytest.mark.parametrize("vdim", [64, 128])
 @pytest.mark.parametrize("lengths", [[64], [1, 127, 64], [65, 0, 200, 63]])
 @pytest.mark.parametrize("whole", [True, False])
