@@ -15,7 +15,8 @@
 //      only serial part, two 64 x 64 x 16 products a chunk;
 //   3. delta_chunks_results: per (chunk, head) o, its norm, gain and gate.
 // The ratios G_i / G_j come from differences of sums of log g that are kept in 64 bits, so that a late token's ratios lose
-// nothing to the size of the sums.  What lies between products is float, and products take it whole (split_products.cuh).
+// nothing to the size of the sums.  What lies between products is float, and products take it whole (split_products.cuh).  A row that is
+// not finite reaches its own and later tokens alone, as in the walk, where it may come out as NaN for an infinity.
 // Against 64 bits, over steps of 64 to 2,048 tokens: the state is off by 1.2e-7 to 1.3e-7 of itself (the walk: 1.9e-7 to 3.3e-7), the
 // results by 1.4e-7 (2e-7).
 // One sequence of 2,048 tokens, 16 heads of 64 x 128: the walk's chain of 2,048 tokens is bound by its latency (618 us, and 30 for
@@ -73,14 +74,7 @@ __device__ __forceinline__ void store_pair(bf16* p, float a, float b) { *reinter
 // (a sequence of n tokens has ceil(n / 64) chunks, and floor(f / 64) + ceil(n / 64) <= floor((f + n) / 64) + 1).
 __device__ __forceinline__ size_t place_of(int first, int seq, int chunk) { return (size_t)(first / kChunk) + seq + chunk; }
 
-// Two floats, and four, as their parts.
-__device__ __forceinline__ void split_two(float a, float b, bf16* at, int plane) {
-    uint32_t hi, mid, lo;
-    split_pair(a, b, hi, mid, lo);
-    *reinterpret_cast<uint32_t*>(at) = hi;
-    *reinterpret_cast<uint32_t*>(at + plane) = mid;
-    *reinterpret_cast<uint32_t*>(at + 2 * plane) = lo;
-}
+// Four floats as their parts.
 __device__ __forceinline__ void split_four(float4 v, bf16* at, int plane) {
     uint2 hi, mid, lo;
     split_pair(v.x, v.y, hi.x, mid.x, lo.x);
@@ -280,14 +274,27 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
         for (int c = 0; c < block; ++c) accumulate(matrix_at + (16 * block * kRow + 16 * c) * 2, kPlane, 16 * c);
         __syncwarp();
         bf16* mine = solved + (row0 + group) * Plan::right_row + column0 + pair;
+        float (&z)[kTiles][4] = right[block];
+        bool finite = true;
 #pragma unroll
         for (int n = 0; n < kTiles; ++n) {
-            split_two(right[block][n][0] - acc[n][0], right[block][n][1] - acc[n][1], mine + 8 * n, Plan::right_plane);
-            split_two(right[block][n][2] - acc[n][2], right[block][n][3] - acc[n][3], mine + 8 * Plan::right_row + 8 * n, Plan::right_plane);
-            acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                z[n][i] -= acc[n][i];
+                finite = finite && has_parts(z[n][i]);
+                acc[n][i] = 0.0f;
+            }
+            split_two(z[n][0], z[n][1], mine + 8 * n, Plan::right_plane);
+            split_two(z[n][2], z[n][3], mine + 8 * Plan::right_row + 8 * n, Plan::right_plane);
         }
+        const bool whole = __all_sync(0xffffffffu, finite);
         __syncwarp();
-        accumulate(inverse_at + 16 * block * Plan::inverse_row * 2, Plan::inverse_plane, row0);
+        if (whole) {
+            accumulate(inverse_at + 16 * block * Plan::inverse_row * 2, Plan::inverse_plane, row0);
+        } else {
+            auto weight = [&](int row, int column) { return whole_one(inverse + (16 * block + row) * Plan::inverse_row + column, Plan::inverse_plane); };
+            causal_products(acc, weight, solved + row0 * Plan::right_row + column0 + pair, Plan::right_row, Plan::right_plane);
+        }
         __syncwarp();
         const int row = 16 * block + group;
 #pragma unroll
@@ -438,7 +445,9 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
     if (count <= 0) return;
     const size_t token0 = (size_t)first + chunk * kChunk;
     const size_t at = place_of(first, seq, chunk) * args.heads + head;
+    bool finite = true;
     auto bring = [&](const float* from) {
+        finite = true;
         constexpr int kPieces = 64 * V / 8 / kResultThreads;
         float x[kPieces][8];
 #pragma unroll
@@ -446,6 +455,8 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
             const int piece = tid + i * kResultThreads;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) finite = finite && has_parts(x[i][j]);
             store_parts(planes + Plan::wide + piece / (V / 8) * Plan::wide_row + piece % (V / 8) * 8, Plan::wide_plane, x[i]);
         }
     };
@@ -485,10 +496,11 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
     for (int n = 0; n < V / 16; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[n][i] *= from_start[i / 2];
-    __syncthreads();
+    const bool spoiled = __syncthreads_or(!finite);
+    const int last = spoiled ? 2 * warp - 2 : 2 * warp;  // (then the warp's own 16 tokens come below)
 #pragma unroll
     for (int n = 0; n < kChunk / 8; n += 2) {
-        if (n > 2 * warp) break;
+        if (n > last) break;
 #pragma unroll
         for (int m = n; m < n + 2; ++m)
 #pragma unroll
@@ -506,6 +518,13 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
             load_parts_turned(b, wide_at + (8 * n * Plan::wide_row + 8 * c) * 2, Plan::wide_plane);
             split_products(acc[c], acc[c + 1], a, b);
         }
+    }
+    if (spoiled) {
+        auto weight = [&](int token, int from) {
+            return whole_dot<kDim>(planes + Plan::queries + (16 * warp + token) * kRow, planes + Plan::keys + (16 * warp + from) * kRow, kPlane) *
+                   expf((float)(logs[16 * warp + token] - logs[16 * warp + from]));
+        };
+        causal_products(acc, weight, planes + Plan::wide + 16 * warp * Plan::wide_row + column0 + pair, Plan::wide_row, Plan::wide_plane);
     }
     // norm, gain and gate: a row's V results lie with four neighbouring lanes of two warps
 #pragma unroll

@@ -5,7 +5,8 @@
 //   o_i = a^(i + 1) S_0^T q_i + sum_(j <= i) a^(i - j) (q_i . k_j) v_j,     S_end = a^n S_0 + sum_j a^(n - 1 - j) k_j v_j^T
 // Three kernels: what every chunk adds to the state, a product per (chunk, head); the states that the chunks start from, element by
 // element in the chunks' order; every chunk's results, with the head's norm and gate where the caller wants them here.
-// The numbers between the first products and the last one are floats, and products take them whole (split_products.cuh).
+// The numbers between the first products and the last one are floats, and products take them whole (split_products.cuh).  A row that is
+// not finite reaches its own and later tokens alone, as in the walk, where it may come out as NaN for an infinity.
 // Against 64 bits, over steps of 64 to 2,048 tokens: the state is off by 6e-8 to 9e-8 of itself (the walk in runs: 0.9e-7 to 1.4e-7), the
 // raw results by 0.7e-7 to 1.1e-7 (0.8e-7 to 1.8e-7); with two parts the operands would be cut to 16 bits.
 // Three sequences of 2,048 tokens in all, 16 heads of 64 x 128 with activated projections: 208 us as the walk in runs (98, 70 and 40),
@@ -226,6 +227,7 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         }
     }
     __syncthreads();  // nobody reads the start any more
+    bool finite = true;
 #pragma unroll
     for (int i = 0; i < kPieces; ++i) {
         const int piece = tid + i * kThreads;
@@ -236,9 +238,12 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         if (args.input_act >= 0 && piece / (V / 8) < count)
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = gate_activation(args.input_act, x[j]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) finite = finite && has_parts(x[j]);
         store_parts(wide + piece / (V / 8) * kRow + piece % (V / 8) * 8, kPlane, x);
     }
-    __syncthreads();
+    const bool spoiled = __syncthreads_or(!finite);
+    const int last = spoiled ? 2 * warp - 2 : 2 * warp;  // (then the warp's own 16 tokens come below)
     const int row = 16 * warp + group;
 #pragma unroll
     for (int n = 0; n < V / 16; ++n)
@@ -246,7 +251,7 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         for (int i = 0; i < 4; ++i) acc[n][i] *= power[row + 8 * (i / 2) + 1];
 #pragma unroll
     for (int n = 0; n < kChunk / 8; n += 2) {
-        if (n > 2 * warp) break;
+        if (n > last) break;
 #pragma unroll
         for (int m = n; m < n + 2; ++m)
 #pragma unroll
@@ -264,6 +269,13 @@ retention_chunk_results_kernel(const RetentionArgs args) {
             load_parts_turned(b, wide_at + (8 * n * kRow + 8 * c) * 2, kPlane);
             split_products(acc[c], acc[c + 1], a, b);
         }
+    }
+    if (spoiled) {
+        auto weight = [&](int token, int from) {
+            return whole_dot<kDim>(queries + (16 * warp + token) * kKeyRow, keys + (16 * warp + from) * kKeyRow, kKeyPlane) *
+                   (args.key_scale * power[max(token - from, 0)]);
+        };
+        causal_products(acc, weight, wide + 16 * warp * kRow + column0 + pair, kRow, kPlane);
     }
     if (args.raw_out == nullptr) {  // a row's V results lie with four neighbouring lanes of two warps
 #pragma unroll

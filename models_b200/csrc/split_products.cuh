@@ -35,7 +35,14 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
     mid = *reinterpret_cast<const uint32_t*>(&m);
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
-// Eight floats into an operand's three planes.
+// Two floats, and eight, into an operand's three planes.
+__device__ __forceinline__ void split_two(float a, float b, bf16* at, int plane) {
+    uint32_t hi, mid, lo;
+    split_pair(a, b, hi, mid, lo);
+    *reinterpret_cast<uint32_t*>(at) = hi;
+    *reinterpret_cast<uint32_t*>(at + plane) = mid;
+    *reinterpret_cast<uint32_t*>(at + 2 * plane) = lo;
+}
 __device__ __forceinline__ void store_parts(bf16* to, int plane, const float (&x)[8]) {
     uint4 hi, mid, lo;
     split_pair(x[0], x[1], hi.x, mid.x, lo.x);
@@ -72,6 +79,39 @@ __device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], c
     mma_bf16(p1, a[0], b[0][2], b[0][3]);
 #pragma unroll
     for (int i = 0; i < 4; ++i) d0[i] += p0[i] + r0[i], d1[i] += p1[i] + r1[i];
+}
+
+// What has three finite parts.  (The largest bfloat16 number is a little smaller than the largest float.)
+__device__ __forceinline__ bool has_parts(float v) { return fabsf(v) < 3.3895e38f; }
+// A float from its parts, and the float dot product of two rows of parts.
+__device__ __forceinline__ float whole_one(const bf16* at, int plane) {
+    const float hi = __bfloat162float(at[0]);
+    return has_parts(hi) ? hi + __bfloat162float(at[plane]) + __bfloat162float(at[2 * plane]) : hi;
+}
+template <int kCount>
+__device__ float whole_dot(const bf16* a, const bf16* b, int plane) {
+    float sum = 0.0f;
+#pragma unroll 1
+    for (int i = 0; i < kCount; ++i) sum = fmaf(whole_one(a + i, plane), whole_one(b + i, plane), sum);
+    return sum;
+}
+// acc += w . v for the weights weight(token, earlier token) of 16 tokens on themselves, where a row of v may not be finite: the zeros that
+// stand for later tokens' weights would make NaN of it in a product, and it must reach its own token and later ones alone.  In float,
+// token by token, slow; `values`: the thread's pair of columns of the first of the 16 rows.
+template <int kTiles, typename Weight>
+__device__ __forceinline__ void causal_products(float (&acc)[kTiles][4], Weight weight, const bf16* values, int row, int plane) {
+    const int group = (threadIdx.x & 31) >> 2;
+#pragma unroll 1
+    for (int j = 0; j < 16; ++j) {
+        const bf16* at = values + j * row;
+        const float upper = j <= group ? weight(group, j) : 0.0f, lower = j <= group + 8 ? weight(group + 8, j) : 0.0f;
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n) {
+            const float x = whole_one(at + 8 * n, plane), y = whole_one(at + 8 * n + 1, plane);
+            if (j <= group) acc[n][0] = fmaf(upper, x, acc[n][0]), acc[n][1] = fmaf(upper, y, acc[n][1]);
+            if (j <= group + 8) acc[n][2] = fmaf(lower, x, acc[n][2]), acc[n][3] = fmaf(lower, y, acc[n][3]);
+        }
+    }
 }
 
 }  // namespace mb

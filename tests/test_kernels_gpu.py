@@ -983,6 +983,59 @@ def test_gated_delta_chunks_without_an_epsilon(cuda_device, lengths):
     close(chunk_out, out, torch.float32, scale=4.0)
 
 
+SPOILED = [("v", 5), ("v", 77), ("v", 90), ("k", 66), ("k", 127), ("q", 20)]  # a row that is not finite: within its 16 tokens, chunk and sequence
+
+
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("part,at", SPOILED)
+def test_gated_delta_chunks_keep_earlier_tokens_apart(cuda_device, vdim, value, part, at):
+    """A row that is not finite spoils its own sequence from its token on, as in the walk; earlier tokens and other sequences give what they
+    give without it."""
+    lengths = [130, 70]
+
+    def spoil(conv):
+        conv[at, {"q": 3, "k": 64 + 7, "v": 128 + vdim + 9}[part]] = value
+
+    clean, clean_state = _delta_call(lengths, 2, 1, vdim, torch.float32, 6)(130)
+    out, state = _delta_call(lengths, 2, 1, vdim, torch.float32, 6, spoil=spoil)(130)
+    # (sixteen tokens beside such a row are added up in another order)
+    close(out[:at], clean[:at], torch.float32, scale=4.0)
+    assert torch.equal(out[130:], clean[130:]) and torch.equal(state[1], clean_state[1])
+    assert not bool(out[at].isfinite().all())
+
+
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("part,at", SPOILED)
+def test_retention_chunks_keep_earlier_tokens_apart(cuda_device, vdim, value, part, at):
+    """The same of retention; in its raw results a value that is not finite spoils its own column alone."""
+    from models_b200.kernels import ops
+
+    heads, dim, lengths = 2, 64, [130, 70]
+    g = torch.Generator().manual_seed(23)
+    proj = torch.randn(sum(lengths), heads * (2 * dim + 2 * vdim), generator=g).bfloat16()
+    decay, state0 = torch.tensor([0.97, 0.5]).cuda(), torch.randn(2, heads, dim, vdim, generator=g).cuda()
+    slots, cu_q, positions = (torch.tensor(v, dtype=torch.int32).cuda() for v in ([0, 1], [0, 130, 200], [0] * 200))
+    found = []
+    for spoiled in (False, True):
+        rows = proj.clone()
+        if spoiled:
+            rows[at, {"q": 3, "k": heads * dim + 7, "v": 2 * heads * dim + 9}[part]] = value
+        q, k, v, _ = rows.cuda().split([heads * dim, heads * dim, heads * vdim, heads * vdim], dim=1)
+        state, raw = state0.clone(), torch.zeros(200, heads * vdim).cuda()
+        ops.retention_scan(q, k, v, None, positions, None, None, 0, decay, 0.3, 1e-6, state, slots, cu_q, heads, dim, vdim, None, 0.5, 130, raw_out=raw)
+        found.append((raw, state))
+    (clean, clean_state), (raw, state) = found
+    touched = torch.zeros_like(clean, dtype=torch.bool)
+    touched[at:130, :vdim] = True
+    if part == "v":
+        touched[:, :9] = touched[:, 10:] = False
+    close(torch.where(touched, clean, raw), clean, torch.float32, scale=4.0 * float(clean.abs().max()))
+    assert torch.equal(raw[130:], clean[130:]) and torch.equal(state[1], clean_state[1])
+    assert not bool(raw[at, :vdim].isfinite().all())
+
+
 @pytest.mark.parametrize("vdim", [64, 128])
 @pytest.mark.parametrize("lengths", [[64], [1, 127, 64], [65, 0, 200, 63]])
 @pytest.mark.parametrize("whole", [True, False])
