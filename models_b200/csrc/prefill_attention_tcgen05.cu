@@ -14,7 +14,7 @@
 // columns (a query may hold anything finite there), and a key may have MB_TURNED_DIM coordinates more that all heads share
 // ([tokens][MB_TURNED_DIM]), the query's own ones beside them ([tokens][heads * MB_TURNED_DIM]), zeros behind their real ones.
 // A step on top of cached positions reads such rows as well, made of the cache's before: every sequence's keys then lie `key_rows`
-// rows apart, from its position 0 on.
+// rows apart, from its position 0 on, or with `key_window` from the multiple of 64 at or before the first position that such a window sees.
 //
 // A block takes 128 consecutive query tokens of one head and walks the visible cache pages (64 keys
 // each).  Its six warps have three roles:
@@ -230,7 +230,8 @@ struct AttentionArgs {
     const bf16* gate;     // [tokens][heads] (row stride gate_stride) or null: head h's result is multiplied by sigmoid(gate[t][h])
     int gate_stride;
     int gate_element;     // != 0: the gate is [tokens][heads * value_columns], element by element
-    int key_rows;         // kContiguous: 0, or how many rows of keys and values a sequence has (from its position 0 on)
+    int key_rows;         // kContiguous: 0, or how many rows of keys and values a sequence has (see above)
+    int key_window;
     // kShaped
     const float* head_scale;  // [heads] factors on the scores, or null
     float softcap;            // 0: scores are not bounded
@@ -277,6 +278,8 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     const int first_needed = (window > 0 && pos0 - window + 1 > 0) ? pos0 - window + 1 : 0;
     const int t_begin = first_needed / kKeys, t_end = last_pos / kKeys + 1;
     const int pages = t_end - t_begin;
+    // the page that a sequence's `key_rows` rows begin with: at most the first tile's t_begin
+    const int seen = kContiguous && args.key_window > 0 ? kv_len - q_len - args.key_window + 1 : 0, t_first = seen > 0 ? seen / kKeys : 0;
     const int kv_head = head / (args.heads / args.kv_heads);
 
     if (threadIdx.x == 0) {
@@ -320,7 +323,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             for (int t = 0; t < pages; ++t) {
                 const int stage = t % kStages;
                 const uint32_t free_parity = ((t / kStages) & 1) ^ 1;
-                const int row = kContiguous ? (args.key_rows > 0 ? seq * args.key_rows : q_begin) + (t_begin + t) * kKeys : (table[t_begin + t] * args.kv_heads + kv_head) * kKeys;
+                const int row = kContiguous ? (args.key_rows > 0 ? seq * args.key_rows : q_begin) + (t_begin - t_first + t) * kKeys : (table[t_begin + t] * args.kv_heads + kv_head) * kKeys;
                 const int key_column = kContiguous ? kv_head * KD : 0, value_column = kContiguous ? kv_head * VD : 0;
                 if (!mbar_wait(k_empty + 8 * stage, free_parity, 1)) break;
                 mbar_expect_tx(k_full + 8 * stage, kKeyTileBytes);
@@ -625,7 +628,7 @@ MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int 
     if (int status = make_map(&map_q, q, total_rows, heads * KD, q_row_stride, kQRows)) return status;
     if (int status = make_map(&map_k, k_pool, pool_pages * kv_heads * kKeys, KD, KD, kKeys)) return status;
     if (int status = make_map(&map_v, v_pool, pool_pages * kv_heads * kKeys, VD, VD, kKeys)) return status;
-    const AttentionArgs args{(bf16*)out, out_row_stride, block_table, max_blocks, cu_q, kv_lens, heads, kv_heads, window, scale, KD, VD, nullptr, 0, 0, 0,
+    const AttentionArgs args{(bf16*)out, out_row_stride, block_table, max_blocks, cu_q, kv_lens, heads, kv_heads, window, scale, KD, VD, nullptr, 0, 0, 0, 0,
                              head_scale, softcap, sink, turn_cos, turn_sin};
     return launch_prefill(map_q, map_k, map_v, map_q, map_k, args, sequences, max_q_len, stream);
 }
@@ -635,12 +638,12 @@ MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int 
 // be finite; q_columns: columns of a row in all); q_turned [total_rows][heads * RD], k_turned [total_rows][RD] (RD > 0).  k, v: rows of
 // total_rows tokens with kv_heads heads of KD and of VD (row stride kv_row_stride).  out: [total_rows][heads * value_columns].
 // gate (or null): bfloat16 [total_rows][heads], the heads' results are multiplied by its sigmoid; gate_element: [total_rows][heads *
-// value_columns], 16-byte aligned rows.  key_rows n > 0 (a multiple of 64): k, v and k_turned have key_total rows, n for every sequence,
-// of which kv_lens say how many are there; the step's tokens are the last of them.
+// value_columns], 16-byte aligned rows.  key_rows n > 0 (a multiple of 64): k, v and k_turned have key_total rows, n for every sequence, which
+// begin where the comment at the top says; kv_lens say how many positions there are, the step's tokens the last of them.
 MB_EXPORT int mb_prompt_attention_tcgen05(const void* q, int q_row_stride, int q_head_columns, int q_columns, const void* q_turned,
                                           const void* k, const void* v, int kv_row_stride, const void* k_turned, int total_rows, void* out,
                                           int out_row_stride, int value_columns, const void* gate, int gate_stride, int gate_element,
-                                          int key_rows, int key_total, const int* cu_q, const int* kv_lens, int sequences, int max_q_len, int heads, int kv_heads, int window,
+                                          int key_rows, int key_window, int key_total, const int* cu_q, const int* kv_lens, int sequences, int max_q_len, int heads, int kv_heads, int window,
                                           float scale, cudaStream_t stream) {
     if (sequences <= 0 || max_q_len <= 0) return 0;
     if (int status = check_prefill(q, q_row_stride, out, out_row_stride, sequences, max_q_len, heads, kv_heads)) return status;
@@ -650,6 +653,8 @@ MB_EXPORT int mb_prompt_attention_tcgen05(const void* q, int q_row_stride, int q
         return fail("prompt_attention_tcgen05: keys, values and shared coordinates must be there and start on 16-byte boundaries");
     if (key_rows < 0 || key_rows % kKeys || (key_rows > 0 && (long long)key_rows * sequences > key_total))
         return fail("prompt_attention_tcgen05: %d rows of keys do not hold %d for each of %d sequences", key_total, key_rows, sequences);
+    if (key_window < 0 || (key_window > 0 && (key_rows == 0 || window == 0 || key_window < window)))
+        return fail("prompt_attention_tcgen05: rows of keys for a window of %d do not hold what one of %d sees", key_window, window);
     if (gate_element && (!gate || gate_stride % 8 || ((uintptr_t)gate & 15))) return fail("prompt_attention_tcgen05: a gate of elements needs 16-byte aligned rows");
     if (key_rows == 0) key_total = total_rows;
     CUtensorMap map_q, map_k, map_v, map_q_turned, map_k_turned;
@@ -663,7 +668,7 @@ MB_EXPORT int mb_prompt_attention_tcgen05(const void* q, int q_row_stride, int q
         if (int status = make_map(&map_k_turned, k_turned, key_total, RD, RD, kKeys)) return status;
     }
     const AttentionArgs args{(bf16*)out, out_row_stride, nullptr, 0, cu_q, kv_lens, heads, kv_heads, window, scale, q_head_columns, value_columns,
-                             (const bf16*)gate, gate_stride, gate_element, key_rows, nullptr, 0.0f, 0, nullptr, nullptr};
+                             (const bf16*)gate, gate_stride, gate_element, key_rows, key_window, nullptr, 0.0f, 0, nullptr, nullptr};
     return launch_prefill(map_q, map_k, map_v, map_q_turned, map_k_turned, args, sequences, max_q_len, stream);
 }
 #endif

@@ -846,14 +846,15 @@ def float_weight_attention_takes(q: torch.Tensor, out: torch.Tensor, k_pool: tor
 def prompt_attention(q: torch.Tensor, q_tail: Optional[torch.Tensor], k: torch.Tensor, v: torch.Tensor, k_tail: Optional[torch.Tensor],
                      out: torch.Tensor, cu_q: torch.Tensor, kv_lens: torch.Tensor, max_q_len: int, heads: int, head_columns: int,
                      value_columns: int, scale: float, gate: Optional[torch.Tensor] = None, window: int = 0,
-                     gate_kind: str = "head", key_rows: int = 0) -> None:
+                     gate_kind: str = "head", key_rows: int = 0, key_window: int = 0) -> None:
     """Causal softmax attention of prompts that start their sequences, on the tcgen05 tensor cores with float weights: every key comes
     from the step's own rows.  bfloat16: k [T, heads * KD] and v [T, heads * VD] (column slices with one row stride; KD, VD multiples
     of 64, heads padded with zero columns), k_tail [T, RD] shared by all heads and q_tail [T, heads * RD] (or None, None); q [T, ...] holds
     head h's own coordinates from column h * head_columns on; out [T, heads * value_columns]; gate [T, heads]: head h's result is
     multiplied by its sigmoid, or, gate_kind "element", a gate [T, heads * value_columns] element by element.  `window` n > 0: query i
     sees key j only if i - j < n.  `key_rows` n > 0 (a multiple of 64): a step on top of cached positions; k, v and k_tail have n rows for
-    every sequence, its positions from 0 on, the step's own ones last."""
+    every sequence, its positions from 0 on, the step's own ones last; `key_window` n > 0 (at least `window`): from the multiple of 64 at or
+    before the first position that a window of n sees (what `latent_gather` leaves)."""
     _cuda(q, q_tail, k, v, k_tail, out, cu_q, kv_lens, gate)
     _int32(cu_q, "cu_q")
     _int32(kv_lens, "kv_lens")
@@ -882,7 +883,7 @@ def prompt_attention(q: torch.Tensor, q_tail: Optional[torch.Tensor], k: torch.T
     _run(lib, lib.mb_prompt_attention_tcgen05(
         _p(q), q.stride(0), int(head_columns), q.shape[1], _p(q_tail), _p(k), _p(v), k.stride(0), _p(k_tail), rows, _p(out), out.stride(0),
         int(value_columns), _p(gate), gate.stride(0) if gate is not None else 0,
-        1 if gate is not None and gate_kind == "element" else 0, int(key_rows), keys, _p(cu_q), _p(kv_lens), kv_lens.numel(), int(max_q_len), heads,
+        1 if gate is not None and gate_kind == "element" else 0, int(key_rows), int(key_window), keys, _p(cu_q), _p(kv_lens), kv_lens.numel(), int(max_q_len), heads,
         heads, int(window), ctypes.c_float(scale), _stream()))
 
 
@@ -1161,21 +1162,26 @@ def latent_rows(k: torch.Tensor, gain: torch.Tensor, turned: int, cos: Optional[
     return own, tail, q_tail
 
 
-def latent_gather(k_pool: torch.Tensor, latent: int, padded: int, block_table: torch.Tensor, kv_lens: torch.Tensor, rows_per: int):
-    """The rows that a latent attention's sequences hold in their cache pool [pages, 1, page_size, latent + turned] (bfloat16), `rows_per`
-    (a multiple of 64) for every sequence, from its position 0 on: latents [sequences * rows_per, latent] and, where there is a tail,
-    tails [sequences * rows_per, padded] with zeros behind the turned numbers.  Rows behind a sequence's last 64 are not written."""
-    _cuda(k_pool, block_table, kv_lens)
+def latent_gather(k_pool: torch.Tensor, latent: int, padded: int, block_table: torch.Tensor, kv_lens: torch.Tensor, rows_per: int,
+                  cu_q: Optional[torch.Tensor] = None, window: int = 0):
+    """The rows of a latent attention's sequences in their cache pool [pages, 1, page_size, latent + turned] (bfloat16), `rows_per`
+    (a multiple of 64) for every sequence, from its position 0 on, or with a `window` (and the step's `cu_q`) from the multiple of 64 at or
+    before the first position that the step's tokens see: latents [sequences * rows_per, latent] and, where there is a tail, tails
+    [sequences * rows_per, padded] with zeros behind the turned numbers.  Rows behind a sequence's last 64 are not written."""
+    _cuda(k_pool, block_table, kv_lens, cu_q)
     _int32(block_table, "block_table")
     _int32(kv_lens, "kv_lens")
+    _int32(cu_q, "cu_q")
     turned, sequences = k_pool.shape[3] - latent, kv_lens.numel()
     if k_pool.dtype != torch.bfloat16 or k_pool.dim() != 4 or k_pool.shape[1] != 1 or not k_pool.is_contiguous() or turned < 0:
         raise KernelError(f"latent_gather: the pool must be contiguous bfloat16 [pages, 1, page_size, latent + turned], got {tuple(k_pool.shape)} {k_pool.dtype}")
+    if window and (cu_q is None or cu_q.numel() != sequences + 1):
+        raise KernelError("latent_gather: a window needs the step's cu_q")
     latents = torch.empty((sequences * rows_per, latent), dtype=k_pool.dtype, device=k_pool.device)
     tails = torch.empty((sequences * rows_per, padded), dtype=k_pool.dtype, device=k_pool.device) if turned else None
     lib = load_library("mb_latent_gather", ["latent_gather.cu"])
-    _run(lib, lib.mb_latent_gather(_p(k_pool), latent, turned, int(padded), _p(block_table), block_table.shape[1], k_pool.shape[2], _p(kv_lens),
-                                   sequences, int(rows_per), _p(latents), _p(tails), _stream()))
+    _run(lib, lib.mb_latent_gather(_p(k_pool), latent, turned, int(padded), _p(block_table), block_table.shape[1], k_pool.shape[2], _p(cu_q),
+                                   _p(kv_lens), sequences, int(window), int(rows_per), _p(latents), _p(tails), _stream()))
     return latents, tails
 
 

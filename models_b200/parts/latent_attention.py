@@ -41,6 +41,7 @@ from .split import SplitPart
 # the kernel's least step on.
 EXPANDED_TOKENS = 512
 EXPANDED_ROWS = 16  # most rows gathered for a token
+EXPANDED_BYTES = 1 << 30  # most workspace for the gathered rows and the keys and values made of them
 
 
 def _whole(size: int) -> int:
@@ -150,8 +151,13 @@ class LatentAttentionMixer(SplitPart, Mixer):
         if fresh:
             return 0
         # (the page tables' width and not the lengths: a captured step replays for every length its class holds)
-        per = -(-group.block_table.shape[1] * run.k_pool.shape[2] // 64) * 64
-        fits = run.k_pool.shape[2] % 64 == 0 and self.turned % 8 == 0 and per * batch.kv_lens.numel() <= EXPANDED_ROWS * mid.shape[0]
+        seen = group.block_table.shape[1] * run.k_pool.shape[2]
+        if self.spec.window:  # nobody sees more: the window's positions before the first token, the step's own, and what is left of a first 64
+            seen = min(seen, self.spec.window - 1 + batch.max_q_len + 63)
+        per = -(-seen // 64) * 64
+        rows, width = per * batch.kv_lens.numel(), self.expand.shape[0] + self.spec.latent_dim + _whole(self.turned)
+        fits = (run.k_pool.shape[2] % 64 == 0 and self.turned % 8 == 0 and rows <= EXPANDED_ROWS * mid.shape[0]
+                and rows * width * self.expand.element_size() <= EXPANDED_BYTES)
         return per if fits else None
 
     def _expanded(self, q, down, gate, mid, batch, group, run: RunContext, cos, sin, key_rows: int) -> None:
@@ -161,11 +167,13 @@ class LatentAttentionMixer(SplitPart, Mixer):
         own, tail, q_tail = ops.latent_rows(down, self.latent_gain, self.turned, cos, sin, batch.positions, s.eps, run.k_pool, group.slot_mapping,
                                             q=q, heads=s.num_heads, head_columns=s.head_dim + self.turned, padded=_whole(self.turned))
         if key_rows:
-            own, tail = ops.latent_gather(run.k_pool, s.latent_dim, _whole(self.turned), group.block_table, batch.kv_lens, key_rows)
+            own, tail = ops.latent_gather(run.k_pool, s.latent_dim, _whole(self.turned), group.block_table, batch.kv_lens, key_rows, batch.cu_q,
+                                          s.window or 0)
         expanded = linear(own, self.expand, own.dtype)
         at = s.num_heads * _whole(s.head_dim)
         ops.prompt_attention(q, q_tail, expanded[:, :at], expanded[:, at:], tail, mid, batch.cu_q, batch.kv_lens, batch.max_q_len, s.num_heads,
-                             s.head_dim + self.turned, s.value_dim, s.scale, gate, s.window or 0, s.gate_kind if gate is not None else "head", key_rows)
+                             s.head_dim + self.turned, s.value_dim, s.scale, gate, s.window or 0, s.gate_kind if gate is not None else "head", key_rows,
+                             (s.window or 0) if key_rows else 0)
 
     def inner(self, proj: torch.Tensor, mid: torch.Tensor, batch, run: RunContext, scale: float = 1.0) -> None:
         s = self.spec

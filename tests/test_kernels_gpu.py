@@ -1267,3 +1267,55 @@ def test_latent_prompts_expand_the_rows_they_see(cuda_device, monkeypatch, query
         outs.append(out.float())
     # keys, values and queries pass through bfloat16 at other places: four roundings' worth
     assert float((outs[0] - outs[1]).norm()) <= 4 * 2.0 ** -8 * float(outs[1].norm())
+
+
+@pytest.mark.parametrize("window,past,q_lens", [(90, [300, 40], [150, 129]), (64, [127, 641], [33, 65]), (1, [200, 0], [70, 64])])
+def test_latent_prompts_expand_only_what_their_window_sees(cuda_device, monkeypatch, window, past, q_lens):
+    """On top of a cache that gave pages back: the rows gathered begin at the window's first page, and what lies before it (not a number here)
+    is not touched; beyond the workspace's bound a step stays in the latent space."""
+    from models_b200.cache import KvCache
+    from models_b200.config.specs import LatentAttentionSpec, RopeSpec
+    from models_b200.engine.batch import build_step_batch
+    from models_b200.kernels import ops
+    from models_b200.parts import RunContext, Runtime, build_part, latent_attention
+
+    monkeypatch.setattr(latent_attention, "EXPANDED_TOKENS", 0)
+    width, heads, dim, vdim, rank, turned = 256, 4, 64, 128, 128, 64
+    roles = ["down_q", "down_q_norm", "up_q", "down", "down_norm", "up_k", "up_v", "o"]
+    spec = LatentAttentionSpec(hidden_size=width, num_heads=heads, head_dim=dim, value_dim=vdim, latent_dim=rank, scale=(dim + turned) ** -0.5, eps=1e-6,
+                               gated=False, weights={r: r for r in roles}, query_latent=128, position=RopeSpec(turned, 1e4, "half"), window=window)
+    outs, gathered, plain_gather = [], [], ops.latent_gather
+
+    def gather(*args):
+        rows = plain_gather(*args)
+        gathered.append((args[5], rows))
+        return rows
+
+    monkeypatch.setattr(ops, "latent_gather", gather)
+    for most in (latent_attention.EXPANDED_BYTES, 0):
+        monkeypatch.setattr(latent_attention, "EXPANDED_BYTES", most)
+        mixer = build_part("mixer", spec, Runtime(torch.device("cuda:0"), "bfloat16", max_positions=1024))
+        draw = torch.Generator().manual_seed(5)
+        mixer.load({p.name: (torch.randn(p.shape, generator=draw) * p.shape[-1] ** -0.5).bfloat16() if len(p.shape) > 1
+                    else 1 + 0.1 * torch.randn(p.shape, generator=draw) for p in mixer.parameters()})
+        cache = KvCache([mixer.kv_request()], [None], 64 * 30, len(q_lens))
+        cache.allocate_storage(lambda shape: torch.full(shape, float("nan"), dtype=torch.bfloat16, device="cuda:0"))
+        run = RunContext(run=0)
+        run.group, run.k_pool, run.v_pool = cache.pools(0)
+        slots = [cache.open_slot() for _ in q_lens]
+        rows = torch.Generator().manual_seed(6)
+        for counts in (past, q_lens):
+            entries = [(s, n) for s, n in zip(slots, counts) if n]
+            cache.append(entries)
+            batch = build_step_batch(cache, [(s, [0] * n, []) for s, n in entries], torch.device("cuda:0"))
+            cache.commit(entries)
+            out = mixer.forward(torch.randn(sum(n for _, n in entries), width, generator=rows).bfloat16().cuda(), batch, run)
+        outs.append(out.float())
+    assert len(gathered) == 1  # (the second mixer's steps stay in the latent space)
+    per, (latents, tails) = gathered[0]
+    assert per % 64 == 0 and per <= max(64, min(-(-max(a + b for a, b in zip(past, q_lens)) // 64) * 64, window + max(q_lens) + 126))
+    for i, (before, n) in enumerate(zip(past, q_lens)):
+        first = max(0, before - window + 1) // 64 * 64
+        for kept in (latents, tails):
+            assert bool(kept[i * per:i * per + before + n - first].isfinite().all())
+    assert bool(outs[0].isfinite().all()) and float((outs[0] - outs[1]).norm()) <= 4 * 2.0 ** -8 * float(outs[1].norm())
