@@ -578,8 +578,6 @@ static int launch_chunks(const DeltaChunkArgs& args, int sequences, int chunks, 
 
 using namespace mb;
 
-MB_EXPORT int mb_gated_delta_chunk_tokens() { return kChunk; }
-
 // Arguments as mb_gated_delta_scan's, with key heads of 64 numbers and value heads of 64 or 128; conv is only read.  scratch: floats,
 // (places * heads) * (2 * 64 * vdim + 3 * 64 * 64 + 128), 16-byte aligned, with places = tokens / 64 + sequences.
 MB_EXPORT int mb_gated_delta_chunks(const float* conv, int conv_stride, const void* a_in, const void* b_in, const void* gate_in, int in_stride,

@@ -1350,6 +1350,13 @@ def gated_delta_chunks_library():
 
 
 DELTA_CHUNK_MIN_ROWS = 64  # steps that bring fewer tokens to every sequence are walked token by token
+DELTA_CHUNK_BYTES = 1 << 30  # most scratch: a token of 16 heads of 64 and 128 takes 29 KB, where the walk takes 8
+
+
+def gated_delta_chunk_floats(tokens: int, sequences: int, heads: int, vdim: int) -> int:
+    """The scratch of a step in chunks: a place for each of a sequence's chunks of 64 tokens, and for each head there x or u, the start, y and
+    the weighted keys in three parts, the sums of log g (two floats each)."""
+    return (tokens // 64 + sequences) * heads * (2 * 64 * vdim + 3 * 64 * 64 + 128)
 
 
 def gated_delta_chunks_takes(conv: torch.Tensor, gate_in: torch.Tensor, gain: torch.Tensor, out: torch.Tensor, dim: int, vdim: int, parts_at,
@@ -1434,10 +1441,10 @@ def gated_delta_scan(conv: torch.Tensor, q_at: int, k_at: int, v_at: int, a_in: 
         if t.dtype != torch.float32 or t.numel() != n or not t.is_contiguous():
             raise KernelError(f"gated_delta_scan: {name} must be contiguous float32 of {n} elements")
     rows, stride = _state_rows(state, state_offset, heads * dim * vdim, "gated_delta_scan")
-    if gated_delta_chunks_takes(conv, gate_in, gain, out, dim, vdim, (q_at, k_at, v_at), max_q_len):
+    floats = gated_delta_chunk_floats(tokens, cu_q.numel() - 1, heads, vdim)
+    if 4 * floats <= DELTA_CHUNK_BYTES and gated_delta_chunks_takes(conv, gate_in, gain, out, dim, vdim, (q_at, k_at, v_at), max_q_len):
         lib = gated_delta_chunks_library()
-        places = tokens // lib.mb_gated_delta_chunk_tokens() + cu_q.numel() - 1
-        scratch = torch.empty((places * heads * (2 * 64 * vdim + 3 * 64 * 64 + 128),), dtype=torch.float32, device=conv.device)
+        scratch = torch.empty((floats,), dtype=torch.float32, device=conv.device)
         _run(lib, lib.mb_gated_delta_chunks(_p(conv), conv.stride(0), _p(a_in), _p(b_in), _p(gate_in), a_in.stride(0), _code(out.dtype), _p(decay),
                                             _p(dt_bias), _p(gain), ctypes.c_float(unit_eps), ctypes.c_float(eps), rows, stride, _p(slots),
                                             _p(cu_q), cu_q.numel() - 1, tokens, int(max_q_len), _p(scratch), _p(out), out.stride(0),

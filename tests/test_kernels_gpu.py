@@ -983,6 +983,18 @@ def test_gated_delta_chunks_without_an_epsilon(cuda_device, lengths):
     close(chunk_out, out, torch.float32, scale=4.0)
 
 
+def test_gated_delta_steps_beyond_the_scratch_bound_are_walked(cuda_device, monkeypatch):
+    from models_b200.kernels import ops
+
+    call = _delta_call([130, 70], 2, 1, 128, torch.bfloat16, 7)
+    # three chunks of one sequence and two of the other: what the launcher asks for
+    assert ops.gated_delta_chunk_floats(200, 2, 2, 128) == 5 * 2 * (2 * 64 * 128 + 3 * 64 * 64 + 128)
+    walked, chunks = call(0), call(130)
+    assert not torch.equal(walked[1], chunks[1])
+    monkeypatch.setattr(ops, "DELTA_CHUNK_BYTES", 4 * ops.gated_delta_chunk_floats(200, 2, 2, 128) - 1)
+    assert all(torch.equal(a, b) for a, b in zip(call(130), walked))
+
+
 SPOILED = [("v", 5), ("v", 77), ("v", 90), ("k", 66), ("k", 127), ("q", 20)]  # a row that is not finite: within its 16 tokens, chunk and sequence
 
 
