@@ -920,7 +920,7 @@ def test_wide_qkv_product_with_rotation_and_cache_write(cuda_device, batch, head
 @pytest.mark.parametrize("vdim", [64, 128])
 @pytest.mark.parametrize("lengths", [[64], [1, 127, 64], [65, 0, 200, 63]])
 def test_gated_delta_chunks(cuda_device, dtype, vdim, lengths):
-    """Chunks of 64 against the walk token by token, from states that are not zero: the same float arithmetic in another order."""
+    """Chunks of 64 against the walk token by token and against the recurrence in 64 bits, from states that are not zero."""
     from models_b200.kernels import ops
 
     heads, kv_heads, dim = 4, 2, 64
@@ -941,10 +941,32 @@ def test_gated_delta_chunks(cuda_device, dtype, vdim, lengths):
                              slots, cu_q, heads, kv_heads, dim, vdim, out, 0.5, max_q_len=most)
         found.append((out.float(), state))
     (out, state), (chunk_out, chunk_state) = found
+    assert ops.gated_delta_chunks_takes(conv, gate, gain, out.to(dtype), dim, vdim, (0, kv_heads * dim, 2 * kv_heads * dim), max(lengths))
     # sums of at most 64 + 64 products a token either way; the states' numbers are of size one to ten
     assert torch.allclose(chunk_state, state, rtol=1e-4, atol=1e-4)
     assert torch.equal(chunk_state[:, :3], state0[:, :3]) and torch.equal(chunk_state[-1], state0[-1])
     close(chunk_out, out, dtype, scale=4.0)
+    # A chunk adds a number up over some 64 + 64 products, whose roundings of 2^-24 grow like the root of their count: 2^-20.5, and what
+    # the gates' functions and the chunks before bring, four times that in all.  (Measured: 1.3e-7.  Operands of two bfloat16
+    # parts would be off by 2^-17.)
+    bound = 2.0 ** -18.5
+    q, k, v = (t.double().cpu().view(tokens, n, -1) for t, n in zip(conv.split([kv_heads * dim, kv_heads * dim, heads * vdim], 1), (kv_heads, kv_heads, heads)))
+    q, k = (t.repeat_interleave(heads // kv_heads, 1) / (t.repeat_interleave(heads // kv_heads, 1).square().sum(-1, keepdim=True) + 1e-6).sqrt() for t in (q, k))
+    forget = torch.exp(decay.double() * torch.nn.functional.softplus(a_in.double() + dt_bias.double())).cpu()
+    beta, results = torch.sigmoid(b_in.double()).cpu(), torch.empty(tokens, heads, vdim, dtype=torch.float64)
+    for i, n in enumerate(lengths):
+        mine = slice(3, 3 + heads * dim * vdim)
+        S = state0[slots[i], mine].double().cpu().view(heads, dim, vdim)
+        for t in range(int(cu_q[i]), int(cu_q[i]) + n):
+            S = S * forget[t, :, None, None]
+            S = S + k[t, :, :, None] * (beta[t, :, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t])))[:, None, :]
+            results[t] = torch.einsum("hdv,hd->hv", S, q[t]) / 8.0
+        got = chunk_state[slots[i], mine].double().cpu().view(heads, dim, vdim)
+        assert float((got - S).norm()) <= bound * float(S.norm())
+    results = 0.5 * results / (results.square().mean(-1, keepdim=True) + 1e-6).sqrt() * gain.double().cpu()
+    results = results.flatten(1) * torch.nn.functional.silu(gate.double().cpu())
+    bound = bound if dtype == torch.float32 else 2.0 ** -8  # (a result's own rounding)
+    assert float((chunk_out.double().cpu() - results).norm()) <= bound * float(results.norm())
 
 
 def _delta_call(lengths, heads, kv_heads, vdim, dtype, seed, unit_eps=1e-6, spoil=None):
@@ -1079,6 +1101,7 @@ def test_retention_chunks(cuda_device, vdim, lengths, whole):
                            input_activation="silu" if whole else None, raw_out=raw)
         found.append(((raw if whole else out).float(), state))
     (out, state), (chunk_out, chunk_state) = found
+    assert ops.retention_chunks_takes(q, k, v, None if whole else gate, None if whole else out.bfloat16(), out if whole else None, state, dim, vdim, max(lengths))
     # three parts hold a float's 24 bits; either side adds up to 200 floats in some order, each addition off by up to 2^-23 of a sum that
     # is no larger than a few times its result: 2^-23 times the root of 200 additions, times four
     assert torch.equal(chunk_state[-1], state0[-1])
@@ -1218,6 +1241,7 @@ def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
                                 max(q_lens), heads, kv_heads, dim, vdim, "softmax", dim ** -0.5, head_scale=head_scale, softcap=cap, sink=sink,
                                 turn_cos=turn[0], turn_sin=turn[1], kernel=kernel)
         assert names == ["gated_attention"]
+        assert ops.float_weight_attention_takes(q, out, k_pool.cuda(), v_pool.cuda(), dim, vdim, max(q_lens))
         outs.append(out.float())
     # float weights either way: what differs is a rounding to bfloat16 of the result here and there
     assert float((outs[0] - outs[1]).abs().max()) <= 2.0 ** -7 * float(outs[1].abs().max())
@@ -1254,8 +1278,10 @@ def test_latent_prompts_expand_the_rows_they_see(cuda_device, monkeypatch, query
     spec = LatentAttentionSpec(hidden_size=width, num_heads=heads, head_dim=dim, value_dim=vdim, latent_dim=rank, scale=(dim + turned) ** -0.5, eps=1e-6,
                                gated=gate_kind is not None, weights={r: r for r in roles}, query_latent=query_latent,
                                position=RopeSpec(turned, 1e4, "half") if turned else None, window=window or None, gate_kind=gate_kind or "head")
-    outs = []
+    outs, ways, plain = [], [], latent_attention.ops.prompt_attention
+    monkeypatch.setattr(latent_attention.ops, "prompt_attention", lambda *args, **kwargs: (ways.append("expanded"), plain(*args, **kwargs))[1])
     for expanded in (True, False):
+        ways.append("step")
         mixer = build_part("mixer", spec, Runtime(torch.device("cuda:0"), "bfloat16", max_positions=512))
         draw = torch.Generator().manual_seed(5)
         mixer.load({p.name: (torch.randn(p.shape, generator=draw) * p.shape[-1] ** -0.5).bfloat16() if len(p.shape) > 1
@@ -1277,6 +1303,7 @@ def test_latent_prompts_expand_the_rows_they_see(cuda_device, monkeypatch, query
                 cache.commit(entries)
                 out = mixer.forward(torch.randn(sum(n for _, n in entries), width, generator=rows).bfloat16().cuda(), batch, run)
         outs.append(out.float())
+    assert ways[-2:] == ["expanded", "step"]  # the first mixer's last step, and none of the second's
     # keys, values and queries pass through bfloat16 at other places: four roundings' worth
     assert float((outs[0] - outs[1]).norm()) <= 4 * 2.0 ** -8 * float(outs[1].norm())
 
