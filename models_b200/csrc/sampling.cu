@@ -446,9 +446,11 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
 // (64 rows of 128,256, k 20 to 64: 119 us with histograms and one block a multiprocessor, 53 with this and two.)
 constexpr int kSampleBlocks = 8;
 constexpr int kFewCandidates = 128;
+constexpr int kAloneBlocks = 128;  // so many blocks of clusters of eight find a multiprocessor each
 constexpr float kThresholdSlack = 1e-5f;  // of a scaled logit: more than the exponential's rounding can turn around
 
-__global__ void __launch_bounds__(kThreads, 2)
+template <int kResident>  // blocks of a multiprocessor
+__global__ void __launch_bounds__(kThreads, kResident)
 sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int vocab, float* __restrict__ work,
                            int* __restrict__ counts, const float* __restrict__ temperature, const int* __restrict__ top_k,
                            const float* __restrict__ top_p, const float* __restrict__ penalty,
@@ -468,7 +470,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     __shared__ int slot_ties;
     __shared__ int gathered;            // first block: candidates gathered so far
     __shared__ int shared_int[4];
-    __shared__ float warp_tops[kSampleBlocks * 32];
+    __shared__ __align__(16) float warp_tops[kSampleBlocks * 32];
     __shared__ float few_threshold;
 
     namespace cg = cooperative_groups;
@@ -567,18 +569,23 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     bool few = k <= kFewCandidates && k < vocab;
     float threshold = CUDART_INF_F;
     if (few) {
-        if (tid < kSampleBlocks * 32) warp_tops[tid] = cluster.map_shared_rank(best_scratch, tid >> 5)[tid & 31].value;
-        __syncthreads();
-        if (tid < kSampleBlocks * 32) {
-            const float mine_top = warp_tops[tid];
-            int above = 0;
-#pragma unroll 8
-            for (int j = 0; j < kSampleBlocks * 32; ++j) above += warp_tops[j] > mine_top || (warp_tops[j] == mine_top && j < tid);
-            if (above == k - 1) few_threshold = mine_top;
+        const float mine_top = tid < kSampleBlocks * 32 ? cluster.map_shared_rank(best_scratch, tid >> 5)[tid & 31].value : -CUDART_INF_F;
+        if (tid < kSampleBlocks * 32) warp_tops[tid] = mine_top;
+        few = __syncthreads_count(mine_top > -CUDART_INF_F) >= k;  // (else every value would reach the threshold)
+        if (few) {
+            if (tid < kSampleBlocks * 32) {
+                int above = 0;
+#pragma unroll 4
+                for (int j = 0; j < kSampleBlocks * 32; j += 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(warp_tops + j);
+                    above += (t.x > mine_top || (t.x == mine_top && j < tid)) + (t.y > mine_top || (t.y == mine_top && j + 1 < tid)) +
+                             (t.z > mine_top || (t.z == mine_top && j + 2 < tid)) + (t.w > mine_top || (t.w == mine_top && j + 3 < tid));
+                }
+                if (above == k - 1) few_threshold = mine_top;
+            }
+            __syncthreads();
+            threshold = few_threshold - kThresholdSlack;
         }
-        __syncthreads();
-        threshold = few_threshold - kThresholdSlack;
-        few = threshold > -CUDART_INF_F;  // (fewer warps than k with a finite value: every value would reach it)
     }
 
     // softmax over the whole vocabulary
@@ -589,7 +596,11 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         w[i] = e;
         local += e;
         if (gathers && v >= threshold) {
-            const int at = atomicAdd(first_gathered, 1);
+            const unsigned peers = __activemask();  // the lanes that are here together add once
+            const int lane = tid & 31, leader = __ffs(peers) - 1;
+            int at = 0;
+            if (lane == leader) at = atomicAdd(first_gathered, __popc(peers));
+            at = __shfl_sync(peers, at, leader) + __popc(peers & ((1u << lane) - 1u));
             if (at < kMaxSorted) {
                 first_p[at] = e;
                 first_id[at] = i;
@@ -884,11 +895,14 @@ MB_EXPORT int mb_sample_rows(const float* logits, int row_stride, int rows, int 
     // than 400,000 ids) takes the kernel that works in the scratch array
     const size_t slice_bytes = (size_t)((vocab + kSampleBlocks - 1) / kSampleBlocks) * sizeof(float);
     if (max_candidates > 0 && max_candidates <= kMaxSorted && slice_bytes <= 200 * 1024) {
-        static size_t reserved = 0;
-        if (slice_bytes > reserved) {
-            cudaError_t status = cudaFuncSetAttribute(sample_rows_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slice_bytes);
+        // Few rows leave multiprocessors idle, and a block has one to itself with all of its registers; more share one.
+        const bool alone = kSampleBlocks * rows <= kAloneBlocks;
+        auto kernel = alone ? sample_rows_cluster_kernel<1> : sample_rows_cluster_kernel<2>;
+        static size_t reserved[2] = {0, 0};
+        if (slice_bytes > reserved[alone]) {
+            cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slice_bytes);
             if (status != cudaSuccess) return fail("sample_rows: cannot reserve %zu bytes of shared memory: %s", slice_bytes, cudaGetErrorString(status));
-            reserved = slice_bytes;
+            reserved[alone] = slice_bytes;
         }
         if (rows > 65535) return fail("sample_rows: %d rows exceed the grid limit 65535", rows);
         cudaLaunchConfig_t config = {};
@@ -903,7 +917,7 @@ MB_EXPORT int mb_sample_rows(const float* logits, int row_stride, int rows, int 
         attribute[0].val.clusterDim.z = 1;
         config.attrs = attribute;
         config.numAttrs = 1;
-        cudaError_t status = cudaLaunchKernelEx(&config, sample_rows_cluster_kernel, logits, row_stride, vocab, work, counts,
+        cudaError_t status = cudaLaunchKernelEx(&config, kernel, logits, row_stride, vocab, work, counts,
                                                 temperature, top_k, top_p, penalty, history, history_stride, history_rows, append, history_len, seeds,
                                                 counters, uniforms, out);
         if (status != cudaSuccess) return fail("sample_rows: launch failed: %s", cudaGetErrorString(status));
