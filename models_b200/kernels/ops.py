@@ -1350,6 +1350,11 @@ def gated_delta_chunks_library():
 
 
 DELTA_CHUNK_MIN_ROWS = 64  # steps that bring fewer tokens to every sequence are walked token by token
+# ... and so are steps of many short sequences: a chunk costs the same however few tokens it has, and the walk takes as long as the longest
+# sequence.  16 heads of 64 and 128, walk / chunks in microseconds: 1 x 64 tokens 37 / 47, 1 x 96 51 / 51, 1 x 128 65 / 51; 8 x 8 20 / 66;
+# 4 x 64 39 / 60, 2 x 128 67 / 58, 1 x 256 122 / 55; 8 x 128 126 / 104; 64 x 32 245 / 456, 32 x 64 225 / 245, 16 x 128 241 / 205.  A
+# captured step knows its tokens and how many sequences share them at most, not how long each one is: hence the mean.
+DELTA_CHUNK_MIN_MEAN = 96
 DELTA_CHUNK_BYTES = 1 << 30  # most scratch: a token of 16 heads of 64 and 128 takes 29 KB, where the walk takes 8
 
 
@@ -1360,10 +1365,10 @@ def gated_delta_chunk_floats(tokens: int, sequences: int, heads: int, vdim: int)
 
 
 def gated_delta_chunks_takes(conv: torch.Tensor, gate_in: torch.Tensor, gain: torch.Tensor, out: torch.Tensor, dim: int, vdim: int, parts_at,
-                             max_q_len: int) -> bool:
-    """Steps of many tokens, key heads of 64 numbers and value heads of 64 or 128, rows of whole fours that start on one's boundary;
+                             max_q_len: int, sequences: int) -> bool:
+    """Steps of many tokens a sequence, key heads of 64 numbers and value heads of 64 or 128, rows of whole fours that start on one's boundary;
     `parts_at`: the first columns of the convolved rows' parts."""
-    return (max_q_len >= DELTA_CHUNK_MIN_ROWS and dim == 64 and vdim in (64, 128) and conv.stride(0) % 4 == 0 and conv.data_ptr() % 16 == 0
+    return (max_q_len >= DELTA_CHUNK_MIN_ROWS and conv.shape[0] >= DELTA_CHUNK_MIN_MEAN * sequences and dim == 64 and vdim in (64, 128) and conv.stride(0) % 4 == 0 and conv.data_ptr() % 16 == 0
             and all(at % 4 == 0 for at in parts_at) and gain.data_ptr() % 16 == 0
             and all(t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0 for t in (gate_in, out)))
 
@@ -1424,7 +1429,7 @@ def gated_delta_scan(conv: torch.Tensor, q_at: int, k_at: int, v_at: int, a_in: 
     row of `state` (updated in place): S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q; out = out_scale * o / rms(o)
     * gain * silu(gate_in), rms over the head (eps `eps`).  a_in, b_in [tokens, heads], gate_in and out [tokens, heads * vdim]
     are column slices; a_in, b_in and gate_in share one row stride.  `max_q_len`: the most new tokens of a sequence (0: not known);
-    steps of many tokens are computed in chunks of 64 where the sizes allow it."""
+    steps of many tokens a sequence are computed in chunks of 64 where the sizes allow it."""
     _cuda(conv, a_in, b_in, gate_in, decay, dt_bias, gain, state, slots, cu_q, out)
     _int32(slots, "slots")
     _int32(cu_q, "cu_q")
@@ -1442,7 +1447,7 @@ def gated_delta_scan(conv: torch.Tensor, q_at: int, k_at: int, v_at: int, a_in: 
             raise KernelError(f"gated_delta_scan: {name} must be contiguous float32 of {n} elements")
     rows, stride = _state_rows(state, state_offset, heads * dim * vdim, "gated_delta_scan")
     floats = gated_delta_chunk_floats(tokens, cu_q.numel() - 1, heads, vdim)
-    if 4 * floats <= DELTA_CHUNK_BYTES and gated_delta_chunks_takes(conv, gate_in, gain, out, dim, vdim, (q_at, k_at, v_at), max_q_len):
+    if 4 * floats <= DELTA_CHUNK_BYTES and gated_delta_chunks_takes(conv, gate_in, gain, out, dim, vdim, (q_at, k_at, v_at), max_q_len, cu_q.numel() - 1):
         lib = gated_delta_chunks_library()
         scratch = torch.empty((floats,), dtype=torch.float32, device=conv.device)
         _run(lib, lib.mb_gated_delta_chunks(_p(conv), conv.stride(0), _p(a_in), _p(b_in), _p(gate_in), a_in.stride(0), _code(out.dtype), _p(decay),

@@ -919,10 +919,11 @@ def test_wide_qkv_product_with_rotation_and_cache_write(cuda_device, batch, head
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("vdim", [64, 128])
 @pytest.mark.parametrize("lengths", [[64], [1, 127, 64], [65, 0, 200, 63]])
-def test_gated_delta_chunks(cuda_device, dtype, vdim, lengths):
+def test_gated_delta_chunks(cuda_device, monkeypatch, dtype, vdim, lengths):
     """Chunks of 64 against the walk token by token and against the recurrence in 64 bits, from states that are not zero."""
     from models_b200.kernels import ops
 
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_MEAN", 1)  # (sequences of edge lengths, not of lengths that are worth it)
     heads, kv_heads, dim = 4, 2, 64
     g = torch.Generator().manual_seed(21)
     tokens, width = sum(lengths), 2 * kv_heads * dim + heads * vdim
@@ -941,7 +942,8 @@ def test_gated_delta_chunks(cuda_device, dtype, vdim, lengths):
                              slots, cu_q, heads, kv_heads, dim, vdim, out, 0.5, max_q_len=most)
         found.append((out.float(), state))
     (out, state), (chunk_out, chunk_state) = found
-    assert ops.gated_delta_chunks_takes(conv, gate, gain, out.to(dtype), dim, vdim, (0, kv_heads * dim, 2 * kv_heads * dim), max(lengths))
+    assert ops.gated_delta_chunks_takes(conv, gate, gain, out.to(dtype), dim, vdim, (0, kv_heads * dim, 2 * kv_heads * dim), max(lengths),
+                                        len(lengths))
     # sums of at most 64 + 64 products a token either way; the states' numbers are of size one to ten
     assert torch.allclose(chunk_state, state, rtol=1e-4, atol=1e-4)
     assert torch.equal(chunk_state[:, :3], state0[:, :3]) and torch.equal(chunk_state[-1], state0[-1])
@@ -996,8 +998,11 @@ def _delta_call(lengths, heads, kv_heads, vdim, dtype, seed, unit_eps=1e-6, spoi
 
 
 @pytest.mark.parametrize("lengths", [[65], [100, 64, 3]])
-def test_gated_delta_chunks_without_an_epsilon(cuda_device, lengths):
+def test_gated_delta_chunks_without_an_epsilon(cuda_device, monkeypatch, lengths):
     """Keys that are divided by their own length alone: the empty rows of a chunk that is not full have none."""
+    from models_b200.kernels import ops
+
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_MEAN", 1)
     call = _delta_call(lengths, 4, 2, 64, torch.float32, 5, unit_eps=0.0)
     (out, state), (chunk_out, chunk_state) = call(0), call(max(lengths))
     # the bounds of the test above
@@ -1015,6 +1020,14 @@ def test_gated_delta_steps_beyond_the_scratch_bound_are_walked(cuda_device, monk
     assert not torch.equal(walked[1], chunks[1])
     monkeypatch.setattr(ops, "DELTA_CHUNK_BYTES", 4 * ops.gated_delta_chunk_floats(200, 2, 2, 128) - 1)
     assert all(torch.equal(a, b) for a, b in zip(call(130), walked))
+
+
+@pytest.mark.parametrize("lengths,most,chunks", [([96], 96, True), ([95], 95, False), ([130, 62], 130, True), ([130, 61], 130, False), ([8] * 8, 64, False),
+                                                 ([24] * 8, 192, False), ([96, 96], 192, True)])
+def test_gated_delta_steps_of_short_sequences_are_walked(cuda_device, lengths, most, chunks):
+    """Either side of the line, and steps that say no more than how many tokens they have in all: as captured ones do."""
+    call = _delta_call(lengths, 2, 1, 64, torch.float32, 8)
+    assert torch.equal(call(most)[1], call(0)[1]) != chunks
 
 
 SPOILED = [("v", 5), ("v", 77), ("v", 90), ("k", 66), ("k", 127), ("q", 20)]  # a row that is not finite: within its 16 tokens, chunk and sequence
