@@ -1198,18 +1198,24 @@ def retention_chunks_library():
 
 
 RETENTION_CHUNK_MIN_ROWS = 64  # steps that bring fewer tokens to every sequence are walked
+# ... and so are steps of many short sequences that need no runs: the walk takes as long as the longest sequence, a chunk the same however few
+# tokens it has.  16 heads of 64 and 128, walk / chunks in microseconds: 1 x 64 tokens 58 / 39, 2 x 32 31 / 32, 4 x 16 18 / 31, 8 x 8
+# 11 / 34, 64 x 1 13 / 118; 2 x 64 59 / 38, 4 x 32 32 / 35, 8 x 16 18 / 35.  Where the walk goes in runs, every class of captured
+# steps of 256 tokens and more, chunks are quicker: 1 x 256 128 / 39, 64 x 4 159 / 130, 1 x 2,048 158 / 79, 64 x 32 329 / 204.
+RETENTION_CHUNK_MIN_MEAN = 32
 
 
 def retention_chunks_takes(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[torch.Tensor], out: Optional[torch.Tensor],
-                           raw_out: Optional[torch.Tensor], state: torch.Tensor, head_dim: int, value_dim: int, max_q_len: int) -> bool:
-    """bfloat16 steps of many tokens, key heads of 64 numbers and value heads of 64 or 128, rows that start on 16 bytes (results on a
+                           raw_out: Optional[torch.Tensor], state: torch.Tensor, head_dim: int, value_dim: int, max_q_len: int,
+                           sequences: int) -> bool:
+    """bfloat16 steps of many tokens a sequence, key heads of 64 numbers and value heads of 64 or 128, rows that start on 16 bytes (results on a
     pair's boundary)."""
     if raw_out is not None:
         pairs = raw_out.stride(0) % 2 == 0 and raw_out.data_ptr() % 8 == 0
     else:
         pairs = out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0 and g.data_ptr() % 4 == 0
     return (pairs and q.dtype == torch.bfloat16 and max_q_len >= RETENTION_CHUNK_MIN_ROWS and head_dim == 64 and value_dim in (64, 128)
-            and q.stride(0) % 8 == 0 and state.data_ptr() % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)))
+            and (max_q_len > 2 * RETENTION_RUN or q.shape[0] >= RETENTION_CHUNK_MIN_MEAN * sequences) and q.stride(0) % 8 == 0 and state.data_ptr() % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)))
 
 
 def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, positions: torch.Tensor,
@@ -1259,7 +1265,7 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.T
             raise KernelError("retention_scan: rotation needs float32 cos/sin tables")
         if cos.shape[-1] != rotary_dim // 2 or cos.shape != sin.shape or not cos.is_contiguous() or not sin.is_contiguous():
             raise KernelError(f"retention_scan: cos/sin tables must be contiguous [positions, {rotary_dim // 2}]")
-    if run_length is None and retention_chunks_takes(q, k, v, g, out, raw_out, state, head_dim, value_dim, max_q_len):
+    if run_length is None and retention_chunks_takes(q, k, v, g, out, raw_out, state, head_dim, value_dim, max_q_len, cu_q.numel() - 1):
         lib = retention_chunks_library()
         items = (tokens // lib.mb_retention_chunk_tokens() + cu_q.numel() - 1) * heads * head_dim * value_dim
         starts = torch.empty((items,), dtype=torch.float32, device=q.device)

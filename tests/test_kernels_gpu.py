@@ -1114,7 +1114,8 @@ def test_retention_chunks(cuda_device, vdim, lengths, whole):
                            input_activation="silu" if whole else None, raw_out=raw)
         found.append(((raw if whole else out).float(), state))
     (out, state), (chunk_out, chunk_state) = found
-    assert ops.retention_chunks_takes(q, k, v, None if whole else gate, None if whole else out.bfloat16(), out if whole else None, state, dim, vdim, max(lengths))
+    assert ops.retention_chunks_takes(q, k, v, None if whole else gate, None if whole else out.bfloat16(), out if whole else None, state, dim, vdim, max(lengths),
+                                      len(lengths))
     # three parts hold a float's 24 bits; either side adds up to 200 floats in some order, each addition off by up to 2^-23 of a sum that
     # is no larger than a few times its result: 2^-23 times the root of 200 additions, times four
     assert torch.equal(chunk_state[-1], state0[-1])
@@ -1123,6 +1124,27 @@ def test_retention_chunks(cuda_device, vdim, lengths, whole):
         assert float((chunk_out - out).norm() / out.norm()) < 2.0 ** -17
     else:
         close(chunk_out, out, torch.bfloat16)
+
+
+@pytest.mark.parametrize("lengths,most,chunks", [([64], 64, True), ([33, 31], 64, True), ([33, 30], 64, False), ([8] * 8, 64, False), ([16] * 8, 128, False),
+                                                 ([16] * 8, 129, True)])
+def test_retention_steps_of_short_sequences_are_walked(cuda_device, lengths, most, chunks):
+    """Either side of the line, and steps that say no more than how many tokens they have in all: as captured ones do."""
+    from models_b200.kernels import ops
+
+    heads, dim, tokens = 2, 64, sum(lengths)
+    g = torch.Generator().manual_seed(24)
+    q, k, v = torch.randn(tokens, 3 * heads * dim, generator=g).bfloat16().cuda().split(heads * dim, dim=1)
+    decay, state0 = torch.tensor([0.97, 0.5]).cuda(), torch.randn(len(lengths), heads, dim, dim, generator=g).cuda()
+    slots, positions = (torch.arange(n, dtype=torch.int32).cuda() for n in (len(lengths), tokens))
+    cu_q = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    found = []
+    for run_length in (0 if most <= 128 else 64, None):
+        state, raw = state0.clone(), torch.zeros(tokens, heads * dim).cuda()
+        ops.retention_scan(q, k, v, None, positions, None, None, 0, decay, 0.3, 1e-6, state, slots, cu_q, heads, dim, dim, None, 0.5, most,
+                           run_length=run_length, raw_out=raw)
+        found.append(raw)
+    assert torch.equal(*found) != chunks
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
