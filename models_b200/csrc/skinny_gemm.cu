@@ -687,8 +687,9 @@ static int skinny_gemm(const void* w, int ldw, int n, int k, int batch, const vo
     const bool streamable = epilogue == EPI_BF16 || epilogue == EPI_F32 || epilogue == EPI_RESIDUAL || epilogue == EPI_TANH;
     args.form = FORM_FOUR;
     // One row tile a block and a K so long that its activations leave room for one block on a multiprocessor: eight warps and rings
-    // for the activations keep twice the weights in flight and halve a warp's steps (2,048 rows, K 8,192: 9.1 us in a chain of them,
-    // and 8.0; at K 2,048 there was nothing to gain).
+    // for the activations keep twice the weights in flight and halve a warp's steps.  Four warps / this, microseconds in a chain of
+    // them at 1 row: 2,048 x 8,192 9.1 / 7.7, 2,048 x 4,104 6.1 / 5.3, 2,368 x 6,144 7.6 / 6.8, 1,024 x 8,192 8.6 / 6.4, 16 x 4,608
+    // 5.0 / 3.9; at 8 rows 9.2 / 8.0, 7.0 / 6.1, 7.8 / 7.1, 8.4 / 6.4, 4.9 / 3.8; at K 2,048 there was nothing to gain.
     if (streamable && prologue == PRO_NONE && split == 1 && batch <= 8 && tiles <= multiprocessors && k > 4096) args.form = FORM_EIGHT_STREAMED;
     const int warps = warps_of(args.form);
     args.k_unit = ((k + split - 1) / split + warps * kStep - 1) / (warps * kStep) * (warps * kStep);

@@ -847,8 +847,8 @@ def prompt_attention(q: torch.Tensor, q_tail: Optional[torch.Tensor], k: torch.T
                      out: torch.Tensor, cu_q: torch.Tensor, kv_lens: torch.Tensor, max_q_len: int, heads: int, head_columns: int,
                      value_columns: int, scale: float, gate: Optional[torch.Tensor] = None, window: int = 0,
                      gate_kind: str = "head", key_rows: int = 0, key_window: int = 0) -> None:
-    """Causal softmax attention of prompts that start their sequences, on the tcgen05 tensor cores with float weights: every key comes
-    from the step's own rows.  bfloat16: k [T, heads * KD] and v [T, heads * VD] (column slices with one row stride; KD, VD multiples
+    """Causal softmax attention of prompts on the tcgen05 tensor cores with float weights, keys and values as rows: the step's own where it
+    starts its sequences, or with `key_rows` rows of all that it sees.  bfloat16: k [T, heads * KD] and v [T, heads * VD] (column slices with one row stride; KD, VD multiples
     of 64, heads padded with zero columns), k_tail [T, RD] shared by all heads and q_tail [T, heads * RD] (or None, None); q [T, ...] holds
     head h's own coordinates from column h * head_columns on; out [T, heads * value_columns]; gate [T, heads]: head h's result is
     multiplied by its sigmoid, or, gate_kind "element", a gate [T, heads * value_columns] element by element.  `window` n > 0: query i
@@ -1215,7 +1215,8 @@ def retention_chunks_takes(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g:
     else:
         pairs = out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0 and g.data_ptr() % 4 == 0
     return (pairs and q.dtype == torch.bfloat16 and max_q_len >= RETENTION_CHUNK_MIN_ROWS and head_dim == 64 and value_dim in (64, 128)
-            and (max_q_len > 2 * RETENTION_RUN or q.shape[0] >= RETENTION_CHUNK_MIN_MEAN * sequences) and q.stride(0) % 8 == 0 and state.data_ptr() % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)))
+            and (max_q_len > 2 * RETENTION_RUN or q.shape[0] >= RETENTION_CHUNK_MIN_MEAN * sequences)
+            and q.stride(0) % 8 == 0 and state.data_ptr() % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)))
 
 
 def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, positions: torch.Tensor,
@@ -1374,7 +1375,8 @@ def gated_delta_chunks_takes(conv: torch.Tensor, gate_in: torch.Tensor, gain: to
                              max_q_len: int, sequences: int) -> bool:
     """Steps of many tokens a sequence, key heads of 64 numbers and value heads of 64 or 128, rows of whole fours that start on one's boundary;
     `parts_at`: the first columns of the convolved rows' parts."""
-    return (max_q_len >= DELTA_CHUNK_MIN_ROWS and conv.shape[0] >= DELTA_CHUNK_MIN_MEAN * sequences and dim == 64 and vdim in (64, 128) and conv.stride(0) % 4 == 0 and conv.data_ptr() % 16 == 0
+    return (max_q_len >= DELTA_CHUNK_MIN_ROWS and conv.shape[0] >= DELTA_CHUNK_MIN_MEAN * sequences and dim == 64 and vdim in (64, 128)
+            and conv.stride(0) % 4 == 0 and conv.data_ptr() % 16 == 0
             and all(at % 4 == 0 for at in parts_at) and gain.data_ptr() % 16 == 0
             and all(t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0 for t in (gate_in, out)))
 

@@ -38,7 +38,8 @@ from .split import SplitPart
 # 128, rows of 256 + 64, queries with a latent and a window of 1,024; microseconds expanded / in the latent space): 128 tokens on 256
 # cached ones 159 / 134, 4 x 128 on 300 152 / 158, 4 x 128 on 1,500 (13 rows gathered for a token) 153 / 226, 2 x 765 on 700 154 / 350,
 # 2,048 on 1,500 155 / 446.  Prompts that start their sequences and whose queries have no latent save a launch as well: they expand from
-# the kernel's least step on.
+# the kernel's least step on.  Without a host between the launches: 2,048 tokens on 30,000 cached ones 124 / 443 (169 while the rows before
+# the window were expanded as well), 600 on 30,000 87 / 234, 4 x 256 on 6,000 114 / 251; without a window 2,048 on 30,000 744 / 6,682.
 EXPANDED_TOKENS = 512
 EXPANDED_ROWS = 16  # most rows gathered for a token
 EXPANDED_BYTES = 1 << 30  # most workspace for the gathered rows and the keys and values made of them
