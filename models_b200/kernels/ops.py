@@ -1025,7 +1025,12 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
         return
     shaped = (weights == "softmax" and slope_exponent == 0.0 and head_bias is None and gate is None and block == 0
               and (turn_cos is None or (turn_cos.data_ptr() % 16 == 0 and turn_sin.data_ptr() % 16 == 0)))
-    if kernel is None and shaped and float_weight_attention_takes(q, out, k_pool, v_pool, head_dim, value_dim, max_q_len):
+    # A captured step says that one sequence may hold all of its tokens: most of its tiles of 128 queries are then empty, and an empty block of
+    # the tcgen05 kernel costs more than one of the mma.sync kernel.  16 heads of 64 and 128, mma.sync / tcgen05 in microseconds: 16 x 40
+    # tokens on 300 as 80 tiles 30 / 41, 32 x 64 on 1,000 as 512 tiles 137 / 164; as what they are, 27 / 24 and 121 / 95; 8 x 64 on
+    # 4,000 as 32 tiles 201 / 163.
+    full = sequences * -(-max_q_len // 128) <= 3 * (-(-q.shape[0] // 128) + sequences)
+    if kernel is None and shaped and full and float_weight_attention_takes(q, out, k_pool, v_pool, head_dim, value_dim, max_q_len):
         lib = float_weight_attention_library(head_dim, value_dim, shaped=True)
         _run(lib, lib.mb_prefill_attention_tcgen05(
             _p(q), q.stride(0), q.shape[0], _p(out), out.stride(0), _p(k_pool), _p(v_pool), k_pool.shape[0], _p(block_table),

@@ -1283,6 +1283,26 @@ def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
     assert float((outs[0] - outs[1]).norm()) <= 2.0 ** -9 * float(outs[1].norm())
 
 
+@pytest.mark.parametrize("sequences,tokens,most,tcgen05", [(8, 40, 40, True), (8, 64, 512, True), (16, 40, 640, False)])
+def test_shaped_scores_of_mostly_empty_tiles(cuda_device, sequences, tokens, most, tcgen05):
+    """A step that says that one sequence may hold all of its tokens (a captured one does) takes the mma.sync kernel where most tiles would be
+    empty."""
+    from models_b200.kernels import ops
+
+    heads, dim, vdim, rows = 2, 64, 128, sequences * tokens
+    g = torch.Generator().manual_seed(33)
+    k_pool, v_pool = (torch.randn(sequences + 1, 1, 64, d, generator=g).bfloat16().cuda() for d in (dim, vdim))
+    q = torch.randn(rows, heads * dim, generator=g).bfloat16().cuda()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()  # noqa: E731
+    outs = []
+    for kernel in (None, "tc"):
+        outs.append(torch.zeros(rows, heads * vdim, dtype=torch.bfloat16, device=cuda_device))
+        ops.gated_attention(q, outs[-1], k_pool, v_pool, i32([[i + 1] for i in range(sequences)]), i32([i * tokens for i in range(sequences + 1)]),
+                            i32([tokens] * sequences), most, heads, 1, dim, vdim, "softmax", 0.125, softcap=20.0, sink=True, kernel=kernel)
+    assert torch.equal(*outs) != tcgen05
+    assert torch.allclose(outs[0].float(), outs[1].float(), rtol=2.0 ** -7, atol=2.0 ** -9)
+
+
 @pytest.mark.parametrize("max_q_len,kernel", [(1, None), (64, None), (64, "tc"), (64, "rows")])
 def test_a_negative_bound_on_scores_is_refused(cuda_device, max_q_len, kernel):
     """Whichever kernel a call meets."""
