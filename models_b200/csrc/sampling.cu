@@ -446,7 +446,7 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
 // (64 rows of 128,256, k 20 to 64: 119 us with histograms and one block a multiprocessor, 53 with this and two.)
 constexpr int kSampleBlocks = 8;
 constexpr int kFewCandidates = 128;
-constexpr int kAloneBlocks = 128;  // so many blocks of clusters of eight find a multiprocessor each
+constexpr int kAloneBlocks = 64;  // so many blocks, clusters of eight, find a multiprocessor each with certainty
 constexpr float kThresholdSlack = 1e-5f;  // of a scaled logit: more than the exponential's rounding can turn around
 
 template <int kResident>  // blocks of a multiprocessor
@@ -895,7 +895,9 @@ MB_EXPORT int mb_sample_rows(const float* logits, int row_stride, int rows, int 
     // than 400,000 ids) takes the kernel that works in the scratch array
     const size_t slice_bytes = (size_t)((vocab + kSampleBlocks - 1) / kSampleBlocks) * sizeof(float);
     if (max_candidates > 0 && max_candidates <= kMaxSorted && slice_bytes <= 200 * 1024) {
-        // Few rows leave multiprocessors idle, and a block has one to itself with all of its registers; more share one.
+        // Few rows leave multiprocessors idle, and a block has one to itself with all of its registers (8 rows masked to ten finite
+        // values, which the histograms decide: 40.7 us, 44.8 with two to a multiprocessor); more share one (16 rows, 40 candidates: 25 us,
+        // and 30 where the last cluster waits for a second round).
         const bool alone = kSampleBlocks * rows <= kAloneBlocks;
         auto kernel = alone ? sample_rows_cluster_kernel<1> : sample_rows_cluster_kernel<2>;
         static size_t reserved[2] = {0, 0};
