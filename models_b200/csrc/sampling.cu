@@ -442,7 +442,9 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
 //
 // Few candidates (k <= kFewCandidates) need no histograms: the maxima of the row's 256 warps are 256 of its values, so the k-th
 // largest of them is at most the row's k-th largest, and hardly more than k values reach it (40 of 128,256 random values: 44).
-// They are gathered while the exponentials are summed; should more reach it than can be sorted, the histograms decide.
+// They are gathered while the exponentials are summed; should more reach it than can be sorted, the histograms decide, and at once where
+// fewer warps than k have a finite value (rows masked to ten finite values, 1 and 64 rows: 39.7 and 133 us; 47.6 and 152 before that was
+// looked at).
 // (64 rows of 128,256, k 20 to 64: 119 us with histograms and one block a multiprocessor, 53 with this and two.)
 constexpr int kSampleBlocks = 8;
 constexpr int kFewCandidates = 128;
@@ -895,9 +897,9 @@ MB_EXPORT int mb_sample_rows(const float* logits, int row_stride, int rows, int 
     // than 400,000 ids) takes the kernel that works in the scratch array
     const size_t slice_bytes = (size_t)((vocab + kSampleBlocks - 1) / kSampleBlocks) * sizeof(float);
     if (max_candidates > 0 && max_candidates <= kMaxSorted && slice_bytes <= 200 * 1024) {
-        // Few rows leave multiprocessors idle, and a block has one to itself with all of its registers (8 rows masked to ten finite
-        // values, which the histograms decide: 40.7 us, 44.8 with two to a multiprocessor); more share one (16 rows, 40 candidates: 25 us,
-        // and 30 where the last cluster waits for a second round).
+        // Few rows leave multiprocessors idle, and a block has one to itself with all of its registers (8 rows of 128,256, 40 and 200
+        // candidates: 17.5 and 37.1 us; 18.2 and 38.2 with the registers of two); more share one (16 rows: 25.3 us, and 30.0 where the last
+        // cluster of eight waits for a second round).
         const bool alone = kSampleBlocks * rows <= kAloneBlocks;
         auto kernel = alone ? sample_rows_cluster_kernel<1> : sample_rows_cluster_kernel<2>;
         static size_t reserved[2] = {0, 0};
