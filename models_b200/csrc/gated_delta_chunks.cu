@@ -21,7 +21,7 @@
 // results by 1.4e-7 (2e-7).
 // One sequence of 2,048 tokens, 16 heads of 64 x 128: the walk's chain of 2,048 tokens is bound by its latency (618 us, and 30 for
 // the kernels around it); the three kernels took 58, 105 and 71 us as float multiply-adds, bound by what the operands take from
-// shared memory and by the latency of few warps; 54, 67 and 60 here (a layer: 310 us, and 247), where the carrying kernel is bound by
+// shared memory and by the latency of few warps; 54, 67 and 60 here (a layer: 310 us, and 247 to 250), where the carrying kernel is bound by
 // its chunk's two products one after the other, the others by six products for one and the splitting of what they read.
 #include "common.cuh"
 #include "split_products.cuh"
@@ -257,6 +257,7 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
     // last block's z takes the first one's place, which nothing reads after it.
     const uint32_t matrix_at = smem_u32(matrix) + lanes_by_row(kRow), inverse_at = smem_u32(inverse) + lanes_by_row(Plan::inverse_row),
                    solved_at = smem_u32(solved) + column0 * 2 + lanes_by_row(Plan::right_row);
+    float fit = 0.0f;
 #pragma unroll
     for (int block = 0; block < kChunk / 16; ++block) {
         const int row0 = 16 * block < Plan::solved_rows ? 16 * block : 0;
@@ -274,27 +275,16 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
         for (int c = 0; c < block; ++c) accumulate(matrix_at + (16 * block * kRow + 16 * c) * 2, kPlane, 16 * c);
         __syncwarp();
         bf16* mine = solved + (row0 + group) * Plan::right_row + column0 + pair;
-        float (&z)[kTiles][4] = right[block];
-        bool finite = true;
 #pragma unroll
         for (int n = 0; n < kTiles; ++n) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                z[n][i] -= acc[n][i];
-                finite = finite && has_parts(z[n][i]);
-                acc[n][i] = 0.0f;
-            }
-            split_two(z[n][0], z[n][1], mine + 8 * n, Plan::right_plane);
-            split_two(z[n][2], z[n][3], mine + 8 * Plan::right_row + 8 * n, Plan::right_plane);
+            split_two(right[block][n][0] - acc[n][0], right[block][n][1] - acc[n][1], mine + 8 * n, Plan::right_plane);
+            split_two(right[block][n][2] - acc[n][2], right[block][n][3] - acc[n][3], mine + 8 * Plan::right_row + 8 * n, Plan::right_plane);
+            acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
         }
-        const bool whole = __all_sync(0xffffffffu, finite);
         __syncwarp();
-        if (whole) {
-            accumulate(inverse_at + 16 * block * Plan::inverse_row * 2, Plan::inverse_plane, row0);
-        } else {
-            auto weight = [&](int row, int column) { return whole_one(inverse + (16 * block + row) * Plan::inverse_row + column, Plan::inverse_plane); };
-            causal_products(acc, weight, solved + row0 * Plan::right_row + column0 + pair, Plan::right_row, Plan::right_plane);
-        }
+        accumulate(inverse_at + 16 * block * Plan::inverse_row * 2, Plan::inverse_plane, row0);
+#pragma unroll
+        for (int n = 0; n < kTiles; ++n) fit += acc[n][0] + acc[n][1];
         __syncwarp();
         const int row = 16 * block + group;
 #pragma unroll
@@ -314,6 +304,28 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
             }
         }
         __syncwarp();
+    }
+    // A row that is not finite has met the inverses' zeros in the earlier rows of its 16, and a thread's upper results show it: the warp's
+    // columns once more by plain substitution, a lane a column.
+    if (!__all_sync(0xffffffffu, isfinite(fit))) {
+        const int column = column0 + (tid & 31);
+        const float* from = of_values ? value_rows + column : key_rows + column - V;
+        float x[kChunk];
+#pragma unroll 1
+        for (int i = 0; i < kChunk; ++i) {
+            float sum = (of_values ? beta[i] : beta[i] * expf((float)logs[i]) * unit[i]) * (i < count ? from[(size_t)i * args.conv_stride] : 0.0f);
+#pragma unroll 1
+            for (int j = 0; j < i; ++j) sum = fmaf(-whole_one(matrix + i * kRow + j, kPlane), x[j], sum);
+            x[i] = sum;
+            if (of_values) {
+                args.u[(at * kChunk + i) * V + column] = sum;
+            } else {
+                uint32_t hi, mid, lo;
+                split_pair(sum, 0.0f, hi, mid, lo);
+                unsigned short* y = reinterpret_cast<unsigned short*>(args.y + kParts * at * kChunk * kDim + (size_t)i * kDim + column - V);
+                y[0] = (unsigned short)hi, y[kChunk * kDim] = (unsigned short)mid, y[2 * kChunk * kDim] = (unsigned short)lo;
+            }
+        }
     }
 }
 
@@ -445,9 +457,9 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
     if (count <= 0) return;
     const size_t token0 = (size_t)first + chunk * kChunk;
     const size_t at = place_of(first, seq, chunk) * args.heads + head;
-    bool finite = true;
+    float fit;
     auto bring = [&](const float* from) {
-        finite = true;
+        fit = 0.0f;
         constexpr int kPieces = 64 * V / 8 / kResultThreads;
         float x[kPieces][8];
 #pragma unroll
@@ -455,8 +467,7 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
             const int piece = tid + i * kResultThreads;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) finite = finite && has_parts(x[i][j]);
+            fit += fitness(x[i]);
             store_parts(planes + Plan::wide + piece / (V / 8) * Plan::wide_row + piece % (V / 8) * 8, Plan::wide_plane, x[i]);
         }
     };
@@ -495,12 +506,11 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
 #pragma unroll
     for (int n = 0; n < V / 16; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][i] *= from_start[i / 2];
-    const bool spoiled = __syncthreads_or(!finite);
-    const int last = spoiled ? 2 * warp - 2 : 2 * warp;  // (then the warp's own 16 tokens come below)
+        for (int i = 0; i < 4; ++i) acc[n][i] = __fmul_rn(acc[n][i], from_start[i / 2]);  // (rounded by itself, whatever follows)
+    const bool spoiled = __syncthreads_or(!isfinite(fit));
 #pragma unroll
     for (int n = 0; n < kChunk / 8; n += 2) {
-        if (n > last) break;
+        if (n > 2 * warp) break;
 #pragma unroll
         for (int m = n; m < n + 2; ++m)
 #pragma unroll
@@ -519,12 +529,15 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
             split_products(acc[c], acc[c + 1], a, b);
         }
     }
-    if (spoiled) {
-        auto weight = [&](int token, int from) {
-            return whole_dot<kDim>(planes + Plan::queries + (16 * warp + token) * kRow, planes + Plan::keys + (16 * warp + from) * kRow, kPlane) *
-                   expf((float)(logs[16 * warp + token] - logs[16 * warp + from]));
-        };
-        causal_products(acc, weight, planes + Plan::wide + 16 * warp * Plan::wide_row + column0 + pair, Plan::wide_row, Plan::wide_plane);
+    if (spoiled) {  // a row of u that is not finite: see causal_products
+        const bf16 *queries = planes + Plan::queries, *keys = planes + Plan::keys;
+        auto weight = [&](int token, int from) { return whole_dot<kDim>(queries + token * kRow, keys + from * kRow, kPlane) * expf((float)(logs[token] - logs[from])); };
+        start_products<kDim>(acc, queries + row * kRow, kRow, kPlane, args.starts + at * kDim * V + column0 + pair, V);
+#pragma unroll
+        for (int n = 0; n < V / 16; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[n][i] *= from_start[i / 2];
+        causal_products(acc, row, weight, planes + Plan::wide + column0 + pair, Plan::wide_row, Plan::wide_plane);
     }
     // norm, gain and gate: a row's V results lie with four neighbouring lanes of two warps
 #pragma unroll

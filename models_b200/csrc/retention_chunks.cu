@@ -227,7 +227,7 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         }
     }
     __syncthreads();  // nobody reads the start any more
-    bool finite = true;
+    float fit = 0.0f;
 #pragma unroll
     for (int i = 0; i < kPieces; ++i) {
         const int piece = tid + i * kThreads;
@@ -238,12 +238,10 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         if (args.input_act >= 0 && piece / (V / 8) < count)
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = gate_activation(args.input_act, x[j]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) finite = finite && has_parts(x[j]);
+        fit += fitness(x);
         store_parts(wide + piece / (V / 8) * kRow + piece % (V / 8) * 8, kPlane, x);
     }
-    const bool spoiled = __syncthreads_or(!finite);
-    const int last = spoiled ? 2 * warp - 2 : 2 * warp;  // (then the warp's own 16 tokens come below)
+    const bool spoiled = __syncthreads_or(!isfinite(fit));
     const int row = 16 * warp + group;
 #pragma unroll
     for (int n = 0; n < V / 16; ++n)
@@ -251,7 +249,7 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         for (int i = 0; i < 4; ++i) acc[n][i] *= power[row + 8 * (i / 2) + 1];
 #pragma unroll
     for (int n = 0; n < kChunk / 8; n += 2) {
-        if (n > last) break;
+        if (n > 2 * warp) break;
 #pragma unroll
         for (int m = n; m < n + 2; ++m)
 #pragma unroll
@@ -270,12 +268,17 @@ retention_chunk_results_kernel(const RetentionArgs args) {
             split_products(acc[c], acc[c + 1], a, b);
         }
     }
-    if (spoiled) {
+    if (spoiled) {  // a value that is not finite: see causal_products
         auto weight = [&](int token, int from) {
-            return whole_dot<kDim>(queries + (16 * warp + token) * kKeyRow, keys + (16 * warp + from) * kKeyRow, kKeyPlane) *
-                   (args.key_scale * power[max(token - from, 0)]);
+            return whole_dot<kDim>(queries + token * kKeyRow, keys + from * kKeyRow, kKeyPlane) * (args.key_scale * power[token - from]);
         };
-        causal_products(acc, weight, wide + 16 * warp * kRow + column0 + pair, kRow, kPlane);
+        start_products<kDim>(acc, queries + row * kKeyRow, kKeyRow, kKeyPlane,
+                             args.starts + (place_of(first, seq, chunk) * args.heads + head) * kDim * V + column0 + pair, V);
+#pragma unroll
+        for (int n = 0; n < V / 16; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[n][i] *= power[row + 8 * (i / 2) + 1];
+        causal_products(acc, row, weight, wide + column0 + pair, kRow, kPlane);
     }
     if (args.raw_out == nullptr) {  // a row's V results lie with four neighbouring lanes of two warps
 #pragma unroll

@@ -81,35 +81,62 @@ __device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], c
     for (int i = 0; i < 4; ++i) d0[i] += p0[i] + r0[i], d1[i] += p1[i] + r1[i];
 }
 
-// What has three finite parts.  (The largest bfloat16 number is a little smaller than the largest float.)
-__device__ __forceinline__ bool has_parts(float v) { return fabsf(v) < 3.3895e38f; }
+// A sum that is finite only where eight floats are, and have three finite parts.  (The largest bfloat16 number is a little smaller than the
+// largest float: four times what lies between them is infinite.)
+__device__ __forceinline__ float fitness(const float (&x)[8]) {
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sum = fmaf(x[j], 4.0f, sum);
+    return sum;
+}
 // A float from its parts, and the float dot product of two rows of parts.
 __device__ __forceinline__ float whole_one(const bf16* at, int plane) {
     const float hi = __bfloat162float(at[0]);
-    return has_parts(hi) ? hi + __bfloat162float(at[plane]) + __bfloat162float(at[2 * plane]) : hi;
+    return isfinite(hi) ? hi + __bfloat162float(at[plane]) + __bfloat162float(at[2 * plane]) : hi;
 }
 template <int kCount>
-__device__ float whole_dot(const bf16* a, const bf16* b, int plane) {
+__device__ __forceinline__ float whole_dot(const bf16* a, const bf16* b, int plane) {
     float sum = 0.0f;
 #pragma unroll 1
     for (int i = 0; i < kCount; ++i) sum = fmaf(whole_one(a + i, plane), whole_one(b + i, plane), sum);
     return sum;
 }
-// acc += w . v for the weights weight(token, earlier token) of 16 tokens on themselves, where a row of v may not be finite: the zeros that
-// stand for later tokens' weights would make NaN of it in a product, and it must reach its own token and later ones alone.  In float,
-// token by token, slow; `values`: the thread's pair of columns of the first of the 16 rows.
+// acc += w . v token by token in float, for two tokens of a chunk a thread (`token` and 8 further on, its group's rows of the warp's 16) over
+// the weights weight(token, earlier token) of the tokens up to each: what the tensor cores compute, but that a row of v that is not
+// finite does not meet the zeros that stand for later tokens' weights.  `values`: the thread's pair of columns of the chunk's first row.
 template <int kTiles, typename Weight>
-__device__ __forceinline__ void causal_products(float (&acc)[kTiles][4], Weight weight, const bf16* values, int row, int plane) {
-    const int group = (threadIdx.x & 31) >> 2;
+__device__ __forceinline__ void causal_products(float (&acc)[kTiles][4], int token, Weight weight, const bf16* values, int row, int plane) {
+    const int lane = threadIdx.x & 31, end = (token & ~15) + 16;
 #pragma unroll 1
-    for (int j = 0; j < 16; ++j) {
-        const bf16* at = values + j * row;
-        const float upper = j <= group ? weight(group, j) : 0.0f, lower = j <= group + 8 ? weight(group + 8, j) : 0.0f;
+    for (int j0 = 0; j0 < end; j0 += 4) {  // a group's four lanes make a weight of either token each
+        const int mine = j0 + (lane & 3);
+        const float upper = mine <= token ? weight(token, mine) : 0.0f, lower = mine <= token + 8 ? weight(token + 8, mine) : 0.0f;
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) {
+            const int j = j0 + e;
+            const float first = __shfl_sync(0xffffffffu, upper, (lane & 28) + e), second = __shfl_sync(0xffffffffu, lower, (lane & 28) + e);
+#pragma unroll
+            for (int n = 0; n < kTiles; ++n) {
+                const float x = whole_one(values + j * row + 8 * n, plane), y = whole_one(values + j * row + 8 * n + 1, plane);
+                if (j <= token) acc[n][0] = fmaf(first, x, acc[n][0]), acc[n][1] = fmaf(first, y, acc[n][1]);
+                if (j <= token + 8) acc[n][2] = fmaf(second, x, acc[n][2]), acc[n][3] = fmaf(second, y, acc[n][3]);
+            }
+        }
+    }
+}
+// acc = S^T q for two tokens a thread, in float; `start`: the thread's pair of columns of the state's first row.
+template <int kDim, int kTiles>
+__device__ __forceinline__ void start_products(float (&acc)[kTiles][4], const bf16* queries, int query_row, int plane, const float* start, int columns) {
+#pragma unroll
+    for (int n = 0; n < kTiles; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+#pragma unroll 1
+    for (int d = 0; d < kDim; ++d) {
+        const float first = whole_one(queries + d, plane), second = whole_one(queries + 8 * query_row + d, plane);
 #pragma unroll
         for (int n = 0; n < kTiles; ++n) {
-            const float x = whole_one(at + 8 * n, plane), y = whole_one(at + 8 * n + 1, plane);
-            if (j <= group) acc[n][0] = fmaf(upper, x, acc[n][0]), acc[n][1] = fmaf(upper, y, acc[n][1]);
-            if (j <= group + 8) acc[n][2] = fmaf(lower, x, acc[n][2]), acc[n][3] = fmaf(lower, y, acc[n][3]);
+            const float2 s = *reinterpret_cast<const float2*>(start + (size_t)d * columns + 8 * n);
+            acc[n][0] = fmaf(first, s.x, acc[n][0]), acc[n][1] = fmaf(first, s.y, acc[n][1]);
+            acc[n][2] = fmaf(second, s.x, acc[n][2]), acc[n][3] = fmaf(second, s.y, acc[n][3]);
         }
     }
 }

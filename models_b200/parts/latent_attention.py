@@ -125,6 +125,7 @@ class LatentAttentionMixer(SplitPart, Mixer):
             pad = lambda m, size: torch.nn.functional.pad(m, (0, 0, 0, _whole(size) - size)).reshape(-1, K)  # noqa: E731
             self.expand = torch.cat([pad(rt.matrix(tensors[n["up_k"]]).to(dtype).view(s.num_heads, D, K), D),
                                      pad(self.out_of_latent, V)]).contiguous()
+            self.row_bytes = (self.expand.shape[0] + K + _whole(self.turned)) * self.expand.element_size()  # of a row gathered and expanded
 
     @property
     def starts_differ(self) -> bool:
@@ -152,13 +153,13 @@ class LatentAttentionMixer(SplitPart, Mixer):
         if fresh:
             return 0
         # (the page tables' width and not the lengths: a captured step replays for every length its class holds)
-        seen = group.block_table.shape[1] * run.k_pool.shape[2]
+        page = run.k_pool.shape[2]
+        seen = group.block_table.shape[1] * page
         if self.spec.window:  # nobody sees more: the window's positions before the first token, the step's own, and what is left of a first 64
             seen = min(seen, self.spec.window - 1 + batch.max_q_len + 63)
         per = -(-seen // 64) * 64
-        rows, width = per * batch.kv_lens.numel(), self.expand.shape[0] + self.spec.latent_dim + _whole(self.turned)
-        fits = (run.k_pool.shape[2] % 64 == 0 and self.turned % 8 == 0 and rows <= EXPANDED_ROWS * mid.shape[0]
-                and rows * width * self.expand.element_size() <= EXPANDED_BYTES)
+        rows = per * batch.kv_lens.numel()
+        fits = page % 64 == 0 and self.turned % 8 == 0 and rows <= EXPANDED_ROWS * mid.shape[0] and rows * self.row_bytes <= EXPANDED_BYTES
         return per if fits else None
 
     def _expanded(self, q, down, gate, mid, batch, group, run: RunContext, cos, sin, key_rows: int) -> None:
