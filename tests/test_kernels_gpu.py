@@ -1046,7 +1046,7 @@ def test_gated_delta_chunks_keep_earlier_tokens_apart(cuda_device, vdim, value, 
 
     clean, clean_state = _delta_call(lengths, 2, 1, vdim, torch.float32, 6)(130)
     out, state = _delta_call(lengths, 2, 1, vdim, torch.float32, 6, spoil=spoil)(130)
-    # (sixteen tokens beside such a row are added up in another order)
+    # (a chunk that holds such a row is added up in another order)
     close(out[:at], clean[:at], torch.float32, scale=4.0)
     assert torch.equal(out[130:], clean[130:]) and torch.equal(state[1], clean_state[1])
     assert not bool(out[at].isfinite().all())
