@@ -466,16 +466,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 tmem_load_32_issue(taddr + c + 32 * part, v);
                                 tmem_load_32_issue(taddr + 128 + c + 32 * part, u);
                                 tmem_load_wait();
-                                // Rows beyond the last are zeros, and a division of zero takes its long way:
-                                // 50 us for 437 rows of 2,048 with 16,384 weight rows where 512 took 34.  A gated zero is zero under
-                                // every activation, so pieces of nothing but zeros stay as they are: 33 us.  (Warps whose rows all lie
-                                // beyond the last idle above; without this test that alone left the 437 rows at 50.6 us.)
-                                uint32_t bits = 0;
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) bits |= __float_as_uint(v[i]) | __float_as_uint(u[i]);
-                                if (bits != 0)
-#pragma unroll
-                                    for (int i = 0; i < 32; ++i) v[i] = gated_pair(args.activation, v[i], u[i], args.clamp);
+                                // The gated epilogue must not take longer than a tile's products (16,400 cycles at K = 2,048).
+                                // With a division per pair it took 21,600 (left out, 2,048 rows and 16,384 weight rows ran in 82 us
+                                // instead of 100): 94.6 us now; 512 rows 33.6 -> 28.5 us, 1,024 rows 57.6 -> 52.0 us.
+                                gate_pairs(args.activation, v, u, args.clamp);
                             } else {
                                 tmem_load_32_issue(taddr + c + 32 * part, v);
                                 tmem_load_wait();

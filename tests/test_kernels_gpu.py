@@ -1221,6 +1221,32 @@ def test_gated_prompt_product_with_rows_of_zeros(cuda_device, activation, rows):
     assert bool((got[empty.cuda()] == 0).all()) and torch.equal(got[~empty.cuda()], want[~empty.cuda()])
 
 
+@pytest.mark.parametrize("clamp", [None, (7.0, 1.702, 1.0)])
+def test_gated_prompt_product_of_unusual_gates(cuda_device, clamp):
+    """Gates whose exponential overflows, vanishes or is at the edge of either: within the rounding to bfloat16 (eight bits: 2^-8), the float
+    operations before it (below 2^-18) and what a float that small holds of a quotient by more than 2^126."""
+    from models_b200.kernels import ops
+
+    gates = torch.tensor([0.0, 1e-30, 1.0, -1.0, -20.0, 20.0, -85.0, -87.5, -88.5, -90.0, -104.0, 104.0, -1e4, 1e4, -3e38, 3e38] * 8)
+    n = gates.numel()
+    a = torch.zeros(130, 2 * n, dtype=torch.bfloat16)
+    a[:, :n] = torch.diag(gates.bfloat16().float())[torch.arange(130) % n].bfloat16()  # row r: gate r alone, and up 0.5
+    a[:, n] = 1.0
+    w = torch.zeros(2 * n, 2 * n, dtype=torch.bfloat16)
+    w[:n, :n] = torch.eye(n)
+    w[n:, n] = 0.5
+    gate = (a.double() @ w.double().t())[:, :n]
+    if clamp is None:
+        want = gate / (1 + torch.exp(-gate)) * 0.5
+        got = ops.gemm_tcgen05(a.cuda(), w.cuda(), ops.EPI_SWIGLU)
+    else:
+        g = gate.clamp(max=clamp[0])
+        want = g / (1 + torch.exp(-clamp[1] * g)) * (0.5 + clamp[2])
+        got = ops.gemm_tcgen05(a.cuda(), w.cuda(), ops.EPI_CLAMPED, clamp=clamp)
+    error = (got.double().cpu() - want).abs()
+    assert bool((error <= want.abs() * (2.0 ** -8 + 2.0 ** -18) + 90.0 * 2.0 ** -126).all())
+
+
 @pytest.mark.parametrize("batch", [1, 3, 8])
 @pytest.mark.parametrize("n,k", [(2048, 4104), (37, 5000), (16, 8192), (2360, 8192)])
 def test_skinny_gemm_streams_activations(cuda_device, batch, n, k):
