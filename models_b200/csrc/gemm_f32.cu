@@ -1,21 +1,37 @@
-// True 32-bit matrix product: C[M, N] = A[M, K] . W[N, K]^T with float operands and float FMAs
-// on the CUDA cores -- no tensor-core mode, no reduced-precision inputs.  It is the matrix
-// product of the 32-bit path of the whole model.
+// 32-bit matrix product on the fifth-generation tensor cores: C[M, N] = A[M, K] . W[N, K]^T of floats, whose 24 bits are all
+// multiplied.  It is the matrix product of the 32-bit path of the whole model.
 //
 // out[r] = sum_c W[r, c] * x[c] (integrallis/models, backend-java/.../ops/TensorOps.java:61-63).
-// Every output element is the sum, in order, of up to eight chains of FMAs over consecutive parts of
-// c = 0..K-1, each in ascending order; the parts follow from N and K alone, so a row's result does not
-// depend on how many other rows the call carries, on where the row sits in a tile, on its alignment or on
-// which of the kernels below computes it.  (A decode product that need not be row-invariant takes gemv_f32_kernel,
-// whose sums run over lanes.)
+// A float is the sum of three bfloat16 numbers (float_parts.cuh), and a product of floats that of six products of these (the other
+// three are below 2^-26 of it), summed in float:
+//   * the products of the two roundings, 64 columns of K at a time, in tensor memory, and these sums by float additions in
+//     registers: a tensor core cuts its sum off where a float addition rounds, so no long sum may stay there;
+//   * the five smaller products, which lose nothing that counts to the cut, in tensor memory over all of the block's columns.
+// Every result is the sum, in order, of up to four such sums over consecutive parts of K; the parts follow from N and K alone, and
+// every call runs the same operations on a row, so a row's result depends neither on the other rows of the call, nor on where it
+// sits in a tile, nor on alignment, nor on which of the kernels below computes it.
 //
-// Bound by shared memory and the FMA pipe together: a lane's 8 x 8 results take 16 operands per column
-// of K, 64 bytes through a 128-byte port for the 64 FMAs, both 16 cycles of a multiprocessor per warp.
-// 384 rows, 16,384 columns, K 2,048: 1,193 us with 4 x 4 results a thread and element loads, 576 now
-// (45 TFLOP/s; the FMA pipes alone would take 346 us); with single FMAs instead of pairs 668; wider results (8 x 16, 12 x 12) lost what they saved to registers.
-#include "common.cuh"
+// Off the sums in 64 bits by 1.0e-7 to 1.4e-7 (2-norm; K 2,048 and 8,192); chains of FMAs over the same parts were 2.9e-7 to 5.8e-7 off.
+// 301 rows, W of 16,384 x 2,048 that are bfloat16 numbers: 92 us, 2,048 x 8,192 55 us, 3,072 x 2,048 38 us, 2,048 x 2,048 21 us (whole
+// floats 118, 67, 44 and 24); FMAs on 8 x 8 results a thread took 480, 274, 114 and 80 us, at 46 of the CUDA cores' 74 TFLOP/s.
+// From 33 rows on a block is bound by the splitting of W (1,500 to 2,000 cycles per 64 columns; 12 or 24 products of 160 rows take the
+// tensor cores 960 or 1,920).  One row: 16,384 x 2,048 in 28 us (29 before), 2,048 x 8,192 in 22 (17 before: sixteen rows of W at a time
+// leave a scheduler one warp), eight rows 30 us (43 before) and 23 (26).
+//
+// 128 rows of W are the products' first operand and up to 160 rows of A the second.  Eight warps bring W from memory (loads of the
+// next columns are under way while these are worked on) and split it into shared memory, one brings A, which a kernel before has
+// split (of up to 32 rows the eight warps split it too: in 301 rows that doubled their work, 127 us for 92), one issues the products,
+// and four hold the sums, a row of W per thread.  Weights that are bfloat16 numbers -- most models' are, in the 32-bit mode too -- have
+// two parts of zeros, whose products are left out: each stage of W says whether it is such.
+//
+// A float that is not finite, or has no finite rounding, spoils the sums of its own row of A or W alone; these results are
+// computed anew from the floats, in the order of K.  Floats below 2^-109 keep fewer bits (off by 2^-134 at most).
+#include "tcgen05.cuh"
+#include "float_parts.cuh"
 
 #include <cooperative_groups.h>
+
+#include <algorithm>
 
 namespace cg = cooperative_groups;
 
@@ -23,383 +39,678 @@ MB_DEFINE_LAST_ERROR()
 
 namespace mb {
 
-constexpr int kTileM = 64, kTileN = 64, kTileK = 16;
+constexpr int kTileN = 128;           // rows of the products' first operand: a block's rows of W, or twice as many
+constexpr int kChunk = 64;            // columns of K per stage: a row of 128 bytes of bfloat16
+constexpr int kAdders = 4, kSplitters = 8;  // warps; after them one issues products and one brings A (two keep their warpgroup company)
+constexpr int kIssuer = kAdders + kSplitters, kBringer = kIssuer + 1;
+constexpr int kThreads = 32 * (kAdders + kSplitters + 4);
+constexpr int kRegisters = 128;       // a thread's at launch; the warpgroups trade them once (what is in flight to a register that is given back would be lost)
+constexpr int kPlaneW = kTileN * 128;
+constexpr int kPlaneA = 32 * 128;     // times NB
+constexpr int kMaxStages = 3;
+constexpr int kInlineRows = 32;       // most rows of A that are split where they are multiplied
+constexpr int kSlabRows = 2048;       // rows of A that are split at a time
 
-// Any sizes, strides and alignments.
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, float* __restrict__ c,
-                int ldc, int m, int n, int k, int part_length) {
-    __shared__ float a_tile[kTileK][kTileM + 4];
-    __shared__ float w_tile[kTileK][kTileN + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
-    const int row0 = blockIdx.y * kTileM, col0 = blockIdx.x * kTileN;
-    float acc[4][4] = {}, sum[4][4] = {};
-    for (int k0 = 0; k0 < k; k0 += kTileK) {
-        if (k0 > 0 && k0 % part_length == 0)  // the next part's chains begin (part_length is a multiple of kTileK)
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sum[i][j] = k0 == part_length ? acc[i][j] : sum[i][j] + acc[i][j];
-                    acc[i][j] = 0.0f;
-                }
-        // 64 rows x 16 columns of each operand; 256 threads, 4 elements each
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int index = threadIdx.x + i * 256;
-            const int r = index / kTileK, kk = index % kTileK;
-            const int gr = row0 + r, gc = col0 + r, gk = k0 + kk;
-            a_tile[kk][r] = (gr < m && gk < k) ? a[(size_t)gr * lda + gk] : 0.0f;
-            w_tile[kk][r] = (gc < n && gk < k) ? w[(size_t)gc * ldw + gk] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < kTileK; ++kk) {
-            float av[4], wv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = a_tile[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) wv[j] = w_tile[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gr = row0 + ty * 4 + i;
-        if (gr >= m) continue;
+// NB: 32 rows of A each.  kRowsW: rows of W per block (64 leave half of the products' first operand to chance, unread).
+template <int NB, int kRowsW>
+struct Plan {
+    static constexpr bool kInline = NB == 1;
+    static constexpr int kRows = 32 * NB;
+    static constexpr int kStageBytes = 3 * (kPlaneW + NB * kPlaneA);
+    static constexpr int kStages = NB <= 2 ? 3 : 2;
+    static constexpr int kBytes = kStages * kStageBytes + 1024;
+    static constexpr int kColumns = 3 * kRows <= 128 ? 128 : 3 * kRows <= 256 ? 256 : 512;  // of tensor memory: two sums, and the smaller products'
+    // Registers a thread: shares of the four warpgroups' 128 a thread at launch.
+    static constexpr int kAdderRegisters = kInline ? 80 : 224, kSplitterRegisters = kInline ? 152 : 112, kIssuerRegisters = 48;
+    static_assert(kAdderRegisters + 2 * kSplitterRegisters + kIssuerRegisters <= 4 * kRegisters && kThreads == 512, "the warpgroups' shares");
+    static_assert(kStages <= kMaxStages && kStages * kStageBytes >= kRows * kRowsW * 4, "the parts' sums take the place of the stages");
+};
+
+// A thread's eight of a row's 64 columns, as four pairs: four columns from `from` and the four 32 further (so that eight threads' loads
+// cover whole lines), left as they are unless `wanted`.  They stand side by side in the stage: both operands have the same order of K
+// there.  kEven: whole 16-byte pieces of whole stages, by loads that a predicate holds back; else column by column, zeros from column
+// `left` on.  (Plain loads: the kernel before may just have written the row.)
+template <bool kEven>
+__device__ __forceinline__ void load_eight(uint64_t (&v)[4], const float* from, int left, bool wanted) {
+    if (kEven) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %5, 0;\n\t"
+            "@p ld.global.v2.b64 {%0, %1}, [%4];\n\t"
+            "@p ld.global.v2.b64 {%2, %3}, [%4 + 128];\n\t}"
+            : "+l"(v[0]), "+l"(v[1]), "+l"(v[2]), "+l"(v[3])
+            : "l"(from), "r"((uint32_t)wanted)
+            : "memory");
+    } else if (wanted) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int gc = col0 + tx * 4 + j;
-            if (gc < n) c[(size_t)gr * ldc + gc] = k > part_length ? sum[i][j] + acc[i][j] : acc[i][j];
+            const int column = 2 * (j % 2) + j / 2 * 32;
+            v[j] = pair_of(column < left ? from[column] : 0.0f, column + 1 < left ? from[column + 1] : 0.0f);
         }
     }
 }
 
-__device__ __forceinline__ uint64_t twice(float v) {
-    uint64_t d;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
-    return d;
-}
-__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {  // two float FMAs, each rounded as fmaf rounds
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
+// Four neighbouring columns, as two pairs, in the same way.
+template <bool kEven>
+__device__ __forceinline__ void load_four(uint64_t (&v)[2], const float* from, int left, bool wanted) {
+    if (kEven) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %3, 0;\n\t"
+            "@p ld.global.v2.b64 {%0, %1}, [%2];\n\t}"
+            : "+l"(v[0]), "+l"(v[1])
+            : "l"(from), "r"((uint32_t)wanted)
+            : "memory");
+    } else if (wanted) {
+        v[0] = pair_of(0 < left ? from[0] : 0.0f, 1 < left ? from[1] : 0.0f);
+        v[1] = pair_of(2 < left ? from[2] : 0.0f, 3 < left ? from[3] : 0.0f);
+    }
 }
 
-__device__ __forceinline__ float low_of(uint64_t v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float high_of(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ const float* tiled_part(float* mine, int rank) { return cg::this_cluster().map_shared_rank(mine, rank); }
+// Whether one of them is not finite, or has a part that is not.  (The largest bfloat16 number is a little smaller than the largest
+// float: four times what lies between them is infinite.)
+__device__ __forceinline__ bool unfit_pairs(const uint64_t (&v)[4]) {
+    uint64_t sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum = pair_fma(v[j], 0x4080000040800000ull, sum);  // 4, 4
+    return !isfinite(low_of(sum) + high_of(sum));
+}
 
-// Rows of 16-byte pieces.  A block of kWarpsM x kWarpsN warps; a warp is 4 x 8 lanes, a lane holds 4 * kM4 rows x 4 * kN4
-// columns, whose fours lie 16 rows (32 columns) apart, so that a four is one 16-byte load from shared memory.  The `parts`
-// blocks of a cluster take `part_length` columns of K each; their sums meet in shared memory, added in the parts' order.
-template <int kWarpsM, int kWarpsN, int kM4, int kN4>
-__global__ void __launch_bounds__(kWarpsM * kWarpsN * 32)
-gemm_f32_tiled_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, float* __restrict__ c, int ldc, int m,
-                      int n, int k, int tiles_n, int parts, int part_length) {
-    constexpr int kThreads = kWarpsM * kWarpsN * 32, kRows = kWarpsM * 16 * kM4, kCols = kWarpsN * 32 * kN4;
-    constexpr int kLoadsA = kRows * (kTileK / 4) / kThreads, kLoadsW = kCols * (kTileK / 4) / kThreads;
-    static_assert(kLoadsA >= 1 && kLoadsW >= 1 && kRows % 32 == 0 && kCols % 32 == 0, "every thread brings whole pieces");
-    // [k][row], the row's bits 3 and 4 turned by k / 4: the eight rows x four pieces that a warp stores at once meet 32 banks
-    extern __shared__ __align__(16) float tiled_shared[];
-    float* a_tiles = tiled_shared;                          // [2][kTileK][kRows]
-    float* w_tiles = tiled_shared + 2 * kTileK * kRows;     // [2][kTileK][kCols]
-    const int part = parts > 1 ? (int)cg::this_cluster().block_rank() : 0, tile = blockIdx.x / parts;
-    const int row0 = (tile / tiles_n) * kRows, col0 = (tile % tiles_n) * kCols;
-    const int k_begin = part * part_length, k_end = min(k, k_begin + part_length);
+// Their parts, 16 bytes to each of three planes; `smaller` gathers the bits of the two smaller ones.
+__device__ __forceinline__ void split_eight(const uint64_t (&v)[4], unsigned char* at, size_t plane_bytes, uint32_t& smaller) {
+    uint4 hi, mid, lo;
+    split_pair(v[0], hi.x, mid.x, lo.x);
+    split_pair(v[1], hi.y, mid.y, lo.y);
+    split_pair(v[2], hi.z, mid.z, lo.z);
+    split_pair(v[3], hi.w, mid.w, lo.w);
+    *reinterpret_cast<uint4*>(at) = hi;
+    *reinterpret_cast<uint4*>(at + plane_bytes) = mid;
+    *reinterpret_cast<uint4*>(at + 2 * plane_bytes) = lo;
+    smaller |= mid.x | mid.y | mid.z | mid.w | lo.x | lo.y | lo.z | lo.w;
+}
+
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t elected;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+    return elected;
+}
+
+// One step of 16 columns: to (+)= a . b.  (Whether it adds is known where it is written, and no lane is masked: a step is issued in
+// half the time that umma() takes, and few rows of A are bound by the issue.)
+template <bool kAdds>
+__device__ __forceinline__ void issue_step(uint32_t to, uint64_t a_desc, uint64_t b_desc, uint32_t instruction) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(to), "l"(a_desc), "l"(b_desc), "r"(instruction), "n"(kAdds ? 1 : 0)
+        : "memory");
+}
+
+struct FloatArgs {
+    const float* a;
+    const float* w;
+    float* c;
+    int lda, ldw, ldc, m, n, k;
+    int parts, part_length;       // blocks of a cluster that share K; columns of each, a multiple of kChunk
+    const unsigned char* unfit;   // of A's rows when they have been split: [m][chunks of K], whether a float there has no finite parts
+};
+
+// A, split: planes [3][m][chunks * 64], a chunk's columns in the order of load_eight, zeros behind the last.  32 chunks of rows a block.
+template <bool kEven>
+__global__ void __launch_bounds__(256)
+split_rows_kernel(const float* __restrict__ a, int lda, int m, int k, int chunks, unsigned char* planes, unsigned char* unfit) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const size_t item = (size_t)blockIdx.x * 32 + (threadIdx.x >> 3);
+    if (item >= (size_t)m * chunks) return;  // (eight threads at once)
+    const int row = (int)(item / chunks), chunk = (int)(item % chunks), unit = threadIdx.x & 7;
+    uint64_t v[4] = {};
+    load_eight<kEven>(v, a + (size_t)row * lda + chunk * kChunk + 4 * unit, k - chunk * kChunk - 4 * unit, true);
+    uint32_t smaller = 0;
+    split_eight(v, planes + item * 128 + unit * 16, (size_t)m * chunks * 128, smaller);
+    const uint32_t eight = 0xffu << (threadIdx.x & 24);
+    const bool bad = __any_sync(eight, unfit_pairs(v));
+    if (unit == 0) unfit[item] = bad;
+}
+
+// grid: parts of K fastest, then the tiles of A, then those of W (so that neighbours share a tile of W).
+template <int NB, int kRowsW, bool kEven>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args) {
+    using P = Plan<NB, kRowsW>;
+    constexpr int kPlane = NB * kPlaneA;
+    constexpr int kPassesW = kRowsW / 16, kPassesA = P::kInline ? 2 * NB : 0, kHeldA = P::kInline ? 2 * NB : 1;
+    constexpr uint32_t kInstruction = instruction_descriptor(kTileN, P::kRows);
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t barriers[2 * kMaxStages + 5];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int whole[kMaxStages];  // one more than the last chunk whose floats of W, in this stage, have parts beyond the first
+    __shared__ unsigned char spoilt_w[kRowsW], spoilt_a[P::kRows];
+    __shared__ int spoilt;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int my_row = (warp / kWarpsN) * 16 * kM4 + (lane >> 3) * 4, my_col = (warp % kWarpsN) * 32 * kN4 + (lane & 7) * 4;
-    uint64_t acc[kM4 * 4][kN4 * 2];
-#pragma unroll
-    for (int i = 0; i < kM4 * 4; ++i)
-#pragma unroll
-        for (int j = 0; j < kN4 * 2; ++j) acc[i][j] = 0;
-    float4 a_next[kLoadsA], w_next[kLoadsW];
-    const int piece = (threadIdx.x & 3) * 4, first = threadIdx.x >> 2;
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int i = 0; i < kLoadsA; ++i) {
-            const int r = row0 + first + i * (kThreads / 4);
-            a_next[i] = (r < m && k0 + piece < k_end) ? __ldg(reinterpret_cast<const float4*>(a + (size_t)r * lda + k0 + piece)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const uint32_t full_bar = smem_u32(&barriers[0]), empty_bar = smem_u32(&barriers[kMaxStages]);
+    const uint32_t sum_full_bar = smem_u32(&barriers[2 * kMaxStages]), sum_empty_bar = sum_full_bar + 16, done_bar = sum_full_bar + 32;
+    const int part = blockIdx.x % args.parts, tile = blockIdx.x / args.parts;
+    const int a_tiles = (args.m + P::kRows - 1) / P::kRows;
+    const int row0 = (tile % a_tiles) * P::kRows, col0 = (tile / a_tiles) * kRowsW;
+    const int k_begin = part * args.part_length, k_end = min(args.k, k_begin + args.part_length);
+    const int chunks = (k_end - k_begin + kChunk - 1) / kChunk;  // (no part is empty)
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < P::kStages; ++s) {
+            mbar_init(full_bar + 8 * s, kSplitters / 2 + (P::kInline ? 0 : 1));
+            mbar_init(empty_bar + 8 * s, 1);
+            whole[s] = 0;
         }
-#pragma unroll
-        for (int i = 0; i < kLoadsW; ++i) {
-            const int r = col0 + first + i * (kThreads / 4);
-            w_next[i] = (r < n && k0 + piece < k_end) ? __ldg(reinterpret_cast<const float4*>(w + (size_t)r * ldw + k0 + piece)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(sum_full_bar + 8 * b, 1);
+            mbar_init(sum_empty_bar + 8 * b, kAdders);
         }
-    };
-    auto store = [&](int buffer) {
-        const int turn = (piece / 4) << 3;
-        float* at = a_tiles + buffer * kTileK * kRows + piece * kRows;
-        float* wt = w_tiles + buffer * kTileK * kCols + piece * kCols;
-#pragma unroll
-        for (int i = 0; i < kLoadsA; ++i) {
-            const int r = (first + i * (kThreads / 4)) ^ turn;
-            at[r] = a_next[i].x, at[kRows + r] = a_next[i].y, at[2 * kRows + r] = a_next[i].z, at[3 * kRows + r] = a_next[i].w;
-        }
-#pragma unroll
-        for (int i = 0; i < kLoadsW; ++i) {
-            const int r = (first + i * (kThreads / 4)) ^ turn;
-            wt[r] = w_next[i].x, wt[kCols + r] = w_next[i].y, wt[2 * kCols + r] = w_next[i].z, wt[3 * kCols + r] = w_next[i].w;
-        }
-    };
-    fetch(k_begin);
-    store(0);
+        mbar_init(done_bar, 1);
+        spoilt = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = threadIdx.x; i < kRowsW + P::kRows; i += kThreads) (i < kRowsW ? spoilt_w[i] : spoilt_a[i - kRowsW]) = 0;
+    if (warp == kIssuer) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "n"(P::kColumns));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    tcgen05_fence_before();
     __syncthreads();
-    const int steps = (k_end - k_begin + kTileK - 1) / kTileK;
-    for (int step = 0; step < steps; ++step) {
-        const int buffer = step & 1;
-        if (step + 1 < steps) fetch(k_begin + (step + 1) * kTileK);
-        const float* at = a_tiles + buffer * kTileK * kRows;
-        const float* wt = w_tiles + buffer * kTileK * kCols;
+    tcgen05_fence_after();
+    const uint32_t tmem_sum = tmem_base_slot, tmem_small = tmem_sum + 2 * P::kRows;  // two sums, taken in turn by the chunks
+    grid_launch_dependents();
+    float* sums = reinterpret_cast<float*>(smem);
+
+    if (warp < kAdders) {
+        // ------------------------------------------------------------------ add
+        if (P::kAdderRegisters > kRegisters) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P::kAdderRegisters));
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P::kAdderRegisters));
+        grid_dependency_wait();
+        uint64_t sum[P::kRows / 2];  // of this thread's row of W, in pairs
 #pragma unroll
-        for (int kk = 0; kk < kTileK; ++kk) {
-            const int turn = (kk / 4) << 3;
-            float4 av[kM4];
-            ulonglong2 wv[kN4];
+        for (int j = 0; j < P::kRows / 2; ++j) sum[j] = 0;
+        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+        bool ok = true;
+        auto add = [&](uint32_t from) {
 #pragma unroll
-            for (int i = 0; i < kM4; ++i) av[i] = *reinterpret_cast<const float4*>(at + kk * kRows + ((my_row + 16 * i) ^ turn));
+            for (int i = 0; i < P::kRows; i += 32) {
+                float v[32];
+                tmem_load_32_issue(from + lanes + i, v);
+                tmem_load_wait();
 #pragma unroll
-            for (int j = 0; j < kN4; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(wt + kk * kCols + ((my_col + 32 * j) ^ turn));
+                for (int j = 0; j < 16; ++j) sum[i / 2 + j] = pair_add(sum[i / 2 + j], pair_of(v[2 * j], v[2 * j + 1]));
+            }
+        };
+        for (int chunk = 0; chunk < chunks && ok; ++chunk) {  // what the tensor cores summed over a chunk
+            const int b = chunk & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait(sum_full_bar + 8 * b, chunk >> 1 & 1, 4));
+            tcgen05_fence_after();
+            if (ok) add(tmem_sum + b * P::kRows);
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sum_empty_bar + 8 * b);
+        }
+        ok = ok && __all_sync(0xffffffffu, mbar_wait(done_bar, 0, 5));
+        tcgen05_fence_after();
+        if (ok) add(tmem_small);
+        tcgen05_fence_before();
+        // To the result, or, as one of several parts, to shared memory (every product has read the stages): [rows of A][kRowsW].
+        const int col = col0 + (int)threadIdx.x;
+        const int rows = (int)threadIdx.x >= kRowsW ? 0 : args.parts > 1 ? P::kRows : col < args.n ? min(P::kRows, args.m - row0) : 0;
+        float* to = args.parts > 1 ? sums + threadIdx.x : args.c + (size_t)row0 * args.ldc + col;
+        const size_t step = args.parts > 1 ? kRowsW : args.ldc;
 #pragma unroll
-            for (int i = 0; i < kM4; ++i) {
-                const uint64_t x[4] = {twice(av[i].x), twice(av[i].y), twice(av[i].z), twice(av[i].w)};
+        for (int j = 0; j < P::kRows; ++j)
+            if (j < rows) to[j * step] = j % 2 ? high_of(sum[j / 2]) : low_of(sum[j / 2]);
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * (kAdders + kSplitters)) : "memory");  // the splitters have seen every float
+        if (*reinterpret_cast<volatile int*>(&spoilt) && (int)threadIdx.x < kRowsW && col < args.n) {
+#pragma unroll 1
+            for (int j = 0; j < min(P::kRows, args.m - row0); ++j)
+                if (spoilt_w[threadIdx.x] || spoilt_a[j]) {
+                    const float *a = args.a + (size_t)(row0 + j) * args.lda, *w = args.w + (size_t)col * args.ldw;
+                    float total = 0.0f;
+#pragma unroll 1
+                    for (int k = k_begin; k < k_end; ++k) total = fmaf(a[k], w[k], total);
+                    to[j * step] = total;
+                }
+        }
+        __syncwarp();
+        if (args.parts > 1) {
+            cluster_sync_all();
+            cluster_leave_together();
+        }
+    } else if (warp < kAdders + kSplitters) {
+        // ------------------------------------------------------------------ bring and split
+        if (P::kSplitterRegisters > kRegisters) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P::kSplitterRegisters));
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P::kSplitterRegisters));
+        // Two groups of four warps take the chunks in turn, so that one splits while the other waits.  Eight threads bring a row's
+        // 64 columns, a group 16 rows a pass; a pass's registers take the group's next chunk as soon as they have been split.
+        const int group = (warp - kAdders) / (kSplitters / 2);
+        const int my_row = (threadIdx.x & 127) >> 3, unit = threadIdx.x & 7;
+        uint64_t w_next[kPassesW][4] = {}, a_next[kHeldA][4] = {};
+        // Rows beyond the last repeat it; nobody reads what becomes of them.
+        const float* w_from = args.w + (size_t)col0 * args.ldw + k_begin + 4 * unit;
+        const float* a_from = args.a + (size_t)row0 * args.lda + k_begin + 4 * unit;
+        const int w_last = args.n - 1 - col0, a_last = args.m - 1 - row0;
+        auto fetch_w = [&](int wanted, int p) {
+            const int at = wanted * kChunk;
+            load_eight<kEven>(w_next[p], w_from + (at + (long long)min(16 * p + my_row, w_last) * args.ldw), k_end - k_begin - at - 4 * unit, wanted < chunks);
+        };
+        auto fetch_a = [&](int wanted, int p) {
+            const int at = wanted * kChunk;
+            load_eight<kEven>(a_next[p], a_from + (at + (long long)min(16 * p + my_row, a_last) * args.lda), k_end - k_begin - at - 4 * unit, wanted < chunks);
+        };
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
+        for (int p = 0; p < kPassesW; ++p) fetch_w(group, p);  // weights depend on nothing
+        grid_dependency_wait();
 #pragma unroll
-                    for (int j = 0; j < kN4; ++j) {
-                        acc[4 * i + r][2 * j] = fma_pair(x[r], wv[j].x, acc[4 * i + r][2 * j]);
-                        acc[4 * i + r][2 * j + 1] = fma_pair(x[r], wv[j].y, acc[4 * i + r][2 * j + 1]);
+        for (int p = 0; p < kPassesA; ++p) fetch_a(group, p);
+        bool ok = true;
+        for (int chunk = group; chunk < chunks && ok; chunk += 2) {
+            const int stage = chunk % P::kStages;
+            ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * stage, (chunk / P::kStages & 1) ^ 1, 1));  // (a stage starts free)
+            if (!ok) break;
+            unsigned char* at = smem + stage * P::kStageBytes + my_row * 128 + ((unit ^ (my_row & 7)) << 4);  // the 128-byte swizzle
+            uint32_t smaller = 0, nothing = 0, unfit = 0;
+#pragma unroll
+            for (int p = 0; p < kPassesW; ++p) {
+                split_eight(w_next[p], at + p * 2048, kPlaneW, smaller);
+                unfit |= (unfit_pairs(w_next[p]) ? 1u : 0u) << p;
+                fetch_w(chunk + 2, p);
+            }
+#pragma unroll
+            for (int p = 0; p < kPassesA; ++p) {
+                split_eight(a_next[p], at + 3 * kPlaneW + p * 2048, kPlane, nothing);
+                unfit |= (unfit_pairs(a_next[p]) ? 1u : 0u) << (kPassesW + p);
+                fetch_a(chunk + 2, p);
+            }
+            if (unfit != 0) {
+                spoilt = 1;
+#pragma unroll 1
+                for (int p = 0; p < kPassesW + kPassesA; ++p)
+                    if (unfit >> p & 1) (p < kPassesW ? spoilt_w[16 * p + my_row] : spoilt_a[16 * (p - kPassesW) + my_row]) = 1;
+            }
+            if ((smaller & 0x7fff7fffu) != 0) whole[stage] = chunk + 1;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full_bar + 8 * stage);
+        }
+        const int row = threadIdx.x - 32 * kAdders;
+        if (!P::kInline && row < P::kRows && row0 + row < args.m) {
+            const int all = (args.k + kChunk - 1) / kChunk;
+            const unsigned char* of_row = args.unfit + (size_t)(row0 + row) * all + k_begin / kChunk;
+            uint32_t bad = 0;
+            for (int i = 0; i < chunks; ++i) bad |= of_row[i];
+            if (bad != 0) spoilt_a[row] = 1, spoilt = 1;
+        }
+        asm volatile("bar.arrive 1, %0;" ::"n"(32 * (kAdders + kSplitters)) : "memory");
+        __syncwarp();
+        if (args.parts > 1) {  // the cluster's blocks share the rows and add the parts in their order
+            cluster_sync_all();
+            for (int i = threadIdx.x - 32 * kAdders; i < P::kRows / args.parts * (kRowsW / 4); i += 32 * kSplitters) {  // (parts is 2 or 4)
+                const int r = i / (kRowsW / 4) * args.parts + part, piece = i % (kRowsW / 4) * 4;
+                const int row = row0 + r, col = col0 + piece;
+                if (row >= args.m || col >= args.n) continue;
+                float4 v[4];
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    if (p < args.parts) v[p] = *reinterpret_cast<const float4*>(cg::this_cluster().map_shared_rank(sums, p) + r * kRowsW + piece);
+                float4 total = v[0];
+#pragma unroll
+                for (int p = 1; p < 4; ++p)
+                    if (p < args.parts) total.x += v[p].x, total.y += v[p].y, total.z += v[p].z, total.w += v[p].w;
+                float* to = args.c + (size_t)row * args.ldc + col;
+                const float out[4] = {total.x, total.y, total.z, total.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (col + e < args.n) to[e] = out[e];
+            }
+            cluster_leave_together();  // the others read this block's sums
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P::kIssuerRegisters));
+        if (warp == kIssuer) {
+            // -------------------------------------------------------------- products (the warp walks together, one thread issues)
+            const uint32_t elected = elect_one();
+            int stage = 0;
+            uint32_t phase = 0;
+            for (int chunk = 0; chunk < chunks; ++chunk) {
+                // The lanes wait together: one that fell behind by two passes over the stages would wait for the wrong one.
+                const int b = chunk & 1;
+                if (!__all_sync(0xffffffffu, mbar_wait(full_bar + 8 * stage, phase, 2))) break;
+                tcgen05_fence_after();
+                const uint32_t w_at = smem_u32(smem) + stage * P::kStageBytes, a_at = w_at + 3 * kPlaneW;
+                const uint64_t w_desc = umma_descriptor(w_at), a_desc = umma_descriptor(a_at);
+                const bool all_parts = *reinterpret_cast<volatile int*>(&whole[stage]) == chunk + 1;
+                auto products = [&](int w_part, int a_part, uint32_t to, bool fresh) {
+#pragma unroll
+                    for (int ks = 0; ks < kChunk / 16; ++ks) {
+                        const uint64_t w_step = w_desc + ((w_part * kPlaneW >> 4) + 2 * ks), a_step = a_desc + ((a_part * kPlane >> 4) + 2 * ks);
+                        if (fresh && ks == 0) issue_step<false>(to, w_step, a_step, kInstruction);
+                        else issue_step<true>(to, w_step, a_step, kInstruction);
                     }
+                };
+                if (elected) {
+                    products(0, 2, tmem_small, chunk == 0);
+                    if (all_parts) {
+                        products(1, 1, tmem_small, false);
+                        products(2, 0, tmem_small, false);
+                    }
+                    products(0, 1, tmem_small, false);
+                    if (all_parts) products(1, 0, tmem_small, false);
+                }
+                // the chunk before the last has been added
+                if (chunk > 1 && !__all_sync(0xffffffffu, mbar_wait(sum_empty_bar + 8 * b, (chunk >> 1 & 1) ^ 1, 3))) break;
+                tcgen05_fence_after();
+                if (elected) {
+                    products(0, 0, tmem_sum + b * P::kRows, true);
+                    umma_commit(sum_full_bar + 8 * b);
+                    umma_commit(empty_bar + 8 * stage);
+                }
+                if (++stage == P::kStages) stage = 0, phase ^= 1;
+            }
+            if (elected) umma_commit(done_bar);
+        } else if (warp == kBringer && !P::kInline) {
+            // -------------------------------------------------------------- A's parts
+            grid_dependency_wait();
+            const uint32_t elected = elect_one();
+            int stage = 0;
+            uint32_t phase = 1;
+            for (int chunk = 0; chunk < chunks; ++chunk) {
+                if (!__all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * stage, phase, 6))) break;
+                if (elected) {
+                    mbar_expect_tx(full_bar + 8 * stage, 3 * kPlane);
+                    const uint32_t to = smem_u32(smem) + stage * P::kStageBytes + 3 * kPlaneW;
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) tma_load_2d(to + p * kPlane, &map_a, k_begin + chunk * kChunk, p * args.m + row0, full_bar + 8 * stage);
+                }
+                if (++stage == P::kStages) stage = 0, phase ^= 1;
             }
         }
-        if (step + 1 < steps) store(buffer ^ 1);  // (the other buffer was last read a step ago, before that step's barrier)
-        __syncthreads();
-    }
-    if (parts == 1) {
-#pragma unroll
-        for (int i = 0; i < kM4 * 4; ++i) {
-            const int r = row0 + my_row + 16 * (i / 4) + i % 4;
-            if (r >= m) continue;
-#pragma unroll
-            for (int j = 0; j < kN4 * 2; ++j) {
-                const int to = col0 + my_col + 32 * (j / 2) + 2 * (j % 2);
-                if (to < n) c[(size_t)r * ldc + to] = low_of(acc[i][j]);
-                if (to + 1 < n) c[(size_t)r * ldc + to + 1] = high_of(acc[i][j]);
-            }
+        __syncwarp();
+        if (args.parts > 1) {
+            cluster_sync_all();
+            cluster_leave_together();
         }
-        return;
     }
-    // this part's sums over the tiles in shared memory (everybody is past the last step), [kRows][kCols]
-#pragma unroll
-    for (int i = 0; i < kM4 * 4; ++i) {
-        const int r = my_row + 16 * (i / 4) + i % 4;
-#pragma unroll
-        for (int j = 0; j < kN4; ++j)
-            *reinterpret_cast<float4*>(tiled_shared + r * kCols + my_col + 32 * j) =
-                make_float4(low_of(acc[i][2 * j]), high_of(acc[i][2 * j]), low_of(acc[i][2 * j + 1]), high_of(acc[i][2 * j + 1]));
+    __syncthreads();
+    if (warp == kIssuer) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_sum), "n"(P::kColumns));
     }
-    cg::this_cluster().sync();
-    const int rows_here = kRows / parts;  // (parts is 2, 4 or 8, kRows a multiple of 32)
-    for (int i = threadIdx.x; i < rows_here * kCols; i += kThreads) {
-        const int r = part * rows_here + i / kCols, col = i % kCols;
-        float sum = tiled_part(tiled_shared, 0)[r * kCols + col];
-        for (int p = 1; p < parts; ++p) sum += tiled_part(tiled_shared, p)[r * kCols + col];
-        if (row0 + r < m && col0 + col < n) c[(size_t)(row0 + r) * ldc + col0 + col] = sum;
-    }
-    cluster_leave_together();  // the others read this block's sums
 }
 
-// Few rows: the weights pass once and bound the product.  A thread owns a column and walks its weights in ascending k; they arrive
-// through a ring of kFewDepth stages of kFewStep columns, the rows' own k beside them.  Parts of K as above.
-constexpr int kFewRows = 8, kFewColumns = 64, kFewStep = 32, kFewDepth = 4;
-constexpr int kFewStride = kFewStep + 4;  // (36 floats: eight lanes' 16-byte loads meet 32 banks)
+// ---- Up to four rows of A: the weights' stream bounds the product, and nothing of W passes through shared memory.  A warp owns 16 rows of W;
+// its lanes load them 16 bytes at a time (kFewAhead chunks in registers), split them there and multiply them by mma.sync, whose sums over
+// 16 columns are the tcgen05 ones, bit by bit, in whatever order these columns stand: the same steps in the same order give the same
+// results.  A's parts lie in shared memory, split by the block itself.
+constexpr int kFewRows = 4, kFewWarps = 4, kFewThreads = 32 * kFewWarps, kFewRowsW = 16 * kFewWarps;
+constexpr int kFewBytes = 200 * 1024;  // most shared memory for A's parts
+constexpr int kFewAlone = 116 * 1024;  // with so much a block has a multiprocessor to itself
+constexpr int kFewAhead = 3;           // (2,048 rows of W, K 8,192, one row of A: 34 us with one, 25 with two, 22 with three, 33 with four)
 
-__device__ __forceinline__ void copy16_async(float* dst, const float* src, bool live) {
-    const int bytes = live ? 16 : 0;  // (0: the sixteen bytes are written as zeros and nothing is read)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+__device__ __forceinline__ void mma_step(float (&d)[4], const uint32_t (&a)[4], uint2 b) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
 }
 
-template <int kRows>
-__global__ void __launch_bounds__(kFewColumns)
-gemm_f32_few_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, float* __restrict__ c, int ldc, int m,
-                    int n, int k, int parts, int part_length) {
-    constexpr int kPieces = kFewStep / 4, kStage = (kFewColumns + kRows) * kFewStride;
-    __shared__ __align__(16) float ring[kFewDepth * kStage];
-    __shared__ float sums[kRows][kFewColumns];
-    const int part = parts > 1 ? (int)cg::this_cluster().block_rank() : 0;
-    const int col0 = (blockIdx.x / parts) * kFewColumns, tid = threadIdx.x;
-    const int k_begin = part * part_length, k_end = min(k, k_begin + part_length);
-    const int steps = (k_end - k_begin + kFewStep - 1) / kFewStep;
-    auto issue = [&](int step) {
-        float* stage = ring + (step % kFewDepth) * kStage;
-        const int at = (tid % kPieces) * 4, kk = k_begin + step * kFewStep + at;
+// Shared memory: A's parts, [row][chunk][16 columns][3 parts][4 lanes] pairs of words (a lane's two operand registers).
+template <bool kEven>
+__global__ void __launch_bounds__(kFewThreads)
+gemm_f32_few_kernel(const FloatArgs args) {
+    extern __shared__ __align__(16) uint2 few_parts[];
+    __shared__ float sums[kFewRows][kFewRowsW];
+    __shared__ int spoilt_a[kFewRows];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = lane >> 2, quad = lane & 3;
+    const int part = blockIdx.x % args.parts, col0 = (blockIdx.x / args.parts) * kFewRowsW;
+    const int k_begin = part * args.part_length, k_end = min(args.k, k_begin + args.part_length);
+    const int chunks = (k_end - k_begin + kChunk - 1) / kChunk, m = args.m;
+    grid_launch_dependents();
+    if (threadIdx.x < kFewRows) spoilt_a[threadIdx.x] = 0;
+
+    // a lane's columns of the sixteen of a step: four from 8 * step + 4 * (quad & 1) + 32 * (quad >> 1)
+    const int my_col = 4 * (quad & 1) + 32 * (quad >> 1);
+    const float* w_from[2];  // (rows beyond the last repeat it)
 #pragma unroll
-        for (int i = 0; i < kPieces; ++i) {  // eight neighbouring threads bring the 128 bytes of a row
-            const int r = tid / kPieces + i * (kFewColumns / kPieces);
-            const bool live = col0 + r < n && kk < k_end;
-            copy16_async(stage + r * kFewStride + at, live ? w + (size_t)(col0 + r) * ldw + kk : w, live);
-        }
-        static_assert(kFewColumns / kPieces >= kFewRows, "one piece of the rows per thread");
-        if (tid / kPieces < kRows) {
-            const int r = tid / kPieces;
-            const bool live = r < m && kk < k_end;
-            copy16_async(stage + (kFewColumns + r) * kFewStride + at, live ? a + (size_t)r * lda + kk : a, live);
-        }
+    for (int h = 0; h < 2; ++h) w_from[h] = args.w + (size_t)min(col0 + warp * 16 + group + 8 * h, args.n - 1) * args.ldw + k_begin + my_col;
+    uint64_t next[kFewAhead][2][4][2] = {};  // [chunk ahead][row][step][pairs of columns]
+    auto fetch = [&](int wanted, uint64_t (&v)[2][4][2]) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int step = 0; step < 4; ++step)
+                load_four<kEven>(v[h][step], w_from[h] + wanted * kChunk + 8 * step, k_end - k_begin - my_col - wanted * kChunk - 8 * step, wanted < chunks);
     };
-    float acc[kRows];
 #pragma unroll
-    for (int r = 0; r < kRows; ++r) acc[r] = 0.0f;
+    for (int i = 0; i < kFewAhead; ++i) fetch(i, next[i]);  // weights depend on nothing
+    __syncthreads();
+    grid_dependency_wait();
+    // A's parts: a thread takes the four columns of one lane of a step
+    const int items = chunks * 16;
+    for (int r = 0; r < m; ++r)
+        for (int i = threadIdx.x; i < items; i += kFewThreads) {
+            const int q = i & 3, at = (i >> 4) * kChunk + 8 * (i >> 2 & 3) + 4 * (q & 1) + 32 * (q >> 1);
+            uint64_t v[2] = {};
+            load_four<kEven>(v, args.a + (size_t)r * args.lda + k_begin + at, k_end - k_begin - at, true);
+            uint2 hi, mid, lo;
+            split_pair(v[0], hi.x, mid.x, lo.x);
+            split_pair(v[1], hi.y, mid.y, lo.y);
+            uint2* to = few_parts + (r * chunks * 4 + (i >> 2)) * 12 + q;
+            to[0] = hi, to[4] = mid, to[8] = lo;
+            const uint64_t fit = pair_fma(v[0], 0x4080000040800000ull, pair_fma(v[1], 0x4080000040800000ull, 0));
+            if (!isfinite(low_of(fit) + high_of(fit))) spoilt_a[r] = 1;
+        }
+    __syncthreads();
+
+    float sum[4] = {}, small[4] = {};
+    uint64_t fit[2] = {0, 0};
+    const bool live = group < m;
+    const uint2* mine = few_parts + (live ? group : 0) * chunks * 48 + quad;
+    for (int chunk0 = 0; chunk0 < chunks; chunk0 += kFewAhead) {
 #pragma unroll
-    for (int s = 0; s < kFewDepth - 1; ++s) {
-        if (s < steps) issue(s);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    for (int step = 0; step < steps; ++step) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(kFewDepth - 2) : "memory");
-        __syncthreads();  // the stage is there for everybody, and everybody is done with the one before
-        if (step + kFewDepth - 1 < steps) issue(step + kFewDepth - 1);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        const float* stage = ring + (step % kFewDepth) * kStage;
+        for (int i = 0; i < kFewAhead; ++i) {
+            const int chunk = chunk0 + i;
+            if (chunk >= chunks) break;
+            uint32_t w[4][3][4];  // [step][part][operand registers: row and row + 8 of the first two columns, then of the others]
+            uint2 a[4][3];
+            uint32_t smaller = 0;
 #pragma unroll
-        for (int i = 0; i < kPieces; ++i) {
-            const float4 wv = *reinterpret_cast<const float4*>(stage + tid * kFewStride + 4 * i);
+            for (int step = 0; step < 4; ++step) {
 #pragma unroll
-            for (int r = 0; r < kRows; ++r) {
-                const float4 x = *reinterpret_cast<const float4*>(stage + (kFewColumns + r) * kFewStride + 4 * i);
-                acc[r] = fmaf(x.x, wv.x, acc[r]);
-                acc[r] = fmaf(x.y, wv.y, acc[r]);
-                acc[r] = fmaf(x.z, wv.z, acc[r]);
-                acc[r] = fmaf(x.w, wv.w, acc[r]);
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const uint64_t v = next[i][h][step][e];
+                        split_pair(v, w[step][0][2 * e + h], w[step][1][2 * e + h], w[step][2][2 * e + h]);
+                        smaller |= w[step][1][2 * e + h] | w[step][2][2 * e + h];
+                        fit[h] = pair_fma(v, 0x4080000040800000ull, fit[h]);
+                    }
+#pragma unroll
+                for (int p = 0; p < 3; ++p) a[step][p] = live ? mine[(chunk * 4 + step) * 12 + p * 4] : make_uint2(0u, 0u);
             }
+            fetch(chunk + kFewAhead, next[i]);
+            const bool all_parts = __any_sync(0xffffffffu, (smaller & 0x7fff7fffu) != 0);
+            auto products = [&](int w_part, int a_part, float (&to)[4]) {
+#pragma unroll
+                for (int step = 0; step < 4; ++step) mma_step(to, w[step][w_part], a[step][a_part]);
+            };
+            float whole[4] = {};
+            products(0, 0, whole);
+            products(0, 2, small);
+            if (all_parts) {
+                products(1, 1, small);
+                products(2, 0, small);
+            }
+            products(0, 1, small);
+            if (all_parts) products(1, 0, small);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum[j] += whole[j];
         }
     }
-    if (parts > 1) {
+    // a lane holds rows group and group + 8 of the warp's sixteen of W, rows 2 * quad and 2 * quad + 1 of A
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) sums[r][tid] = acc[r];
+    for (int h = 0; h < 2; ++h) {
+        const bool bad = (__ballot_sync(0xffffffffu, !isfinite(low_of(fit[h]) + high_of(fit[h]))) >> (lane & 28) & 15u) != 0;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int r = 2 * quad + e, of_block = warp * 16 + group + 8 * h, col = col0 + of_block;
+            if (r >= m) continue;
+            float total = sum[2 * h + e] + small[2 * h + e];
+            if (bad || spoilt_a[r] != 0) {
+                const float *a = args.a + (size_t)r * args.lda, *w = args.w + (size_t)min(col, args.n - 1) * args.ldw;
+                total = 0.0f;
+#pragma unroll 1
+                for (int k = k_begin; k < k_end; ++k) total = fmaf(a[k], w[k], total);
+            }
+            if (args.parts > 1) sums[r][of_block] = total;
+            else if (col < args.n) args.c[(size_t)r * args.ldc + col] = total;
+        }
+    }
+    if (args.parts > 1) {  // the first block of the cluster adds the parts in their order
         cg::this_cluster().sync();
         if (part == 0)
+            for (int i = threadIdx.x; i < m * kFewRowsW; i += kFewThreads) {
+                const int r = i / kFewRowsW, col = i % kFewRowsW;
+                float v[4];
 #pragma unroll
-            for (int r = 0; r < kRows; ++r)
-                for (int p = 1; p < parts; ++p) acc[r] += tiled_part(&sums[0][0], p)[r * kFewColumns + tid];
+                for (int p = 0; p < 4; ++p)
+                    if (p < args.parts) v[p] = cg::this_cluster().map_shared_rank(&sums[0][0], p)[i];
+                float total = v[0];
+#pragma unroll
+                for (int p = 1; p < 4; ++p)
+                    if (p < args.parts) total += v[p];
+                if (col0 + col < args.n) args.c[(size_t)r * args.ldc + col0 + col] = total;
+            }
         cluster_leave_together();
-        if (part != 0) return;
-    }
-    if (col0 + tid < n)
-#pragma unroll
-        for (int r = 0; r < kRows; ++r)
-            if (r < m) c[(size_t)r * ldc + col0 + tid] = acc[r];
-}
-
-// Few rows (decode): one warp per output column, lanes stride over K, rows kept in registers.
-// The per-lane partial sums are combined in a fixed butterfly, so results are reproducible; the
-// order differs from the other kernels' sums of chains, which is rounding only.
-template <int kRows>
-__global__ void __launch_bounds__(256)
-gemv_f32_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, float* __restrict__ c,
-                int ldc, int m, int n, int k) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const float* w_row = w + (size_t)warp * ldw;
-    float acc[kRows];
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) acc[r] = 0.0f;
-    for (int kk = lane; kk < k; kk += 32) {
-        const float wv = w_row[kk];
-#pragma unroll
-        for (int r = 0; r < kRows; ++r)
-            if (r < m) acc[r] = fmaf(a[(size_t)r * lda + kk], wv, acc[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-        const float total = warp_sum(acc[r]);
-        if (lane == 0 && r < m) c[(size_t)r * ldc + warp] = total;
     }
 }
 
-template <typename... Params, typename... Args>
-static int launch_parts(void (*kernel)(Params...), unsigned blocks, int threads, int smem, int parts, cudaStream_t stream, Args... args) {
-    if (smem > 48 * 1024) {
-        cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (status != cudaSuccess) return fail("gemm_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(status));
-    }
+template <int NB, int kRowsW, bool kEven>
+static int launch(const CUtensorMap& map_a, const FloatArgs& args, cudaStream_t stream) {
+    using P = Plan<NB, kRowsW>;
+    auto kernel = gemm_f32_kernel<NB, kRowsW, kEven>;
+    static const cudaError_t reserved = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::kBytes);
+    if (reserved != cudaSuccess) return fail("gemm_f32: cannot reserve %d bytes of shared memory: %s", P::kBytes, cudaGetErrorString(reserved));
+    const long long blocks = (long long)((args.n + kRowsW - 1) / kRowsW) * ((args.m + P::kRows - 1) / P::kRows) * args.parts;
+    if (blocks > 0x7fffffff) return fail("gemm_f32: %d x %d results exceed the grid limit", args.m, args.n);
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(blocks);
-    config.blockDim = dim3(threads);
-    config.dynamicSmemBytes = smem;
+    config.gridDim = dim3((unsigned)blocks);
+    config.blockDim = dim3(kThreads);
+    config.dynamicSmemBytes = P::kBytes;
     config.stream = stream;
-    cudaLaunchAttribute attribute[1];
+    cudaLaunchAttribute attribute[2];
     attribute[0].id = cudaLaunchAttributeClusterDimension;
-    attribute[0].val.clusterDim.x = parts;
+    attribute[0].val.clusterDim.x = args.parts;
     attribute[0].val.clusterDim.y = 1;
     attribute[0].val.clusterDim.z = 1;
+    attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attribute;
-    config.numAttrs = parts > 1 ? 1 : 0;
-    cudaError_t status = cudaLaunchKernelEx(&config, kernel, args...);
+    config.numAttrs = dependent_launches_allowed() ? 2 : 1;
+    const cudaError_t status = cudaLaunchKernelEx(&config, kernel, map_a, args);
     if (status != cudaSuccess) return fail("gemm_f32: launch failed: %s", cudaGetErrorString(status));
     return check_launch("gemm_f32");
 }
 
-template <int kWarpsM, int kWarpsN, int kM4, int kN4>
-static int launch_tiled(const float* a, int lda, const float* w, int ldw, float* c, int ldc, int m, int n, int k, int parts, int part_length,
-                        cudaStream_t stream) {
-    constexpr int kRows = kWarpsM * 16 * kM4, kCols = kWarpsN * 32 * kN4;
-    constexpr int tiles_bytes = 2 * kTileK * (kRows + kCols) * (int)sizeof(float), sums_bytes = kRows * kCols * (int)sizeof(float);
-    const long long tiles_n = (n + kCols - 1) / kCols, blocks = tiles_n * ((m + kRows - 1) / kRows) * parts;
-    if (blocks > 0x7fffffff) return fail("gemm_f32: %d x %d results exceed the grid limit", m, n);
-    return launch_parts(gemm_f32_tiled_kernel<kWarpsM, kWarpsN, kM4, kN4>, (unsigned)blocks, kWarpsM * kWarpsN * 32,
-                        parts > 1 && sums_bytes > tiles_bytes ? sums_bytes : tiles_bytes, parts, stream, a, lda, w, ldw, c, ldc, m, n, k,
-                        (int)tiles_n, parts, part_length);
+template <bool kEven>
+static int launch_few(const FloatArgs& args, cudaStream_t stream) {
+    int bytes = args.part_length * args.m * 6;
+    static const cudaError_t reserved = cudaFuncSetAttribute(gemm_f32_few_kernel<kEven>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewBytes);
+    if (reserved != cudaSuccess) return fail("gemm_f32: cannot reserve %d bytes of shared memory: %s", kFewBytes, cudaGetErrorString(reserved));
+    const long long blocks = (long long)((args.n + kFewRowsW - 1) / kFewRowsW) * args.parts;
+    if (blocks > 0x7fffffff) return fail("gemm_f32: %d x %d results exceed the grid limit", args.m, args.n);
+    cudaLaunchConfig_t config = {};
+    if (blocks <= 148) bytes = std::max(bytes, kFewAlone);  // (the blocks of a cluster share a multiprocessor where two fit, and leave others idle)
+    config.gridDim = dim3((unsigned)blocks);
+    config.blockDim = dim3(kFewThreads);
+    config.dynamicSmemBytes = bytes;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[2];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = args.parts;
+    attribute[0].val.clusterDim.y = 1;
+    attribute[0].val.clusterDim.z = 1;
+    attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attribute;
+    config.numAttrs = dependent_launches_allowed() ? 2 : 1;
+    const cudaError_t status = cudaLaunchKernelEx(&config, gemm_f32_few_kernel<kEven>, args);
+    if (status != cudaSuccess) return fail("gemm_f32: launch failed: %s", cudaGetErrorString(status));
+    return check_launch("gemm_f32");
 }
 
-template <int kRows>
-static int launch_few(const float* a, int lda, const float* w, int ldw, float* c, int ldc, int m, int n, int k, int parts, int part_length,
-                      cudaStream_t stream) {
-    return launch_parts(gemm_f32_few_kernel<kRows>, (unsigned)((n + kFewColumns - 1) / kFewColumns * parts), kFewColumns, 0, parts, stream, a, lda,
-                        w, ldw, c, ldc, m, n, k, parts, part_length);
+template <int NB, int kRowsW>
+static int launch_rows(const CUtensorMap& map_a, const FloatArgs& args, bool even, cudaStream_t stream) {
+    return even ? launch<NB, kRowsW, true>(map_a, args, stream) : launch<NB, kRowsW, false>(map_a, args, stream);
 }
+
+static size_t plane_bytes(int m, int k) { return (size_t)m * ((k + kChunk - 1) / kChunk) * 128; }
 
 }  // namespace mb
 
 using namespace mb;
 
+// Bytes of scratch that a product of m rows and k columns takes (0 for few rows); they start on a 16-byte boundary.
+MB_EXPORT size_t mb_gemm_f32_scratch(int m, int k) {
+    const int rows = std::min(m, kSlabRows);
+    return m <= kInlineRows ? 0 : 3 * plane_bytes(rows, k) + (size_t)rows * ((k + kChunk - 1) / kChunk);
+}
+
 // A: [m, k] with row stride lda; W: [n, k] with row stride ldw; C: [m, n] with row stride ldc.
-// `row_invariant` != 0 always takes kernels whose result for a row does not depend on m.
-MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, float* c, int ldc, int m, int n, int k,
-                          int row_invariant, cudaStream_t stream) {
+MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, float* c, int ldc, int m, int n, int k, void* scratch,
+                          cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return fail("gemm_f32: k %d must be positive", k);
     if (lda < k || ldw < k || ldc < n) return fail("gemm_f32: row strides (%d, %d, %d) are shorter than the rows (%d, %d, %d)", lda, ldw, ldc, k, k, n);
-    if (!row_invariant && m <= 8) {
-        const int blocks = (n * 32 + 255) / 256;
-        gemv_f32_kernel<8><<<blocks, 256, 0, stream>>>(a, lda, w, ldw, c, ldc, m, n, k);
-        return check_launch("gemv_f32");
+    if (m > kInlineRows && (scratch == nullptr || ((uintptr_t)scratch & 15))) return fail("gemm_f32: scratch for the split rows is missing or not on a 16-byte boundary");
+    FloatArgs args{a, w, c, lda, ldw, ldc, m, n, k, 1, 0, nullptr};
+    // Parts of K, by n and k alone, so that every m gives a row the same bits: matrices of few tiles put more multiprocessors to work.
+    const int tiles = (n + kTileN - 1) / kTileN;
+    auto length = [&](int parts) { return ((k + parts - 1) / parts + kChunk - 1) / kChunk * kChunk; };
+    args.parts = tiles <= 37 ? 4 : tiles <= 74 ? 2 : 1;
+    while (args.parts > 1 && (k < 2 * kChunk * args.parts || length(args.parts) * (args.parts - 1) >= k)) args.parts /= 2;
+    args.part_length = length(args.parts);
+    const bool even_w = k % kChunk == 0 && ldw % 4 == 0 && !((uintptr_t)w & 15), even_a = k % kChunk == 0 && lda % 4 == 0 && !((uintptr_t)a & 15);
+    if (m <= kFewRows && (long long)args.part_length * m * 6 <= kFewBytes) return even_w && even_a ? launch_few<true>(args, stream) : launch_few<false>(args, stream);
+    CUtensorMap map_a{};
+    if (m <= kInlineRows) {
+        // 64 rows of W a block while that puts more multiprocessors to work.
+        if (tiles * args.parts <= 74) return launch_rows<1, 64>(map_a, args, even_w && even_a, stream);
+        return launch_rows<1, 128>(map_a, args, even_w && even_a, stream);
     }
-    // Parts of K, by n and k alone, so that every m and every kernel gives a row the same bits: one chain of 2,048 to 8,192
-    // products per result leaves a matrix of few columns with too few of them at work (384 rows, 2,048 columns, K 8,192: 689 us
-    // whole, 322 in eight; 2,048 columns, K 2,048: 174 and 94), and shorter chains round less (1.6e-6 and 0.6e-6 from the sums
-    // in 64 bits).  Wide matrices gain less (16,384 columns: 596 us whole, 576 in four, 625 in eight).
-    int parts = n <= 8192 ? 8 : 4;
-    while (parts > 1 && k < 128 * parts) parts /= 2;
-    const int part_length = ((k + parts - 1) / parts + kFewStep - 1) / kFewStep * kFewStep;
-    if (k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)a & 15) && !((uintptr_t)w & 15)) {
-        if (m <= kFewRows) {
-            if (m <= 2) return launch_few<2>(a, lda, w, ldw, c, ldc, m, n, k, parts, part_length, stream);
-            if (m <= 4) return launch_few<4>(a, lda, w, ldw, c, ldc, m, n, k, parts, part_length, stream);
-            return launch_few<8>(a, lda, w, ldw, c, ldc, m, n, k, parts, part_length, stream);
+    const int chunks = (k + kChunk - 1) / kChunk;
+    for (int first = 0; first < m; first += kSlabRows) {
+        args.m = std::min(kSlabRows, m - first);
+        args.a = a + (size_t)first * lda;
+        args.c = c + (size_t)first * ldc;
+        unsigned char* planes = static_cast<unsigned char*>(scratch);
+        unsigned char* unfit = planes + 3 * plane_bytes(args.m, k);
+        args.unfit = unfit;
+        const unsigned blocks = (unsigned)(((size_t)args.m * chunks + 31) / 32);
+        int status = even_a ? launch_dependent("gemm_f32", split_rows_kernel<true>, dim3(blocks), dim3(256), 0, stream, true, args.a, lda, args.m, k, chunks, planes, unfit)
+                            : launch_dependent("gemm_f32", split_rows_kernel<false>, dim3(blocks), dim3(256), 0, stream, true, args.a, lda, args.m, k, chunks, planes, unfit);
+        if (status) return status;
+        // As few tiles of A as there must be, and these as low as that allows.
+        const int a_tiles = (args.m + 159) / 160, rows = (args.m + a_tiles - 1) / a_tiles, nb = std::max(2, (rows + 31) / 32);
+        if ((status = make_map(&map_a, planes, 3 * args.m, chunks * kChunk, chunks * kChunk, 32 * nb))) return status;
+        switch (nb) {
+            case 2: status = launch_rows<2, 128>(map_a, args, even_w, stream); break;
+            case 3: status = launch_rows<3, 128>(map_a, args, even_w, stream); break;
+            case 4: status = launch_rows<4, 128>(map_a, args, even_w, stream); break;
+            default: status = launch_rows<5, 128>(map_a, args, even_w, stream);
         }
-        // Tiles of 64 x 128 where there are two or more per multiprocessor (64 rows, 16,384 columns: 121 us, and 152 in tiles of
-        // 32 x 64); else, and where they would be half empty, of 32 x 64 (64 rows, 2,048 columns, K 8,192: 90 us, and 120).
-        const long long tiles = (long long)((m + 63) / 64) * ((n + 127) / 128) * parts;
-        if (m <= 32 || tiles < 296) return launch_tiled<2, 1, 1, 2>(a, lda, w, ldw, c, ldc, m, n, k, parts, part_length, stream);
-        return launch_tiled<2, 2, 2, 2>(a, lda, w, ldw, c, ldc, m, n, k, parts, part_length, stream);
+        if (status) return status;
     }
-    const dim3 grid((n + kTileN - 1) / kTileN, (m + kTileM - 1) / kTileM);
-    if (grid.y > 65535) return fail("gemm_f32: %d rows exceed the grid limit", m);
-    gemm_f32_kernel<<<grid, 256, 0, stream>>>(a, lda, w, ldw, c, ldc, m, n, k, part_length);
-    return check_launch("gemm_f32");
+    return 0;
+}
+
+// 0 when no wait ever gave up; else 1 + (role << 8): 1 splitter, 2 and 3 issuer (operands, sums), 4 and 5 adder, 6 bringer.
+MB_EXPORT int mb_gemm_f32_status() {
+    int status = 0;
+    if (cudaMemcpyFromSymbol(&status, g_gemm_status, sizeof(int)) != cudaSuccess) return -1;
+    return status;
 }

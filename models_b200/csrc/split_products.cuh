@@ -3,8 +3,7 @@
 // other three are below 2^-26 of the product).  Operands lie in shared memory as three planes, one after another.
 #pragma once
 
-#include <cuda_bf16.h>
-#include <stdint.h>
+#include "float_parts.cuh"
 
 namespace mb {
 
@@ -22,18 +21,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// Two floats as pairs of bfloat16 numbers: their roundings, the roundings of what those left, and of what these left.
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    float2 back = __bfloat1622float2(h);
-    a -= back.x, b -= back.y;
-    const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
-    back = __bfloat1622float2(m);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(a - back.x, b - back.y);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    mid = *reinterpret_cast<const uint32_t*>(&m);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 // Two floats, and eight, into an operand's three planes.
 __device__ __forceinline__ void split_two(float a, float b, bf16* at, int plane) {
@@ -81,14 +68,6 @@ __device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], c
     for (int i = 0; i < 4; ++i) d0[i] += p0[i] + r0[i], d1[i] += p1[i] + r1[i];
 }
 
-// A sum that is finite only where eight floats are, and have three finite parts.  (The largest bfloat16 number is a little smaller than the
-// largest float: four times what lies between them is infinite.)
-__device__ __forceinline__ float fitness(const float (&x)[8]) {
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) sum = fmaf(x[j], 4.0f, sum);
-    return sum;
-}
 // A float from its parts, and the float dot product of two rows of parts.
 __device__ __forceinline__ float whole_one(const bf16* at, int plane) {
     const float hi = __bfloat162float(at[0]);

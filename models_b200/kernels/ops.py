@@ -1747,7 +1747,8 @@ def prefill_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, 
 # ------------------------------------------------------------------------------------ matrix products
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, row_invariant: bool = True) -> torch.Tensor:
-    """a [m, k] . w[n, k]^T in true 32-bit arithmetic."""
+    """a [m, k] . w[n, k]^T in 32 bits: every bit of the floats is multiplied, and a row's result depends on
+    nothing but that row (`row_invariant` or not)."""
     _cuda(a, w)
     if a.dtype != torch.float32 or w.dtype != torch.float32:
         raise KernelError(f"gemm_f32 takes float32 operands, got {a.dtype} and {w.dtype}")
@@ -1757,8 +1758,10 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, row_invariant: bool = True) -> to
     n = w.shape[0]
     c = torch.empty((m, n), dtype=torch.float32, device=a.device)
     lib = gemm32()
-    _run(lib, lib.mb_gemm_f32(_p(a), a.stride(0), _p(w), w.stride(0), _p(c), n, m, n, k, 1 if row_invariant else 0,
-                              _stream()))
+    lib.mb_gemm_f32_scratch.restype = ctypes.c_size_t
+    need = lib.mb_gemm_f32_scratch(m, k)
+    scratch = torch.empty((need,), dtype=torch.uint8, device=a.device) if need else None
+    _run(lib, lib.mb_gemm_f32(_p(a), a.stride(0), _p(w), w.stride(0), _p(c), n, m, n, k, _p(scratch), _stream()))
     return c
 
 
@@ -2220,6 +2223,11 @@ def tensor_core_gemm(a: torch.Tensor, weight: torch.Tensor, epilogue: int = EPI_
 def prefill_attention_tcgen05_status(head_dim: int) -> int:
     """0 unless a bounded wait inside the tcgen05 prefill attention ever gave up (1 + (role << 8))."""
     return int(prefill_attention_tc(head_dim).mb_prefill_attention_tc_status())
+
+
+def gemm_f32_status() -> int:
+    """0 while no wait of the 32-bit product ever gave up (see csrc/gemm_f32.cu)."""
+    return gemm32().mb_gemm_f32_status()
 
 
 def gemm_tcgen05_status() -> int:

@@ -99,6 +99,58 @@ def test_gemm_f32_rows_of_pieces(cuda_device, m, n, k):
             assert torch.equal(ops.gemm_f32(a[:rows], w), out[:rows])  # whichever kernel and tile a row meets
 
 
+@pytest.mark.parametrize("weights", ["floats", "bfloat16", "mixed"])
+@pytest.mark.parametrize("m,n,k", [(161, 129, 640), (321, 65, 63), (200, 5000, 576), (2049, 130, 1088)])
+def test_gemm_f32_gives_a_row_the_same_bits_in_every_kernel(cuda_device, weights, m, n, k):
+    """Up to 4 rows, up to 32, and tiles of 64 to 160; more rows than are split at once; weights whose smaller parts are zero, are
+    not, and are in some tiles."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(m + n)
+    a, w = torch.randn(m, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    if weights != "floats":
+        rounded = w.bfloat16().float()
+        w = rounded if weights == "bfloat16" else torch.where(torch.arange(n, device=cuda_device)[:, None] == 70 % n, w, rounded)
+    out = ops.gemm_f32(a, w)
+    exact = a.double() @ w.double().t()
+    # three parts hold 24 bits of each factor and drop 2^-26 of a product; sums over 64 columns are cut off four times (2^-23 each),
+    # the sums of these are rounded k / 64 + 8 times
+    bound = (2.0 ** -21 + (k / 64 + 8) * 2.0 ** -24) * (a.abs().double() @ w.abs().double().t())
+    assert bool(((out.double() - exact).abs() <= bound).all())
+    for rows in (1, 4, 5, 32, 33, 65, 97, 129, 160, 161):
+        for first in {0, m - rows}:
+            if 0 <= first:
+                assert torch.equal(ops.gemm_f32(a[first:first + rows], w), out[first:first + rows])
+    assert ops.gemm_f32_status() == 0
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
+@pytest.mark.parametrize("m", [3, 20, 70, 200])
+def test_gemm_f32_keeps_rows_that_are_not_finite_apart(cuda_device, m, value):
+    """A float without three finite parts, in a row of A and in one of W: their results are those of the floats, all others stay."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(m)
+    a, w = torch.randn(m, 1088, generator=g).cuda(), (torch.randn(200, 1088, generator=g) * 0.01).cuda()
+    a[:, 3] *= 0.1  # (so that products with the largest value stay within the floats)
+    before = ops.gemm_f32(a, w)
+    a2, w2 = a.clone(), w.clone()
+    a2[2, 700] = value
+    w2[130, 3] = value
+    w2[17, 700] = 0.0
+    before[:, 17] = ops.gemm_f32(a, w2)[:, 17]
+    got, want = ops.gemm_f32(a2, w2).cpu(), (a2.double() @ w2.double().t()).cpu()
+    rows, columns = torch.arange(m) == 2, torch.arange(200) == 130
+    hit = rows[:, None] | columns[None]
+    assert torch.equal(got[~hit], before.cpu()[~hit])
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    for x, y in zip(got[hit].tolist(), want[hit].tolist()):
+        if abs(y) == float("inf"):
+            assert x == y
+        elif y == y:
+            assert abs(x - y) <= 1e-5 * abs(y) + 1e-4
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 72, 2048), (5, 200, 260), (40, 130, 1028), (70, 8200, 516), (130, 64, 2048)])
 def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
     """Operands whose rows do not start on 16 bytes meet another kernel: the same chains over the same parts of K."""
