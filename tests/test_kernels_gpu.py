@@ -290,6 +290,37 @@ def test_paged_attention_rows(cuda_device, dtype, heads, kv_heads, head_dim, win
     close(out, expected, dtype)
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,window", [(8, 2, 64, None), (3, 1, 64, None), (40, 1, 64, 37), (2, 2, 128, None), (6, 2, 128, 70)])
+def test_prompt_rows_of_floats_are_the_single_tokens_bits(cuda_device, heads, kv_heads, head_dim, window):
+    """Prompts in tiles of 16 rows (heads that do not fill or do not divide one, windows that end in a chunk, cached positions before) against the
+    kernel of a warp a row, which single tokens take: the same bits, also beside a later position whose key and value are not finite."""
+    from models_b200.kernels import ops
+
+    page = 64
+    q_lens, kv_lens = [1, 70, 5, 33], [1, 70, 133, 200]
+    pages_needed = [-(-n // page) for n in kv_lens]
+    k_pool, v_pool = (t.cuda() for t in _pools(sum(pages_needed) + 1, kv_heads, page, head_dim, torch.float32, 6))
+    table, at = torch.zeros(len(q_lens), max(pages_needed), dtype=torch.int32), 1
+    for b, n in enumerate(pages_needed):
+        table[b, :n] = torch.arange(at, at + n, dtype=torch.int32)
+        at += n
+    k_pool[1, :, 1:], v_pool[1, :, 1:] = float("nan"), float("nan")  # behind the first sequence's end
+    last = int(table[1, 69 // page])
+    v_pool[last, :, 69 % page] = float("inf")  # the second sequence's last position: only its last token sees it
+    q = torch.randn(sum(q_lens), heads * head_dim, generator=torch.Generator().manual_seed(8)).cuda()
+    cu_q = torch.tensor([0] + list(np.cumsum(q_lens)), dtype=torch.int32).cuda()
+    out = torch.zeros_like(q)
+    ops.paged_attention_rows(q, out, k_pool, v_pool, table.cuda(), cu_q, torch.tensor(kv_lens, dtype=torch.int32).cuda(), max(q_lens), heads,
+                             kv_heads, head_dim, window, 0.1)
+    singles = [(b, kv_lens[b] - q_lens[b] + i + 1) for b in range(len(q_lens)) for i in range(q_lens[b])]
+    alone = torch.zeros_like(q)
+    ops.paged_attention_rows(q, alone, k_pool, v_pool, table[[b for b, _ in singles]].contiguous().cuda(),
+                             torch.arange(len(singles) + 1, dtype=torch.int32).cuda(),
+                             torch.tensor([n for _, n in singles], dtype=torch.int32).cuda(), 1, heads, kv_heads, head_dim, window, 0.1)
+    assert torch.equal(out.nan_to_num(nan=7.0), alone.nan_to_num(nan=7.0))
+    assert bool(torch.isfinite(out[:70]).all()) and not bool(torch.isfinite(out[70]).all())
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,window", [(4, 2, 16, None), (3, 1, 32, None), (6, 3, 48, None),
                                                             (32, 8, 64, None), (8, 2, 128, None), (5, 5, 80, 37),
                                                             (4, 1, 64, 64), (40, 2, 64, None), (2, 1, 256, 100)])
