@@ -21,7 +21,7 @@
 // results by 1.4e-7 (2e-7).
 // One sequence of 2,048 tokens, 16 heads of 64 x 128: the walk's chain of 2,048 tokens is bound by its latency (618 us, and 30 for
 // the kernels around it); the three kernels took 58, 105 and 71 us as float multiply-adds, bound by what the operands take from
-// shared memory and by the latency of few warps; 54, 67 and 60 here (a layer: 310 us, and 247 to 250), where the carrying kernel is bound by
+// shared memory and by the latency of few warps; 47, 45 and 58 here (a layer: 310 us, and 220), where the carrying kernel is bound by
 // its chunk's two products one after the other, the others by six products for one and the splitting of what they read.
 #include "common.cuh"
 #include "split_products.cuh"
@@ -33,7 +33,7 @@ namespace mb {
 constexpr int kChunk = 64;    // tokens of a chunk
 constexpr int kDim = 64;      // a key head's coordinates
 constexpr int kColumns = 16;  // columns of S that a block of the carrying kernel owns
-constexpr int kCarryThreads = 128, kResultThreads = 256;
+constexpr int kCarryThreads = 256, kResultThreads = 256;
 constexpr int kRow = kDim + 8;            // bfloat16 numbers of a padded row of 64: ldmatrix without bank conflicts
 constexpr int kPlane = kChunk * kRow;
 constexpr int kNarrowRow = kColumns + 8;  // and of rows of 16
@@ -52,8 +52,8 @@ struct DeltaChunkArgs {
     void* out;
     int out_stride;
     int heads, kv_heads;
-    // scratch by (place of the chunk, head): x, then u [64][V]; S_0 [64][V]; in three parts y [64 i][64 d] and weighted keys [64 i][64 d];
-    // sums of log g [64]
+    // scratch by (place of the chunk, head): x, then u [64][V]; S_0 [64][V]; in three parts y [64 i][64 d] and weighted keys [64 i][64 d], as
+    // `turned` says; sums of log g [64]
     float *u, *starts;
     bf16 *y, *keys;
     double* logs;
@@ -62,9 +62,6 @@ struct DeltaChunkArgs {
 __device__ __forceinline__ float sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float softplus(float v) { return fmaxf(v, 0.0f) + log1pf(expf(-fabsf(v))); }
 
-__device__ __forceinline__ void copy16_async(bf16* dst, const bf16* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ float2 load_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ float2 load_pair(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 __device__ __forceinline__ void store_pair(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
@@ -73,6 +70,10 @@ __device__ __forceinline__ void store_pair(bf16* p, float a, float b) { *reinter
 // Where a chunk's scratch lies: every sequence's chunks one after another, a sequence's first place being floor(first / 64) + seq
 // (a sequence of n tokens has ceil(n / 64) chunks, and floor(f / 64) + ceil(n / 64) <= floor((f + n) / 64) + 1).
 __device__ __forceinline__ size_t place_of(int first, int seq, int chunk) { return (size_t)(first / kChunk) + seq + chunk; }
+
+// Where number d of row i of a plane of y or of keys lies: the carrying kernel copies planes as they are, and its ldmatrix reads rows of 128
+// bytes without bank conflicts if their 16-byte units are turned by the row.
+__device__ __forceinline__ int turned(int i, int d) { return i * kDim + ((d >> 3 ^ (i & 7)) << 3) + (d & 7); }
 
 // Four floats as their parts.
 __device__ __forceinline__ void split_four(float4 v, bf16* at, int plane) {
@@ -178,13 +179,13 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
     if (tid >= 32 && tid < kChunk) logs[tid] = log_g + logs[31];
     __syncthreads();
     {
-        bf16* weighted = args.keys + kParts * at * kChunk * kDim + (tid % 16) * 4;
+        bf16* weighted = args.keys + kParts * at * kChunk * kDim;
 #pragma unroll
         for (int i = 0; i < k.passes; ++i) {
             const int row = tid / 16 + k.at_once * i;
             if (row >= kChunk) break;
             const float to_end = expf((float)(logs[kChunk - 1] - logs[row]));
-            split_four(make_float4(to_end * k.x[i].x, to_end * k.x[i].y, to_end * k.x[i].z, to_end * k.x[i].w), weighted + row * kDim, kChunk * kDim);
+            split_four(make_float4(to_end * k.x[i].x, to_end * k.x[i].y, to_end * k.x[i].z, to_end * k.x[i].w), weighted + turned(row, (tid % 16) * 4), kChunk * kDim);
         }
         if (tid < kChunk) args.logs[at * kChunk + tid] = logs[tid];
     }
@@ -298,7 +299,7 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
                 store_pair(x, acc[n][0], acc[n][1]);
                 store_pair(x + 8 * V, acc[n][2], acc[n][3]);
             } else {
-                bf16* y = args.y + kParts * at * kChunk * kDim + (size_t)row * kDim + column0 - V + 8 * n + pair;
+                bf16* y = args.y + kParts * at * kChunk * kDim + turned(row, column0 - V + 8 * n + pair);  // (row + 8 is turned alike)
                 split_two(acc[n][0], acc[n][1], y, kChunk * kDim);
                 split_two(acc[n][2], acc[n][3], y + 8 * kDim, kChunk * kDim);
             }
@@ -322,17 +323,42 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
             } else {
                 uint32_t hi, mid, lo;
                 split_pair(sum, 0.0f, hi, mid, lo);
-                unsigned short* y = reinterpret_cast<unsigned short*>(args.y + kParts * at * kChunk * kDim + (size_t)i * kDim + column - V);
+                unsigned short* y = reinterpret_cast<unsigned short*>(args.y + kParts * at * kChunk * kDim + turned(i, column - V));
                 y[0] = (unsigned short)hi, y[kChunk * kDim] = (unsigned short)mid, y[2 * kChunk * kDim] = (unsigned short)lo;
             }
         }
     }
 }
 
-// grid (V / kColumns, heads, sequences); block kCarryThreads: a warp has 16 coordinates of S (and 16 tokens of u) at the block's columns,
-// as its products leave them.  The next chunk's y and keys arrive by cp.async, its x in registers, while this one's are used.
-constexpr int kCarryStage = 2 * kParts * kPlane;                                          // y, keys
-constexpr int kCarryBytes = (2 * kCarryStage + 2 * kParts * kNarrowPlane) * 2;            // and S, u
+// grid (V / kColumns, heads, sequences); block kCarryThreads: a warp has 16 coordinates of S (and 16 tokens of u) at eight of the block's
+// columns, as its products leave them.  The next two chunks' y and keys arrive by bulk copies, the next one's x in registers, while this one's are
+// used.  (Bound by the latency of the two products one after the other.  2,048 tokens: 65 us with four warps of sixteen columns each, one to a
+// scheduler, 59 with eight; 45.5 when the copies were no longer 3,072 of 16 bytes, whose issue took 850 of a chunk's 3,100 cycles.)
+constexpr int kCarryPlane = kChunk * kDim;
+constexpr int kCarryStage = 2 * kParts * kCarryPlane, kCarryStages = 3;                    // y, keys
+constexpr int kCarryBytes = (kCarryStages * kCarryStage + 2 * kParts * kNarrowPlane) * 2;  // and S, u
+
+static __device__ int g_carry_status = 0;  // 1: a copy did not arrive within about two seconds
+
+// The bounded wait for a stage: false in every thread that gave up.
+__device__ __forceinline__ bool carry_wait(uint32_t bar, uint32_t parity) {
+    const long long start = clock64();
+    uint32_t done = 0;
+    for (;;) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (clock64() - start > 4000000000LL) {
+            atomicExch(&g_carry_status, 1);
+            return false;
+        }
+    }
+}
 
 template <int V>
 __global__ void __launch_bounds__(kCarryThreads)
@@ -340,97 +366,104 @@ delta_chunks_carry_kernel(const DeltaChunkArgs args) {
     grid_launch_dependents();
     grid_dependency_wait();
     extern __shared__ __align__(16) unsigned char shared[];
+    __shared__ __align__(8) uint64_t arrived[kCarryStages];
     bf16* stages = reinterpret_cast<bf16*>(shared);
-    bf16 *s_planes = stages + 2 * kCarryStage, *u_planes = s_planes + kParts * kNarrowPlane;
+    bf16 *s_planes = stages + kCarryStages * kCarryStage, *u_planes = s_planes + kParts * kNarrowPlane;
     const int column0 = blockIdx.x * kColumns, head = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
     const int first = args.cu_q[seq], tokens = args.cu_q[seq + 1] - first;
     if (tokens <= 0) return;
     const int chunks = (tokens + kChunk - 1) / kChunk;
-    const int warp = tid >> 5, group = (tid & 31) >> 2, pair = 2 * (tid & 3);
-    const int row = 16 * warp + group;  // and row + 8
+    const int warp = (tid >> 5) & 3, tile0 = 8 * (tid >> 7), group = (tid & 31) >> 2, pair = 2 * (tid & 3);
+    const int row = 16 * warp + group;             // and row + 8
+    const int column = column0 + tile0 + pair;     // and the next one
     const size_t place0 = place_of(first, seq, 0);
     auto item = [&](int chunk) { return (place0 + chunk) * args.heads + head; };
+    if (tid == 0) {
+#pragma unroll
+        for (int i = 0; i < kCarryStages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&arrived[i])));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
     auto fetch = [&](int chunk) {
-        bf16* stage = stages + (chunk & 1) * kCarryStage;
+        if (tid != 0 || chunk >= chunks) return;
+        const uint32_t bar = smem_u32(&arrived[chunk % kCarryStages]), to = smem_u32(stages + chunk % kCarryStages * kCarryStage);
+        constexpr uint32_t half = kParts * kCarryPlane * 2;
         const bf16 *y = args.y + kParts * item(chunk) * kChunk * kDim, *keys = args.keys + kParts * item(chunk) * kChunk * kDim;
-#pragma unroll
-        for (int i = tid; i < kParts * kChunk * kDim / 8; i += kCarryThreads) {  // (the planes' rows run on)
-            copy16_async(stage + i / 8 * kRow + i % 8 * 8, y + 8 * i);
-            copy16_async(stage + kParts * kPlane + i / 8 * kRow + i % 8 * 8, keys + 8 * i);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * half) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to), "l"(y), "r"(half), "r"(bar) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to + half), "l"(keys), "r"(half), "r"(bar) : "memory");
     };
-    float2 x[2][2];
-    float log_keep;
+    float2 x[2];
+    double log_keep;
     auto fetch_x = [&](int chunk) {
-        const float* from = args.u + item(chunk) * kChunk * V + column0 + pair;
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            x[n][0] = load_pair(from + (size_t)row * V + 8 * n);
-            x[n][1] = load_pair(from + (size_t)(row + 8) * V + 8 * n);
-        }
-        log_keep = (float)args.logs[item(chunk) * kChunk + kChunk - 1];
+        const float* from = args.u + item(chunk) * kChunk * V + column;
+        x[0] = load_pair(from + (size_t)row * V);
+        x[1] = load_pair(from + (size_t)(row + 8) * V);
+        log_keep = args.logs[item(chunk) * kChunk + kChunk - 1];  // (made a float where it is used: that waits for it)
     };
     fetch(0);
+    fetch(1);
     fetch_x(0);
-    float* stored = args.state + (size_t)args.slots[seq] * args.state_stride + (size_t)head * kDim * V + column0 + pair;
-    float s[2][4];
+    float* stored = args.state + (size_t)args.slots[seq] * args.state_stride + (size_t)head * kDim * V + column;
+    float s[4];
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
+    for (int i = 0; i < 4; ++i) s[i] = stored[(size_t)(row + 8 * (i / 2)) * V + i % 2];
+    // right operands: 32 rows at once, for two steps of 16
+    const int lane = tid & 31, turn = lane & 7;
+    const uint32_t right_lanes = (lane * kNarrowRow + tile0) * 2, s_at = smem_u32(s_planes) + right_lanes, u_at = smem_u32(u_planes) + right_lanes;
+    // y [16 rows of the warp][k] by rows, keys [k][16 columns of the warp] by columns; units turned by the row, whose low bits are the lane's
+    const uint32_t y_at = smem_u32(stages) + (16 * warp + (lane & 15)) * kDim * 2;
+    const uint32_t key_at = smem_u32(stages) + kParts * kCarryPlane * 2 + ((lane >> 4) * 8 + turn) * kDim * 2 + ((2 * warp + (lane >> 3 & 1)) ^ turn) * 16;
+    auto steps = [&](float (&d)[4], float scale, uint32_t left, bool keys, uint32_t right) {  // d = scale * d + left (16 x 64) . right (64 x 8)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) s[n][i] = stored[(size_t)(row + 8 * (i / 2)) * V + 8 * n + i % 2];
-    const uint32_t s_at = smem_u32(s_planes) + lanes_by_row(kNarrowRow), u_at = smem_u32(u_planes) + lanes_by_row(kNarrowRow);
-    const uint32_t y_at = smem_u32(stages) + 16 * warp * kRow * 2 + lanes_by_row(kRow);
-    const uint32_t key_at = smem_u32(stages) + (kParts * kPlane + 16 * warp) * 2 + lanes_by_column(kRow);
-    for (int chunk = 0; chunk < chunks; ++chunk) {
-        float* start = args.starts + item(chunk) * kDim * V + column0 + pair;
+        for (int k = 0; k < 64; k += 32) {
+            uint32_t both[kParts][4];
+            Parts a[2];
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+            for (int p = 0; p < kParts; ++p) {
+                ldmatrix4_turned(both[p], right + (k * kNarrowRow + p * kNarrowPlane) * 2);
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                split_two(s[n][2 * half], s[n][2 * half + 1], s_planes + (row + 8 * half) * kNarrowRow + 8 * n + pair, kNarrowPlane);
-                store_pair(start + (size_t)(row + 8 * half) * V + 8 * n, s[n][2 * half], s[n][2 * half + 1]);
+                for (int half = 0; half < 2; ++half) {
+                    if (keys) ldmatrix4_turned(a[half][p], left + (p * kCarryPlane + (k + 16 * half) * kDim) * 2);
+                    else ldmatrix4(a[half][p], left + p * kCarryPlane * 2 + (((k + 16 * half) / 8 + (lane >> 4)) ^ turn) * 16);
+                }
             }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();  // S, y and the keys are there; nobody reads the other stage any more
-        if (chunk + 1 < chunks) fetch(chunk + 1);
-        const uint32_t stage = (chunk & 1) * kCarryStage * 2;
-        const float keep = expf(log_keep);
-        float product[2][4] = {};
-#pragma unroll
-        for (int d = 0; d < kDim; d += 16) {
-            Parts a, b;
-            load_parts(a, y_at + stage + d * 2, kPlane);
-            load_parts_turned(b, s_at + d * kNarrowRow * 2, kNarrowPlane);
-            split_products(product[0], product[1], a, b);
+            const HalfParts first_half = {{both[0][0], both[0][1]}, {both[1][0], both[1][1]}, {both[2][0], both[2][1]}};
+            const HalfParts second_half = {{both[0][2], both[0][3]}, {both[1][2], both[1][3]}, {both[2][2], both[2][3]}};
+            split_product_twice(d, k == 0 ? scale : 1.0f, a[0], first_half, a[1], second_half);
         }
-        float* to = args.u + item(chunk) * kChunk * V + column0 + pair;
+    };
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+        float* start = args.starts + item(chunk) * kDim * V + column;
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int half = 0; half < 2; ++half) {
+            split_two(s[2 * half], s[2 * half + 1], s_planes + (row + 8 * half) * kNarrowRow + tile0 + pair, kNarrowPlane);
+            store_pair(start + (size_t)(row + 8 * half) * V, s[2 * half], s[2 * half + 1]);
+        }
+        const bool here = carry_wait(smem_u32(&arrived[chunk % kCarryStages]), chunk / kCarryStages & 1);
+        if (!__syncthreads_and(here)) {  // (nobody leaves while copies may still arrive)
+            for (int later = chunk + 1; later < min(chunks, chunk + kCarryStages - 1); ++later) carry_wait(smem_u32(&arrived[later % kCarryStages]), later / kCarryStages & 1);
+            return;
+        }
+        // S, y and the keys are there; nobody reads the stage before any more
+        fetch(chunk + kCarryStages - 1);
+        const uint32_t stage = chunk % kCarryStages * kCarryStage * 2;
+        const float keep = expf((float)log_keep);
+        float product[4] = {};
+        steps(product, 1.0f, y_at + stage, false, s_at);
+        float* to = args.u + item(chunk) * kChunk * V + column;
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const float lo = x[n][half].x - product[n][2 * half], hi = x[n][half].y - product[n][2 * half + 1];
-                split_two(lo, hi, u_planes + (row + 8 * half) * kNarrowRow + 8 * n + pair, kNarrowPlane);
-                store_pair(to + (size_t)(row + 8 * half) * V + 8 * n, lo, hi);
-            }
+        for (int half = 0; half < 2; ++half) {
+            const float lo = x[half].x - product[2 * half], hi = x[half].y - product[2 * half + 1];
+            split_two(lo, hi, u_planes + (row + 8 * half) * kNarrowRow + tile0 + pair, kNarrowPlane);
+            store_pair(to + (size_t)(row + 8 * half) * V, lo, hi);
+        }
         if (chunk + 1 < chunks) fetch_x(chunk + 1);
         __syncthreads();
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) s[n][i] *= keep;
-#pragma unroll
-        for (int i = 0; i < kChunk; i += 16) {
-            Parts a, b;
-            load_parts_turned(a, key_at + stage + i * kRow * 2, kPlane);
-            load_parts_turned(b, u_at + i * kNarrowRow * 2, kNarrowPlane);
-            split_products(s[0], s[1], a, b);
-        }
+        steps(s, keep, key_at + stage, true, u_at);
     }
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) stored[(size_t)(row + 8 * (i / 2)) * V + 8 * n + i % 2] = s[n][i];
+    for (int i = 0; i < 4; ++i) stored[(size_t)(row + 8 * (i / 2)) * V + i % 2] = s[i];
 }
 
 // grid (heads, most chunks of a sequence, sequences); block kResultThreads: a warp has 16 tokens and half of the V columns of their
@@ -623,4 +656,11 @@ MB_EXPORT int mb_gated_delta_chunks(const float* conv, int conv_stride, const vo
     if (dtype == MB_BF16)
         return vdim == 64 ? launch_chunks<__nv_bfloat16, 64>(args, sequences, chunks, stream) : launch_chunks<__nv_bfloat16, 128>(args, sequences, chunks, stream);
     return fail("gated_delta_chunks: unknown dtype code %d", dtype);
+}
+
+// 0 while no wait for a copy ever gave up.
+MB_EXPORT int mb_gated_delta_chunks_status() {
+    int status = 0;
+    if (cudaMemcpyFromSymbol(&status, g_carry_status, sizeof(int)) != cudaSuccess) return -1;
+    return status;
 }

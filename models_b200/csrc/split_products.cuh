@@ -65,7 +65,31 @@ __device__ __forceinline__ void split_products(float (&d0)[4], float (&d1)[4], c
     mma_bf16(p0, a[0], b[0][0], b[0][1]);
     mma_bf16(p1, a[0], b[0][2], b[0][3]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) d0[i] += p0[i] + r0[i], d1[i] += p1[i] + r1[i];
+    for (int i = 0; i < 4; i += 2) {  // (two additions an instruction, each rounded as one by itself)
+        const uint64_t s0 = pair_add(pair_of(d0[i], d0[i + 1]), pair_add(pair_of(p0[i], p0[i + 1]), pair_of(r0[i], r0[i + 1])));
+        const uint64_t s1 = pair_add(pair_of(d1[i], d1[i + 1]), pair_add(pair_of(p1[i], p1[i + 1]), pair_of(r1[i], r1[i + 1])));
+        d0[i] = low_of(s0), d0[i + 1] = high_of(s0), d1[i] = low_of(s1), d1[i + 1] = high_of(s1);
+    }
+}
+// d = scale * d + a0 . b0 + a1 . b1 in the same way for one tile of eight columns and two steps of K; b: each part's two registers.
+using HalfParts = uint32_t[kParts][2];
+__device__ __forceinline__ void split_product_twice(float (&d)[4], float scale, const Parts& a0, const HalfParts& b0, const Parts& a1, const HalfParts& b1) {
+    float p0[4] = {}, p1[4] = {}, r0[4] = {}, r1[4] = {};
+#pragma unroll
+    for (int order = kParts - 1; order > 0; --order)
+#pragma unroll
+        for (int i = 0; i <= order; ++i) {
+            mma_bf16(r0, a0[i], b0[order - i][0], b0[order - i][1]);
+            mma_bf16(r1, a1[i], b1[order - i][0], b1[order - i][1]);
+        }
+    mma_bf16(p0, a0[0], b0[0][0], b0[0][1]);
+    mma_bf16(p1, a1[0], b1[0][0], b1[0][1]);
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+        uint64_t sum = pair_fma(pair_of(d[i], d[i + 1]), pair_of(scale, scale), pair_add(pair_of(p0[i], p0[i + 1]), pair_of(r0[i], r0[i + 1])));
+        sum = pair_add(sum, pair_add(pair_of(p1[i], p1[i + 1]), pair_of(r1[i], r1[i + 1])));
+        d[i] = low_of(sum), d[i + 1] = high_of(sum);
+    }
 }
 
 // A float from its parts, and the float dot product of two rows of parts.

@@ -1080,6 +1080,22 @@ def _delta_call(lengths, heads, kv_heads, vdim, dtype, seed, unit_eps=1e-6, spoi
     return call
 
 
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("lengths", [[128], [192, 129], [449, 640]])
+def test_gated_delta_chunks_carry_through_their_ring(cuda_device, vdim, lengths):
+    """Two to ten chunks of a sequence through three places in shared memory, the last ones not full."""
+    from models_b200.kernels import ops
+
+    call = _delta_call(lengths, 4, 2, vdim, torch.float32, 11)
+    (out, state), (chunk_out, chunk_state) = call(0), call(max(lengths))
+    # the bounds of test_gated_delta_chunks, and the same bits once more
+    assert torch.allclose(chunk_state, state, rtol=1e-4, atol=1e-4)
+    close(chunk_out, out, torch.float32, scale=4.0)
+    again = call(max(lengths))
+    assert torch.equal(again[0], chunk_out) and torch.equal(again[1], chunk_state)
+    assert ops.gated_delta_chunks_library().mb_gated_delta_chunks_status() == 0
+
+
 @pytest.mark.parametrize("lengths", [[65], [100, 64, 3]])
 def test_gated_delta_chunks_without_an_epsilon(cuda_device, monkeypatch, lengths):
     """Keys that are divided by their own length alone: the empty rows of a chunk that is not full have none."""
