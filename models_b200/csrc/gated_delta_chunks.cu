@@ -21,7 +21,7 @@
 // results by 1.4e-7 (2e-7).
 // One sequence of 2,048 tokens, 16 heads of 64 x 128: the walk's chain of 2,048 tokens is bound by its latency (618 us, and 30 for
 // the kernels around it); the three kernels took 58, 105 and 71 us as float multiply-adds, bound by what the operands take from
-// shared memory and by the latency of few warps; 47, 45 and 58 here (a layer: 310 us, and 220), where the carrying kernel is bound by
+// shared memory and by the latency of few warps; 47, 46 and 58 here (a layer: 310 us, and 220), where the carrying kernel is bound by
 // its chunk's two products one after the other, the others by six products for one and the splitting of what they read.
 #include "common.cuh"
 #include "split_products.cuh"

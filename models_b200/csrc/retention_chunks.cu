@@ -10,7 +10,7 @@
 // Against 64 bits, over steps of 64 to 2,048 tokens: the state is off by 6e-8 to 9e-8 of itself (the walk in runs: 0.9e-7 to 1.4e-7), the
 // raw results by 0.7e-7 to 1.1e-7 (0.8e-7 to 1.8e-7); with two parts the operands would be cut to 16 bits.
 // Three sequences of 2,048 tokens in all, 16 heads of 64 x 128 with activated projections: 208 us as the walk in runs (98, 70 and 40),
-// which float multiply-adds from shared memory bound; here 32, 14 and 58 us, bound by the six products for one and by the
+// which float multiply-adds from shared memory bound; here 29, 14 and 54 us (sums of products added one by one: 32, 14 and 58), bound by the six products for one and by the
 // instructions that activate and split what every chunk reads.
 #include "common.cuh"
 #include "split_products.cuh"
