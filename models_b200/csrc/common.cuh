@@ -54,31 +54,6 @@ __device__ __forceinline__ float gated_pair(int activation, float gate, float up
     return gate_activation(activation, gate) * up;
 }
 
-// The same for a pair whose result is rounded to bfloat16, many to a thread: the quotient is a product with the approximate reciprocal
-// (within one unit of a float's last place; 0 for a denominator of infinity, as the quotient is).  A division has a long way for
-// unusual operands, and a branch to it after every pair keeps pairs from being worked on side by side: see gemm_tcgen05.cu.
-__device__ __forceinline__ float quick_reciprocal(float x) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-template <int kCount>
-__device__ __forceinline__ void gate_pairs(int activation, float (&gate)[kCount], const float (&up)[kCount], const ClampedPair& clamp) {
-    if (activation == MB_ACT_SILU) {
-#pragma unroll
-        for (int i = 0; i < kCount; ++i) gate[i] = gate[i] * quick_reciprocal(1.0f + expf(-gate[i])) * up[i];
-    } else if (activation == MB_ACT_CLAMPED_SWISH) {
-#pragma unroll
-        for (int i = 0; i < kCount; ++i) {
-            const float g = fminf(gate[i], clamp.limit), u = fminf(fmaxf(up[i], -clamp.limit), clamp.limit);
-            gate[i] = g * quick_reciprocal(1.0f + expf(-clamp.slope * g)) * (u + clamp.up_offset);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < kCount; ++i) gate[i] = gate_activation(activation, gate[i]) * up[i];
-    }
-}
-
 // Whether a launcher knows the code; `clamp` (three floats on the host, or null) is copied out for the clamped form.
 inline bool gate_known(int activation, const float* clamp, ClampedPair* out) {
     if (clamp != nullptr) *out = ClampedPair{clamp[0], clamp[1], clamp[2]};

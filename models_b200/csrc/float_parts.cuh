@@ -1,29 +1,11 @@
 // A float as three bfloat16 numbers that hold its 24 bits: its rounding, the rounding of what that left and of what this left.
 #pragma once
 
+#include "float_pairs.cuh"
+
 #include <cuda_bf16.h>
-#include <stdint.h>
 
 namespace mb {
-
-// Two floats side by side in a 64-bit register, as the paired float instructions take them.
-__device__ __forceinline__ uint64_t pair_of(float low, float high) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(low), "f"(high));
-    return v;
-}
-__device__ __forceinline__ uint64_t pair_fma(uint64_t a, uint64_t b, uint64_t c) {  // each rounded as fmaf rounds
-    uint64_t v;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
-    return v;
-}
-__device__ __forceinline__ uint64_t pair_add(uint64_t a, uint64_t b) {
-    uint64_t v;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-    return v;
-}
-__device__ __forceinline__ float low_of(uint64_t v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float high_of(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
 __device__ __forceinline__ uint32_t round_pair(uint64_t v) {
     const __nv_bfloat162 r = __floats2bfloat162_rn(low_of(v), high_of(v));

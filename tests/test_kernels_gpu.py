@@ -1346,6 +1346,32 @@ def test_gated_prompt_product_of_unusual_gates(cuda_device, clamp):
     assert bool((error <= want.abs() * (2.0 ** -8 + 2.0 ** -18) + 90.0 * 2.0 ** -126).all())
 
 
+@pytest.mark.parametrize("clamp", [None, (7.0, 1.702, 1.0), (7.0, -0.5, 1.0), (1e30, 2.0 ** -31, 0.0)])
+def test_prompts_gate_with_the_bits_of_decode(cuda_device, clamp):
+    """Gates of 24 bits beside a million ups: the quotients of prompts, which are made without a division, are those of decode's division.
+    (Sums of three parts and a zero are exact in either product.)"""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(31)
+    n, rows = 4096, 256
+    gates = torch.randn(n, generator=g) * torch.exp(torch.rand(n, generator=g) * 8 - 5)
+    gates[:64] = torch.tensor([0.0, -0.0, 1e-30, -1e-38, 39.9, -39.9, -40.1, -87.5, -89.0, -104.0, 104.0, 1e17, 2e18, -2e18, 3e38, -3e38]).repeat(4)
+    w = torch.zeros(2 * n, 64, dtype=torch.bfloat16)
+    left = gates.clone()
+    for part in range(3):
+        w[:n, part] = left.bfloat16()
+        left = left - w[:n, part].float()
+    w[n:, 3] = torch.randn(n, generator=g).bfloat16()
+    a = torch.zeros(rows, 64, dtype=torch.bfloat16)
+    a[:, :3] = 1.0
+    a[:, 3] = torch.randn(rows, generator=g).bfloat16()
+    epilogue = ops.EPI_SWIGLU if clamp is None else ops.EPI_CLAMPED
+    a, w = a.cuda(), w.cuda()
+    got = ops.gemm_tcgen05(a, w, epilogue, clamp=clamp)
+    decoded = torch.cat([ops.skinny_gemm(w, epilogue, x=a[i:i + 8].contiguous(), clamp=clamp) for i in range(0, rows, 8)])
+    assert torch.equal(got.view(torch.int16), decoded.view(torch.int16))
+
+
 @pytest.mark.parametrize("batch", [1, 3, 8])
 @pytest.mark.parametrize("n,k", [(2048, 4104), (37, 5000), (16, 8192), (2360, 8192)])
 def test_skinny_gemm_streams_activations(cuda_device, batch, n, k):
