@@ -154,6 +154,7 @@ struct FloatArgs {
     int lda, ldw, ldc, m, n, k;
     int parts, part_length;       // blocks of a cluster that share K; columns of each, a multiple of kChunk
     const unsigned char* unfit;   // of A's rows when they have been split: [m][chunks of K], whether a float there has no finite parts
+    int weights_ready;            // W depends on no kernel that may still be running: it is asked for before the wait for the one before
 };
 
 // A, split: planes [3][m][chunks * 64], a chunk's columns in the order of load_eight, zeros behind the last.  32 chunks of rows a block.
@@ -303,8 +304,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
             const int at = wanted * kChunk;
             load_eight<kEven>(a_next[p], a_from + (at + (long long)min(16 * p + my_row, a_last) * args.lda), k_end - k_begin - at - 4 * unit, wanted < chunks);
         };
+        if (!args.weights_ready) grid_dependency_wait();
 #pragma unroll
-        for (int p = 0; p < kPassesW; ++p) fetch_w(group, p);  // weights depend on nothing
+        for (int p = 0; p < kPassesW; ++p) fetch_w(group, p);
         grid_dependency_wait();
 #pragma unroll
         for (int p = 0; p < kPassesA; ++p) fetch_a(group, p);
@@ -485,8 +487,9 @@ gemm_f32_few_kernel(const FloatArgs args) {
             for (int step = 0; step < 4; ++step)
                 load_four<kEven>(v[h][step], w_from[h] + wanted * kChunk + 8 * step, k_end - k_begin - my_col - wanted * kChunk - 8 * step, wanted < chunks);
     };
+    if (!args.weights_ready) grid_dependency_wait();
 #pragma unroll
-    for (int i = 0; i < kFewAhead; ++i) fetch(i, next[i]);  // weights depend on nothing
+    for (int i = 0; i < kFewAhead; ++i) fetch(i, next[i]);
     __syncthreads();
     grid_dependency_wait();
     // A's parts: a thread takes the four columns of one lane of a step
@@ -660,14 +663,15 @@ MB_EXPORT size_t mb_gemm_f32_scratch(int m, int k) {
     return m <= kInlineRows ? 0 : 3 * plane_bytes(rows, k) + (size_t)rows * ((k + kChunk - 1) / kChunk);
 }
 
-// A: [m, k] with row stride lda; W: [n, k] with row stride ldw; C: [m, n] with row stride ldc.
+// A: [m, k] with row stride lda; W: [n, k] with row stride ldw; C: [m, n] with row stride ldc.  `weights_ready` != 0 only for a W that no
+// kernel still queued writes (a loaded weight): the kernels before start their followers early, and W is then read while they run.
 MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, float* c, int ldc, int m, int n, int k, void* scratch,
-                          cudaStream_t stream) {
+                          int weights_ready, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return fail("gemm_f32: k %d must be positive", k);
     if (lda < k || ldw < k || ldc < n) return fail("gemm_f32: row strides (%d, %d, %d) are shorter than the rows (%d, %d, %d)", lda, ldw, ldc, k, k, n);
     if (m > kInlineRows && (scratch == nullptr || ((uintptr_t)scratch & 15))) return fail("gemm_f32: scratch for the split rows is missing or not on a 16-byte boundary");
-    FloatArgs args{a, w, c, lda, ldw, ldc, m, n, k, 1, 0, nullptr};
+    FloatArgs args{a, w, c, lda, ldw, ldc, m, n, k, 1, 0, nullptr, weights_ready};
     // Parts of K, by n and k alone, so that every m gives a row the same bits: matrices of few tiles put more multiprocessors to work.
     const int tiles = (n + kTileN - 1) / kTileN;
     auto length = [&](int parts) { return ((k + parts - 1) / parts + kChunk - 1) / kChunk * kChunk; };

@@ -1746,9 +1746,10 @@ def prefill_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, 
 
 # ------------------------------------------------------------------------------------ matrix products
 
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, row_invariant: bool = True) -> torch.Tensor:
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, row_invariant: bool = True, weights_ready: bool = False) -> torch.Tensor:
     """a [m, k] . w[n, k]^T in 32 bits: every bit of the floats is multiplied, and a row's result depends on
-    nothing but that row (`row_invariant` or not)."""
+    nothing but that row (`row_invariant` or not).  `weights_ready`: no kernel still queued writes `w` (a loaded
+    weight), so that it may be read while the kernels before this product still run."""
     _cuda(a, w)
     if a.dtype != torch.float32 or w.dtype != torch.float32:
         raise KernelError(f"gemm_f32 takes float32 operands, got {a.dtype} and {w.dtype}")
@@ -1761,7 +1762,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, row_invariant: bool = True) -> to
     lib.mb_gemm_f32_scratch.restype = ctypes.c_size_t
     need = lib.mb_gemm_f32_scratch(m, k)
     scratch = torch.empty((need,), dtype=torch.uint8, device=a.device) if need else None
-    _run(lib, lib.mb_gemm_f32(_p(a), a.stride(0), _p(w), w.stride(0), _p(c), n, m, n, k, _p(scratch), _stream()))
+    _run(lib, lib.mb_gemm_f32(_p(a), a.stride(0), _p(w), w.stride(0), _p(c), n, m, n, k, _p(scratch), 1 if weights_ready else 0, _stream()))
     return c
 
 

@@ -20,11 +20,12 @@ from ..kernels import ops
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
+    """x . weight^T; `weight` is a loaded weight, which the products read ahead of the kernels before them."""
     if not x.is_cuda:
         raise ops.KernelError("models_b200 runs on a CUDA device only; there is no CPU path")
     if weight.dtype == torch.float32:
         a = x if x.dtype == torch.float32 else x.float()
-        out = ops.gemm_f32(a, weight)
+        out = ops.gemm_f32(a, weight, weights_ready=True)
         return out if out_dtype == torch.float32 else out.to(out_dtype)
     if weight.dtype != torch.bfloat16:
         raise ops.KernelError(f"matrices are bfloat16 or float32, got {weight.dtype}")

@@ -166,6 +166,26 @@ def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
         assert torch.equal(ops.gemm_f32(*moved), aligned)
 
 
+@pytest.mark.parametrize("m,n,k", [(3, 2048, 2048), (20, 2048, 2048), (200, 512, 1088)])
+def test_gemm_f32_takes_the_result_of_the_product_before(cuda_device, m, n, k):
+    """Products queued one after another, captured, whose second operand is what the one before writes."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(m)
+    x, z = torch.randn(m, n, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    ys = [torch.randn(n, k, generator=g).cuda() for _ in range(3)]
+    want = [ops.gemm_f32(x, w) for w in [(torch.cuda.synchronize(), ops.gemm_f32(y, z), torch.cuda.synchronize())[1] for y in ys]]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = [ops.gemm_f32(x, ops.gemm_f32(y, z)) for y in ys]
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_swiglu_and_bias(cuda_device, dtype):
     from models_b200.kernels import ops
