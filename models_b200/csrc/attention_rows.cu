@@ -277,9 +277,8 @@ template <int HD>
 static int launch_row_tiles(const float* q, int q_row_stride, float* out, int out_row_stride, const float* k_pool, const float* v_pool,
                             const int* block_table, int max_blocks, const int* cu_q, const int* kv_lens, int sequences, long long rows,
                             int heads, int kv_heads, int page_size, int window, float scale, cudaStream_t stream) {
-    static const cudaError_t reserved =
-        cudaFuncSetAttribute(paged_attention_row_tiles_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, RowTiles<HD>::kBytes);
-    if (reserved != cudaSuccess) return fail("paged_attention_rows: cannot reserve %d bytes of shared memory: %s", RowTiles<HD>::kBytes, cudaGetErrorString(reserved));
+    static DeviceSet devices{0};
+    if (int status = reserve_shared("paged_attention_rows", paged_attention_row_tiles_kernel<HD>, RowTiles<HD>::kBytes, devices)) return status;
     const dim3 grid((unsigned)((rows + kTileRows - 1) / kTileRows), kv_heads, sequences);
     paged_attention_row_tiles_kernel<HD><<<grid, kTileThreads, RowTiles<HD>::kBytes, stream>>>(
         q, q_row_stride, out, out_row_stride, k_pool, v_pool, block_table, max_blocks, cu_q, kv_lens, heads, kv_heads, page_size, window, scale);

@@ -9,6 +9,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include "reserve.h"
+
 #define MB_EXPORT extern "C" __attribute__((visibility("default")))
 
 // dtype codes that cross the C boundary
@@ -88,6 +90,15 @@ inline int check_launch(const char* what) {
         return fail("%s: %s", what, cudaGetErrorString(status));
     }
     return 0;
+}
+
+// Lets `kernel` ask for `bytes` of dynamic shared memory on the current device; `devices`: where it may already (a static of the launcher's).
+template <typename Kernel>
+inline int reserve_shared(const char* what, Kernel kernel, int bytes, DeviceSet& devices) {
+    const cudaError_t status = reserve_on_device((const void*)kernel, bytes, devices);
+    if (status == cudaSuccess) return 0;
+    cudaGetLastError();
+    return fail("%s: cannot reserve %d bytes of shared memory: %s", what, bytes, cudaGetErrorString(status));
 }
 
 template <typename T>

@@ -596,8 +596,8 @@ template <int NB, int kRowsW, bool kEven>
 static int launch(const CUtensorMap& map_a, const FloatArgs& args, cudaStream_t stream) {
     using P = Plan<NB, kRowsW>;
     auto kernel = gemm_f32_kernel<NB, kRowsW, kEven>;
-    static const cudaError_t reserved = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::kBytes);
-    if (reserved != cudaSuccess) return fail("gemm_f32: cannot reserve %d bytes of shared memory: %s", P::kBytes, cudaGetErrorString(reserved));
+    static DeviceSet devices{0};
+    if (int status = reserve_shared("gemm_f32", kernel, P::kBytes, devices)) return status;
     const long long blocks = (long long)((args.n + kRowsW - 1) / kRowsW) * ((args.m + P::kRows - 1) / P::kRows) * args.parts;
     if (blocks > 0x7fffffff) return fail("gemm_f32: %d x %d results exceed the grid limit", args.m, args.n);
     cudaLaunchConfig_t config = {};
@@ -622,8 +622,8 @@ static int launch(const CUtensorMap& map_a, const FloatArgs& args, cudaStream_t 
 template <bool kEven>
 static int launch_few(const FloatArgs& args, cudaStream_t stream) {
     int bytes = args.part_length * args.m * 6;
-    static const cudaError_t reserved = cudaFuncSetAttribute(gemm_f32_few_kernel<kEven>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewBytes);
-    if (reserved != cudaSuccess) return fail("gemm_f32: cannot reserve %d bytes of shared memory: %s", kFewBytes, cudaGetErrorString(reserved));
+    static DeviceSet devices{0};
+    if (int status = reserve_shared("gemm_f32", gemm_f32_few_kernel<kEven>, kFewBytes, devices)) return status;
     const long long blocks = (long long)((args.n + kFewRowsW - 1) / kFewRowsW) * args.parts;
     if (blocks > 0x7fffffff) return fail("gemm_f32: %d x %d results exceed the grid limit", args.m, args.n);
     cudaLaunchConfig_t config = {};
