@@ -24,7 +24,8 @@
 // and four hold the sums, a row of W per thread.  Weights that are bfloat16 numbers -- most models' are, in the 32-bit mode too -- have
 // two parts of zeros, whose products are left out: each stage of W says whether it is such.
 //
-// A float that is not finite, or has no finite rounding, spoils the sums of its own row of A or W alone; these results are
+// A float that is not finite, or has no finite rounding, spoils the sums of its own row of A or W alone; these results, and those whose
+// sums are not finite (the roundings' product may pass the largest float on one side and a smaller one on the other), are
 // computed anew from the floats, in the order of K.  Floats below 2^-109 keep fewer bits (off by 2^-134 at most).
 #include "tcgen05.cuh"
 #include "float_parts.cuh"
@@ -267,10 +268,13 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
         for (int j = 0; j < P::kRows; ++j)
             if (j < rows) to[j * step] = j % 2 ? high_of(sum[j / 2]) : low_of(sum[j / 2]);
         asm volatile("bar.sync 1, %0;" ::"n"(32 * (kAdders + kSplitters)) : "memory");  // the splitters have seen every float
-        if (*reinterpret_cast<volatile int*>(&spoilt) && (int)threadIdx.x < kRowsW && col < args.n) {
+        uint64_t finite = 0;  // 0, 0 or NaN
+#pragma unroll
+        for (int j = 0; j < P::kRows / 2; ++j) finite = pair_fma(sum[j], 0, finite);
+        if ((*reinterpret_cast<volatile int*>(&spoilt) || low_of(finite) + high_of(finite) != 0.0f) && (int)threadIdx.x < kRowsW && col < args.n) {
 #pragma unroll 1
             for (int j = 0; j < min(P::kRows, args.m - row0); ++j)
-                if (spoilt_w[threadIdx.x] || spoilt_a[j]) {
+                if (spoilt_w[threadIdx.x] || spoilt_a[j] || !isfinite(to[j * step])) {
                     const float *a = args.a + (size_t)(row0 + j) * args.lda, *w = args.w + (size_t)col * args.ldw;
                     float total = 0.0f;
 #pragma unroll 1
@@ -563,7 +567,7 @@ gemm_f32_few_kernel(const FloatArgs args) {
             const int r = 2 * quad + e, of_block = warp * 16 + group + 8 * h, col = col0 + of_block;
             if (r >= m) continue;
             float total = sum[2 * h + e] + small[2 * h + e];
-            if (bad || spoilt_a[r] != 0) {
+            if (bad || spoilt_a[r] != 0 || !isfinite(total)) {
                 const float *a = args.a + (size_t)r * args.lda, *w = args.w + (size_t)min(col, args.n - 1) * args.ldw;
                 total = 0.0f;
 #pragma unroll 1

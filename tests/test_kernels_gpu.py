@@ -151,6 +151,23 @@ def test_gemm_f32_keeps_rows_that_are_not_finite_apart(cuda_device, m, value):
             assert abs(x - y) <= 1e-5 * abs(y) + 1e-4
 
 
+@pytest.mark.parametrize("m", [3, 20, 70, 200])
+def test_gemm_f32_overflows_as_floats_do(cuda_device, m):
+    """Finite operands whose products pass the largest float by far: infinite where the float sum is, whatever signs the smaller parts have."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(m)
+    a, w = torch.randn(m, 1088, generator=g), torch.randn(200, 1088, generator=g)
+    a[2, 700], w[:, 700] = 2.5e30, 3.1e30 * (1 + torch.rand(200, generator=g))
+    w[100:, 700] *= -1
+    a[1, 30], w[150:, 30] = -2.2e25, 1.7e25  # (other results stay finite beside them)
+    got, want = ops.gemm_f32(a.cuda(), w.cuda()).cpu(), (a.double() @ w.double().t()).float()
+    assert torch.equal(got[2], want[2]) and bool(torch.isinf(want[2]).all())
+    assert torch.equal(torch.isinf(got), torch.isinf(want)) and torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+    assert bool(torch.isfinite(got[torch.isfinite(want)]).all())
+    assert bool(((got.double() - want.double()).abs() <= 1e-5 * (a.abs().double() @ w.abs().double().t()))[torch.isfinite(want)].all())
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 72, 2048), (5, 200, 260), (40, 130, 1028), (70, 8200, 516), (130, 64, 2048)])
 def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
     """Operands whose rows do not start on 16 bytes meet another kernel: the same chains over the same parts of K."""
