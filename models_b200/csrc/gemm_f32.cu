@@ -24,8 +24,8 @@
 // and four hold the sums, a row of W per thread.  Weights that are bfloat16 numbers -- most models' are, in the 32-bit mode too -- have
 // two parts of zeros, whose products are left out: each stage of W says whether it is such.
 //
-// A float that is not finite, or has no finite rounding, spoils the sums of its own row of A or W alone; these results, and those whose
-// sums are not finite (the roundings' product may pass the largest float on one side and a smaller one on the other), are
+// A float that is not finite, or whose rounding is not, leaves no finite sum in its own row of A or W, and no other row sees it; the
+// roundings' product may also pass the largest float on one side and a smaller one on the other.  Results that are not finite are
 // computed anew from the floats, in the order of K.  Floats below 2^-109 keep fewer bits (off by 2^-134 at most).
 #include "tcgen05.cuh"
 #include "float_parts.cuh"
@@ -108,15 +108,6 @@ __device__ __forceinline__ void load_four(uint64_t (&v)[2], const float* from, i
     }
 }
 
-// Whether one of them is not finite, or has a part that is not.  (The largest bfloat16 number is a little smaller than the largest
-// float: four times what lies between them is infinite.)
-__device__ __forceinline__ bool unfit_pairs(const uint64_t (&v)[4]) {
-    uint64_t sum = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) sum = pair_fma(v[j], 0x4080000040800000ull, sum);  // 4, 4
-    return !isfinite(low_of(sum) + high_of(sum));
-}
-
 // Their parts, 16 bytes to each of three planes; `smaller` gathers the bits of the two smaller ones.
 __device__ __forceinline__ void split_eight(const uint64_t (&v)[4], unsigned char* at, size_t plane_bytes, uint32_t& smaller) {
     uint4 hi, mid, lo;
@@ -154,26 +145,22 @@ struct FloatArgs {
     float* c;
     int lda, ldw, ldc, m, n, k;
     int parts, part_length;       // blocks of a cluster that share K; columns of each, a multiple of kChunk
-    const unsigned char* unfit;   // of A's rows when they have been split: [m][chunks of K], whether a float there has no finite parts
     int weights_ready;            // W depends on no kernel that may still be running: it is asked for before the wait for the one before
 };
 
 // A, split: planes [3][m][chunks * 64], a chunk's columns in the order of load_eight, zeros behind the last.  32 chunks of rows a block.
 template <bool kEven>
 __global__ void __launch_bounds__(256)
-split_rows_kernel(const float* __restrict__ a, int lda, int m, int k, int chunks, unsigned char* planes, unsigned char* unfit) {
+split_rows_kernel(const float* __restrict__ a, int lda, int m, int k, int chunks, unsigned char* planes) {
     grid_launch_dependents();
     grid_dependency_wait();
     const size_t item = (size_t)blockIdx.x * 32 + (threadIdx.x >> 3);
-    if (item >= (size_t)m * chunks) return;  // (eight threads at once)
+    if (item >= (size_t)m * chunks) return;
     const int row = (int)(item / chunks), chunk = (int)(item % chunks), unit = threadIdx.x & 7;
     uint64_t v[4] = {};
     load_eight<kEven>(v, a + (size_t)row * lda + chunk * kChunk + 4 * unit, k - chunk * kChunk - 4 * unit, true);
     uint32_t smaller = 0;
     split_eight(v, planes + item * 128 + unit * 16, (size_t)m * chunks * 128, smaller);
-    const uint32_t eight = 0xffu << (threadIdx.x & 24);
-    const bool bad = __any_sync(eight, unfit_pairs(v));
-    if (unit == 0) unfit[item] = bad;
 }
 
 // grid: parts of K fastest, then the tiles of A, then those of W (so that neighbours share a tile of W).
@@ -189,8 +176,6 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
     __shared__ __align__(8) uint64_t barriers[2 * kMaxStages + 5];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int whole[kMaxStages];  // one more than the last chunk whose floats of W, in this stage, have parts beyond the first
-    __shared__ unsigned char spoilt_w[kRowsW], spoilt_a[P::kRows];
-    __shared__ int spoilt;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full_bar = smem_u32(&barriers[0]), empty_bar = smem_u32(&barriers[kMaxStages]);
     const uint32_t sum_full_bar = smem_u32(&barriers[2 * kMaxStages]), sum_empty_bar = sum_full_bar + 16, done_bar = sum_full_bar + 32;
@@ -211,10 +196,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
             mbar_init(sum_empty_bar + 8 * b, kAdders);
         }
         mbar_init(done_bar, 1);
-        spoilt = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < kRowsW + P::kRows; i += kThreads) (i < kRowsW ? spoilt_w[i] : spoilt_a[i - kRowsW]) = 0;
     if (warp == kIssuer) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "n"(P::kColumns));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
@@ -267,14 +250,13 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
 #pragma unroll
         for (int j = 0; j < P::kRows; ++j)
             if (j < rows) to[j * step] = j % 2 ? high_of(sum[j / 2]) : low_of(sum[j / 2]);
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * (kAdders + kSplitters)) : "memory");  // the splitters have seen every float
         uint64_t finite = 0;  // 0, 0 or NaN
 #pragma unroll
         for (int j = 0; j < P::kRows / 2; ++j) finite = pair_fma(sum[j], 0, finite);
-        if ((*reinterpret_cast<volatile int*>(&spoilt) || low_of(finite) + high_of(finite) != 0.0f) && (int)threadIdx.x < kRowsW && col < args.n) {
+        if (low_of(finite) + high_of(finite) != 0.0f && (int)threadIdx.x < kRowsW && col < args.n) {
 #pragma unroll 1
             for (int j = 0; j < min(P::kRows, args.m - row0); ++j)
-                if (spoilt_w[threadIdx.x] || spoilt_a[j] || !isfinite(to[j * step])) {
+                if (!isfinite(to[j * step])) {
                     const float *a = args.a + (size_t)(row0 + j) * args.lda, *w = args.w + (size_t)col * args.ldw;
                     float total = 0.0f;
 #pragma unroll 1
@@ -320,39 +302,22 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
             ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * stage, (chunk / P::kStages & 1) ^ 1, 1));  // (a stage starts free)
             if (!ok) break;
             unsigned char* at = smem + stage * P::kStageBytes + my_row * 128 + ((unit ^ (my_row & 7)) << 4);  // the 128-byte swizzle
-            uint32_t smaller = 0, nothing = 0, unfit = 0;
+            uint32_t smaller = 0, nothing = 0;
 #pragma unroll
             for (int p = 0; p < kPassesW; ++p) {
                 split_eight(w_next[p], at + p * 2048, kPlaneW, smaller);
-                unfit |= (unfit_pairs(w_next[p]) ? 1u : 0u) << p;
                 fetch_w(chunk + 2, p);
             }
 #pragma unroll
             for (int p = 0; p < kPassesA; ++p) {
                 split_eight(a_next[p], at + 3 * kPlaneW + p * 2048, kPlane, nothing);
-                unfit |= (unfit_pairs(a_next[p]) ? 1u : 0u) << (kPassesW + p);
                 fetch_a(chunk + 2, p);
-            }
-            if (unfit != 0) {
-                spoilt = 1;
-#pragma unroll 1
-                for (int p = 0; p < kPassesW + kPassesA; ++p)
-                    if (unfit >> p & 1) (p < kPassesW ? spoilt_w[16 * p + my_row] : spoilt_a[16 * (p - kPassesW) + my_row]) = 1;
             }
             if ((smaller & 0x7fff7fffu) != 0) whole[stage] = chunk + 1;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(full_bar + 8 * stage);
         }
-        const int row = threadIdx.x - 32 * kAdders;
-        if (!P::kInline && row < P::kRows && row0 + row < args.m) {
-            const int all = (args.k + kChunk - 1) / kChunk;
-            const unsigned char* of_row = args.unfit + (size_t)(row0 + row) * all + k_begin / kChunk;
-            uint32_t bad = 0;
-            for (int i = 0; i < chunks; ++i) bad |= of_row[i];
-            if (bad != 0) spoilt_a[row] = 1, spoilt = 1;
-        }
-        asm volatile("bar.arrive 1, %0;" ::"n"(32 * (kAdders + kSplitters)) : "memory");
         __syncwarp();
         if (args.parts > 1) {  // the cluster's blocks share the rows and add the parts in their order
             cluster_sync_all();
@@ -470,13 +435,11 @@ __global__ void __launch_bounds__(kFewThreads)
 gemm_f32_few_kernel(const FloatArgs args) {
     extern __shared__ __align__(16) uint2 few_parts[];
     __shared__ float sums[kFewRows][kFewRowsW];
-    __shared__ int spoilt_a[kFewRows];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = lane >> 2, quad = lane & 3;
     const int part = blockIdx.x % args.parts, col0 = (blockIdx.x / args.parts) * kFewRowsW;
     const int k_begin = part * args.part_length, k_end = min(args.k, k_begin + args.part_length);
     const int chunks = (k_end - k_begin + kChunk - 1) / kChunk, m = args.m;
     grid_launch_dependents();
-    if (threadIdx.x < kFewRows) spoilt_a[threadIdx.x] = 0;
 
     // a lane's columns of the sixteen of a step: four from 8 * step + 4 * (quad & 1) + 32 * (quad >> 1)
     const int my_col = 4 * (quad & 1) + 32 * (quad >> 1);
@@ -494,7 +457,6 @@ gemm_f32_few_kernel(const FloatArgs args) {
     if (!args.weights_ready) grid_dependency_wait();
 #pragma unroll
     for (int i = 0; i < kFewAhead; ++i) fetch(i, next[i]);
-    __syncthreads();
     grid_dependency_wait();
     // A's parts: a thread takes the four columns of one lane of a step
     const int items = chunks * 16;
@@ -508,13 +470,10 @@ gemm_f32_few_kernel(const FloatArgs args) {
             split_pair(v[1], hi.y, mid.y, lo.y);
             uint2* to = few_parts + (r * chunks * 4 + (i >> 2)) * 12 + q;
             to[0] = hi, to[4] = mid, to[8] = lo;
-            const uint64_t fit = pair_fma(v[0], 0x4080000040800000ull, pair_fma(v[1], 0x4080000040800000ull, 0));
-            if (!isfinite(low_of(fit) + high_of(fit))) spoilt_a[r] = 1;
         }
     __syncthreads();
 
     float sum[4] = {}, small[4] = {};
-    uint64_t fit[2] = {0, 0};
     const bool live = group < m;
     const uint2* mine = few_parts + (live ? group : 0) * chunks * 48 + quad;
     for (int chunk0 = 0; chunk0 < chunks; chunk0 += kFewAhead) {
@@ -534,7 +493,6 @@ gemm_f32_few_kernel(const FloatArgs args) {
                         const uint64_t v = next[i][h][step][e];
                         split_pair(v, w[step][0][2 * e + h], w[step][1][2 * e + h], w[step][2][2 * e + h]);
                         smaller |= w[step][1][2 * e + h] | w[step][2][2 * e + h];
-                        fit[h] = pair_fma(v, 0x4080000040800000ull, fit[h]);
                     }
 #pragma unroll
                 for (int p = 0; p < 3; ++p) a[step][p] = live ? mine[(chunk * 4 + step) * 12 + p * 4] : make_uint2(0u, 0u);
@@ -561,13 +519,12 @@ gemm_f32_few_kernel(const FloatArgs args) {
     // a lane holds rows group and group + 8 of the warp's sixteen of W, rows 2 * quad and 2 * quad + 1 of A
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        const bool bad = (__ballot_sync(0xffffffffu, !isfinite(low_of(fit[h]) + high_of(fit[h]))) >> (lane & 28) & 15u) != 0;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int r = 2 * quad + e, of_block = warp * 16 + group + 8 * h, col = col0 + of_block;
             if (r >= m) continue;
             float total = sum[2 * h + e] + small[2 * h + e];
-            if (bad || spoilt_a[r] != 0 || !isfinite(total)) {
+            if (!isfinite(total)) {
                 const float *a = args.a + (size_t)r * args.lda, *w = args.w + (size_t)min(col, args.n - 1) * args.ldw;
                 total = 0.0f;
 #pragma unroll 1
@@ -664,7 +621,7 @@ using namespace mb;
 // Bytes of scratch that a product of m rows and k columns takes (0 for few rows); they start on a 16-byte boundary.
 MB_EXPORT size_t mb_gemm_f32_scratch(int m, int k) {
     const int rows = std::min(m, kSlabRows);
-    return m <= kInlineRows ? 0 : 3 * plane_bytes(rows, k) + (size_t)rows * ((k + kChunk - 1) / kChunk);
+    return m <= kInlineRows ? 0 : 3 * plane_bytes(rows, k);
 }
 
 // A: [m, k] with row stride lda; W: [n, k] with row stride ldw; C: [m, n] with row stride ldc.  `weights_ready` != 0 only for a W that no
@@ -675,7 +632,7 @@ MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, floa
     if (k <= 0) return fail("gemm_f32: k %d must be positive", k);
     if (lda < k || ldw < k || ldc < n) return fail("gemm_f32: row strides (%d, %d, %d) are shorter than the rows (%d, %d, %d)", lda, ldw, ldc, k, k, n);
     if (m > kInlineRows && (scratch == nullptr || ((uintptr_t)scratch & 15))) return fail("gemm_f32: scratch for the split rows is missing or not on a 16-byte boundary");
-    FloatArgs args{a, w, c, lda, ldw, ldc, m, n, k, 1, 0, nullptr, weights_ready};
+    FloatArgs args{a, w, c, lda, ldw, ldc, m, n, k, 1, 0, weights_ready};
     // Parts of K, by n and k alone, so that every m gives a row the same bits: matrices of few tiles put more multiprocessors to work.
     const int tiles = (n + kTileN - 1) / kTileN;
     auto length = [&](int parts) { return ((k + parts - 1) / parts + kChunk - 1) / kChunk * kChunk; };
@@ -696,11 +653,9 @@ MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, floa
         args.a = a + (size_t)first * lda;
         args.c = c + (size_t)first * ldc;
         unsigned char* planes = static_cast<unsigned char*>(scratch);
-        unsigned char* unfit = planes + 3 * plane_bytes(args.m, k);
-        args.unfit = unfit;
         const unsigned blocks = (unsigned)(((size_t)args.m * chunks + 31) / 32);
-        int status = even_a ? launch_dependent("gemm_f32", split_rows_kernel<true>, dim3(blocks), dim3(256), 0, stream, true, args.a, lda, args.m, k, chunks, planes, unfit)
-                            : launch_dependent("gemm_f32", split_rows_kernel<false>, dim3(blocks), dim3(256), 0, stream, true, args.a, lda, args.m, k, chunks, planes, unfit);
+        int status = even_a ? launch_dependent("gemm_f32", split_rows_kernel<true>, dim3(blocks), dim3(256), 0, stream, true, args.a, lda, args.m, k, chunks, planes)
+                            : launch_dependent("gemm_f32", split_rows_kernel<false>, dim3(blocks), dim3(256), 0, stream, true, args.a, lda, args.m, k, chunks, planes);
         if (status) return status;
         // As few tiles of A as there must be, and these as low as that allows.
         const int a_tiles = (args.m + 159) / 160, rows = (args.m + a_tiles - 1) / a_tiles, nb = std::max(2, (rows + 31) / 32);

@@ -168,6 +168,25 @@ def test_gemm_f32_overflows_as_floats_do(cuda_device, m):
     assert bool(((got.double() - want.double()).abs() <= 1e-5 * (a.abs().double() @ w.abs().double().t()))[torch.isfinite(want)].all())
 
 
+@pytest.mark.parametrize("value", [1e36, 1.5e37, 5e37])
+@pytest.mark.parametrize("side", ["a", "w"])
+def test_gemm_f32_gives_rows_of_large_floats_the_same_bits(cuda_device, side, value):
+    """Whether results are computed anew from the floats is decided by the results, which are the same in every kernel."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(17)
+    a, w = torch.randn(161, 1088, generator=g).cuda(), torch.randn(200, 1088, generator=g).cuda()
+    large, small = (a, w) if side == "a" else (w, a)
+    large[0] = value
+    large[3] = value * torch.rand(1088, generator=g).cuda()
+    large[:, 8:16] = value  # eight neighbours of every row
+    small *= 1e-4
+    out = ops.gemm_f32(a, w)
+    assert bool(torch.isfinite(out).all())
+    for rows in (1, 4, 5, 8, 32, 33, 64, 160):
+        assert torch.equal(ops.gemm_f32(a[:rows], w), out[:rows])
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 72, 2048), (5, 200, 260), (40, 130, 1028), (70, 8200, 516), (130, 64, 2048)])
 def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
     """Operands whose rows do not start on 16 bytes meet another kernel: the same chains over the same parts of K."""
