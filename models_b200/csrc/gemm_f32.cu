@@ -24,9 +24,10 @@
 // and four hold the sums, a row of W per thread.  Weights that are bfloat16 numbers -- most models' are, in the 32-bit mode too -- have
 // two parts of zeros, whose products are left out: each stage of W says whether it is such.
 //
-// A float that is not finite, or whose rounding is not, leaves no finite sum in its own row of A or W, and no other row sees it; the
-// roundings' product may also pass the largest float on one side and a smaller one on the other.  Results that are not finite are
-// computed anew from the floats, in the order of K.  Floats below 2^-109 keep fewer bits (off by 2^-134 at most).
+// Both operands are split times 2^24, and the sums divided by 2^48: the parts of every float are whole then, also where it is so small that
+// bfloat16 would have no bits left for its third.  Sums that are not finite -- a float was not, or was above 2^103, or the result is above
+// 2^79 -- are computed anew from the floats, in the order of K: no other row of A or W sees such a float.  (That results are judged, and not
+// operands, gives every kernel below the same judgement.)
 #include "tcgen05.cuh"
 #include "float_parts.cuh"
 
@@ -51,6 +52,7 @@ constexpr int kPlaneA = 32 * 128;     // times NB
 constexpr int kMaxStages = 3;
 constexpr int kInlineRows = 32;       // most rows of A that are split where they are multiplied
 constexpr int kSlabRows = 2048;       // rows of A that are split at a time
+constexpr uint64_t kUp = 0x4b8000004b800000ull, kDown = 0x2780000027800000ull;  // pairs of 2^24, times which both operands are split, and of 2^-48
 
 // NB: 32 rows of A each.  kRowsW: rows of W per block (64 leave half of the products' first operand to chance, unread).
 template <int NB, int kRowsW>
@@ -111,10 +113,10 @@ __device__ __forceinline__ void load_four(uint64_t (&v)[2], const float* from, i
 // Their parts, 16 bytes to each of three planes; `smaller` gathers the bits of the two smaller ones.
 __device__ __forceinline__ void split_eight(const uint64_t (&v)[4], unsigned char* at, size_t plane_bytes, uint32_t& smaller) {
     uint4 hi, mid, lo;
-    split_pair(v[0], hi.x, mid.x, lo.x);
-    split_pair(v[1], hi.y, mid.y, lo.y);
-    split_pair(v[2], hi.z, mid.z, lo.z);
-    split_pair(v[3], hi.w, mid.w, lo.w);
+    split_pair(pair_mul(v[0], kUp), hi.x, mid.x, lo.x);
+    split_pair(pair_mul(v[1], kUp), hi.y, mid.y, lo.y);
+    split_pair(pair_mul(v[2], kUp), hi.z, mid.z, lo.z);
+    split_pair(pair_mul(v[3], kUp), hi.w, mid.w, lo.w);
     *reinterpret_cast<uint4*>(at) = hi;
     *reinterpret_cast<uint4*>(at + plane_bytes) = mid;
     *reinterpret_cast<uint4*>(at + 2 * plane_bytes) = lo;
@@ -242,6 +244,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
         tcgen05_fence_after();
         if (ok) add(tmem_small);
         tcgen05_fence_before();
+#pragma unroll
+        for (int j = 0; j < P::kRows / 2; ++j) sum[j] = pair_mul(sum[j], kDown);
         // To the result, or, as one of several parts, to shared memory (every product has read the stages): [rows of A][kRowsW].
         const int col = col0 + (int)threadIdx.x;
         const int rows = (int)threadIdx.x >= kRowsW ? 0 : args.parts > 1 ? P::kRows : col < args.n ? min(P::kRows, args.m - row0) : 0;
@@ -466,8 +470,8 @@ gemm_f32_few_kernel(const FloatArgs args) {
             uint64_t v[2] = {};
             load_four<kEven>(v, args.a + (size_t)r * args.lda + k_begin + at, k_end - k_begin - at, true);
             uint2 hi, mid, lo;
-            split_pair(v[0], hi.x, mid.x, lo.x);
-            split_pair(v[1], hi.y, mid.y, lo.y);
+            split_pair(pair_mul(v[0], kUp), hi.x, mid.x, lo.x);
+            split_pair(pair_mul(v[1], kUp), hi.y, mid.y, lo.y);
             uint2* to = few_parts + (r * chunks * 4 + (i >> 2)) * 12 + q;
             to[0] = hi, to[4] = mid, to[8] = lo;
         }
@@ -490,7 +494,7 @@ gemm_f32_few_kernel(const FloatArgs args) {
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const uint64_t v = next[i][h][step][e];
+                        const uint64_t v = pair_mul(next[i][h][step][e], kUp);
                         split_pair(v, w[step][0][2 * e + h], w[step][1][2 * e + h], w[step][2][2 * e + h]);
                         smaller |= w[step][1][2 * e + h] | w[step][2][2 * e + h];
                     }
@@ -523,7 +527,7 @@ gemm_f32_few_kernel(const FloatArgs args) {
         for (int e = 0; e < 2; ++e) {
             const int r = 2 * quad + e, of_block = warp * 16 + group + 8 * h, col = col0 + of_block;
             if (r >= m) continue;
-            float total = sum[2 * h + e] + small[2 * h + e];
+            float total = (sum[2 * h + e] + small[2 * h + e]) * low_of(kDown);
             if (!isfinite(total)) {
                 const float *a = args.a + (size_t)r * args.lda, *w = args.w + (size_t)min(col, args.n - 1) * args.ldw;
                 total = 0.0f;

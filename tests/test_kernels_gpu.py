@@ -187,6 +187,22 @@ def test_gemm_f32_gives_rows_of_large_floats_the_same_bits(cuda_device, side, va
         assert torch.equal(ops.gemm_f32(a[:rows], w), out[:rows])
 
 
+@pytest.mark.parametrize("size", [1e-33, 1e-36, 1e-37, 1e-41])
+@pytest.mark.parametrize("m", [3, 20, 70])
+def test_gemm_f32_multiplies_every_bit_of_small_floats(cuda_device, m, size):
+    """Operands down to those below the normal floats beside large ones: the bound of test_gemm_f32_gives_a_row_the_same_bits_in_every_kernel."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(m)
+    for small in (0, 1):
+        a, w = torch.randn(m, 640, generator=g), torch.randn(130, 640, generator=g)
+        (a, w)[small].mul_(size)
+        (a, w)[1 - small].mul_(1e25)
+        exact = a.double() @ w.double().t()
+        bound = (2.0 ** -21 + (640 / 64 + 8) * 2.0 ** -24) * (a.abs().double() @ w.abs().double().t())
+        assert bool(((ops.gemm_f32(a.cuda(), w.cuda()).double().cpu() - exact).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 72, 2048), (5, 200, 260), (40, 130, 1028), (70, 8200, 516), (130, 64, 2048)])
 def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
     """Operands whose rows do not start on 16 bytes meet another kernel: the same chains over the same parts of K."""
