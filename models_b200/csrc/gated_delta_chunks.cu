@@ -441,8 +441,14 @@ delta_chunks_carry_kernel(const DeltaChunkArgs args) {
             store_pair(start + (size_t)(row + 8 * half) * V, s[2 * half], s[2 * half + 1]);
         }
         const bool here = carry_wait(smem_u32(&arrived[chunk % kCarryStages]), chunk / kCarryStages & 1);
-        if (!__syncthreads_and(here)) {  // (nobody leaves while copies may still arrive)
-            for (int later = chunk + 1; later < min(chunks, chunk + kCarryStages - 1); ++later) carry_wait(smem_u32(&arrived[later % kCarryStages]), later / kCarryStages & 1);
+        if (!__syncthreads_and(here)) {
+            // Nobody leaves while copies may still arrive, and nobody takes what was not computed for a result: the state and the starts of the
+            // chunks that are left are no numbers.
+            for (int later = chunk; later < min(chunks, chunk + kCarryStages - 1); ++later) carry_wait(smem_u32(&arrived[later % kCarryStages]), later / kCarryStages & 1);
+            const float none = __int_as_float(0x7fffffff);
+            for (int later = chunk; later < chunks; ++later)
+                for (int half = 0; half < 2; ++half) store_pair(args.starts + item(later) * kDim * V + column + (size_t)(row + 8 * half) * V, none, none);
+            for (int i = 0; i < 4; ++i) stored[(size_t)(row + 8 * (i / 2)) * V + i % 2] = none;
             return;
         }
         // S, y and the keys are there; nobody reads the stage before any more

@@ -234,6 +234,7 @@ class Engine:
     def diagnostics(self) -> Dict[str, object]:
         props = torch.cuda.get_device_properties(self.device)
         element = 2 if self.runtime.mode == "bfloat16" else 4
+        from ..kernels import ops
         from ..kernels.build import loaded_libraries
 
         return {
@@ -248,4 +249,5 @@ class Engine:
             "state_bytes": self.state.bytes,
             "max_positions": self.runtime.max_positions,
             "kernel_libraries": loaded_libraries(),
+            "waits_given_up": ops.waits_given_up(),
         }

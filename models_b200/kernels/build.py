@@ -163,3 +163,7 @@ def load_library(name: str, sources: Sequence[str], defines: Mapping[str, object
 
 def loaded_libraries():
     return sorted(_loaded)
+
+
+def loaded_library(path: str) -> ctypes.CDLL:
+    return _loaded[path]

@@ -7,11 +7,12 @@ library that cannot be built, raises.
 from __future__ import annotations
 
 import ctypes
-from typing import Optional
+import os
+from typing import Dict, Optional
 
 import torch
 
-from .build import load_library
+from .build import load_library, loaded_libraries, loaded_library
 
 _F32, _BF16 = 0, 1
 
@@ -2229,6 +2230,23 @@ def prefill_attention_tcgen05_status(head_dim: int) -> int:
 def gemm_f32_status() -> int:
     """0 while no wait of the 32-bit product ever gave up (see csrc/gemm_f32.cu)."""
     return gemm32().mb_gemm_f32_status()
+
+
+_WAIT_STATUSES = ("mb_gemm_tc_status", "mb_wide_gemm_status", "mb_prefill_attention_tc_status", "mb_gemm_f32_status",
+                  "mb_gated_delta_chunks_status")
+
+
+def waits_given_up() -> Dict[str, int]:
+    """Every kernel wait is bounded; the libraries in use that have had one run out, with the code each of them gives it.  It waits for
+    the GPU."""
+    found = {}
+    for path in loaded_libraries():
+        for name in _WAIT_STATUSES:
+            read = getattr(loaded_library(path), name, None)
+            status = int(read()) if read is not None else 0
+            if status:
+                found[f"{os.path.basename(path)}: {name}"] = status
+    return found
 
 
 def gemm_tcgen05_status() -> int:

@@ -1,8 +1,8 @@
-"""What the 32-bit product is told about its weights, without a GPU: a library that only notes its calls."""
+"""What the kernels' launchers are told and asked, without a GPU: libraries that only note and answer calls."""
 
 import torch
 
-from models_b200.kernels import ops
+from models_b200.kernels import build, ops
 from models_b200.parts.linear import linear
 
 
@@ -19,7 +19,7 @@ class Noted:
         return 0
 
     class mb_gemm_f32_scratch:
-        def __new__(cls, m, k):
+        def __new__(cls, *sizes):
             return 0
 
 
@@ -35,3 +35,15 @@ def test_only_loaded_weights_are_read_ahead(monkeypatch):
     assert lib.ready == [0, 0]
     linear(a.as_subclass(OnCard), w, torch.float32)
     assert lib.ready == [0, 0, 1]
+
+
+def test_waits_that_gave_up_are_found_in_every_library(monkeypatch):
+    class Library:
+        def __init__(self, **statuses):
+            for name, status in statuses.items():
+                setattr(self, name, lambda status=status: status)
+
+    libraries = {"/somewhere/libmb_a.so": Library(mb_gemm_f32_status=0, mb_gated_delta_chunks_status=1),
+                 "/somewhere/libmb_b.so": Library(mb_gemm_tc_status=513), "/somewhere/libmb_c.so": Library()}
+    monkeypatch.setattr(build, "_loaded", libraries)
+    assert ops.waits_given_up() == {"libmb_a.so: mb_gated_delta_chunks_status": 1, "libmb_b.so: mb_gemm_tc_status": 513}
