@@ -70,19 +70,20 @@ struct Plan {
 };
 
 // A thread's eight of a row's 64 columns, as four pairs: four columns from `from` and the four 32 further (so that eight threads' loads
-// cover whole lines), left as they are unless `wanted`.  They stand side by side in the stage: both operands have the same order of K
-// there.  kEven: whole 16-byte pieces of whole stages, by loads that a predicate holds back; else column by column, zeros from column
-// `left` on.  (Plain loads: the kernel before may just have written the row.)
+// cover whole lines); `left` columns are left from `from` on, and none is wanted of a stage that is not there.  They stand side by side in
+// the stage: both operands have the same order of K there.  kEven: whole 16-byte pieces, by loads that a predicate holds back (pieces
+// behind the last column are left as they are); else column by column, zeros behind the last.  (Plain loads: the kernel before may just have written the row.)
 template <bool kEven>
 __device__ __forceinline__ void load_eight(uint64_t (&v)[4], const float* from, int left, bool wanted) {
     if (kEven) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %5, 0;\n\t"
+            "{\n\t.reg .pred p, q;\n\t"
+            "setp.gt.s32 p, %5, 0;\n\t"
+            "setp.gt.s32 q, %5, 32;\n\t"
             "@p ld.global.v2.b64 {%0, %1}, [%4];\n\t"
-            "@p ld.global.v2.b64 {%2, %3}, [%4 + 128];\n\t}"
+            "@q ld.global.v2.b64 {%2, %3}, [%4 + 128];\n\t}"
             : "+l"(v[0]), "+l"(v[1]), "+l"(v[2]), "+l"(v[3])
-            : "l"(from), "r"((uint32_t)wanted)
+            : "l"(from), "r"(left)
             : "memory");
     } else if (wanted) {
 #pragma unroll
@@ -95,16 +96,16 @@ __device__ __forceinline__ void load_eight(uint64_t (&v)[4], const float* from, 
 
 // Four neighbouring columns, as two pairs, in the same way.
 template <bool kEven>
-__device__ __forceinline__ void load_four(uint64_t (&v)[2], const float* from, int left, bool wanted) {
+__device__ __forceinline__ void load_four(uint64_t (&v)[2], const float* from, int left) {
     if (kEven) {
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %3, 0;\n\t"
+            "setp.gt.s32 p, %3, 0;\n\t"
             "@p ld.global.v2.b64 {%0, %1}, [%2];\n\t}"
             : "+l"(v[0]), "+l"(v[1])
-            : "l"(from), "r"((uint32_t)wanted)
+            : "l"(from), "r"(left)
             : "memory");
-    } else if (wanted) {
+    } else {
         v[0] = pair_of(0 < left ? from[0] : 0.0f, 1 < left ? from[1] : 0.0f);
         v[1] = pair_of(2 < left ? from[2] : 0.0f, 3 < left ? from[3] : 0.0f);
     }
@@ -282,7 +283,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
         const int group = (warp - kAdders) / (kSplitters / 2);
         const int my_row = (threadIdx.x & 127) >> 3, unit = threadIdx.x & 7;
         uint64_t w_next[kPassesW][4] = {}, a_next[kHeldA][4] = {};
-        // Rows beyond the last repeat it; nobody reads what becomes of them.
+        // Rows beyond the last repeat it; nobody reads what becomes of them.  Columns beyond the last are zeros in A, and in W zeros or
+        // what a load before left: floats of the same row, which zeros leave without a trace unless one of them is not finite, and then
+        // the row's results are not either.
         const float* w_from = args.w + (size_t)col0 * args.ldw + k_begin + 4 * unit;
         const float* a_from = args.a + (size_t)row0 * args.lda + k_begin + 4 * unit;
         const int w_last = args.n - 1 - col0, a_last = args.m - 1 - row0;
@@ -292,7 +295,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
         };
         auto fetch_a = [&](int wanted, int p) {
             const int at = wanted * kChunk;
-            load_eight<kEven>(a_next[p], a_from + (at + (long long)min(16 * p + my_row, a_last) * args.lda), k_end - k_begin - at - 4 * unit, wanted < chunks);
+            const int left = k_end - k_begin - at - 4 * unit;
+            if (kEven && left < 36) a_next[p][2] = a_next[p][3] = 0;
+            if (kEven && left <= 0) a_next[p][0] = a_next[p][1] = 0;
+            load_eight<kEven>(a_next[p], a_from + (at + (long long)min(16 * p + my_row, a_last) * args.lda), left, wanted < chunks);
         };
         if (!args.weights_ready) grid_dependency_wait();
 #pragma unroll
@@ -456,7 +462,7 @@ gemm_f32_few_kernel(const FloatArgs args) {
         for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int step = 0; step < 4; ++step)
-                load_four<kEven>(v[h][step], w_from[h] + wanted * kChunk + 8 * step, k_end - k_begin - my_col - wanted * kChunk - 8 * step, wanted < chunks);
+                load_four<kEven>(v[h][step], w_from[h] + wanted * kChunk + 8 * step, k_end - k_begin - my_col - wanted * kChunk - 8 * step);
     };
     if (!args.weights_ready) grid_dependency_wait();
 #pragma unroll
@@ -468,7 +474,7 @@ gemm_f32_few_kernel(const FloatArgs args) {
         for (int i = threadIdx.x; i < items; i += kFewThreads) {
             const int q = i & 3, at = (i >> 4) * kChunk + 8 * (i >> 2 & 3) + 4 * (q & 1) + 32 * (q >> 1);
             uint64_t v[2] = {};
-            load_four<kEven>(v, args.a + (size_t)r * args.lda + k_begin + at, k_end - k_begin - at, true);
+            load_four<kEven>(v, args.a + (size_t)r * args.lda + k_begin + at, k_end - k_begin - at);
             uint2 hi, mid, lo;
             split_pair(pair_mul(v[0], kUp), hi.x, mid.x, lo.x);
             split_pair(pair_mul(v[1], kUp), hi.y, mid.y, lo.y);
@@ -643,7 +649,7 @@ MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, floa
     args.parts = tiles <= 37 ? 4 : tiles <= 74 ? 2 : 1;
     while (args.parts > 1 && (k < 2 * kChunk * args.parts || length(args.parts) * (args.parts - 1) >= k)) args.parts /= 2;
     args.part_length = length(args.parts);
-    const bool even_w = k % kChunk == 0 && ldw % 4 == 0 && !((uintptr_t)w & 15), even_a = k % kChunk == 0 && lda % 4 == 0 && !((uintptr_t)a & 15);
+    const bool even_w = k % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)w & 15), even_a = k % 4 == 0 && lda % 4 == 0 && !((uintptr_t)a & 15);
     if (m <= kFewRows && (long long)args.part_length * m * 6 <= kFewBytes) return even_w && even_a ? launch_few<true>(args, stream) : launch_few<false>(args, stream);
     CUtensorMap map_a{};
     if (m <= kInlineRows) {

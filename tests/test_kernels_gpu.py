@@ -203,6 +203,26 @@ def test_gemm_f32_multiplies_every_bit_of_small_floats(cuda_device, m, size):
         assert bool(((ops.gemm_f32(a.cuda(), w.cuda()).double().cpu() - exact).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("m", [3, 7, 20, 70])
+@pytest.mark.parametrize("k", [4, 32, 36, 60, 68, 132, 164, 1100])
+def test_gemm_f32_rows_that_end_within_a_stage(cuda_device, m, k):
+    """What lies behind the last column is not a number, and so is a float of one row: neither reaches another result."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(k)
+    wide_a, wide_w = torch.full((m, k + 64), float("nan")), torch.full((200, k + 64), float("nan"))
+    wide_a[:, :k], wide_w[:, :k] = torch.randn(m, k, generator=g), torch.randn(200, k, generator=g)
+    a, w = wide_a.cuda()[:, :k], wide_w.cuda()[:, :k]
+    exact = wide_a[:, :k].double() @ wide_w[:, :k].double().t()
+    bound = (2.0 ** -21 + (k / 64 + 8) * 2.0 ** -24) * (wide_a[:, :k].abs().double() @ wide_w[:, :k].abs().double().t())
+    out = ops.gemm_f32(a, w)
+    assert bool(((out.double().cpu() - exact).abs() <= bound).all())
+    w[5, k // 2], w[9, 0] = float("nan"), float("inf")
+    again = ops.gemm_f32(a, w)
+    others = [i for i in range(200) if i not in (5, 9)]
+    assert torch.equal(again[:, others], out[:, others]) and bool(torch.isnan(again[:, 5]).all()) and bool(torch.isinf(again[:, 9]).all())
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 72, 2048), (5, 200, 260), (40, 130, 1028), (70, 8200, 516), (130, 64, 2048)])
 def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
     """Operands whose rows do not start on 16 bytes meet another kernel: the same chains over the same parts of K."""
