@@ -12,15 +12,13 @@
 // sits in a tile, nor on alignment, nor on which of the kernels below computes it.
 //
 // Off the sums in 64 bits by 1.0e-7 to 1.4e-7 (2-norm; K 2,048 and 8,192); chains of FMAs over the same parts were 2.9e-7 to 5.8e-7 off.
-// 301 rows, W of 16,384 x 2,048 that are bfloat16 numbers: 92 us, 2,048 x 8,192 55 us, 3,072 x 2,048 38 us, 2,048 x 2,048 21 us (whole
-// floats 118, 67, 44 and 24); FMAs on 8 x 8 results a thread took 480, 274, 114 and 80 us, at 46 of the CUDA cores' 74 TFLOP/s.
-// From 33 rows on a block is bound by the splitting of W (1,500 to 2,000 cycles per 64 columns; 12 or 24 products of 160 rows take the
-// tensor cores 960 or 1,920).  One row: 16,384 x 2,048 in 28 us (29 before), 2,048 x 8,192 in 22 (17 before: sixteen rows of W at a time
-// leave a scheduler one warp), eight rows 30 us (43 before) and 23 (26).
+// 301 rows, W of 16,384 x 2,048 that are bfloat16 numbers: 89 us, 2,048 x 8,192 52 us, 3,072 x 2,048 37 us, 2,048 x 2,048 21 us (whole
+// floats 104, 62, 41 and 24); FMAs on 8 x 8 results a thread took 480, 274, 114 and 80 us, at 46 of the CUDA cores' 74 TFLOP/s.
+// From 33 rows on a block is bound by the splitting of W; the kernel for few rows says what bounds it.
 //
 // 128 rows of W are the products' first operand and up to 160 rows of A the second.  Eight warps bring W from memory (loads of the
 // next columns are under way while these are worked on) and split it into shared memory, one brings A, which a kernel before has
-// split (of up to 32 rows the eight warps split it too: in 301 rows that doubled their work, 127 us for 92), one issues the products,
+// split (of few rows, and in small products, the eight warps split it too: in 301 rows that doubled their work, 127 us for 92), one issues the products,
 // and four hold the sums, a row of W per thread.  Weights that are bfloat16 numbers -- most models' are, in the 32-bit mode too -- have
 // two parts of zeros, whose products are left out: each stage of W says whether it is such.
 //
@@ -424,140 +422,193 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
     }
 }
 
-// ---- Up to four rows of A: the weights' stream bounds the product, and nothing of W passes through shared memory.  A warp owns 16 rows of W;
-// its lanes load them 16 bytes at a time (kFewAhead chunks in registers), split them there and multiply them by mma.sync, whose sums over
-// 16 columns are the tcgen05 ones, bit by bit, in whatever order these columns stand: the same steps in the same order give the same
-// results.  A's parts lie in shared memory, split by the block itself.
-constexpr int kFewRows = 4, kFewWarps = 4, kFewThreads = 32 * kFewWarps, kFewRowsW = 16 * kFewWarps;
-constexpr int kFewBytes = 200 * 1024;  // most shared memory for A's parts
-constexpr int kFewAlone = 116 * 1024;  // with so much a block has a multiprocessor to itself
-constexpr int kFewAhead = 3;           // (2,048 rows of W, K 8,192, one row of A: 34 us with one, 25 with two, 22 with three, 33 with four)
+// ---- Up to eight rows of A: the weights' stream bounds the product.  A warp owns sixteen rows of W and copies them to shared memory in
+// whole lines, kStages - 1 chunks ahead, in a ring of its own; its lanes split them and multiply them by mma.sync, whose sums over 16
+// columns are the tcgen05 ones, bit by bit, in whatever order these columns stand: the same steps in the same order give the same results.
+// A's parts lie in shared memory, split by the block itself.
+// Bound, over long rows, by what a warp does with a chunk, 3.5 to 7 warps to a multiprocessor, else by the stream (268 MB at 5.5 TB/s).
+// One row, us, W of bfloat16 numbers and of floats (before that as chains of float FMAs): 2,048 x 2,048 6.7 and 7.7 (6.5), 3,072 x 2,048 8.1
+// and 9.4 (7.7), 2,048 x 8,192 17.3 and 21.8 (17.0), 4,096 x 4,096 14.0 and 16.7 (16.2), 16,384 x 2,048 25.5 and 28.3 (30.5), 32,768 x 2,048
+// 48.9 and 47 (52).  Chunks in registers, 16 bytes of a row to a lane, took 7.5, 8.9, 22.6, 17, 30.4 and 57.6; smaller parts made of
+// weights that have none 7.5, 8.9, 21.8, 16.9, 29.4 and 50.1; tiles of eight rows, the instruction's other eight zeros, 6.8, 7.9, 18.4, 16.3
+// and, of 4,096 x 4,096 floats, 20.2.
+constexpr int kFewRows = 8, kFewTile = 16, kFewMostWarps = 16;
+constexpr int kFewBytes = 216 * 1024;  // most shared memory that a block asks for
+constexpr int kFewChunkBytes = kFewTile * kChunk * (int)sizeof(float);
+constexpr int kFewBatch = 4;           // a thread's loads of A that are under way together
+// A's parts: [row][chunk][16 columns][3 parts][4 lanes] pairs of words (a lane's two operand registers); rows lie a few words apart from
+// whole lines, so that the lanes of different rows meet different banks.
+__host__ __device__ constexpr int few_row(int chunks) { return chunks * 48 + 4; }
 
 __device__ __forceinline__ void mma_step(float (&d)[4], const uint32_t (&a)[4], uint2 b) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
 }
-
-// Shared memory: A's parts, [row][chunk][16 columns][3 parts][4 lanes] pairs of words (a lane's two operand registers).
+// Four neighbouring columns, zeros behind the last.
 template <bool kEven>
-__global__ void __launch_bounds__(kFewThreads)
+__device__ __forceinline__ void copy_four(uint32_t to, const float* from, int left) {
+    if (kEven) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(left > 0 ? from : from + left - 4), "r"(left > 0 ? 16 : 0) : "memory");
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + 4 * e), "l"(e < left ? from + e : from + left - 1), "r"(e < left ? 4 : 0) : "memory");
+    }
+}
+// Where 16-byte piece `piece` of a row's chunk lies: what eight lanes read together (two rows, pieces 0, 1, 8 and 9 from an even one on) and
+// what they copy together (eight pieces of a row) meet all banks.
+__device__ __forceinline__ int few_place(int row, int piece) { return row * 256 + (piece >> 3) * 128 + (((piece & 7) ^ (piece >> 3) * 2 ^ (row & 1) * 4) << 4); }
+
+// One part of K: a block's warps take tiles of W in turn.  Several: a warp takes one tile, and the part's cluster rank is blockIdx.x % parts.
+template <bool kEven, int kStages>
+__global__ void __launch_bounds__(32 * kFewMostWarps)
 gemm_f32_few_kernel(const FloatArgs args) {
     extern __shared__ __align__(16) uint2 few_parts[];
-    __shared__ float sums[kFewRows][kFewRowsW];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = lane >> 2, quad = lane & 3;
-    const int part = blockIdx.x % args.parts, col0 = (blockIdx.x / args.parts) * kFewRowsW;
-    const int k_begin = part * args.part_length, k_end = min(args.k, k_begin + args.part_length);
-    const int chunks = (k_end - k_begin + kChunk - 1) / kChunk, m = args.m;
+    __shared__ float sums[kFewRows][kFewTile * kFewMostWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = lane >> 2, quad = lane & 3, threads = blockDim.x, warps = threads >> 5;
+    const int part = blockIdx.x % args.parts, block = blockIdx.x / args.parts;
+    const int k_begin = part * args.part_length, columns = min(args.k - k_begin, args.part_length);
+    const int chunks = (columns + kChunk - 1) / kChunk, m = args.m, row_pairs = few_row(chunks);
+    const int tiles = (args.n + kFewTile - 1) / kFewTile;
+    const int first_tile = args.parts > 1 ? block * warps + warp : warp * gridDim.x + block, stride = args.parts > 1 ? tiles : warps * gridDim.x;
     grid_launch_dependents();
 
-    // a lane's columns of the sixteen of a step: four from 8 * step + 4 * (quad & 1) + 32 * (quad >> 1)
-    const int my_col = 4 * (quad & 1) + 32 * (quad >> 1);
-    const float* w_from[2];  // (rows beyond the last repeat it)
+    unsigned char* ring = reinterpret_cast<unsigned char*>(few_parts + m * few_row(args.part_length / kChunk)) + warp * (kStages * kFewChunkBytes);
+    const int piece = lane & 15;  // what the lane copies: two rows at a time
+    const uint32_t put_at = (uint32_t)__cvta_generic_to_shared(ring) + few_place(lane >> 4, piece);
+    const float* from[kFewTile / 2];
+    int next_tile = first_tile, next_chunk = 0, next_slot = 0;
+    auto begin_tile = [&]() {  // rows beyond the last repeat it
 #pragma unroll
-    for (int h = 0; h < 2; ++h) w_from[h] = args.w + (size_t)min(col0 + warp * 16 + group + 8 * h, args.n - 1) * args.ldw + k_begin + my_col;
-    uint64_t next[kFewAhead][2][4][2] = {};  // [chunk ahead][row][step][pairs of columns]
-    auto fetch = [&](int wanted, uint64_t (&v)[2][4][2]) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int step = 0; step < 4; ++step)
-                load_four<kEven>(v[h][step], w_from[h] + wanted * kChunk + 8 * step, k_end - k_begin - my_col - wanted * kChunk - 8 * step);
+        for (int i = 0; i < kFewTile / 2; ++i) from[i] = args.w + (size_t)min(next_tile * kFewTile + 2 * i + (lane >> 4), args.n - 1) * args.ldw + k_begin + 4 * piece;
     };
+    auto fetch = [&]() {
+        if (next_tile < tiles) {
+            const int left = columns - next_chunk * kChunk - 4 * piece;
+#pragma unroll
+            for (int i = 0; i < kFewTile / 2; ++i) {
+                copy_four<kEven>(put_at + next_slot * kFewChunkBytes + i * few_place(2, 0), from[i], left);
+                from[i] += kChunk;
+            }
+            if (++next_chunk == chunks) {
+                next_chunk = 0, next_tile += stride;
+                begin_tile();
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (++next_slot == kStages) next_slot = 0;
+    };
+    begin_tile();
     if (!args.weights_ready) grid_dependency_wait();
 #pragma unroll
-    for (int i = 0; i < kFewAhead; ++i) fetch(i, next[i]);
+    for (int i = 0; i < kStages - 1; ++i) fetch();
     grid_dependency_wait();
-    // A's parts: a thread takes the four columns of one lane of a step
+    // A's parts: a thread takes the four columns of one lane of a step, from 8 * step + 4 * (quad & 1) + 32 * (quad >> 1)
     const int items = chunks * 16;
-    for (int r = 0; r < m; ++r)
-        for (int i = threadIdx.x; i < items; i += kFewThreads) {
-            const int q = i & 3, at = (i >> 4) * kChunk + 8 * (i >> 2 & 3) + 4 * (q & 1) + 32 * (q >> 1);
-            uint64_t v[2] = {};
-            load_four<kEven>(v, args.a + (size_t)r * args.lda + k_begin + at, k_end - k_begin - at);
+    for (int first = threadIdx.x; first < m * items; first += kFewBatch * threads) {
+        uint64_t v[kFewBatch][2] = {};
+#pragma unroll
+        for (int b = 0; b < kFewBatch; ++b) {
+            const int i = first + b * threads, r = i / items, item = i - r * items, q = item & 3;
+            const int at = (item >> 4) * kChunk + 8 * (item >> 2 & 3) + 4 * (q & 1) + 32 * (q >> 1);
+            if (r < m) load_four<kEven>(v[b], args.a + (size_t)r * args.lda + k_begin + at, columns - at);
+        }
+#pragma unroll
+        for (int b = 0; b < kFewBatch; ++b) {
+            const int i = first + b * threads, r = i / items, item = i - r * items;
+            if (r >= m) break;
             uint2 hi, mid, lo;
-            split_pair(pair_mul(v[0], kUp), hi.x, mid.x, lo.x);
-            split_pair(pair_mul(v[1], kUp), hi.y, mid.y, lo.y);
-            uint2* to = few_parts + (r * chunks * 4 + (i >> 2)) * 12 + q;
+            split_pair(pair_mul(v[b][0], kUp), hi.x, mid.x, lo.x);
+            split_pair(pair_mul(v[b][1], kUp), hi.y, mid.y, lo.y);
+            uint2* to = few_parts + r * row_pairs + (item >> 2) * 12 + (item & 3);
             to[0] = hi, to[4] = mid, to[8] = lo;
         }
+    }
     __syncthreads();
 
-    float sum[4] = {}, small[4] = {};
-    const bool live = group < m;
-    const uint2* mine = few_parts + (live ? group : 0) * chunks * 48 + quad;
-    for (int chunk0 = 0; chunk0 < chunks; chunk0 += kFewAhead) {
+    const uint2* mine = few_parts + min(group, m - 1) * row_pairs + quad;  // (nobody reads the results of rows beyond the last)
+    int slot = 0;
+#pragma unroll 1
+    for (int tile = first_tile; tile < tiles; tile += stride) {
+        float sum[4] = {}, small[4] = {};  // rows group and group + 8 of W with rows 2 * quad and 2 * quad + 1 of A
+#pragma unroll 1
+        for (int chunk = 0; chunk < chunks; ++chunk) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+            __syncwarp();  // the chunk is there for every lane, and every lane has read the one before
+            uint32_t w[4][3][4] = {};  // [step][part][operand registers: row and row + 8 of the first two columns, then of the others]
+            uint64_t rest[4][4];  // what their roundings leave
+            uint64_t any = 0;
+            const unsigned char* at = ring + slot * kFewChunkBytes;
 #pragma unroll
-        for (int i = 0; i < kFewAhead; ++i) {
-            const int chunk = chunk0 + i;
-            if (chunk >= chunks) break;
-            uint32_t w[4][3][4];  // [step][part][operand registers: row and row + 8 of the first two columns, then of the others]
-            uint2 a[4][3];
-            uint32_t smaller = 0;
+            for (int step = 0; step < 4; ++step)
 #pragma unroll
-            for (int step = 0; step < 4; ++step) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
+                for (int h = 0; h < 2; ++h) {
+                    const float4 x = *reinterpret_cast<const float4*>(at + few_place(group + 8 * h, (quad & 1) + 8 * (quad >> 1) + 2 * step));
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const uint64_t v = pair_mul(next[i][h][step][e], kUp);
-                        split_pair(v, w[step][0][2 * e + h], w[step][1][2 * e + h], w[step][2][2 * e + h]);
-                        smaller |= w[step][1][2 * e + h] | w[step][2][2 * e + h];
+                        const uint64_t v = pair_mul(e == 0 ? pair_of(x.x, x.y) : pair_of(x.z, x.w), kUp);
+                        w[step][0][2 * e + h] = round_pair(v);
+                        rest[step][2 * e + h] = minus_rounding(v, w[step][0][2 * e + h]);
+                        any |= rest[step][2 * e + h];
                     }
-#pragma unroll
-                for (int p = 0; p < 3; ++p) a[step][p] = live ? mine[(chunk * 4 + step) * 12 + p * 4] : make_uint2(0u, 0u);
-            }
-            fetch(chunk + kFewAhead, next[i]);
-            const bool all_parts = __any_sync(0xffffffffu, (smaller & 0x7fff7fffu) != 0);
+                }
+            fetch();  // to the place of the chunk before
+            if (++slot == kStages) slot = 0;
+            const bool all_parts = __any_sync(0xffffffffu, any != 0);
             auto products = [&](int w_part, int a_part, float (&to)[4]) {
 #pragma unroll
-                for (int step = 0; step < 4; ++step) mma_step(to, w[step][w_part], a[step][a_part]);
+                for (int step = 0; step < 4; ++step) mma_step(to, w[step][w_part], mine[(chunk * 4 + step) * 12 + a_part * 4]);
             };
             float whole[4] = {};
             products(0, 0, whole);
             products(0, 2, small);
             if (all_parts) {
+#pragma unroll
+                for (int step = 0; step < 4; ++step)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        w[step][1][i] = round_pair(rest[step][i]);
+                        w[step][2][i] = round_pair(minus_rounding(rest[step][i], w[step][1][i]));
+                    }
                 products(1, 1, small);
                 products(2, 0, small);
             }
             products(0, 1, small);
             if (all_parts) products(1, 0, small);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) sum[j] += whole[j];
+            for (int i = 0; i < 4; ++i) sum[i] += whole[i];
         }
-    }
-    // a lane holds rows group and group + 8 of the warp's sixteen of W, rows 2 * quad and 2 * quad + 1 of A
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int r = 2 * quad + e, of_block = warp * 16 + group + 8 * h, col = col0 + of_block;
+        for (int i = 0; i < 4; ++i) {
+            const int r = 2 * quad + i % 2, of_tile = group + i / 2 * 8, col = tile * kFewTile + of_tile;
             if (r >= m) continue;
-            float total = (sum[2 * h + e] + small[2 * h + e]) * low_of(kDown);
+            float total = (sum[i] + small[i]) * low_of(kDown);
             if (!isfinite(total)) {
                 const float *a = args.a + (size_t)r * args.lda, *w = args.w + (size_t)min(col, args.n - 1) * args.ldw;
                 total = 0.0f;
 #pragma unroll 1
-                for (int k = k_begin; k < k_end; ++k) total = fmaf(a[k], w[k], total);
+                for (int k = k_begin; k < k_begin + columns; ++k) total = fmaf(a[k], w[k], total);
             }
-            if (args.parts > 1) sums[r][of_block] = total;
+            if (args.parts > 1) sums[r][warp * kFewTile + of_tile] = total;
             else if (col < args.n) args.c[(size_t)r * args.ldc + col] = total;
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (args.parts > 1) {  // the first block of the cluster adds the parts in their order
         cg::this_cluster().sync();
         if (part == 0)
-            for (int i = threadIdx.x; i < m * kFewRowsW; i += kFewThreads) {
-                const int r = i / kFewRowsW, col = i % kFewRowsW;
+            for (int i = threadIdx.x; i < m * warps * kFewTile; i += threads) {
+                const int r = i / (warps * kFewTile), c = i % (warps * kFewTile), col = block * warps * kFewTile + c;
                 float v[4];
 #pragma unroll
                 for (int p = 0; p < 4; ++p)
-                    if (p < args.parts) v[p] = cg::this_cluster().map_shared_rank(&sums[0][0], p)[i];
+                    if (p < args.parts) v[p] = cg::this_cluster().map_shared_rank(&sums[r][c], p)[0];
                 float total = v[0];
 #pragma unroll
                 for (int p = 1; p < 4; ++p)
                     if (p < args.parts) total += v[p];
-                if (col0 + col < args.n) args.c[(size_t)r * args.ldc + col0 + col] = total;
+                if (col < args.n) args.c[(size_t)r * args.ldc + col] = total;
             }
         cluster_leave_together();
     }
@@ -590,18 +641,36 @@ static int launch(const CUtensorMap& map_a, const FloatArgs& args, cudaStream_t 
     return check_launch("gemm_f32");
 }
 
-template <bool kEven>
-static int launch_few(const FloatArgs& args, cudaStream_t stream) {
-    int bytes = args.part_length * args.m * 6;
+// How few rows are launched: a block to a multiprocessor, of the fewest warps that have a tile each, 16 that take tiles in turn where there
+// are more.  (Two blocks of four warps, 3,072 x 2,048: 7.7 us, one of eight 8.0; 5,000 x 4,100: 26.5 and 25.4.)  Chunks under way: eight warps
+// with two stages lose to the kernel of many rows (eight rows, 16,384 x 2,048: 38.4 us, and 33.3), which takes what finds no place here.
+struct FewPlan {
+    int warps, stages, bytes, blocks;
+};
+static FewPlan few_plan(const FloatArgs& args) {
+    const long long rows = (long long)few_row(args.part_length / kChunk) * args.m * sizeof(uint2);
+    const int tiles = (args.n + kFewTile - 1) / kFewTile;
+    auto blocks = [&](int warps) { return (tiles + warps - 1) / warps * args.parts; };
+    FewPlan plan{};
+    for (int warps = blocks(4) <= 148 ? 4 : blocks(8) <= 148 ? 8 : 16; warps >= 4 && plan.warps == 0; warps = warps == 16 ? 8 : 0)
+        for (int stages = warps == 16 ? 3 : 4; stages >= (warps == 16 ? 2 : 3) && plan.warps == 0; --stages) {
+            const long long bytes = rows + stages * warps * kFewChunkBytes;
+            if (bytes > kFewBytes) continue;
+            plan.warps = warps, plan.stages = stages, plan.blocks = std::min(blocks(warps), 148);
+            plan.bytes = (int)std::max<long long>(bytes, 116 * 1024);  // (so that there is no room for another block)
+        }
+    return plan;
+}
+
+template <bool kEven, int kStages>
+static int launch_few(const FloatArgs& args, const FewPlan& plan, cudaStream_t stream) {
+    auto kernel = gemm_f32_few_kernel<kEven, kStages>;
     static DeviceSet devices{0};
-    if (int status = reserve_shared("gemm_f32", gemm_f32_few_kernel<kEven>, kFewBytes, devices)) return status;
-    const long long blocks = (long long)((args.n + kFewRowsW - 1) / kFewRowsW) * args.parts;
-    if (blocks > 0x7fffffff) return fail("gemm_f32: %d x %d results exceed the grid limit", args.m, args.n);
+    if (int status = reserve_shared("gemm_f32", kernel, kFewBytes, devices)) return status;
     cudaLaunchConfig_t config = {};
-    if (blocks <= 148) bytes = std::max(bytes, kFewAlone);  // (the blocks of a cluster share a multiprocessor where two fit, and leave others idle)
-    config.gridDim = dim3((unsigned)blocks);
-    config.blockDim = dim3(kFewThreads);
-    config.dynamicSmemBytes = bytes;
+    config.gridDim = dim3(plan.blocks);
+    config.blockDim = dim3(32 * plan.warps);
+    config.dynamicSmemBytes = plan.bytes;
     config.stream = stream;
     cudaLaunchAttribute attribute[2];
     attribute[0].id = cudaLaunchAttributeClusterDimension;
@@ -612,9 +681,15 @@ static int launch_few(const FloatArgs& args, cudaStream_t stream) {
     attribute[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attribute;
     config.numAttrs = dependent_launches_allowed() ? 2 : 1;
-    const cudaError_t status = cudaLaunchKernelEx(&config, gemm_f32_few_kernel<kEven>, args);
+    const cudaError_t status = cudaLaunchKernelEx(&config, kernel, args);
     if (status != cudaSuccess) return fail("gemm_f32: launch failed: %s", cudaGetErrorString(status));
     return check_launch("gemm_f32");
+}
+
+template <bool kEven>
+static int launch_few_stages(const FloatArgs& args, const FewPlan& plan, cudaStream_t stream) {
+    if (plan.stages == 4) return launch_few<kEven, 4>(args, plan, stream);
+    return plan.stages == 3 ? launch_few<kEven, 3>(args, plan, stream) : launch_few<kEven, 2>(args, plan, stream);
 }
 
 template <int NB, int kRowsW>
@@ -650,7 +725,10 @@ MB_EXPORT int mb_gemm_f32(const float* a, int lda, const float* w, int ldw, floa
     while (args.parts > 1 && (k < 2 * kChunk * args.parts || length(args.parts) * (args.parts - 1) >= k)) args.parts /= 2;
     args.part_length = length(args.parts);
     const bool even_w = k % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)w & 15), even_a = k % 4 == 0 && lda % 4 == 0 && !((uintptr_t)a & 15);
-    if (m <= kFewRows && (long long)args.part_length * m * 6 <= kFewBytes) return even_w && even_a ? launch_few<true>(args, stream) : launch_few<false>(args, stream);
+    if (m <= kFewRows) {
+        const FewPlan plan = few_plan(args);
+        if (plan.warps > 0) return even_w && even_a ? launch_few_stages<true>(args, plan, stream) : launch_few_stages<false>(args, plan, stream);
+    }
     CUtensorMap map_a{};
     // More rows than 32 are split where they are multiplied, too, while tiles of 32 make no more blocks than multiprocessors: that saves the
     // kernel that splits (64 rows, 2,048 x 2,048: 14.4 -> 10.9 us, 2,048 x 8,192 38.4 -> 28.7, 301 rows, 256 x 64: 6.6 -> 2.7).  Element loads

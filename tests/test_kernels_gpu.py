@@ -223,6 +223,26 @@ def test_gemm_f32_rows_that_end_within_a_stage(cuda_device, m, k):
     assert torch.equal(again[:, others], out[:, others]) and bool(torch.isnan(again[:, 5]).all()) and bool(torch.isinf(again[:, 9]).all())
 
 
+@pytest.mark.parametrize("n,k", [(5, 64), (300, 100), (2048, 2048), (3076, 2048), (9480, 512), (4100, 516), (9480, 4100), (15000, 132), (40000, 260), (40000, 1900), (37, 8192)])
+def test_gemm_f32_few_rows(cuda_device, n, k):
+    """Up to eight rows: tiles of W that do and do not fill blocks of 4, 8 and 16 warps, one after another where there are more tiles than
+    warps, one to four parts of K, A's parts that leave room for fewer stages; the bits of the kernel that many rows take."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(n)
+    a, w = torch.randn(40, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    out = ops.gemm_f32(a, w)
+    exact = a.double() @ w.double().t()
+    bound = (2.0 ** -21 + (k / 64 + 8) * 2.0 ** -24) * (a.abs().double() @ w.abs().double().t())
+    assert bool(((out.double() - exact).abs() <= bound).all())
+    for rows in range(1, 9):
+        assert torch.equal(ops.gemm_f32(a[:rows], w), out[:rows])
+    rounded = w.bfloat16().float()  # (weights with two parts of zeros)
+    out = ops.gemm_f32(a, rounded)
+    for rows in (1, 4, 8):
+        assert torch.equal(ops.gemm_f32(a[:rows], rounded, weights_ready=True), out[:rows])
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 72, 2048), (5, 200, 260), (40, 130, 1028), (70, 8200, 516), (130, 64, 2048)])
 def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
     """Operands whose rows do not start on 16 bytes meet another kernel: the same chains over the same parts of K."""
