@@ -244,7 +244,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const FloatArgs args)
         if (ok) add(tmem_small);
         tcgen05_fence_before();
 #pragma unroll
-        for (int j = 0; j < P::kRows / 2; ++j) sum[j] = pair_mul(sum[j], kDown);
+        for (int j = 0; j < P::kRows / 2; ++j) sum[j] = ok ? pair_mul(sum[j], kDown) : ~0ull;  // (NaN, where a wait gave up: computed anew)
         // To the result, or, as one of several parts, to shared memory (every product has read the stages): [rows of A][kRowsW].
         const int col = col0 + (int)threadIdx.x;
         const int rows = (int)threadIdx.x >= kRowsW ? 0 : args.parts > 1 ? P::kRows : col < args.n ? min(P::kRows, args.m - row0) : 0;
