@@ -1,8 +1,9 @@
-// Causal grouped-query attention over a paged cache, one warp per (token, head) row.
+// Causal grouped-query attention over a paged cache in plain arithmetic: one warp per (token, head) row, or, for the prompts of
+// the 32-bit path with heads of 64 and 128, rows in tiles that share keys and values.
 //
-// This is the plain-arithmetic kernel: every size of head (up to 256), float or bfloat16 storage,
-// prompts and single decoded tokens alike.  It is the whole attention of the 32-bit path and the
-// fallback of the bfloat16 path for head sizes its tensor-core kernels do not take.
+// The first takes every size of head (up to 256), float or bfloat16 storage, prompts and single decoded tokens alike.  The two
+// are the whole attention of the 32-bit path; the first is the fallback of the bfloat16 path for head sizes its tensor-core
+// kernels do not take.
 //
 // Formula (integrallis/models, backend-java/.../llama/LlamaForwardPass.java:1543-1670 and
 // backend-java/.../ops/TensorOps.java:1247-1279): kvHead = head / (heads / kv_heads);

@@ -3,10 +3,11 @@
 //
 // out[r] = sum_c W[r, c] * x[c] (integrallis/models, backend-java/.../ops/TensorOps.java:61-63).
 // A float is the sum of three bfloat16 numbers (float_parts.cuh), and a product of floats that of six products of these (the other
-// three are below 2^-26 of it), summed in float:
+// three are 2^-24 of it at most: a second part is up to 2^-8 of its float, a third up to 2^-17), summed in float:
 //   * the products of the two roundings, 64 columns of K at a time, in tensor memory, and these sums by float additions in
 //     registers: a tensor core cuts its sum off where a float addition rounds, so no long sum may stay there;
-//   * the five smaller products, which lose nothing that counts to the cut, in tensor memory over all of the block's columns.
+//   * the five smaller products, 2^-7 of the whole together, in tensor memory over all of the block's columns: the cut takes up to
+//     2^-31 K of the whole from them (20 steps a stage, 2^-23 of their sum each).
 // Every result is the sum, in order, of up to four such sums over consecutive parts of K; the parts follow from N and K alone, and
 // every call runs the same operations on a row, so a row's result depends neither on the other rows of the call, nor on where it
 // sits in a tile, nor on alignment, nor on which of the kernels below computes it.

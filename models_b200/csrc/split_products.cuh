@@ -1,6 +1,7 @@
 // Products of floats on the tensor cores (mma.sync m16n8k16) that keep a float's 24 bits: every operand is three bfloat16 numbers, its
 // rounding, the rounding of what that left and of what this left, and six of the nine products of parts are added up in float (the
-// other three are below 2^-26 of the product).  Operands lie in shared memory as three planes, one after another.
+// other three are 2^-24 of the product at most: a second part is up to 2^-8 of its float, a third up to 2^-17).  Operands lie in shared
+// memory as three planes, one after another.
 #pragma once
 
 #include "float_parts.cuh"

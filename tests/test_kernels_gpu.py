@@ -91,7 +91,7 @@ def test_gemm_f32_rows_of_pieces(cuda_device, m, n, k):
     g = torch.Generator().manual_seed(12)
     a, w = torch.randn(m, k + 4, generator=g).cuda()[:, :k], torch.randn(n, k + 8, generator=g).cuda()[:, :k]
     out = ops.gemm_f32(a, w)
-    # a chain of k FMAs is off by at most k roundings of its partial sums, each within the sum of the products' sizes
+    # what test_gemm_f32_sums_of_one_sign derives is below this for every k here
     bound = 2.0 ** -24 * k * (a.abs().double() @ w.abs().double().t())
     assert bool(((out.double() - a.double() @ w.double().t()).abs() <= bound).all())
     for rows in (1, 3, 9, 33):
@@ -113,8 +113,8 @@ def test_gemm_f32_gives_a_row_the_same_bits_in_every_kernel(cuda_device, weights
         w = rounded if weights == "bfloat16" else torch.where(torch.arange(n, device=cuda_device)[:, None] == 70 % n, w, rounded)
     out = ops.gemm_f32(a, w)
     exact = a.double() @ w.double().t()
-    # three parts hold 24 bits of each factor and drop 2^-26 of a product; sums over 64 columns are cut off four times (2^-23 each),
-    # the sums of these are rounded k / 64 + 8 times
+    # the sums of the roundings' products and their float additions; what is dropped (2^-24) and what the small products' sum loses
+    # (2^-31 k at most, see test_gemm_f32_sums_of_one_sign) is far from all of one sign here
     bound = (2.0 ** -21 + (k / 64 + 8) * 2.0 ** -24) * (a.abs().double() @ w.abs().double().t())
     assert bool(((out.double() - exact).abs() <= bound).all())
     for rows in (1, 4, 5, 32, 33, 65, 97, 129, 160, 161):
@@ -223,6 +223,26 @@ def test_gemm_f32_rows_that_end_within_a_stage(cuda_device, m, k):
     assert torch.equal(again[:, others], out[:, others]) and bool(torch.isnan(again[:, 5]).all()) and bool(torch.isinf(again[:, 9]).all())
 
 
+@pytest.mark.parametrize("weights", ["the float that loses most", "near one"])
+@pytest.mark.parametrize("m,n,k", [(2, 130, 2048), (20, 130, 2048), (70, 9480, 8192)])
+def test_gemm_f32_sums_of_one_sign(cuda_device, weights, m, n, k):
+    """The bound of the split products where nothing cancels.  A float's second part is up to 2^-8 of it, its third up to 2^-17, so that the
+    three products left out are up to 2^-24 of the whole; sums of 64 columns of the roundings' products are cut off four times (2^-23
+    each) and added with k / 64 + 8 roundings (2^-24 each); the five small products, 2^-7 of the whole together, stay in one sum that is
+    cut off 20 times a stage (20 / 64 k 2^-30)."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(k)
+    if weights == "near one":
+        a, w = 1 + torch.rand(m, k, generator=g) * 2.0 ** -7, 1 + torch.rand(n, k, generator=g) * 2.0 ** -7
+    else:
+        worst = torch.tensor([0x3F807FC0], dtype=torch.int32).view(torch.float32)  # 1 + 2^-8 - 2^-17: parts 1, 2^-8 and -2^-17
+        a, w = worst.expand(m, k).contiguous(), worst.expand(n, k).contiguous()
+    exact = a.cuda().double() @ w.cuda().double().t()
+    bound = 2.0 ** -24 + 2.0 ** -21 + (k / 64 + 8) * 2.0 ** -24 + k * 2.0 ** -31
+    assert bool(((ops.gemm_f32(a.cuda(), w.cuda()).double() - exact).abs() <= bound * exact).all())
+
+
 @pytest.mark.parametrize("n,k", [(5, 64), (300, 100), (2048, 2048), (3076, 2048), (9480, 512), (4100, 516), (9480, 4100), (15000, 132), (40000, 260), (40000, 1900), (37, 8192)])
 def test_gemm_f32_few_rows(cuda_device, n, k):
     """Up to eight rows: tiles of W that do and do not fill blocks of 4, 8 and 16 warps, one after another where there are more tiles than
@@ -245,7 +265,7 @@ def test_gemm_f32_few_rows(cuda_device, n, k):
 
 @pytest.mark.parametrize("m,n,k", [(1, 72, 2048), (5, 200, 260), (40, 130, 1028), (70, 8200, 516), (130, 64, 2048)])
 def test_gemm_f32_gives_the_same_bits_off_its_alignment(cuda_device, m, n, k):
-    """Operands whose rows do not start on 16 bytes meet another kernel: the same chains over the same parts of K."""
+    """Operands whose rows do not start on 16 bytes are loaded float by float: the same sums over the same parts of K."""
     from models_b200.kernels import ops
 
     g = torch.Generator().manual_seed(13)
