@@ -21,6 +21,17 @@ __device__ __forceinline__ uint64_t minus_quotients(uint64_t x, float y0, float 
     return pair_fma(pair_fma(y, q, x), r, q);
 }
 
+__device__ __forceinline__ float min_of(float a, float b, float c) {  // NaN counts for nothing, as in fminf
+    float m;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
+}
+__device__ __forceinline__ float max_of(float a, float b, float c) {
+    float m;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
+}
+
 // gate[i] = gated_pair(activation, gate[i], up[i], clamp).  A division has a long way for unusual operands, and a branch to it after every pair
 // keeps pairs from being worked on side by side; here one branch says whether all of a thread's gates are usual ones: exponentials up to e^40
 // (every divisor then lies from 1 to 2^58, and no remainder that counts is below the floats), gates up to 2^60.  NaN passes through either way.
@@ -30,7 +41,7 @@ __device__ __forceinline__ void gate_pairs(int activation, float (&gate)[kCount]
     if (activation == MB_ACT_SILU || activation == MB_ACT_CLAMPED_SWISH) {
         float lowest = gate[0], highest = gate[0];
 #pragma unroll
-        for (int i = 1; i < kCount; ++i) lowest = fminf(lowest, gate[i]), highest = fmaxf(highest, gate[i]);
+        for (int i = 0; i < kCount; i += 2) lowest = min_of(lowest, gate[i], gate[i + 1]), highest = max_of(highest, gate[i], gate[i + 1]);
         if (activation == MB_ACT_SILU) {
             if (lowest >= -40.0f && highest <= 0x1p60f) {
 #pragma unroll
