@@ -333,7 +333,8 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
 // grid (V / kColumns, heads, sequences); block kCarryThreads: a warp has 16 coordinates of S (and 16 tokens of u) at eight of the block's
 // columns, as its products leave them.  The next two chunks' y and keys arrive by bulk copies, the next one's x in registers, while this one's are
 // used.  (Bound by the latency of the two products one after the other.  2,048 tokens: 65 us with four warps of sixteen columns each, one to a
-// scheduler, 59 with eight; 45.5 when the copies were no longer 3,072 of 16 bytes, whose issue took 850 of a chunk's 3,100 cycles.)
+// scheduler, 59 with eight; 45.5 when the copies were no longer 3,072 of 16 bytes, whose issue took 850 of a chunk's 3,100 cycles.  Two and
+// three chunks, where the ring's start weighs most: a layer of 128 tokens 85.3 -> 79.1 us, of 192 92.4 -> 86.3.)
 constexpr int kCarryPlane = kChunk * kDim;
 constexpr int kCarryStage = 2 * kParts * kCarryPlane, kCarryStages = 3;                    // y, keys
 constexpr int kCarryBytes = (kCarryStages * kCarryStage + 2 * kParts * kNarrowPlane) * 2;  // and S, u

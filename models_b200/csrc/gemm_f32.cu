@@ -25,8 +25,8 @@
 //
 // Both operands are split times 2^24, and the sums divided by 2^48: the parts of every float are whole then, also where it is so small that
 // bfloat16 would have no bits left for its third.  Sums that are not finite -- a float was not, or was above 2^103, or the result is above
-// 2^79 -- are computed anew from the floats, in the order of K: no other row of A or W sees such a float.  (That results are judged, and not
-// operands, gives every kernel below the same judgement.)
+// 2^79 -- are computed anew from the floats, in the order of K: no other row of A or W sees such a float.  (Results decide, and not
+// operands, so that every kernel below decides alike.)
 #include "tcgen05.cuh"
 #include "float_parts.cuh"
 

@@ -469,8 +469,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 tmem_load_wait();
                                 // The gated epilogue must not take longer than a tile's products (16,400 cycles at K = 2,048).
                                 // With a division per pair it took 21,600 (left out, 2,048 rows and 16,384 weight rows ran in 82 us
-                                // instead of 100).  A prompt step of 2,048 tokens through 16 layers 4,553 -> 4,309 us, five prompts of
-                                // 467 tokens through 4 layers 501 -> 405 us, every bit as before.
+                                // instead of 100).  Without: 2,048 rows 99.4 -> 94.8 us, 512 rows 34.3 -> 28.6, 437 rows 34.2 -> 28.1, every
+                                // bit as before (gate_pairs.cuh); with the bare reciprocal 93.8, 28.2 and 27.7.
                                 gate_pairs(args.activation, v, u, args.clamp);
                             } else {
                                 tmem_load_32_issue(taddr + c + 32 * part, v);

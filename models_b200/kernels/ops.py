@@ -1749,7 +1749,7 @@ def prefill_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, row_invariant: bool = True, weights_ready: bool = False) -> torch.Tensor:
     """a [m, k] . w[n, k]^T in 32 bits: every bit of the floats is multiplied, and a row's result depends on
-    nothing but that row (`row_invariant` or not).  `weights_ready`: no kernel still queued writes `w` (a loaded
+    nothing but that row (`row_invariant` once chose between two orders of the sums; calls may still give it).  `weights_ready`: no kernel still queued writes `w` (a loaded
     weight), so that it may be read while the kernels before this product still run."""
     _cuda(a, w)
     if a.dtype != torch.float32 or w.dtype != torch.float32:

@@ -74,9 +74,12 @@ def test_gemm_f32(cuda_device, m, n, k):
     g = torch.Generator().manual_seed(2)
     a, w = torch.randn(m, k, generator=g), torch.randn(n, k, generator=g)
     expected = (a.double() @ w.double().t())
+    outs = []
     for invariant in (True, False):
         out = ops.gemm_f32(a.cuda(), w.cuda(), row_invariant=invariant)
         close(out, expected, torch.float32, scale=float(expected.abs().max()) * 4)
+        outs.append(out)
+    assert torch.equal(*outs)  # every product is row-invariant
     # a row's result does not depend on the other rows of the call
     alone = ops.gemm_f32(a[:1].cuda(), w.cuda(), row_invariant=True)
     together = ops.gemm_f32(a.cuda(), w.cuda(), row_invariant=True)
