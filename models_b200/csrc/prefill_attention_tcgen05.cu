@@ -5,9 +5,10 @@
 //
 // -DMB_SHAPED=1 (paged, float weights): scores and results with the variations of gated_attention.cu -- a factor per head, a bound
 // cap * tanh(score / cap), one more term of score 0 in the denominator, a result whose pairs (2m, 2m + 1) are turned back by the
-// query's position.  The bound costs a thread two more special-function results per score (tanh(x) = 1 - 2 / (1 + e^(2x))), and
-// that unit is what bounds it: 2,048 tokens, 16 heads of 64 and 128, 64 us under a profiler (166 in
-// gated_attention_tc.cu).
+// query's position.  Where a warp's scores of a page are small, tanh is a polynomial and the page needs no maximum (kTanhReach); elsewhere the
+// bound costs a thread two more special-function results per score (tanh(x) = 1 - 2 / (1 + e^(2x))).  2,048 tokens, 16 heads of 64 and 128:
+// 46 us (63 by the general form alone, with a result's tables read along its row), bound by the longest blocks' pages one after another
+// (about 2,100 cycles each, 1,500 of them a warp's own arithmetic).
 //
 // MB_CONTIGUOUS: a prompt that starts its sequence brings every key it sees itself, so keys and values are read from the step's own
 // rows ([tokens][heads * size]) instead of the cache's pages.  Key and value heads may then be padded to these sizes with zero
@@ -48,6 +49,7 @@
 // meet at the final barrier, tensor memory is freed and the kernel returns.
 // mb_prefill_attention_tc_status() reads the record.
 #include "tcgen05.cuh"
+#include "gate_pairs.cuh"
 
 #include <math_constants.h>
 
@@ -101,7 +103,14 @@ constexpr int kScoreColumns = 64;
 constexpr int kTmemColumns = 256;  // two score buffers and the output: 2 * 64 + VD
 static_assert(2 * kScoreColumns + VD <= kTmemColumns, "tensor memory budget");
 constexpr float kSlack = 8.0f;     // how far (in the exponent) the maximum may run ahead of the base
-constexpr size_t kSmemBytes = (size_t)kQBytes + (size_t)kStages * (kKeyTileBytes + kValueTileBytes) + 1024;
+constexpr int kTileBytes = kQBytes + kStages * (kKeyTileBytes + kValueTileBytes);
+// Where gates of elements (boxes of 64 columns) and then the results lie: gates in the queries' place where they fit, results behind them, over
+// tiles that have been read.
+constexpr int kGateBytes = kContiguous ? kValueBoxes * kQBoxBytes : 0, kResultBytes = kFloatWeights ? kQRows * VD * 4 : 0;
+constexpr int kGatesAt = kGateBytes <= kQBytes ? 0 : kTileBytes, kResultsAt = kGatesAt == 0 ? kGateBytes : 0;
+static_assert(kGatesAt == 0 || kResultsAt + kResultBytes <= kGatesAt, "results and gates do not meet");
+constexpr int larger(int a, int b) { return a > b ? a : b; }
+constexpr size_t kSmemBytes = larger(larger(kTileBytes, kGatesAt + kGateBytes), kResultsAt + kResultBytes) + 1024;
 
 constexpr uint32_t kScoreInstruction = instruction_descriptor(kQRows, kKeys);
 constexpr uint32_t kOutputInstruction = instruction_descriptor(kQRows, VD) | (1u << 16);  // B is MN-major
@@ -156,6 +165,11 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -206,6 +220,12 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
+__device__ __forceinline__ float max3_magnitude(float a, float b, float c) { return max3(fabsf(a), fabsf(b), fabsf(c)); }
+
+// Of a bound cap * tanh(z / cap): up to which |z / cap| a polynomial stands for it, and up to which |score * log2 e| a page needs no maximum.
+// (Unit-normed queries and keys of 64 numbers have |score| <= 8 times the head's factor: within either at a bound of 50.)
+constexpr float kTanhReach = 0.5f, kFlatReach = 16.0f;
+
 // tcgen05.mma with the 128 x 16 A operand in tensor memory (lane = row, two bfloat16 per 32-bit column)
 __device__ __forceinline__ void umma_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t instruction, uint32_t accumulate) {
     asm volatile(
@@ -214,6 +234,26 @@ __device__ __forceinline__ void umma_a_tmem(uint32_t tmem_d, uint32_t tmem_a, ui
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(instruction), "r"(accumulate)
         : "memory");
+}
+
+// v[i] *= sigmoid(z[i]), by reciprocals that are rounded as divisions are (see minus_quotients); with one z beyond them by divisions.  (One
+// branch for all, so that they are worked on side by side: four at a time were 365 cycles of latency.)
+template <int kRows>
+__device__ __forceinline__ void gate_by_sigmoids(float (&v)[kRows][4], const float (&z)[kRows][4]) {
+    float lowest = z[0][0];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) lowest = min_of(min_of(lowest, z[i][0], z[i][1]), z[i][2], z[i][3]);
+    if (lowest >= -40.0f) {
+#pragma unroll
+        for (int i = 0; i < 2 * kRows; ++i) {
+            const int r = i / 2, c = i % 2 * 2;
+            const uint64_t q = minus_quotients(0x3f8000003f800000ull, 1.0f + expf(-z[r][c]), 1.0f + expf(-z[r][c + 1]));  // 1, 1
+            v[r][c] *= -low_of(q), v[r][c + 1] *= -high_of(q);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4 * kRows; ++i) v[i / 4][i % 4] *= 1.0f / (1.0f + expf(-z[i / 4][i % 4]));
+    }
 }
 
 struct AttentionArgs {
@@ -241,11 +281,11 @@ struct AttentionArgs {
 };
 
 // roles in the status record: 1 TMA (stage free), 2 MMA (queries), 3 MMA (keys), 4 MMA (probabilities),
-// 5 softmax (scores), 6 softmax (output of a page)
+// 5 softmax (scores), 6 softmax (output of a page), 7 TMA (last scores, for the gates), 8 softmax (gates)
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                  const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_q_turned,
-                                 const __grid_constant__ CUtensorMap map_k_turned, const AttentionArgs args) {
+                                 const __grid_constant__ CUtensorMap map_k_turned, const __grid_constant__ CUtensorMap map_gate, const AttentionArgs args) {
     // blocks start in the order of their index: all heads of the query tile with the most keys first, then
     // the next tile, so that the long blocks are under way early and the short ones fill the end
     const int seq = blockIdx.z, head = blockIdx.x;
@@ -256,7 +296,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t barriers[4 * kStages + 7];
+    __shared__ __align__(8) uint64_t barriers[4 * kStages + 8];
     __shared__ uint32_t tmem_base_slot;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t q_smem = smem_u32(smem);
@@ -269,6 +309,8 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     const uint32_t s_full = smem_u32(&barriers[4 * kStages + 1]);  // two
     const uint32_t p_full = smem_u32(&barriers[4 * kStages + 3]);  // two
     const uint32_t o_full = smem_u32(&barriers[4 * kStages + 5]);  // two
+    const uint32_t gate_full = smem_u32(&barriers[4 * kStages + 7]);
+    const bool gated = kContiguous && args.gate_element != 0;
 
     const int valid = min(kQRows, q_len - t0);
     const int kv_len = args.kv_lens[seq];
@@ -290,6 +332,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             mbar_init(v_empty + 8 * s, 1);
         }
         mbar_init(q_full, 1);
+        mbar_init(gate_full, 1);
         for (int b = 0; b < 2; ++b) {
             mbar_init(s_full + 8 * b, 1);
             mbar_init(p_full + 8 * b, kSoftmaxWarps);  // one arrival per softmax warp
@@ -320,24 +363,40 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             for (int b = kKeyBoxes; b < kBoxes; ++b)
                 tma_load_2d(q_smem + b * kQBoxBytes, &map_q_turned, head * RD + (b - kKeyBoxes) * 64, q_begin + t0, q_full);
             const int* table = args.block_table + (size_t)seq * args.max_blocks;
-            for (int t = 0; t < pages; ++t) {
-                const int stage = t % kStages;
-                const uint32_t free_parity = ((t / kStages) & 1) ^ 1;
-                const int row = kContiguous ? (args.key_rows > 0 ? seq * args.key_rows : q_begin) + (t_begin - t_first + t) * kKeys : (table[t_begin + t] * args.kv_heads + kv_head) * kKeys;
-                const int key_column = kContiguous ? kv_head * KD : 0, value_column = kContiguous ? kv_head * VD : 0;
-                if (!mbar_wait(k_empty + 8 * stage, free_parity, 1)) break;
+            auto row_of = [&](int t) {
+                return kContiguous ? (args.key_rows > 0 ? seq * args.key_rows : q_begin) + (t_begin - t_first + t) * kKeys : (table[t_begin + t] * args.kv_heads + kv_head) * kKeys;
+            };
+            auto bring_keys = [&](int t) {
+                const int stage = t % kStages, row = row_of(t), column = kContiguous ? kv_head * KD : 0;
+                if (!mbar_wait(k_empty + 8 * stage, ((t / kStages) & 1) ^ 1, 1)) return false;
                 mbar_expect_tx(k_full + 8 * stage, kKeyTileBytes);
 #pragma unroll
                 for (int b = 0; b < kKeyBoxes; ++b)
-                    tma_load_2d(k_smem + stage * kKeyTileBytes + b * kKVBoxBytes, &map_k, key_column + b * 64, row, k_full + 8 * stage);
+                    tma_load_2d(k_smem + stage * kKeyTileBytes + b * kKVBoxBytes, &map_k, column + b * 64, row, k_full + 8 * stage);
 #pragma unroll
                 for (int b = kKeyBoxes; b < kBoxes; ++b)
                     tma_load_2d(k_smem + stage * kKeyTileBytes + b * kKVBoxBytes, &map_k_turned, (b - kKeyBoxes) * 64, row, k_full + 8 * stage);
-                if (!mbar_wait(v_empty + 8 * stage, free_parity, 1)) break;
+                return true;
+            };
+            // A key tile is free as soon as its scores are there, a value tile a softmax and a product later: keys are asked for a ring's
+            // length ahead of the values, not behind the values of the page before.
+            constexpr int kAhead = kStages - 1;
+            bool ok = true;
+            for (int t = 0; t < min(kAhead, pages) && ok; ++t) ok = bring_keys(t);
+            for (int t = 0; t < pages && ok; ++t) {
+                if (t + kAhead < pages && !(ok = bring_keys(t + kAhead))) break;
+                const int stage = t % kStages, row = row_of(t), column = kContiguous ? kv_head * VD : 0;
+                if (!(ok = mbar_wait(v_empty + 8 * stage, ((t / kStages) & 1) ^ 1, 1))) break;
                 mbar_expect_tx(v_full + 8 * stage, kValueTileBytes);
 #pragma unroll
                 for (int b = 0; b < kValueBoxes; ++b)
-                    tma_load_2d(v_smem + stage * kValueTileBytes + b * kKVBoxBytes, &map_v, value_column + b * 64, row, v_full + 8 * stage);
+                    tma_load_2d(v_smem + stage * kValueTileBytes + b * kKVBoxBytes, &map_v, column + b * 64, row, v_full + 8 * stage);
+            }
+            // gates of elements take the queries' place as soon as the last scores are there
+            if (gated && ok && mbar_wait(s_full + 8 * ((pages - 1) & 1), ((pages - 1) >> 1) & 1, 7)) {
+                mbar_expect_tx(gate_full, kGateBytes);
+#pragma unroll
+                for (int b = 0; b < kValueBoxes; ++b) tma_load_2d(q_smem + kGatesAt + b * kQBoxBytes, &map_gate, head * args.value_columns + b * 64, q_begin + t0, gate_full);
             }
         }
     } else if (warp == 1) {
@@ -396,6 +455,11 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         const float cap = kShaped ? args.softcap : 0.0f, cap_exponent = cap > 0.0f ? shaped_scale * (2.0f * 1.4426950408889634f / cap) : 0.0f;
         const float scale_log2 = (kShaped ? 1.0f : args.scale) * 1.4426950408889634f;
         const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
+        // the polynomial for small scores (see kTanhReach)
+        const float per_cap = cap > 0.0f ? shaped_scale / cap : 0.0f, flat_reach = fminf(kTanhReach * cap, kFlatReach / 1.4426950408889634f) / fabsf(shaped_scale);
+        auto both = [](float v) { return pack_f32x2(v, v); };
+        const uint64_t per_cap2 = both(per_cap), cap_log2 = both(cap * 1.4426950408889634f), one = both(1.0f);
+        const uint64_t tanh_c0 = both(-0.33333148f), tanh_c1 = both(0.13325987f), tanh_c2 = both(-0.053052945f), tanh_c3 = both(0.017256979f);
         // `base` is the score the exponents are taken against.  It follows the running maximum lazily:
         // it moves (and the output so far is rescaled) only when the maximum has grown by more than
         // kSlack in the exponent, so most pages cost no pass over the output.  Until then the
@@ -413,57 +477,92 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 #pragma unroll
             for (int c = 0; c < kCols; c += 32) tmem_load_32_raw(my_scores + c, &s[c]);
             tmem_wait_loads();
-            if (kShaped) {
-                if (cap > 0.0f) {
-#pragma unroll
-                    for (int i = 0; i < kCols; ++i)  // cap * tanh(z / cap)
-                        s[i] = __float_as_uint(cap - __fdividef(2.0f * cap, 1.0f + fast_exp2(__uint_as_float(s[i]) * cap_exponent)));
-                } else {
-#pragma unroll
-                    for (int i = 0; i < kCols; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) * shaped_scale);
-                }
-            }
             const int key_base = (t_begin + t) * kKeys;
-            if (!(key_base + kCols - 1 <= row_pos && key_base >= row_first)) {  // not the whole page is visible to this row
+            auto hide = [&] {
+                if (key_base + kCols - 1 <= row_pos && key_base >= row_first) return;  // the whole page is visible to this row
 #pragma unroll
                 for (int i = 0; i < kCols; ++i) {
                     const int key = key_base + i;
                     if (!(key <= row_pos && key >= row_first)) s[i] = __float_as_uint(-CUDART_INF_F);
                 }
-            }
-            float part[8];  // eight chains, two more scores a step
-#pragma unroll
-            for (int i = 0; i < 8; ++i) part[i] = fmaxf(__uint_as_float(s[i]), __uint_as_float(s[8 + i]));
-#pragma unroll
-            for (int i = 16; i < kCols; i += 16)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) part[j] = max3(part[j], __uint_as_float(s[i + j]), __uint_as_float(s[i + 8 + j]));
-            const float page_max = max3(max3(part[0], part[1], part[2]), max3(part[3], part[4], part[5]), fmaxf(part[6], part[7]));
-            // scores stay raw; the scale (times log2 e) is folded into the exponent: 2^(s*c - base*c)
+            };
             float factor = 1.0f;
-            if (base == -CUDART_INF_F) {
-                base = page_max;  // nothing accumulated so far (or still nothing visible)
-            } else if ((page_max - base) * scale_log2 > kSlack) {
-                factor = fast_exp2((base - page_max) * scale_log2);
-                base = page_max;
+            bool flat = false;
+            if (kShaped && cap > 0.0f) {
+                float most[4];  // magnitudes: four chains
+#pragma unroll
+                for (int i = 0; i < 4; ++i) most[i] = max3_magnitude(__uint_as_float(s[i]), __uint_as_float(s[4 + i]), __uint_as_float(s[8 + i]));
+#pragma unroll
+                for (int i = 12; i + 8 <= kCols; i += 8)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) most[j] = max3_magnitude(most[j], __uint_as_float(s[i + j]), __uint_as_float(s[i + 4 + j]));
+#pragma unroll
+                for (int i = kCols - 4; i < kCols; ++i) most[i & 3] = fmaxf(most[i & 3], fabsf(__uint_as_float(s[i])));
+                const bool mine = max3(fmaxf(most[0], most[1]), most[2], most[3]) <= flat_reach && (base == -CUDART_INF_F || fabsf(base) <= kFlatReach / 1.4426950408889634f);
+                flat = __all_sync(0xffffffffu, mine || row_pos < 0);
             }
-            run_sum *= factor;
-            // a row that has seen nothing yet keeps -inf; subtract 0 then so that the exponent is -inf, not NaN
-            const float offset = base == -CUDART_INF_F ? 0.0f : fmaf(-base, scale_log2, kTruncationLift);
-            const uint64_t offset2 = pack_f32x2(offset, offset);
+            if (flat) {
+                // z (1 + u (c0 + u (c1 + ...))), u = (z / cap)^2 (relative error 1.5e-8), log2 e and the base: eight instructions for two scores,
+                // where the general form waits for three special-function results each
+                if (base == -CUDART_INF_F && key_base <= row_pos && key_base + kCols > row_first) base = 0.0f;
+                const float offset = base == -CUDART_INF_F ? 0.0f : -base * scale_log2;
+                const uint64_t offset2 = pack_f32x2(offset, offset);
+#pragma unroll
+                for (int i = 0; i < kCols; i += 2) {
+                    const uint64_t z = mul_f32x2(pack_f32x2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), per_cap2), u = mul_f32x2(z, z);
+                    const uint64_t p = fma_f32x2(u, fma_f32x2(u, fma_f32x2(u, fma_f32x2(u, tanh_c3, tanh_c2), tanh_c1), tanh_c0), one);
+                    const uint64_t x = fma_f32x2(mul_f32x2(z, cap_log2), p, offset2);
+                    s[i] = (uint32_t)x, s[i + 1] = (uint32_t)(x >> 32);
+                }
+                hide();
+            } else {
+                if (kShaped) {
+                    if (cap > 0.0f) {
+#pragma unroll
+                        for (int i = 0; i < kCols; ++i)  // cap * tanh(z / cap)
+                            s[i] = __float_as_uint(cap - __fdividef(2.0f * cap, 1.0f + fast_exp2(__uint_as_float(s[i]) * cap_exponent)));
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < kCols; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) * shaped_scale);
+                    }
+                }
+                hide();
+                float part[8];  // eight chains, two more scores a step
+#pragma unroll
+                for (int i = 0; i < 8; ++i) part[i] = fmaxf(__uint_as_float(s[i]), __uint_as_float(s[8 + i]));
+#pragma unroll
+                for (int i = 16; i < kCols; i += 16)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) part[j] = max3(part[j], __uint_as_float(s[i + j]), __uint_as_float(s[i + 8 + j]));
+                const float page_max = max3(max3(part[0], part[1], part[2]), max3(part[3], part[4], part[5]), fmaxf(part[6], part[7]));
+                // scores stay raw; the scale (times log2 e) is folded into the exponent: 2^(s*c - base*c)
+                if (base == -CUDART_INF_F) {
+                    base = page_max;  // nothing accumulated so far (or still nothing visible)
+                } else if ((page_max - base) * scale_log2 > kSlack) {
+                    factor = fast_exp2((base - page_max) * scale_log2);
+                    base = page_max;
+                }
+                run_sum *= factor;
+                // a row that has seen nothing yet keeps -inf; subtract 0 then so that the exponent is -inf, not NaN
+                const float offset = base == -CUDART_INF_F ? 0.0f : fmaf(-base, scale_log2, kTruncationLift);
+                const uint64_t offset2 = pack_f32x2(offset, offset);
+#pragma unroll
+                for (int i = 0; i < kCols; i += 2) {
+                    const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), scale2, offset2);
+                    s[i] = (uint32_t)x, s[i + 1] = (uint32_t)(x >> 32);
+                }
+            }
             uint64_t sums[4] = {0ull, 0ull, 0ull, 0ull};  // eight partial sums, two per register pair
             uint32_t packed[kCols / 2], rest[kFloatWeights ? kCols / 2 : 1];
 #pragma unroll
             for (int c = 0; c < kCols / 8; ++c) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(s[c * 8 + 2 * i]), __uint_as_float(s[c * 8 + 2 * i + 1])), scale2, offset2);
+                    const float x0 = __uint_as_float(s[c * 8 + 2 * i]), x1 = __uint_as_float(s[c * 8 + 2 * i + 1]);
                     float e0, e1;
                     if (i < kSoftPairs) {
-                        soft_exp2_x2(x2, e0, e1);
+                        soft_exp2_x2(pack_f32x2(x0, x1), e0, e1);
                     } else {
-                        float x0, x1;
-                        unpack_f32x2(x2, x0, x1);
                         e0 = fast_exp2(x0);
                         e1 = fast_exp2(x1);
                     }
@@ -515,8 +614,22 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full + 8 * (t & 1));
         }
+        // A warp's rows on their way out (see below), so many at a time; the first ones' tables are asked for while the last products are under way.
+        constexpr int kFours = VD / 4, kRowsAtOnce = 32 / kFours, kBatch = kContiguous ? 2 : kShaped ? 16 : 8;
+        const int four = lane % kFours, first = quarter * 32 + lane / kFours, last = min(quarter * 32 + 32, valid);
+        const size_t token = q_begin + t0, column = (size_t)head * args.value_columns + 4 * four;
+        const bool turns = kShaped && args.turn_cos != nullptr, mine_stored = 4 * four < args.value_columns && first < last;
+        float2 cs[kShaped ? kBatch : 1], sn[kShaped ? kBatch : 1];
+        auto ask = [&](int from) {
+#pragma unroll
+            for (int i = 0; i < kBatch && kShaped; ++i) {
+                const size_t turn = (size_t)(pos0 + min(from + i * kRowsAtOnce, last - 1)) * (VD / 2) + 2 * four;
+                cs[i] = __ldg(reinterpret_cast<const float2*>(args.turn_cos + turn)), sn[i] = __ldg(reinterpret_cast<const float2*>(args.turn_sin + turn));
+            }
+        };
+        if (turns && mine_stored) ask(first);
         if (ok) {
-            ok = mbar_wait(o_full + 8 * ((pages - 1) & 1), ((pages - 1) >> 1) & 1, 6);
+            ok = mbar_wait(o_full + 8 * ((pages - 1) & 1), ((pages - 1) >> 1) & 1, 6) && (!gated || mbar_wait(gate_full, 0, 8));
             ok = __all_sync(0xffffffffu, ok);
         }
         if (ok) {
@@ -525,38 +638,80 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             float inv = exp2f(kTruncationLift) / run_sum;  // the sum holds the lifted probabilities, the products their truncations
             if (kFloatWeights && args.gate != nullptr && !args.gate_element && row < valid)
                 inv *= 1.0f / (1.0f + expf(-__bfloat162float(args.gate[(size_t)(q_begin + t0 + row) * args.gate_stride + head])));
-            const int value_columns = kFloatWeights ? args.value_columns : VD;
-            bf16* dst = args.out + (size_t)(q_begin + t0 + row) * args.out_row_stride + (size_t)head * value_columns;
+            if (kFloatWeights) {
+                // Through shared memory (every product has read its tiles): a thread brings its row, and then the warp's lanes lie along the
+                // columns of its rows, one after another, so that tables and results are whole lines of memory; gates are there by then.  (A
+                // thread by itself along its row waited for its loads time and again: 26,000 cycles a block with gates of elements, 9,300
+                // with tables.  1,531 tokens on top of 700 cached positions each, 16 heads of 64 + 64 and 128: 48.3 -> 39.5 us.)
+                float4* rows = reinterpret_cast<float4*>(smem + kResultsAt);  // [128][VD], the fours of a row turned by it
 #pragma unroll
-            for (int c = 0; c < VD; c += 32) {
-                uint32_t r[32];
-                tmem_load_32_raw(my_output + c, r);
-                tmem_wait_loads();
-                if (row < valid) {
+                for (int c = 0; c < VD; c += 32) {
+                    uint32_t r[32];
+                    tmem_load_32_raw(my_output + c, r);
+                    tmem_wait_loads();
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        if (kFloatWeights && c + i >= value_columns) continue;
-                        float piece[8];
+                    for (int i = 0; i < 32; i += 4)
+                        rows[row * kFours + ((c + i) / 4 ^ (row & 7))] = make_float4(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv,
+                                                                                   __uint_as_float(r[i + 2]) * inv, __uint_as_float(r[i + 3]) * inv);
+                }
+                __syncwarp();
+                auto store = [&](int at, const float (&v)[4]) {
+                    const __nv_bfloat162 low = __floats2bfloat162_rn(v[0], v[1]), high = __floats2bfloat162_rn(v[2], v[3]);
+                    *reinterpret_cast<uint2*>(args.out + (token + at) * args.out_row_stride + column) =
+                        make_uint2(*reinterpret_cast<const uint32_t*>(&low), *reinterpret_cast<const uint32_t*>(&high));
+                };
+                if (mine_stored && gated) {
+#pragma unroll 1
+                    for (int at0 = first; at0 < last; at0 += kBatch * kRowsAtOnce) {
+                        float v[kBatch][4], z[kBatch][4];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) piece[j] = __uint_as_float(r[i + j]) * inv;
-                        if (kContiguous && args.gate_element) {
-                            float z[8];
-                            load8(args.gate + (size_t)(q_begin + t0 + row) * args.gate_stride + (size_t)head * value_columns + c + i, z);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) piece[j] *= 1.0f / (1.0f + expf(-z[j]));
+                        for (int i = 0; i < kBatch; ++i) {
+                            const int at = min(at0 + i * kRowsAtOnce, last - 1);
+                            *reinterpret_cast<float4*>(v[i]) = rows[at * kFours + (four ^ (at & 7))];
+                            const uint2 raw = *reinterpret_cast<const uint2*>(  // (in the 128-byte swizzle, as TMA leaves it)
+                                smem + kGatesAt + four / 16 * kQBoxBytes + at * 128 + ((four % 16 / 2 ^ (at & 7)) << 4) + four % 2 * 8);
+                            z[i][0] = __uint_as_float(raw.x << 16), z[i][1] = __uint_as_float(raw.x & 0xffff0000u);
+                            z[i][2] = __uint_as_float(raw.y << 16), z[i][3] = __uint_as_float(raw.y & 0xffff0000u);
                         }
-                        if (kShaped && args.turn_cos != nullptr) {  // back by the query's position
-                            const size_t at = (size_t)row_pos * (VD / 2) + (c + i) / 2;
-                            const float4 cs = *reinterpret_cast<const float4*>(args.turn_cos + at), sn = *reinterpret_cast<const float4*>(args.turn_sin + at);
-                            const float cosines[4] = {cs.x, cs.y, cs.z, cs.w}, sines[4] = {sn.x, sn.y, sn.z, sn.w};
+                        gate_by_sigmoids(v, z);
 #pragma unroll
-                            for (int m = 0; m < 4; ++m) {
-                                const float x = piece[2 * m], y = piece[2 * m + 1];
-                                piece[2 * m] = x * cosines[m] + y * sines[m];
-                                piece[2 * m + 1] = y * cosines[m] - x * sines[m];
+                        for (int i = 0; i < kBatch; ++i)
+                            if (at0 + i * kRowsAtOnce < last) store(at0 + i * kRowsAtOnce, v[i]);
+                    }
+                } else if (mine_stored) {
+#pragma unroll 1
+                    for (int at0 = first; at0 < last; at0 += kBatch * kRowsAtOnce) {
+                        if (turns && at0 > first) ask(at0);
+#pragma unroll
+                        for (int i = 0; i < kBatch; ++i) {
+                            const int at = at0 + i * kRowsAtOnce;
+                            if (at >= last) break;
+                            const float4 r = rows[at * kFours + (four ^ (at & 7))];
+                            float v[4] = {r.x, r.y, r.z, r.w};
+                            if (turns) {  // back by the query's position
+                                const int m = kShaped ? i : 0;
+                                v[0] = r.x * cs[m].x + r.y * sn[m].x, v[1] = r.y * cs[m].x - r.x * sn[m].x;
+                                v[2] = r.z * cs[m].y + r.w * sn[m].y, v[3] = r.w * cs[m].y - r.z * sn[m].y;
                             }
+                            store(at, v);
                         }
-                        store8(dst + c + i, piece);
+                    }
+                }
+            } else {
+                bf16* dst = args.out + (size_t)(q_begin + t0 + row) * args.out_row_stride + (size_t)head * VD;
+#pragma unroll
+                for (int c = 0; c < VD; c += 32) {
+                    uint32_t r[32];
+                    tmem_load_32_raw(my_output + c, r);
+                    tmem_wait_loads();
+                    if (row < valid) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 8) {
+                            float piece[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) piece[j] = __uint_as_float(r[i + j]) * inv;
+                            store8(dst + c + i, piece);
+                        }
                     }
                 }
             }
@@ -577,7 +732,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 using namespace mb;
 
 static int launch_prefill(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_q_turned,
-                          const CUtensorMap& map_k_turned, const AttentionArgs& args, int sequences, int max_q_len, cudaStream_t stream) {
+                          const CUtensorMap& map_k_turned, const CUtensorMap& map_gate, const AttentionArgs& args, int sequences, int max_q_len, cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
         cudaError_t status = cudaFuncSetAttribute(prefill_attention_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
@@ -587,7 +742,7 @@ static int launch_prefill(const CUtensorMap& map_q, const CUtensorMap& map_k, co
     }
     const dim3 grid(args.heads, (max_q_len + kQRows - 1) / kQRows, sequences);
     return launch_dependent("prefill_attention_tcgen05", prefill_attention_tcgen05_kernel, grid, dim3(kThreads), kSmemBytes, stream,
-                            true, map_q, map_k, map_v, map_q_turned, map_k_turned, args);
+                            true, map_q, map_k, map_v, map_q_turned, map_k_turned, map_gate, args);
 }
 
 static int check_prefill(const void* q, int q_row_stride, const void* out, int out_row_stride, int sequences, int max_q_len, int heads, int kv_heads) {
@@ -630,7 +785,7 @@ MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int 
     if (int status = make_map(&map_v, v_pool, pool_pages * kv_heads * kKeys, VD, VD, kKeys)) return status;
     const AttentionArgs args{(bf16*)out, out_row_stride, block_table, max_blocks, cu_q, kv_lens, heads, kv_heads, window, scale, KD, VD, nullptr, 0, 0, 0, 0,
                              head_scale, softcap, sink, turn_cos, turn_sin};
-    return launch_prefill(map_q, map_k, map_v, map_q, map_k, args, sequences, max_q_len, stream);
+    return launch_prefill(map_q, map_k, map_v, map_q, map_k, map_q, args, sequences, max_q_len, stream);
 }
 #else
 // Prompts that start their sequences: kv_lens are the lengths of the prompts themselves.  q: bfloat16 rows of total_rows tokens, head h's
@@ -669,7 +824,10 @@ MB_EXPORT int mb_prompt_attention_tcgen05(const void* q, int q_row_stride, int q
     }
     const AttentionArgs args{(bf16*)out, out_row_stride, nullptr, 0, cu_q, kv_lens, heads, kv_heads, window, scale, q_head_columns, value_columns,
                              (const bf16*)gate, gate_stride, gate_element, key_rows, key_window, nullptr, 0.0f, 0, nullptr, nullptr};
-    return launch_prefill(map_q, map_k, map_v, map_q_turned, map_k_turned, args, sequences, max_q_len, stream);
+    CUtensorMap map_gate = map_q;
+    if (gate_element)
+        if (int status = make_map(&map_gate, gate, total_rows, heads * value_columns, gate_stride, kQRows)) return status;
+    return launch_prefill(map_q, map_k, map_v, map_q_turned, map_k_turned, map_gate, args, sequences, max_q_len, stream);
 }
 #endif
 

@@ -1569,6 +1569,39 @@ def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
     assert float((outs[0] - outs[1]).norm()) <= 2.0 ** -9 * float(outs[1].norm())
 
 
+@pytest.mark.parametrize("cap", [50.0, 8.0])
+@pytest.mark.parametrize("size", [0.3, 1.0, 2.2, 6.0])
+def test_bounded_scores_small_and_large(cuda_device, cap, size):
+    """Scores from well within the polynomial's reach to far beyond it, in the same rows and in rows of their own, against 64 bits: the
+    weights' two bfloat16 parts (2^-16), the score's float arithmetic and the result's rounding (eight bits: up to 2^-8 of it)."""
+    from models_b200.kernels import ops
+
+    heads, dim, vdim, lens = 2, 64, 128, [200, 65]
+    g = torch.Generator().manual_seed(int(cap))
+    k_pool, v_pool = (torch.randn(7, 1, 64, d, generator=g).bfloat16() for d in (dim, vdim))
+    k_pool[2] *= 5.0  # positions 64 to 127 of the first sequence
+    table = torch.tensor([[1, 2, 3, 4], [5, 6, 0, 0]], dtype=torch.int32)
+    T = sum(lens)
+    q = (torch.randn(T, heads * dim, generator=g) * size).bfloat16()
+    q[100:140] *= 0.05
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()  # noqa: E731
+    out = torch.zeros(T, heads * vdim, dtype=torch.bfloat16, device=cuda_device)
+    ops.gated_attention(q.cuda(), out, k_pool.cuda(), v_pool.cuda(), table.cuda(), i32([0, 200, 265]), i32(lens), 200, heads, 1, dim, vdim, "softmax",
+                        0.125, softcap=cap, sink=True)
+    at = 0
+    for i, n in enumerate(lens):
+        k, v = (torch.cat([p[t, 0] for t in table[i]])[:n].double() for p in (k_pool, v_pool))
+        for h in range(heads):
+            s = cap * torch.tanh(q[at:at + n, h * dim:(h + 1) * dim].double() @ k.t() * 0.125 / cap)
+            s = s.masked_fill(torch.ones(n, n, dtype=torch.bool).triu(1), -math.inf)
+            top = s.amax(1, keepdim=True).clamp(min=0)
+            w = torch.exp(s - top)
+            want = w / (w.sum(1, keepdim=True) + torch.exp(-top)) @ v
+            error = (out[at:at + n, h * vdim:(h + 1) * vdim].double().cpu() - want).abs()
+            assert bool((error <= 2.0 ** -8 * want.abs() + 2.0 ** -14 * v.abs().max()).all())
+        at += n
+
+
 @pytest.mark.parametrize("sequences,tokens,most,tcgen05", [(8, 40, 40, True), (8, 64, 512, True), (16, 40, 640, False)])
 def test_shaped_scores_of_mostly_empty_tiles(cuda_device, sequences, tokens, most, tcgen05):
     """A step that says that one sequence may hold all of its tokens (a captured one does) takes the mma.sync kernel where most tiles would be

@@ -370,6 +370,38 @@ def test_prompt_attention_on_its_own_rows(cuda_device, heads, dim, rot, value_di
     assert bool((out[T:] == 7).all()) and bool((out[:, heads * value_dim:] == 7).all())
 
 
+@pytest.mark.parametrize("heads,dim,rot,value_dim", [(3, 64, 64, 128), (2, 64, 0, 128), (2, 8, 8, 40), (1, 64, 0, 64), (2, 128, 128, 72)])
+def test_prompt_attention_with_gates_of_elements(cuda_device, heads, dim, rot, value_dim):
+    """Gates of every size, some beyond e^40 or not numbers, beside queries' tiles of one to 128 rows: what the result without gates is, times
+    the sigmoids in 64 bits, within two roundings to bfloat16 (the ungated result's and the result's: eight bits, up to 2^-8 of it each) and
+    the float arithmetic."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(dim + rot + value_dim)
+    whole = lambda n: -(-n // 64) * 64  # noqa: E731
+    lengths = [70, 1, 300, 128, 33]
+    T, KD, RD, VD = sum(lengths), whole(dim), whole(rot), whole(value_dim)
+    normal = lambda *shape: torch.randn(*shape, generator=g).bfloat16().to(cuda_device)  # noqa: E731
+    q, q_tail, tail = normal(T, heads * KD), normal(T, heads * RD) if rot else None, normal(T, RD) if rot else None
+    kv = normal(T, heads * (KD + VD))
+    gate = (torch.randn(T, heads * value_dim + 8, generator=g) * 12).bfloat16().to(cuda_device)[:, :heads * value_dim]
+    gate[5, 3], gate[6, 1], gate[7, 0], gate[8, 2], gate[40, 4] = -60.0, -3e38, 3e38, float("nan"), -float("inf")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda_device)  # noqa: E731
+    outs = []
+    for gates in (None, gate):
+        out = torch.full((T, heads * value_dim + 8), 7.0, dtype=torch.bfloat16, device=cuda_device)
+        ops.prompt_attention(q, q_tail, kv[:, :heads * KD], kv[:, heads * KD:], tail, out[:, :heads * value_dim],
+                             i32(np.concatenate([[0], np.cumsum(lengths)]).tolist()), i32(lengths), max(lengths), heads, KD, value_dim,
+                             (dim + rot) ** -0.5, gates, gate_kind="element")
+        assert bool((out[:, heads * value_dim:] == 7).all())
+        outs.append(out[:, :heads * value_dim].double())
+    want = outs[0] * torch.sigmoid(gate.double())
+    nan = torch.isnan(gate)
+    assert torch.equal(torch.isnan(outs[1]), nan)
+    error = (outs[1] - want)[~nan].abs()
+    assert bool((error <= 2.0 ** -6.99 * want[~nan].abs() + 1e-37).all())
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,kv_heads,dim,rot,interleaved", [(20, 4, 128, 64, False), (96, 16, 128, 128, False), (3, 1, 24, 8, True), (5, 5, 10, 6, False),
                                                                 (4, 2, 16, 16, True), (2, 1, 40, 0, False), (6, 3, 32, 8, False)])
