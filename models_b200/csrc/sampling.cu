@@ -451,6 +451,34 @@ constexpr int kFewCandidates = 128;
 constexpr int kAloneBlocks = 64;  // so many blocks, clusters of eight, find a multiprocessor each with certainty
 constexpr float kThresholdSlack = 1e-5f;  // of a scaled logit: more than the exponential's rounding can turn around
 
+__device__ __forceinline__ float max3(float a, float b, float c) {  // NaN counts for nothing, as in fmaxf
+    float m;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
+}
+// Integers in the order of the floats, and back.
+__device__ __forceinline__ int ordered_bits(float v) { return __float_as_int(v) >= 0 ? __float_as_int(v) : __float_as_int(v) ^ 0x7fffffff; }
+__device__ __forceinline__ float float_of_ordered(int v) { return __int_as_float(v >= 0 ? v : v ^ 0x7fffffff); }
+
+// Four logits divided by the temperature, rounded as divisions are.  Where the temperature (`usual`: from 2^-30 to 2^30) and all four are far
+// from the ends of the floats, by its reciprocal: the second remainder, which an FMA has whole, is taken of a quotient that is off by less
+// than a unit of its last place, and rounds it to nearest (P. Markstein, IBM J. Res. Dev. 34, 1990).
+__device__ __forceinline__ void divide_four(float4& q, float by, float inverse, bool usual) {
+    const float most = max3(fabsf(q.x), fabsf(q.y), fmaxf(fabsf(q.z), fabsf(q.w))), least = fminf(fminf(fabsf(q.x), fabsf(q.y)), fminf(fabsf(q.z), fabsf(q.w)));
+    float* v = &q.x;
+    if (usual && least >= 0x1p-60f && most <= 0x1p60f) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float a = v[i] * inverse;
+            a = fmaf(fmaf(-a, by, v[i]), inverse, a);
+            v[i] = fmaf(fmaf(-a, by, v[i]), inverse, a);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = v[i] / by;
+    }
+}
+
 template <int kResident>  // blocks of a multiprocessor
 __global__ void __launch_bounds__(kThreads, kResident)
 sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int vocab, float* __restrict__ work,
@@ -460,20 +488,21 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
                    const int* __restrict__ history_len,
                            const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters,
                            const float* __restrict__ uniforms, int* __restrict__ out) {
-    __shared__ Best best_scratch[32];
+    __shared__ float block_tops[32];    // the maxima of this block's warps
     __shared__ float float_scratch[32];
     __shared__ int int_scratch[32];
     __shared__ int histogram[256];      // of this block's ids
     __shared__ int histogram_all[256];  // of the whole row
     __shared__ __align__(16) float sorted_p[kMaxSorted];  // the candidates: filled and used in the cluster's first block only
     __shared__ int sorted_id[kMaxSorted];
-    __shared__ Best slot_best;
     __shared__ float slot_sum;
     __shared__ int slot_ties;
     __shared__ int gathered;            // first block: candidates gathered so far
     __shared__ int shared_int[4];
     __shared__ __align__(16) float warp_tops[kSampleBlocks * 32];
-    __shared__ float few_threshold;
+    __shared__ __align__(16) float eighth_tops[kSampleBlocks];
+    __shared__ int few_threshold;       // ordered_bits of it
+    __shared__ int first_index;         // first block: the lowest id of the row's maximum
 
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -483,7 +512,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     const int begin = min(vocab, part * slice), end = min(vocab, begin + slice);
     const float* row = logits + (size_t)r * row_stride;
     // the block's part of the row lives in shared memory from the first pass to the last: w[i] for begin <= i < end
-    extern __shared__ float slice_values[];
+    extern __shared__ __align__(16) float slice_values[];
     float* w = slice_values - begin;
     const float temp = temperature[r];
     const float pen = penalty[r];
@@ -492,6 +521,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
                               : (history ? const_cast<int*>(history) + (size_t)r * history_stride : nullptr);
     const bool penalised = pen > 1.0f && h_row && history_len[r] > 0;
 
+    if (tid == 0) few_threshold = first_index = 0x7fffffff;
     if (part == 0) {
         if (tid == 0) gathered = 0;
         for (int i = tid; i < kMaxSorted; i += kThreads) {
@@ -513,22 +543,20 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         cluster.sync();
     }
 
-    // adjusted logits, and their first maximum
-    Best mine = {-CUDART_INF_F, 0x7fffffff};
+    // adjusted logits, and the maxima of the warps
+    float mine = -CUDART_INF_F;
     int scalar_from = begin;
     if (!penalised && !(begin & 3) && !((uintptr_t)row & 15)) {
-        // four logits a load where the block's part starts on a 16-byte boundary (every thread still walks ascending ids,
-        // so the first maximum stays the first)
+        // four logits a load where the block's part starts on a 16-byte boundary
         const int whole = begin + ((end - begin) & ~3);
+        const bool divides = temp > 0.0f && temp != 1.0f, usual = temp >= 0x1p-30f && temp <= 0x1p30f;
+        const float inverse = divides ? 1.0f / temp : 1.0f;
+#pragma unroll 4
         for (int i = begin + 4 * tid; i < whole; i += 4 * kThreads) {
-            const float4 q = *reinterpret_cast<const float4*>(row + i);
-            float v4[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float v = temp > 0.0f ? v4[j] / temp : v4[j];
-                w[i + j] = v;
-                if (v > mine.value) mine = {v, i + j};
-            }
+            float4 q = *reinterpret_cast<const float4*>(row + i);
+            if (divides) divide_four(q, temp, inverse, usual);
+            *reinterpret_cast<float4*>(w + i) = q;
+            mine = max3(mine, max3(q.x, q.y, q.z), q.w);
         }
         scalar_from = whole;
     }
@@ -540,22 +568,37 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         }
         if (temp > 0.0f) v = v / temp;
         w[i] = v;
-        if (v > mine.value) mine = {v, i};
+        mine = fmaxf(mine, v);
     }
-    {
-        const Best block = block_best(mine, best_scratch);
-        if (tid == 0) slot_best = block;
-    }
+    mine = warp_max(mine);
+    if ((tid & 31) == 0) block_tops[tid >> 5] = mine;
     cluster.sync();
-    Best top = *cluster.map_shared_rank(&slot_best, 0);
-    for (int b = 1; b < kSampleBlocks; ++b) top = better(top, *cluster.map_shared_rank(&slot_best, b));
-    if (temp <= 0.0f) {
+    constexpr int kTops = kSampleBlocks * 32;
+    if (tid < kTops) {
+        const float t = cluster.map_shared_rank(block_tops, tid >> 5)[tid & 31], eighth = warp_max(t);
+        warp_tops[tid] = t;
+        if ((tid & 31) == 0) eighth_tops[tid >> 5] = eighth;
+    }
+    __syncthreads();
+    float top = -CUDART_INF_F;
+#pragma unroll
+    for (int b = 0; b < kSampleBlocks; b += 2) top = max3(top, eighth_tops[b], eighth_tops[b + 1]);
+    // Where a row takes its first maximum (greedily, or as there is no order to draw from): its lowest id, 0 if nothing is above -infinity.
+    auto take_first_maximum = [&]() {
+        int lowest = 0x7fffffff;
+        if (top > -CUDART_INF_F)
+            for (int i = begin + tid; i < end && lowest == 0x7fffffff; i += kThreads)
+                if (w[i] == top) lowest = i;
+        if (lowest != 0x7fffffff) atomicMin(cluster.map_shared_rank(&first_index, 0), lowest);
+        cluster.sync();
         if (part == 0 && tid == 0) {
-            const int token = top.index == 0x7fffffff ? 0 : top.index;
+            const int token = first_index == 0x7fffffff ? 0 : first_index;
             out[r] = token;
             if (append && h_row) h_row[history_len[r]] = token;
         }
-        cluster.sync();  // nobody leaves while its shared memory may still be read
+    };
+    if (temp <= 0.0f) {
+        take_first_maximum();
         return;
     }
 
@@ -571,33 +614,34 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     bool few = k <= kFewCandidates && k < vocab;
     float threshold = CUDART_INF_F;
     if (few) {
-        const float mine_top = tid < kSampleBlocks * 32 ? cluster.map_shared_rank(best_scratch, tid >> 5)[tid & 31].value : -CUDART_INF_F;
-        if (tid < kSampleBlocks * 32) warp_tops[tid] = mine_top;
-        few = __syncthreads_count(mine_top > -CUDART_INF_F) >= k;  // (else every value would reach the threshold)
+        few = __syncthreads_count(tid < kTops && warp_tops[tid] > -CUDART_INF_F) >= k;  // (else every value would reach the threshold)
         if (few) {
-            if (tid < kSampleBlocks * 32) {
-                int above = 0;
+            // the k-th largest is the smallest that has fewer than k above it: four neighbouring lanes count for one value
+            static_assert(4 * kTops == kThreads, "four threads a value");
+            const float of = warp_tops[tid >> 2];
+            int above = 0;
 #pragma unroll 4
-                for (int j = 0; j < kSampleBlocks * 32; j += 4) {
-                    const float4 t = *reinterpret_cast<const float4*>(warp_tops + j);
-                    above += (t.x > mine_top || (t.x == mine_top && j < tid)) + (t.y > mine_top || (t.y == mine_top && j + 1 < tid)) +
-                             (t.z > mine_top || (t.z == mine_top && j + 2 < tid)) + (t.w > mine_top || (t.w == mine_top && j + 3 < tid));
-                }
-                if (above == k - 1) few_threshold = mine_top;
+            for (int j = 4 * (tid & 3); j < kTops; j += 16) {
+                const float4 t = *reinterpret_cast<const float4*>(warp_tops + j);
+                above += (t.x > of) + (t.y > of) + (t.z > of) + (t.w > of);
             }
+            above += __shfl_xor_sync(0xffffffffu, above, 1);
+            above += __shfl_xor_sync(0xffffffffu, above, 2);
+            const int lowest = __reduce_min_sync(0xffffffffu, above < k ? ordered_bits(of) : 0x7fffffff);
+            if ((tid & 31) == 0) atomicMin(&few_threshold, lowest);
             __syncthreads();
-            threshold = few_threshold - kThresholdSlack;
+            threshold = float_of_ordered(few_threshold) - kThresholdSlack;
         }
     }
 
-    // softmax over the whole vocabulary
+    // softmax over the whole vocabulary: the sum of the exponentials, each thread's in the order of its ids
     float local = 0.0f;
     bool gathers = few;  // a thread that finds no place left stops: the histograms will decide
+#pragma unroll 4
     for (int i = begin + tid; i < end; i += kThreads) {
-        const float v = w[i], e = expf(v - top.value);
-        w[i] = e;
+        const float v = w[i], e = expf(v - top);
         local += e;
-        if (gathers && v >= threshold) {
+        if (v >= threshold && gathers) {
             const unsigned peers = __activemask();  // the lanes that are here together add once
             const int lane = tid & 31, leader = __ffs(peers) - 1;
             int at = 0;
@@ -619,12 +663,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     float sum = 0.0f;
     for (int b = 0; b < kSampleBlocks; ++b) sum += *cluster.map_shared_rank(&slot_sum, b);
     if (!(sum == sum)) {  // a NaN or an infinity among the logits: no order to draw from, the row takes its first maximum
-        if (part == 0 && tid == 0) {
-            const int token = top.index == 0x7fffffff ? 0 : top.index;
-            out[r] = token;
-            if (grown) *grown = token;
-        }
-        cluster.sync();  // everybody has read the sums
+        take_first_maximum();
         return;
     }
     if (few) {
@@ -666,7 +705,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         }
         // (the histograms' barriers lie between this and the next candidate)
     }
-    for (int i = begin + tid; i < end; i += kThreads) w[i] = w[i] / sum;
+    for (int i = begin + tid; i < end; i += kThreads) w[i] = expf(w[i] - top) / sum;
     __syncthreads();
 
     if (k == vocab && nucleus >= 1.0f && vocab > kMaxSorted) {
