@@ -140,7 +140,7 @@ def build_library(name: str, sources: Sequence[str], defines: Mapping[str, objec
 def load_library(name: str, sources: Sequence[str], defines: Mapping[str, object] | None = None,
                  extra_flags: Sequence[str] = ()) -> ctypes.CDLL:
     """The loaded library (compiled first if needed).  Raises KernelBuildError; never falls back."""
-    quick = (name, tuple(sources), tuple(sorted((defines or {}).items())), tuple(extra_flags))
+    quick = (name, tuple(sources), tuple(sorted(defines.items())) if defines else (), tuple(extra_flags))
     lib = _by_request.get(quick)  # the common case: no hashing of sources on the way to a launch
     if lib is not None:
         return lib

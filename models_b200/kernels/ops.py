@@ -37,15 +37,18 @@ def _cuda(*tensors):
                 f"{t.device}); there is no CPU path")
 
 
+_pointer = ctypes.c_void_p
+
+
 def _p(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return None if t is None else _pointer(t.data_ptr())
 
 
 def _stream():
     """The current stream of the current device, as the raw handle the launchers take (the two
     calls below are what torch.cuda.current_stream() ends in, without its Python layers: this runs
     once per kernel launch)."""
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return _pointer(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 _launches = [0]
@@ -119,8 +122,8 @@ TCGEN05_ATTENTION_MIN_ROWS = 33  # shorter steps go to the mma.sync kernel, whos
 
 def prefill_attention_tcgen05_takes(q: torch.Tensor, out: torch.Tensor, head_dim: int, max_q_len: int) -> bool:
     """Head sizes 64 and 128, steps of more than a few tokens, rows that TMA and 16-byte stores can address."""
-    return (head_dim in (64, 128) and max_q_len >= TCGEN05_ATTENTION_MIN_ROWS and q.stride(0) % 8 == 0
-            and out.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0)
+    return (head_dim in (64, 128) and max_q_len >= TCGEN05_ATTENTION_MIN_ROWS and q.stride()[0] % 8 == 0
+            and out.stride()[0] % 8 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0)
 
 
 def gemm32():
@@ -192,7 +195,7 @@ def rope_cache_write(qkv: torch.Tensor, positions: Optional[torch.Tensor], cos: 
     """Rotates the query heads of `qkv` ([T, (heads + 2*kv_heads) * head_dim]) in place; rotates the
     key heads and copies the value heads into the pools at `slot_mapping`."""
     _cuda(qkv, positions, cos, sin, k_pool, v_pool, slot_mapping)
-    if qkv.dim() != 2 or qkv.stride(1) != 1:
+    if qkv.dim() != 2 or qkv.stride()[1] != 1:
         raise KernelError("qkv must be a [tokens, columns] tensor with unit column stride")
     need = (heads + (2 * kv_heads if write_cache else 0)) * head_dim
     if qkv.shape[1] < need:
@@ -207,7 +210,7 @@ def rope_cache_write(qkv: torch.Tensor, positions: Optional[torch.Tensor], cos: 
     if write_cache and (k_pool.dtype != qkv.dtype or v_pool.dtype != qkv.dtype):
         raise KernelError(f"cache pools ({k_pool.dtype}) must have the dtype of qkv ({qkv.dtype})")
     lib = elementwise()
-    _run(lib, lib.mb_rope_cache_write(_p(qkv), _code(qkv.dtype), qkv.stride(0), _p(positions), _p(cos), _p(sin),
+    _run(lib, lib.mb_rope_cache_write(_p(qkv), _code(qkv.dtype), qkv.stride()[0], _p(positions), _p(cos), _p(sin),
                                       _p(k_pool), _p(v_pool), _p(slot_mapping), qkv.shape[0], heads, kv_heads,
                                       head_dim, rotary_dim, 1 if interleaved else 0, page_size,
                                       1 if write_cache else 0, _stream()))
@@ -254,10 +257,10 @@ def logit_epilogue(logits: torch.Tensor, scale: float, softcap: float) -> torch.
     """In place on float32 logits [rows, vocab]: times `scale`, then softcap * tanh(logits / softcap)
     unless softcap is 0."""
     _cuda(logits)
-    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1:
+    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride()[1] != 1:
         raise KernelError("logit_epilogue takes float32 [rows, vocab] logits")
     lib = elementwise()
-    _run(lib, lib.mb_logit_epilogue(_p(logits), logits.stride(0), logits.shape[0], logits.shape[1], ctypes.c_float(scale),
+    _run(lib, lib.mb_logit_epilogue(_p(logits), logits.stride()[0], logits.shape[0], logits.shape[1], ctypes.c_float(scale),
                                     ctypes.c_float(softcap), _stream()))
     return logits
 
@@ -360,10 +363,10 @@ def store_columns(x: torch.Tensor, dst: torch.Tensor, copy: Optional[torch.Tenso
     for t in (dst, copy):
         if t is not None:
             _columns(t, "store_columns")
-            if t.shape != x.shape or t.dtype != dst.dtype or t.stride(0) != dst.stride(0):
+            if t.shape != x.shape or t.dtype != dst.dtype or t.stride()[0] != dst.stride()[0]:
                 raise KernelError(f"store_columns: {tuple(t.shape)} {t.dtype} does not take rows of {tuple(x.shape)}")
     lib = elementwise()
-    _run(lib, lib.mb_store_columns(_p(x), _p(dst), _p(copy), _code(dst.dtype), x.shape[0], x.shape[1], dst.stride(0), _stream()))
+    _run(lib, lib.mb_store_columns(_p(x), _p(dst), _p(copy), _code(dst.dtype), x.shape[0], x.shape[1], dst.stride()[0], _stream()))
 
 
 def result_norm_library():
@@ -458,13 +461,13 @@ def side_gate(gate: torch.Tensor, table: torch.Tensor, tokens: torch.Tensor, col
         raise KernelError(f"side_gate: gates {tuple(gate.shape)} {gate.dtype} do not fit the table {tuple(table.shape)}")
     out = torch.empty((gate.shape[0], columns), dtype=table.dtype, device=gate.device)
     lib = result_norm_library()
-    _run(lib, lib.mb_side_gate(_p(gate), gate.stride(0), _p(table), _p(tokens), table.shape[1], _p(out), columns, _code(table.dtype),
+    _run(lib, lib.mb_side_gate(_p(gate), gate.stride()[0], _p(table), _p(tokens), table.shape[1], _p(out), columns, _code(table.dtype),
                                gate.shape[0], _stream()))
     return out
 
 
 def _columns(t: torch.Tensor, name: str):
-    if t.dim() != 2 or t.stride(1) != 1:
+    if t.dim() != 2 or t.stride()[1] != 1:
         raise KernelError(f"{name} must be a [rows, columns] tensor (or column slice) with unit column stride")
 
 
@@ -476,7 +479,7 @@ def activate(src: torch.Tensor, dst: torch.Tensor, activation: str, scale: float
     if src.shape != dst.shape or src.dtype != dst.dtype:
         raise KernelError(f"activate: {tuple(src.shape)} {src.dtype} does not fit {tuple(dst.shape)} {dst.dtype}")
     lib = elementwise()
-    _run(lib, lib.mb_activate(_p(src), src.stride(0), _p(dst), dst.stride(0), _code(src.dtype), src.shape[0], src.shape[1],
+    _run(lib, lib.mb_activate(_p(src), src.stride()[0], _p(dst), dst.stride()[0], _code(src.dtype), src.shape[0], src.shape[1],
                               activation_code(activation), ctypes.c_float(scale), _stream()))
     return dst
 
@@ -490,7 +493,7 @@ def xielu(src: torch.Tensor, dst: torch.Tensor, a_pos: float, a_neg: float, scal
     if src.shape != dst.shape or src.dtype != dst.dtype:
         raise KernelError(f"xielu: {tuple(src.shape)} {src.dtype} does not fit {tuple(dst.shape)} {dst.dtype}")
     lib = elementwise()
-    _run(lib, lib.mb_xielu(_p(src), src.stride(0), _p(dst), dst.stride(0), _code(src.dtype), src.shape[0], src.shape[1],
+    _run(lib, lib.mb_xielu(_p(src), src.stride()[0], _p(dst), dst.stride()[0], _code(src.dtype), src.shape[0], src.shape[1],
                            ctypes.c_float(a_pos), ctypes.c_float(a_neg), ctypes.c_float(scale), _stream()))
     return dst
 
@@ -507,7 +510,7 @@ def gated_residual_add(x: torch.Tensor, gate: torch.Tensor, bias: torch.Tensor, 
     if bias.dtype != torch.float32 or bias.numel() != x.shape[1] or not bias.is_contiguous():
         raise KernelError(f"gated_residual_add: bias must be contiguous float32 of {x.shape[1]} elements")
     lib = elementwise()
-    _run(lib, lib.mb_gated_residual_add(_p(x), _p(gate), gate.stride(0), _code(gate.dtype), _p(bias), _p(delta), _code(delta.dtype),
+    _run(lib, lib.mb_gated_residual_add(_p(x), _p(gate), gate.stride()[0], _code(gate.dtype), _p(bias), _p(delta), _code(delta.dtype),
                                         x.shape[0], x.shape[1], _stream()))
     return x
 
@@ -523,7 +526,7 @@ def paged_attention_rows(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tenso
     _int32(block_table, "block_table")
     _int32(cu_q, "cu_q")
     _int32(kv_lens, "kv_lens")
-    if q.stride(1) != 1 or out.stride(1) != 1:
+    if q.stride()[1] != 1 or out.stride()[1] != 1:
         raise KernelError("q and out need unit column stride")
     if k_pool.dim() != 4 or k_pool.shape[1] != kv_heads or k_pool.shape[3] != head_dim or not k_pool.is_contiguous():
         raise KernelError(f"k_pool must be contiguous [pages, {kv_heads}, page_size, {head_dim}], got {tuple(k_pool.shape)}")
@@ -533,7 +536,7 @@ def paged_attention_rows(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tenso
         raise KernelError("q, out and the pools must share one dtype")
     sequences = kv_lens.numel()
     lib = attention_rows()
-    _run(lib, lib.mb_paged_attention_rows(_p(q), q.stride(0), _p(out), out.stride(0), _code(q.dtype), _p(k_pool),
+    _run(lib, lib.mb_paged_attention_rows(_p(q), q.stride()[0], _p(out), out.stride()[0], _code(q.dtype), _p(k_pool),
                                           _p(v_pool), _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_lens),
                                           sequences, max_q_len, heads, kv_heads, head_dim, k_pool.shape[2],
                                           window or 0, ctypes.c_float(scale), _stream()))
@@ -568,7 +571,7 @@ def rotate_store(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, positions: t
             or not k_pool.is_contiguous() or not v_pool.is_contiguous()):
         raise KernelError(f"pools must be contiguous [pages, {kv_heads}, page_size, {head_dim}] and [.., {value_dim}]")
     lib = talking_attention_library()
-    _run(lib, lib.mb_rotate_store(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _code(q.dtype), _p(positions),
+    _run(lib, lib.mb_rotate_store(_p(q), q.stride()[0], _p(k), k.stride()[0], _p(v), v.stride()[0], _code(q.dtype), _p(positions),
                                   _p(cos), _p(sin), _p(k_pool), _p(v_pool), _p(slot_mapping), q.shape[0], heads, kv_heads,
                                   head_dim, value_dim, rotary_dim, page_size, _stream()))
 
@@ -604,7 +607,7 @@ def talking_attention_tc_takes(q: torch.Tensor, out: torch.Tensor, k_pool: torch
         return False
     if head_dim % 16 or value_dim % 16 or not 16 <= head_dim <= 256 or not 16 <= value_dim <= (256 if heads <= 8 else 128):
         return False
-    if q.stride(0) % 8 or out.stride(0) % 2 or q.data_ptr() % 16 or out.data_ptr() % 4 or k_pool.data_ptr() % 16 or v_pool.data_ptr() % 16:
+    if q.stride()[0] % 8 or out.stride()[0] % 2 or q.data_ptr() % 16 or out.data_ptr() % 4 or k_pool.data_ptr() % 16 or v_pool.data_ptr() % 16:
         return False
     block = (heads * 16 * (2 * head_dim + 16) + 2 * kv_heads * 32 * (2 * head_dim + 2 * value_dim + 32) + 4 * (2 * 16 * 516 + heads * heads))
     return block <= 227 * 1024
@@ -657,9 +660,9 @@ def talking_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, 
         scratch = torch.empty((lib.mb_talking_decode_scratch_floats(sequences, heads, value_dim, bound, window or 0, keep_first),),
                               dtype=torch.float32, device=q.device)
         _run(lib, lib.mb_talking_attention_decode(
-            _p(q), q.stride(0), _p(out), out.stride(0), _code(q.dtype), _p(k_pool), _p(v_pool), _p(block_table),
+            _p(q), q.stride()[0], _p(out), out.stride()[0], _code(q.dtype), _p(k_pool), _p(v_pool), _p(block_table),
             block_table.shape[1], _p(cu_q), _p(kv_lens), sequences, bound, _p(talk), _p(gate),
-            gate.stride(0) if gate is not None else 0, heads, kv_heads, head_dim, value_dim, page_size, window or 0, keep_first,
+            gate.stride()[0] if gate is not None else 0, heads, kv_heads, head_dim, value_dim, page_size, window or 0, keep_first,
             ctypes.c_float(scale), ctypes.c_float(out_scale), _p(scratch), _p(_zero_tickets(q.device, sequences)), _stream()))
         _launches[0] += 1  # two kernels
         return
@@ -669,15 +672,15 @@ def talking_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, 
             raise KernelError("the tensor-core form takes bfloat16")
         lib = talking_attention_tc_library(heads, head_dim, value_dim)
         _run(lib, lib.mb_talking_attention_tc(
-            _p(q), q.stride(0), _p(out), out.stride(0), _p(k_pool), _p(v_pool), _p(block_table), block_table.shape[1], _p(cu_q),
-            _p(kv_lens), kv_lens.numel(), max_q_len, _p(talk), _p(gate), gate.stride(0) if gate is not None else 0, kv_heads,
+            _p(q), q.stride()[0], _p(out), out.stride()[0], _p(k_pool), _p(v_pool), _p(block_table), block_table.shape[1], _p(cu_q),
+            _p(kv_lens), kv_lens.numel(), max_q_len, _p(talk), _p(gate), gate.stride()[0] if gate is not None else 0, kv_heads,
             page_size, window or 0, keep_first, ctypes.c_float(scale), ctypes.c_float(out_scale), _stream()))
         return
     lib = talking_attention_library()
     _run(lib, lib.mb_talking_attention_rows(
-        _p(q), q.stride(0), _p(out), out.stride(0), _code(q.dtype), _p(k_pool), _p(v_pool), _p(block_table),
+        _p(q), q.stride()[0], _p(out), out.stride()[0], _code(q.dtype), _p(k_pool), _p(v_pool), _p(block_table),
         block_table.shape[1], _p(cu_q), _p(kv_lens), kv_lens.numel(), max_q_len, _p(talk), _p(gate),
-        gate.stride(0) if gate is not None else 0, heads, kv_heads, head_dim, value_dim, page_size, window or 0, keep_first,
+        gate.stride()[0] if gate is not None else 0, heads, kv_heads, head_dim, value_dim, page_size, window or 0, keep_first,
         ctypes.c_float(scale), ctypes.c_float(out_scale), _stream()))
 
 
@@ -715,8 +718,8 @@ def norm_store(q: Optional[torch.Tensor], k: torch.Tensor, v: Optional[torch.Ten
                       or v_pool.dtype != k.dtype):
         raise KernelError(f"norm_store: the value pool must be contiguous [pages, {kv_heads}, page_size, {value_dim}] of {k.dtype}")
     lib = gated_attention_library()
-    _run(lib, lib.mb_norm_store(_p(q), q.stride(0) if q is not None else 0, _p(k), k.stride(0), _p(v),
-                                v.stride(0) if v is not None else 0, _code(k.dtype), _p(positions), _p(q_gain), _p(k_gain),
+    _run(lib, lib.mb_norm_store(_p(q), q.stride()[0] if q is not None else 0, _p(k), k.stride()[0], _p(v),
+                                v.stride()[0] if v is not None else 0, _code(k.dtype), _p(positions), _p(q_gain), _p(k_gain),
                                 ctypes.c_float(eps), ctypes.c_float(temperature_coef), int(temperature_every), _p(k_pool),
                                 _p(v_pool) if value_dim else None, _p(slot_mapping), tokens, heads, kv_heads, head_dim, value_dim,
                                 page_size, _stream()))
@@ -751,7 +754,7 @@ def rotate_norm_store(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, positio
     if tuple(v_pool.shape[1:]) != (kv_heads, page_size, value_dim) or not v_pool.is_contiguous() or v_pool.dtype != k.dtype:
         raise KernelError(f"rotate_norm_store: the value pool must be contiguous [pages, {kv_heads}, page_size, {value_dim}] of {k.dtype}")
     lib = gated_attention_library()
-    _run(lib, lib.mb_rotate_norm_store(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _code(k.dtype), _p(positions),
+    _run(lib, lib.mb_rotate_norm_store(_p(q), q.stride()[0], _p(k), k.stride()[0], _p(v), v.stride()[0], _code(k.dtype), _p(positions),
                                        _p(cos) if rotary_dim else None, _p(sin) if rotary_dim else None, int(rotary_dim),
                                        1 if interleaved else 0, 1 if unit_norm else 0, ctypes.c_float(eps),
                                        _p(value_cos) if value_rotary_dim else None, _p(value_sin) if value_rotary_dim else None,
@@ -793,7 +796,7 @@ def project_norm_rotate_store(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
         raise KernelError(f"project_norm_rotate_store: the value pool must be contiguous [pages, {kv_heads}, page_size, {value_dim}] of {k.dtype}")
     lib = gated_attention_library()
     _run(lib, lib.mb_project_norm_rotate_store(
-        _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _code(k.dtype), _p(q_bias), _p(k_bias), _p(v_bias), _p(q_gain),
+        _p(q), q.stride()[0], _p(k), k.stride()[0], _p(v), v.stride()[0], _code(k.dtype), _p(q_bias), _p(k_bias), _p(v_bias), _p(q_gain),
         _p(k_gain), ctypes.c_float(eps), _p(positions), _p(cos) if rotary_dim else None, _p(sin) if rotary_dim else None,
         int(rotary_dim), 1 if interleaved else 0, _p(k_pool), _p(v_pool), _p(slot_mapping), tokens, heads, kv_heads, head_dim,
         value_dim, page_size, _stream()))
@@ -822,9 +825,9 @@ def gated_attention_tc_takes(q: torch.Tensor, out: torch.Tensor, k_pool: torch.T
         return False
     if v_pool is not None and head_dim > 256:
         return False
-    if q.stride(0) % 8 or q.data_ptr() % 16 or out.stride(0) % 2 or out.data_ptr() % 4 or k_pool.data_ptr() % 16:
+    if q.stride()[0] % 8 or q.data_ptr() % 16 or out.stride()[0] % 2 or out.data_ptr() % 4 or k_pool.data_ptr() % 16:
         return False
-    return gate is None or gate_kind != "element" or (gate.stride(0) % 2 == 0 and gate.data_ptr() % 4 == 0)
+    return gate is None or gate_kind != "element" or (gate.stride()[0] % 2 == 0 and gate.data_ptr() % 4 == 0)
 
 
 def float_weight_attention_library(key_dim: int, value_dim: int, turned: int = 0, contiguous: bool = False, shaped: bool = False):
@@ -840,7 +843,7 @@ def float_weight_attention_takes(q: torch.Tensor, out: torch.Tensor, k_pool: tor
     """bfloat16, cache pages of 64, keys of 64, 128, 192 or 256 numbers and values of 64 or 128 of their own, steps of more than a
     few tokens, rows that TMA and 16-byte stores can address."""
     return (q.dtype == torch.bfloat16 and v_pool is not None and k_pool.shape[2] == 64 and head_dim % 64 == 0 and 64 <= head_dim <= 256
-            and value_dim in (64, 128) and max_q_len >= TCGEN05_ATTENTION_MIN_ROWS and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
+            and value_dim in (64, 128) and max_q_len >= TCGEN05_ATTENTION_MIN_ROWS and q.stride()[0] % 8 == 0 and out.stride()[0] % 8 == 0
             and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0 and k_pool.data_ptr() % 16 == 0 and v_pool.data_ptr() % 16 == 0)
 
 
@@ -866,7 +869,7 @@ def prompt_attention(q: torch.Tensor, q_tail: Optional[torch.Tensor], k: torch.T
         if t.dtype != torch.bfloat16 or t.shape[0] != n:
             raise KernelError(f"prompt_attention: {name} must be bfloat16 with {n} rows, got {tuple(t.shape)} {t.dtype}")
     key_dim, value_dim = k.shape[1] // heads, v.shape[1] // heads
-    if k.shape[1] != heads * key_dim or v.shape[1] != heads * value_dim or k.stride(0) != v.stride(0) or key_dim % 64 or value_dim % 64:
+    if k.shape[1] != heads * key_dim or v.shape[1] != heads * value_dim or k.stride()[0] != v.stride()[0] or key_dim % 64 or value_dim % 64:
         raise KernelError(f"prompt_attention: keys {tuple(k.shape)} and values {tuple(v.shape)} are no {heads} heads of whole 64 columns")
     if out.shape[1] != heads * value_columns or value_columns > value_dim or q.shape[1] < heads * head_columns:
         raise KernelError(f"prompt_attention: q {tuple(q.shape)} or out {tuple(out.shape)} does not fit {heads} heads")
@@ -882,8 +885,8 @@ def prompt_attention(q: torch.Tensor, q_tail: Optional[torch.Tensor], k: torch.T
             raise KernelError(f"prompt_attention: a gate of kind {gate_kind!r} cannot be {tuple(gate.shape)} {gate.dtype}")
     lib = float_weight_attention_library(key_dim, value_dim, turned, True)
     _run(lib, lib.mb_prompt_attention_tcgen05(
-        _p(q), q.stride(0), int(head_columns), q.shape[1], _p(q_tail), _p(k), _p(v), k.stride(0), _p(k_tail), rows, _p(out), out.stride(0),
-        int(value_columns), _p(gate), gate.stride(0) if gate is not None else 0,
+        _p(q), q.stride()[0], int(head_columns), q.shape[1], _p(q_tail), _p(k), _p(v), k.stride()[0], _p(k_tail), rows, _p(out), out.stride()[0],
+        int(value_columns), _p(gate), gate.stride()[0] if gate is not None else 0,
         1 if gate is not None and gate_kind == "element" else 0, int(key_rows), int(key_window), keys, _p(cu_q), _p(kv_lens), kv_lens.numel(), int(max_q_len), heads,
         heads, int(window), ctypes.c_float(scale), _stream()))
 
@@ -971,7 +974,7 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
     extras = (_p(head_scale), ctypes.c_float(softcap), 1 if sink else 0, _p(turn_cos), _p(turn_sin), int(block), int(window))
     softmax = 1 if weights == "softmax" else 0
     sequences = kv_lens.numel()
-    gate_stride = gate.stride(0) if gate is not None else 0
+    gate_stride = gate.stride()[0] if gate is not None else 0
     plain_scores = head_scale is None and head_bias is None and softcap == 0.0 and slope_exponent == 0.0 and turn_cos is None
     shared_decode = (v_pool is None and kv_heads == 1 and heads >= 8 and weights == "softmax" and plain_scores and max_q_len == 1
                      and gated_attention_tc_takes(q, out, k_pool, head_dim, value_dim, GATED_TC_MIN_ROWS, None))
@@ -988,11 +991,11 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
         runs = -(-pages // span)
         partial = torch.empty((sequences * heads * runs * (2 + value_dim),), dtype=torch.float32, device=q.device)
         lib = gated_attention_tc_library(head_dim, value_dim, True)
-        _run(lib, lib.mb_gated_attention_tc_decode(_p(q), q.stride(0), _p(k_pool), _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_lens),
+        _run(lib, lib.mb_gated_attention_tc_decode(_p(q), q.stride()[0], _p(k_pool), _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_lens),
                                                    _p(partial), runs, span, sequences, heads, page_size, ctypes.c_float(scale), int(block),
                                                    int(window), _stream()))
         lib = gated_attention_library()
-        _run(lib, lib.mb_gated_attention_combine(_p(partial), runs, _p(out), out.stride(0), _p(cu_q), _p(kv_lens), _p(gate), gate_stride,
+        _run(lib, lib.mb_gated_attention_combine(_p(partial), runs, _p(out), out.stride()[0], _p(cu_q), _p(kv_lens), _p(gate), gate_stride,
                                                  GATE_KINDS[gate_kind], sequences, heads, value_dim, 1 if sink else 0, _stream()))
         return
     if kernel == "decode" or (kernel is None and max_q_len == 1):
@@ -1008,7 +1011,7 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
         scratch = torch.empty((lib.mb_gated_attention_decode_scratch_floats(sequences, heads, value_dim, runs),), dtype=torch.float32,
                               device=q.device)
         _run(lib, lib.mb_gated_attention_decode(
-            _p(q), q.stride(0), _p(out), out.stride(0), _code(q.dtype), _p(k_pool), _p(values), values.shape[3], _p(block_table),
+            _p(q), q.stride()[0], _p(out), out.stride()[0], _code(q.dtype), _p(k_pool), _p(values), values.shape[3], _p(block_table),
             block_table.shape[1], _p(cu_q), _p(kv_lens), _p(head_bias), _p(gate), gate_stride, GATE_KINDS[gate_kind], sequences,
             heads, kv_heads, head_dim, value_dim, page_size, softmax, ctypes.c_float(scale), ctypes.c_float(slope_exponent), runs,
             span, _p(scratch), *extras, _stream()))
@@ -1020,7 +1023,7 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
             raise KernelError("the tcgen05 form takes plain softmax attention in bfloat16, pages of 64, and sizes that are multiples of 64")
         lib = float_weight_attention_library(head_dim, value_dim)
         _run(lib, lib.mb_prefill_attention_tcgen05(
-            _p(q), q.stride(0), q.shape[0], _p(out), out.stride(0), _p(k_pool), _p(v_pool), k_pool.shape[0], _p(block_table),
+            _p(q), q.stride()[0], q.shape[0], _p(out), out.stride()[0], _p(k_pool), _p(v_pool), k_pool.shape[0], _p(block_table),
             block_table.shape[1], _p(cu_q), _p(kv_lens), sequences, max_q_len, heads, kv_heads, page_size, int(window), ctypes.c_float(scale),
             _stream()))
         return
@@ -1034,7 +1037,7 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
     if kernel is None and shaped and full and float_weight_attention_takes(q, out, k_pool, v_pool, head_dim, value_dim, max_q_len):
         lib = float_weight_attention_library(head_dim, value_dim, shaped=True)
         _run(lib, lib.mb_prefill_attention_tcgen05(
-            _p(q), q.stride(0), q.shape[0], _p(out), out.stride(0), _p(k_pool), _p(v_pool), k_pool.shape[0], _p(block_table),
+            _p(q), q.stride()[0], q.shape[0], _p(out), out.stride()[0], _p(k_pool), _p(v_pool), k_pool.shape[0], _p(block_table),
             block_table.shape[1], _p(cu_q), _p(kv_lens), sequences, max_q_len, heads, kv_heads, page_size, int(window), ctypes.c_float(scale),
             _p(head_scale), ctypes.c_float(softcap), 1 if sink else 0, _p(turn_cos), _p(turn_sin), _stream()))
         return
@@ -1043,13 +1046,13 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
             raise KernelError("the tensor-core form takes bfloat16, pages of 64 and key and value sizes that are multiples of 16 up to 256")
         lib = gated_attention_tc_library(head_dim, value_dim, v_pool is None)
         _run(lib, lib.mb_gated_attention_tc(
-            _p(q), q.stride(0), _p(out), out.stride(0), _p(k_pool), _p(values), _p(block_table), block_table.shape[1], _p(cu_q),
+            _p(q), q.stride()[0], _p(out), out.stride()[0], _p(k_pool), _p(values), _p(block_table), block_table.shape[1], _p(cu_q),
             _p(kv_lens), _p(head_bias), _p(gate), gate_stride, GATE_KINDS[gate_kind], sequences, max_q_len, heads, kv_heads,
             page_size, softmax, ctypes.c_float(scale), ctypes.c_float(slope_exponent), *extras, _stream()))
         return
     lib = gated_attention_library()
     _run(lib, lib.mb_gated_attention_rows(
-        _p(q), q.stride(0), _p(out), out.stride(0), _code(q.dtype), _p(k_pool), _p(values), values.shape[3], _p(block_table),
+        _p(q), q.stride()[0], _p(out), out.stride()[0], _code(q.dtype), _p(k_pool), _p(values), values.shape[3], _p(block_table),
         block_table.shape[1], _p(cu_q), _p(kv_lens), _p(head_bias), _p(gate), gate_stride, GATE_KINDS[gate_kind], sequences,
         max_q_len, heads, kv_heads, head_dim, value_dim, page_size, softmax, ctypes.c_float(scale), ctypes.c_float(slope_exponent),
         *extras, _stream()))
@@ -1085,8 +1088,8 @@ def head_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, heads:
             if table is None or table.dtype != torch.float32 or table.dim() != 2 or table.shape[1] * 2 != turned or not table.is_contiguous():
                 raise KernelError(f"head_linear: a tail of {turned} needs contiguous float32 tables [positions, {turned // 2}]")
     lib = gated_attention_library()
-    _run(lib, lib.mb_head_linear(_p(x), x.stride(0), _p(weight), _p(out), out.stride(0), _code(x.dtype), _p(gate),
-                                 gate.stride(0) if gate is not None else 0, 1 if gate_kind == "element" else 0, x.shape[0], heads, n_in,
+    _run(lib, lib.mb_head_linear(_p(x), x.stride()[0], _p(weight), _p(out), out.stride()[0], _code(x.dtype), _p(gate),
+                                 gate.stride()[0] if gate is not None else 0, 1 if gate_kind == "element" else 0, x.shape[0], heads, n_in,
                                  n_out, n_in + turned, n_out + turned, int(turned), _p(cos) if turned else None, _p(sin) if turned else None,
                                  _p(positions) if turned else None, 1 if tensor_cores else 0, _stream()))
 
@@ -1123,8 +1126,8 @@ def latent_prepare(q: Optional[torch.Tensor], q_gain: Optional[torch.Tensor], q_
                 if table is None or table.dtype != torch.float32 or table.dim() != 2 or table.shape[1] * 2 != turned or not table.is_contiguous():
                     raise KernelError(f"latent_prepare: a tail of {turned} needs contiguous float32 tables [positions, {turned // 2}]")
     lib = gated_attention_library()
-    _run(lib, lib.mb_latent_prepare(_p(q), q.stride(0) if q is not None else 0, _p(q_gain), q.shape[1] if q is not None else 0, _p(out),
-                                    int(q_columns), _p(k), k.stride(0) if k is not None else 0, _p(k_gain), latent, int(turned),
+    _run(lib, lib.mb_latent_prepare(_p(q), q.stride()[0] if q is not None else 0, _p(q_gain), q.shape[1] if q is not None else 0, _p(out),
+                                    int(q_columns), _p(k), k.stride()[0] if k is not None else 0, _p(k_gain), latent, int(turned),
                                     _p(cos) if turned else None, _p(sin) if turned else None, _p(positions), ctypes.c_float(eps),
                                     _p(k_pool) if k is not None else None, _p(slot_mapping), _code(dtype), rows, _stream()))
     return out
@@ -1161,9 +1164,9 @@ def latent_rows(k: torch.Tensor, gain: torch.Tensor, turned: int, cos: Optional[
             tail = torch.empty((rows, padded), dtype=k.dtype, device=k.device)
             q_tail = torch.empty((rows, heads * padded), dtype=k.dtype, device=k.device)
     lib = gated_attention_library()
-    _run(lib, lib.mb_latent_rows(_p(k), k.stride(0), _p(gain), latent, int(turned), _p(cos) if turned else None, _p(sin) if turned else None,
+    _run(lib, lib.mb_latent_rows(_p(k), k.stride()[0], _p(gain), latent, int(turned), _p(cos) if turned else None, _p(sin) if turned else None,
                                  _p(positions), ctypes.c_float(eps), _p(k_pool), _p(slot_mapping), _p(own), _p(tail), _p(q),
-                                 q.stride(0) if q is not None else 0, head_columns - turned, heads, _p(q_tail), int(padded), _code(k.dtype), rows,
+                                 q.stride()[0] if q is not None else 0, head_columns - turned, heads, _p(q_tail), int(padded), _code(k.dtype), rows,
                                  _stream()))
     return own, tail, q_tail
 
@@ -1217,12 +1220,12 @@ def retention_chunks_takes(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g:
     """bfloat16 steps of many tokens a sequence, key heads of 64 numbers and value heads of 64 or 128, rows that start on 16 bytes (results on a
     pair's boundary)."""
     if raw_out is not None:
-        pairs = raw_out.stride(0) % 2 == 0 and raw_out.data_ptr() % 8 == 0
+        pairs = raw_out.stride()[0] % 2 == 0 and raw_out.data_ptr() % 8 == 0
     else:
-        pairs = out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0 and g.data_ptr() % 4 == 0
+        pairs = out.stride()[0] % 2 == 0 and out.data_ptr() % 4 == 0 and g.data_ptr() % 4 == 0
     return (pairs and q.dtype == torch.bfloat16 and max_q_len >= RETENTION_CHUNK_MIN_ROWS and head_dim == 64 and value_dim in (64, 128)
             and (max_q_len > 2 * RETENTION_RUN or q.shape[0] >= RETENTION_CHUNK_MIN_MEAN * sequences)
-            and q.stride(0) % 8 == 0 and state.data_ptr() % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)))
+            and q.stride()[0] % 8 == 0 and state.data_ptr() % 16 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, k, v)))
 
 
 def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, positions: torch.Tensor,
@@ -1261,7 +1264,7 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.T
         _columns(t, name)
         if tuple(t.shape) != (tokens, width) or t.dtype != q.dtype:
             raise KernelError(f"retention_scan: {name} is {tuple(t.shape)} {t.dtype}; [{tokens}, {width}] {q.dtype} is needed")
-    if not (q.stride(0) == k.stride(0) == v.stride(0) == g.stride(0)):
+    if not (q.stride()[0] == k.stride()[0] == v.stride()[0] == g.stride()[0]):
         raise KernelError("retention_scan: q, k, v and g must share one row stride")
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, head_dim, value_dim) or not state.is_contiguous():
         raise KernelError(f"retention_scan: the state must be contiguous float32 [slots, {heads}, {head_dim}, {value_dim}]")
@@ -1276,11 +1279,11 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.T
         lib = retention_chunks_library()
         items = (tokens // lib.mb_retention_chunk_tokens() + cu_q.numel() - 1) * heads * head_dim * value_dim
         starts = torch.empty((items,), dtype=torch.float32, device=q.device)
-        _run(lib, lib.mb_retention_chunks(_p(q), _p(k), _p(v), _p(g), q.stride(0), _p(positions), _p(cos), _p(sin), rotary_dim, _p(decay),
+        _run(lib, lib.mb_retention_chunks(_p(q), _p(k), _p(v), _p(g), q.stride()[0], _p(positions), _p(cos), _p(sin), rotary_dim, _p(decay),
                                           ctypes.c_float(key_scale), ctypes.c_float(eps), _p(state), _p(slots), _p(cu_q), cu_q.numel() - 1, heads,
-                                          head_dim, value_dim, _p(out), out.stride(0) if out is not None else 0, ctypes.c_float(out_scale),
+                                          head_dim, value_dim, _p(out), out.stride()[0] if out is not None else 0, ctypes.c_float(out_scale),
                                           max_q_len, _p(starts), activation_code(input_activation) if input_activation is not None else -1,
-                                          _p(raw_out), raw_out.stride(0) if raw_out is not None else 0, _stream()))
+                                          _p(raw_out), raw_out.stride()[0] if raw_out is not None else 0, _stream()))
         _launches[0] += 2  # three kernels
         return
     lib = retention_library()
@@ -1290,12 +1293,12 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.T
     lib.mb_retention_scratch_floats.restype = ctypes.c_size_t
     floats = lib.mb_retention_scratch_floats(sequences, heads, head_dim, value_dim, max_q_len, run_length)
     scratch = torch.empty((floats,), dtype=torch.float32, device=q.device) if floats else None
-    _run(lib, lib.mb_retention_scan(_p(q), _p(k), _p(v), _p(g), q.stride(0), _code(q.dtype), _p(positions), _p(cos), _p(sin),
+    _run(lib, lib.mb_retention_scan(_p(q), _p(k), _p(v), _p(g), q.stride()[0], _code(q.dtype), _p(positions), _p(cos), _p(sin),
                                     rotary_dim, _p(decay), ctypes.c_float(key_scale), ctypes.c_float(eps), _p(state), _p(slots),
-                                    _p(cu_q), sequences, heads, head_dim, value_dim, _p(out), out.stride(0) if out is not None else 0,
+                                    _p(cu_q), sequences, heads, head_dim, value_dim, _p(out), out.stride()[0] if out is not None else 0,
                                     ctypes.c_float(out_scale), max_q_len, run_length, _p(scratch),
                                     activation_code(input_activation) if input_activation is not None else -1, _p(raw_out),
-                                    raw_out.stride(0) if raw_out is not None else 0, _stream()))
+                                    raw_out.stride()[0] if raw_out is not None else 0, _stream()))
     if floats:
         _launches[0] += 2  # three kernels
 
@@ -1316,7 +1319,7 @@ def group_norm_gate(raw: torch.Tensor, gain: torch.Tensor, gate: torch.Tensor, o
     if gain.dtype != torch.float32 or gain.numel() != width or not gain.is_contiguous():
         raise KernelError(f"group_norm_gate: gain must be contiguous float32 of {width} elements")
     lib = retention_library()
-    _run(lib, lib.mb_group_norm_gate(_p(raw), raw.stride(0), _p(gain), _p(gate), gate.stride(0), _p(out), out.stride(0),
+    _run(lib, lib.mb_group_norm_gate(_p(raw), raw.stride()[0], _p(gain), _p(gate), gate.stride()[0], _p(out), out.stride()[0],
                                      _code(out.dtype), rows, width, ctypes.c_float(eps), 1 if gate_activation == "sigmoid" else 0,
                                      _stream()))
 
@@ -1340,7 +1343,7 @@ def mingru_scan(zin: torch.Tensor, xin: torch.Tensor, gin: torch.Tensor, z_bias:
         _columns(t, name)
         if t.shape != zin.shape or t.shape[1] != width or t.dtype != zin.dtype:
             raise KernelError(f"mingru_scan: {name} is {tuple(t.shape)} {t.dtype}; [{zin.shape[0]}, {width}] {zin.dtype} is needed")
-    if not (zin.stride(0) == xin.stride(0) == gin.stride(0)):
+    if not (zin.stride()[0] == xin.stride()[0] == gin.stride()[0]):
         raise KernelError("mingru_scan: zin, xin and gin must share one row stride")
     if state.dtype != torch.float32 or not state.is_contiguous():
         raise KernelError("mingru_scan: the state must be contiguous float32 [slots, width]")
@@ -1348,8 +1351,8 @@ def mingru_scan(zin: torch.Tensor, xin: torch.Tensor, gin: torch.Tensor, z_bias:
         if t.dtype != torch.float32 or t.numel() != width or not t.is_contiguous():
             raise KernelError(f"mingru_scan: {name} must be contiguous float32 of {width} elements")
     lib = gated_recurrence_library()
-    _run(lib, lib.mb_mingru_scan(_p(zin), _p(xin), _p(gin), zin.stride(0), _code(zin.dtype), _p(z_bias), _p(x_bias), _p(state),
-                                 _p(slots), _p(cu_q), cu_q.numel() - 1, max_q_len, width, _p(out), out.stride(0),
+    _run(lib, lib.mb_mingru_scan(_p(zin), _p(xin), _p(gin), zin.stride()[0], _code(zin.dtype), _p(z_bias), _p(x_bias), _p(state),
+                                 _p(slots), _p(cu_q), cu_q.numel() - 1, max_q_len, width, _p(out), out.stride()[0],
                                  ctypes.c_float(out_scale), _stream()))
 
 
@@ -1382,9 +1385,9 @@ def gated_delta_chunks_takes(conv: torch.Tensor, gate_in: torch.Tensor, gain: to
     """Steps of many tokens a sequence, key heads of 64 numbers and value heads of 64 or 128, rows of whole fours that start on one's boundary;
     `parts_at`: the first columns of the convolved rows' parts."""
     return (max_q_len >= DELTA_CHUNK_MIN_ROWS and conv.shape[0] >= DELTA_CHUNK_MIN_MEAN * sequences and dim == 64 and vdim in (64, 128)
-            and conv.stride(0) % 4 == 0 and conv.data_ptr() % 16 == 0
+            and conv.stride()[0] % 4 == 0 and conv.data_ptr() % 16 == 0
             and all(at % 4 == 0 for at in parts_at) and gain.data_ptr() % 16 == 0
-            and all(t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0 for t in (gate_in, out)))
+            and all(t.stride()[0] % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0 for t in (gate_in, out)))
 
 
 CONV_ACTIVATIONS = {None: 0, "silu": 1}
@@ -1426,8 +1429,8 @@ def short_conv(x: torch.Tensor, weights: torch.Tensor, state: torch.Tensor, stat
         raise KernelError(f"short_conv: {channels} channels are no whole blocks of {split_per}")
     split = torch.empty((x.shape[0], 2 * channels), dtype=torch.bfloat16, device=x.device) if split_per else None
     lib = gated_delta_library()
-    _run(lib, lib.mb_short_conv(_p(x), x.stride(0), _code(x.dtype), _p(in_bias), _p(weights), _p(out_bias), CONV_ACTIVATIONS[activation],
-                                _p(out), out.stride(0), _code(out_dtype), tail, stride, _p(slots), _p(cu_q), cu_q.numel() - 1, max_q_len, channels, taps,
+    _run(lib, lib.mb_short_conv(_p(x), x.stride()[0], _code(x.dtype), _p(in_bias), _p(weights), _p(out_bias), CONV_ACTIVATIONS[activation],
+                                _p(out), out.stride()[0], _code(out_dtype), tail, stride, _p(slots), _p(cu_q), cu_q.numel() - 1, max_q_len, channels, taps,
                                 1 if store_tail else 0, _p(split), int(split_per), _stream()))
     return (out, split) if split_per else out
 
@@ -1448,13 +1451,13 @@ def gated_delta_scan(conv: torch.Tensor, q_at: int, k_at: int, v_at: int, a_in: 
     _int32(slots, "slots")
     _int32(cu_q, "cu_q")
     tokens = conv.shape[0]
-    if conv.dtype != torch.float32 or conv.stride(1) != 1 or max(q_at, k_at) + kv_heads * dim > conv.shape[1] or v_at + heads * vdim > conv.shape[1]:
+    if conv.dtype != torch.float32 or conv.stride()[1] != 1 or max(q_at, k_at) + kv_heads * dim > conv.shape[1] or v_at + heads * vdim > conv.shape[1]:
         raise KernelError(f"gated_delta_scan: the convolved rows {tuple(conv.shape)} {conv.dtype} do not hold the q, k and v parts")
     for name, t, width in (("a_in", a_in, heads), ("b_in", b_in, heads), ("gate_in", gate_in, heads * vdim), ("out", out, heads * vdim)):
         _columns(t, name)
         if tuple(t.shape) != (tokens, width) or t.dtype != out.dtype:
             raise KernelError(f"gated_delta_scan: {name} is {tuple(t.shape)} {t.dtype}; [{tokens}, {width}] {out.dtype} is needed")
-    if not (a_in.stride(0) == b_in.stride(0) == gate_in.stride(0)):
+    if not (a_in.stride()[0] == b_in.stride()[0] == gate_in.stride()[0]):
         raise KernelError("gated_delta_scan: a_in, b_in and gate_in must share one row stride")
     for name, t, n in (("decay", decay, heads), ("dt_bias", dt_bias, heads), ("gain", gain, vdim)):
         if t.dtype != torch.float32 or t.numel() != n or not t.is_contiguous():
@@ -1464,17 +1467,17 @@ def gated_delta_scan(conv: torch.Tensor, q_at: int, k_at: int, v_at: int, a_in: 
     if 4 * floats <= DELTA_CHUNK_BYTES and gated_delta_chunks_takes(conv, gate_in, gain, out, dim, vdim, (q_at, k_at, v_at), max_q_len, cu_q.numel() - 1):
         lib = gated_delta_chunks_library()
         scratch = torch.empty((floats,), dtype=torch.float32, device=conv.device)
-        _run(lib, lib.mb_gated_delta_chunks(_p(conv), conv.stride(0), _p(a_in), _p(b_in), _p(gate_in), a_in.stride(0), _code(out.dtype), _p(decay),
+        _run(lib, lib.mb_gated_delta_chunks(_p(conv), conv.stride()[0], _p(a_in), _p(b_in), _p(gate_in), a_in.stride()[0], _code(out.dtype), _p(decay),
                                             _p(dt_bias), _p(gain), ctypes.c_float(unit_eps), ctypes.c_float(eps), rows, stride, _p(slots),
-                                            _p(cu_q), cu_q.numel() - 1, tokens, int(max_q_len), _p(scratch), _p(out), out.stride(0),
+                                            _p(cu_q), cu_q.numel() - 1, tokens, int(max_q_len), _p(scratch), _p(out), out.stride()[0],
                                             ctypes.c_float(out_scale), heads, kv_heads, dim, vdim, q_at, k_at, v_at, _stream()))
         _launches[0] += 2  # three kernels: the chunks' systems, the carried states, the results
         return
     raw = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=conv.device)  # the read-outs, between the walk and the norm
     lib = gated_delta_library()
-    _run(lib, lib.mb_gated_delta_scan(_p(conv), conv.stride(0), _p(a_in), _p(b_in), _p(gate_in), a_in.stride(0), _code(out.dtype), _p(decay),
+    _run(lib, lib.mb_gated_delta_scan(_p(conv), conv.stride()[0], _p(a_in), _p(b_in), _p(gate_in), a_in.stride()[0], _code(out.dtype), _p(decay),
                                       _p(dt_bias), _p(gain), ctypes.c_float(unit_eps), ctypes.c_float(eps), rows, stride, _p(slots),
-                                      _p(cu_q), cu_q.numel() - 1, tokens, _p(raw), _p(out), out.stride(0), ctypes.c_float(out_scale), heads,
+                                      _p(cu_q), cu_q.numel() - 1, tokens, _p(raw), _p(out), out.stride()[0], ctypes.c_float(out_scale), heads,
                                       kv_heads, dim, vdim, q_at, k_at, v_at, _stream()))
     _launches[0] += 2  # three kernels: unit vectors, the walk, norm and gate
 
@@ -1500,7 +1503,7 @@ def state_space_walk(rows: torch.Tensor, x_at: int, b_at: int, c_at: int, dt_in:
     at, stride = _state_rows(state, state_offset, heads * state_rows * vdim, "state_space_walk")
     y = torch.empty((rows.shape[0], heads * vdim), dtype=torch.float32, device=rows.device)
     lib = state_space_library()
-    _run(lib, lib.mb_state_space_walk(_p(rows), rows.stride(0), _code(rows.dtype), _p(dt_in), dt_in.stride(0), _code(dt_in.dtype), _p(decay),
+    _run(lib, lib.mb_state_space_walk(_p(rows), rows.stride()[0], _code(rows.dtype), _p(dt_in), dt_in.stride()[0], _code(dt_in.dtype), _p(decay),
                                       _p(dt_bias), _p(skip), at, stride, _p(slots), _p(cu_q), cu_q.numel() - 1, _p(y), heads, groups,
                                       state_rows, vdim, x_at, b_at, c_at, _stream()))
     return y
@@ -1540,7 +1543,7 @@ def state_space_chunks(rows: torch.Tensor, x_at: int, b_at: int, c_at: int, dt_i
     added = torch.empty((places, heads, state_rows * vdim), dtype=torch.float32, device=device)
     starts = torch.empty((2, places, heads, state_rows * vdim), dtype=torch.bfloat16, device=device)
     keep = torch.empty((places, heads), dtype=torch.float32, device=device)
-    _run(lib, lib.mb_state_space_chunks(_p(rows), rows.stride(0), _p(dt_in), dt_in.stride(0), _p(decay), _p(dt_bias), _p(skip), at, stride,
+    _run(lib, lib.mb_state_space_chunks(_p(rows), rows.stride()[0], _p(dt_in), dt_in.stride()[0], _p(decay), _p(dt_bias), _p(skip), at, stride,
                                         _p(slots), _p(cu_q), sequences, max_q_len, _p(y), _p(added), _p(starts[0]), _p(starts[1]), _p(keep),
                                         heads, groups, x_at, b_at, c_at, _stream()))
     _launches[0] += 2  # three kernels
@@ -1567,7 +1570,7 @@ def gate_part_norm(y: torch.Tensor, z: torch.Tensor, gain: torch.Tensor, eps: fl
         raise KernelError(f"gate_part_norm: y {tuple(y.shape)}, z {tuple(z.shape)} and out {tuple(out.shape)} do not fit {parts} parts")
     _vectors(y.shape[1], "gate_part_norm", gain=gain)
     lib = state_space_library()
-    _run(lib, lib.mb_gate_part_norm(_p(y), _code(y.dtype), _p(z), z.stride(0), _p(gain), ctypes.c_float(eps), _p(out), out.stride(0),
+    _run(lib, lib.mb_gate_part_norm(_p(y), _code(y.dtype), _p(z), z.stride()[0], _p(gain), ctypes.c_float(eps), _p(out), out.stride()[0],
                                     _code(out.dtype), ctypes.c_float(out_scale), y.shape[0], y.shape[1], parts, _stream()))
 
 
@@ -1583,7 +1586,7 @@ def rglru_scan(gates: torch.Tensor, per: int, u: torch.Tensor, y_in: torch.Tenso
     _int32(slots, "slots")
     _int32(cu_q, "cu_q")
     tokens, width = u.shape
-    if gates.dtype != torch.float32 or u.dtype != torch.float32 or gates.stride(1) != 1 or u.stride(1) != 1 or tuple(gates.shape) != (tokens, 2 * width):
+    if gates.dtype != torch.float32 or u.dtype != torch.float32 or gates.stride()[1] != 1 or u.stride()[1] != 1 or tuple(gates.shape) != (tokens, 2 * width):
         raise KernelError(f"rglru_scan: gates {tuple(gates.shape)} and u {tuple(u.shape)} must be float32 [tokens, 2 * width] and [tokens, width]")
     for name, t in (("y_in", y_in), ("out", out)):
         _columns(t, name)
@@ -1594,9 +1597,9 @@ def rglru_scan(gates: torch.Tensor, per: int, u: torch.Tensor, y_in: torch.Tenso
             raise KernelError(f"rglru_scan: {name} must be contiguous float32 of {width} elements")
     rows, stride = _state_rows(state, state_offset, width, "rglru_scan")
     lib = gated_recurrence_library()
-    _run(lib, lib.mb_rglru_scan(_p(gates), gates.stride(0), int(per), _p(u), u.stride(0), _p(y_in), y_in.stride(0), _code(out.dtype),
+    _run(lib, lib.mb_rglru_scan(_p(gates), gates.stride()[0], int(per), _p(u), u.stride()[0], _p(y_in), y_in.stride()[0], _code(out.dtype),
                                 _p(r_bias), _p(i_bias), _p(y_bias), _p(rate), rows, stride, _p(slots), _p(cu_q), cu_q.numel() - 1,
-                                max_q_len, width, _p(out), out.stride(0), ctypes.c_float(out_scale), _stream()))
+                                max_q_len, width, _p(out), out.stride()[0], ctypes.c_float(out_scale), _stream()))
 
 
 def _check_paged(q, out, k_pool, v_pool, block_table, cu_q, kv_lens, kv_heads, head_dim):
@@ -1604,7 +1607,7 @@ def _check_paged(q, out, k_pool, v_pool, block_table, cu_q, kv_lens, kv_heads, h
     _int32(block_table, "block_table")
     _int32(cu_q, "cu_q")
     _int32(kv_lens, "kv_lens")
-    if q.stride(1) != 1 or out.stride(1) != 1:
+    if q.stride()[1] != 1 or out.stride()[1] != 1:
         raise KernelError("q and out need unit column stride")
     if k_pool.dim() != 4 or k_pool.shape[1] != kv_heads or k_pool.shape[3] != head_dim or not k_pool.is_contiguous():
         raise KernelError(f"k_pool must be contiguous [pages, {kv_heads}, page_size, {head_dim}], got {tuple(k_pool.shape)}")
@@ -1712,7 +1715,7 @@ def decode_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v
     if splits > 1 and (use_scratch or splits not in (2, 4, 8)):
         lib.mb_decode_scratch_floats.restype = ctypes.c_size_t
         scratch = torch.empty((lib.mb_decode_scratch_floats(sequences, heads, splits),), dtype=torch.float32, device=q.device)
-    _run(lib, lib.mb_decode_attention(_p(q), q.stride(0), _p(out), out.stride(0), _p(k_pool), _p(v_pool),
+    _run(lib, lib.mb_decode_attention(_p(q), q.stride()[0], _p(out), out.stride()[0], _p(k_pool), _p(v_pool),
                                       _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_lens), sequences, heads,
                                       kv_heads, k_pool.shape[2], window or 0, ctypes.c_float(scale), splits,
                                       _p(scratch), _stream()))
@@ -1734,12 +1737,12 @@ def prefill_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, 
             raise KernelError(f"the tcgen05 prefill attention is built for head sizes 64 and 128, got {head_dim}")
         lib = prefill_attention_tc(head_dim)
         _run(lib, lib.mb_prefill_attention_tcgen05(
-            _p(q), q.stride(0), q.shape[0], _p(out), out.stride(0), _p(k_pool), _p(v_pool), k_pool.shape[0],
+            _p(q), q.stride()[0], q.shape[0], _p(out), out.stride()[0], _p(k_pool), _p(v_pool), k_pool.shape[0],
             _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_lens), kv_lens.numel(), max_q_len, heads, kv_heads,
             k_pool.shape[2], window or 0, ctypes.c_float(scale), _stream()))
         return
     lib = attention_tc(head_dim)
-    _run(lib, lib.mb_prefill_attention(_p(q), q.stride(0), _p(out), out.stride(0), _p(k_pool), _p(v_pool),
+    _run(lib, lib.mb_prefill_attention(_p(q), q.stride()[0], _p(out), out.stride()[0], _p(k_pool), _p(v_pool),
                                        _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_lens), kv_lens.numel(),
                                        max_q_len, heads, kv_heads, k_pool.shape[2], window or 0, ctypes.c_float(scale),
                                        _stream()))
@@ -1754,7 +1757,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, row_invariant: bool = True, weigh
     _cuda(a, w)
     if a.dtype != torch.float32 or w.dtype != torch.float32:
         raise KernelError(f"gemm_f32 takes float32 operands, got {a.dtype} and {w.dtype}")
-    if a.dim() != 2 or w.dim() != 2 or a.shape[1] != w.shape[1] or a.stride(1) != 1 or w.stride(1) != 1:
+    if a.dim() != 2 or w.dim() != 2 or a.shape[1] != w.shape[1] or a.stride()[1] != 1 or w.stride()[1] != 1:
         raise KernelError(f"gemm_f32: shapes {tuple(a.shape)} x {tuple(w.shape)}^T do not fit")
     m, k = a.shape
     n = w.shape[0]
@@ -1763,7 +1766,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, row_invariant: bool = True, weigh
     lib.mb_gemm_f32_scratch.restype = ctypes.c_size_t
     need = lib.mb_gemm_f32_scratch(m, k)
     scratch = torch.empty((need,), dtype=torch.uint8, device=a.device) if need else None
-    _run(lib, lib.mb_gemm_f32(_p(a), a.stride(0), _p(w), w.stride(0), _p(c), n, m, n, k, _p(scratch), 1 if weights_ready else 0, _stream()))
+    _run(lib, lib.mb_gemm_f32(_p(a), a.stride()[0], _p(w), w.stride()[0], _p(c), n, m, n, k, _p(scratch), 1 if weights_ready else 0, _stream()))
     return c
 
 
@@ -1777,8 +1780,8 @@ def skinny():
 
 def skinny_takes(weight: torch.Tensor, rows: int, with_norm: bool = False) -> bool:
     """Whether the decode matrix product takes this weight with this many activation rows."""
-    return (weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.stride(1) == 1 and weight.shape[1] % 8 == 0
-            and weight.stride(0) % 8 == 0 and weight.data_ptr() % 16 == 0
+    return (weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.stride()[1] == 1 and weight.shape[1] % 8 == 0
+            and weight.stride()[0] % 8 == 0 and weight.data_ptr() % 16 == 0
             and 0 < rows <= (SKINNY_NORM_ROWS if with_norm else SKINNY_ROWS))
 
 
@@ -1823,14 +1826,14 @@ def skinny_gemm(weight: torch.Tensor, epilogue: int, x: Optional[torch.Tensor] =
     n, k = weight.shape
     norm = gain is not None
     if norm:
-        if xf is None or xf.dtype != torch.float32 or xf.stride(1) != 1 or xf.shape[1] != k:
+        if xf is None or xf.dtype != torch.float32 or xf.stride()[1] != 1 or xf.shape[1] != k:
             raise KernelError("the norm prologue needs float32 rows of the weight's width")
         if gain.dtype != torch.float32 or gain.numel() != k:
             raise KernelError("the norm gain must be float32 of the weight's width")
         _int32(rows, "rows")
         batch = rows.numel() if rows is not None else xf.shape[0]
     else:
-        if x is None or x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.shape[1] != k:
+        if x is None or x.dtype != torch.bfloat16 or x.stride()[1] != 1 or x.shape[1] != k:
             raise KernelError("activations must be bfloat16 rows of the weight's width")
         batch = x.shape[0]
     if not skinny_takes(weight, batch, norm):
@@ -1838,7 +1841,7 @@ def skinny_gemm(weight: torch.Tensor, epilogue: int, x: Optional[torch.Tensor] =
     kind = epilogue & 0xFF  # a gated epilogue carries its activation above
     out_cols = n // 2 if kind == EPI_SWIGLU else n
     if kind == EPI_RESIDUAL:
-        if out is None or out.dtype != torch.float32 or out.shape != (batch, n) or out.stride(1) != 1:
+        if out is None or out.dtype != torch.float32 or out.shape != (batch, n) or out.stride()[1] != 1:
             raise KernelError("the residual epilogue adds into a float32 [rows, n] tensor")
     elif out is None:
         out = torch.empty((batch, out_cols), dtype=torch.float32 if kind == EPI_F32 else torch.bfloat16,
@@ -1854,11 +1857,11 @@ def skinny_gemm(weight: torch.Tensor, epilogue: int, x: Optional[torch.Tensor] =
         emit_rows = _emitted_rows(kind, emit_gain, emit_rows, batch, n, weight.device)
         emit_ssq = torch.empty((-(-n // 16), SSQ_COLUMNS), dtype=torch.float32, device=weight.device)
     lib = skinny()
-    _run(lib, lib.mb_skinny_gemm(_p(weight), weight.stride(0), n, k, batch, _p(x), x.stride(0) if x is not None else 0,
-                                 _p(xf), xf.stride(0) if xf is not None else 0, _p(gain),
+    _run(lib, lib.mb_skinny_gemm(_p(weight), weight.stride()[0], n, k, batch, _p(x), x.stride()[0] if x is not None else 0,
+                                 _p(xf), xf.stride()[0] if xf is not None else 0, _p(gain),
                                  part_eps if norm_parts is not None else ctypes.c_float(eps), _p(rows),
-                                 _p(out), out.stride(0), epilogue, _sm_count(weight.device), 1, ssq, count, _p(emit_gain),
-                                 _p(emit_rows), emit_rows.stride(0) if emit_rows is not None else 0, _p(emit_ssq),
+                                 _p(out), out.stride()[0], epilogue, _sm_count(weight.device), 1, ssq, count, _p(emit_gain),
+                                 _p(emit_rows), emit_rows.stride()[0] if emit_rows is not None else 0, _p(emit_ssq),
                                  ctypes.byref(written), _clamp_args(epilogue, clamp), _stream()))
     if emit_gain is not None:
         return out, emit_rows, emit_ssq, written.value
@@ -1872,7 +1875,7 @@ def _emitted_rows(kind: int, emit_gain: torch.Tensor, emit_rows: Optional[torch.
     if emit_rows is None:
         return torch.empty((batch, n), dtype=torch.bfloat16, device=device)
     _columns(emit_rows, "emit_rows")
-    if emit_rows.dtype != torch.bfloat16 or tuple(emit_rows.shape) != (batch, n) or emit_rows.stride(0) % 4 or emit_rows.data_ptr() % 8:
+    if emit_rows.dtype != torch.bfloat16 or tuple(emit_rows.shape) != (batch, n) or emit_rows.stride()[0] % 4 or emit_rows.data_ptr() % 8:
         raise KernelError(f"the next norm's rows need an aligned bfloat16 slice [{batch}, {n}], got {tuple(emit_rows.shape)} {emit_rows.dtype}")
     return emit_rows
 
@@ -1887,11 +1890,11 @@ def skinny_gemm_pairs(weight: torch.Tensor, plain_rows: int, mid: torch.Tensor, 
     n, k = weight.shape
     norm = gain is not None
     if norm:
-        if xf is None or xf.dtype != torch.float32 or xf.stride(1) != 1 or xf.shape[1] != k or gain.dtype != torch.float32 or gain.numel() != k:
+        if xf is None or xf.dtype != torch.float32 or xf.stride()[1] != 1 or xf.shape[1] != k or gain.dtype != torch.float32 or gain.numel() != k:
             raise KernelError("the norm prologue needs float32 rows and a float32 gain of the weight's width")
         if norm_parts is not None:
             raise KernelError("a product normalises float32 rows itself or takes rows with parts of their sums of squares, not both")
-    elif x is None or x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.shape[1] != k:
+    elif x is None or x.dtype != torch.bfloat16 or x.stride()[1] != 1 or x.shape[1] != k:
         raise KernelError("activations must be bfloat16 rows of the weight's width")
     batch = (xf if norm else x).shape[0]
     _columns(mid, "mid")
@@ -1907,9 +1910,9 @@ def skinny_gemm_pairs(weight: torch.Tensor, plain_rows: int, mid: torch.Tensor, 
         raise KernelError("the norm's width is the product's k")
     out = torch.empty((batch, plain_rows), dtype=torch.bfloat16, device=weight.device)
     lib = skinny()
-    _run(lib, lib.mb_skinny_gemm_pairs(_p(weight), weight.stride(0), int(plain_rows), pairs, k, batch, _p(x), x.stride(0) if x is not None else 0,
-                                       _p(xf), xf.stride(0) if xf is not None else 0, _p(gain), part_eps, _p(out), out.stride(0), _p(mid),
-                                       mid.stride(0), EPI_CLAMPED >> 8, _clamp_args(EPI_CLAMPED, clamp), _sm_count(weight.device), 1, ssq, count,
+    _run(lib, lib.mb_skinny_gemm_pairs(_p(weight), weight.stride()[0], int(plain_rows), pairs, k, batch, _p(x), x.stride()[0] if x is not None else 0,
+                                       _p(xf), xf.stride()[0] if xf is not None else 0, _p(gain), part_eps, _p(out), out.stride()[0], _p(mid),
+                                       mid.stride()[0], EPI_CLAMPED >> 8, _clamp_args(EPI_CLAMPED, clamp), _sm_count(weight.device), 1, ssq, count,
                                        _stream()))
     return out
 
@@ -1921,17 +1924,17 @@ def skinny_gemm_gated_residual(weight: torch.Tensor, x: torch.Tensor, out: torch
     _cuda(weight, x, out, gate, bias)
     n, k = weight.shape
     batch = x.shape[0]
-    if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.shape[1] != k or not skinny_takes(weight, batch):
+    if x.dtype != torch.bfloat16 or x.stride()[1] != 1 or x.shape[1] != k or not skinny_takes(weight, batch):
         raise KernelError(f"skinny_gemm_gated_residual does not take a {tuple(weight.shape)} weight with {tuple(x.shape)} {x.dtype} rows")
-    if out.dtype != torch.float32 or tuple(out.shape) != (batch, n) or out.stride(1) != 1:
+    if out.dtype != torch.float32 or tuple(out.shape) != (batch, n) or out.stride()[1] != 1:
         raise KernelError("the residual epilogue adds into a float32 [rows, n] tensor")
     _columns(gate, "gate")
     if gate.dtype != torch.bfloat16 or tuple(gate.shape) != (batch, n) or bias.dtype != torch.float32 or bias.numel() != n \
             or not bias.is_contiguous():
         raise KernelError("the gate must be bfloat16 [rows, n] and its bias float32 [n]")
     lib = skinny()
-    _run(lib, lib.mb_skinny_gemm_gated_residual(_p(weight), weight.stride(0), n, k, batch, _p(x), x.stride(0), _p(out), out.stride(0),
-                                                _p(gate), gate.stride(0), _p(bias), _sm_count(weight.device), 1, _stream()))
+    _run(lib, lib.mb_skinny_gemm_gated_residual(_p(weight), weight.stride()[0], n, k, batch, _p(x), x.stride()[0], _p(out), out.stride()[0],
+                                                _p(gate), gate.stride()[0], _p(bias), _sm_count(weight.device), 1, _stream()))
 
 
 def skinny_gemm_tanh_residual(weight: torch.Tensor, x: torch.Tensor, out: torch.Tensor, alpha: float, norm_weight: torch.Tensor,
@@ -1941,7 +1944,7 @@ def skinny_gemm_tanh_residual(weight: torch.Tensor, x: torch.Tensor, out: torch.
     _cuda(weight, x, out, norm_weight, norm_bias)
     n, k = weight.shape
     batch = x.shape[0]
-    if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.shape[1] != k or not skinny_takes(weight, batch):
+    if x.dtype != torch.bfloat16 or x.stride()[1] != 1 or x.shape[1] != k or not skinny_takes(weight, batch):
         raise KernelError(f"skinny_gemm_tanh_residual does not take a {tuple(weight.shape)} weight with {tuple(x.shape)} {x.dtype} rows")
     _stream_rows(out, "skinny_gemm_tanh_residual")
     if tuple(out.shape) != (batch, n):
@@ -1949,7 +1952,7 @@ def skinny_gemm_tanh_residual(weight: torch.Tensor, x: torch.Tensor, out: torch.
     _vectors(n, "skinny_gemm_tanh_residual", weight=norm_weight, bias=norm_bias)
     (kind, then_alpha, then_weight, then_bias, rows_at, _), rows = _then_args(out, then, torch.bfloat16, "skinny_gemm_tanh_residual")
     lib = skinny()
-    _run(lib, lib.mb_skinny_gemm_tanh_residual(_p(weight), weight.stride(0), n, k, batch, _p(x), x.stride(0), _p(out), out.stride(0),
+    _run(lib, lib.mb_skinny_gemm_tanh_residual(_p(weight), weight.stride()[0], n, k, batch, _p(x), x.stride()[0], _p(out), out.stride()[0],
                                                ctypes.c_float(alpha), _p(norm_weight), _p(norm_bias), kind, then_alpha, then_weight, then_bias,
                                                rows_at, n, _sm_count(weight.device), 1, _stream()))
     return rows
@@ -1961,13 +1964,13 @@ def skinny_gemm_side(weight: torch.Tensor, x: torch.Tensor, table: torch.Tensor,
     _int32(tokens, "tokens")
     n, k = weight.shape
     batch = x.shape[0]
-    if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.shape[1] != k or not skinny_takes(weight, batch) or n != columns:
+    if x.dtype != torch.bfloat16 or x.stride()[1] != 1 or x.shape[1] != k or not skinny_takes(weight, batch) or n != columns:
         raise KernelError(f"skinny_gemm_side does not take a {tuple(weight.shape)} weight with {tuple(x.shape)} {x.dtype} rows")
     if table.dtype != torch.bfloat16 or table.dim() != 2 or not table.is_contiguous() or table.shape[1] > n or tokens.numel() != batch:
         raise KernelError(f"skinny_gemm_side: the table {tuple(table.shape)} {table.dtype} does not fit {n} columns")
     out = torch.empty((batch, n), dtype=torch.bfloat16, device=weight.device)
     lib = skinny()
-    _run(lib, lib.mb_skinny_gemm_side(_p(weight), weight.stride(0), n, k, batch, _p(x), x.stride(0), _p(out), n, _p(table), _p(tokens),
+    _run(lib, lib.mb_skinny_gemm_side(_p(weight), weight.stride()[0], n, k, batch, _p(x), x.stride()[0], _p(out), n, _p(table), _p(tokens),
                                       table.shape[1], _sm_count(weight.device), 1, _stream()))
     return out
 
@@ -1987,9 +1990,9 @@ def skinny_qkv_rope(weight: torch.Tensor, xf: Optional[torch.Tensor], gain: Opti
     batch, k = (xf if xf is not None else x).shape
     if weight.shape != ((heads + 2 * kv_heads) * head_dim, k) or not skinny_takes(weight, batch, True):
         raise KernelError(f"skinny_qkv_rope does not take a {tuple(weight.shape)} {weight.dtype} weight with {batch} rows")
-    if xf is not None and (xf.dtype != torch.float32 or xf.stride(1) != 1 or gain.dtype != torch.float32 or gain.numel() != k):
+    if xf is not None and (xf.dtype != torch.float32 or xf.stride()[1] != 1 or gain.dtype != torch.float32 or gain.numel() != k):
         raise KernelError("skinny_qkv_rope needs float32 residual rows and gain")
-    if x is not None and (x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or norm_parts[2] != k):
+    if x is not None and (x.dtype != torch.bfloat16 or x.stride()[1] != 1 or x.stride()[0] % 8 or x.data_ptr() % 16 or norm_parts[2] != k):
         raise KernelError("skinny_qkv_rope needs aligned bfloat16 rows of the weight's width")
     _int32(positions, "positions")
     _int32(slot_mapping, "slot_mapping")
@@ -2000,9 +2003,9 @@ def skinny_qkv_rope(weight: torch.Tensor, xf: Optional[torch.Tensor], gain: Opti
     q = torch.empty((batch, heads * head_dim), dtype=torch.bfloat16, device=weight.device)
     ssq, count, _, _, part_eps = _norm_args(norm_parts, batch, SSQ_COLUMNS)
     lib = skinny()
-    _run(lib, lib.mb_skinny_qkv_rope(_p(weight), weight.stride(0), k, batch, _p(x), x.stride(0) if x is not None else 0, _p(xf),
-                                     xf.stride(0) if xf is not None else 0, _p(gain),
-                                     part_eps if norm_parts is not None else ctypes.c_float(eps), _p(q), q.stride(0), heads,
+    _run(lib, lib.mb_skinny_qkv_rope(_p(weight), weight.stride()[0], k, batch, _p(x), x.stride()[0] if x is not None else 0, _p(xf),
+                                     xf.stride()[0] if xf is not None else 0, _p(gain),
+                                     part_eps if norm_parts is not None else ctypes.c_float(eps), _p(q), q.stride()[0], heads,
                                      kv_heads, head_dim, _p(positions), _p(cos), _p(sin), _p(k_pool), _p(v_pool),
                                      _p(slot_mapping), k_pool.shape[2], _sm_count(weight.device), 1, ssq, count, _stream()))
     return q
@@ -2024,8 +2027,8 @@ def gemm_tcgen05_takes(weight: torch.Tensor, epilogue: int = EPI_BF16, rows: Opt
     n = weight.shape[0] // 2 if epilogue == EPI_SWIGLU else weight.shape[0]
     if rows is not None and rows < TCGEN05_MIN_ROWS:
         return False
-    return (weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.stride(1) == 1 and weight.shape[1] % 8 == 0
-            and weight.stride(0) % 8 == 0 and weight.data_ptr() % 16 == 0 and n % 8 == 0
+    return (weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.stride()[1] == 1 and weight.shape[1] % 8 == 0
+            and weight.stride()[0] % 8 == 0 and weight.data_ptr() % 16 == 0 and n % 8 == 0
             and (epilogue != EPI_SWIGLU or weight.shape[0] % 2 == 0))
 
 
@@ -2043,16 +2046,16 @@ def gemm_tcgen05(a: torch.Tensor, weight: torch.Tensor, epilogue: int = EPI_BF16
     result is the same bits in every run; `arrival_order` lets each part add into `out` as it finishes
     instead (a little quicker, the last bit of an element then depends on timing)."""
     _cuda(a, weight, out)
-    if a.dtype != torch.bfloat16 or a.dim() != 2 or a.stride(1) != 1 or a.shape[1] != weight.shape[1]:
+    if a.dtype != torch.bfloat16 or a.dim() != 2 or a.stride()[1] != 1 or a.shape[1] != weight.shape[1]:
         raise KernelError(f"gemm_tcgen05: activations {tuple(a.shape)} {a.dtype} do not fit the weight {tuple(weight.shape)}")
-    if not gemm_tcgen05_takes(weight, epilogue) or a.stride(0) % 8 or a.data_ptr() % 16:
+    if not gemm_tcgen05_takes(weight, epilogue) or a.stride()[0] % 8 or a.data_ptr() % 16:
         raise KernelError(f"gemm_tcgen05 does not take a {tuple(weight.shape)} {weight.dtype} weight")
     m, k = a.shape
     n_w = weight.shape[0]
     kind = epilogue & 0xFF
     n = n_w // 2 if kind == EPI_SWIGLU else n_w
     if kind == EPI_RESIDUAL:
-        if out is None or out.dtype != torch.float32 or out.shape != (m, n) or out.stride(1) != 1:
+        if out is None or out.dtype != torch.float32 or out.shape != (m, n) or out.stride()[1] != 1:
             raise KernelError("the residual epilogue adds into a float32 [m, n] tensor")
     elif out is None:
         out = torch.empty((m, n), dtype=torch.float32 if kind == EPI_F32 else torch.bfloat16, device=a.device)
@@ -2068,7 +2071,7 @@ def gemm_tcgen05(a: torch.Tensor, weight: torch.Tensor, epilogue: int = EPI_BF16
         if tickets is None:
             # zero once; every launch leaves the tickets at zero
             tickets = _split_tickets[key] = torch.zeros((need_tickets.value,), dtype=torch.int32, device=a.device)
-    _run(lib, lib.mb_gemm_tcgen05(_p(a), a.stride(0), _p(weight), weight.stride(0), _p(out), out.stride(0), m, n_w, k,
+    _run(lib, lib.mb_gemm_tcgen05(_p(a), a.stride()[0], _p(weight), weight.stride()[0], _p(out), out.stride()[0], m, n_w, k,
                                   epilogue, sms, tile_width, pair, _p(partial), _p(tickets), _clamp_args(epilogue, clamp), _stream()))
     return out
 
@@ -2088,7 +2091,7 @@ def gemm_tcgen05_qkv_rope(a: torch.Tensor, weight: torch.Tensor, heads: int, kv_
     cache write of keys and values.  Returns the rotated queries, bfloat16 [rows, heads * head_dim]."""
     _cuda(a, weight, positions, cos, sin, k_pool, v_pool, slot_mapping)
     m, k = a.shape
-    if a.dtype != torch.bfloat16 or a.stride(1) != 1 or a.stride(0) % 8 or a.data_ptr() % 16 or weight.shape[1] != k:
+    if a.dtype != torch.bfloat16 or a.stride()[1] != 1 or a.stride()[0] % 8 or a.data_ptr() % 16 or weight.shape[1] != k:
         raise KernelError(f"gemm_tcgen05_qkv_rope: activations {tuple(a.shape)} {a.dtype} do not fit the weight {tuple(weight.shape)}")
     if not gemm_tcgen05_qkv_rope_takes(weight, m, heads, kv_heads, head_dim):
         raise KernelError(f"gemm_tcgen05_qkv_rope does not take a {tuple(weight.shape)} {weight.dtype} weight with {m} rows "
@@ -2104,7 +2107,7 @@ def gemm_tcgen05_qkv_rope(a: torch.Tensor, weight: torch.Tensor, heads: int, kv_
         raise KernelError("cache pools must be contiguous bfloat16 [pages, kv_heads, page_size, head_dim]")
     q = torch.empty((m, heads * head_dim), dtype=torch.bfloat16, device=a.device)
     lib = gemm_tc()
-    _run(lib, lib.mb_gemm_tcgen05_qkv_rope(_p(a), a.stride(0), _p(weight), weight.stride(0), _p(q), q.stride(0), m, k, heads,
+    _run(lib, lib.mb_gemm_tcgen05_qkv_rope(_p(a), a.stride()[0], _p(weight), weight.stride()[0], _p(q), q.stride()[0], m, k, heads,
                                            kv_heads, head_dim, _p(positions), _p(cos), _p(sin), _p(k_pool), _p(v_pool),
                                            _p(slot_mapping), k_pool.shape[2], _sm_count(a.device), _stream()))
     return q
@@ -2124,10 +2127,10 @@ def _norm_args(norm_parts, rows: int, columns: Optional[int] = None):
     if norm_parts is None:
         return None, 0, 0, 0, ctypes.c_float(0.0)
     ssq, count, width, eps = norm_parts
-    if (ssq.dtype != torch.float32 or ssq.dim() != 2 or ssq.stride(1) != 1 or ssq.shape[1] < rows or ssq.shape[0] < count or count <= 0
-            or (columns is not None and (ssq.shape[1] != columns or ssq.stride(0) != columns))):
+    if (ssq.dtype != torch.float32 or ssq.dim() != 2 or ssq.stride()[1] != 1 or ssq.shape[1] < rows or ssq.shape[0] < count or count <= 0
+            or (columns is not None and (ssq.shape[1] != columns or ssq.stride()[0] != columns))):
         raise KernelError(f"parts of sums of squares must be a float32 [parts, {columns or 'rows'}] table with a column per row")
-    return _p(ssq), int(count), ssq.stride(0), int(width), ctypes.c_float(eps)
+    return _p(ssq), int(count), ssq.stride()[0], int(width), ctypes.c_float(eps)
 
 
 def wide_gemm(x: torch.Tensor, weight: torch.Tensor, epilogue: int = EPI_BF16, out: Optional[torch.Tensor] = None,
@@ -2143,16 +2146,16 @@ def wide_gemm(x: torch.Tensor, weight: torch.Tensor, epilogue: int = EPI_BF16, o
     `emit_gain` (that norm's gain) it returns (out, rows of the new `out` times the gain as bfloat16, parts of
     their sums of squares, how many parts)."""
     _cuda(x, weight, out, emit_gain)
-    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.stride(1) != 1 or x.shape[1] != weight.shape[1] or x.shape[0] > WIDE_ROWS:
+    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.stride()[1] != 1 or x.shape[1] != weight.shape[1] or x.shape[0] > WIDE_ROWS:
         raise KernelError(f"wide_gemm: activations {tuple(x.shape)} {x.dtype} do not fit the weight {tuple(weight.shape)}")
-    if not gemm_tcgen05_takes(weight, epilogue) or x.stride(0) % 8 or x.data_ptr() % 16:
+    if not gemm_tcgen05_takes(weight, epilogue) or x.stride()[0] % 8 or x.data_ptr() % 16:
         raise KernelError(f"wide_gemm does not take a {tuple(weight.shape)} {weight.dtype} weight")
     batch, k = x.shape
     n_w = weight.shape[0]
     kind = epilogue & 0xFF
     n = n_w // 2 if kind == EPI_SWIGLU else n_w
     if kind == EPI_RESIDUAL:
-        if out is None or out.dtype != torch.float32 or out.shape != (batch, n) or out.stride(1) != 1:
+        if out is None or out.dtype != torch.float32 or out.shape != (batch, n) or out.stride()[1] != 1:
             raise KernelError("the residual epilogue adds into a float32 [rows, n] tensor")
     elif out is None:
         out = torch.empty((batch, n), dtype=torch.float32 if kind == EPI_F32 else torch.bfloat16, device=x.device)
@@ -2163,9 +2166,9 @@ def wide_gemm(x: torch.Tensor, weight: torch.Tensor, epilogue: int = EPI_BF16, o
         emit_ssq = torch.empty((8 * -(-n // 128), SSQ_COLUMNS), dtype=torch.float32, device=x.device)
     ssq, count, _, width, eps = _norm_args(norm_parts, batch, SSQ_COLUMNS)
     lib = wide_gemm_lib()
-    _run(lib, lib.mb_wide_gemm(_p(x), x.stride(0), _p(weight), weight.stride(0), _p(out), out.stride(0), batch, n_w, k,
+    _run(lib, lib.mb_wide_gemm(_p(x), x.stride()[0], _p(weight), weight.stride()[0], _p(out), out.stride()[0], batch, n_w, k,
                                epilogue, _sm_count(x.device), ssq, count, width, eps, _p(emit_gain), _p(emit_rows),
-                               emit_rows.stride(0) if emit_rows is not None else 0, _p(emit_ssq), ctypes.byref(written),
+                               emit_rows.stride()[0] if emit_rows is not None else 0, _p(emit_ssq), ctypes.byref(written),
                                _clamp_args(epilogue, clamp), _stream()))
     if emit_gain is not None:
         return out, emit_rows, emit_ssq, written.value
@@ -2187,7 +2190,7 @@ def wide_qkv_rope(x: torch.Tensor, weight: torch.Tensor, heads: int, kv_heads: i
     Returns the rotated queries, bfloat16 [rows, heads * head_dim].  `norm_parts` as for wide_gemm."""
     _cuda(x, weight, positions, cos, sin, k_pool, v_pool, slot_mapping)
     batch, k = x.shape
-    if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or weight.shape[1] != k:
+    if x.dtype != torch.bfloat16 or x.stride()[1] != 1 or x.stride()[0] % 8 or x.data_ptr() % 16 or weight.shape[1] != k:
         raise KernelError(f"wide_qkv_rope: activations {tuple(x.shape)} {x.dtype} do not fit the weight {tuple(weight.shape)}")
     if not wide_qkv_rope_takes(weight, batch, heads, kv_heads, head_dim):
         raise KernelError(f"wide_qkv_rope does not take a {tuple(weight.shape)} {weight.dtype} weight with {batch} rows and heads of {head_dim}")
@@ -2203,7 +2206,7 @@ def wide_qkv_rope(x: torch.Tensor, weight: torch.Tensor, heads: int, kv_heads: i
     q = torch.empty((batch, heads * head_dim), dtype=torch.bfloat16, device=x.device)
     ssq, count, _, width, eps = _norm_args(norm_parts, batch, SSQ_COLUMNS)
     lib = wide_gemm_lib()
-    _run(lib, lib.mb_wide_qkv_rope(_p(x), x.stride(0), _p(weight), weight.stride(0), _p(q), q.stride(0), batch, k, heads, kv_heads,
+    _run(lib, lib.mb_wide_qkv_rope(_p(x), x.stride()[0], _p(weight), weight.stride()[0], _p(q), q.stride()[0], batch, k, heads, kv_heads,
                                    head_dim, _p(positions), _p(cos), _p(sin), _p(k_pool), _p(v_pool), _p(slot_mapping),
                                    k_pool.shape[2], _sm_count(x.device), ssq, count, width, eps, _stream()))
     return q
@@ -2270,11 +2273,11 @@ def decode_step(lib, step, sms: int) -> None:
 
 def argmax_rows(logits: torch.Tensor) -> torch.Tensor:
     _cuda(logits)
-    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1:
+    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride()[1] != 1:
         raise KernelError("argmax_rows takes float32 [rows, vocab] logits")
     out = torch.empty((logits.shape[0],), dtype=torch.int32, device=logits.device)
     lib = sampling()
-    _run(lib, lib.mb_argmax_rows(_p(logits), logits.stride(0), logits.shape[0], logits.shape[1], _p(out), _stream()))
+    _run(lib, lib.mb_argmax_rows(_p(logits), logits.stride()[0], logits.shape[0], logits.shape[1], _p(out), _stream()))
     return out
 
 
@@ -2295,7 +2298,7 @@ def sample_rows(logits: torch.Tensor, work: torch.Tensor, counts: Optional[torch
     them either way.  With `append` the kernel stores each row's new id behind its history (the arrays
     of `history_rows` need room for it)."""
     _cuda(logits, work, counts, temperature, top_k, top_p, penalty, history, history_len, seeds, counters, uniforms, history_rows)
-    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1:
+    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride()[1] != 1:
         raise KernelError("sample_rows takes float32 [rows, vocab] logits")
     rows, vocab = logits.shape
     if work.dtype != torch.float32 or work.numel() < rows * vocab:
@@ -2317,11 +2320,45 @@ def sample_rows(logits: torch.Tensor, work: torch.Tensor, counts: Optional[torch
     if out is None:
         out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
     lib = sampling()
-    _run(lib, lib.mb_sample_rows(_p(logits), logits.stride(0), rows, vocab, _p(work), _p(counts), _p(temperature),
+    _run(lib, lib.mb_sample_rows(_p(logits), logits.stride()[0], rows, vocab, _p(work), _p(counts), _p(temperature),
                                  _p(top_k), _p(top_p), _p(penalty), _p(history),
-                                 history.stride(0) if history is not None else 0, _p(history_rows), 1 if append else 0,
+                                 history.stride()[0] if history is not None else 0, _p(history_rows), 1 if append else 0,
                                  _p(history_len), _p(seeds),
                                  _p(counters), _p(uniforms), _p(out), int(max_candidates), _stream()))
+    return out
+
+
+def sample_parameter_words(rows: int) -> int:
+    """8-byte words of the options of so many rows, as `sample_rows_packed` takes them."""
+    return 3 * rows + (5 * rows + 1) // 2
+
+
+def sample_rows_packed(logits: torch.Tensor, work: torch.Tensor, counts: Optional[torch.Tensor], parameters: torch.Tensor,
+                       max_candidates: int = 0, append: bool = False) -> torch.Tensor:
+    """`sample_rows` with the rows' options in one int64 array on the device: three words per row (all seeds, all draw counters, all
+    addresses of the histories, which count only with `counts`), then five 4-byte numbers per row (temperatures, top_p, penalties as
+    floats, top_k, lengths of the histories as integers)."""
+    _cuda(logits, work, counts, parameters)
+    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride()[1] != 1:
+        raise KernelError("sample_rows takes float32 [rows, vocab] logits")
+    rows, vocab = logits.shape
+    if work.dtype != torch.float32 or work.numel() < rows * vocab:
+        raise KernelError("sample_rows needs rows*vocab floats of scratch")
+    if counts is not None and (counts.dtype != torch.int32 or counts.numel() < rows * vocab):
+        raise KernelError("sample_rows needs rows*vocab int32 counters for the repetition penalty")
+    if parameters.dtype != torch.int64 or not parameters.is_contiguous() or parameters.numel() < sample_parameter_words(rows):
+        raise KernelError(f"the options of {rows} rows are {sample_parameter_words(rows)} contiguous int64 words")
+    if append and counts is None:
+        raise KernelError("a token history needs its lengths and the counters scratch")
+    out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
+    words = parameters.data_ptr()
+    number = lambda i: ctypes.c_void_p(words + 24 * rows + 4 * rows * i)  # noqa: E731
+    histories = counts is not None
+    lib = sampling()
+    _run(lib, lib.mb_sample_rows(_p(logits), logits.stride()[0], rows, vocab, _p(work), _p(counts), number(0), number(3), number(1), number(2),
+                                 None, 0, ctypes.c_void_p(words + 16 * rows) if histories else None, 1 if append else 0,
+                                 number(4) if histories else None, ctypes.c_void_p(words), ctypes.c_void_p(words + 8 * rows), None, _p(out),
+                                 int(max_candidates), _stream()))
     return out
 
 
@@ -2387,7 +2424,7 @@ def hyper_write(x: torch.Tensor, y: torch.Tensor, out_coefficients: torch.Tensor
         if t.dtype != torch.float32 or t.numel() != count or not t.is_contiguous():
             raise KernelError(f"hyper_write: {name} must be contiguous float32 of {count} elements")
     lib = hyper_streams_library()
-    _run(lib, lib.mb_hyper_write(_p(x), _p(y), y.stride(0), _code(y.dtype), _p(out_coefficients), _p(mix), x.shape[0], width, streams,
+    _run(lib, lib.mb_hyper_write(_p(x), _p(y), y.stride()[0], _code(y.dtype), _p(out_coefficients), _p(mix), x.shape[0], width, streams,
                                  _stream()))
 
 
@@ -2407,7 +2444,7 @@ def hyper_write_read_norm(x: torch.Tensor, y: torch.Tensor, out_coefficients: to
             raise KernelError(f"hyper_write_read_norm: {name} must be contiguous float32 of {count} elements")
     out = torch.empty((x.shape[0], width), dtype=out_dtype, device=x.device)
     lib = hyper_streams_library()
-    _run(lib, lib.mb_hyper_write_read_norm(_p(x), _p(y), y.stride(0), _p(out_coefficients), _p(mix), _p(coefficients), _p(gain), _p(out),
+    _run(lib, lib.mb_hyper_write_read_norm(_p(x), _p(y), y.stride()[0], _p(out_coefficients), _p(mix), _p(coefficients), _p(gain), _p(out),
                                            _code(out_dtype), x.shape[0], width, streams, ctypes.c_float(eps), _stream()))
     return out
 
@@ -2439,7 +2476,7 @@ def router_topk(x: torch.Tensor, router: torch.Tensor, top: int, scored: bool = 
     chosen = torch.empty((tokens, top), dtype=torch.int32, device=x.device)
     weights = torch.empty((tokens, top), dtype=torch.float32, device=x.device)
     lib = routed_experts_library()
-    _run(lib, lib.mb_router_topk(_p(x), x.stride(0), _p(router), _code(x.dtype), _p(chosen), _p(weights), tokens, x.shape[1], experts,
+    _run(lib, lib.mb_router_topk(_p(x), x.stride()[0], _p(router), _code(x.dtype), _p(chosen), _p(weights), tokens, x.shape[1], experts,
                                  top, 1 if scored else 0, _p(correction), int(groups), int(keep), ctypes.c_float(weight_scale), _stream()))
     return chosen, weights
 
@@ -2500,7 +2537,7 @@ def expert_first_product(x: torch.Tensor, gate_w: torch.Tensor, up_w: torch.Tens
     n, k = gate_w.shape[1], gate_w.shape[2]
     mid = torch.empty((plan.entries, n), dtype=x.dtype, device=x.device)
     lib = routed_experts_library()
-    _run(lib, lib.mb_expert_product(_p(x), x.stride(0), _p(gate_w), _p(up_w), _p(mid), None, n, _code(x.dtype), _p(plan.sorted),
+    _run(lib, lib.mb_expert_product(_p(x), x.stride()[0], _p(gate_w), _p(up_w), _p(mid), None, n, _code(x.dtype), _p(plan.sorted),
                                     _p(plan.offsets), _p(plan.tile_expert), _p(plan.tile_row), plan.max_tiles, plan.top, n, k,
                                     ctypes.c_float(limit), ctypes.c_float(slope), ctypes.c_float(up_offset), 1, 1 if tensor_cores else 0, _stream()))
     return mid
@@ -2515,7 +2552,7 @@ def expert_second_product(mid: torch.Tensor, down_w: torch.Tensor, plan: RoutePl
     n, k = down_w.shape[1], down_w.shape[2]
     slot_out = torch.empty((plan.entries, n), dtype=torch.float32, device=mid.device)
     lib = routed_experts_library()
-    _run(lib, lib.mb_expert_product(_p(mid), mid.stride(0), _p(down_w), None, None, _p(slot_out), n, _code(mid.dtype), _p(plan.sorted),
+    _run(lib, lib.mb_expert_product(_p(mid), mid.stride()[0], _p(down_w), None, None, _p(slot_out), n, _code(mid.dtype), _p(plan.sorted),
                                     _p(plan.offsets), _p(plan.tile_expert), _p(plan.tile_row), plan.max_tiles, plan.top, n, k,
                                     ctypes.c_float(0.0), ctypes.c_float(0.0), ctypes.c_float(0.0), 0, 1 if tensor_cores else 0, _stream()))
     return slot_out
@@ -2564,7 +2601,7 @@ def gather_rows(x: torch.Tensor, plan: PaddedRoutePlan) -> torch.Tensor:
         raise KernelError("gather_rows: bfloat16 rows are needed")
     out = torch.empty((plan.rows, x.shape[1]), dtype=torch.bfloat16, device=x.device)
     lib = routed_experts_library()
-    _run(lib, lib.mb_gather_rows(_p(x), x.stride(0), _p(plan.sorted), _p(plan.tile_group), _p(out), plan.rows, plan.top, x.shape[1],
+    _run(lib, lib.mb_gather_rows(_p(x), x.stride()[0], _p(plan.sorted), _p(plan.tile_group), _p(out), plan.rows, plan.top, x.shape[1],
                                  _stream()))
     return out
 
@@ -2589,7 +2626,7 @@ def grouped_first_product(a: torch.Tensor, gate_up: torch.Tensor, plan: PaddedRo
         raise KernelError(f"grouped_first_product: rows {tuple(a.shape)} do not fit matrices {tuple(gate_up.shape)}")
     mid = torch.empty((plan.rows, ff), dtype=torch.bfloat16, device=a.device)
     lib = gemm_tc()
-    _run(lib, lib.mb_gemm_tcgen05_grouped(_p(a), a.stride(0), _p(gate_up), width, 2 * experts * ff, _p(mid), ff, plan.rows, ff, width,
+    _run(lib, lib.mb_gemm_tcgen05_grouped(_p(a), a.stride()[0], _p(gate_up), width, 2 * experts * ff, _p(mid), ff, plan.rows, ff, width,
                                           1, experts * ff, _p(plan.tile_group), ctypes.c_float(limit), ctypes.c_float(slope), ctypes.c_float(up_offset),
                                           _sm_count(a.device), _stream()))
     return mid
@@ -2642,7 +2679,7 @@ def expert_rows_first(x: torch.Tensor, gate_w: torch.Tensor, up_w: torch.Tensor,
     n, k, top = gate_w.shape[1], gate_w.shape[2], chosen.shape[1]
     mid = torch.empty((entries, n), dtype=x.dtype, device=x.device)
     lib = routed_experts_library()
-    _run(lib, lib.mb_expert_rows(_p(x), x.stride(0), _p(gate_w), _p(up_w), _p(mid), None, n, _code(x.dtype), _p(chosen), _p(tokens), entries,
+    _run(lib, lib.mb_expert_rows(_p(x), x.stride()[0], _p(gate_w), _p(up_w), _p(mid), None, n, _code(x.dtype), _p(chosen), _p(tokens), entries,
                                  top, experts, n, k, ctypes.c_float(limit), ctypes.c_float(slope), ctypes.c_float(up_offset), 1, _stream()))
     return mid
 
@@ -2659,7 +2696,7 @@ def expert_rows_second(mid: torch.Tensor, down_w: torch.Tensor, chosen: torch.Te
     n, k = down_w.shape[1], down_w.shape[2]
     slot_out = torch.empty((mid.shape[0], n), dtype=torch.float32, device=mid.device)
     lib = routed_experts_library()
-    _run(lib, lib.mb_expert_rows(_p(mid), mid.stride(0), _p(down_w), None, None, _p(slot_out), n, _code(mid.dtype), _p(chosen),
+    _run(lib, lib.mb_expert_rows(_p(mid), mid.stride()[0], _p(down_w), None, None, _p(slot_out), n, _code(mid.dtype), _p(chosen),
                                  _p(tokens), entries, chosen.shape[1], experts, n, k, ctypes.c_float(0.0), ctypes.c_float(0.0), ctypes.c_float(0.0), 0, _stream()))
     return slot_out
 
@@ -2670,10 +2707,10 @@ def clamped_swish(gate: torch.Tensor, up: torch.Tensor, out: torch.Tensor, limit
     _cuda(gate, up, out)
     for name, t in (("gate", gate), ("up", up), ("out", out)):
         _columns(t, name)
-    if gate.shape != up.shape or out.shape != gate.shape or gate.stride(0) != up.stride(0) or not (gate.dtype == up.dtype == out.dtype):
+    if gate.shape != up.shape or out.shape != gate.shape or gate.stride()[0] != up.stride()[0] or not (gate.dtype == up.dtype == out.dtype):
         raise KernelError("clamped_swish: gate, up and out must share shape and dtype, gate and up one row stride")
     lib = routed_experts_library()
-    _run(lib, lib.mb_clamped_swish(_p(gate), _p(up), gate.stride(0), _p(out), out.stride(0), _code(gate.dtype), gate.shape[0],
+    _run(lib, lib.mb_clamped_swish(_p(gate), _p(up), gate.stride()[0], _p(out), out.stride()[0], _code(gate.dtype), gate.shape[0],
                                    gate.shape[1], ctypes.c_float(limit), ctypes.c_float(slope), ctypes.c_float(up_offset), _stream()))
 
 
@@ -2716,7 +2753,7 @@ def expert_combine(slot_out: torch.Tensor, weights: torch.Tensor, shared: Option
         dtype = _code(rows.dtype)
     out = torch.empty((tokens, width), dtype=torch.float32, device=slot_out.device)
     lib = routed_experts_library()
-    _run(lib, lib.mb_expert_combine(_p(slot_out), _p(weights), _p(shared), _p(score), score.stride(0) if score is not None else 0,
+    _run(lib, lib.mb_expert_combine(_p(slot_out), _p(weights), _p(shared), _p(score), score.stride()[0] if score is not None else 0,
                                     dtype, _p(out), tokens, width, top, _p(position), _p(chosen), int(experts), _p(rows),
-                                    rows.stride(0) if rows is not None else 0, _stream()))
+                                    rows.stride()[0] if rows is not None else 0, _stream()))
     return out

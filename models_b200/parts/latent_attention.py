@@ -144,8 +144,8 @@ class LatentAttentionMixer(SplitPart, Mixer):
 
     def _expanded_rows(self, batch, group, run: RunContext, mid: torch.Tensor, gate):
         """How many rows of every sequence the step expands into keys and values: 0 for its own rows alone, None for none."""
-        if (self.expand is None or batch.max_q_len < ops.TCGEN05_ATTENTION_MIN_ROWS or mid.stride(0) % 8 or mid.data_ptr() % 16
-                or (gate is not None and self.spec.gate_kind == "element" and (gate.stride(0) % 8 or gate.data_ptr() % 16))):
+        if (self.expand is None or batch.max_q_len < ops.TCGEN05_ATTENTION_MIN_ROWS or mid.stride()[0] % 8 or mid.data_ptr() % 16
+                or (gate is not None and self.spec.gate_kind == "element" and (gate.stride()[0] % 8 or gate.data_ptr() % 16))):
             return None
         fresh = getattr(batch, "fresh", False)
         if mid.shape[0] < EXPANDED_TOKENS and (not fresh or self.spec.query_latent or self.spec.gate_kind == "element"):
@@ -164,7 +164,7 @@ class LatentAttentionMixer(SplitPart, Mixer):
 
     def _expanded(self, q, down, gate, mid, batch, group, run: RunContext, cos, sin, key_rows: int) -> None:
         s = self.spec
-        if q.stride(0) % 8 or q.data_ptr() % 16:
+        if q.stride()[0] % 8 or q.data_ptr() % 16:
             q = q.contiguous()
         own, tail, q_tail = ops.latent_rows(down, self.latent_gain, self.turned, cos, sin, batch.positions, s.eps, run.k_pool, group.slot_mapping,
                                             q=q, heads=s.num_heads, head_columns=s.head_dim + self.turned, padded=_whole(self.turned))

@@ -30,11 +30,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype) -> tor
     if weight.dtype != torch.bfloat16:
         raise ops.KernelError(f"matrices are bfloat16 or float32, got {weight.dtype}")
     a = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
-    if ops.skinny_pays(weight, a.shape[0]) and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 \
+    if ops.skinny_pays(weight, a.shape[0]) and a.stride()[1] == 1 and a.stride()[0] % 8 == 0 and a.data_ptr() % 16 == 0 \
             and out_dtype in (torch.bfloat16, torch.float32):
         # decode: few rows, the weights stream once through this package's own kernel
         return ops.skinny_gemm(weight, ops.EPI_F32 if out_dtype == torch.float32 else ops.EPI_BF16, x=a)
-    if (ops.gemm_tcgen05_takes(weight, rows=a.shape[0]) and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
+    if (ops.gemm_tcgen05_takes(weight, rows=a.shape[0]) and a.stride()[1] == 1 and a.stride()[0] % 8 == 0 and a.data_ptr() % 16 == 0
             and out_dtype in (torch.bfloat16, torch.float32)):
         # many rows: this package's tcgen05 kernels (wide decode form up to 128 rows, prefill form above)
         return ops.tensor_core_gemm(a, weight, ops.EPI_F32 if out_dtype == torch.float32 else ops.EPI_BF16)
@@ -50,7 +50,7 @@ def add_linear(x: torch.Tensor, a: torch.Tensor, weight: torch.Tensor) -> None:
     if not x.is_cuda:
         raise ops.KernelError("models_b200 runs on a CUDA device only; there is no CPU path")
     rows = a.shape[0]
-    if weight.dtype == torch.bfloat16 and a.dtype == torch.bfloat16 and a.stride(1) == 1 and a.stride(0) % 8 == 0 \
+    if weight.dtype == torch.bfloat16 and a.dtype == torch.bfloat16 and a.stride()[1] == 1 and a.stride()[0] % 8 == 0 \
             and a.data_ptr() % 16 == 0:
         if ops.skinny_pays(weight, rows):
             ops.skinny_gemm(weight, ops.EPI_RESIDUAL, x=a, out=x)

@@ -8,6 +8,7 @@ Each request draws from its own stream: Philox keyed by its seed, counted by its
 from __future__ import annotations
 
 import secrets
+import struct
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -59,21 +60,20 @@ class BatchSampler:
         rows = len(requests)
         if logits.shape[0] < rows or logits.shape[1] != self.vocab:
             raise ValueError(f"logits {tuple(logits.shape)} do not fit {rows} requests of vocabulary {self.vocab}")
-        if all(r.options.greedy for r in requests):
+        options = [r.options for r in requests]
+        if all(o.greedy for o in options):
             return greedy(logits)[:rows] if greedy is not None else ops.argmax_rows(logits[:rows])
-        logits = logits[:rows]
-        penalised = any(r.history is not None for r in requests)
+        if logits.shape[0] > rows:
+            logits = logits[:rows]
+        penalised = any([r.history is not None for r in requests])
         if penalised:
             for r in requests:
                 if r.history is not None:
                     self._history_on_device(r)
-        temperature, top_k, top_p, penalty, seeds, counters, history_rows, history_len, most = self._parameters(requests)
+        parameters, most = self._parameters(requests, options)
         counts = torch.empty((rows, self.vocab), dtype=torch.int32, device=self.device) if penalised else None
-        if not penalised:
-            history_rows = history_len = None
         work = torch.empty((rows, self.vocab), dtype=torch.float32, device=self.device)
-        out = ops.sample_rows(logits, work, counts, temperature, top_k, top_p, penalty, None, history_len, seeds, counters,
-                              max_candidates=most, history_rows=history_rows, append=history_rows is not None)
+        out = ops.sample_rows_packed(logits, work, counts, parameters, max_candidates=most, append=penalised)
         for r in requests:
             if r.options.temperature > 0.0:
                 r.draws += 1
@@ -92,14 +92,13 @@ class BatchSampler:
             r.history_device = host.to(self.device)
             r.history_sent = len(r.history)
 
-    def _parameters(self, requests: Sequence[RequestSampling]):
-        """The per-row options on the device, sent as one asynchronous copy from pinned memory (a copy from ordinary memory
-        would wait for every step that is still queued), and the largest candidate set among the rows that cut anything (1 if
-        none does): it picks the kernel.  The buffer holds 8-byte words: three per row (seed, draws, address of the history),
-        then five 4-byte numbers per row (temperature, top_p, penalty, top_k, length of the history).  The rows are walked once
-        and filled in through numpy: building tensors of lists took longer than the kernel."""
+    def _parameters(self, requests: Sequence[RequestSampling], options: Sequence[SamplingOptions]):
+        """The per-row options on the device as `ops.sample_rows_packed` takes them, sent as one asynchronous copy from pinned memory (a copy
+        from ordinary memory would wait for every step that is still queued), and the largest candidate set among the rows that cut
+        anything (1 if none does): it picks the kernel.  A list per option, packed at once: a walk over the rows, numpy's conversion of
+        lists and a tensor for every option took 100 us of the host's time for 64 rows, twice the kernel's."""
         rows, vocab = len(requests), self.vocab
-        words = 3 * rows + (5 * rows + 1) // 2
+        words = ops.sample_parameter_words(rows)
         if self._staging is None or self._staging[0][0].numel() < words:
             size = max(6 * 64, words)
             self._staging = []
@@ -109,31 +108,27 @@ class BatchSampler:
         host, longs, event = self._staging[self._staging_next]
         self._staging_next = (self._staging_next + 1) % len(self._staging)
         event.synchronize()  # the copy that last read this buffer, four calls ago
-        seeds, draws, addresses, temperatures, top_ps, penalties, top_ks, lengths, most = [], [], [], [], [], [], [], [], 1
-        for r in requests:
-            o, history = r.options, r.history_device
-            top_k = min(o.top_k, vocab)
-            if top_k > most and (o.top_k < vocab or o.top_p < 1.0):
-                most = top_k
-            seeds.append(r.seed)
-            draws.append(r.draws)
-            addresses.append(history.data_ptr() if history is not None else 0)
-            temperatures.append(o.temperature)
-            top_ps.append(o.top_p)
-            penalties.append(o.repetition_penalty)
-            top_ks.append(top_k)
-            lengths.append(r.history_sent if history is not None else 0)
-        longs[:3 * rows] = seeds + draws + addresses
-        small = longs[3 * rows:words]
-        small.view(np.float32)[:3 * rows] = temperatures + top_ps + penalties
-        small.view(np.int32)[3 * rows:5 * rows] = top_ks + lengths
+        top_ks = [o.top_k for o in options]
+        most = max(top_ks)
+        if most >= vocab:
+            most = max([min(o.top_k, vocab) for o in options if o.top_k < vocab or o.top_p < 1.0], default=1)
+            top_ks = [min(k, vocab) for k in top_ks]
+        histories = [r.history_device for r in requests]
+        addresses = [0 if h is None else h.data_ptr() for h in histories]
+        lengths = [0 if h is None else r.history_sent for h, r in zip(histories, requests)]
+        whole = [r.seed for r in requests] + [r.draws for r in requests] + addresses
+        floats = [o.temperature for o in options] + [o.top_p for o in options] + [o.repetition_penalty for o in options]
+        try:
+            struct.pack_into(f"={3 * rows}q{3 * rows}f{2 * rows}i", longs, 0, *whole, *floats, *top_ks, *lengths)
+        except (struct.error, OverflowError):  # numbers beyond their type: as numpy takes or refuses them
+            longs[:3 * rows] = whole
+            small = longs[3 * rows:words]
+            small.view(np.float32)[:3 * rows] = floats
+            small.view(np.int32)[3 * rows:5 * rows] = top_ks + lengths
         device = torch.empty((words,), dtype=torch.int64, device=self.device)
         device.copy_(host[:words], non_blocking=True)
-        event.record()
-        seeds, draws, addresses, rest = device.split((rows, rows, rows, words - 3 * rows))
-        temperature, top_p, penalty, _ = rest.view(torch.float32).split((rows, rows, rows, 2 * (words - 3 * rows) - 3 * rows))
-        top_k, length = rest.view(torch.int32)[3 * rows:5 * rows].split(rows)
-        return temperature, top_k, top_p, penalty, seeds, draws, addresses, length, most
+        event.record(torch.cuda.current_stream(self.device))  # (without one torch asks the driver and the environment which device it is)
+        return device, most
 
     @staticmethod
     def record(requests: Sequence[RequestSampling], tokens: Sequence[int]) -> None:
