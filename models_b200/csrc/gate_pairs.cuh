@@ -32,6 +32,25 @@ __device__ __forceinline__ float max_of(float a, float b, float c) {
     return m;
 }
 
+// z[i] <- 1 / (1 + e^(-z[i])), rounded as the division rounds it: with one number beyond e^40 by divisions, else side by side.
+template <int kCount>
+__device__ __forceinline__ void sigmoids(float (&z)[kCount]) {
+    static_assert(kCount % 2 == 0, "whole pairs");
+    float lowest = z[0];
+#pragma unroll
+    for (int i = 0; i < kCount; i += 2) lowest = min_of(lowest, z[i], z[i + 1]);
+    if (lowest >= -40.0f) {
+#pragma unroll
+        for (int i = 0; i < kCount; i += 2) {
+            const uint64_t q = minus_quotients(0x3f8000003f800000ull, 1.0f + expf(-z[i]), 1.0f + expf(-z[i + 1]));  // 1, 1
+            z[i] = -low_of(q), z[i + 1] = -high_of(q);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kCount; ++i) z[i] = 1.0f / (1.0f + expf(-z[i]));
+    }
+}
+
 // gate[i] = gated_pair(activation, gate[i], up[i], clamp).  A division has a long way for unusual operands, and a branch to it after every pair
 // keeps pairs from being worked on side by side; here one branch says whether all of a thread's gates are usual ones: exponentials up to e^40
 // (every divisor then lies from 1 to 2^58, and no remainder that counts is below the floats), gates up to 2^60.  NaN passes through either way.

@@ -91,13 +91,16 @@ template <int kThreads>
 struct UnitRows {
     static constexpr int at_once = kThreads / 16, passes = (kChunk + at_once - 1) / at_once;
     float4 x[passes];
-    __device__ __forceinline__ UnitRows(const float* rows, int stride, int count, float unit_eps, float factor, bf16* planes, float* unit) {
+    __device__ __forceinline__ UnitRows(const float* rows, int stride, int count) {  // asks for the rows
         const int d = (threadIdx.x % 16) * 4;
 #pragma unroll
         for (int i = 0; i < passes; ++i) {
             const int row = threadIdx.x / 16 + at_once * i;
             x[i] = row < count ? *reinterpret_cast<const float4*>(rows + (size_t)row * stride + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
+    }
+    __device__ __forceinline__ void put(int count, float unit_eps, float factor, bf16* planes, float* unit) {
+        const int d = (threadIdx.x % 16) * 4;
 #pragma unroll
         for (int i = 0; i < passes; ++i) {
             const int row = threadIdx.x / 16 + at_once * i;
@@ -155,6 +158,7 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
     const float* rows = args.conv + token0 * args.conv_stride;
     const float* key_rows = rows + args.k_at + head / (args.heads / args.kv_heads) * kDim;
     const float* value_rows = rows + args.v_at + (size_t)head * V;
+    UnitRows<Plan::threads> k(key_rows, args.conv_stride, count);
     // gates: a token beyond the chunk's last neither forgets nor writes
     double log_g = 0.0;
     if (tid < kChunk) {
@@ -174,7 +178,7 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
         }
         logs[tid] = log_g;
     }
-    const UnitRows<Plan::threads> k(key_rows, args.conv_stride, count, args.unit_eps, 1.0f, keys, unit);
+    k.put(count, args.unit_eps, 1.0f, keys, unit);
     __syncthreads();
     if (tid >= 32 && tid < kChunk) logs[tid] = log_g + logs[31];
     __syncthreads();
@@ -497,32 +501,40 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
     if (count <= 0) return;
     const size_t token0 = (size_t)first + chunk * kChunk;
     const size_t at = place_of(first, seq, chunk) * args.heads + head;
-    float fit;
-    auto bring = [&](const float* from) {
-        fit = 0.0f;
-        constexpr int kPieces = 64 * V / 8 / kResultThreads;
-        float x[kPieces][8];
+    constexpr int kPieces = 64 * V / 8 / kResultThreads;  // eights of the start, and of u, that a thread brings
+    float x[kPieces][8];
+    auto ask = [&](const float* from) {
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) load8(from + 8 * (tid + i * kResultThreads), x[i]);
+    };
+    auto put = [&]() {
+        float fit = 0.0f;
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
             const int piece = tid + i * kResultThreads;
             fit += fitness(x[i]);
             store_parts(planes + Plan::wide + piece / (V / 8) * Plan::wide_row + piece % (V / 8) * 8, Plan::wide_plane, x[i]);
         }
+        return fit;
     };
-    bring(args.starts + at * kDim * V);
-    if (tid < kChunk) logs[tid] = args.logs[at * kChunk + tid];
+    // everything is asked for before any of it is waited for
     const float* rows = args.conv + token0 * args.conv_stride;
     const int qk_head = head / (args.heads / args.kv_heads);
-    UnitRows<kResultThreads>(rows + args.k_at + qk_head * kDim, args.conv_stride, count, args.unit_eps, 1.0f, planes + Plan::keys, nullptr);
-    UnitRows<kResultThreads>(rows + args.q_at + qk_head * kDim, args.conv_stride, count, args.unit_eps, 0.125f, planes + Plan::queries, nullptr);  // 64^(-1/2)
+    {
+        UnitRows<kResultThreads> k(rows + args.k_at + qk_head * kDim, args.conv_stride, count), q(rows + args.q_at + qk_head * kDim, args.conv_stride, count);
+        if (tid < kChunk) logs[tid] = args.logs[at * kChunk + tid];
+        ask(args.starts + at * kDim * V);
+        k.put(count, args.unit_eps, 1.0f, planes + Plan::keys, nullptr);
+        q.put(count, args.unit_eps, 0.125f, planes + Plan::queries, nullptr);  // 64^(-1/2)
+        put();
+    }
     __syncthreads();
     const int warp = (tid >> 5) & 3, half_columns = tid >> 7, column0 = half_columns * (V / 2), group = (tid & 31) >> 2, pair = 2 * (tid & 3);
     const uint32_t base = smem_u32(planes);
     const uint32_t query_at = base + (Plan::queries + 16 * warp * kRow) * 2 + lanes_by_row(kRow), key_at = base + Plan::keys * 2 + lanes_by_column(kRow);
     const uint32_t wide_at = base + (Plan::wide + column0) * 2 + lanes_by_row(Plan::wide_row);
     float acc[V / 16][4] = {}, weights[kChunk / 8][4] = {};
+    ask(args.u + at * kChunk * V);  // (arrives while the start is multiplied)
 #pragma unroll
     for (int d = 0; d < kDim; d += 16) {
         Parts a, b;
@@ -532,6 +544,13 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
             load_parts_turned(b, wide_at + (d * Plan::wide_row + 8 * n) * 2, Plan::wide_plane);
             split_products(acc[n], acc[n + 1], a, b);
         }
+    }
+    __syncthreads();  // nobody reads the start any more
+    const float fit = put();
+#pragma unroll
+    for (int d = 0; d < kDim; d += 16) {
+        Parts a, b;
+        load_parts(a, query_at + d * 2, kPlane);
 #pragma unroll
         for (int n = 0; n < kChunk / 8; n += 2) {  // q . k over the tokens up to the warp's last
             if (n > 2 * warp) break;
@@ -539,8 +558,6 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
             split_products(weights[n], weights[n + 1], a, b);
         }
     }
-    __syncthreads();  // nobody reads the start any more
-    bring(args.u + at * kChunk * V);
     const int row = 16 * warp + group;
     const float from_start[2] = {expf((float)logs[row]), expf((float)logs[row + 8])};
 #pragma unroll

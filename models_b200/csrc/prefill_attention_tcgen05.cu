@@ -236,26 +236,6 @@ __device__ __forceinline__ void umma_a_tmem(uint32_t tmem_d, uint32_t tmem_a, ui
         : "memory");
 }
 
-// v[i] *= sigmoid(z[i]), by reciprocals that are rounded as divisions are (see minus_quotients); with one z beyond them by divisions.  (One
-// branch for all, so that they are worked on side by side: four at a time were 365 cycles of latency.)
-template <int kRows>
-__device__ __forceinline__ void gate_by_sigmoids(float (&v)[kRows][4], const float (&z)[kRows][4]) {
-    float lowest = z[0][0];
-#pragma unroll
-    for (int i = 0; i < kRows; ++i) lowest = min_of(min_of(lowest, z[i][0], z[i][1]), z[i][2], z[i][3]);
-    if (lowest >= -40.0f) {
-#pragma unroll
-        for (int i = 0; i < 2 * kRows; ++i) {
-            const int r = i / 2, c = i % 2 * 2;
-            const uint64_t q = minus_quotients(0x3f8000003f800000ull, 1.0f + expf(-z[r][c]), 1.0f + expf(-z[r][c + 1]));  // 1, 1
-            v[r][c] *= -low_of(q), v[r][c + 1] *= -high_of(q);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4 * kRows; ++i) v[i / 4][i % 4] *= 1.0f / (1.0f + expf(-z[i / 4][i % 4]));
-    }
-}
-
 struct AttentionArgs {
     bf16* out;
     int out_row_stride;
@@ -663,17 +643,19 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 if (mine_stored && gated) {
 #pragma unroll 1
                     for (int at0 = first; at0 < last; at0 += kBatch * kRowsAtOnce) {
-                        float v[kBatch][4], z[kBatch][4];
+                        float v[kBatch][4], z[4 * kBatch];
 #pragma unroll
                         for (int i = 0; i < kBatch; ++i) {
                             const int at = min(at0 + i * kRowsAtOnce, last - 1);
                             *reinterpret_cast<float4*>(v[i]) = rows[at * kFours + (four ^ (at & 7))];
                             const uint2 raw = *reinterpret_cast<const uint2*>(  // (in the 128-byte swizzle, as TMA leaves it)
                                 smem + kGatesAt + four / 16 * kQBoxBytes + at * 128 + ((four % 16 / 2 ^ (at & 7)) << 4) + four % 2 * 8);
-                            z[i][0] = __uint_as_float(raw.x << 16), z[i][1] = __uint_as_float(raw.x & 0xffff0000u);
-                            z[i][2] = __uint_as_float(raw.y << 16), z[i][3] = __uint_as_float(raw.y & 0xffff0000u);
+                            z[4 * i] = __uint_as_float(raw.x << 16), z[4 * i + 1] = __uint_as_float(raw.x & 0xffff0000u);
+                            z[4 * i + 2] = __uint_as_float(raw.y << 16), z[4 * i + 3] = __uint_as_float(raw.y & 0xffff0000u);
                         }
-                        gate_by_sigmoids(v, z);
+                        sigmoids(z);  // (one branch for all: four at a time were 365 cycles of latency)
+#pragma unroll
+                        for (int i = 0; i < 4 * kBatch; ++i) v[i / 4][i % 4] *= z[i];
 #pragma unroll
                         for (int i = 0; i < kBatch; ++i)
                             if (at0 + i * kRowsAtOnce < last) store(at0 + i * kRowsAtOnce, v[i]);

@@ -13,6 +13,7 @@
 // which float multiply-adds from shared memory bound; here 29, 14 and 54 us (sums of products added one by one: 32, 14 and 58), bound by the six products for one and by the
 // instructions that activate and split what every chunk reads.
 #include "common.cuh"
+#include "gate_pairs.cuh"
 #include "split_products.cuh"
 
 MB_DEFINE_LAST_ERROR()
@@ -87,6 +88,43 @@ __device__ __forceinline__ void stage_rows(bf16* planes, int row_numbers, int pl
     }
 }
 
+// A thread's part of the same rows without rotation: asked for, all of a block's rows before any is waited for, and later put in place.
+template <int kCols>
+struct RawRows {
+    static constexpr int kPieces = kChunk * kCols / 8 / kThreads;
+    uint4 raw[kPieces];
+    __device__ __forceinline__ void ask(const bf16* src, int stride, int count) {
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int piece = threadIdx.x + i * kThreads, row = piece / (kCols / 8);
+            raw[i] = make_uint4(0, 0, 0, 0);
+            if (row < count) raw[i] = *reinterpret_cast<const uint4*>(src + (size_t)row * stride + piece % (kCols / 8) * 8);
+        }
+    }
+    // Returns a sum that is finite only where every number is, and has three finite parts.
+    __device__ __forceinline__ float put(bf16* planes, int row_numbers, int plane_numbers, int activation, int count, const float* weight) const {
+        float fit = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int piece = threadIdx.x + i * kThreads, row = piece / (kCols / 8);
+            const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[2 * j] = __uint_as_float(w[j] << 16), x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+            if (activation >= 0 && row < count) {
+                const float ones[8] = {1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f};
+                gate_pairs(activation, x, ones, ClampedPair{});
+            }
+            if (weight != nullptr)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] *= weight[row];
+            fit += fitness(x);
+            store_parts(planes + row * row_numbers + piece % (kCols / 8) * 8, plane_numbers, x);
+        }
+        return fit;
+    }
+};
+
 // grid (heads, most chunks of a sequence, sequences); block kThreads.  A warp has 16 coordinates and half of the columns of what the
 // chunk adds.
 template <int V>
@@ -102,11 +140,16 @@ retention_chunk_adds_kernel(const RetentionArgs args) {
     const int first = args.cu_q[seq], count = min(kChunk, args.cu_q[seq + 1] - first - chunk * kChunk);
     if (count <= 0) return;
     const size_t token0 = (size_t)first + chunk * kChunk;
+    const bf16* key_rows = args.k + token0 * args.in_stride + (size_t)head * kDim;
+    RawRows<V> v;
+    RawRows<kDim> k;
+    v.ask(args.v + token0 * args.in_stride + (size_t)head * V, args.in_stride, count);
+    if (args.rotary_dim == 0) k.ask(key_rows, args.in_stride, count);
     if (tid < kChunk) weight[tid] = tid < count ? args.key_scale * powf(args.decay[head], (float)(count - 1 - tid)) : 0.0f;
-    stage_rows<V>(values, Values<V>::row, Values<V>::plane, args.v + token0 * args.in_stride + (size_t)head * V, args, count, 0, 0, nullptr);
+    v.put(values, Values<V>::row, Values<V>::plane, args.input_act, count, nullptr);
     __syncthreads();
-    const int position0 = args.rotary_dim > 0 ? args.positions[first] + chunk * kChunk : 0;
-    stage_rows<kDim>(keys, kKeyRow, kKeyPlane, args.k + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, weight);
+    if (args.rotary_dim == 0) k.put(keys, kKeyRow, kKeyPlane, args.input_act, count, weight);
+    else stage_rows<kDim>(keys, kKeyRow, kKeyPlane, key_rows, args, count, args.rotary_dim, args.positions[first] + chunk * kChunk, weight);
     __syncthreads();
     const int tile = (tid >> 5) & 3, column0 = (tid >> 7) * (V / 2), lane = tid & 31;
     float acc[V / 16][4] = {};
@@ -181,28 +224,31 @@ retention_chunk_results_kernel(const RetentionArgs args) {
     const int first = args.cu_q[seq], count = min(kChunk, args.cu_q[seq + 1] - first - chunk * kChunk);
     if (count <= 0) return;
     const size_t token0 = (size_t)first + chunk * kChunk;
-    constexpr int kPieces = 64 * V / 8 / kThreads;  // eights of the start, and of the values, that a thread brings
+    const bf16 *query_rows = args.q + token0 * args.in_stride + (size_t)head * kDim, *key_rows = args.k + token0 * args.in_stride + (size_t)head * kDim;
+    RawRows<V> v;
     {
+        constexpr int kPieces = 64 * V / 8 / kThreads;  // eights of the start that a thread brings
         const float* from = args.starts + (place_of(first, seq, chunk) * args.heads + head) * kDim * V;
         float x[kPieces][8];
+        RawRows<kDim> q, k;
+        if (args.rotary_dim == 0) q.ask(query_rows, args.in_stride, count), k.ask(key_rows, args.in_stride, count);
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) load8(from + 8 * (tid + i * kThreads), x[i]);
+        v.ask(args.v + token0 * args.in_stride + (size_t)head * V, args.in_stride, count);
+        if (tid <= kChunk) power[tid] = powf(args.decay[head], (float)tid);
+        if (args.rotary_dim == 0) {
+            q.put(queries, kKeyRow, kKeyPlane, args.input_act, count, nullptr);
+            k.put(keys, kKeyRow, kKeyPlane, args.input_act, count, nullptr);
+        } else {
+            const int position0 = args.positions[first] + chunk * kChunk;
+            stage_rows<kDim>(queries, kKeyRow, kKeyPlane, query_rows, args, count, args.rotary_dim, position0, nullptr);
+            stage_rows<kDim>(keys, kKeyRow, kKeyPlane, key_rows, args, count, args.rotary_dim, position0, nullptr);
+        }
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
             const int piece = tid + i * kThreads;
             store_parts(wide + piece / (V / 8) * kRow + piece % (V / 8) * 8, kPlane, x[i]);
         }
-    }
-    if (tid <= kChunk) power[tid] = powf(args.decay[head], (float)tid);
-    const int position0 = args.rotary_dim > 0 ? args.positions[first] + chunk * kChunk : 0;
-    stage_rows<kDim>(queries, kKeyRow, kKeyPlane, args.q + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, nullptr);
-    stage_rows<kDim>(keys, kKeyRow, kKeyPlane, args.k + token0 * args.in_stride + (size_t)head * kDim, args, count, args.rotary_dim, position0, nullptr);
-    uint4 raw_values[kPieces];
-#pragma unroll
-    for (int i = 0; i < kPieces; ++i) {
-        const int piece = tid + i * kThreads, row = piece / (V / 8);
-        raw_values[i] = make_uint4(0, 0, 0, 0);
-        if (row < count) raw_values[i] = *reinterpret_cast<const uint4*>(args.v + (token0 + row) * args.in_stride + (size_t)head * V + piece % (V / 8) * 8);
     }
     __syncthreads();
     const int warp = (tid >> 5) & 3, half_columns = tid >> 7, column0 = half_columns * (V / 2), lane = tid & 31, group = lane >> 2, pair = 2 * (lane & 3);
@@ -227,20 +273,7 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         }
     }
     __syncthreads();  // nobody reads the start any more
-    float fit = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kPieces; ++i) {
-        const int piece = tid + i * kThreads;
-        const uint32_t w[4] = {raw_values[i].x, raw_values[i].y, raw_values[i].z, raw_values[i].w};
-        float x[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) x[2 * j] = __uint_as_float(w[j] << 16), x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
-        if (args.input_act >= 0 && piece / (V / 8) < count)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = gate_activation(args.input_act, x[j]);
-        fit += fitness(x);
-        store_parts(wide + piece / (V / 8) * kRow + piece % (V / 8) * 8, kPlane, x);
-    }
+    const float fit = v.put(wide, kRow, kPlane, args.input_act, count, nullptr);
     const bool spoiled = __syncthreads_or(!isfinite(fit));
     const int row = 16 * warp + group;
 #pragma unroll
