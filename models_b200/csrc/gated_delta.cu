@@ -152,7 +152,7 @@ short_conv_fours_kernel(const T* __restrict__ in, int in_stride, const float* __
         }
     }
     // Inputs are asked for eight tokens ahead (one by one every token waited for its own), and sigmoids divided four at a time.
-    // (2,048 tokens, 3,072 channels: @CONV@.)
+    // (3,072 channels: 2,048 tokens 17.0 -> 15.5 us, four sequences of 600 in all 12.5 -> 7.3.)
     constexpr int kAtOnce = 8;
     RawFour<T> next[kAtOnce];
     auto ask = [&](int j) {

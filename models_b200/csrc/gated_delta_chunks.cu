@@ -21,9 +21,11 @@
 // results by 1.4e-7 (2e-7).
 // One sequence of 2,048 tokens, 16 heads of 64 x 128: the walk's chain of 2,048 tokens is bound by its latency (618 us, and 30 for
 // the kernels around it); the three kernels took 58, 105 and 71 us as float multiply-adds, bound by what the operands take from
-// shared memory and by the latency of few warps; 47, 46 and 58 here (a layer: 310 us, and 220), where the carrying kernel is bound by
-// its chunk's two products one after the other, the others by six products for one and the splitting of what they read.
+// shared memory and by the latency of few warps; 37, 46 and 52 here (a layer: 310 us, and 199; 47, 46 and 58 and 221 with every loop unrolled
+// and a block's gates asked for one by one), where the carrying kernel is bound by its chunk's two products one after the other, the others
+// by six products for one and by the latency of what each phase of a block waits for.
 #include "common.cuh"
+#include "gate_pairs.cuh"
 #include "split_products.cuh"
 
 MB_DEFINE_LAST_ERROR()
@@ -62,6 +64,18 @@ struct DeltaChunkArgs {
 __device__ __forceinline__ float sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float softplus(float v) { return fmaxf(v, 0.0f) + log1pf(expf(-fabsf(v))); }
 
+template <typename T>
+struct Pairs;  // two numbers as they are stored
+template <>
+struct Pairs<float> {
+    using type = float2;
+};
+template <>
+struct Pairs<bf16> {
+    using type = uint32_t;
+};
+template <typename T>
+using Pair = typename Pairs<T>::type;
 __device__ __forceinline__ float2 load_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ float2 load_pair(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 __device__ __forceinline__ void store_pair(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
@@ -194,34 +208,29 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
         if (tid < kChunk) args.logs[at * kChunk + tid] = logs[tid];
     }
     const int warp = tid >> 5, group = (tid & 31) >> 2, pair = 2 * (tid & 3);
-    if (warp < kChunk / 16) {
-        // matrix[i][j] = beta_i G_i / G_j (k_i . k_j) for j < i: rows 16 * warp .. + 15, the columns up to them
-        float acc[kChunk / 8][4] = {};
-        const uint32_t left = smem_u32(keys) + 16 * warp * kRow * 2 + lanes_by_row(kRow), right = smem_u32(keys) + lanes_by_column(kRow);
-#pragma unroll
+    // matrix[i][j] = beta_i G_i / G_j (k_i . k_j) for j < i: of every 16 rows the columns up to them, 16 a warp at a time
+    for (int unit_at = warp; unit_at < 10; unit_at += Plan::threads / 32) {
+        const int rows16 = unit_at >= 6 ? 3 : unit_at >= 3 ? 2 : unit_at >= 1 ? 1 : 0, columns16 = unit_at - rows16 * (rows16 + 1) / 2;
+        float acc[2][4] = {};
+        const uint32_t left = smem_u32(keys) + 16 * rows16 * kRow * 2 + lanes_by_row(kRow), right = smem_u32(keys) + 16 * columns16 * kRow * 2 + lanes_by_column(kRow);
+#pragma unroll 1
         for (int d = 0; d < kDim; d += 16) {
             Parts a, b;
             load_parts(a, left + d * 2, kPlane);
-#pragma unroll
-            for (int n = 0; n < kChunk / 8; n += 2) {
-                if (n > 2 * warp) break;
-                load_parts(b, right + (8 * n * kRow + d) * 2, kPlane);
-                split_products(acc[n], acc[n + 1], a, b);
-            }
+            load_parts(b, right + d * 2, kPlane);
+            split_products(acc[0], acc[1], a, b);
         }
 #pragma unroll
-        for (int n = 0; n < kChunk / 8; ++n) {
-            if (n > 2 * warp + 1) break;
+        for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                const int i = 16 * warp + group + 8 * half, j = 8 * n + pair;
+                const int i = 16 * rows16 + group + 8 * half, j = 16 * columns16 + 8 * n + pair;
                 const float b = beta[i];
                 const float lo = j < i ? acc[n][2 * half] * b * expf((float)(logs[i] - logs[j])) : 0.0f;
                 const float hi = j + 1 < i ? acc[n][2 * half + 1] * b * expf((float)(logs[i] - logs[j + 1])) : 0.0f;
                 split_two(lo, hi, matrix + i * kRow + j, kPlane);
-                if (n >= 2 * warp) diagonal[i * Plan::diagonal_row + j % 16] = lo, diagonal[i * Plan::diagonal_row + j % 16 + 1] = hi;
+                if (columns16 == rows16) diagonal[i * Plan::diagonal_row + j % 16] = lo, diagonal[i * Plan::diagonal_row + j % 16 + 1] = hi;
             }
-        }
     }
     // a warp's columns of the right sides, beta v and beta G k, as products leave their results; all four blocks of 16 rows
     constexpr int kTiles = 4;  // tiles of eight columns
@@ -244,13 +253,14 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
     if (tid < kChunk) {
         // a column of the inverse of a diagonal block I + M: z_r = (r == c) - sum_(s < r) M[r][s] z_s
         const int block = tid / 16, c = tid % 16;
-        float z[16];
-#pragma unroll
+        float z[16] = {};
+#pragma unroll 1
         for (int r = 0; r < 16; ++r) {
             float sum = r == c ? 1.0f : 0.0f;
 #pragma unroll
-            for (int s = 0; s < r; ++s) sum = fmaf(-diagonal[(16 * block + r) * Plan::diagonal_row + s], z[s], sum);
-            z[r] = sum;
+            for (int s = 0; s < 16; ++s) sum = fmaf(-diagonal[(16 * block + r) * Plan::diagonal_row + s], z[s], sum);  // (from s = r on zeros meet zeros)
+#pragma unroll
+            for (int s = 0; s < 16; ++s) z[s] = s == r ? sum : z[s];
             uint32_t hi, mid, lo;
             split_pair(sum, 0.0f, hi, mid, lo);
             unsigned short* to = reinterpret_cast<unsigned short*>(inverse + (16 * block + r) * Plan::inverse_row + c);
@@ -263,7 +273,8 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
     const uint32_t matrix_at = smem_u32(matrix) + lanes_by_row(kRow), inverse_at = smem_u32(inverse) + lanes_by_row(Plan::inverse_row),
                    solved_at = smem_u32(solved) + column0 * 2 + lanes_by_row(Plan::right_row);
     float fit = 0.0f;
-#pragma unroll
+    // (Rolled loops: see move_up.)
+#pragma unroll 1
     for (int block = 0; block < kChunk / 16; ++block) {
         const int row0 = 16 * block < Plan::solved_rows ? 16 * block : 0;
         float acc[kTiles][4] = {};
@@ -276,15 +287,20 @@ delta_chunks_solve_kernel(const DeltaChunkArgs args) {
                 split_products(acc[n], acc[n + 1], a, b);
             }
         };
-#pragma unroll
+#pragma unroll 1
         for (int c = 0; c < block; ++c) accumulate(matrix_at + (16 * block * kRow + 16 * c) * 2, kPlane, 16 * c);
         __syncwarp();
         bf16* mine = solved + (row0 + group) * Plan::right_row + column0 + pair;
 #pragma unroll
         for (int n = 0; n < kTiles; ++n) {
-            split_two(right[block][n][0] - acc[n][0], right[block][n][1] - acc[n][1], mine + 8 * n, Plan::right_plane);
-            split_two(right[block][n][2] - acc[n][2], right[block][n][3] - acc[n][3], mine + 8 * Plan::right_row + 8 * n, Plan::right_plane);
-            acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+            split_two(right[0][n][0] - acc[n][0], right[0][n][1] - acc[n][1], mine + 8 * n, Plan::right_plane);
+            split_two(right[0][n][2] - acc[n][2], right[0][n][3] - acc[n][3], mine + 8 * Plan::right_row + 8 * n, Plan::right_plane);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc[n][i] = 0.0f;
+#pragma unroll
+                for (int r = 0; r + 1 < kChunk / 16; ++r) right[r][n][i] = right[r + 1][n][i];  // the next block's to the first place
+            }
         }
         __syncwarp();
         accumulate(inverse_at + 16 * block * Plan::inverse_row * 2, Plan::inverse_plane, row0);
@@ -535,7 +551,7 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
     const uint32_t wide_at = base + (Plan::wide + column0) * 2 + lanes_by_row(Plan::wide_row);
     float acc[V / 16][4] = {}, weights[kChunk / 8][4] = {};
     ask(args.u + at * kChunk * V);  // (arrives while the start is multiplied)
-#pragma unroll
+#pragma unroll 1
     for (int d = 0; d < kDim; d += 16) {
         Parts a, b;
         load_parts(a, query_at + d * 2, kPlane);
@@ -547,7 +563,7 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
     }
     __syncthreads();  // nobody reads the start any more
     const float fit = put();
-#pragma unroll
+#pragma unroll 1
     for (int d = 0; d < kDim; d += 16) {
         Parts a, b;
         load_parts(a, query_at + d * 2, kPlane);
@@ -565,26 +581,26 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[n][i] = __fmul_rn(acc[n][i], from_start[i / 2]);  // (rounded by itself, whatever follows)
     const bool spoiled = __syncthreads_or(!isfinite(fit));
+#pragma unroll 1
+    for (int n = 0; n <= 2 * warp; n += 2) {
 #pragma unroll
-    for (int n = 0; n < kChunk / 8; n += 2) {
-        if (n > 2 * warp) break;
-#pragma unroll
-        for (int m = n; m < n + 2; ++m)
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int to = row + 8 * (i / 2), from = 8 * m + pair + i % 2;
+                const int to = row + 8 * (i / 2), from = 8 * (n + m) + pair + i % 2;
                 weights[m][i] = from <= to ? weights[m][i] * expf((float)(logs[to] - logs[from])) : 0.0f;
             }
         Parts a, b;
-        split_pair(weights[n][0], weights[n][1], a[0][0], a[1][0], a[2][0]);
-        split_pair(weights[n][2], weights[n][3], a[0][1], a[1][1], a[2][1]);
-        split_pair(weights[n + 1][0], weights[n + 1][1], a[0][2], a[1][2], a[2][2]);
-        split_pair(weights[n + 1][2], weights[n + 1][3], a[0][3], a[1][3], a[2][3]);
+        split_pair(weights[0][0], weights[0][1], a[0][0], a[1][0], a[2][0]);
+        split_pair(weights[0][2], weights[0][3], a[0][1], a[1][1], a[2][1]);
+        split_pair(weights[1][0], weights[1][1], a[0][2], a[1][2], a[2][2]);
+        split_pair(weights[1][2], weights[1][3], a[0][3], a[1][3], a[2][3]);
 #pragma unroll
         for (int c = 0; c < V / 16; c += 2) {
             load_parts_turned(b, wide_at + (8 * n * Plan::wide_row + 8 * c) * 2, Plan::wide_plane);
             split_products(acc[c], acc[c + 1], a, b);
         }
+        move_up<2>(weights);
     }
     if (spoiled) {  // a row of u that is not finite: see causal_products
         const bf16 *queries = planes + Plan::queries, *keys = planes + Plan::keys;
@@ -596,7 +612,18 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
             for (int i = 0; i < 4; ++i) acc[n][i] *= from_start[i / 2];
         causal_products(acc, row, weight, planes + Plan::wide + column0 + pair, Plan::wide_row, Plan::wide_plane);
     }
-    // norm, gain and gate: a row's V results lie with four neighbouring lanes of two warps
+    // norm, gain and gate: a row's V results lie with four neighbouring lanes of two warps.  Gates and gains are asked for at once, before the
+    // sums: one after another, each behind a store and a division, they were 20,000 of a block's 52,000 cycles.
+    const size_t column = (size_t)head * V + column0 + pair;
+    Pair<T> gates[2][V / 16];
+    float2 gain[V / 16];
+#pragma unroll
+    for (int n = 0; n < V / 16; ++n) {
+        gain[n] = load_pair(args.gain + column0 + 8 * n + pair);
+#pragma unroll
+        for (int half = 0; half < 2; ++half)  // (rows beyond the chunk's last: that one's, and not used)
+            gates[half][n] = *reinterpret_cast<const Pair<T>*>((const T*)args.gate_in + (token0 + min(row + 8 * half, count - 1)) * args.in_stride + column + 8 * n);
+    }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         float squares = 0.0f;
@@ -612,13 +639,18 @@ delta_chunks_results_kernel(const DeltaChunkArgs args) {
         const int to = row + 8 * half;
         if (to >= count) continue;
         const float inv = args.out_scale / sqrtf((square_sums[0][to] + square_sums[1][to]) / (float)V + args.eps);
-        const size_t column = (size_t)head * V + column0 + pair;
-        const T* gate = (const T*)args.gate_in + (token0 + to) * args.in_stride + column;
         T* dst = (T*)args.out + (token0 + to) * args.out_stride + column;
+        float open[V / 8];
 #pragma unroll
         for (int n = 0; n < V / 16; ++n) {
-            const float2 z = load_pair(gate + 8 * n), gain = load_pair(args.gain + column0 + 8 * n + pair);
-            store_pair(dst + 8 * n, acc[n][2 * half] * inv * gain.x * (z.x * sigmoid(z.x)), acc[n][2 * half + 1] * inv * gain.y * (z.y * sigmoid(z.y)));
+            const float2 z = load_pair(reinterpret_cast<const T*>(&gates[half][n]));
+            open[2 * n] = z.x, open[2 * n + 1] = z.y;
+        }
+        sigmoids(open);
+#pragma unroll
+        for (int n = 0; n < V / 16; ++n) {
+            const float2 z = load_pair(reinterpret_cast<const T*>(&gates[half][n]));
+            store_pair(dst + 8 * n, acc[n][2 * half] * inv * gain[n].x * (z.x * open[2 * n]), acc[n][2 * half + 1] * inv * gain[n].y * (z.y * open[2 * n + 1]));
         }
     }
 }

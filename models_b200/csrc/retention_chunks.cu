@@ -10,8 +10,8 @@
 // Against 64 bits, over steps of 64 to 2,048 tokens: the state is off by 6e-8 to 9e-8 of itself (the walk in runs: 0.9e-7 to 1.4e-7), the
 // raw results by 0.7e-7 to 1.1e-7 (0.8e-7 to 1.8e-7); with two parts the operands would be cut to 16 bits.
 // Three sequences of 2,048 tokens in all, 16 heads of 64 x 128 with activated projections: 208 us as the walk in runs (98, 70 and 40),
-// which float multiply-adds from shared memory bound; here 29, 14 and 54 us (sums of products added one by one: 32, 14 and 58), bound by the six products for one and by the
-// instructions that activate and split what every chunk reads.
+// which float multiply-adds from shared memory bound; here 24, 14 and 49 us (29, 14 and 54 with a division for every activation and a block's
+// rows asked for one after the other), bound by the six products for one and by the instructions that activate and split what every chunk reads.
 #include "common.cuh"
 #include "gate_pairs.cuh"
 #include "split_products.cuh"
@@ -101,13 +101,16 @@ struct RawRows {
             if (row < count) raw[i] = *reinterpret_cast<const uint4*>(src + (size_t)row * stride + piece % (kCols / 8) * 8);
         }
     }
-    // Returns a sum that is finite only where every number is, and has three finite parts.
-    __device__ __forceinline__ float put(bf16* planes, int row_numbers, int plane_numbers, int activation, int count, const float* weight) const {
+    // Returns a sum that is finite only where every number is, and has three finite parts.  The pieces side by side, or (kOneByOne) by one body
+    // of code: adds 23.0 -> 21.4 us so, but results of short steps 22.0 -> 24.2.
+    template <bool kOneByOne>
+    __device__ __forceinline__ float put(bf16* planes, int row_numbers, int plane_numbers, int activation, int count, const float* weight) {
         float fit = 0.0f;
-#pragma unroll
+#pragma unroll (kOneByOne ? 1 : kPieces)
         for (int i = 0; i < kPieces; ++i) {
             const int piece = threadIdx.x + i * kThreads, row = piece / (kCols / 8);
-            const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+            const uint32_t w[4] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w};
+            move_up<1>(raw);
             float x[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) x[2 * j] = __uint_as_float(w[j] << 16), x[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
@@ -146,16 +149,16 @@ retention_chunk_adds_kernel(const RetentionArgs args) {
     v.ask(args.v + token0 * args.in_stride + (size_t)head * V, args.in_stride, count);
     if (args.rotary_dim == 0) k.ask(key_rows, args.in_stride, count);
     if (tid < kChunk) weight[tid] = tid < count ? args.key_scale * powf(args.decay[head], (float)(count - 1 - tid)) : 0.0f;
-    v.put(values, Values<V>::row, Values<V>::plane, args.input_act, count, nullptr);
+    v.template put<true>(values, Values<V>::row, Values<V>::plane, args.input_act, count, nullptr);
     __syncthreads();
-    if (args.rotary_dim == 0) k.put(keys, kKeyRow, kKeyPlane, args.input_act, count, weight);
+    if (args.rotary_dim == 0) k.template put<true>(keys, kKeyRow, kKeyPlane, args.input_act, count, weight);
     else stage_rows<kDim>(keys, kKeyRow, kKeyPlane, key_rows, args, count, args.rotary_dim, args.positions[first] + chunk * kChunk, weight);
     __syncthreads();
     const int tile = (tid >> 5) & 3, column0 = (tid >> 7) * (V / 2), lane = tid & 31;
     float acc[V / 16][4] = {};
     const uint32_t key_at = smem_u32(keys) + (((lane >> 4) * 8 + (lane & 7)) * kKeyRow + 16 * tile + ((lane >> 3) & 1) * 8) * 2;
     const uint32_t value_at = smem_u32(values) + ((lane & 15) * Values<V>::row + column0 + (lane >> 4) * 8) * 2;
-#pragma unroll
+#pragma unroll 1
     for (int j = 0; j < kChunk; j += 16) {
         Parts a, b;
         load_parts_turned(a, key_at + j * kKeyRow * 2, kKeyPlane);
@@ -237,8 +240,8 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         v.ask(args.v + token0 * args.in_stride + (size_t)head * V, args.in_stride, count);
         if (tid <= kChunk) power[tid] = powf(args.decay[head], (float)tid);
         if (args.rotary_dim == 0) {
-            q.put(queries, kKeyRow, kKeyPlane, args.input_act, count, nullptr);
-            k.put(keys, kKeyRow, kKeyPlane, args.input_act, count, nullptr);
+            q.template put<false>(queries, kKeyRow, kKeyPlane, args.input_act, count, nullptr);
+            k.template put<false>(keys, kKeyRow, kKeyPlane, args.input_act, count, nullptr);
         } else {
             const int position0 = args.positions[first] + chunk * kChunk;
             stage_rows<kDim>(queries, kKeyRow, kKeyPlane, query_rows, args, count, args.rotary_dim, position0, nullptr);
@@ -256,7 +259,7 @@ retention_chunk_results_kernel(const RetentionArgs args) {
     const uint32_t wide_at = smem_u32(wide) + ((lane & 15) * kRow + column0 + (lane >> 4) * 8) * 2;  // [k][column] tiles of V columns
     const uint32_t key_at = smem_u32(keys) + (((lane >> 4) * 8 + (lane & 7)) * kKeyRow + ((lane >> 3) & 1) * 8) * 2;
     float acc[V / 16][4] = {}, weights[kChunk / 8][4] = {};
-#pragma unroll
+#pragma unroll 1
     for (int d = 0; d < kDim; d += 16) {
         Parts a, b;
         load_parts(a, query_at + d * 2, kKeyPlane);
@@ -273,33 +276,33 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         }
     }
     __syncthreads();  // nobody reads the start any more
-    const float fit = v.put(wide, kRow, kPlane, args.input_act, count, nullptr);
+    const float fit = v.template put<false>(wide, kRow, kPlane, args.input_act, count, nullptr);
     const bool spoiled = __syncthreads_or(!isfinite(fit));
     const int row = 16 * warp + group;
 #pragma unroll
     for (int n = 0; n < V / 16; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[n][i] *= power[row + 8 * (i / 2) + 1];
+#pragma unroll 1
+    for (int n = 0; n <= 2 * warp; n += 2) {
 #pragma unroll
-    for (int n = 0; n < kChunk / 8; n += 2) {
-        if (n > 2 * warp) break;
-#pragma unroll
-        for (int m = n; m < n + 2; ++m)
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int age = row + 8 * (i / 2) - (8 * m + pair + i % 2);
+                const int age = row + 8 * (i / 2) - (8 * (n + m) + pair + i % 2);
                 weights[m][i] = age >= 0 ? weights[m][i] * (args.key_scale * power[max(age, 0)]) : 0.0f;
             }
         Parts a, b;
-        split_pair(weights[n][0], weights[n][1], a[0][0], a[1][0], a[2][0]);
-        split_pair(weights[n][2], weights[n][3], a[0][1], a[1][1], a[2][1]);
-        split_pair(weights[n + 1][0], weights[n + 1][1], a[0][2], a[1][2], a[2][2]);
-        split_pair(weights[n + 1][2], weights[n + 1][3], a[0][3], a[1][3], a[2][3]);
+        split_pair(weights[0][0], weights[0][1], a[0][0], a[1][0], a[2][0]);
+        split_pair(weights[0][2], weights[0][3], a[0][1], a[1][1], a[2][1]);
+        split_pair(weights[1][0], weights[1][1], a[0][2], a[1][2], a[2][2]);
+        split_pair(weights[1][2], weights[1][3], a[0][3], a[1][3], a[2][3]);
 #pragma unroll
         for (int c = 0; c < V / 16; c += 2) {
             load_parts_turned(b, wide_at + (8 * n * kRow + 8 * c) * 2, kPlane);
             split_products(acc[c], acc[c + 1], a, b);
         }
+        move_up<2>(weights);
     }
     if (spoiled) {  // a value that is not finite: see causal_products
         auto weight = [&](int token, int from) {
@@ -339,11 +342,18 @@ retention_chunk_results_kernel(const RetentionArgs args) {
         } else {
             const bf16* gate = args.g + (token0 + to) * args.in_stride + column;
             bf16* dst = args.out + (token0 + to) * args.out_stride + column;
+            uint32_t raw[V / 16];  // (all of them before the first store: one by one each waited for itself)
 #pragma unroll
-            for (int n = 0; n < V / 16; ++n) {
-                const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gate + 8 * n));
-                *reinterpret_cast<__nv_bfloat162*>(dst + 8 * n) = __floats2bfloat162_rn(acc[n][2 * half] * factor * (z.x / (1.0f + expf(-z.x))),
-                                                                                       acc[n][2 * half + 1] * factor * (z.y / (1.0f + expf(-z.y))));
+            for (int n = 0; n < V / 16; ++n) raw[n] = *reinterpret_cast<const uint32_t*>(gate + 8 * n);
+#pragma unroll
+            for (int n = 0; n < V / 16; n += 2) {
+                float z[4] = {__uint_as_float(raw[n] << 16), __uint_as_float(raw[n] & 0xffff0000u), __uint_as_float(raw[n + 1] << 16), __uint_as_float(raw[n + 1] & 0xffff0000u)};
+                const float ones[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+                gate_pairs(MB_ACT_SILU, z, ones, ClampedPair{});
+#pragma unroll
+                for (int m = n; m < n + 2; ++m)
+                    *reinterpret_cast<__nv_bfloat162*>(dst + 8 * m) =
+                        __floats2bfloat162_rn(acc[m][2 * half] * factor * z[2 * (m - n)], acc[m][2 * half + 1] * factor * z[2 * (m - n) + 1]);
             }
         }
     }
