@@ -515,6 +515,13 @@ __global__ void project_norm_rotate_store_vec8_kernel(T* __restrict__ q, int q_s
 // position (pairs (i, i + turned / 2), tables [positions][turned / 2]) -- into the pool at the token's slot.  For a prompt that reads
 // its own rows (prompt.latent given) the row is also left in the step's order, [tokens][latent] and [tokens][padded] with zeros behind
 // the tail, and the other warps rotate the query heads' tails into [tokens][heads * padded].
+//
+// A prompt on top of cached positions reads `rows_per` rows of every sequence (prompt.rows_per > 0): the step's own go to their places among
+// them, and the blocks behind the tokens' copy what is cached, kCopies rows a warp.  A sequence's first row is the position 0,
+// or with a window the multiple of 64 at or before the first position that the step's first token sees: what lies before it may be gone
+// from the cache.  Rows behind the sequence's end are left as they are, but for those up to the next multiple of 64, which become zeros.
+// (Bound by its launch and its memory; by itself the copy took a launch, 4 us and 15 us of the host's time more.)
+constexpr int kCopies = 4;
 struct PromptRows {
     void* latent;         // [tokens][latent]
     void* tail;           // [tokens][padded], null where there is no tail
@@ -522,7 +529,50 @@ struct PromptRows {
     int q_stride, q_head, heads;
     void* q_tail;         // [tokens][heads * padded]
     int padded;
+    int tokens, rows_per;         // rows_per 0: the rows in the step's order
+    const int* block_table;       // [sequences][max_blocks]
+    int max_blocks, page_size;
+    const int *cu_q, *kv_lens;    // cu_q null: nothing but the copy, of all positions
+    int sequences, window;
 };
+// The position that sequence `seq`'s first row of rows_per holds, and how many of its positions were cached before the step.
+__device__ __forceinline__ int first_position(const PromptRows& prompt, int seq, int* cached) {
+    const int length = prompt.kv_lens[seq], brought = prompt.cu_q != nullptr ? prompt.cu_q[seq + 1] - prompt.cu_q[seq] : 0;
+    const int seen = prompt.window > 0 ? length - brought - prompt.window + 1 : 0;
+    *cached = length - brought;
+    return seen > 0 ? seen / 64 * 64 : 0;
+}
+__device__ __forceinline__ void copy_cached_rows(const uint4* pool, int latent, int turned, const PromptRows& prompt) {
+    const int latent_pieces = latent / 8, row_pieces = (latent + turned) / 8, tail_pieces = turned > 0 ? prompt.padded / 8 : 0;
+    const int row0 = ((blockIdx.x - prompt.tokens) * 4 + (threadIdx.x >> 5)) * kCopies;
+    const uint4* from[kCopies];  // null: zeros
+    bool wanted[kCopies];
+#pragma unroll
+    for (int j = 0; j < kCopies; ++j) {
+        const int seq = (row0 + j) / prompt.rows_per;
+        from[j] = nullptr;
+        wanted[j] = seq < prompt.sequences;
+        if (!wanted[j]) continue;
+        int cached;
+        const int position = first_position(prompt, seq, &cached) + (row0 + j) % prompt.rows_per, length = prompt.kv_lens[seq];
+        wanted[j] = position < (length + 63) / 64 * 64 && !(position >= cached && position < length && prompt.tokens > 0);
+        if (wanted[j] && position < length) {
+            const size_t page = prompt.block_table[(size_t)seq * prompt.max_blocks + position / prompt.page_size];
+            from[j] = pool + (page * prompt.page_size + position % prompt.page_size) * row_pieces;
+        }
+    }
+    for (int piece = threadIdx.x & 31; piece < latent_pieces + tail_pieces; piece += 32) {
+        uint4 v[kCopies];
+#pragma unroll
+        for (int j = 0; j < kCopies; ++j) v[j] = from[j] != nullptr && piece < row_pieces ? from[j][piece] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int j = 0; j < kCopies; ++j) {
+            if (!wanted[j]) continue;
+            if (piece < latent_pieces) ((uint4*)prompt.latent)[(size_t)(row0 + j) * latent_pieces + piece] = v[j];
+            else ((uint4*)prompt.tail)[(size_t)(row0 + j) * tail_pieces + piece - latent_pieces] = v[j];
+        }
+    }
+}
 
 template <typename T, bool kVector>
 __global__ void __launch_bounds__(128)
@@ -530,6 +580,11 @@ latent_rows_kernel(const T* __restrict__ k, int k_stride, const float* __restric
                    const float* __restrict__ sin, const int* __restrict__ positions, float eps, T* __restrict__ k_pool,
                    const int* __restrict__ slot_mapping, PromptRows prompt) {
     grid_launch_dependents();
+    if (prompt.rows_per > 0 && blockIdx.x >= prompt.tokens) {
+        grid_dependency_wait();
+        copy_cached_rows(reinterpret_cast<const uint4*>(k_pool), latent, turned, prompt);
+        return;
+    }
     const size_t token = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = turned / 2;
     const float* cos_row = nullptr;
@@ -542,11 +597,26 @@ latent_rows_kernel(const T* __restrict__ k, int k_stride, const float* __restric
     const int slot = warp == 0 ? slot_mapping[token] : -1;
     grid_dependency_wait();
     if (warp == 0) {
-        if (slot < 0 && prompt.latent == nullptr) return;
+        long long own_row = prompt.latent != nullptr ? (long long)token : -1;
+        if (prompt.rows_per > 0) {  // the token's place among its sequence's rows (none for one that no sequence has)
+            own_row = -1;
+            int seq = 0, behind = prompt.sequences;  // the sequence is among [seq, behind)
+            while (behind - seq > 1) {
+                const int middle = (seq + behind) / 2;
+                if ((int)token >= prompt.cu_q[middle]) seq = middle;
+                else behind = middle;
+            }
+            if ((int)token >= prompt.cu_q[seq] && (int)token < prompt.cu_q[seq + 1]) {
+                int cached;
+                const int first = first_position(prompt, seq, &cached), at = cached + (int)token - prompt.cu_q[seq] - first;
+                if (at >= 0 && at < prompt.rows_per) own_row = (long long)seq * prompt.rows_per + at;
+            }
+        }
+        if (slot < 0 && own_row < 0) return;
         const T* src = k + token * k_stride;
         T* row = slot >= 0 ? k_pool + (size_t)slot * (latent + turned) : nullptr;  // [page][1][page_size][latent + turned]: the slot counts rows
-        T* own = prompt.latent != nullptr ? (T*)prompt.latent + token * latent : nullptr;
-        T* own_tail = prompt.latent != nullptr && turned > 0 ? (T*)prompt.tail + token * prompt.padded : nullptr;
+        T* own = own_row >= 0 ? (T*)prompt.latent + own_row * latent : nullptr;
+        T* own_tail = own_row >= 0 && turned > 0 ? (T*)prompt.tail + own_row * prompt.padded : nullptr;
         float squares = 0.0f;
         if (kVector) {
             for (int i = lane * 8; i < latent; i += 256) {
@@ -1719,12 +1789,14 @@ static int launch_latent_rows(const void* k, int k_stride, const float* gain, in
     const bool wide = latent % 8 == 0 && turned % 8 == 0 && k_stride % 8 == 0 && prompt.padded % 8 == 0 && prompt.q_stride % 8 == 0 && prompt.q_head % 8 == 0 &&
                       !(((uintptr_t)k | (uintptr_t)k_pool | (uintptr_t)prompt.latent | (uintptr_t)prompt.q | (uintptr_t)prompt.q_tail) & row_bytes) &&
                       !(((uintptr_t)gain | (uintptr_t)cos | (uintptr_t)sin) & 15);
-    const dim3 block(prompt.latent != nullptr && turned > 0 ? 128 : 32);
+    const dim3 block(prompt.latent != nullptr && (turned > 0 || prompt.rows_per > 0) ? 128 : 32);
+    const long long rows = (long long)prompt.sequences * prompt.rows_per, blocks = tokens + (rows + 4 * kCopies - 1) / (4 * kCopies);
+    if (rows > 0x3fffffff || blocks > 0x7fffffff) return fail("latent_rows: %d tokens and %d rows of each of %d sequences exceed the grid", tokens, prompt.rows_per, prompt.sequences);
     if (wide)
-        MB_LAUNCH("latent_rows", (latent_rows_kernel<T, true>), dim3(tokens), block, 0, stream, true, (const T*)k, k_stride, gain, latent, turned,
+        MB_LAUNCH("latent_rows", (latent_rows_kernel<T, true>), dim3((unsigned)blocks), block, 0, stream, true, (const T*)k, k_stride, gain, latent, turned,
                   cos, sin, positions, eps, (T*)k_pool, slot_mapping, prompt);
     else
-        MB_LAUNCH("latent_rows", (latent_rows_kernel<T, false>), dim3(tokens), block, 0, stream, true, (const T*)k, k_stride, gain, latent, turned,
+        MB_LAUNCH("latent_rows", (latent_rows_kernel<T, false>), dim3((unsigned)blocks), block, 0, stream, true, (const T*)k, k_stride, gain, latent, turned,
                   cos, sin, positions, eps, (T*)k_pool, slot_mapping, prompt);
     return check_launch("latent_rows");
 }
@@ -1739,11 +1811,31 @@ MB_EXPORT int mb_latent_rows(const void* k, int k_stride, const float* gain, int
     if (latent <= 0 || turned < 0 || turned % 2 || (turned > 0 && (cos == nullptr || sin == nullptr))) return fail("latent_rows: rows of %d and %d numbers", latent, turned);
     if (own_latent != nullptr && turned > 0 && (!own_tail || !q || !q_tail || padded < turned || heads <= 0))
         return fail("latent_rows: a prompt's tails of %d numbers in %d columns need their tensors", turned, padded);
-    const PromptRows prompt{own_latent, own_tail, q, q_stride, q_head, heads, q_tail, padded};
+    const PromptRows prompt{own_latent, own_tail, q, q_stride, q_head, heads, q_tail, padded, tokens, 0, nullptr, 0, 0, nullptr, nullptr, 0, 0};
     if (dtype == MB_F32) return launch_latent_rows<float>(k, k_stride, gain, latent, turned, cos, sin, positions, eps, k_pool, slot_mapping, prompt, tokens, stream);
     if (dtype == MB_BF16)
         return launch_latent_rows<__nv_bfloat16>(k, k_stride, gain, latent, turned, cos, sin, positions, eps, k_pool, slot_mapping, prompt, tokens, stream);
     return fail("latent_rows: unknown dtype code %d", dtype);
+}
+
+// Rows that a step on top of cached positions reads (bfloat16): rows_per (a multiple of 64) of every sequence, latents [sequences *
+// rows_per][latent] and tails [..][padded] (null without a tail), from where the comment at PromptRows says; sizes in numbers, multiples of 8,
+// page_size positions a page.  tokens > 0: the step's own rows are made of k, as mb_latent_rows makes them, and go to the pool and to their
+// places, and its queries' tails to q_tail; tokens 0: every row is in the pool already (cu_q may then be null where there is no window).
+MB_EXPORT int mb_latent_gather(const void* k, int k_stride, const float* gain, int latent, int turned, const float* cos, const float* sin,
+                               const int* positions, float eps, void* k_pool, const int* slot_mapping, const void* q, int q_stride, int q_head,
+                               int heads, void* q_tail, int padded, int tokens, const int* block_table, int max_blocks, int page_size, const int* cu_q,
+                               const int* kv_lens, int sequences, int window, int rows_per, void* latents, void* tails, cudaStream_t stream) {
+    if (sequences <= 0 || rows_per <= 0) return 0;
+    if (latent <= 0 || latent % 8 || turned < 0 || turned % 8 || padded % 8 || padded < turned || (turned > 0 && !tails) || ((uintptr_t)k_pool & 15) ||
+        !latents || ((uintptr_t)latents & 15) || ((uintptr_t)tails & 15) || rows_per % 64 || window < 0 || ((window > 0 || tokens > 0) && !cu_q) ||
+        (long long)max_blocks * page_size < rows_per)
+        return fail("latent_gather: rows of %d and %d numbers (%d with zeros), %d of each of %d sequences", latent, turned, padded, rows_per, sequences);
+    if (tokens < 0 || (tokens > 0 && (!k || !gain || !positions || !slot_mapping || (turned > 0 && (!cos || !sin || !q || !q_tail || heads <= 0)))))
+        return fail("latent_gather: the step's own rows and its queries' tails need their tensors");
+    const PromptRows prompt{latents, tails, q, q_stride, q_head, heads, q_tail, padded, tokens, rows_per, block_table, max_blocks, page_size,
+                            cu_q, kv_lens, sequences, window};
+    return launch_latent_rows<__nv_bfloat16>(k, k_stride, gain, latent, turned, cos, sin, positions, eps, k_pool, slot_mapping, prompt, tokens, stream);
 }
 
 // The second half of mb_gated_attention_decode alone: adds the runs that another kernel left in `partial` (bfloat16 results, softmax).

@@ -15,7 +15,6 @@ LIBRARIES = [
     ("mb_gated_delta", ["gated_delta.cu"], {}),
     ("mb_gated_delta_chunks", ["gated_delta_chunks.cu"], {}),
     ("mb_gated_attention", ["gated_attention.cu"], {}),
-    ("mb_latent_gather", ["latent_gather.cu"], {}),
     ("mb_retention", ["retention.cu"], {}),
     ("mb_retention_chunks", ["retention_chunks.cu"], {}),
     ("mb_result_norm", ["result_norm.cu"], {}),

@@ -1133,6 +1133,30 @@ def latent_prepare(q: Optional[torch.Tensor], q_gain: Optional[torch.Tensor], q_
     return out
 
 
+def _latent_row_checks(name: str, k, gain, turned: int, cos, sin, positions, k_pool, slot_mapping):
+    """Raises unless k [T, latent + turned] can be made cached rows in the pool; (T, latent)."""
+    _cuda(k, gain, cos, sin, positions, k_pool, slot_mapping)
+    _int32(positions, "positions")
+    _int32(slot_mapping, "slot_mapping")
+    _columns(k, "k")
+    rows, latent = k.shape[0], k.shape[1] - turned
+    if gain.dtype != torch.float32 or gain.numel() != latent or not gain.is_contiguous():
+        raise KernelError(f"{name}: rows {tuple(k.shape)} with a tail of {turned} do not fit the gain")
+    if k_pool.dim() != 4 or k_pool.shape[1] != 1 or k_pool.shape[3] != k.shape[1] or not k_pool.is_contiguous() or k_pool.dtype != k.dtype:
+        raise KernelError(f"{name}: the pool must be contiguous [pages, 1, page_size, {k.shape[1]}] of {k.dtype}")
+    if turned:
+        for table in (cos, sin):
+            if table is None or table.dtype != torch.float32 or table.dim() != 2 or table.shape[1] * 2 != turned or not table.is_contiguous():
+                raise KernelError(f"{name}: a tail of {turned} needs contiguous float32 tables [positions, {turned // 2}]")
+    return rows, latent
+
+
+def _latent_query_checks(name: str, q, k, heads: int, head_columns: int, turned: int, padded: int) -> None:
+    _columns(q, "q")
+    if q.dtype != k.dtype or q.shape[0] != k.shape[0] or q.shape[1] < heads * head_columns or head_columns < turned or padded < turned:
+        raise KernelError(f"{name}: queries {tuple(q.shape)} {q.dtype} are no {heads} heads of {head_columns}")
+
+
 def latent_rows(k: torch.Tensor, gain: torch.Tensor, turned: int, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor],
                 positions: torch.Tensor, eps: float, k_pool: torch.Tensor, slot_mapping: torch.Tensor, q: Optional[torch.Tensor] = None,
                 heads: int = 0, head_columns: int = 0, padded: int = 0):
@@ -1141,24 +1165,11 @@ def latent_rows(k: torch.Tensor, gain: torch.Tensor, turned: int, cos: Optional[
     [pages, 1, page_size, latent + turned] at `slot_mapping`.  With `q` (a prompt that reads its own rows): also returns, in the step's
     order, the latents [T, latent], the tails [T, padded] and the query heads' rotated tails [T, heads * padded], zeros behind
     the `turned` numbers (None, None without a tail); head h's tail ends at column (h + 1) * head_columns of q."""
-    _cuda(k, gain, cos, sin, positions, k_pool, slot_mapping, q)
-    _int32(positions, "positions")
-    _int32(slot_mapping, "slot_mapping")
-    _columns(k, "k")
-    rows, latent = k.shape[0], k.shape[1] - turned
-    if gain.dtype != torch.float32 or gain.numel() != latent or not gain.is_contiguous():
-        raise KernelError(f"latent_rows: rows {tuple(k.shape)} with a tail of {turned} do not fit the gain")
-    if k_pool.dim() != 4 or k_pool.shape[1] != 1 or k_pool.shape[3] != k.shape[1] or not k_pool.is_contiguous() or k_pool.dtype != k.dtype:
-        raise KernelError(f"latent_rows: the pool must be contiguous [pages, 1, page_size, {k.shape[1]}] of {k.dtype}")
-    if turned:
-        for table in (cos, sin):
-            if table is None or table.dtype != torch.float32 or table.dim() != 2 or table.shape[1] * 2 != turned or not table.is_contiguous():
-                raise KernelError(f"latent_rows: a tail of {turned} needs contiguous float32 tables [positions, {turned // 2}]")
+    rows, latent = _latent_row_checks("latent_rows", k, gain, turned, cos, sin, positions, k_pool, slot_mapping)
+    _cuda(q)
     own = tail = q_tail = None
     if q is not None:
-        _columns(q, "q")
-        if q.dtype != k.dtype or q.shape[0] != rows or q.shape[1] < heads * head_columns or head_columns < turned or padded < turned:
-            raise KernelError(f"latent_rows: queries {tuple(q.shape)} {q.dtype} are no {heads} heads of {head_columns}")
+        _latent_query_checks("latent_rows", q, k, heads, head_columns, turned, padded)
         own = torch.empty((rows, latent), dtype=k.dtype, device=k.device)
         if turned:
             tail = torch.empty((rows, padded), dtype=k.dtype, device=k.device)
@@ -1172,11 +1183,15 @@ def latent_rows(k: torch.Tensor, gain: torch.Tensor, turned: int, cos: Optional[
 
 
 def latent_gather(k_pool: torch.Tensor, latent: int, padded: int, block_table: torch.Tensor, kv_lens: torch.Tensor, rows_per: int,
-                  cu_q: Optional[torch.Tensor] = None, window: int = 0):
+                  cu_q: Optional[torch.Tensor] = None, window: int = 0, step: Optional[tuple] = None):
     """The rows of a latent attention's sequences in their cache pool [pages, 1, page_size, latent + turned] (bfloat16), `rows_per`
     (a multiple of 64) for every sequence, from its position 0 on, or with a `window` (and the step's `cu_q`) from the multiple of 64 at or
     before the first position that the step's tokens see: latents [sequences * rows_per, latent] and, where there is a tail, tails
-    [sequences * rows_per, padded] with zeros behind the turned numbers.  Rows behind a sequence's last 64 are not written."""
+    [sequences * rows_per, padded] with zeros behind the turned numbers.  Rows behind a sequence's last 64 are not written.
+
+    `step` (k, gain, cos, sin, positions, eps, slot_mapping, q, heads, head_columns, q_tail): the step's own rows are made here, as
+    `latent_rows` makes them, and stored in the pool and in their places among the others; its query heads' rotated tails go into
+    q_tail [T, heads * padded] (None without a tail)."""
     _cuda(k_pool, block_table, kv_lens, cu_q)
     _int32(block_table, "block_table")
     _int32(kv_lens, "kv_lens")
@@ -1184,13 +1199,26 @@ def latent_gather(k_pool: torch.Tensor, latent: int, padded: int, block_table: t
     turned, sequences = k_pool.shape[3] - latent, kv_lens.numel()
     if k_pool.dtype != torch.bfloat16 or k_pool.dim() != 4 or k_pool.shape[1] != 1 or not k_pool.is_contiguous() or turned < 0:
         raise KernelError(f"latent_gather: the pool must be contiguous bfloat16 [pages, 1, page_size, latent + turned], got {tuple(k_pool.shape)} {k_pool.dtype}")
-    if window and (cu_q is None or cu_q.numel() != sequences + 1):
-        raise KernelError("latent_gather: a window needs the step's cu_q")
+    if (window or step is not None) and (cu_q is None or cu_q.numel() != sequences + 1):
+        raise KernelError("latent_gather: a window, and a step's own rows, need the step's cu_q")
+    k = gain = cos = sin = positions = slot_mapping = q = q_tail = None
+    rows = heads = head_columns = 0
+    eps = 0.0
+    if step is not None:
+        k, gain, cos, sin, positions, eps, slot_mapping, q, heads, head_columns, q_tail = step
+        rows, width = _latent_row_checks("latent_gather", k, gain, turned, cos, sin, positions, k_pool, slot_mapping)
+        _latent_query_checks("latent_gather", q, k, heads, head_columns, turned, padded)
+        _cuda(q, q_tail)
+        if width != latent or (turned and (q_tail is None or tuple(q_tail.shape) != (rows, heads * padded) or not q_tail.is_contiguous() or q_tail.dtype != k.dtype)):
+            raise KernelError(f"latent_gather: rows of {width} numbers, or the queries' tails, do not fit {latent} and [{rows}, {heads * padded}]")
     latents = torch.empty((sequences * rows_per, latent), dtype=k_pool.dtype, device=k_pool.device)
     tails = torch.empty((sequences * rows_per, padded), dtype=k_pool.dtype, device=k_pool.device) if turned else None
-    lib = load_library("mb_latent_gather", ["latent_gather.cu"])
-    _run(lib, lib.mb_latent_gather(_p(k_pool), latent, turned, int(padded), _p(block_table), block_table.shape[1], k_pool.shape[2], _p(cu_q),
-                                   _p(kv_lens), sequences, int(window), int(rows_per), _p(latents), _p(tails), _stream()))
+    lib = gated_attention_library()
+    _run(lib, lib.mb_latent_gather(_p(k), k.stride()[0] if k is not None else 0, _p(gain), latent, turned, _p(cos) if turned else None,
+                                   _p(sin) if turned else None, _p(positions), ctypes.c_float(eps), _p(k_pool), _p(slot_mapping), _p(q),
+                                   q.stride()[0] if q is not None else 0, head_columns - turned, heads, _p(q_tail), int(padded), rows,
+                                   _p(block_table), block_table.shape[1], k_pool.shape[2], _p(cu_q), _p(kv_lens), sequences, int(window), int(rows_per),
+                                   _p(latents), _p(tails), _stream()))
     return latents, tails
 
 

@@ -166,11 +166,14 @@ class LatentAttentionMixer(SplitPart, Mixer):
         s = self.spec
         if q.stride()[0] % 8 or q.data_ptr() % 16:
             q = q.contiguous()
-        own, tail, q_tail = ops.latent_rows(down, self.latent_gain, self.turned, cos, sin, batch.positions, s.eps, run.k_pool, group.slot_mapping,
-                                            q=q, heads=s.num_heads, head_columns=s.head_dim + self.turned, padded=_whole(self.turned))
+        padded, head_columns = _whole(self.turned), s.head_dim + self.turned
         if key_rows:
-            own, tail = ops.latent_gather(run.k_pool, s.latent_dim, _whole(self.turned), group.block_table, batch.kv_lens, key_rows, batch.cu_q,
-                                          s.window or 0)
+            q_tail = torch.empty((q.shape[0], s.num_heads * padded), dtype=q.dtype, device=q.device) if self.turned else None
+            own, tail = ops.latent_gather(run.k_pool, s.latent_dim, padded, group.block_table, batch.kv_lens, key_rows, batch.cu_q, s.window or 0,
+                                          (down, self.latent_gain, cos, sin, batch.positions, s.eps, group.slot_mapping, q, s.num_heads, head_columns, q_tail))
+        else:
+            own, tail, q_tail = ops.latent_rows(down, self.latent_gain, self.turned, cos, sin, batch.positions, s.eps, run.k_pool, group.slot_mapping,
+                                                q=q, heads=s.num_heads, head_columns=head_columns, padded=padded)
         expanded = linear(own, self.expand, own.dtype)
         at = s.num_heads * _whole(s.head_dim)
         ops.prompt_attention(q, q_tail, expanded[:, :at], expanded[:, at:], tail, mid, batch.cu_q, batch.kv_lens, batch.max_q_len, s.num_heads,

@@ -482,6 +482,47 @@ def test_latent_rows_for_the_cache_and_for_the_step(cuda_device, latent_dim, tur
                 assert scaled_error(got[..., :turned].double().cpu(), q_tail) < bound and bool((got[..., turned:] == 0).all())
 
 
+@pytest.mark.parametrize("latent_dim,turned", [(128, 64), (64, 0), (256, 16)])
+@pytest.mark.parametrize("window", [0, 1, 90])
+def test_rows_gathered_with_the_steps_own(cuda_device, latent_dim, turned, window):
+    """The step's rows made on their way to their places are, bit for bit, those that the pool's rows are copied to after they were stored;
+    lengths around the multiples of 64, a step's token that no sequence has, a sequence that brings none."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(latent_dim + window)
+    heads, dim, padded, per = 3, 40, -(-turned // 64) * 64, 320
+    lens, brought = [64, 130, 5, 255, 65], [64, 1, 5, 63, 0]
+    T = sum(brought) + 1
+    width = latent_dim + turned
+    normal = lambda *shape: torch.randn(*shape, generator=g).bfloat16().to(cuda_device)  # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda_device)  # noqa: E731
+    table = (torch.randperm(25, generator=g) + 1).view(5, 5).to(torch.int32)
+    positions = [n - b + i for n, b in zip(lens, brought) for i in range(b)]
+    slots = [int(table[s, p // 64]) * 64 + p % 64 for s, (n, b) in enumerate(zip(lens, brought)) for p in range(n - b, n)]
+    k, q, pool = normal(T, width), normal(T, heads * (dim + turned)), normal(26, 1, 64, width)
+    gain = (1 + 0.3 * torch.randn(latent_dim, generator=g)).to(cuda_device)
+    angle = torch.rand(256, max(turned // 2, 1), generator=g) * 6
+    tables = tuple(f(angle).to(cuda_device) if turned else None for f in (torch.cos, torch.sin))
+    cu = i32(np.concatenate([[0], np.cumsum(brought)]).tolist())
+    results = []
+    for fused in (True, False):
+        mine = pool.clone()
+        rest = (i32(positions + [7]), 1e-5, mine, i32(slots + [-1]))
+        if fused:
+            q_tail = torch.empty(T, heads * padded, dtype=torch.bfloat16, device=cuda_device) if turned else None
+            latents, tails = ops.latent_gather(mine, latent_dim, padded, table.to(cuda_device), i32(lens), per, cu, window,
+                                               (k, gain, *tables, rest[0], rest[1], rest[3], q, heads, dim + turned, q_tail))
+        else:
+            _, _, q_tail = ops.latent_rows(k, gain, turned, *tables, *rest, q=q, heads=heads, head_columns=dim + turned, padded=padded)
+            latents, tails = ops.latent_gather(mine, latent_dim, padded, table.to(cuda_device), i32(lens), per, cu, window)
+        kept = [mine] + ([q_tail] if turned else [])
+        for i, (n, b) in enumerate(zip(lens, brought)):
+            first = max(0, n - b - window + 1) // 64 * 64 if window else 0
+            kept += [t[i * per:i * per + -(-n // 64) * 64 - first] for t in (latents, tails) if t is not None]
+        results.append(kept)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 CUTS = ([200], [2, 60, 1, 77, 60], [70] + [1] * 130)
 MIXERS = {
     "latent-small": latent(4, 16, 8, 8, 32, 0.3, 10000.0, 0), "latent-cores": latent(2, 64, 16, 32, 112, 0.11, 20000.0, 0),
