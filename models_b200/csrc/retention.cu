@@ -23,6 +23,7 @@
 // states follow from the stored state in run order, S_(r+1) = decay^(n_r) S_r + B_r (the last one is the sequence's new
 // state); then every run walks its tokens again from its starting state and writes the results.
 #include "common.cuh"
+#include "gate_pairs.cuh"
 
 MB_DEFINE_LAST_ERROR()
 
@@ -375,11 +376,13 @@ group_norm_gate_vec8_kernel(const float* __restrict__ raw, int raw_stride, const
         if (c >= width) break;
         float scale[8];
         load8(gain + c, scale);
+        // (Divided side by side: 64 rows of 2,048 2.3 -> 2.0 us, of 4,096 3.3 -> 2.7, 2,048 of 4,096 18.8 -> 15.8; 2,048 of 2,048 7.1 and 7.2.)
+        float s[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float s = 1.0f / (1.0f + expf(-g[i][j]));
-            x[i][j] = x[i][j] * inverse * scale[j] * (gate_sigmoid ? s : g[i][j] * s);
-        }
+        for (int j = 0; j < 8; ++j) s[j] = g[i][j];
+        sigmoids(s);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[i][j] = x[i][j] * inverse * scale[j] * (gate_sigmoid ? s[j] : g[i][j] * s[j]);
         store8(out + row * out_stride + c, x[i]);
     }
 }
