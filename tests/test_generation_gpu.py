@@ -405,6 +405,28 @@ def test_sampling_with_few_candidates_at_the_edges_of_its_rule(cuda_device, voca
         assert got[row] == want, (row, o, got[row], want)
 
 
+@pytest.mark.parametrize("scale,temperature", [(s, t) for s in (1e-39, 1e-25, 1.0, 1e20, 1e36) for t in (1e-12, 0.37, 1.0, 1.9, 3e10)
+                                               if s / t < 1e37])  # (beyond the floats no order is left to draw from)
+def test_sampling_divides_by_the_temperature_as_a_division_does(cuda_device, scale, temperature):
+    """Logits near the ends of the floats and zeros among usual ones, whole fours and not: the tokens of the plain pipeline, whose quotients
+    are divisions; where every exponential is 1 the lower ids tie.  (Quotients are ordinary or below 2^-30: between, 2^-20 to 2^-27, numpy's and
+    the kernel's exponentials order neighbours by their last bit, whatever the quotients.)"""
+    from models_b200.sampling import BatchSampler, RequestSampling, SamplingOptions, philox_uniform
+
+    vocab = 4103
+    g = torch.Generator().manual_seed(17)
+    logits = torch.randn(4, vocab, generator=g) * 3 * scale
+    logits[1, ::5] = 0.0
+    logits[2] = torch.randn(vocab, generator=g)
+    logits[2, 40] = 2.0 * scale
+    logits[3, 100:] = -float("inf")
+    options = [SamplingOptions(temperature=temperature, top_k=k, top_p=p, seed=k) for k, p in ((40, 0.9), (5, 1.0), (128, 0.8), (64, 0.95))]
+    with np.errstate(all="ignore"):
+        wants = [expected_draw(logits[i].numpy(), [], o, philox_uniform(o.seed, 0))[0] for i, o in enumerate(options)]
+    got = BatchSampler(vocab, "cuda:0").sample(logits.cuda(), [RequestSampling(o, [0]) for o in options]).tolist()
+    assert got == wants
+
+
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 @pytest.mark.parametrize("top_p", [0.9, 1.0])
 def test_a_row_without_an_order_takes_its_first_maximum(cuda_device, value, top_p):
