@@ -445,7 +445,9 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
 // They are gathered while the exponentials are summed; should more reach it than can be sorted, the histograms decide, and at once where
 // fewer warps than k have a finite value (rows masked to ten finite values, 1 and 64 rows: 39.7 and 133 us; 47.6 and 152 before that was
 // looked at).
-// (64 rows of 128,256, k 20 to 64: 119 us with histograms and one block a multiprocessor, 53 with this and two.)
+// (64 rows of 128,256, k 20 to 64: 119 us with histograms and one block a multiprocessor, 53 with this and two, 41.6 since maxima carry no
+// index, quotients are corrected reciprocals and a sum's exponentials are not stored: 110 instructions a logit had been its bound.  What
+// bounds it now is a chain of passes, cluster barriers and the first block's draw, in two rounds of clusters; one row takes 13.4 us.)
 constexpr int kSampleBlocks = 8;
 constexpr int kFewCandidates = 128;
 constexpr int kAloneBlocks = 64;  // so many blocks, clusters of eight, find a multiprocessor each with certainty
@@ -937,7 +939,7 @@ MB_EXPORT int mb_sample_rows(const float* logits, int row_stride, int rows, int 
     const size_t slice_bytes = (size_t)((vocab + kSampleBlocks - 1) / kSampleBlocks) * sizeof(float);
     if (max_candidates > 0 && max_candidates <= kMaxSorted && slice_bytes <= 200 * 1024) {
         // Few rows leave multiprocessors idle, and a block has one to itself with all of its registers (8 rows of 128,256, 40 and 200
-        // candidates: 17.5 and 37.1 us; 18.2 and 38.2 with the registers of two); more share one (16 rows: 25.3 us, and 30.0 where the last
+        // candidates: 17.5 and 37.1 us; 18.2 and 38.2 with the registers of two; 16.4 since); more share one (16 rows: 25.3 us, and 30.0 where the last
         // cluster of eight waits for a second round).
         const bool alone = kSampleBlocks * rows <= kAloneBlocks;
         auto kernel = alone ? sample_rows_cluster_kernel<1> : sample_rows_cluster_kernel<2>;
