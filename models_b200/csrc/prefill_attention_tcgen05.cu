@@ -261,7 +261,7 @@ struct AttentionArgs {
 };
 
 // roles in the status record: 1 TMA (stage free), 2 MMA (queries), 3 MMA (keys), 4 MMA (probabilities),
-// 5 softmax (scores), 6 softmax (output of a page), 7 TMA (last scores, for the gates), 8 softmax (gates)
+// 5 softmax (scores), 6 softmax (output of a page), 7 TMA (last key tile free, for the gates), 8 softmax (gates)
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                  const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_q_turned,
@@ -372,8 +372,10 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 for (int b = 0; b < kValueBoxes; ++b)
                     tma_load_2d(v_smem + stage * kValueTileBytes + b * kKVBoxBytes, &map_v, column + b * 64, row, v_full + 8 * stage);
             }
-            // gates of elements take the queries' place as soon as the last scores are there
-            if (gated && ok && mbar_wait(s_full + 8 * ((pages - 1) & 1), ((pages - 1) >> 1) & 1, 7)) {
+            // Gates of elements take the queries' place as soon as the last scores have read them, which also frees the last key tile.  (This
+            // thread has followed the key ring's barriers use by use.  Those of the scores it has not: with three stages and three pages the
+            // one wait for the last page's parity passes before its buffer's first scores are there.)
+            if (gated && ok && mbar_wait(k_empty + 8 * ((pages - 1) % kStages), ((pages - 1) / kStages) & 1, 7)) {
                 mbar_expect_tx(gate_full, kGateBytes);
 #pragma unroll
                 for (int b = 0; b < kValueBoxes; ++b) tma_load_2d(q_smem + kGatesAt + b * kQBoxBytes, &map_gate, head * args.value_columns + b * 64, q_begin + t0, gate_full);

@@ -1682,6 +1682,44 @@ def test_latent_prompts_expand_the_rows_they_see(cuda_device, monkeypatch, query
     assert float((outs[0] - outs[1]).norm()) <= 4 * 2.0 ** -8 * float(outs[1].norm())
 
 
+@pytest.mark.parametrize("query_latent,window,value_dim", [(0, 0, 64), (128, 0, 64), (0, 64, 64), (0, 0, 40)])
+@pytest.mark.parametrize("q_lens", [[129, 160, 192], [160] * 40, [600]])
+def test_latent_prompts_without_a_position_gated_by_elements(cuda_device, monkeypatch, query_latent, window, value_dim, q_lens):
+    """Heads of 64 with no rotated part keep three tiles in flight: prompts whose last tiles see three pages, and all of a window's."""
+    from models_b200.cache import KvCache
+    from models_b200.config.specs import LatentAttentionSpec
+    from models_b200.engine.batch import build_step_batch
+    from models_b200.parts import RunContext, Runtime, build_part, latent_attention
+
+    monkeypatch.setattr(latent_attention, "EXPANDED_TOKENS", 0)
+    width, heads, dim, rank = 256, 4, 64, 128
+    roles = ["down_q", "down_q_norm", "up_q", "q", "down", "down_norm", "up_k", "up_v", "gate", "o"]
+    spec = LatentAttentionSpec(hidden_size=width, num_heads=heads, head_dim=dim, value_dim=value_dim, latent_dim=rank, scale=dim ** -0.5, eps=1e-6,
+                               gated=True, weights={r: r for r in roles}, query_latent=query_latent, position=None, window=window or None,
+                               gate_kind="element")
+    outs = []
+    for expanded in (True, False):
+        mixer = build_part("mixer", spec, Runtime(torch.device("cuda:0"), "bfloat16", max_positions=1024))
+        draw = torch.Generator().manual_seed(5)
+        mixer.load({p.name: (torch.randn(p.shape, generator=draw) * p.shape[-1] ** -0.5).bfloat16() if len(p.shape) > 1
+                    else 1 + 0.1 * torch.randn(p.shape, generator=draw) for p in mixer.parameters()})
+        assert mixer.expand is not None
+        if not expanded:
+            mixer.expand = None
+        cache = KvCache([mixer.kv_request()], [None], sum(q_lens) + 64 * 2 * len(q_lens), len(q_lens))
+        cache.allocate_storage(lambda shape: torch.full(shape, float("nan"), dtype=torch.bfloat16, device="cuda:0"))
+        run = RunContext(run=0)
+        run.group, run.k_pool, run.v_pool = cache.pools(0)
+        entries = [(cache.open_slot(), n) for n in q_lens]
+        cache.append(entries)
+        batch = build_step_batch(cache, [(s, [0] * n, []) for s, n in entries], torch.device("cuda:0"))
+        cache.commit(entries)
+        x = torch.randn(sum(q_lens), width, generator=torch.Generator().manual_seed(6)).bfloat16().cuda()
+        outs.append(mixer.forward(x, batch, run).float())
+    # keys, values and queries pass through bfloat16 at other places: four roundings' worth
+    assert float((outs[0] - outs[1]).norm()) <= 4 * 2.0 ** -8 * float(outs[1].norm())
+
+
 @pytest.mark.parametrize("window,past,q_lens", [(90, [300, 40], [150, 129]), (64, [127, 641], [33, 65]), (1, [200, 0], [70, 64])])
 def test_latent_prompts_expand_only_what_their_window_sees(cuda_device, monkeypatch, window, past, q_lens):
     """On top of a cache that gave pages back: the rows gathered begin at the window's first page, and what lies before it (not a number here)

@@ -402,6 +402,37 @@ def test_prompt_attention_with_gates_of_elements(cuda_device, heads, dim, rot, v
     assert bool((error <= 2.0 ** -6.99 * want[~nan].abs() + 1e-37).all())
 
 
+@pytest.mark.parametrize("heads,dim,rot,value_dim", [(2, 64, 0, 64), (2, 64, 64, 64), (2, 64, 0, 128), (1, 40, 24, 40)])
+@pytest.mark.parametrize("lengths,window", [([129, 160, 192], 0), ([193, 256, 257, 320], 0), ([64, 65, 128], 0), ([700], 1), ([700], 64), ([513, 129], 90),
+                                            ([700], 200), ([1500] * 40, 0), ([160] * 200, 0)])
+def test_gates_of_elements_come_after_the_last_scores(cuda_device, heads, dim, rot, value_dim, lengths, window):
+    """Tiles that see one to six pages and all of a window's, in rings of two and of three stages, many blocks at a time: the gates that are
+    brought into the queries' place do not meet their products.  Against the result without gates times the sigmoids (two roundings to
+    bfloat16), and every run gives the same bits."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator(device="cuda").manual_seed(dim + rot + value_dim)
+    whole = lambda n: -(-n // 64) * 64  # noqa: E731
+    T, KD, RD, VD = sum(lengths), whole(dim), whole(rot), whole(value_dim)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device=cuda_device).bfloat16()  # noqa: E731
+    q, q_tail, tail = normal(T, heads * KD), normal(T, heads * RD) if rot else None, normal(T, RD) if rot else None
+    kv, gate = normal(T, heads * (KD + VD)), normal(T, heads * value_dim) * 6
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda_device)  # noqa: E731
+    cu_q, lens = i32(np.concatenate([[0], np.cumsum(lengths)]).tolist()), i32(lengths)
+
+    def run(gates):
+        out = torch.zeros(T, heads * value_dim, dtype=torch.bfloat16, device=cuda_device)
+        ops.prompt_attention(q, q_tail, kv[:, :heads * KD], kv[:, heads * KD:], tail, out, cu_q, lens, max(lengths), heads, KD, value_dim,
+                             (dim + rot) ** -0.5, gates, window=window, gate_kind="element")
+        return out
+
+    want = run(None).double() * torch.sigmoid(gate.double())
+    first = run(gate)
+    assert bool(((first.double() - want).abs() <= 2.0 ** -6.99 * want.abs() + 1e-37).all())
+    for _ in range(10):
+        assert torch.equal(run(gate).view(torch.int16), first.view(torch.int16))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,kv_heads,dim,rot,interleaved", [(20, 4, 128, 64, False), (96, 16, 128, 128, False), (3, 1, 24, 8, True), (5, 5, 10, 6, False),
                                                                 (4, 2, 16, 16, True), (2, 1, 40, 0, False), (6, 3, 32, 8, False)])
