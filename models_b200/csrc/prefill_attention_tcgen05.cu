@@ -5,10 +5,12 @@
 //
 // -DMB_SHAPED=1 (paged, float weights): scores and results with the variations of gated_attention.cu -- a factor per head, a bound
 // cap * tanh(score / cap), one more term of score 0 in the denominator, a result whose pairs (2m, 2m + 1) are turned back by the
-// query's position.  Where a warp's scores of a page are small, tanh is a polynomial and the page needs no maximum (kTanhReach); elsewhere the
-// bound costs a thread two more special-function results per score (tanh(x) = 1 - 2 / (1 + e^(2x))).  2,048 tokens, 16 heads of 64 and 128:
-// 46 us (63 by the general form alone, with a result's tables read along its row), bound by the longest blocks' pages one after another
-// (about 2,100 cycles each, 1,500 of them a warp's own arithmetic).
+// query's position.  The bound costs a thread two more special-function results per score (tanh(x) = 1 - 2 / (1 + e^(2x))); where
+// the caller's word keeps a head's scores small (score_bound), tanh is a polynomial.  2,048 tokens, 16 heads of 64 and 128, between two events:
+// 51 us by the polynomial and 68 by the general form, bound by the longest blocks' pages one
+// after another; two prompts of 400 on top of 300 positions 27 and 33.  (Chosen page by page, from the scores of a warp's rows, a row's
+// bits followed from other rows and from what lay behind its end, and the general form took 69 and 37; from every score by itself, both forms
+// were worked out: 58 to 104 us.)
 //
 // MB_CONTIGUOUS: a prompt that starts its sequence brings every key it sees itself, so keys and values are read from the step's own
 // rows ([tokens][heads * size]) instead of the cache's pages.  Key and value heads may then be padded to these sizes with zero
@@ -220,11 +222,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-__device__ __forceinline__ float max3_magnitude(float a, float b, float c) { return max3(fabsf(a), fabsf(b), fabsf(c)); }
-
-// Of a bound cap * tanh(z / cap): up to which |z / cap| a polynomial stands for it, and up to which |score * log2 e| a page needs no maximum.
-// (Unit-normed queries and keys of 64 numbers have |score| <= 8 times the head's factor: within either at a bound of 50.)
-constexpr float kTanhReach = 0.5f, kFlatReach = 16.0f;
+// Of a bound cap * tanh(z), z = score / cap: up to which |z| a polynomial stands for it.
+constexpr float kTanhReach = 0.5f;
 
 // tcgen05.mma with the 128 x 16 A operand in tensor memory (lane = row, two bfloat16 per 32-bit column)
 __device__ __forceinline__ void umma_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t instruction, uint32_t accumulate) {
@@ -255,6 +254,7 @@ struct AttentionArgs {
     // kShaped
     const float* head_scale;  // [heads] factors on the scores, or null
     float softcap;            // 0: scores are not bounded
+    float score_bound;        // what |q . k| does not exceed where a row sees the key, or 0
     int sink;                 // != 0: one more term of score 0 in the denominator
     const float* turn_cos;    // [positions][VD / 2] with turn_sin, or null
     const float* turn_sin;
@@ -437,11 +437,18 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         const float cap = kShaped ? args.softcap : 0.0f, cap_exponent = cap > 0.0f ? shaped_scale * (2.0f * 1.4426950408889634f / cap) : 0.0f;
         const float scale_log2 = (kShaped ? 1.0f : args.scale) * 1.4426950408889634f;
         const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
-        // the polynomial for small scores (see kTanhReach)
-        const float per_cap = cap > 0.0f ? shaped_scale / cap : 0.0f, flat_reach = fminf(kTanhReach * cap, kFlatReach / 1.4426950408889634f) / fabsf(shaped_scale);
+        // Where the caller's word on |q . k| keeps a head's scores within kTanhReach, tanh is a polynomial, z (1 + u (c0 + u (c1 + ...))), u = z^2,
+        // of relative error 2.0e-8 (1.8e-7 with the roundings of its evaluation): nothing that a block reads has a say in it, so that a
+        // row's bits follow from what the row sees.
+        const bool small = cap > 0.0f && args.score_bound > 0.0f && args.score_bound * fabsf(shaped_scale) <= kTanhReach * cap;
+        const float per_cap = small ? shaped_scale / cap : 0.0f;
         auto both = [](float v) { return pack_f32x2(v, v); };
         const uint64_t per_cap2 = both(per_cap), cap_log2 = both(cap * 1.4426950408889634f), one = both(1.0f);
         const uint64_t tanh_c0 = both(-0.33333148f), tanh_c1 = both(0.13325987f), tanh_c2 = both(-0.053052945f), tanh_c3 = both(0.017256979f);
+        auto tanh_factors = [&](uint64_t z) {  // tanh(z) / z of two small z
+            const uint64_t u = mul_f32x2(z, z);
+            return fma_f32x2(u, fma_f32x2(u, fma_f32x2(u, fma_f32x2(u, tanh_c3, tanh_c2), tanh_c1), tanh_c0), one);
+        };
         // `base` is the score the exponents are taken against.  It follows the running maximum lazily:
         // it moves (and the output so far is rescaled) only when the maximum has grown by more than
         // kSlack in the exponent, so most pages cost no pass over the output.  Until then the
@@ -460,74 +467,55 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             for (int c = 0; c < kCols; c += 32) tmem_load_32_raw(my_scores + c, &s[c]);
             tmem_wait_loads();
             const int key_base = (t_begin + t) * kKeys;
-            auto hide = [&] {
-                if (key_base + kCols - 1 <= row_pos && key_base >= row_first) return;  // the whole page is visible to this row
+            if (kShaped && small) {
+#pragma unroll
+                for (int i = 0; i < kCols; i += 2) {  // z, of which a hidden key's -infinity stays one
+                    const uint64_t z = mul_f32x2(pack_f32x2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), per_cap2);
+                    s[i] = (uint32_t)z, s[i + 1] = (uint32_t)(z >> 32);
+                }
+            } else if (kShaped && cap > 0.0f) {
+#pragma unroll
+                for (int i = 0; i < kCols; ++i)  // cap * tanh(z)
+                    s[i] = __float_as_uint(cap - __fdividef(2.0f * cap, 1.0f + fast_exp2(__uint_as_float(s[i]) * cap_exponent)));
+            } else if (kShaped) {
+#pragma unroll
+                for (int i = 0; i < kCols; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) * shaped_scale);
+            }
+            if (!(key_base + kCols - 1 <= row_pos && key_base >= row_first)) {  // not the whole page is visible to this row
 #pragma unroll
                 for (int i = 0; i < kCols; ++i) {
                     const int key = key_base + i;
                     if (!(key <= row_pos && key >= row_first)) s[i] = __float_as_uint(-CUDART_INF_F);
                 }
-            };
-            float factor = 1.0f;
-            bool flat = false;
-            if (kShaped && cap > 0.0f) {
-                float most[4];  // magnitudes: four chains
-#pragma unroll
-                for (int i = 0; i < 4; ++i) most[i] = max3_magnitude(__uint_as_float(s[i]), __uint_as_float(s[4 + i]), __uint_as_float(s[8 + i]));
-#pragma unroll
-                for (int i = 12; i + 8 <= kCols; i += 8)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) most[j] = max3_magnitude(most[j], __uint_as_float(s[i + j]), __uint_as_float(s[i + 4 + j]));
-#pragma unroll
-                for (int i = kCols - 4; i < kCols; ++i) most[i & 3] = fmaxf(most[i & 3], fabsf(__uint_as_float(s[i])));
-                const bool mine = max3(fmaxf(most[0], most[1]), most[2], most[3]) <= flat_reach && (base == -CUDART_INF_F || fabsf(base) <= kFlatReach / 1.4426950408889634f);
-                flat = __all_sync(0xffffffffu, mine || row_pos < 0);
             }
-            if (flat) {
-                // z (1 + u (c0 + u (c1 + ...))), u = (z / cap)^2 (relative error 1.5e-8), log2 e and the base: eight instructions for two scores,
-                // where the general form waits for three special-function results each
-                if (base == -CUDART_INF_F && key_base <= row_pos && key_base + kCols > row_first) base = 0.0f;
-                const float offset = base == -CUDART_INF_F ? 0.0f : -base * scale_log2;
-                const uint64_t offset2 = pack_f32x2(offset, offset);
+            float part[8];  // eight chains, two more scores a step
 #pragma unroll
-                for (int i = 0; i < kCols; i += 2) {
-                    const uint64_t z = mul_f32x2(pack_f32x2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), per_cap2), u = mul_f32x2(z, z);
-                    const uint64_t p = fma_f32x2(u, fma_f32x2(u, fma_f32x2(u, fma_f32x2(u, tanh_c3, tanh_c2), tanh_c1), tanh_c0), one);
-                    const uint64_t x = fma_f32x2(mul_f32x2(z, cap_log2), p, offset2);
+            for (int i = 0; i < 8; ++i) part[i] = fmaxf(__uint_as_float(s[i]), __uint_as_float(s[8 + i]));
+#pragma unroll
+            for (int i = 16; i < kCols; i += 16)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) part[j] = max3(part[j], __uint_as_float(s[i + j]), __uint_as_float(s[i + 8 + j]));
+            float page_max = max3(max3(part[0], part[1], part[2]), max3(part[3], part[4], part[5]), fmaxf(part[6], part[7]));
+            if (kShaped && small) page_max = page_max * cap * __uint_as_float((uint32_t)tanh_factors(both(page_max)));
+            // scores stay raw; the scale (times log2 e) is folded into the exponent: 2^(s*c - base*c)
+            float factor = 1.0f;
+            if (base == -CUDART_INF_F) {
+                base = page_max;  // nothing accumulated so far (or still nothing visible)
+            } else if ((page_max - base) * scale_log2 > kSlack) {
+                factor = fast_exp2((base - page_max) * scale_log2);
+                base = page_max;
+            }
+            run_sum *= factor;
+            // a row that has seen nothing yet keeps -inf; subtract 0 then so that the exponent is -inf, not NaN
+            const float offset = base == -CUDART_INF_F ? 0.0f : fmaf(-base, scale_log2, kTruncationLift);
+            const uint64_t offset2 = pack_f32x2(offset, offset);
+            if (kShaped && small) {
+#pragma unroll
+                for (int i = 0; i < kCols; i += 2) {  // eight instructions for two scores in all, where the general form waits for four special-function results more
+                    const uint64_t z = pack_f32x2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), x = fma_f32x2(mul_f32x2(z, cap_log2), tanh_factors(z), offset2);
                     s[i] = (uint32_t)x, s[i + 1] = (uint32_t)(x >> 32);
                 }
-                hide();
             } else {
-                if (kShaped) {
-                    if (cap > 0.0f) {
-#pragma unroll
-                        for (int i = 0; i < kCols; ++i)  // cap * tanh(z / cap)
-                            s[i] = __float_as_uint(cap - __fdividef(2.0f * cap, 1.0f + fast_exp2(__uint_as_float(s[i]) * cap_exponent)));
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < kCols; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) * shaped_scale);
-                    }
-                }
-                hide();
-                float part[8];  // eight chains, two more scores a step
-#pragma unroll
-                for (int i = 0; i < 8; ++i) part[i] = fmaxf(__uint_as_float(s[i]), __uint_as_float(s[8 + i]));
-#pragma unroll
-                for (int i = 16; i < kCols; i += 16)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) part[j] = max3(part[j], __uint_as_float(s[i + j]), __uint_as_float(s[i + 8 + j]));
-                const float page_max = max3(max3(part[0], part[1], part[2]), max3(part[3], part[4], part[5]), fmaxf(part[6], part[7]));
-                // scores stay raw; the scale (times log2 e) is folded into the exponent: 2^(s*c - base*c)
-                if (base == -CUDART_INF_F) {
-                    base = page_max;  // nothing accumulated so far (or still nothing visible)
-                } else if ((page_max - base) * scale_log2 > kSlack) {
-                    factor = fast_exp2((base - page_max) * scale_log2);
-                    base = page_max;
-                }
-                run_sum *= factor;
-                // a row that has seen nothing yet keeps -inf; subtract 0 then so that the exponent is -inf, not NaN
-                const float offset = base == -CUDART_INF_F ? 0.0f : fmaf(-base, scale_log2, kTruncationLift);
-                const uint64_t offset2 = pack_f32x2(offset, offset);
 #pragma unroll
                 for (int i = 0; i < kCols; i += 2) {
                     const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), scale2, offset2);
@@ -741,18 +729,18 @@ static int check_prefill(const void* q, int q_row_stride, const void* out, int o
 // q: bfloat16 rows (row stride q_row_stride) of total_rows tokens, head h at columns [h * KD, +KD); out likewise with VD.
 // k_pool [pages][kv_heads][64][KD], v_pool [pages][kv_heads][64][VD]: bfloat16.  block_table: int32 [sequences][max_blocks];
 // cu_q: int32 [sequences + 1]; kv_lens: int32 [sequences] (the new tokens included).
-// MB_SHAPED: also head_scale (or null), softcap, sink and the tables that turn the result back (16-byte aligned, or null).
+// MB_SHAPED: also head_scale (or null), softcap, score_bound (what |q . k| does not exceed where a row sees the key; 0: not known), sink and the tables that turn the result back (16-byte aligned, or null).
 MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int total_rows, void* out, int out_row_stride,
                                            const void* k_pool, const void* v_pool, int pool_pages, const int* block_table,
                                            int max_blocks, const int* cu_q, const int* kv_lens, int sequences, int max_q_len,
                                            int heads, int kv_heads, int page_size, int window, float scale,
 #if MB_SHAPED
-                                           const float* head_scale, float softcap, int sink, const float* turn_cos, const float* turn_sin,
+                                           const float* head_scale, float softcap, float score_bound, int sink, const float* turn_cos, const float* turn_sin,
 #endif
                                            cudaStream_t stream) {
 #if !MB_SHAPED
     const float *head_scale = nullptr, *turn_cos = nullptr, *turn_sin = nullptr;
-    const float softcap = 0.0f;
+    const float softcap = 0.0f, score_bound = 0.0f;
     const int sink = 0;
 #endif
     if (((uintptr_t)turn_cos | (uintptr_t)turn_sin) & 15) return fail("prefill_attention_tcgen05: the tables that turn the result back must start on 16-byte boundaries");
@@ -768,7 +756,7 @@ MB_EXPORT int mb_prefill_attention_tcgen05(const void* q, int q_row_stride, int 
     if (int status = make_map(&map_k, k_pool, pool_pages * kv_heads * kKeys, KD, KD, kKeys)) return status;
     if (int status = make_map(&map_v, v_pool, pool_pages * kv_heads * kKeys, VD, VD, kKeys)) return status;
     const AttentionArgs args{(bf16*)out, out_row_stride, block_table, max_blocks, cu_q, kv_lens, heads, kv_heads, window, scale, KD, VD, nullptr, 0, 0, 0, 0,
-                             head_scale, softcap, sink, turn_cos, turn_sin};
+                             head_scale, softcap, score_bound, sink, turn_cos, turn_sin};
     return launch_prefill(map_q, map_k, map_v, map_q, map_k, map_q, args, sequences, max_q_len, stream);
 }
 #else
@@ -807,7 +795,7 @@ MB_EXPORT int mb_prompt_attention_tcgen05(const void* q, int q_row_stride, int q
         if (int status = make_map(&map_k_turned, k_turned, key_total, RD, RD, kKeys)) return status;
     }
     const AttentionArgs args{(bf16*)out, out_row_stride, nullptr, 0, cu_q, kv_lens, heads, kv_heads, window, scale, q_head_columns, value_columns,
-                             (const bf16*)gate, gate_stride, gate_element, key_rows, key_window, nullptr, 0.0f, 0, nullptr, nullptr};
+                             (const bf16*)gate, gate_stride, gate_element, key_rows, key_window, nullptr, 0.0f, 0.0f, 0, nullptr, nullptr};
     CUtensorMap map_gate = map_q;
     if (gate_element)
         if (int status = make_map(&map_gate, gate, total_rows, heads * value_columns, gate_stride, kQRows)) return status;

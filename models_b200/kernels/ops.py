@@ -910,7 +910,7 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
                     head_bias: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
                     gate_kind: Optional[str] = None, kernel: Optional[str] = None, head_scale: Optional[torch.Tensor] = None,
                     softcap: float = 0.0, sink: bool = False, turn_cos: Optional[torch.Tensor] = None,
-                    turn_sin: Optional[torch.Tensor] = None, block: int = 0, window: int = 0) -> None:
+                    turn_sin: Optional[torch.Tensor] = None, block: int = 0, window: int = 0, score_bound: float = 0.0) -> None:
     """Causal attention over the paged cache with `weights` "softmax" or "sigmoid" (independent sigmoids of the scores,
     not normalised over keys); score = scale * q.k - 2^(-slope_exponent (h + 1) / heads) * (i - j) + head_bias[h]
     (slope_exponent 0: no distance term; head_bias None: 0).  `v_pool` None: the values are the first `value_dim`
@@ -921,7 +921,9 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
     `turn_cos`, `turn_sin` (float32 [positions, value_dim / 2]): the values were stored rotated by their own positions
     (pairs 2m, 2m + 1), and every head's sum is turned back by the query's position before any gate.
     `block` n > 0: query i sees key j <= i only if floor(i / n) = floor(j / n), blocks of n positions counted from the
-    sequence's position 0; `window` n > 0: only if i - j < n.
+    sequence's position 0; `window` n > 0: only if i - j < n.  `score_bound` b > 0: the caller's word that |q.k| is at most b for every
+    key that a row sees (heads divided by their root mean square: `head_dim` and a little for the rounding of either side); it lets the
+    tcgen05 form take small bounded scores by a polynomial, to the same precision.
     `kernel`: None picks the decode form for steps of one token per sequence (the keys cut into runs with a block each;
     the grid follows the page table's width, not the lengths, so that a captured step stays valid), the tensor-core form
     where it applies (bfloat16 steps of many tokens; softmax attention of suitable sizes without distance, bias or gate on the tcgen05 ones; plain scores: "tcgen05"), else the form with a warp per (token, head); decode steps of 8 heads and
@@ -971,6 +973,8 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
         raise KernelError("gated_attention: a sink belongs to softmax weights")
     if block < 0 or window < 0:
         raise KernelError(f"gated_attention: a block of {block} positions, a window of {window}")
+    if not 0.0 <= score_bound < float("inf"):
+        raise KernelError(f"gated_attention: scores bounded by {score_bound}")
     extras = (_p(head_scale), ctypes.c_float(softcap), 1 if sink else 0, _p(turn_cos), _p(turn_sin), int(block), int(window))
     softmax = 1 if weights == "softmax" else 0
     sequences = kv_lens.numel()
@@ -1039,7 +1043,7 @@ def gated_attention(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_
         _run(lib, lib.mb_prefill_attention_tcgen05(
             _p(q), q.stride()[0], q.shape[0], _p(out), out.stride()[0], _p(k_pool), _p(v_pool), k_pool.shape[0], _p(block_table),
             block_table.shape[1], _p(cu_q), _p(kv_lens), sequences, max_q_len, heads, kv_heads, page_size, int(window), ctypes.c_float(scale),
-            _p(head_scale), ctypes.c_float(softcap), 1 if sink else 0, _p(turn_cos), _p(turn_sin), _stream()))
+            _p(head_scale), ctypes.c_float(softcap), ctypes.c_float(score_bound), 1 if sink else 0, _p(turn_cos), _p(turn_sin), _stream()))
         return
     if kernel == "tc" or (kernel is None and gated_attention_tc_takes(q, out, k_pool, head_dim, value_dim, max_q_len, gate, gate_kind, v_pool)):
         if not gated_attention_tc_takes(q, out, k_pool, head_dim, value_dim, max(max_q_len, GATED_TC_MIN_ROWS), gate, gate_kind, v_pool):

@@ -22,6 +22,8 @@ from .linear import stack_rows
 from .registry import build_part, register_part
 from .split import SplitPart
 
+NORMED = 1.01  # q.k of heads divided by their root mean square is at most head_dim times this: either side is rounded to eight bits
+
 
 class CappedAttentionMixer(SplitPart, Mixer):
     def __init__(self, spec, runtime):
@@ -99,7 +101,8 @@ class CappedAttentionMixer(SplitPart, Mixer):
         ops.gated_attention(q, mid, run.k_pool, run.v_pool, group.block_table, batch.cu_q, batch.kv_lens, batch.max_q_len,
                             s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, "softmax", s.scale,
                             head_scale=self.temperature, softcap=s.softcap, sink=s.sink,
-                            turn_cos=vpos.cos if vpos else None, turn_sin=vpos.sin if vpos else None)
+                            turn_cos=vpos.cos if vpos else None, turn_sin=vpos.sin if vpos else None,
+                            score_bound=NORMED * s.head_dim if s.unit_norm else 0.0)
 
 
 register_part("mixer", "capped_attention", CappedAttentionMixer)

@@ -1622,6 +1622,107 @@ def test_shaped_scores_of_mostly_empty_tiles(cuda_device, sequences, tokens, mos
     assert torch.allclose(outs[0].float(), outs[1].float(), rtol=2.0 ** -7, atol=2.0 ** -9)
 
 
+@pytest.mark.parametrize("cap", [50.0, 8.0])
+@pytest.mark.parametrize("size,word", [(0.05, True), (0.2, True), (0.3, False), (2.2, False), (6.0, False)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_bounded_scores_of_what_a_row_does_not_see(cuda_device, cap, size, word, window):
+    """A row's bits follow from what it sees: not from what an earlier sequence left in the last page, not from keys and queries of later
+    tokens, of other rows of its warp or before its window, with and without a word on the scores."""
+    from models_b200.kernels import ops
+
+    heads, dim, vdim, past, lens = 2, 64, 128, [70, 0, 10], [200, 65, 128]
+    g = torch.Generator().manual_seed(int(cap))
+    ends = [a + b for a, b in zip(past, lens)]
+    pages = [-(-n // 64) for n in ends]
+    table, at = torch.zeros(3, max(pages), dtype=torch.int32), 1
+    for i, n in enumerate(pages):
+        table[i, :n], at = torch.arange(at, at + n), at + n
+    k, v = ([torch.randn(n * 64, d, generator=g).bfloat16() for n in pages] for d in (dim, vdim))
+    q = [(torch.randn(n, heads * dim, generator=g) * size).bfloat16() for n in lens]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()  # noqa: E731
+    bound = max(float((a.float().view(-1, heads, dim) @ b.float().t()).abs().max()) for a, b in zip(q, k)) if word else 0.0
+    assert not word or bound * 0.125 <= 0.5 * cap  # (the polynomial's reach)
+
+    def run(k, v, q):
+        pools = [torch.cat([torch.zeros(64, x[0].shape[1]).bfloat16(), *x]).view(-1, 1, 64, x[0].shape[1]).cuda() for x in (k, v)]
+        out = torch.zeros(sum(lens), heads * vdim, dtype=torch.bfloat16, device=cuda_device)
+        ops.gated_attention(torch.cat(q).cuda(), out, *pools, table.cuda(), i32(np.concatenate([[0], np.cumsum(lens)]).tolist()), i32(ends), max(lens), heads, 1,
+                            dim, vdim, "softmax", 0.125, softcap=cap, sink=True, window=window, score_bound=bound)
+        return list(out.view(torch.int16).split(lens))
+
+    want = run(k, v, q)
+    for left in (0.0, 3.0, 3e4, -3e38, float("nan")):  # behind the sequences' ends
+        stale = [[torch.cat([x[:n], torch.full_like(x[n:], left)]) for x, n in zip(xs, ends)] for xs in (k, v)]
+        assert all(torch.equal(a, b) for a, b in zip(run(*stale, q), want))
+    for keep in (40, 64, 100):  # rows from there on, queries and keys, become loud or still
+        for factor in (0.0, 30.0):
+            changed = [[torch.cat([x[:b + min(keep, n)], x[b + min(keep, n):] * factor]) for x, b, n in zip(k, past, lens)],
+                       [torch.cat([x[:keep], x[keep:] * factor]) for x in q]]
+            assert all(torch.equal(a[:keep], b[:keep]) for a, b in zip(run(changed[0], v, changed[1]), want))
+    if window:  # positions that the rows from 100 on do not see any more
+        changed = [torch.cat([x[:b + 100 - window] * 30.0, x[b + 100 - window:]]) if n > 100 else x for x, b, n in zip(k, past, lens)]
+        assert all(torch.equal(a[100:], b[100:]) for a, b in zip(run(changed, v, q), want))
+
+
+@pytest.mark.parametrize("cap", [50.0, 8.0])
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 64)])
+@pytest.mark.parametrize("lens,past,window", [([200, 65], [0, 100], 0), ([128, 33], [64, 0], 0), ([300], [10], 70), ([129], [0], 1)])
+def test_small_bounded_scores_by_the_callers_word(cuda_device, cap, dim, vdim, lens, past, window):
+    """Scores that fill the polynomial's reach, heads of either sign, one whose scores the word does not keep small and one of factor 0, against
+    64 bits: the score's float arithmetic (2^-22 of at most cap / 2), the weights' two bfloat16 parts (2^-16) and the result's rounding
+    (2^-8).  The general form stays within the same, and what is not covered by the word gives its bits."""
+    from models_b200.kernels import ops
+
+    heads, ends = 4, [a + b for a, b in zip(past, lens)]
+    g = torch.Generator().manual_seed(int(cap) + dim)
+    pages = [-(-n // 64) for n in ends]
+    table, at = torch.zeros(len(lens), max(pages), dtype=torch.int32), 0
+    for i, n in enumerate(pages):
+        table[i, :n], at = torch.arange(at, at + n), at + n
+    unit = lambda x: (x / x.square().mean(-1, keepdim=True).sqrt()).bfloat16()  # noqa: E731
+    k_pool, v_pool = unit(torch.randn(at, 1, 64, dim, generator=g)), torch.randn(at, 1, 64, vdim, generator=g).bfloat16()
+    q = unit(torch.randn(sum(lens), heads, dim, generator=g))
+    q[::7] = k_pool[table[0, 0], 0, 3]  # (the largest score there is)
+    scale = dim ** -0.5
+    whole = 0.5 * cap / (1.01 * dim * scale)  # the factor that fills the reach
+    factors = torch.tensor([whole, -whole, 3.0 * whole, 0.0]).float()
+    factors[0] = factors[0] * (1 - 2.0 ** -20)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()  # noqa: E731
+    outs = []
+    for bound in (1.01 * dim * (1 - 2.0 ** -20), 0.0):
+        out = torch.zeros(sum(lens), heads * vdim, dtype=torch.bfloat16, device=cuda_device)
+        ops.gated_attention(q.view(sum(lens), -1).cuda(), out, k_pool.cuda(), v_pool.cuda(), table.cuda(), i32(np.concatenate([[0], np.cumsum(lens)]).tolist()),
+                            i32(ends), max(lens), heads, 1, dim, vdim, "softmax", scale, head_scale=factors.cuda(), softcap=cap, sink=True, window=window,
+                            score_bound=bound)
+        outs.append(out.view(-1, heads, vdim))
+    assert torch.equal(outs[0][:, 2].view(torch.int16), outs[1][:, 2].view(torch.int16))
+    at = 0
+    for i, (n, before) in enumerate(zip(lens, past)):
+        k, v = (torch.cat([p[t, 0] for t in table[i]])[:before + n].double() for p in (k_pool, v_pool))
+        i_at, j_at = torch.arange(before, before + n)[:, None], torch.arange(before + n)[None]
+        unseen = (j_at > i_at) | ((i_at - j_at >= window) if window else False)
+        for h in range(heads):
+            s = (cap * torch.tanh(q[at:at + n, h].double() @ k.t() * scale * float(factors[h]) / cap)).masked_fill(unseen, -math.inf)
+            top = s.amax(1, keepdim=True).clamp(min=0)
+            w = torch.exp(s - top)
+            w = w / (w.sum(1, keepdim=True) + torch.exp(-top))
+            for out in outs:
+                error = (out[at:at + n, h].double().cpu() - w @ v).abs()
+                assert bool((error <= 2.0 ** -8 * (w @ v).abs() + (cap * 2.0 ** -21 + 2.0 ** -15) * (w @ v.abs()) + 1e-30).all())
+        at += n
+
+
+@pytest.mark.parametrize("bound", [-1.0, math.inf, math.nan])
+def test_a_word_that_is_no_bound_is_refused(cuda_device, bound):
+    from models_b200.kernels import ops
+
+    q, out = (torch.zeros(64, 2 * 64, dtype=torch.bfloat16, device=cuda_device) for _ in range(2))
+    pools = [torch.zeros(2, 1, 64, 64, dtype=torch.bfloat16, device=cuda_device) for _ in range(2)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda_device)  # noqa: E731
+    with pytest.raises(ops.KernelError, match="scores bounded by"):
+        ops.gated_attention(q, out, *pools, i32([[1]]), i32([0, 64]), i32([64]), 64, 2, 1, 64, 64, "softmax", 0.125, softcap=5.0, score_bound=bound)
+
+
 @pytest.mark.parametrize("max_q_len,kernel", [(1, None), (64, None), (64, "tc"), (64, "rows")])
 def test_a_negative_bound_on_scores_is_refused(cuda_device, max_q_len, kernel):
     """Whichever kernel a call meets."""
