@@ -497,7 +497,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     __shared__ int histogram_all[256];  // of the whole row
     __shared__ __align__(16) float sorted_p[kMaxSorted];  // the candidates: filled and used in the cluster's first block only
     __shared__ int sorted_id[kMaxSorted];
-    __shared__ float slot_sum;
+    __shared__ float slot_sum, slot_mass;  // this block's, for the others: one place each, as some may still read the first when the second is there
     __shared__ int slot_ties;
     __shared__ int gathered;            // first block: candidates gathered so far
     __shared__ int shared_int[4];
@@ -718,13 +718,12 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         for (int i = begin + tid; i < end; i += kThreads) mass += w[i];
         {
             const float block = block_sum(mass, float_scratch);
-            __syncthreads();
-            if (tid == 0) slot_sum = block;
+            if (tid == 0) slot_mass = block;
         }
         cluster.sync();
         float prefix[kSampleBlocks + 1];
         prefix[0] = 0.0f;
-        for (int b = 0; b < kSampleBlocks; ++b) prefix[b + 1] = prefix[b] + *cluster.map_shared_rank(&slot_sum, b);
+        for (int b = 0; b < kSampleBlocks; ++b) prefix[b + 1] = prefix[b] + *cluster.map_shared_rank(&slot_mass, b);
         const float target = u * prefix[kSampleBlocks];
         int owner = 0;  // the first block whose range reaches the target; else the last block that has ids
         for (int b = 0; b < kSampleBlocks; ++b) {

@@ -385,6 +385,27 @@ def test_sampling_over_a_cluster_follows_the_reference_pipeline(cuda_device, voc
     assert float(seen.sum()) == 1.0 and float((seen - expected).abs().max()) < 0.07, seen
 
 
+@pytest.mark.parametrize("rows", [1, 8, 64, 300])
+@pytest.mark.parametrize("vocab", [1025, 5003])
+def test_rows_that_cut_nothing_draw_the_same_every_time(cuda_device, vocab, rows):
+    """Between the blocks' sums of exponentials and their masses lies little work here: each is read whole, whatever the blocks' pace."""
+    from models_b200.sampling import BatchSampler, RequestSampling, SamplingOptions, philox_uniform
+
+    g = torch.Generator().manual_seed(vocab + rows)
+    logits = torch.randn(rows, vocab, generator=g) * 3
+    sampler, on_device = BatchSampler(vocab, "cuda:0"), logits.cuda()
+
+    def draw():
+        return sampler.sample(on_device, [RequestSampling(SamplingOptions(temperature=0.9, top_k=vocab, top_p=1.0, seed=i), [0]) for i in range(rows)])
+
+    first = draw()
+    assert all(torch.equal(draw(), first) for _ in range(50))
+    running = torch.cumsum(torch.softmax(logits.double() / 0.9, 1), 1)
+    for i, token in enumerate(first.tolist()):  # (float masses against 64 bits: a neighbour where the target falls between two)
+        u = float(philox_uniform(i, 0))
+        assert (running[i, token - 1] if token else 0.0) - 1e-5 <= u <= running[i, token] + 1e-5
+
+
 @pytest.mark.parametrize("vocab", [1031, 5003])
 def test_sampling_with_few_candidates_at_the_edges_of_its_rule(cuda_device, vocab):
     """k at both sides of the rule's line, more values at the threshold than can be sorted, values that are almost equal, and -inf."""
