@@ -1659,12 +1659,8 @@ MB_EXPORT int mb_head_linear(const void* in, int in_stride, const void* w, void*
     if (tensor_cores && dtype == MB_BF16 && tokens >= 16 && n_in % 16 == 0 && n_out % 16 == 0 && n_in <= 512 && in_stride % 8 == 0 &&
         in_head % 8 == 0 && out_stride % 2 == 0 && out_head % 2 == 0 && !((uintptr_t)in & 15) && !((uintptr_t)w & 15) && !((uintptr_t)out & 3)) {
         const size_t smem = 3 * (size_t)tc::kTile * (n_in * 2 + 16);
-        static int reserved = 0;
-        if ((int)smem > reserved) {
-            cudaError_t status = cudaFuncSetAttribute(tc::head_linear_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (status != cudaSuccess) return fail("head_linear: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(status));
-            reserved = (int)smem;
-        }
+        static DeviceSet devices{0};
+        if (int status = reserve_shared("head_linear", tc::head_linear_tc_kernel, 3 * tc::kTile * (512 * 2 + 16), devices)) return status;
         MB_LAUNCH("head_linear_tc", tc::head_linear_tc_kernel, dim3((tokens + tc::kTile - 1) / tc::kTile, heads), dim3(128), smem, stream, true,
                   (const __nv_bfloat16*)in, in_stride, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, out_stride, (const __nv_bfloat16*)gate,
                   gate_stride, tokens, n_in, n_out, layout);

@@ -554,12 +554,8 @@ MB_EXPORT int mb_gated_attention_tc_decode(const void* q, int q_stride, const vo
     if (sequences > 65535 || heads > 65535 * 16) return fail("gated_attention_tc_decode: %d sequences or %d heads exceed the grid limit", sequences, heads);
     if (q_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)k_pool & 15) || ((uintptr_t)partial & 7)) return fail("gated_attention_tc_decode: rows must start on 16 bytes");
     const ScoreExtras extras{nullptr, 0.0f, 0, nullptr, nullptr, block, window};
-    static bool reserved = false;
-    if (!reserved) {
-        if (cudaFuncSetAttribute(gated_attention_tc_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecodeBytes) != cudaSuccess)
-            return fail("gated_attention_tc_decode: cannot reserve %zu bytes of shared memory", kDecodeBytes);
-        reserved = true;
-    }
+    static DeviceSet devices{0};
+    if (int status = reserve_shared("gated_attention_tc_decode", gated_attention_tc_decode_kernel, (int)kDecodeBytes, devices)) return status;
     MB_LAUNCH("gated_attention_tc_decode", gated_attention_tc_decode_kernel, dim3(runs, (heads + 15) / 16, sequences), dim3(kThreads), kDecodeBytes,
               stream, true, (const bf16*)q, q_stride, (const bf16*)k_pool, block_table, max_blocks, cu_q, kv_lens, partial, span, heads, scale, extras);
     return check_launch("gated_attention_tc_decode");
@@ -588,13 +584,9 @@ MB_EXPORT int mb_gated_attention_tc(const void* q, int q_stride, void* out, int 
         return fail("gated_attention_tc: query rows must start on 16 bytes and result rows on 4");
     if (gate_kind < 0 || gate_kind > 2 || (gate_kind != 0 && gate == nullptr)) return fail("gated_attention_tc: gate kind %d", gate_kind);
     if (gate_kind == kGateElement && (gate_stride % 2 || ((uintptr_t)gate & 3))) return fail("gated_attention_tc: gate rows must start on 4 bytes");
-    static bool configured[2] = {false, false};
-    if (!configured[softmax ? 1 : 0]) {
-        cudaError_t status = softmax ? cudaFuncSetAttribute(gated_attention_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes)
-                                     : cudaFuncSetAttribute(gated_attention_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (status != cudaSuccess) return fail("gated_attention_tc: cannot reserve %zu bytes of shared memory: %s", kSmemBytes, cudaGetErrorString(status));
-        configured[softmax ? 1 : 0] = true;
-    }
+    static DeviceSet devices[2] = {{0}, {0}};
+    if (int status = reserve_shared("gated_attention_tc", softmax ? gated_attention_tc_kernel<true> : gated_attention_tc_kernel<false>, (int)kSmemBytes, devices[softmax ? 1 : 0]))
+        return status;
     const dim3 grid((max_q_len + kQRows - 1) / kQRows, heads, sequences);
     if (softmax)
         MB_LAUNCH("gated_attention_tc", gated_attention_tc_kernel<true>, dim3(grid), dim3(kThreads), kSmemBytes, stream, true, (const bf16*)q,

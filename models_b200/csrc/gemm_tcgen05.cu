@@ -675,12 +675,8 @@ static int launch_tile(const CUtensorMap& map_a, const CUtensorMap& map_w, const
     constexpr int kOutCols = EPI == EPI_SWIGLU ? 128 : BN;
     const size_t smem = (size_t)kRingBytes + kEpilogueWarps * kStagingBytes + 1024;
     auto kernel = gemm_tcgen05_kernel<EPI, BN, kPair>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (status != cudaSuccess) return fail("gemm_tcgen05: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(status));
-        configured = true;
-    }
+    static DeviceSet devices{0};
+    if (int status = reserve_shared("gemm_tcgen05", kernel, (int)smem, devices)) return status;
     GemmArgs args = given;
     int tiles = ((args.m + kBlockM * kPair - 1) / (kBlockM * kPair)) * ((args.n + kOutCols - 1) / kOutCols);
     if (EPI == EPI_RESIDUAL) {

@@ -705,13 +705,8 @@ using namespace mb;
 
 static int launch_prefill(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_q_turned,
                           const CUtensorMap& map_k_turned, const CUtensorMap& map_gate, const AttentionArgs& args, int sequences, int max_q_len, cudaStream_t stream) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t status = cudaFuncSetAttribute(prefill_attention_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (status != cudaSuccess)
-            return fail("prefill_attention_tcgen05: cannot reserve %zu bytes of shared memory: %s", kSmemBytes, cudaGetErrorString(status));
-        configured = true;
-    }
+    static DeviceSet devices{0};
+    if (int status = reserve_shared("prefill_attention_tcgen05", prefill_attention_tcgen05_kernel, (int)kSmemBytes, devices)) return status;
     const dim3 grid(args.heads, (max_q_len + kQRows - 1) / kQRows, sequences);
     return launch_dependent("prefill_attention_tcgen05", prefill_attention_tcgen05_kernel, grid, dim3(kThreads), kSmemBytes, stream,
                             true, map_q, map_k, map_v, map_q_turned, map_k_turned, map_gate, args);

@@ -887,12 +887,8 @@ MB_EXPORT int mb_route_pad(const int* chosen, int entries, int experts, int* sor
     const int staged = smem + (size_t)entries * sizeof(int) <= 160 * 1024 ? 1 : 0;  // the entries' experts in shared memory, if they fit
     if (staged) smem += (size_t)entries * sizeof(int);
     if (smem > 48 * 1024) {
-        static size_t allowed = 0;  // (raised as needed; the attribute is per device context and function)
-        if (smem > allowed) {
-            if (cudaFuncSetAttribute(route_pad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024 + 48 * 1024) != cudaSuccess)
-                return fail("route_pad: cannot have %zu bytes of shared memory", smem);
-            allowed = 208 * 1024;
-        }
+        static DeviceSet devices{0};
+        if (int status = reserve_shared("route_pad", route_pad_kernel, 160 * 1024 + 48 * 1024, devices)) return status;
     }
     MB_LAUNCH("route_pad", route_pad_kernel, dim3(1), dim3(1024), smem, stream, true, chosen, entries, experts, sorted, position,
               tile_group, max_tiles, staged);
@@ -923,22 +919,14 @@ MB_EXPORT int mb_expert_product(const void* a, int a_stride, const void* w0, con
         using namespace tc;
         if (first) {
             const size_t smem = 2 * 3 * (size_t)kTileRows * kRowBytes;
-            static bool configured = false;
-            if (!configured) {
-                cudaError_t status = cudaFuncSetAttribute(expert_product_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (status != cudaSuccess) return fail("expert_product: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(status));
-                configured = true;
-            }
+            static DeviceSet devices{0};
+            if (int status = reserve_shared("expert_product", expert_product_tc_kernel<true>, (int)smem, devices)) return status;
             MB_LAUNCH("expert_product_tc", expert_product_tc_kernel<true>, grid, dim3(128), smem, stream, true, (const bf16*)a, a_stride,
                       (const bf16*)w0, (const bf16*)w1, (bf16*)mid, slot_out, out_stride, sorted, offsets, tile_expert, tile_row, top, N, K, limit, slope, up_offset);
         } else {
             const size_t smem = 2 * 2 * (size_t)kTileRows * kRowBytes;
-            static bool configured = false;
-            if (!configured) {
-                cudaError_t status = cudaFuncSetAttribute(expert_product_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (status != cudaSuccess) return fail("expert_product: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(status));
-                configured = true;
-            }
+            static DeviceSet devices{0};
+            if (int status = reserve_shared("expert_product", expert_product_tc_kernel<false>, (int)smem, devices)) return status;
             MB_LAUNCH("expert_product_tc", expert_product_tc_kernel<false>, grid, dim3(128), smem, stream, true, (const bf16*)a, a_stride,
                       (const bf16*)w0, (const bf16*)w1, (bf16*)mid, slot_out, out_stride, sorted, offsets, tile_expert, tile_row, top, N, K, limit, slope, up_offset);
         }

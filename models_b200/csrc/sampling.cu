@@ -449,6 +449,7 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
 // index, quotients are corrected reciprocals and a sum's exponentials are not stored: 110 instructions a logit had been its bound.  What
 // bounds it now is a chain of passes, cluster barriers and the first block's draw, in two rounds of clusters; one row takes 13.4 us.)
 constexpr int kSampleBlocks = 8;
+constexpr int kSliceBytes = 200 * 1024;  // most of a row that a block holds
 constexpr int kFewCandidates = 128;
 constexpr int kAloneBlocks = 64;  // so many blocks, clusters of eight, find a multiprocessor each with certainty
 constexpr float kThresholdSlack = 1e-5f;  // of a scaled logit: more than the exponential's rounding can turn around
@@ -936,18 +937,14 @@ MB_EXPORT int mb_sample_rows(const float* logits, int row_stride, int rows, int 
     // a block of the cluster kernel keeps its eighth of a row in shared memory; a vocabulary too large for that (more
     // than 400,000 ids) takes the kernel that works in the scratch array
     const size_t slice_bytes = (size_t)((vocab + kSampleBlocks - 1) / kSampleBlocks) * sizeof(float);
-    if (max_candidates > 0 && max_candidates <= kMaxSorted && slice_bytes <= 200 * 1024) {
+    if (max_candidates > 0 && max_candidates <= kMaxSorted && slice_bytes <= kSliceBytes) {
         // Few rows leave multiprocessors idle, and a block has one to itself with all of its registers (8 rows of 128,256, 40 and 200
         // candidates: 17.5 and 37.1 us; 18.2 and 38.2 with the registers of two; 16.4 since); more share one (16 rows: 25.3 us, and 30.0 where the last
         // cluster of eight waits for a second round).
         const bool alone = kSampleBlocks * rows <= kAloneBlocks;
         auto kernel = alone ? sample_rows_cluster_kernel<1> : sample_rows_cluster_kernel<2>;
-        static size_t reserved[2] = {0, 0};
-        if (slice_bytes > reserved[alone]) {
-            cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slice_bytes);
-            if (status != cudaSuccess) return fail("sample_rows: cannot reserve %zu bytes of shared memory: %s", slice_bytes, cudaGetErrorString(status));
-            reserved[alone] = slice_bytes;
-        }
+        static DeviceSet devices[2] = {{0}, {0}};
+        if (int status = reserve_shared("sample_rows", kernel, kSliceBytes, devices[alone])) return status;
         if (rows > 65535) return fail("sample_rows: %d rows exceed the grid limit 65535", rows);
         cudaLaunchConfig_t config = {};
         config.gridDim = dim3(kSampleBlocks, rows);

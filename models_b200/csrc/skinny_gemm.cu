@@ -176,6 +176,8 @@ struct SmemPlan {
     }
 };
 
+constexpr int kMostShared = 227 * 1024;  // that a block can have
+
 template <int NT, int PRO, int EPI, int kForm>
 __global__ void __launch_bounds__(warps_of(kForm) * 32)
 skinny_gemm_kernel(const SkinnyArgs args) {
@@ -587,12 +589,9 @@ static int launch(const SkinnyArgs& args, cudaStream_t stream) {
     using Plan = SmemPlan<NT, EPI, kForm>;
     const int smem = Plan::total(args.k_unit);
     auto kernel = skinny_gemm_kernel<NT, PRO, EPI, kForm>;
-    static int reserved = 0;
-    if (smem > reserved) {
-        cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (status != cudaSuccess) return fail("skinny_gemm: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(status));
-        reserved = smem;
-    }
+    if (smem > kMostShared) return fail("skinny_gemm: cannot reserve %d bytes of shared memory", smem);
+    static DeviceSet devices{0};
+    if (int status = reserve_shared("skinny_gemm", kernel, kMostShared, devices)) return status;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(args.clusters * args.k_split);
     config.blockDim = dim3(warps_of(kForm) * 32);

@@ -378,13 +378,9 @@ MB_EXPORT int mb_state_space_chunks(const void* rows, int row_stride, const void
     if (heads <= 0 || groups <= 0 || heads % groups) return fail("state_space_chunks: %d heads in %d groups", heads, groups);
     if (sequences > 65535 || heads > 65535) return fail("state_space_chunks: %d sequences or %d heads exceed the grid limit 65535", sequences, heads);
     if (row_stride % 8 || x_at % 8 || b_at % 8 || c_at % 8 || ((uintptr_t)rows & 15)) return fail("state_space_chunks: rows must start on 16 bytes");
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(chunk_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStatesBytes) != cudaSuccess ||
-            cudaFuncSetAttribute(chunk_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOutputBytes) != cudaSuccess)
-            return fail("state_space_chunks: cannot reserve %zu bytes of shared memory", kOutputBytes);
-        configured = true;
-    }
+    static DeviceSet states_devices{0}, output_devices{0};
+    if (int status = reserve_shared("state_space_chunks", chunk_states_kernel, (int)kStatesBytes, states_devices)) return status;
+    if (int status = reserve_shared("state_space_chunks", chunk_outputs_kernel, (int)kOutputBytes, output_devices)) return status;
     const ChunkShape shape{heads, groups, x_at, b_at, c_at};
     const dim3 grid((max_q_len + L - 1) / L, heads, sequences);
     const int aligned = state_stride % 4 == 0 && !((uintptr_t)state & 15) ? 1 : 0;

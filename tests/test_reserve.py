@@ -47,3 +47,10 @@ def test_no_launcher_keeps_the_first_answer_for_every_device():
     for path in sorted(build.CSRC.glob("*.cu")):
         text = path.read_text()
         assert not re.search(r"static\s+const\s+cudaError_t", text), f"{path.name}: an attribute of one device is kept for all"
+
+
+def test_no_launcher_remembers_a_reservation_for_every_device():
+    """What a launcher keeps about attributes it keeps for each device: in a DeviceSet, or in an array that the device's number indexes."""
+    for path in sorted(build.CSRC.glob("*.cu")):
+        for kept, count in re.findall(r"static\s+(?:bool|int|size_t)\s+(\w+)(?:\[(\w+)\])?\s*=", path.read_text()):
+            assert count in ("64", "kMaxDevices"), f"{path.name}: {kept} is kept for all devices"
