@@ -219,10 +219,8 @@ __global__ void __launch_bounds__(kThreads)
 sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, float* __restrict__ work,
                    int* __restrict__ counts, const float* __restrict__ temperature, const int* __restrict__ top_k,
                    const float* __restrict__ top_p, const float* __restrict__ penalty,
-                   const int* __restrict__ history, int history_stride, const long long* __restrict__ history_rows, int append,
-                   const int* __restrict__ history_len,
-                   const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters,
-                   const float* __restrict__ uniforms, int* __restrict__ out) {
+                   const long long* __restrict__ history_rows, int append, const int* __restrict__ history_len,
+                   const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters, int* __restrict__ out) {
     __shared__ Best best_scratch[32];
     __shared__ float float_scratch[32];
     __shared__ int int_scratch[32];
@@ -236,9 +234,8 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
     float* w = work + (size_t)r * vocab;
     const float temp = temperature[r];
     const float pen = penalty[r];
-    // the row's earlier tokens: a row of the `history` matrix, or the array whose address history_rows[r] holds (0: none)
-    int* h_row = history_rows ? reinterpret_cast<int*>(history_rows[r])
-                              : (history ? const_cast<int*>(history) + (size_t)r * history_stride : nullptr);
+    // the row's earlier tokens: the array whose address history_rows[r] holds (0: none)
+    int* h_row = history_rows ? reinterpret_cast<int*>(history_rows[r]) : nullptr;
     const bool penalised = pen > 1.0f && h_row && history_len[r] > 0;
 
     if (penalised) {
@@ -294,7 +291,7 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
     for (int i = tid; i < vocab; i += kThreads) w[i] = w[i] / sum;
     __syncthreads();
 
-    const float u = uniforms ? uniforms[r] : philox_uniform(seeds[r], counters[r]);
+    const float u = philox_uniform(seeds[r], counters[r]);
     int k = top_k[r];
     if (k <= 0 || k > vocab) k = vocab;
     const float nucleus = top_p[r];
@@ -487,10 +484,8 @@ __global__ void __launch_bounds__(kThreads, kResident)
 sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int vocab, float* __restrict__ work,
                            int* __restrict__ counts, const float* __restrict__ temperature, const int* __restrict__ top_k,
                            const float* __restrict__ top_p, const float* __restrict__ penalty,
-                           const int* __restrict__ history, int history_stride, const long long* __restrict__ history_rows, int append,
-                   const int* __restrict__ history_len,
-                           const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters,
-                           const float* __restrict__ uniforms, int* __restrict__ out) {
+                           const long long* __restrict__ history_rows, int append, const int* __restrict__ history_len,
+                           const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters, int* __restrict__ out) {
     __shared__ float block_tops[32];    // the maxima of this block's warps
     __shared__ float float_scratch[32];
     __shared__ int int_scratch[32];
@@ -519,9 +514,8 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
     float* w = slice_values - begin;
     const float temp = temperature[r];
     const float pen = penalty[r];
-    // the row's earlier tokens: a row of the `history` matrix, or the array whose address history_rows[r] holds (0: none)
-    int* h_row = history_rows ? reinterpret_cast<int*>(history_rows[r])
-                              : (history ? const_cast<int*>(history) + (size_t)r * history_stride : nullptr);
+    // the row's earlier tokens: the array whose address history_rows[r] holds (0: none)
+    int* h_row = history_rows ? reinterpret_cast<int*>(history_rows[r]) : nullptr;
     const bool penalised = pen > 1.0f && h_row && history_len[r] > 0;
 
     if (tid == 0) few_threshold = first_index = 0x7fffffff;
@@ -605,7 +599,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         return;
     }
 
-    const float u = uniforms ? uniforms[r] : philox_uniform(seeds[r], counters[r]);
+    const float u = philox_uniform(seeds[r], counters[r]);
     int k = top_k[r];
     if (k <= 0 || k > vocab) k = vocab;
     const float nucleus = top_p[r];
@@ -919,7 +913,7 @@ MB_EXPORT int mb_argmax_rows(const float* logits, int row_stride, int rows, int 
     return check_launch("argmax_rows");
 }
 
-// Per-row arrays live on the device.  `uniforms` (optional) overrides the generator, for tests.
+// Per-row arrays live on the device.
 // The host guarantees top_p == 1 for rows whose candidate count (top_k, or the vocabulary when
 // top_k <= 0) exceeds `mb_sample_max_sorted()`.
 // max_candidates: the host's bound on min(top_k, vocab) over the rows that cut anything (a row with top_k >= vocab and
@@ -927,13 +921,13 @@ MB_EXPORT int mb_argmax_rows(const float* logits, int row_stride, int rows, int 
 // kernel that spreads a row over a cluster of blocks.
 MB_EXPORT int mb_sample_rows(const float* logits, int row_stride, int rows, int vocab, float* work, int* counts,
                              const float* temperature, const int* top_k, const float* top_p, const float* penalty,
-                             const int* history, int history_stride, const long long* history_rows, int append, const int* history_len,
+                             const long long* history_rows, int append, const int* history_len,
                              const unsigned long long* seeds, const unsigned long long* counters,
-                             const float* uniforms, int* out, int max_candidates, cudaStream_t stream) {
+                             int* out, int max_candidates, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (vocab <= 0 || row_stride < vocab) return fail("sample_rows: vocab %d, row stride %d", vocab, row_stride);
     if (!work) return fail("sample_rows: needs rows * vocab floats of scratch");
-    if (!uniforms && (!seeds || !counters)) return fail("sample_rows: needs seeds and counters, or uniforms");
+    if (!seeds || !counters) return fail("sample_rows: needs seeds and counters");
     // a block of the cluster kernel keeps its eighth of a row in shared memory; a vocabulary too large for that (more
     // than 400,000 ids) takes the kernel that works in the scratch array
     const size_t slice_bytes = (size_t)((vocab + kSampleBlocks - 1) / kSampleBlocks) * sizeof(float);
@@ -959,14 +953,13 @@ MB_EXPORT int mb_sample_rows(const float* logits, int row_stride, int rows, int 
         config.attrs = attribute;
         config.numAttrs = 1;
         cudaError_t status = cudaLaunchKernelEx(&config, kernel, logits, row_stride, vocab, work, counts,
-                                                temperature, top_k, top_p, penalty, history, history_stride, history_rows, append, history_len, seeds,
-                                                counters, uniforms, out);
+                                                temperature, top_k, top_p, penalty, history_rows, append, history_len, seeds,
+                                                counters, out);
         if (status != cudaSuccess) return fail("sample_rows: launch failed: %s", cudaGetErrorString(status));
         return check_launch("sample_rows");
     }
     sample_rows_kernel<<<rows, kThreads, 0, stream>>>(logits, row_stride, vocab, work, counts, temperature, top_k, top_p,
-                                                      penalty, history, history_stride, history_rows, append, history_len, seeds, counters,
-                                                      uniforms, out);
+                                                      penalty, history_rows, append, history_len, seeds, counters, out);
     return check_launch("sample_rows");
 }
 

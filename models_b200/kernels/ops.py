@@ -2317,49 +2317,6 @@ def sample_max_sorted() -> int:
     return int(sampling().mb_sample_max_sorted())
 
 
-def sample_rows(logits: torch.Tensor, work: torch.Tensor, counts: Optional[torch.Tensor], temperature: torch.Tensor,
-                top_k: torch.Tensor, top_p: torch.Tensor, penalty: torch.Tensor, history: Optional[torch.Tensor],
-                history_len: Optional[torch.Tensor], seeds: Optional[torch.Tensor], counters: Optional[torch.Tensor],
-                uniforms: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-                max_candidates: int = 0, history_rows: Optional[torch.Tensor] = None, append: bool = False) -> torch.Tensor:
-    """One token per row of `logits` by the sampling pipeline.  `max_candidates`: the caller's bound on
-    min(top_k, vocabulary) over the rows, 0 if it has none; when every row keeps at most
-    sample_max_sorted() candidates a row is spread over a cluster of blocks instead of one block.
-    The earlier tokens of the rows (for the repetition penalty) are the rows of `history`, or the int32
-    arrays whose device addresses `history_rows` (int64 per row, 0: none) holds; `history_len` counts
-    them either way.  With `append` the kernel stores each row's new id behind its history (the arrays
-    of `history_rows` need room for it)."""
-    _cuda(logits, work, counts, temperature, top_k, top_p, penalty, history, history_len, seeds, counters, uniforms, history_rows)
-    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride()[1] != 1:
-        raise KernelError("sample_rows takes float32 [rows, vocab] logits")
-    rows, vocab = logits.shape
-    if work.dtype != torch.float32 or work.numel() < rows * vocab:
-        raise KernelError("sample_rows needs rows*vocab floats of scratch")
-    if counts is not None and (counts.dtype != torch.int32 or counts.numel() < rows * vocab):
-        raise KernelError("sample_rows needs rows*vocab int32 counters for the repetition penalty")
-    for name, t, dt in (("temperature", temperature, torch.float32), ("top_k", top_k, torch.int32),
-                        ("top_p", top_p, torch.float32), ("penalty", penalty, torch.float32)):
-        if t.dtype != dt or t.numel() < rows:
-            raise KernelError(f"{name} must hold {rows} values of {dt}")
-    _int32(history, "history")
-    _int32(history_len, "history_len")
-    if (history is not None or history_rows is not None) and (counts is None or history_len is None):
-        raise KernelError("a token history needs its lengths and the counters scratch")
-    if history_rows is not None and (history is not None or history_rows.dtype != torch.int64 or history_rows.numel() < rows):
-        raise KernelError(f"history_rows must hold {rows} int64 addresses and comes instead of a history matrix")
-    if append and history_rows is None:
-        raise KernelError("appending needs history_rows: a row of a history matrix has no room of its own")
-    if out is None:
-        out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
-    lib = sampling()
-    _run(lib, lib.mb_sample_rows(_p(logits), logits.stride()[0], rows, vocab, _p(work), _p(counts), _p(temperature),
-                                 _p(top_k), _p(top_p), _p(penalty), _p(history),
-                                 history.stride()[0] if history is not None else 0, _p(history_rows), 1 if append else 0,
-                                 _p(history_len), _p(seeds),
-                                 _p(counters), _p(uniforms), _p(out), int(max_candidates), _stream()))
-    return out
-
-
 def sample_parameter_words(rows: int) -> int:
     """8-byte words of the options of so many rows, as `sample_rows_packed` takes them."""
     return 3 * rows + (5 * rows + 1) // 2
@@ -2367,9 +2324,12 @@ def sample_parameter_words(rows: int) -> int:
 
 def sample_rows_packed(logits: torch.Tensor, work: torch.Tensor, counts: Optional[torch.Tensor], parameters: torch.Tensor,
                        max_candidates: int = 0, append: bool = False) -> torch.Tensor:
-    """`sample_rows` with the rows' options in one int64 array on the device: three words per row (all seeds, all draw counters, all
-    addresses of the histories, which count only with `counts`), then five 4-byte numbers per row (temperatures, top_p, penalties as
-    floats, top_k, lengths of the histories as integers)."""
+    """One token per row of `logits` by the sampling pipeline.  `parameters`: the rows' options in one int64 array on the device, three words
+    per row (all seeds, all draw counters, all addresses of the histories, int32 arrays of the rows' earlier tokens or 0, which count only
+    with `counts`), then five 4-byte numbers per row (temperatures, top_p, penalties as floats, top_k, lengths of the histories as
+    integers).  `max_candidates`: the caller's bound on min(top_k, vocabulary) over the rows, 0 if it has none; when every row keeps at
+    most sample_max_sorted() candidates a row is spread over a cluster of blocks instead of one block.  With `append` the kernel stores
+    each row's new id behind its history (which needs room for it)."""
     _cuda(logits, work, counts, parameters)
     if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride()[1] != 1:
         raise KernelError("sample_rows takes float32 [rows, vocab] logits")
@@ -2388,8 +2348,8 @@ def sample_rows_packed(logits: torch.Tensor, work: torch.Tensor, counts: Optiona
     histories = counts is not None
     lib = sampling()
     _run(lib, lib.mb_sample_rows(_p(logits), logits.stride()[0], rows, vocab, _p(work), _p(counts), number(0), number(3), number(1), number(2),
-                                 None, 0, ctypes.c_void_p(words + 16 * rows) if histories else None, 1 if append else 0,
-                                 number(4) if histories else None, ctypes.c_void_p(words), ctypes.c_void_p(words + 8 * rows), None, _p(out),
+                                 ctypes.c_void_p(words + 16 * rows) if histories else None, 1 if append else 0,
+                                 number(4) if histories else None, ctypes.c_void_p(words), ctypes.c_void_p(words + 8 * rows), _p(out),
                                  int(max_candidates), _stream()))
     return out
 
