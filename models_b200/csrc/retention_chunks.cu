@@ -53,15 +53,12 @@ struct RetentionArgs {
 // ceil(n / 64) chunks, and floor(f / 64) + ceil(n / 64) <= floor((f + n) / 64) + 1).
 __device__ __forceinline__ size_t place_of(int first, int seq, int chunk) { return (size_t)(first / kChunk) + seq + chunk; }
 
-// The rows of `count` tokens (64 with zeros behind them) of a head, `kCols` columns from `src`, activated, rotated (rotary > 0),
-// times weight[row] (or 1), in planes of rows of `row_numbers`.
-template <int kCols>
-__device__ __forceinline__ void stage_rows(bf16* planes, int row_numbers, int plane_numbers, const bf16* src, const RetentionArgs& args, int count,
-                                           int rotary, int position0, const float* weight) {
-    const int half = rotary / 2;
+// The queries or keys of `count` tokens (64 with zeros behind them) of a head, activated, rotated, times weight[row] (or 1), in planes.
+__device__ __forceinline__ void stage_turned_rows(bf16* planes, const bf16* src, const RetentionArgs& args, int count, int position0, const float* weight) {
+    const int rotary = args.rotary_dim, half = rotary / 2;
 #pragma unroll 2
-    for (int i = threadIdx.x; i < kChunk * kCols / 8; i += kThreads) {
-        const int row = i / (kCols / 8), c = i % (kCols / 8) * 8;
+    for (int i = threadIdx.x; i < kChunk * kDim / 8; i += kThreads) {
+        const int row = i / (kDim / 8), c = i % (kDim / 8) * 8;
         float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         if (row < count) {
             const bf16* from = src + (size_t)row * args.in_stride;
@@ -84,11 +81,12 @@ __device__ __forceinline__ void stage_rows(bf16* planes, int row_numbers, int pl
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] *= factor;
         }
-        store_parts(planes + row * row_numbers + c, plane_numbers, x);
+        store_parts(planes + row * kKeyRow + c, kKeyPlane, x);
     }
 }
 
-// A thread's part of the same rows without rotation: asked for, all of a block's rows before any is waited for, and later put in place.
+// A thread's part of rows of kCols columns (values, and queries and keys without rotation): asked for, all of a block's rows before any is
+// waited for, and later activated and put in place, the same numbers as above.
 template <int kCols>
 struct RawRows {
     static constexpr int kPieces = kChunk * kCols / 8 / kThreads;
@@ -152,7 +150,7 @@ retention_chunk_adds_kernel(const RetentionArgs args) {
     v.template put<true>(values, Values<V>::row, Values<V>::plane, args.input_act, count, nullptr);
     __syncthreads();
     if (args.rotary_dim == 0) k.template put<true>(keys, kKeyRow, kKeyPlane, args.input_act, count, weight);
-    else stage_rows<kDim>(keys, kKeyRow, kKeyPlane, key_rows, args, count, args.rotary_dim, args.positions[first] + chunk * kChunk, weight);
+    else stage_turned_rows(keys, key_rows, args, count, args.positions[first] + chunk * kChunk, weight);
     __syncthreads();
     const int tile = (tid >> 5) & 3, column0 = (tid >> 7) * (V / 2), lane = tid & 31;
     float acc[V / 16][4] = {};
@@ -244,8 +242,8 @@ retention_chunk_results_kernel(const RetentionArgs args) {
             k.template put<false>(keys, kKeyRow, kKeyPlane, args.input_act, count, nullptr);
         } else {
             const int position0 = args.positions[first] + chunk * kChunk;
-            stage_rows<kDim>(queries, kKeyRow, kKeyPlane, query_rows, args, count, args.rotary_dim, position0, nullptr);
-            stage_rows<kDim>(keys, kKeyRow, kKeyPlane, key_rows, args, count, args.rotary_dim, position0, nullptr);
+            stage_turned_rows(queries, query_rows, args, count, position0, nullptr);
+            stage_turned_rows(keys, key_rows, args, count, position0, nullptr);
         }
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {

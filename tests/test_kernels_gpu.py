@@ -1360,6 +1360,36 @@ def test_retention_chunks(cuda_device, vdim, lengths, whole):
         close(chunk_out, out, torch.bfloat16)
 
 
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("activation", [None, "silu", "gelu_tanh", "relu2"])
+def test_retention_chunks_rotated_by_nothing(cuda_device, vdim, activation):
+    """Rows that are rotated and rows that are not are activated by two pieces of code: one bit pattern, also where the activations' divisions are
+    unusual ones (gates below -40 and beyond 2^60)."""
+    from models_b200.kernels import ops
+
+    heads, dim, lengths = 2, 64, [100, 64, 33]
+    tokens = sum(lengths)
+    g = torch.Generator().manual_seed(vdim)
+    proj = torch.randn(tokens, heads * (2 * dim + vdim), generator=g) * 3
+    proj[::5, ::9] = -torch.rand(proj[::5, ::9].shape, generator=g) * 100
+    proj[7, heads * dim + 3], proj[90, heads * dim + 70], proj[120, 5], proj[130, -2] = 2.0 ** 61, 2.0 ** 60, 2.0 ** 40, -2.0 ** 61
+    q, k, v = proj.bfloat16().cuda().split([heads * dim, heads * dim, heads * vdim], dim=1)
+    decay, state0 = torch.tensor([0.97, 0.5]).cuda(), torch.randn(3, heads, dim, vdim, generator=g).cuda()
+    slots = torch.arange(3, dtype=torch.int32).cuda()
+    cu_q = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    positions = torch.cat([torch.arange(n) for n in lengths]).to(torch.int32).cuda()
+    found = []
+    for rotary in (0, 48, 64):
+        cos, sin = torch.ones(100, max(rotary, 2) // 2).cuda(), torch.zeros(100, max(rotary, 2) // 2).cuda()
+        state, raw = state0.clone(), torch.zeros(tokens, heads * vdim).cuda()
+        ops.retention_scan(q, k, v, None, positions, cos if rotary else None, sin if rotary else None, rotary, decay, 2.0 ** -70, 1e-6, state, slots, cu_q,
+                           heads, dim, vdim, None, 0.5, max(lengths), input_activation=activation, raw_out=raw)
+        found.append((raw, state))
+    assert bool(found[0][0].isfinite().all()) and bool(found[0][1].isfinite().all())
+    for raw, state in found[1:]:
+        assert torch.equal(raw, found[0][0]) and torch.equal(state, found[0][1])
+
+
 @pytest.mark.parametrize("lengths,most,chunks", [([64], 64, True), ([33, 31], 64, True), ([33, 30], 64, False), ([8] * 8, 64, False), ([16] * 8, 128, False),
                                                  ([16] * 8, 129, True)])
 def test_retention_steps_of_short_sequences_are_walked(cuda_device, lengths, most, chunks):
