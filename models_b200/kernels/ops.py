@@ -883,6 +883,8 @@ def prompt_attention(q: torch.Tensor, q_tail: Optional[torch.Tensor], k: torch.T
         _columns(gate, "gate")
         if gate.dtype != q.dtype or gate_kind not in ("head", "element") or tuple(gate.shape) != (rows, heads if gate_kind == "head" else out.shape[1]):
             raise KernelError(f"prompt_attention: a gate of kind {gate_kind!r} cannot be {tuple(gate.shape)} {gate.dtype}")
+        if gate_kind == "element" and gate.stride()[0] < gate.shape[1]:
+            gate = gate.clone(memory_format=torch.contiguous_format)  # (rows that overlap, one row for all for instance: TMA takes none)
     lib = float_weight_attention_library(key_dim, value_dim, turned, True)
     _run(lib, lib.mb_prompt_attention_tcgen05(
         _p(q), q.stride()[0], int(head_columns), q.shape[1], _p(q_tail), _p(k), _p(v), k.stride()[0], _p(k_tail), rows, _p(out), out.stride()[0],

@@ -402,6 +402,28 @@ def test_prompt_attention_with_gates_of_elements(cuda_device, heads, dim, rot, v
     assert bool((error <= 2.0 ** -6.99 * want[~nan].abs() + 1e-37).all())
 
 
+@pytest.mark.parametrize("lengths", [[130, 70], [1, 40]])
+def test_one_row_of_element_gates_for_every_token(cuda_device, lengths):
+    """Gates whose rows overlap are the rows that they stand for: an expanded row, and one of a single token whose stride says nothing."""
+    from models_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(len(lengths))
+    heads, dim = 2, 64
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda_device)  # noqa: E731
+
+    def run(lens, gate):
+        T = sum(lens)
+        q, kv = (torch.randn(T, n, generator=torch.Generator().manual_seed(n)).bfloat16().to(cuda_device) for n in (heads * dim, 2 * heads * dim))
+        out = torch.zeros(T, heads * dim, dtype=torch.bfloat16, device=cuda_device)
+        ops.prompt_attention(q, None, kv[:, :heads * dim], kv[:, heads * dim:], None, out, i32(np.concatenate([[0], np.cumsum(lens)]).tolist()), i32(lens),
+                             max(lens), heads, dim, dim, dim ** -0.5, gate, gate_kind="element")
+        return out
+
+    row = torch.randn(1, heads * dim, generator=g).bfloat16().to(cuda_device)
+    assert torch.equal(run(lengths, row.expand(sum(lengths), -1)), run(lengths, row.repeat(sum(lengths), 1)))
+    assert torch.equal(run([1], row.as_strided((1, heads * dim), (8, 1))), run([1], row))
+
+
 @pytest.mark.parametrize("heads,dim,rot,value_dim", [(2, 64, 0, 64), (2, 64, 64, 64), (2, 64, 0, 128), (1, 40, 24, 40)])
 @pytest.mark.parametrize("lengths,window", [([129, 160, 192], 0), ([193, 256, 257, 320], 0), ([64, 65, 128], 0), ([700], 1), ([700], 64), ([513, 129], 90),
                                             ([700], 200), ([1500] * 40, 0), ([160] * 200, 0)])
