@@ -359,8 +359,10 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 return true;
             };
             // A key tile is free as soon as its scores are there, a value tile a softmax and a product later: keys are asked for a ring's
-            // length ahead of the values, not behind the values of the page before.
-            constexpr int kAhead = kStages - 1;
+            // length ahead of the values, not behind the values of the page before.  (2,048 tokens, 16 heads, one launch after another: rows of
+            // 64 + 64 and 128 42.2 -> 41.7 us, gated by elements 45.6 -> 44.8, bounded scores 58.6 -> 58.1; plain pages, heads of 128, 41.0
+            // either way or slower, 41.3, and so is plain attention with rounded weights: there a page's keys and values come together.)
+            constexpr int kAhead = kContiguous || kShaped ? kStages - 1 : 0;
             bool ok = true;
             for (int t = 0; t < min(kAhead, pages) && ok; ++t) ok = bring_keys(t);
             for (int t = 0; t < pages && ok; ++t) {
@@ -585,7 +587,9 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             if (lane == 0) mbar_arrive(p_full + 8 * (t & 1));
         }
         // A warp's rows on their way out (see below), so many at a time; the first ones' tables are asked for while the last products are under way.
-        constexpr int kFours = VD / 4, kRowsAtOnce = 32 / kFours, kBatch = kContiguous ? 2 : kShaped ? 16 : 8;
+        // (Gates of elements, 1 / 2 / 4 / 8 rows: 100 tokens 17.4 / 15.4 / 16.5 / 17.3 us between two events, 2,048 48.2 / 48.1 / 48.1 / 49.1;
+        // tables, 4 / 8 / 16 / 32 rows: 17.5 / 15.4 / 14.5 / 14.4 and 55.3 / 53.3 / 52.3 / 54.3.)
+        constexpr int kFours = VD / 4, kRowsAtOnce = 32 / kFours, kBatch = kContiguous ? 2 : 16;
         const int four = lane % kFours, first = quarter * 32 + lane / kFours, last = min(quarter * 32 + 32, valid);
         const size_t token = q_begin + t0, column = (size_t)head * args.value_columns + 4 * four;
         const bool turns = kShaped && args.turn_cos != nullptr, mine_stored = 4 * four < args.value_columns && first < last;
@@ -608,11 +612,12 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             float inv = exp2f(kTruncationLift) / run_sum;  // the sum holds the lifted probabilities, the products their truncations
             if (kFloatWeights && args.gate != nullptr && !args.gate_element && row < valid)
                 inv *= 1.0f / (1.0f + expf(-__bfloat162float(args.gate[(size_t)(q_begin + t0 + row) * args.gate_stride + head])));
-            if (kFloatWeights) {
+            if (kFloatWeights && (gated || turns)) {
                 // Through shared memory (every product has read its tiles): a thread brings its row, and then the warp's lanes lie along the
                 // columns of its rows, one after another, so that tables and results are whole lines of memory; gates are there by then.  (A
                 // thread by itself along its row waited for its loads time and again: 26,000 cycles a block with gates of elements, 9,300
-                // with tables.  1,531 tokens on top of 700 cached positions each, 16 heads of 64 + 64 and 128: 48.3 -> 39.5 us.)
+                // with tables.  1,531 tokens on top of 700 cached positions each, 16 heads of 64 + 64 and 128: 48.3 -> 39.5 us.  With neither
+                // a thread's stores are quicker by themselves: launched one after another, 100 tokens 7.1 -> 6.0 us, 2 x 400 14.8 -> 13.6.)
                 float4* rows = reinterpret_cast<float4*>(smem + kResultsAt);  // [128][VD], the fours of a row turned by it
 #pragma unroll
                 for (int c = 0; c < VD; c += 32) {
@@ -630,7 +635,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                     *reinterpret_cast<uint2*>(args.out + (token + at) * args.out_row_stride + column) =
                         make_uint2(*reinterpret_cast<const uint32_t*>(&low), *reinterpret_cast<const uint32_t*>(&high));
                 };
-                if (mine_stored && gated) {
+                if (kContiguous && mine_stored) {
 #pragma unroll 1
                     for (int at0 = first; at0 < last; at0 += kBatch * kRowsAtOnce) {
                         float v[kBatch][4], z[4 * kBatch];
@@ -653,24 +658,21 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 } else if (mine_stored) {
 #pragma unroll 1
                     for (int at0 = first; at0 < last; at0 += kBatch * kRowsAtOnce) {
-                        if (turns && at0 > first) ask(at0);
+                        if (at0 > first) ask(at0);
 #pragma unroll
                         for (int i = 0; i < kBatch; ++i) {
-                            const int at = at0 + i * kRowsAtOnce;
+                            const int at = at0 + i * kRowsAtOnce, m = kShaped ? i : 0;
                             if (at >= last) break;
                             const float4 r = rows[at * kFours + (four ^ (at & 7))];
-                            float v[4] = {r.x, r.y, r.z, r.w};
-                            if (turns) {  // back by the query's position
-                                const int m = kShaped ? i : 0;
-                                v[0] = r.x * cs[m].x + r.y * sn[m].x, v[1] = r.y * cs[m].x - r.x * sn[m].x;
-                                v[2] = r.z * cs[m].y + r.w * sn[m].y, v[3] = r.w * cs[m].y - r.z * sn[m].y;
-                            }
+                            const float v[4] = {r.x * cs[m].x + r.y * sn[m].x, r.y * cs[m].x - r.x * sn[m].x,  // back by the query's position
+                                                r.z * cs[m].y + r.w * sn[m].y, r.w * cs[m].y - r.z * sn[m].y};
                             store(at, v);
                         }
                     }
                 }
             } else {
-                bf16* dst = args.out + (size_t)(q_begin + t0 + row) * args.out_row_stride + (size_t)head * VD;
+                const int value_columns = kFloatWeights ? args.value_columns : VD;
+                bf16* dst = args.out + (size_t)(q_begin + t0 + row) * args.out_row_stride + (size_t)head * value_columns;
 #pragma unroll
                 for (int c = 0; c < VD; c += 32) {
                     uint32_t r[32];
@@ -679,6 +681,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                     if (row < valid) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {
+                            if (c + i >= value_columns) continue;
                             float piece[8];
 #pragma unroll
                             for (int j = 0; j < 8; ++j) piece[j] = __uint_as_float(r[i + j]) * inv;
