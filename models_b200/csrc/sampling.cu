@@ -440,8 +440,8 @@ sample_rows_kernel(const float* __restrict__ logits, int row_stride, int vocab, 
 // Few candidates (k <= kFewCandidates) need no histograms: the maxima of the row's 256 warps are 256 of its values, so the k-th
 // largest of them is at most the row's k-th largest, and hardly more than k values reach it (40 of 128,256 random values: 44).
 // They are gathered while the exponentials are summed; should more reach it than can be sorted, the histograms decide, and at once where
-// fewer warps than k have a finite value (rows masked to ten finite values, 1 and 64 rows: 39.7 and 133 us; 47.6 and 152 before that was
-// looked at).
+// fewer warps than k have a finite value (rows masked to ten finite values, 1 and 64 rows: 36 and 116 us; 42 and 135 while four infinities
+// were divided like numbers).
 // (64 rows of 128,256, k 20 to 64: 119 us with histograms and one block a multiprocessor, 53 with this and two, 41.6 since maxima carry no
 // index, quotients are corrected reciprocals and a sum's exponentials are not stored: 110 instructions a logit had been its bound.  What
 // bounds it now is a chain of passes, cluster barriers and the first block's draw, in two rounds of clusters; one row takes 13.4 us.)
@@ -473,7 +473,7 @@ __device__ __forceinline__ void divide_four(float4& q, float by, float inverse, 
             a = fmaf(fmaf(-a, by, v[i]), inverse, a);
             v[i] = fmaf(fmaf(-a, by, v[i]), inverse, a);
         }
-    } else {
+    } else if (!(usual && least == CUDART_INF_F)) {  // (four infinities stay what they are: most of a masked row)
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = v[i] / by;
     }
@@ -631,7 +631,8 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int row_stride, int
         }
     }
 
-    // softmax over the whole vocabulary: the sum of the exponentials, each thread's in the order of its ids
+    // softmax over the whole vocabulary: the sum of the exponentials, each thread's in the order of its ids.  (They are not stored: a row of few
+    // candidates does not need them again, and one whose sum is no number looks for its maximum among the values.)
     float local = 0.0f;
     bool gathers = few;  // a thread that finds no place left stops: the histograms will decide
 #pragma unroll 4

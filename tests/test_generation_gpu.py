@@ -385,6 +385,27 @@ def test_sampling_over_a_cluster_follows_the_reference_pipeline(cuda_device, voc
     assert float(seen.sum()) == 1.0 and float((seen - expected).abs().max()) < 0.07, seen
 
 
+@pytest.mark.parametrize("temperature", [0.7, 2.0 ** -31, 3e9])
+@pytest.mark.parametrize("vocab", [4100, 5003])
+def test_masked_rows_under_a_temperature(cuda_device, vocab, temperature):
+    """Fours of infinities, which are not divided, beside fours with one finite number, few candidates and many; a row with +infinity takes its
+    first maximum."""
+    from models_b200.sampling import BatchSampler, RequestSampling, SamplingOptions, philox_uniform
+
+    g = torch.Generator().manual_seed(vocab)
+    options = [SamplingOptions(temperature=temperature, top_k=k, top_p=p, seed=k) for k in (1, 40, 200) for p in (0.6, 1.0)] * 2
+    logits = torch.full((len(options), vocab), -float("inf"))
+    for row in range(len(options)):
+        finite = torch.randperm(vocab, generator=g)[:10 if row < 6 else 1500]
+        logits[row, finite] = torch.randn(len(finite), generator=g) * 4 * min(temperature, 1e6)
+    got = BatchSampler(vocab, "cuda:0").sample(logits.cuda(), [RequestSampling(o, [0]) for o in options]).tolist()
+    for row, o in enumerate(options):
+        want, _ = expected_draw(logits[row].numpy(), [], o, philox_uniform(o.seed, 0))
+        assert got[row] == want, (row, o, got[row], want)
+    logits[:, 2050] = logits[:, 2049] = float("inf")
+    assert BatchSampler(vocab, "cuda:0").sample(logits.cuda(), [RequestSampling(o, [0]) for o in options]).tolist() == [2049] * len(options)
+
+
 @pytest.mark.parametrize("rows", [1, 8, 64, 300])
 @pytest.mark.parametrize("vocab", [1025, 5003])
 def test_rows_that_cut_nothing_draw_the_same_every_time(cuda_device, vocab, rows):
