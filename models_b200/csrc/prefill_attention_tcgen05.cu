@@ -616,7 +616,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 // Through shared memory (every product has read its tiles): a thread brings its row, and then the warp's lanes lie along the
                 // columns of its rows, one after another, so that tables and results are whole lines of memory; gates are there by then.  (A
                 // thread by itself along its row waited for its loads time and again: 26,000 cycles a block with gates of elements, 9,300
-                // with tables.  1,531 tokens on top of 700 cached positions each, 16 heads of 64 + 64 and 128: 48.3 -> 39.5 us.  With neither
+                // with tables.  1,531 tokens on top of 700 cached positions each, 16 heads of 64 + 64 and 128, gated: 51.7 -> 41.4 us.  With neither
                 // a thread's stores are quicker by themselves: launched one after another, 100 tokens 7.1 -> 6.0 us, 2 x 400 14.8 -> 13.6.)
                 float4* rows = reinterpret_cast<float4*>(smem + kResultsAt);  // [128][VD], the fours of a row turned by it
 #pragma unroll

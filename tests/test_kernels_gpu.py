@@ -1602,7 +1602,7 @@ def test_shaped_scores_on_tcgen05(cuda_device, dim, vdim, cap, sink, turned):
 @pytest.mark.parametrize("cap", [50.0, 8.0])
 @pytest.mark.parametrize("size", [0.3, 1.0, 2.2, 6.0])
 def test_bounded_scores_small_and_large(cuda_device, cap, size):
-    """Scores from well within the polynomial's reach to far beyond it, in the same rows and in rows of their own, against 64 bits: the
+    """Scores without a word on their size, from small ones to far beyond the bound, in the same rows and in rows of their own, against 64 bits: the
     weights' two bfloat16 parts (2^-16), the score's float arithmetic and the result's rounding (eight bits: up to 2^-8 of it)."""
     from models_b200.kernels import ops
 
